@@ -149,6 +149,37 @@ def run_reference(args, rank, world):
 NCU_BWD_TRAFFIC_B2 = {"fp8": 163.8e6, "fp4": 221.8e6}
 
 
+def kernel_calls(q, k, v, g, causal, fp4):
+    """The kernel-level calls of one fwd+bwd step on the default route, in order, as (name, function, args, keywords), each run
+    once here for the next ones' operands: the launches of the public call."""
+    import torch
+    from flamia_blackwell_attention_b200 import kernels as K, _lib as L
+    b, s, h, d = q.shape
+    sm = 1.0 / math.sqrt(d)
+    mode = L.FL_MODE_FP4 if fp4 else L.FL_MODE_FP8
+    calls = []
+
+    def call(f, *a, **kw):
+        calls.append((f.__name__, f, a, kw))
+        return f(*a, **kw)
+    qk = dict(apply_hadamard_rotation=True, hadamard_rotation_scope="nvfp4_copy" if fp4 else "all", also_make_nvfp4_copy=fp4,
+              output_exponent_table=False)
+    status = K.new_status(q.device)
+    qq = call(K.quantize_fp8_blocks, q, status=status, **qk)
+    kq = call(K.quantize_fp8_blocks, k, status=status, output_tile_stats=True, **qk)
+    vq = call(K.quantize_fp8_blocks, v, status=status, output_tile_stats=True, output_exponent_table=False)
+    out, lse, _ = call(K.attn_fwd, qq, kq, vq, causal=causal, softmax_scale=sm, out_dtype=q.dtype, mode=mode, status=status,
+                       p_group=fp4)
+    acc = torch.empty(b, h, s, d, dtype=torch.float16, device=q.device)
+    gq = call(K.quantize_fp8_blocks, g, compute_d_with_output=out, shifted_log2_lse_from=lse, log2_lse_shift=8.0,
+              d_multiplier=-2.0 ** -8, zero_accumulator=acc, output_tile_stats=True, status=status, output_exponent_table=False)
+    ks, ps = call(K.dq_prescale, gq["tile_stats"], vq["tile_stats"], kq["tile_stats"])
+    call(K.attn_bwd, qq, kq, vq, gq, lse_log2=gq["lse_log2"], d_rows=gq["D"], dq_acc=acc, dq_scale=ks, causal=causal,
+         softmax_scale=sm, out_dtype=q.dtype, mode=mode, had_dk=not fp4, status=status)
+    call(K.dq_post, acc, ps, sm, b=b, s=s, h=h, d=d, unrotate=not fp4, out_dtype=q.dtype)
+    return calls
+
+
 def measure_route(fn, route, causal, tensors, args, world, dist, K, clock_gpu=None):
     """Sustained step time of one public fwd+bwd call + per-kernel CUDA-event times. Returns a dict (this rank's values)."""
     import torch
@@ -202,26 +233,10 @@ def measure_route(fn, route, causal, tensors, args, world, dist, K, clock_gpu=No
     wall1 = time.time()
     clocks = sampler.stop((wall0, wall1)) if sampler else None
     ms = sorted(batches)[len(batches) // 2]
-    # ---- per-kernel device times: the arguments of every kernel-level call of one eager step are recorded, then each
-    # call is captured alone in a CUDA graph (10 launches) and replayed for ~0.25 s: a sustained time per launch without
-    # host launch gaps (events around eager launches measure the host when a kernel is shorter than its launch)
-    calls = []
-    names = ("quantize_fp8_blocks", "attn_fwd", "dq_prescale", "attn_bwd", "dq_post")
-    orig = {n: getattr(K, n) for n in names}
-
-    def recorder(name, f):
-        def w(*a, **kw):
-            calls.append((name, f, a, kw))
-            return f(*a, **kw)
-        return w
-    for n in names:
-        setattr(K, n, recorder(n, orig[n]))
-    try:
-        step()
-        torch.cuda.synchronize()
-    finally:
-        for n, f in orig.items():
-            setattr(K, n, f)
+    # ---- per-kernel device times: every kernel-level call of one step is captured alone in a CUDA graph (10 launches) and
+    # replayed for ~0.25 s: a sustained time per launch without host launch gaps (events around eager launches measure the
+    # host when a kernel is shorter than its launch)
+    calls = kernel_calls(q.detach(), k.detach(), v.detach(), g, causal, route == "fp4")
     per = {}
     labels = []
     n_rep = 10

@@ -10,6 +10,7 @@ import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libflamia_b200.so")
+HOST_PATH = os.path.join(HERE, "_host.so")
 
 # status codes (csrc/sm100.cuh)
 ABI_VERSION = 8
@@ -57,6 +58,8 @@ EXPORTS = {
     "fl_token_aux": (i32, [vp, C.c_int64, vp, vp, vp]),
     "fl_dq_post_packed": (i32, [vp, vp, f32, vp, i32, i32, i32, i32, i32, vp, vp, vp]),
     "fl_dq_prescale_rows": (i32, [vp, vp, vp, i32, i32, f32, vp, vp, vp]),
+    "fl_doc_tables": (i32, [vp, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp]),
+    "fl_unpack_lse": (i32, [vp, vp, vp, i32, i32, i32, i32, vp, vp]),
     "fl_pack_rows": (i32, [vp, vp, vp, i32, i32, vp]),
     "fl_unpack_rows": (i32, [vp, vp, vp, i32, i32, vp]),
     "fl_selftest_mma": (i32, [i32, vp, vp, vp, vp, vp, vp, i64, vp]),
@@ -81,6 +84,23 @@ def load():
         fn.restype, fn.argtypes = res, args
     _lib = lib
     return lib
+
+
+_host = None
+
+
+def host():
+    """The native host module (cached): the registered ops' implementations and the call path (csrc/host.cpp). Importing it
+    registers the CUDA and autograd kernels of lowbit_attn::fp8 / ::fp4."""
+    global _host
+    if _host is None:
+        if not os.path.exists(HOST_PATH):
+            raise ImportError(f"{HOST_PATH} is missing: build it with `python -m flamia_blackwell_attention_b200.build`. "
+                              "There is no fallback path.")
+        load()
+        from . import _host as h
+        _host = h
+    return _host
 
 
 def check(rc: int, what: str):

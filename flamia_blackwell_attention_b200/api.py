@@ -5,7 +5,7 @@ registered op lowbit_attn::fp8 / ::fp4, whose autograd node carries the plan han
 """
 from __future__ import annotations
 
-import functools
+import threading
 import warnings
 from dataclasses import dataclass
 from typing import Callable, Optional, Tuple
@@ -13,6 +13,7 @@ from typing import Callable, Optional, Tuple
 import torch
 
 from . import _op
+from . import interface_bwd_fp4 as _switches
 from .options import FP4AttnOptions, FP8AttnOptions
 from .plan import AttnPlan, _fail, resolve_fp4, resolve_fp8
 
@@ -21,64 +22,65 @@ __all__ = ["flash_attn_fp4", "flash_attn_fp8"]
 _REPACK_WARNED = False
 REPACK_WARNING = (
     "flash_attn_{entry} got cu_seqlens_q / cu_seqlens_k without seqused_q / seqused_k. No tensor is copied (the kernels "
-    "read and write the packed rows in place), but the document tables are rebuilt on the device on every call (a dozen "
-    "small launches) and the intermediates take a padded buffer of up to 127 extra rows per document. Build the tables "
+    "read and write the packed rows in place), but the document tables are rebuilt on the device on every call (one "
+    "small launch) and the intermediates take a padded buffer of up to 127 extra rows per document. Build the tables "
     "once with DocMaps.from_cu_seqlens(...) and pass doc_maps=, or lay the documents out at starts that are multiples of "
     "128 and pass the true lengths as seqused_q / seqused_k. (Warned once.)")
 
 
 @dataclass(frozen=True)
-class _TensorFacts:
+class _Resolved:
+    """A resolved plan as the call path uses it."""
+    plan: AttnPlan
+    handle: int          # of the native plan registry
+    plain: bool          # batched, native head dim, whole tiles, no seqused_k: nothing to check or to convert per call
+
+
+# Call key -> _Resolved. A plan is a pure function of the argument values and of the tensors' metadata, which is what the key
+# holds (a flat tuple: building and hashing frozen dataclasses of the same facts was 40 us of every call). Bounded: the oldest
+# entry goes first; a refusal raises and is not remembered.
+_CALLS: dict = {}
+_CALLS_MAX = 1024
+_CALLS_LOCK = threading.Lock()
+
+
+def _facts(t):
     """What plan resolution may look at in a tensor argument: nothing but metadata."""
-    shape: Tuple[int, ...]
-    dtype: torch.dtype
-    requires_grad: bool
-
-    @staticmethod
-    def of(t):
-        return _TensorFacts(tuple(t.shape), t.dtype, bool(t.requires_grad)) if isinstance(t, torch.Tensor) else t
-
-    def stand_in(self):
-        grad = self.requires_grad and self.dtype.is_floating_point
-        return torch.empty(self.shape, dtype=self.dtype, device="meta", requires_grad=grad)
+    return t.shape, t.dtype, t.requires_grad
 
 
-@dataclass(frozen=True)
-class _CallFacts:
-    """Hashable description of one call: everything a plan depends on and nothing else."""
-    entry: str
-    grad_mode: bool
-    dq_causal_prescale: Tuple[bool, str]      # the module switches the resolver reads: (on, granularity)
-    q: _TensorFacts
-    k: _TensorFacts
-    v: _TensorFacts
-    keywords: Tuple[Tuple[str, object], ...]
+def _stand_in(t):
+    if not isinstance(t, torch.Tensor):
+        return t
+    return torch.empty(t.shape, dtype=t.dtype, device="meta", requires_grad=t.requires_grad and t.dtype.is_floating_point)
 
 
-@functools.lru_cache(maxsize=1024)
-def _plan_of(facts: _CallFacts) -> AttnPlan:
-    # plans are pure functions of argument values and tensor metadata, so they are resolved on meta stand-ins; a refusal
-    # raises out of here and is not remembered
-    resolve = resolve_fp8 if facts.entry == "fp8" else resolve_fp4
-    kw = {n: (x.stand_in() if isinstance(x, _TensorFacts) else x) for n, x in facts.keywords}
-    with torch.set_grad_enabled(facts.grad_mode):
-        return resolve(facts.q.stand_in(), facts.k.stand_in(), facts.v.stand_in(), **kw)
+def _resolve(entry, resolve, q, k, v, kw) -> _Resolved:
+    if all(isinstance(t, torch.Tensor) for t in (q, k, v)):     # (otherwise the resolver words the refusal)
+        q, k, v = _stand_in(q), _stand_in(k), _stand_in(v)
+        kw = {n: _stand_in(x) for n, x in kw.items()}
+    plan = resolve(q, k, v, **kw)
+    plain = not (plan.shape.varlen or plan.fwd.ragged_documents or plan.fwd.seqused_k or plan.pad_from)
+    return _Resolved(plan, _op.register_plan(plan), plain)
 
 
-def _cached_plan(resolve, q, k, v, kw) -> AttnPlan:
-    from . import interface_bwd_fp4
-    entry = "fp8" if resolve is resolve_fp8 else "fp4"
-    if not all(isinstance(t, torch.Tensor) for t in (q, k, v)):
-        return resolve(q, k, v, **kw)           # the resolver words the refusal
-    facts = _CallFacts(entry, torch.is_grad_enabled(),
-                       (bool(interface_bwd_fp4.DQ_CAUSAL_PRESCALE), str(interface_bwd_fp4.DQ_CAUSAL_GRANULARITY)), _TensorFacts.of(q),
-                       _TensorFacts.of(k), _TensorFacts.of(v), tuple(sorted((n, _TensorFacts.of(x)) for n, x in kw.items())))
+def _resolved(entry, resolve, names, q, k, v, *values) -> _Resolved:
+    """The resolved plan of a call; names / values: its keyword arguments in the resolver's names."""
     try:
-        return _plan_of(facts)
-    except TypeError as exc:
-        if getattr(exc, "rule", None) is not None:
-            raise
-        return resolve(q, k, v, **kw)           # an unhashable argument (e.g. a callable object): resolve uncached
+        # (entry, mode, the module switches the resolver reads, tensor metadata, argument values)
+        key = (entry, torch.is_grad_enabled(), _switches.DQ_CAUSAL_PRESCALE, _switches.DQ_CAUSAL_GRANULARITY,
+               q.shape, q.dtype, q.requires_grad, k.shape, k.dtype, k.requires_grad, v.shape, v.dtype, v.requires_grad,
+               *[x if not isinstance(x, torch.Tensor) else _facts(x) for x in values])
+        hit = _CALLS.get(key)
+    except (AttributeError, TypeError):         # not tensors, or an unhashable argument (e.g. a callable object): uncached
+        return _resolve(entry, resolve, q, k, v, dict(zip(names, values)))
+    if hit is None:
+        hit = _resolve(entry, resolve, q, k, v, dict(zip(names, values)))
+        with _CALLS_LOCK:
+            while len(_CALLS) >= _CALLS_MAX:
+                del _CALLS[next(iter(_CALLS))]
+            _CALLS[key] = hit
+    return hit
 
 
 def _doc_maps_args(maps, q, cu_q, cu_k, su_q, su_k):
@@ -95,10 +97,14 @@ def _doc_maps_args(maps, q, cu_q, cu_k, su_q, su_k):
     return maps.cu, maps.cu, maps.max_seqlen, maps.max_seqlen
 
 
-def _run(plan, q, k, v, cu_q, cu_k, su_q, su_k, return_lse, doc_maps=None):
+def _run(call, q, k, v, cu_q, cu_k, su_q, su_k, return_lse, doc_maps=None):
     global _REPACK_WARNED
+    plan = call.plan
     if not q.is_cuda:
         raise RuntimeError(f"flash_attn_{plan.entry}: q, k, v must be CUDA tensors (this library has no CPU path)")
+    if call.plain:
+        out, lse = _op.op_apply(plan.entry, call.handle, q, k, v, ())
+        return (out, lse) if return_lse else out
     sh = plan.shape
     if sh.varlen and sh.tot_q != sh.tot_k:
         _fail("B8", NotImplementedError, "packed documents are self-attention documents here: q and k must share "
@@ -119,16 +125,16 @@ def _run(plan, q, k, v, cu_q, cu_k, su_q, su_k, return_lse, doc_maps=None):
         _REPACK_WARNED = True
         warnings.warn(REPACK_WARNING.format(entry=plan.entry), UserWarning, stacklevel=3)
     if doc_maps is not None:
-        docs = doc_maps.tensors()           # cu, start, len, row_map, slot_src, slot_rows: nothing is computed per call
+        docs = tuple(doc_maps.tensors())    # cu, start, len, row_map, slot_src, slot_rows: nothing is computed per call
     else:
-        docs = [t for t in (cu_q, cu_k, su_q, su_k) if t is not None] if sh.varlen else \
-            ([su_k.contiguous()] if plan.fwd.seqused_k else [])
+        docs = tuple(t for t in (cu_q, cu_k, su_q, su_k) if t is not None) if sh.varlen else \
+            ((su_k.contiguous(),) if plan.fwd.seqused_k else ())
     if plan.pad_from:
         # head dim below the kernels' 64 / 128: zero columns on the way in (differentiable: the gradients of the pad
         # are the first head_dim columns of dQ / dK / dV), the first head_dim columns of O on the way out
         extra = sh.d - plan.pad_from
         q, k, v = (torch.nn.functional.pad(t, (0, extra)) for t in (q, k, v))
-    out, lse = _op.op_apply(plan, q, k, v, docs)
+    out, lse = _op.op_apply(plan.entry, call.handle, q, k, v, docs)
     if plan.pad_from:
         out = out[..., :plan.pad_from].contiguous()
     if return_lse:
@@ -137,6 +143,12 @@ def _run(plan, q, k, v, cu_q, cu_k, su_q, su_k, return_lse, doc_maps=None):
                                     "repacked documents")
         return out, lse
     return out
+
+
+_COMMON_NAMES = ("softmax_scale", "causal", "window_size", "softcap", "score_mod", "score_mod_bwd", "mask_mod", "cu_seqlens_q",
+                 "cu_seqlens_k", "max_seqlen_q", "max_seqlen_k", "seqused_k", "seqused_q", "deterministic", "return_lse")
+_FP8_NAMES = _COMMON_NAMES + ("qk_hadamard", "q_quantized", "k_quantized", "q_scale_fused", "options")
+_FP4_NAMES = _COMMON_NAMES + ("pv_precision", "backward", "causal_safety", "qk_hadamard", "options")
 
 
 def flash_attn_fp8(q, k, v, *, softmax_scale: Optional[float] = None, causal: bool = False,
@@ -173,13 +185,10 @@ def flash_attn_fp8(q, k, v, *, softmax_scale: Optional[float] = None, causal: bo
             cu_seqlens_k=cu_seqlens_k, max_seqlen_q=max_seqlen_q, max_seqlen_k=max_seqlen_k, seqused_k=seqused_k,
             seqused_q=seqused_q, deterministic=deterministic, return_lse=return_lse, qk_hadamard=qk_hadamard,
             q_quantized=q_quantized, k_quantized=k_quantized, q_scale_fused=q_scale_fused, options=options), return_lse)
-    plan = _cached_plan(resolve_fp8, q, k, v, dict(
-        softmax_scale=softmax_scale, causal=causal, window_size=tuple(window_size), softcap=softcap, score_mod=score_mod,
-        score_mod_bwd=score_mod_bwd, mask_mod=mask_mod, cu_seqlens_q=cu_seqlens_q, cu_seqlens_k=cu_seqlens_k,
-        max_seqlen_q=max_seqlen_q, max_seqlen_k=max_seqlen_k, seqused_k=seqused_k, seqused_q=seqused_q,
-        deterministic=deterministic, return_lse=return_lse, qk_hadamard=qk_hadamard, q_quantized=q_quantized,
-        k_quantized=k_quantized, q_scale_fused=q_scale_fused, options=options))
-    return _run(plan, q, k, v, cu_seqlens_q, cu_seqlens_k, seqused_q, seqused_k, return_lse, doc_maps)
+    call = _resolved("fp8", resolve_fp8, _FP8_NAMES, q, k, v, softmax_scale, causal, tuple(window_size), softcap, score_mod,
+                     score_mod_bwd, mask_mod, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, seqused_k, seqused_q,
+                     deterministic, return_lse, qk_hadamard, q_quantized, k_quantized, q_scale_fused, options)
+    return _run(call, q, k, v, cu_seqlens_q, cu_seqlens_k, seqused_q, seqused_k, return_lse, doc_maps)
 
 
 def flash_attn_fp4(q, k, v, *, softmax_scale: Optional[float] = None, causal: bool = False,
@@ -205,10 +214,7 @@ def flash_attn_fp4(q, k, v, *, softmax_scale: Optional[float] = None, causal: bo
                                "feature of the reference and are not built here")
     if aux_tensors is not None:
         _fail("B3", NotImplementedError, "aux_tensors belong to score_mod / mask_mod, which this library does not take")
-    plan = _cached_plan(resolve_fp4, q, k, v, dict(
-        softmax_scale=softmax_scale, causal=causal, window_size=tuple(window_size), softcap=softcap, score_mod=score_mod,
-        score_mod_bwd=score_mod_bwd, mask_mod=mask_mod, cu_seqlens_q=cu_seqlens_q, cu_seqlens_k=cu_seqlens_k,
-        max_seqlen_q=max_seqlen_q, max_seqlen_k=max_seqlen_k, seqused_k=seqused_k, seqused_q=seqused_q,
-        deterministic=deterministic, return_lse=return_lse, pv_precision=pv_precision, backward=backward,
-        causal_safety=causal_safety, qk_hadamard=qk_hadamard, options=options))
-    return _run(plan, q, k, v, cu_seqlens_q, cu_seqlens_k, seqused_q, seqused_k, return_lse, doc_maps)
+    call = _resolved("fp4", resolve_fp4, _FP4_NAMES, q, k, v, softmax_scale, causal, tuple(window_size), softcap, score_mod,
+                     score_mod_bwd, mask_mod, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, seqused_k, seqused_q,
+                     deterministic, return_lse, pv_precision, backward, causal_safety, qk_hadamard, options)
+    return _run(call, q, k, v, cu_seqlens_q, cu_seqlens_k, seqused_q, seqused_k, return_lse, doc_maps)

@@ -264,6 +264,67 @@ __global__ void __launch_bounds__(128) code_stats_kernel(const uint8_t* __restri
   }
 }
 
+// ------------------------------------------------------------------------------------------------ document tables
+// Packed documents (boundaries cu, or n documents of one length) laid out at 128-aligned starts of a buffer of `capacity`
+// rows: start / len per document, the source row of every buffer row (-1: padding), and per 128-row slot its first source
+// row and its number of real rows. One launch; as tensor operations the same tables were a dozen launches.
+// Each CTA owns DT_SLOTS slots: it scans all documents (the padded lengths' prefix sum: n / DT_THREADS documents per thread,
+// in document order), notes the document of each of its slots in shared memory, then writes its rows coalesced.
+static constexpr int DT_THREADS = 256, DT_SLOTS = 16;
+__global__ void __launch_bounds__(DT_THREADS) doc_tables_kernel(const int32_t* __restrict__ cu, int n, int fixed_len, int total,
+                                                                int capacity, int32_t* __restrict__ start,
+                                                                int32_t* __restrict__ len, int32_t* __restrict__ row_map,
+                                                                int32_t* __restrict__ slot_src, int32_t* __restrict__ slot_rows) {
+  __shared__ int s_warp[DT_THREADS / 32];
+  __shared__ int s_src[DT_SLOTS], s_rows[DT_SLOTS];      // first source row of the slot, real rows from there
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int slot0 = blockIdx.x * DT_SLOTS, n_slots = min(DT_SLOTS, capacity / 128 - slot0);
+  if (tid < DT_SLOTS) { s_src[tid] = -1; s_rows[tid] = 0; }
+  auto doc_len = [&](int i) { return cu ? cu[i + 1] - cu[i] : fixed_len; };
+  auto slots_of = [](int l) { return l > 0 ? (l + 127) / 128 : 0; };
+  const int per = (n + DT_THREADS - 1) / DT_THREADS, lo = min(n, tid * per), hi = min(n, lo + per);
+  int mine = 0;
+  for (int i = lo; i < hi; ++i) mine += slots_of(doc_len(i));
+  int inc = mine;                                        // inclusive scan over the threads
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  if (lane == 31) s_warp[warp] = inc;
+  __syncthreads();
+  int at = inc - mine;
+  for (int w = 0; w < warp; ++w) at += s_warp[w];
+  for (int i = lo; i < hi; ++i) {
+    const int l = doc_len(i), ns = slots_of(l), src = cu ? cu[i] : i * fixed_len;
+    if (blockIdx.x == 0) { start[i] = at * 128; len[i] = l; }
+    for (int x = max(at, slot0); x < min(at + ns, slot0 + n_slots); ++x) {
+      const int r0 = src + (x - at) * 128;
+      // (a row outside the source is nobody's: a boundary past the end must not send a kernel out of bounds)
+      const int rows = r0 < 0 ? 0 : min(min(128, l - (x - at) * 128), total - r0);
+      if (rows > 0) { s_src[x - slot0] = r0; s_rows[x - slot0] = rows; }
+    }
+    at += ns;
+  }
+  __syncthreads();
+  if (tid < n_slots) { slot_src[slot0 + tid] = s_src[tid]; slot_rows[slot0 + tid] = s_rows[tid]; }
+  for (int i = tid; i < n_slots * 128; i += DT_THREADS) {
+    const int x = i >> 7, r = i & 127;
+    row_map[slot0 * 128 + i] = r < s_rows[x] ? s_src[x] + r : -1;
+  }
+}
+
+// The live rows of the aligned buffer's LSE (h, capacity) to the caller's rows: packed row g = seq * k + i goes to
+// out[k][head][i] (packed documents: seq = total, so out is (h, total)).
+__global__ void __launch_bounds__(128) unpack_lse_kernel(const float* __restrict__ lse, const int32_t* __restrict__ slot_src,
+                                                         const int32_t* __restrict__ slot_rows, int capacity, int h, int seq,
+                                                         float* __restrict__ out) {
+  const int slot = blockIdx.x, head = blockIdx.y, r = threadIdx.x;
+  if (slot_src[slot] < 0 || r >= slot_rows[slot]) return;
+  const int g = slot_src[slot] + r;
+  out[((size_t)(g / seq) * h + head) * seq + g % seq] = lse[(size_t)head * capacity + slot * 128 + r];
+}
+
 // ------------------------------------------------------------------------------------------------ packed rows
 __global__ void pack_rows_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, const int32_t* __restrict__ map,
                                  int n_rows, int chunks) {
@@ -380,6 +441,27 @@ extern "C" int fl_code_stats(const void* codes, const float* descale, int32_t b,
   if (h > 65535 || b > 65535) return FL_ERR_TOO_LARGE;
   code_stats_kernel<<<dim3(s / 128, h, b), 128, 0, (cudaStream_t)stream>>>((const uint8_t*)codes, descale, s, h, d, tile_stats);
   return launch_result("fl_code_stats: kernel launch");
+}
+
+extern "C" int fl_doc_tables(const int32_t* cu, int32_t n_docs, int32_t fixed_len, int32_t total, int32_t capacity, int32_t* start,
+                             int32_t* len, int32_t* row_map, int32_t* slot_src, int32_t* slot_rows, void* stream) {
+  using namespace fl;
+  if (!start || !len || !row_map || !slot_src || !slot_rows || n_docs <= 0 || total <= 0 || capacity <= 0 || (capacity % 128) ||
+      (!cu && (fixed_len <= 0 || (long long)fixed_len * n_docs > total)))
+    return FL_ERR_BAD_ARG;
+  const int grid = (capacity / 128 + DT_SLOTS - 1) / DT_SLOTS;
+  doc_tables_kernel<<<grid, DT_THREADS, 0, (cudaStream_t)stream>>>(cu, n_docs, fixed_len, total, capacity, start, len, row_map, slot_src,
+                                                                   slot_rows);
+  return launch_result("fl_doc_tables: kernel launch");
+}
+
+extern "C" int fl_unpack_lse(const float* lse, const int32_t* slot_src, const int32_t* slot_rows, int32_t capacity, int32_t h,
+                             int32_t seq, int32_t total, float* out, void* stream) {
+  using namespace fl;
+  if (!lse || !slot_src || !slot_rows || !out || capacity <= 0 || (capacity % 128) || h <= 0 || seq <= 0 || total % seq) return FL_ERR_BAD_ARG;
+  if (h > 65535) return FL_ERR_TOO_LARGE;
+  unpack_lse_kernel<<<dim3(capacity / 128, h), 128, 0, (cudaStream_t)stream>>>(lse, slot_src, slot_rows, capacity, h, seq, out);
+  return launch_result("fl_unpack_lse: kernel launch");
 }
 
 extern "C" int fl_pack_rows(const void* src, void* dst, const int32_t* row_map, int32_t n_dst_rows, int32_t row_bytes,

@@ -64,7 +64,7 @@ def mantissa(f):
 class _PrequantAttn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, pq, pk, pv, q8, k8, v8, qd, kd, vd, plan, seqused_k):
-        out, lse, state = _routes.forward(plan, q8, k8, v8, None, seqused_k, prequant=(qd, kd, vd))
+        out, lse, state = _routes.forward_prequant(plan, q8, k8, v8, (qd, kd, vd), seqused_k)
         ctx.plan = plan
         ctx.save_for_backward(*state)
         ctx.mark_non_differentiable(lse)
@@ -72,7 +72,7 @@ class _PrequantAttn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dout, _dlse):
-        dq, dk, dv = _routes.backward(ctx.plan, list(ctx.saved_tensors), dout.contiguous(), None)
+        dq, dk, dv = _routes.backward_prequant(ctx.plan, ctx.saved_tensors, dout.contiguous())
         return dq, dk, dv, None, None, None, None, None, None, None, None
 
 

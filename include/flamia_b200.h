@@ -226,6 +226,18 @@ int fl_dq_post(const void* dq_acc, const float* post_scale, float mult, void* dq
 #define FL_STATIC_ACC_MAX_ELEMS (1 << 23)   /* 16 MiB of f16: e.g. b1 h16 s4096 d128 */
 int fl_bwd_static_acc(const fl_attn_args* args, const float* post_scale, float mult, void* dq, void* stream);
 
+/* Tables of packed documents laid out at 128-aligned starts of a buffer of `capacity` rows (capacity % 128 == 0), in one launch
+ * (the counterpart of the reference's per-call map building, flash_attn/cute/lp_docmaps.py:107): cu (n_docs + 1) int32
+ * boundaries in the packed rows, or NULL = n_docs documents of fixed_len rows; total = packed rows. Writes start / len
+ * (n_docs), row_map (capacity; packed row of each buffer row, -1 = padding) and slot_src / slot_rows (capacity / 128). */
+int fl_doc_tables(const int32_t* cu, int32_t n_docs, int32_t fixed_len, int32_t total, int32_t capacity, int32_t* start, int32_t* len,
+                  int32_t* row_map, int32_t* slot_src, int32_t* slot_rows, void* stream);
+
+/* The live rows of the aligned buffer's LSE (h, capacity) in the caller's rows: packed row g goes to out[g / seq][head][g % seq]
+ * (packed documents: seq = total, out is (h, total); batch rows run as documents: seq = s, out is (b, h, s)). */
+int fl_unpack_lse(const float* lse, const int32_t* slot_src, const int32_t* slot_rows, int32_t capacity, int32_t h, int32_t seq,
+                  int32_t total, float* out, void* stream);
+
 /* Row gather / scatter between a packed (total, h, d) tensor and its 128-aligned repacked buffer.
  * Replaces flash_attn/cute/lp_varlen.py:421 pack_rows / unpack_rows. row_map[i] = source row of padded row i or -1. */
 int fl_pack_rows(const void* src, void* dst, const int32_t* row_map, int32_t n_dst_rows, int32_t row_bytes, void* stream);
