@@ -47,6 +47,7 @@ class AttnArgs(C.Structure):
 EXPORTS = {
     "fl_abi_version": (i32, []),
     "fl_quant_blocks": (i32, [C.POINTER(QuantArgs), vp]),
+    "fl_quant_qkv": (i32, [C.POINTER(QuantArgs), C.POINTER(QuantArgs), C.POINTER(QuantArgs), vp]),
     "fl_fwd": (i32, [C.POINTER(AttnArgs), vp]),
     "fl_bwd": (i32, [C.POINTER(AttnArgs), vp]),
     "fl_dq_prescale": (i32, [vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp, vp, vp]),
@@ -56,6 +57,7 @@ EXPORTS = {
     "fl_dq_post_ex": (i32, [vp, vp, i32, vp, f32, vp, i32, i32, i32, i32, i32, i32, vp]),
     "fl_code_stats": (i32, [vp, vp, i32, i32, i32, i32, vp, vp]),
     "fl_token_aux": (i32, [vp, C.c_int64, vp, vp, vp]),
+    "fl_dq_post_cols": (i32, [vp, vp, i32, vp, f32, vp, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp]),
     "fl_dq_post_packed": (i32, [vp, vp, f32, vp, i32, i32, i32, i32, i32, vp, vp, vp]),
     "fl_dq_prescale_rows": (i32, [vp, vp, vp, i32, i32, f32, vp, vp, vp]),
     "fl_doc_tables": (i32, [vp, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp]),

@@ -35,7 +35,7 @@ def _plan_facts(plan) -> dict:
                 rowlocal=bw.ds_dq_rowlocal == "all", prescale={"row": 0, "causal_tile": 1, "causal_row": 2}[bw.dq_prescale],
                 window_left_p1=0 if win[0] is None else win[0] + 1, window_right_p1=0 if win[1] is None else win[1] + 1,
                 softcap=f.softcap, softmax_scale=plan.softmax_scale, b=sh.b, s_q=sh.s_q, s_k=sh.s_k, h=sh.h, h_kv=sh.h_kv, d=sh.d,
-                tot_q=sh.tot_q)
+                tot_q=sh.tot_q, d_call=plan.pad_from or sh.d)
 
 
 def register_plan(plan) -> int:
@@ -75,11 +75,8 @@ def _fake_fwd(q, k, v, docs, plan, docs_id):
 
 
 def _fake_bwd(dout, state, entry):
-    sh = _PLANS[L.host().entry(entry)[0]].shape
-    if sh.varlen:
-        kshape = (sh.tot_k, sh.h_kv, sh.d)
-    else:
-        kshape = (sh.b, sh.s_k, sh.h_kv, sh.d)
+    sh, d = _PLANS[L.host().entry(entry)[0]].shape, dout.shape[-1]
+    kshape = (sh.tot_k, sh.h_kv, d) if sh.varlen else (sh.b, sh.s_k, sh.h_kv, d)
     return torch.empty_like(dout), dout.new_empty(kshape), dout.new_empty(kshape)
 
 

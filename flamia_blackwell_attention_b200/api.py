@@ -33,7 +33,7 @@ class _Resolved:
     """A resolved plan as the call path uses it."""
     plan: AttnPlan
     handle: int          # of the native plan registry
-    plain: bool          # batched, native head dim, whole tiles, no seqused_k: nothing to check or to convert per call
+    plain: bool          # batched, whole tiles, no seqused_k: nothing to check or to convert per call
 
 
 # Call key -> _Resolved. A plan is a pure function of the argument values and of the tensors' metadata, which is what the key
@@ -60,7 +60,7 @@ def _resolve(entry, resolve, q, k, v, kw) -> _Resolved:
         q, k, v = _stand_in(q), _stand_in(k), _stand_in(v)
         kw = {n: _stand_in(x) for n, x in kw.items()}
     plan = resolve(q, k, v, **kw)
-    plain = not (plan.shape.varlen or plan.fwd.ragged_documents or plan.fwd.seqused_k or plan.pad_from)
+    plain = not (plan.shape.varlen or plan.fwd.ragged_documents or plan.fwd.seqused_k)
     return _Resolved(plan, _op.register_plan(plan), plain)
 
 
@@ -129,14 +129,7 @@ def _run(call, q, k, v, cu_q, cu_k, su_q, su_k, return_lse, doc_maps=None):
     else:
         docs = tuple(t for t in (cu_q, cu_k, su_q, su_k) if t is not None) if sh.varlen else \
             ((su_k.contiguous(),) if plan.fwd.seqused_k else ())
-    if plan.pad_from:
-        # head dim below the kernels' 64 / 128: zero columns on the way in (differentiable: the gradients of the pad
-        # are the first head_dim columns of dQ / dK / dV), the first head_dim columns of O on the way out
-        extra = sh.d - plan.pad_from
-        q, k, v = (torch.nn.functional.pad(t, (0, extra)) for t in (q, k, v))
     out, lse = _op.op_apply(plan.entry, call.handle, q, k, v, docs)
-    if plan.pad_from:
-        out = out[..., :plan.pad_from].contiguous()
     if return_lse:
         if lse.numel() == 0:
             _fail("B8", ValueError, "return_lse is served on the batched and the aligned varlen forms, not under "

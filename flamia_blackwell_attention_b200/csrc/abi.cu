@@ -1,5 +1,8 @@
 // Host-side helpers of the C ABI: tensor-map construction, status word, version.
 #include <cstdio>
+#include <map>
+#include <mutex>
+#include <utility>
 
 #include "flamia_internal.h"
 
@@ -29,6 +32,20 @@ int cuda_fail(int cuda_code, const char* where) {
 int launch_result(const char* where) {
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? FL_OK : cuda_fail((int)e, where);
+}
+
+int set_smem(const void* kern, int bytes, const char* where) {
+  static std::mutex lock;
+  static std::map<std::pair<const void*, int>, int> have;
+  int dev = 0;
+  if (cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return cuda_fail((int)e, where);
+  std::lock_guard<std::mutex> g(lock);
+  int& h = have[{kern, dev}];
+  if (bytes <= h) return FL_OK;
+  if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); e != cudaSuccess)
+    return cuda_fail((int)e, where);
+  h = bytes;
+  return FL_OK;
 }
 
 int sm_count() {

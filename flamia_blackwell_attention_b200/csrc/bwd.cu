@@ -67,6 +67,7 @@ struct BwdParams {
   int32_t* dq_order;     // deterministic dQ: (b, h, s_q / 128, 2) counters, zero on entry, or null
   int n_docs;
   int b, s_q, s_k, h, h_kv;
+  int d_out;             // columns of a gradient row (D, or fewer: zero-padded head dims)
   float scale_log2;
   float softmax_scale;
   float cap_a, cap_b;    // soft cap c: x = cap_a tanh(s * factor * cap_b) in log2 units, cap_a = c log2 e, cap_b = 1 / cap_a
@@ -951,8 +952,8 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
               }
             }
             if (by_rows) {
-              if (r < out_n)
-                *reinterpret_cast<uint4*>(out_base + ((size_t)(out_row + r) * p.h_kv + hkv) * D + 64 * pass + 8 * c8) =
+              if (r < out_n && 64 * pass + 8 * c8 < p.d_out)
+                *reinterpret_cast<uint4*>(out_base + ((size_t)(out_row + r) * p.h_kv + hkv) * p.d_out + 64 * pass + 8 * c8) =
                     make_uint4(w[0], w[1], w[2], w[3]);
             } else {
               sts128(srow + ((c8 ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
@@ -1026,8 +1027,11 @@ extern "C" int fl_bwd(const fl_attn_args* a, void* stream) {
   if ((rc = make_rows_map(&mk4, fp4 ? (const void*)a->k4 : (const void*)a->k_codes, a->b, a->s_k, a->h_kv, fp4 ? 64 : a->d,
                           128)))
     return rc;
-  if ((rc = make_rows_map_16(&mdk, a->dk, a->b, a->slot_src ? a->out_rows : a->s_k, a->h_kv, a->d, 128))) return rc;
-  if ((rc = make_rows_map_16(&mdv, a->dv, a->b, a->slot_src ? a->out_rows : a->s_k, a->h_kv, a->d, 128))) return rc;
+  // a box that reaches past a row's last column (zero-padded head dims) stores the columns inside only
+  const int d_out = (a->flags >> 16) > 0 ? (a->flags >> 16) : a->d;
+  if (d_out > a->d || d_out % 8) return FL_ERR_BAD_ARG;
+  if ((rc = make_rows_map_16(&mdk, a->dk, a->b, a->slot_src ? a->out_rows : a->s_k, a->h_kv, d_out, 128))) return rc;
+  if ((rc = make_rows_map_16(&mdv, a->dv, a->b, a->slot_src ? a->out_rows : a->s_k, a->h_kv, d_out, 128))) return rc;
   BwdParams p;
   p.fac_q = a->fac_q; p.fac_k = a->fac_k; p.fac_v = a->fac_v; p.fac_do = a->fac_do; p.lse_log2 = a->lse_log2;
   p.d_rows = a->d_rows; p.dq_scale = a->dq_scale; p.dq_scale_rows = a->dq_scale_rows; p.dk = a->dk; p.dv = a->dv;
@@ -1040,7 +1044,7 @@ extern "C" int fl_bwd(const fl_attn_args* a, void* stream) {
   p.doc_start = a->doc_start; p.doc_len = a->doc_len; p.n_docs = a->n_docs;
   p.seqused_k = a->seqused_k;
   p.dq_order = a->dq_order;
-  p.b = a->b; p.s_q = a->s_q; p.s_k = a->s_k; p.h = a->h; p.h_kv = a->h_kv;
+  p.b = a->b; p.s_q = a->s_q; p.s_k = a->s_k; p.h = a->h; p.h_kv = a->h_kv; p.d_out = d_out;
   p.softmax_scale = a->softmax_scale;
   p.scale_log2 = a->softmax_scale * 1.4426950408889634f;
   const bool sc = a->softcap > 0.f;
@@ -1065,8 +1069,7 @@ extern "C" int fl_bwd(const fl_attn_args* a, void* stream) {
   const int smem = 8 * 128 * a->d + 2 * 8192 + 2 * 16384 + 2048 + ((a->d == 64 || !fp4) ? 2 * 16384 : 0) + 1024 +
                    (fp4 ? 4 * 8192 + 4 * 1024 : 0);
   auto launch = [&](auto kern) -> int {
-    if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); e != cudaSuccess)
-      return cuda_fail((int)e, "fl_bwd: cudaFuncSetAttribute");
+    if (int e = set_smem(kern, smem, "fl_bwd: cudaFuncSetAttribute")) return e;
     kern<<<grid, 512, smem, (cudaStream_t)stream>>>(mq, mk, mv, mdo, macc, mq4, mk4, mdk, mdv, p);
     return FL_OK;
   };

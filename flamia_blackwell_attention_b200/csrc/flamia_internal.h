@@ -27,6 +27,14 @@ int cuda_fail(int cuda_code, const char* where);
 // the result of a kernel launch just made: FL_OK, or cuda_fail() of cudaGetLastError()
 int launch_result(const char* where);
 
+// Allows a kernel `bytes` of dynamic shared memory on the current device. The attribute is set when a launch wants more than any
+// before it and never lowered (setting it at every launch cost about a microsecond of host time each). FL_OK or cuda_fail().
+int set_smem(const void* kern, int bytes, const char* where);
+template <typename... A>
+int set_smem(void (*kern)(A...), int bytes, const char* where) {
+  return set_smem(reinterpret_cast<const void*>(kern), bytes, where);
+}
+
 // multiprocessors of the current device (cached per device): the size of a persistent grid
 int sm_count();
 

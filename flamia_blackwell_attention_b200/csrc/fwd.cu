@@ -69,6 +69,7 @@ struct FwdParams {
   void* out;                  // packed output: the (out_rows, h, d) tensor (row stores of a document's last rows)
   int n_docs;
   int b, s_q, s_k, h, h_kv;
+  int d_out;             // columns of an output row (D, or fewer: zero-padded head dims)
   float scale_log2;
   float cap_a, cap_b;    // soft cap c: x = cap_a tanh(s * factor * cap_b) in log2 units, cap_a = c log2 e, cap_b = 1 / cap_a
   int causal;
@@ -642,9 +643,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
               }
             }
             if (by_rows) {
-              if (r < out_n)
+              if (r < out_n && 64 * pass + 8 * (cc * 4 + q4) < p.d_out)
                 *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) +
-                                          ((size_t)(out_row + r) * p.h + head) * D + 64 * pass + 8 * (cc * 4 + q4)) =
+                                          ((size_t)(out_row + r) * p.h + head) * p.d_out + 64 * pass + 8 * (cc * 4 + q4)) =
                     make_uint4(w[0], w[1], w[2], w[3]);
             } else {
               fwd_sts128(srow + (((cc * 4 + q4) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
@@ -708,7 +709,10 @@ extern "C" int fl_fwd(const fl_attn_args* a, void* stream) {
   if ((rc = make_rows_map(&mq, fp4 ? a->q4 : a->q_codes, a->b, a->s_q, a->h, fp4 ? a->d / 2 : a->d, 128))) return rc;
   if ((rc = make_rows_map(&mk, fp4 ? a->k4 : a->k_codes, a->b, a->s_k, a->h_kv, fp4 ? a->d / 2 : a->d, 128))) return rc;
   if ((rc = make_rows_map(&mv, a->v_codes, a->b, a->s_k, a->h_kv, a->d, 128))) return rc;
-  if ((rc = make_rows_map_16(&mo, a->out, a->b, a->slot_src ? a->out_rows : a->s_q, a->h, a->d, 128))) return rc;
+  // a box that reaches past a row's last column (zero-padded head dims) stores the columns inside only
+  const int d_out = (a->flags >> 16) > 0 ? (a->flags >> 16) : a->d;
+  if (d_out > a->d || d_out % 8) return FL_ERR_BAD_ARG;
+  if ((rc = make_rows_map_16(&mo, a->out, a->b, a->slot_src ? a->out_rows : a->s_q, a->h, d_out, 128))) return rc;
   FwdParams p;
   p.fac_q = a->fac_q; p.fac_k = a->fac_k; p.fac_v = a->fac_v; p.lse = a->lse;
   p.sfq4 = a->sfq4; p.sfk4 = a->sfk4;
@@ -719,7 +723,7 @@ extern "C" int fl_fwd(const fl_attn_args* a, void* stream) {
   if (a->o_mult && a->doc_start) return FL_ERR_UNSUPPORTED;      // per-(batch row, head) factors: the batched form
   p.slot_src = a->slot_src; p.slot_rows = a->slot_rows; p.out = a->out;
   if (a->slot_src && (!a->doc_start || !a->slot_rows || a->out_rows <= 0)) return FL_ERR_BAD_ARG;
-  p.b = a->b; p.s_q = a->s_q; p.s_k = a->s_k; p.h = a->h; p.h_kv = a->h_kv;
+  p.b = a->b; p.s_q = a->s_q; p.s_k = a->s_k; p.h = a->h; p.h_kv = a->h_kv; p.d_out = d_out;
   p.scale_log2 = a->softmax_scale * 1.4426950408889634f;
   p.causal = (a->flags & FL_A_CAUSAL) ? 1 : 0;
   p.win_l = a->window_left_p1 - 1;
@@ -739,8 +743,7 @@ extern "C" int fl_fwd(const fl_attn_args* a, void* stream) {
   const int smem = 4 * Q_STRIDE + 2 * KV_STAGES * 128 * a->d + 1024 + (fp4 ? 4096 + KV_STAGES * 1024 : 0);
   cudaStream_t st = (cudaStream_t)stream;
   auto launch = [&](auto kern) -> int {
-    if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); e != cudaSuccess)
-      return cuda_fail((int)e, "fl_fwd: cudaFuncSetAttribute");
+    if (int e = set_smem(kern, smem, "fl_fwd: cudaFuncSetAttribute")) return e;
     kern<<<grid, 384, smem, st>>>(mq, mk, mv, mo, p);
     return FL_OK;
   };

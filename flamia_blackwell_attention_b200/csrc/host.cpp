@@ -3,7 +3,7 @@
 // forward and backward (the launch sequence of the reference's flash_attn/cute/lowprec/_routes.py, _fp8_forward_mx :709,
 // _fp8_backward_mx :911, _e4pv_forward_blk32 :308, run_documents :1388):
 //
-//   forward   3 quantiser launches (Q, K [rotated], V) + 1 forward kernel
+//   forward   1 quantiser launch (Q, K [rotated], V) + 1 forward kernel
 //   backward  1 fused prologue (dO quantiser + D + shifted LSE + zeroed accumulator) + 1 pre-scale + 1 main kernel
 //             + 1 dQ postprocess
 //
@@ -49,6 +49,7 @@ struct Plan {
   int window_left_p1, window_right_p1;
   double softcap, softmax_scale;
   int64_t b, s_q, s_k, h, h_kv, d, tot_q;
+  int64_t d_call;            // the call's own head dim: d, or less where the kernels run it with zero columns up to d
 };
 struct Entry {
   int64_t plan, capacity;    // capacity < 0: the batched form
@@ -213,6 +214,30 @@ Docs docs_of(const Plan& p, const Tensor& q, at::TensorList t, cudaStream_t st) 
 // ---------------------------------------------------------------------------------------------------- forward
 struct Quantised {
   Tensor codes, fac, token_factors, x4, sf4, tile_stats;
+  fl_quant_args args = {};
+};
+
+// Tensors of one call over one allocation: every tensor object of its own costs an allocator round trip of about half a
+// microsecond, a view made directly a fifth of that. Two passes over the same requests: sizes first, then the tensors.
+class Pool {
+ public:
+  explicit Pool(at::Device dev) : dev_(dev) {}
+  void add(at::IntArrayRef sizes, at::ScalarType dt) { size_ = round(size_ + bytes(sizes, dt)); }
+  void allocate() { buf_ = empty({(int64_t)size_}, at::kByte, dev_); size_ = 0; }
+  Tensor take(at::IntArrayRef sizes, at::ScalarType dt) {
+    Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(buf_.storage()), buf_.key_set(), c10::scalarTypeToTypeMeta(dt));
+    t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+    t.unsafeGetTensorImpl()->set_storage_offset((int64_t)(size_ / c10::elementSize(dt)));
+    size_ = round(size_ + bytes(sizes, dt));
+    return t;
+  }
+
+ private:
+  static size_t round(size_t n) { return (n + 255) & ~size_t(255); }
+  static size_t bytes(at::IntArrayRef sizes, at::ScalarType dt) { return (size_t)c10::multiply_integers(sizes) * c10::elementSize(dt); }
+  at::Device dev_;
+  size_t size_ = 0;
+  Tensor buf_;
 };
 
 struct Shapes {            // the kernels' view of the call: one batch entry of `capacity` rows under documents
@@ -222,42 +247,38 @@ Shapes shapes_of(const Plan& p, int64_t capacity) {
   return capacity >= 0 ? Shapes{1, capacity, capacity} : Shapes{p.b, p.s_q, p.s_k};
 }
 
-Quantised quantise(const Plan& p, const Tensor& x, int64_t b, int64_t s, int64_t heads, bool scores, bool tile_stats, const Docs* docs,
-                   const Tensor& row_stat, int row_stat_kind, int32_t* status, cudaStream_t st) {
-  Quantised o;
-  const auto dev = x.device();
+// The outputs of one operand's quantiser: `make` allocates (or sizes) a tensor.
+template <typename Make>
+void quantised_tensors(Quantised& o, const Plan& p, int64_t b, int64_t s, int64_t heads, bool scores, bool tile_stats, Make make) {
   const int64_t d = p.d;
-  fl_quant_args a = {};
+  o.codes = make({b, s, heads, d}, at::kFloat8_e4m3fn);
+  o.fac = make({b, heads, s / 32}, at::kFloat);
+  if (p.token_local) o.token_factors = make({b, heads, s}, at::kFloat);
+  if (scores && p.fp4) {
+    o.x4 = make({b, s, heads, d / 2}, at::kByte);
+    o.sf4 = make({b, heads, s / 128, d / 64, 32, 4, 4}, at::kByte);
+  }
+  if (tile_stats) o.tile_stats = make({b, heads, s / 128, 2}, at::kFloat);
+}
+
+void quantise_args(Quantised& o, const Plan& p, const Tensor& x, int64_t b, int64_t s, int64_t heads, bool scores, const Docs* docs,
+                   const Tensor& row_stat, int row_stat_kind, int32_t* status) {
+  fl_quant_args& a = o.args;
   a.x = ptr<void>(x);
-  a.b = (int32_t)b; a.s = (int32_t)s; a.h = (int32_t)heads; a.d = (int32_t)d;
+  a.b = (int32_t)b; a.s = (int32_t)s; a.h = (int32_t)heads; a.d = (int32_t)p.d;
   a.in_f16 = x.scalar_type() == at::kHalf;
   // rotation: the 8-bit route rotates the E4M3 codes; the mixed route rotates only the NVFP4 S operands
   if (scores && p.hadamard) a.flags |= p.fp4 ? FL_Q_HADAMARD_NVFP4_ONLY : FL_Q_HADAMARD;
   if (p.token_local) a.flags |= FL_Q_TOKEN_LOCAL;
-  o.codes = empty({b, s, heads, d}, at::kFloat8_e4m3fn, dev);
-  o.fac = empty({b, heads, s / 32}, at::kFloat, dev);
-  a.codes = ptr<uint8_t>(o.codes); a.fac = ptr<float>(o.fac);
-  if (p.token_local) {
-    o.token_factors = empty({b, heads, s}, at::kFloat, dev);
-    a.token_factors = ptr<float>(o.token_factors);
-  }
-  if (scores && p.fp4) {
-    o.x4 = empty({b, s, heads, d / 2}, at::kByte, dev);
-    o.sf4 = empty({b, heads, s / 128, d / 64, 32, 4, 4}, at::kByte, dev);
-    a.x4 = ptr<uint8_t>(o.x4); a.sf4 = ptr<uint8_t>(o.sf4);
-  }
-  if (tile_stats) {
-    o.tile_stats = empty({b, heads, s / 128, 2}, at::kFloat, dev);
-    a.tile_stats = ptr<float>(o.tile_stats);
-  }
+  if (p.d_call != p.d) a.flags |= FL_Q_COLS(p.d_call);
+  a.codes = ptr<uint8_t>(o.codes); a.fac = ptr<float>(o.fac); a.token_factors = ptr<float>(o.token_factors);
+  a.x4 = ptr<uint8_t>(o.x4); a.sf4 = ptr<uint8_t>(o.sf4); a.tile_stats = ptr<float>(o.tile_stats);
   if (docs && !docs->aligned) {
     a.slot_src = ptr<int32_t>(docs->slot_src); a.slot_rows = ptr<int32_t>(docs->slot_rows);
-    a.src_rows = (int32_t)(x.numel() / (heads * d));
+    a.src_rows = (int32_t)(x.numel() / (heads * p.d_call));
   }
   if (row_stat.defined()) { a.row_stat = ptr<float>(row_stat); a.row_stat_kind = row_stat_kind; }
   a.status = status;
-  check(fl_quant_blocks(&a, st), "fl_quant_blocks");
-  return o;
 }
 
 void attn_common(fl_attn_args& a, const Plan& p, const Shapes& sh, bool f16) {
@@ -265,7 +286,8 @@ void attn_common(fl_attn_args& a, const Plan& p, const Shapes& sh, bool f16) {
   a.h = (int32_t)p.h; a.h_kv = (int32_t)p.h_kv; a.d = (int32_t)p.d;
   a.softmax_scale = (float)p.softmax_scale;
   a.mode = p.fp4 ? FL_MODE_FP4 : FL_MODE_FP8;
-  a.flags = (p.causal ? FL_A_CAUSAL : 0) | (f16 ? FL_A_OUT_F16 : 0) | (p.token_local ? FL_A_TOKEN_LOCAL : 0);
+  a.flags = (p.causal ? FL_A_CAUSAL : 0) | (f16 ? FL_A_OUT_F16 : 0) | (p.token_local ? FL_A_TOKEN_LOCAL : 0) |
+            (p.d_call != p.d ? FL_A_COLS(p.d_call) : 0);
   a.window_left_p1 = p.window_left_p1; a.window_right_p1 = p.window_right_p1;
   a.softcap = (float)p.softcap;
 }
@@ -280,7 +302,8 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> forward(int64_t handle, const Te
   const auto dev = q_.device();
   const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
   const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
-  TORCH_CHECK(q.numel() == (p.varlen ? p.tot_q : p.b * p.s_q) * p.h * p.d && k.numel() == (p.varlen ? p.tot_q : p.b * p.s_k) * p.h_kv * p.d &&
+  TORCH_CHECK(q.numel() == (p.varlen ? p.tot_q : p.b * p.s_q) * p.h * p.d_call &&
+                  k.numel() == (p.varlen ? p.tot_q : p.b * p.s_k) * p.h_kv * p.d_call &&
                   v.numel() == k.numel() && k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(),
               "q, k, v do not have the shapes and types of their plan");
   Tensor seqused;
@@ -305,10 +328,21 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> forward(int64_t handle, const Te
     k_rows = both.select(0, 0); v_rows = both.select(0, 1);
   }
   const bool stats = p.need_bwd && !rows;
-  const Quantised qq = quantise(p, q, sh.b, sh.s_q, p.h, true, false, dp, Tensor(), 0, stp, st);
+  Quantised qq, kq, vq;
+  Pool pool(dev);
+  auto tensors = [&](auto make) {
+    quantised_tensors(qq, p, sh.b, sh.s_q, p.h, true, false, make);
+    quantised_tensors(kq, p, sh.b, sh.s_k, p.h_kv, true, stats, make);
+    quantised_tensors(vq, p, sh.b, sh.s_k, p.h_kv, false, stats, make);
+  };
+  tensors([&](std::initializer_list<int64_t> sz, at::ScalarType dt) { pool.add(sz, dt); return Tensor(); });
+  pool.allocate();
+  tensors([&](std::initializer_list<int64_t> sz, at::ScalarType dt) { return pool.take(sz, dt); });
+  quantise_args(qq, p, q, sh.b, sh.s_q, p.h, true, dp, Tensor(), 0, stp);
   // max |K_j| of the codes' values; where those are rotated, the rotation-invariant 2-norm bounds it
-  const Quantised kq = quantise(p, k, sh.b, sh.s_k, p.h_kv, true, stats, dp, k_rows, p.hadamard && !p.fp4 ? 3 : 2, stp, st);
-  const Quantised vq = quantise(p, v, sh.b, sh.s_k, p.h_kv, false, stats, dp, v_rows, 1, stp, st);
+  quantise_args(kq, p, k, sh.b, sh.s_k, p.h_kv, true, dp, k_rows, p.hadamard && !p.fp4 ? 3 : 2, stp);
+  quantise_args(vq, p, v, sh.b, sh.s_k, p.h_kv, false, dp, v_rows, 1, stp);
+  check(fl_quant_qkv(&qq.args, &kq.args, &vq.args, st), "fl_quant_qkv");
 
   // O has the caller's rows: under repacked documents the kernel writes the packed rows itself. On the aligned form the
   // kernel writes the rows of its documents only, and the padding rows read as zeros. (The LSE of repacked documents keeps
@@ -390,7 +424,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
   const Tensor dout = dout_.contiguous();
   const bool has_docs = capacity >= 0, repacked = has_docs && !aligned;
   const Shapes sh = shapes_of(p, capacity);
-  TORCH_CHECK(dout.numel() == (p.varlen ? p.tot_q : p.b * p.s_q) * p.h * p.d, "dout does not have the shape of the output");
+  TORCH_CHECK(dout.numel() == (p.varlen ? p.tot_q : p.b * p.s_q) * p.h * p.d_call, "dout does not have the shape of the output");
   size_t i = 0;
   auto next = [&]() -> const Tensor& {
     TORCH_CHECK(i < state.size(), "the saved state of the forward is incomplete");
@@ -441,6 +475,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
   g.b = (int32_t)sh.b; g.s = (int32_t)sh.s_q; g.h = (int32_t)p.h; g.d = (int32_t)p.d;
   g.in_f16 = dout.scalar_type() == at::kHalf;
   TORCH_CHECK(dout.scalar_type() == out.scalar_type(), "dout is ", dout.scalar_type(), ", the output ", out.scalar_type());
+  if (p.d_call != p.d) g.flags |= FL_Q_COLS(p.d_call);
   if (p.token_local) { g.flags |= FL_Q_TOKEN_LOCAL; g.token_factors = ptr<float>(ws.at(w_tok)); }
   g.codes = ptr<uint8_t>(ws.at(w_codes)); g.fac = ptr<float>(ws.at(w_fac));
   g.d_out = ptr<float>(ws.at(w_D)); g.lse_log2 = ptr<float>(ws.at(w_lse)); g.zero_acc = ws.at(w_acc);
@@ -470,7 +505,8 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
 
   const bool had8 = p.hadamard && !p.fp4;      // only the 8-bit route's E4M3 codes are rotated
   // the gradients in the caller's shapes: the kernels write the caller's rows (packed ones through the slot tables)
-  const std::vector<int64_t> kshape = p.varlen ? std::vector<int64_t>{p.tot_q, p.h_kv, p.d} : std::vector<int64_t>{p.b, p.s_k, p.h_kv, p.d};
+  const std::vector<int64_t> kshape = p.varlen ? std::vector<int64_t>{p.tot_q, p.h_kv, p.d_call}
+                                               : std::vector<int64_t>{p.b, p.s_k, p.h_kv, p.d_call};
   const Tensor dq = empty(dout.sizes(), out.scalar_type(), dev), dk = empty(kshape, out.scalar_type(), dev),
                dv = empty(kshape, out.scalar_type(), dev);
   a.flags |= (had8 ? FL_A_HAD_DK : 0) | (p.rowlocal ? FL_A_DQ_ROWLOCAL : 0);
@@ -481,14 +517,9 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
   if (p.deterministic) a.dq_order = ptr<int32_t>(ws.at(w_order));
   a.status = stp;
   check(fl_bwd(&a, st), "fl_bwd");
-  if (repacked)
-    check(fl_dq_post_packed(g.zero_acc, ps, a.softmax_scale, ptr<void>(dq), (int32_t)sh.s_q, (int32_t)p.h, (int32_t)p.d, had8, f16,
-                            slot_src, slot_rows, st),
-          "fl_dq_post_packed");
-  else
-    check(fl_dq_post_ex(g.zero_acc, ps, rows, ptr<float>(dq_mult), a.softmax_scale, ptr<void>(dq), (int32_t)sh.b, (int32_t)sh.s_q,
-                        (int32_t)p.h, (int32_t)p.d, had8, f16, st),
-          "fl_dq_post_ex");
+  check(fl_dq_post_cols(g.zero_acc, ps, rows, ptr<float>(dq_mult), a.softmax_scale, ptr<void>(dq), (int32_t)sh.b, (int32_t)sh.s_q,
+                        (int32_t)p.h, (int32_t)p.d, (int32_t)p.d_call, had8, f16, slot_src, slot_rows, st),
+        "fl_dq_post_cols");
   check_status_if_asked(dev);
   return {dq, dk, dv};
 }
@@ -617,7 +648,7 @@ int64_t register_plan(const pybind11::dict& d) {
   p.return_lse = b("return_lse"); p.deterministic = b("deterministic"); p.rowlocal = b("rowlocal");
   p.prescale = (int)i("prescale"); p.window_left_p1 = (int)i("window_left_p1"); p.window_right_p1 = (int)i("window_right_p1");
   p.softcap = d["softcap"].cast<double>(); p.softmax_scale = d["softmax_scale"].cast<double>();
-  p.b = i("b"); p.s_q = i("s_q"); p.s_k = i("s_k"); p.h = i("h"); p.h_kv = i("h_kv"); p.d = i("d"); p.tot_q = i("tot_q");
+  p.b = i("b"); p.s_q = i("s_q"); p.s_k = i("s_k"); p.h = i("h"); p.h_kv = i("h_kv"); p.d = i("d"); p.tot_q = i("tot_q"); p.d_call = i("d_call");
   std::lock_guard<std::mutex> g(g_lock);
   g_plans.push_back(p);
   return (int64_t)g_plans.size() - 1;

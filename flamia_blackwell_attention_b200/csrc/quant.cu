@@ -490,19 +490,45 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
 }
 
 // ------------------------------------------------------------------------------------------------ one thread per row
-// The plain launches at head_dim 128 (and, unrotated, 64) (codes, exponent / factor tables, statistics; no
-// prologue, no token-local exponents, no packed source) run with ONE THREAD PER TOKEN ROW: CTA = 128 threads = one
-// 128-token tile, warp = one 32-token block, so the block maximum is a warp reduction, the Hadamard butterflies need no
-// shuffles, and one barrier per tile remains (it hands the input stage back to the loader and the codes to a TMA store).
-// Every floating-point operation is the one the four-lanes-per-row kernel above performs on the same operands in the same
-// order, so the two kernels' outputs are bit-identical (tests/test_gpu_quant.py compares them).
+// The launches of the forward (codes, exponent / factor tables, NVFP4 copy, statistics; no prologue, no token-local exponents)
+// run with ONE THREAD PER TOKEN ROW: CTA = 128 threads = one 128-token tile, warp = one 32-token block, so the block maximum
+// is a warp reduction, the Hadamard butterflies need no shuffles, and one barrier per tile remains (it hands the input stage
+// back to the loader and the codes to a TMA store). Every floating-point operation is the one the four-lanes-per-row kernel
+// above performs on the same operands in the same order, so the two kernels' outputs are bit-identical
+// (tests/test_gpu_quant.py compares them).
+// One launch takes up to three operands (Q, K and V of a call): their tiles form one list, so that a short call pays one
+// launch instead of three and a long one has one tail instead of three.
 static constexpr int QR_STAGES = 2;
 
+struct QuantOperand {
+  uint8_t* e_tab;         // outputs as in QuantParams; the codes leave through the operand's tensor map
+  float* fac;
+  uint8_t* x4;
+  uint8_t* sf4;
+  float* tile_stats;
+  uint32_t* row_stat;
+  int row_stat_kind;
+  int s, h;
+  int first;              // first tile of the operand in the launch's list
+  int plain;              // no rotation and no NVFP4 copy for this operand (V), whatever the kernel's MODE
+};
+struct QuantRowsParams {
+  QuantOperand op[3];
+  int n_ops, n_tiles;
+  const int32_t* slot_src;   // packed source, see QuantParams
+  const int32_t* slot_rows;
+  int in_f16;
+  DevCtl ctl;
+};
+struct QuantRowsMaps {
+  CUtensorMap x[3], c[3];
+};
+
 // MODE as in the four-lane kernel: bit 0 = the E4M3 codes are of the rotated row, bit 1 = also the NVFP4 copy, bit 2 =
-// rotate only the NVFP4 copy.
-template <int MODE, int D = 128>
+// rotate only the NVFP4 copy. PK: packed source.
+template <int MODE, int D, bool PK>
 __global__ void __launch_bounds__(128, 2)
-quant_rows_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_c, const QuantParams p) {
+quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_constant__ QuantRowsParams p) {
   static_assert(D == 128 || (D == 64 && MODE == 0), "head_dim 64 has no rotation and no NVFP4 copy");
   constexpr int QR_TILE_B = QT * D * 2;            // one 16-bit input tile (boxes of 64 columns: 128-byte rows)
   constexpr int QR_CODE_B = QT * D;                // its codes (rows of D bytes, the swizzle of that width)
@@ -516,22 +542,27 @@ quant_rows_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r = tid;                               // token row of the tile
   const int G = gridDim.x;
-  const int ntile = p.s / QT;
   volatile int* abortp = &abort_s;
 
+  auto operand_of = [&](int L) { return (p.n_ops > 1 && L >= p.op[1].first) ? ((p.n_ops > 2 && L >= p.op[2].first) ? 2 : 1) : 0; };
   auto issue = [&](int L, int st) {
-    const int head = L % p.h, tile = (L / p.h) % ntile, bat = L / (p.h * ntile);
+    const int o = operand_of(L);
+    const int l = L - p.op[o].first, h = p.op[o].h, ntile = p.op[o].s / QT;
+    const int head = l % h, tile = (l / h) % ntile, bat = l / (h * ntile);
     uint8_t* dst = smem + st * QR_TILE_B;
-    mbar_arrive_expect_tx(&full[st], QR_TILE_B);
-    tma_load_4d(dst, &tm_x, &full[st], 0, head, tile * QT, bat);
-    if (D == 128) tma_load_4d(dst + QR_TILE_B / 2, &tm_x, &full[st], 64, head, tile * QT, bat);
+    // packed source (documents stored back to back): the slot's rows start at an arbitrary row of the (1, total, h, d)
+    // tensor; only the innermost TMA coordinate has an alignment rule. An empty slot loads nothing.
+    const int xrow = PK ? p.slot_src[tile] : tile * QT;
+    mbar_arrive_expect_tx(&full[st], xrow >= 0 ? QR_TILE_B : 0);
+    if (xrow >= 0) {
+      tma_load_4d(dst, &maps.x[o], &full[st], 0, head, xrow, bat);
+      if (D == 128) tma_load_4d(dst + QR_TILE_B / 2, &maps.x[o], &full[st], 64, head, xrow, bat);
+    }
   };
   if (tid == 0) {
     abort_s = 0;
     for (int i = 0; i < QR_STAGES; ++i) mbar_init(&full[i], 1);
     fence_barrier_init();
-    tma_prefetch_desc(&tm_x);
-    tma_prefetch_desc(&tm_c);
     for (int i = 0; i < QR_STAGES; ++i)
       if (blockIdx.x + i * G < p.n_tiles) issue(blockIdx.x + i * G, i);
   }
@@ -540,10 +571,16 @@ quant_rows_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   int it = 0;
   for (int L = blockIdx.x; L < p.n_tiles; L += G, ++it) {
     const int st = it % QR_STAGES, par = it & 1;
-    const int head = L % p.h, tile = (L / p.h) % ntile, bat = L / (p.h * ntile);
+    const int oi = operand_of(L);
+    const QuantOperand& op = p.op[oi];
+    const int l = L - op.first, h = op.h, s = op.s, ntile = s / QT;
+    const int head = l % h, tile = (l / h) % ntile, bat = l / (h * ntile);
     const int t0 = tile * QT;
-    const size_t bh = (size_t)bat * p.h + head;
+    const size_t bh = (size_t)bat * h + head;
     const uint32_t tile_addr = smem_u32(smem + st * QR_TILE_B);
+    const bool plain = MODE == 0 || op.plain;      // (CTA-uniform)
+    const bool stats = op.tile_stats || op.row_stat;
+    const bool live = !PK || r < p.slot_rows[tile];     // packed source: rows past the slot's document read as zero
     bool ok = mbar_wait(&full[st], (it / QR_STAGES) & 1, p.ctl, abortp, 51);
 
     // ---- the row: D / 8 chunks of 8 elements (element 8 g + e in chunk g), rotation signs applied to the raw bits
@@ -554,6 +591,7 @@ quant_rows_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
       for (int g = 0; g < D / 8; ++g) {
         const uint32_t box = (uint32_t)(g >> 3) * (QR_TILE_B / 2);
         uint4 v = lds_u4(tile_addr + box + r * 128 + (((g & 7) ^ (r & 7)) << 4));
+        if (PK && !live) v = make_uint4(0, 0, 0, 0);
         uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -602,8 +640,8 @@ quant_rows_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     // NVFP4 copy of x: per 16 along d: SF = E4M3_rn(amax * f32(1/6)); codes = E2M1_rn(ftz(x * m)), m = 1 / SF | +inf (SF
     // rounds to 0, amax > 0) | 0. Scale bytes: group g of the row = byte g % 4 of the row's word in atom g / 4.
     auto nvfp4_row = [&]() {
-      const size_t row_off = (((size_t)bat * p.s + t0 + r) * p.h + head) * D;
-      uint8_t* x4row = p.x4 + row_off / 2;
+      const size_t row_off = (((size_t)bat * s + t0 + r) * h + head) * D;
+      uint8_t* x4row = op.x4 + row_off / 2;
       uint32_t sfw[2] = {0u, 0u};
 #pragma unroll
       for (int g2 = 0; g2 < D / 32; ++g2) {           // two groups of 16 elements = one 16-byte store
@@ -640,26 +678,26 @@ quant_rows_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         }
         *reinterpret_cast<uint4*>(x4row + g2 * 16) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
       }
-      if (p.sf4) {
-        uint8_t* atom = p.sf4 + ((bh * ntile + tile) * (D / 64)) * 512;
+      if (op.sf4) {
+        uint8_t* atom = op.sf4 + ((bh * ntile + tile) * (D / 64)) * 512;
 #pragma unroll
         for (int a = 0; a < D / 64; ++a) *reinterpret_cast<uint32_t*>(atom + a * 512 + (r & 31) * 16 + (r >> 5) * 4) = sfw[a];
       }
     };
-    if (ROT4) {          // NVFP4 codes of the rotated row, E4M3 codes of the row as read
+    if (ROT4 && !plain) {          // NVFP4 codes of the rotated row, E4M3 codes of the row as read
       load_row(true);
       rotate_row();
       nvfp4_row();
       load_row(false);
-    } else if (ROT) {
+    } else if (ROT && !plain) {
       load_row(true);
       rotate_row();
       if (NV4) nvfp4_row();
     } else {
       load_row(false);
-      if (NV4) nvfp4_row();
+      if (NV4 && !plain) nvfp4_row();
     }
-    if (!ROT || ROT4) {  // subnormal -> zero of the same sign (rotated rows were flushed by their scaling)
+    if (!ROT || ROT4 || plain) {  // subnormal -> zero of the same sign (rotated rows were flushed by their scaling)
 #pragma unroll
       for (int i = 0; i < D; i += 2) unpack2(mul2_ftz(pack2(x[i], x[i + 1]), pack2(1.0f, 1.0f)), x[i], x[i + 1]);
     }
@@ -676,7 +714,7 @@ quant_rows_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
           for (int e = 0; e < 8; e += 2)
             aq[q] = fmax3_abs(aq[q], x[32 * j + 8 * q + e], x[32 * j + 8 * q + e + 1]);
       amax = fmaxf(fmaxf(aq[0], aq[1]), fmaxf(aq[2], aq[3]));
-      if (p.tile_stats || p.row_stat) {
+      if (stats) {
         float lq[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -690,9 +728,9 @@ quant_rows_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
         sumsq = (lq[0] + lq[1]) + (lq[2] + lq[3]);
       }
     }
-    if (p.row_stat) {
-      const float v = p.row_stat_kind == 2 ? amax : (p.row_stat_kind == 3 ? __fsqrt_rn(sumsq) : sumsq);
-      atomicMax(p.row_stat + (size_t)bat * p.s + t0 + r, __float_as_uint(v));
+    if (op.row_stat && live) {
+      const float v = op.row_stat_kind == 2 ? amax : (op.row_stat_kind == 3 ? __fsqrt_rn(sumsq) : sumsq);
+      atomicMax(op.row_stat + (size_t)bat * s + t0 + r, __float_as_uint(v));
     }
     // the 32-token block = this warp (non-negative floats order as their bit patterns)
     uint32_t bm_bits, bs_bits;
@@ -731,27 +769,27 @@ quant_rows_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     if (!ok) break;
     if (tid == 0) {
       if (L + QR_STAGES * G < p.n_tiles) issue(L + QR_STAGES * G, st);
-      tma_store_4d(&tm_c, s_out + par * QR_CODE_B, 0, head, t0, bat);
+      tma_store_4d(&maps.c[oi], s_out + par * QR_CODE_B, 0, head, t0, bat);
       tma_store_commit();
     }
     // ---- side tables
     const float* wm = s_wmax[par];
     if (lane == 0) {
       const uint32_t b0 = ue8m0_byte(wm[0]), b1 = ue8m0_byte(wm[1]), b2 = ue8m0_byte(wm[2]), b3 = ue8m0_byte(wm[3]);
-      if (p.e_tab) {
-        uint8_t* e = p.e_tab + (bh * (p.s / 32) + tile * 4 + warp) * (D / 32);
+      if (op.e_tab) {
+        uint8_t* e = op.e_tab + (bh * (s / 32) + tile * 4 + warp) * (D / 32);
 #pragma unroll
         for (int g = 0; g < D / 32; ++g) e[g] = (uint8_t)bbyte;
       }
-      if (p.fac) {
+      if (op.fac) {
         const uint32_t tm = max(max(b0, b1), max(b2, b3));
         const uint32_t e0 = bbyte ? bbyte : tm;
-        p.fac[bh * (p.s / 32) + tile * 4 + warp] = e0 ? pow2_from_field((int)e0) : 1.0f;
+        op.fac[bh * (s / 32) + tile * 4 + warp] = e0 ? pow2_from_field((int)e0) : 1.0f;
       }
     }
-    if (p.tile_stats && tid == 0) {
-      p.tile_stats[(bh * ntile + tile) * 2] = fmaxf(fmaxf(wm[0], wm[1]), fmaxf(wm[2], wm[3]));
-      p.tile_stats[(bh * ntile + tile) * 2 + 1] = fmaxf(fmaxf(s_wsq[par][0], s_wsq[par][1]), fmaxf(s_wsq[par][2], s_wsq[par][3]));
+    if (op.tile_stats && tid == 0) {
+      op.tile_stats[(bh * ntile + tile) * 2] = fmaxf(fmaxf(wm[0], wm[1]), fmaxf(wm[2], wm[3]));
+      op.tile_stats[(bh * ntile + tile) * 2 + 1] = fmaxf(fmaxf(s_wsq[par][0], s_wsq[par][1]), fmaxf(s_wsq[par][2], s_wsq[par][3]));
     }
   }
   // the staging buffers must outlive the stores that read them; a CTA that gave up must not exit while loads may still land
@@ -761,15 +799,16 @@ quant_rows_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   }
 }
 
-template <int MODE, int D = 128>
-static int launch_quant_rows(const CUtensorMap& mx, const CUtensorMap& mc, const QuantParams& p, cudaStream_t st) {
+template <int MODE, int D>
+static int launch_quant_rows(const QuantRowsMaps& maps, const QuantRowsParams& p, cudaStream_t st) {
   const int smem = QR_STAGES * QT * D * 2 + 2 * QT * D + 1024;
-  auto kern = quant_rows_kernel<MODE, D>;
-  if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); e != cudaSuccess)
-    return cuda_fail((int)e, "fl_quant_blocks: cudaFuncSetAttribute");
   const int grid = min(p.n_tiles, sm_count() * 2);
-  kern<<<grid, 128, smem, st>>>(mx, mc, p);
-  return FL_OK;
+  auto launch = [&](auto kern) -> int {
+    if (int rc = set_smem(kern, smem, "fl_quant_blocks: cudaFuncSetAttribute")) return rc;
+    kern<<<grid, 128, smem, st>>>(maps, p);
+    return FL_OK;
+  };
+  return p.slot_src ? launch(quant_rows_kernel<MODE, D, true>) : launch(quant_rows_kernel<MODE, D, false>);
 }
 
 template <int D, int MODE, bool PRO, bool PK>
@@ -777,8 +816,7 @@ static int launch_quant_pk(const CUtensorMap& mx, const CUtensorMap& mo, const Q
   constexpr int TILE_B = QT * D * 2;
   const int smem = QSTAGES * (PRO ? 2 : 1) * TILE_B + 1024 + (want_t ? QT * (D + 16) : 0);
   auto kern = quant_blocks_kernel<D, MODE, PRO, PK>;
-  if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); e != cudaSuccess)
-      return cuda_fail((int)e, "fl_quant_blocks: cudaFuncSetAttribute");
+  if (int rc = set_smem(kern, smem, "fl_quant_blocks: cudaFuncSetAttribute")) return rc;
   const int per_sm = (PRO || want_t) ? 1 : 2;
   const int grid = min(p.n_tiles, sm_count() * per_sm);
   kern<<<grid, QTHREADS, smem, st>>>(mx, mo, p);
@@ -791,19 +829,77 @@ static int launch_quant(const CUtensorMap& mx, const CUtensorMap& mo, const Quan
                     : launch_quant_pk<D, MODE, PRO, false>(mx, mo, p, want_t, st);
 }
 
-}  // namespace fl
+static int quant_cols(const fl_quant_args* a) { return (a->flags >> 16) > 0 ? (a->flags >> 16) : a->d; }
 
-extern "C" int fl_quant_blocks(const fl_quant_args* a, void* stream) {
-  using namespace fl;
+static int check_quant_args(const fl_quant_args* a) {
   if (!a || !a->x || !a->codes) return FL_ERR_BAD_ARG;
   if (a->b <= 0 || a->s <= 0 || a->h <= 0 || (a->s % 128) != 0) return FL_ERR_BAD_ARG;
   if (a->d != 64 && a->d != 128) return FL_ERR_UNSUPPORTED;
+  if (quant_cols(a) > a->d || quant_cols(a) % 8) return FL_ERR_BAD_ARG;
   if ((a->flags & (FL_Q_HADAMARD | FL_Q_HADAMARD_NVFP4_ONLY)) && a->d != 128) return FL_ERR_UNSUPPORTED;
   if ((a->flags & FL_Q_HADAMARD) && (a->flags & FL_Q_TOKEN_LOCAL)) return FL_ERR_UNSUPPORTED;
   if ((a->flags & FL_Q_HADAMARD_NVFP4_ONLY) && !a->x4) return FL_ERR_BAD_ARG;
   if (a->h > 65535 || a->b > 65535) return FL_ERR_TOO_LARGE;
+  if ((long long)a->b * (a->s / 128) * a->h > 0x7FFFFFFF) return FL_ERR_TOO_LARGE;
+  if (a->row_stat && (a->row_stat_kind < 1 || a->row_stat_kind > 3)) return FL_ERR_BAD_ARG;
+  if (a->slot_src && (!a->slot_rows || a->b != 1 || a->src_rows <= 0)) return FL_ERR_BAD_ARG;
+  return FL_OK;
+}
+
+// what the one-thread-per-row kernel serves (same bits as the other one, fewer instructions, no shuffles)
+static bool rows_kernel_serves(const fl_quant_args* a) {
+  return (a->d == 128 || !(a->flags & (FL_Q_HADAMARD | FL_Q_HADAMARD_NVFP4_ONLY) || a->x4)) && !(a->d_out && a->o) && !a->codes_t &&
+         !(a->flags & (FL_Q_TOKEN_LOCAL | FL_Q_LEGACY)) && !a->sf_tok && !a->sf_dim && !a->token_factors && !a->zero_acc && !a->lse_log2;
+}
+// MODE of an operand: bit 0 = rotate the codes, bit 1 = NVFP4 copy, bit 2 = rotate the copy only
+static int quant_mode(const fl_quant_args* a) {
+  if (a->flags & FL_Q_HADAMARD_NVFP4_ONLY) return 6;
+  return ((a->flags & FL_Q_HADAMARD) ? 1 : 0) | (a->x4 ? 2 : 0);
+}
+
+static int quant_rows(const fl_quant_args* const* args, int n, cudaStream_t st) {
+  QuantRowsMaps maps;
+  QuantRowsParams p = {};
+  int mode = 0;
+  long long tiles = 0;
+  for (int i = 0; i < n; ++i) {
+    const fl_quant_args* a = args[i];
+    const int m = quant_mode(a);
+    if (m) mode = m;
+    QuantOperand& o = p.op[i];
+    o.e_tab = a->e_tab; o.fac = a->fac; o.x4 = a->x4; o.sf4 = a->sf4; o.tile_stats = a->tile_stats;
+    o.row_stat = (uint32_t*)a->row_stat; o.row_stat_kind = a->row_stat_kind;
+    o.s = a->s; o.h = a->h; o.first = (int)tiles; o.plain = m == 0;
+    tiles += (long long)a->b * (a->s / 128) * a->h;
+    int rc;
+    if ((rc = make_rows_map_16(&maps.x[i], a->x, a->b, a->slot_src ? a->src_rows : a->s, a->h, quant_cols(a), 128))) return rc;
+    if ((rc = make_rows_map(&maps.c[i], a->codes, a->b, a->s, a->h, a->d, 128))) return rc;
+  }
+  if (tiles > 0x7FFFFFFF) return FL_ERR_TOO_LARGE;
+  const fl_quant_args* a = args[0];
+  p.n_ops = n; p.n_tiles = (int)tiles;
+  p.slot_src = a->slot_src; p.slot_rows = a->slot_rows;
+  p.in_f16 = a->in_f16;
+  p.ctl.status = a->status;
+  p.ctl.wait_cycles = a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles;
+  int rc;
+  if (a->d == 64) rc = launch_quant_rows<0, 64>(maps, p, st);
+  else if (mode == 6) rc = launch_quant_rows<6, 128>(maps, p, st);
+  else if (mode == 3) rc = launch_quant_rows<3, 128>(maps, p, st);
+  else if (mode == 2) rc = launch_quant_rows<2, 128>(maps, p, st);
+  else if (mode == 1) rc = launch_quant_rows<1, 128>(maps, p, st);
+  else rc = launch_quant_rows<0, 128>(maps, p, st);
+  return rc ? rc : launch_result("fl_quant_blocks: kernel launch");
+}
+
+}  // namespace fl
+
+extern "C" int fl_quant_blocks(const fl_quant_args* a, void* stream) {
+  using namespace fl;
+  if (int rc = check_quant_args(a)) return rc;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (rows_kernel_serves(a)) return quant_rows(&a, 1, st);
   const long long n_tiles = (long long)a->b * (a->s / 128) * a->h;
-  if (n_tiles > 0x7FFFFFFF) return FL_ERR_TOO_LARGE;
   const bool pro = a->d_out != nullptr && a->o != nullptr;
   const bool rot = (a->flags & FL_Q_HADAMARD) != 0, rot4 = (a->flags & FL_Q_HADAMARD_NVFP4_ONLY) != 0;
   const bool nv4 = a->x4 != nullptr;
@@ -813,11 +909,10 @@ extern "C" int fl_quant_blocks(const fl_quant_args* a, void* stream) {
   p.sf_dim = a->sf_dim; p.token_factors = a->token_factors; p.x4 = a->x4; p.sf4 = a->sf4; p.d_out = a->d_out;
   p.lse_log2 = a->lse_log2; p.zero_acc = (uint16_t*)a->zero_acc; p.tile_stats = a->tile_stats;
   p.row_stat = (uint32_t*)a->row_stat; p.row_stat_kind = a->row_stat_kind;
-  if (a->row_stat && (a->row_stat_kind < 1 || a->row_stat_kind > 3)) return FL_ERR_BAD_ARG;
   p.b = a->b; p.s = a->s; p.h = a->h; p.n_tiles = (int)n_tiles;
   p.slot_src = a->slot_src; p.slot_rows = a->slot_rows;
   const bool packed = a->slot_src != nullptr;
-  if (packed && (!a->slot_rows || a->b != 1 || a->src_rows <= 0)) return FL_ERR_BAD_ARG;
+  const int d_src = quant_cols(a);
   p.token_local = (a->flags & FL_Q_TOKEN_LOCAL) ? 1 : 0;
   p.in_f16 = a->in_f16;
   p.lse_shift = a->lse_shift; p.d_multiplier = a->d_multiplier;
@@ -825,23 +920,10 @@ extern "C" int fl_quant_blocks(const fl_quant_args* a, void* stream) {
   p.ctl.wait_cycles = a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles;
   CUtensorMap mx, mo;
   int rc;
-  if ((rc = make_rows_map_16(&mx, a->x, a->b, packed ? a->src_rows : a->s, a->h, a->d, 128))) return rc;
+  if ((rc = make_rows_map_16(&mx, a->x, a->b, packed ? a->src_rows : a->s, a->h, d_src, 128))) return rc;
   p.o_packed = (packed && (a->flags & FL_Q_O_PACKED)) ? 1 : 0;
-  if ((rc = make_rows_map_16(&mo, pro ? a->o : a->x, a->b, p.o_packed ? a->src_rows : a->s, a->h, a->d, 128))) return rc;
-  cudaStream_t st = (cudaStream_t)stream;
+  if ((rc = make_rows_map_16(&mo, pro ? a->o : a->x, a->b, p.o_packed ? a->src_rows : a->s, a->h, d_src, 128))) return rc;
   const bool wt = a->codes_t != nullptr;
-  // the plain launches of the 8-bit route: one thread per row (same bits, fewer instructions, no shuffles)
-  if ((a->d == 128 || (a->d == 64 && !rot && !rot4 && !nv4)) && !pro && !wt && !packed && !p.token_local && !a->sf_tok &&
-      !a->sf_dim && !a->token_factors && !a->zero_acc && !a->lse_log2 && !(a->flags & FL_Q_LEGACY)) {
-    CUtensorMap mc;
-    if ((rc = make_rows_map(&mc, a->codes, a->b, a->s, a->h, a->d, 128))) return rc;
-    if (a->d == 64) rc = launch_quant_rows<0, 64>(mx, mc, p, st);
-    else if (rot4) rc = launch_quant_rows<6>(mx, mc, p, st);
-    else if (rot) rc = nv4 ? launch_quant_rows<3>(mx, mc, p, st) : launch_quant_rows<1>(mx, mc, p, st);
-    else rc = nv4 ? launch_quant_rows<2>(mx, mc, p, st) : launch_quant_rows<0>(mx, mc, p, st);
-    if (rc) return rc;
-    return launch_result("fl_quant_blocks: kernel launch");
-  }
   if (a->d == 64) {
     if (pro) rc = launch_quant<64, 0, true>(mx, mo, p, wt, st);
     else rc = nv4 ? launch_quant<64, 2, false>(mx, mo, p, wt, st) : launch_quant<64, 0, false>(mx, mo, p, wt, st);
@@ -856,4 +938,19 @@ extern "C" int fl_quant_blocks(const fl_quant_args* a, void* stream) {
   }
   if (rc) return rc;
   return launch_result("fl_quant_blocks: kernel launch");
+}
+
+extern "C" int fl_quant_qkv(const fl_quant_args* q, const fl_quant_args* k, const fl_quant_args* v, void* stream) {
+  using namespace fl;
+  const fl_quant_args* a[3] = {q, k, v};
+  for (const fl_quant_args* x : a)
+    if (int rc = check_quant_args(x)) return rc;
+  const int mq = quant_mode(q), mk = quant_mode(k), mv = quant_mode(v);
+  const bool one = rows_kernel_serves(q) && rows_kernel_serves(k) && rows_kernel_serves(v) && mq == mk && mv == 0 && q->d == k->d &&
+                   q->d == v->d && q->in_f16 == k->in_f16 && q->in_f16 == v->in_f16 && q->slot_src == k->slot_src &&
+                   q->slot_src == v->slot_src;
+  if (one) return quant_rows(a, 3, (cudaStream_t)stream);
+  for (const fl_quant_args* x : a)
+    if (int rc = fl_quant_blocks(x, stream)) return rc;
+  return FL_OK;
 }

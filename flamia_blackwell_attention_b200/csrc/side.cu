@@ -13,6 +13,9 @@ __device__ __forceinline__ float pow2_floor_clamped(float x, int lo, int hi) {
   return __uint_as_float((uint32_t)(e + 127) << 23);
 }
 
+// Grid (query tiles, batch rows) with the causal form, where every query tile has its own bound; (1, batch rows) otherwise: one CTA
+// reduces the batch row's statistics once and writes the value of every tile (as one CTA per tile, each of them read all
+// the statistics again: 34 us at 256 tiles x 16 heads).
 __global__ void dq_prescale_kernel(const float* __restrict__ st_do, const float* __restrict__ st_v,
                                    const float* __restrict__ st_k, int h, int h_kv, int nt_q, int nt_k, int causal_local,
                                    float unit, float* kernel_scale, float* post_scale) {
@@ -21,8 +24,10 @@ __global__ void dq_prescale_kernel(const float* __restrict__ st_do, const float*
   const int k_lo = 0, k_hi = causal_local ? min(t + 1 + max(nt_k - nt_q, 0), nt_k) : nt_k;
   float dn = 0.f, vn = 0.f, km = 0.f;
   const int nq = q_hi - q_lo, nk = k_hi - k_lo;
+#pragma unroll 4
   for (int j = tid; j < h * nq; j += blockDim.x)
     dn = fmaxf(dn, st_do[(((size_t)bq * h + j / nq) * nt_q + q_lo + j % nq) * 2 + 1]);
+#pragma unroll 4
   for (int j = tid; j < h_kv * nk; j += blockDim.x) {
     const size_t o = (((size_t)bq * h_kv + j / nk) * nt_k + k_lo + j % nk) * 2;
     vn = fmaxf(vn, st_v[o + 1]);
@@ -43,8 +48,13 @@ __global__ void dq_prescale_kernel(const float* __restrict__ st_do, const float*
     }
     float bnd = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(4.0f, unit), 2.0f), __fsqrt_rn(dn)), __fsqrt_rn(vn)), km);
     float bb = pow2_floor_clamped(__fdiv_rn(65504.0f, bnd), -40, 40);
-    kernel_scale[(size_t)bq * nt_q + t] = bb;
-    post_scale[(size_t)bq * nt_q + t] = __fdiv_rn(1.0f, __fmul_rn(unit, bb));
+    red[0][0] = bb;
+    red[1][0] = __fdiv_rn(1.0f, __fmul_rn(unit, bb));
+  }
+  __syncthreads();
+  for (int i = causal_local ? t + tid : tid; i < (causal_local ? t + 1 : nt_q); i += blockDim.x) {
+    kernel_scale[(size_t)bq * nt_q + i] = red[0][0];
+    post_scale[(size_t)bq * nt_q + i] = red[1][0];
   }
 }
 
@@ -96,7 +106,7 @@ __device__ __forceinline__ uint32_t cvt_out2(float a, float b, int out_f16) {
 
 // head dim 64: the accumulator is (b, h, s, 64); a straight scaled copy into the (b, s, h, 64) gradient
 __global__ void __launch_bounds__(128) dq_post_rows64_kernel(const __half* __restrict__ acc, const float* __restrict__ post,
-                                                             uint16_t* __restrict__ dq, int s, int h, float mult,
+                                                             uint16_t* __restrict__ dq, int s, int h, int d_out, float mult,
                                                              int out_f16, int per_row, const float* __restrict__ head_mult,
                                                              const int32_t* __restrict__ slot_src,
                                                              const int32_t* __restrict__ slot_rows) {
@@ -108,11 +118,11 @@ __global__ void __launch_bounds__(128) dq_post_rows64_kernel(const __half* __res
   const float sc_tile = per_row ? 0.f : post[(size_t)bat * (s / 128) + tile] * mult;
   // packed output: the tile's rows go to the packed rows slot_src[tile] .. + slot_rows[tile] of dq
   const int n_rows = slot_src ? (slot_src[tile] >= 0 ? min(slot_rows[tile], 128) : 0) : 128;
-  uint16_t* dst = dq + (((size_t)bat * s + (slot_src ? (n_rows ? slot_src[tile] : 0) : t0)) * h + head) * D;
-  const size_t row_stride = (size_t)h * D;
+  uint16_t* dst = dq + (((size_t)bat * s + (slot_src ? (n_rows ? slot_src[tile] : 0) : t0)) * h + head) * d_out;
+  const size_t row_stride = (size_t)h * d_out;
   for (int i = tid; i < 128 * CPR; i += 128) {
     const int r = i / CPR, c = i % CPR;
-    if (r >= n_rows) continue;
+    if (r >= n_rows || c * 8 >= d_out) continue;
     const float sc = per_row ? post[(size_t)bat * s + t0 + r] * mult : sc_tile;
     uint4 v = *reinterpret_cast<const uint4*>(src + (size_t)r * D + c * 8);
     const __half2* hv = reinterpret_cast<const __half2*>(&v);
@@ -132,7 +142,7 @@ __global__ void __launch_bounds__(128) dq_post_rows64_kernel(const __half* __res
 // as coalesced 16-byte stores.
 __global__ void __launch_bounds__(128) dq_post_t128_kernel(const __grid_constant__ CUtensorMap tm_acc,
                                                            const float* __restrict__ post, uint16_t* __restrict__ dq,
-                                                           int s, int h, float mult, int unrotate, int out_f16,
+                                                           int s, int h, int d_out, float mult, int unrotate, int out_f16,
                                                            int per_row, const float* __restrict__ head_mult,
                                                            const int32_t* __restrict__ slot_src,
                                                            const int32_t* __restrict__ slot_rows) {
@@ -213,11 +223,11 @@ __global__ void __launch_bounds__(128) dq_post_t128_kernel(const __grid_constant
     __syncthreads();
     // packed output: the tile's rows go to the packed rows slot_src[tile] .. + slot_rows[tile] of dq
     const int n_rows = slot_src ? (slot_src[tile] >= 0 ? min(slot_rows[tile], 128) : 0) : 128;
-    uint16_t* dst = dq + (((size_t)bat * s + (slot_src ? (n_rows ? slot_src[tile] : 0) : t0)) * h + head) * D;
-    const size_t row_stride = (size_t)h * D;
+    uint16_t* dst = dq + (((size_t)bat * s + (slot_src ? (n_rows ? slot_src[tile] : 0) : t0)) * h + head) * d_out;
+    const size_t row_stride = (size_t)h * d_out;
     for (int i = tid; i < 128 * CPR; i += 128) {
       const int r = i / CPR, c = i % CPR;
-      if (r < n_rows)
+      if (r < n_rows && c * 8 < d_out)
         *reinterpret_cast<uint4*>(dst + (size_t)r * row_stride + c * 8) = *reinterpret_cast<const uint4*>(s_out + r * ROWB + c * 16);
     }
   } else {
@@ -351,7 +361,8 @@ extern "C" int fl_dq_prescale(const float* stats_do, const float* stats_v, const
   using namespace fl;
   if (!stats_do || !stats_v || !stats_k || !kernel_scale || !post_scale || b <= 0 || nt_q <= 0 || nt_k <= 0)
     return FL_ERR_BAD_ARG;
-  dq_prescale_kernel<<<dim3(nt_q, b), 128, 0, (cudaStream_t)stream>>>(stats_do, stats_v, stats_k, h, h_kv, nt_q, nt_k,
+  const int threads = causal_local ? 128 : 1024;
+  dq_prescale_kernel<<<dim3(causal_local ? nt_q : 1, b), threads, 0, (cudaStream_t)stream>>>(stats_do, stats_v, stats_k, h, h_kv, nt_q, nt_k,
                                                                       causal_local, unit, kernel_scale, post_scale);
   return launch_result("fl_dq_prescale: kernel launch");
 }
@@ -360,11 +371,13 @@ extern "C" int fl_dq_prescale(const float* stats_do, const float* stats_v, const
 // transposed dQ tiles), (b, h, s, d) for head_dim 64.
 static int dq_post_launch(const void* dq_acc, const float* post_scale, float mult, void* dq, int32_t b, int32_t s,
                           int32_t h, int32_t d, int32_t unrotate, int32_t out_f16, int per_row, const float* head_mult,
-                          void* stream, const int32_t* slot_src = nullptr, const int32_t* slot_rows = nullptr) {
+                          void* stream, const int32_t* slot_src = nullptr, const int32_t* slot_rows = nullptr, int d_out = 0) {
   using namespace fl;
   if (!dq_acc || !post_scale || !dq || b <= 0 || s <= 0 || (s % 128) || h <= 0) return FL_ERR_BAD_ARG;
   if ((d != 64 && d != 128) || (unrotate && d != 128)) return FL_ERR_UNSUPPORTED;
   if (h > 65535 || b > 65535) return FL_ERR_TOO_LARGE;
+  if (d_out == 0) d_out = d;
+  if (d_out < 0 || d_out > d || d_out % 8) return FL_ERR_BAD_ARG;
   dim3 grid(s / 128, h, b);
   cudaStream_t st = (cudaStream_t)stream;
   if (d == 128) {
@@ -372,12 +385,11 @@ static int dq_post_launch(const void* dq_acc, const float* post_scale, float mul
     int rc = make_acc_t_map_16(&macc, dq_acc, b, h, d, s);
     if (rc) return rc;
     const int sm = 32768 + 128 * 272 + 1024;
-    if (cudaError_t e = cudaFuncSetAttribute(dq_post_t128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm); e != cudaSuccess)
-      return cuda_fail((int)e, "fl_dq_post: cudaFuncSetAttribute");
-    dq_post_t128_kernel<<<grid, 128, sm, st>>>(macc, post_scale, (uint16_t*)dq, s, h, mult, unrotate, out_f16, per_row,
+    if (int e = set_smem(dq_post_t128_kernel, sm, "fl_dq_post: cudaFuncSetAttribute")) return e;
+    dq_post_t128_kernel<<<grid, 128, sm, st>>>(macc, post_scale, (uint16_t*)dq, s, h, d_out, mult, unrotate, out_f16, per_row,
                                                head_mult, slot_src, slot_rows);
   } else {
-    dq_post_rows64_kernel<<<grid, 128, 0, st>>>((const __half*)dq_acc, post_scale, (uint16_t*)dq, s, h, mult, out_f16,
+    dq_post_rows64_kernel<<<grid, 128, 0, st>>>((const __half*)dq_acc, post_scale, (uint16_t*)dq, s, h, d_out, mult, out_f16,
                                                 per_row, head_mult, slot_src, slot_rows);
   }
   return launch_result("fl_dq_post: kernel launch");
@@ -404,6 +416,14 @@ extern "C" int fl_dq_post_packed(const void* dq_acc, const float* post_scale, fl
                                  const int32_t* slot_rows, void* stream) {
   if (!slot_src || !slot_rows) return fl::FL_ERR_BAD_ARG;
   return dq_post_launch(dq_acc, post_scale, mult, dq, 1, s, h, d, unrotate, out_f16, 0, nullptr, stream, slot_src, slot_rows);
+}
+
+extern "C" int fl_dq_post_cols(const void* dq_acc, const float* post_scale, int32_t per_row, const float* head_mult, float mult, void* dq,
+                               int32_t b, int32_t s, int32_t h, int32_t d, int32_t d_out, int32_t unrotate, int32_t out_f16,
+                               const int32_t* slot_src, const int32_t* slot_rows, void* stream) {
+  if (slot_src && (!slot_rows || b != 1 || per_row || head_mult)) return fl::FL_ERR_BAD_ARG;
+  return dq_post_launch(dq_acc, post_scale, mult, dq, b, s, h, d, unrotate, out_f16, per_row ? 1 : 0, head_mult, stream, slot_src,
+                        slot_rows, d_out);
 }
 
 extern "C" int fl_dq_prescale_rows(const float* row_do, float* row_v, float* row_k, int32_t b, int32_t s, float unit,

@@ -27,6 +27,10 @@ extern "C" {
 #define FL_Q_O_PACKED 8            /* packed source with the prologue: o has x's packed rows (else the outputs' rows) */
 #define FL_Q_LEGACY 16             /* keep the four-lanes-per-row kernel where the one-thread-per-row kernel would serve
                                       (the two are bit-identical; for tests that compare them) */
+/* Columns of a row of x and o when they are fewer than d (a multiple of 8; bits 16.. of the flags): the missing columns read
+ * as zeros, so a head dim between the kernels' own needs no padded copy (the reference's quantisers stage the zeros
+ * themselves too, flash_attn/cute/lowprec/plan.py:1529-1541). */
+#define FL_Q_COLS(n) ((int32_t)(n) << 16)
 
 /* Fused block-scaled quantiser + backward prologue.
  * Replaces flash_attn/cute/quant/fp8.py:2512 quantize_fp8_blocks (kernel :1639), the fused NVFP4 S-operand copy
@@ -74,6 +78,11 @@ typedef struct fl_quant_args {
 
 int fl_quant_blocks(const fl_quant_args* args, void* stream);
 
+/* The Q, K and V launches of one forward call in one: the same outputs, bit for bit, as three fl_quant_blocks calls. One kernel
+ * launch where the three are plain (no prologue, token-local exponents, atoms or transposed copies), share d, dtype and slot
+ * tables, and Q and K ask for the same rotation and copy, V for neither; three launches otherwise. */
+int fl_quant_qkv(const fl_quant_args* q, const fl_quant_args* k, const fl_quant_args* v, void* stream);
+
 /* fl_attn_args.mode */
 #define FL_MODE_FP8 0   /* S = E4M3 x E4M3 with the token-block factors folded into the softmax */
 #define FL_MODE_FP4 1   /* S = NVFP4 x NVFP4 block-scaled (kind::mxf4nvf4, scale_vec::4X) */
@@ -84,6 +93,7 @@ int fl_quant_blocks(const fl_quant_args* args, void* stream);
 #define FL_A_DQ_ROWLOCAL 8   /* backward: the dQ side of dS-hat gets one exponent per query row of each 32-key block */
 #define FL_A_HAD_DQ 16       /* backward: dQ accumulator holds rotated rows (post kernel rotates back) */
 #define FL_A_HAD_DK 32       /* backward: rotate dK back in the epilogue */
+#define FL_A_COLS(n) ((int32_t)(n) << 16) /* columns of a row of out / dk / dv when they are fewer than d (see FL_Q_COLS) */
 #define FL_A_P_GROUP 64      /* forward: group-frame P-hat (one UE8M0 exponent per query row and 32 keys) instead of the row frame */
 
 /* One attention problem. Operands are the quantiser's outputs; q / k / v / dO codes are (b, s, heads, d) E4M3. */
@@ -198,6 +208,10 @@ int fl_dq_post_ex(const void* dq_acc, const float* post_scale, int32_t per_row, 
  * tensor: rows of slot i go to slot_src[i] .. + slot_rows[i] (see fl_attn_args.slot_src). */
 int fl_dq_post_packed(const void* dq_acc, const float* post_scale, float mult, void* dq, int32_t s, int32_t h, int32_t d,
                       int32_t unrotate, int32_t out_f16, const int32_t* slot_src, const int32_t* slot_rows, void* stream);
+/* fl_dq_post_cols: both, and dq rows of d_out <= d columns (a multiple of 8, see FL_Q_COLS). slot_src / slot_rows NULL = batched. */
+int fl_dq_post_cols(const void* dq_acc, const float* post_scale, int32_t per_row, const float* head_mult, float mult, void* dq,
+                    int32_t b, int32_t s, int32_t h, int32_t d, int32_t d_out, int32_t unrotate, int32_t out_f16,
+                    const int32_t* slot_src, const int32_t* slot_rows, void* stream);
 /* Tile statistics of E4M3 codes times a factor per (batch row, head): tile_stats (b, h, s/128, 2) = the largest
  * magnitude and the largest row sum of squares of codes * descale[b, h] per 128-row tile, the figures the quantiser
  * writes for operands it quantises itself (the reference sizes the f16 dQ pre-scale of pre-quantised inputs from one

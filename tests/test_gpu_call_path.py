@@ -1,0 +1,80 @@
+"""GPU: the launches of a whole call against the single-operand kernels: the one-launch Q / K / V quantiser (batched, packed rows,
+head dims read with zero columns), the document tables and the LSE's way back, bit for bit."""
+import pytest
+import torch
+
+from inputs import attention_inputs
+
+pytestmark = pytest.mark.gpu
+
+LENS = [300, 1, 128, 77, 515, 127, 129]
+
+
+def _state(entry, q, k, v, docs, **kw):
+    """(out, lse, state) of the registered op under the plan of these arguments, with gradients in the plan."""
+    import flamia_blackwell_attention_b200 as F
+    from flamia_blackwell_attention_b200 import _op
+    q, k, v = (t.clone().requires_grad_(True) for t in (q, k, v))
+    plan = (F.resolve_fp8 if entry == "fp8" else F.resolve_fp4)(q, k, v, causal=True, **kw)
+    pid = _op.register_plan(plan)
+    return getattr(torch.ops.lowbit_attn, entry)(q.detach(), k.detach(), v.detach(), docs, pid, 0)
+
+
+@pytest.mark.parametrize("entry,d,dtype", [("fp8", 128, "bfloat16"), ("fp4", 128, "float16"), ("fp8", 64, "bfloat16"), ("fp8", 96, "float16"),
+                                           ("fp8", 80, "bfloat16"), ("fp8", 32, "bfloat16")])
+@pytest.mark.parametrize("form", ["batched", "packed"])
+def test_one_launch_quantiser_equals_single_launches(entry, d, dtype, form):
+    from flamia_blackwell_attention_b200 import kernels as K
+    h, hk, dt = 3, 1, getattr(torch, dtype)
+    dp = d if d in (64, 128) else (64 if d < 64 else 128)
+    rot = dict(apply_hadamard_rotation=d == 128, hadamard_rotation_scope="nvfp4_copy" if entry == "fp4" else "all",
+               also_make_nvfp4_copy=entry == "fp4")
+    if form == "batched":
+        q, k, v, _ = (t.to(dt).cuda() for t in attention_inputs(2, 384, h, hk, d, seed=3))
+        _, _, st = _state(entry, q, k, v, [])
+        slots, base = None, 0
+    else:
+        q, k, v, _ = (t[0].to(dt).cuda() for t in attention_inputs(1, sum(LENS), h, hk, d, seed=3))
+        cu = torch.tensor([0] + list(torch.tensor(LENS).cumsum(0)), dtype=torch.int32, device="cuda")
+        _, _, st = _state(entry, q, k, v, [cu, cu], cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=max(LENS), max_seqlen_k=max(LENS))
+        slots, base = (st[-3], st[-2], st[-4].numel()), 1
+    pad = lambda t: torch.nn.functional.pad(t, (0, dp - d))      # noqa: E731
+    want = [K.quantize_fp8_blocks(pad(t), legacy_kernel=True, packed_slots=slots, output_tile_stats=i > 0, **(rot if i < 2 else {}))
+            for i, t in enumerate((q, k, v))]
+    for i, w in enumerate(want):
+        assert torch.equal(st[base + 2 * i].view(torch.uint8), w["codes"].view(torch.uint8)), i
+        assert torch.equal(st[base + 2 * i + 1], w["fac"]), i
+    assert torch.equal(st[base + 7], want[1]["tile_stats"]) and torch.equal(st[base + 8], want[2]["tile_stats"])
+    if entry == "fp4":
+        for i in range(2):
+            assert torch.equal(st[base + 9 + 2 * i], want[i]["x4"]) and torch.equal(st[base + 10 + 2 * i], want[i]["sf4_raw"])
+
+
+@pytest.mark.parametrize("lens", [LENS, [5], [128] * 3, [1] * 700, [2049, 3]])
+def test_document_tables_in_one_launch(lens):
+    """fl_doc_tables against the host construction, and the call's LSE rows in the caller's order."""
+    from flamia_blackwell_attention_b200._routes import Docs
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32)
+    total = int(cu[-1])
+    ref = Docs(cu, cu[1:] - cu[:-1], total, False)
+    q, k, v, _ = (t[0].cuda() for t in attention_inputs(1, total, 2, 1, 64, seed=4))
+    c = cu.cuda()
+    _, lse, st = _state("fp8", q, k, v, [c, c], cu_seqlens_q=c, cu_seqlens_k=c, max_seqlen_q=max(lens), max_seqlen_k=max(lens), return_lse=True)
+    for name, t in zip(("start", "len", "row_map", "slot_src", "slot_rows"), st[-6:-1]):
+        assert torch.equal(t.cpu(), getattr(ref, name)), name
+    rows = ref.row_map.cuda().long()
+    assert torch.equal(lse[:, rows[rows >= 0]], st[0][0][:, rows >= 0])
+
+
+@pytest.mark.parametrize("b,h,hk,nt,causal", [(1, 1, 1, 1, False), (3, 5, 5, 7, False), (2, 16, 4, 40, False), (2, 3, 1, 9, True)])
+def test_dq_prescale_of_many_tiles(b, h, hk, nt, causal):
+    """The pre-scale table against the maxima taken directly (the bound's arithmetic itself is pinned elsewhere)."""
+    from flamia_blackwell_attention_b200 import kernels as K
+    g = torch.Generator().manual_seed(5)
+    do, v, k = (torch.rand(b, n, nt, 2, generator=g).cuda() * 100 for n in (h, hk, hk))
+    ks, ps = K.dq_prescale(do, v, k, causal_local=causal)
+    for t in range(nt):
+        q_sl, k_sl = (slice(t, t + 1), slice(0, t + 1)) if causal else (slice(0, nt), slice(0, nt))
+        bound = 8.0 * do[:, :, q_sl, 1].amax((1, 2)).sqrt() * v[:, :, k_sl, 1].amax((1, 2)).sqrt() * k[:, :, k_sl, 0].amax((1, 2))
+        want = torch.exp2(torch.floor(torch.log2(65504.0 / bound)))
+        assert torch.equal(ks[:, t], want) and torch.equal(ps[:, t], 1.0 / want)
