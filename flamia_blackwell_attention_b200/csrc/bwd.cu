@@ -25,16 +25,26 @@
 //   unused rows 64..127 of the result) and B = the K tile; rows = queries, accumulator layout (b, h, s, d)
 //   warps 0-3 compute half 0, warps 4-7 compute half 1 (thread = key row = TMEM lane, 64 query columns)
 //   warps 8-11 dQ reduction (thread = head-dim row)      warp 12 UMMA issuer      warp 13 TMA producer
-// TMEM: [0,64) / [64,128) S^T_x, then P-hat +0, dS-hat +16, six scale tiles +32..+56; [128,256) dV;
-//       [256,320) / [320,384) dP^T_x, then dQ^T_x; [384,512) dK.  Every wait is bounded (sm100.cuh).
+// TMEM: [0,64) / [64,128) S^T_x; [128,256) dV; [256,320) / [320,384) dP^T_x, then dQ^T_x; [384,512) dK.
+// P-hat, dS-hat and the scale tiles of a half go to the OTHER half's S^T columns (P-hat +0, dS-hat +16, scale tiles +32..+56): the
+// compute warps read all 64 scores of a row into registers at once, so their own S^T columns take the next scores while they
+// work, and a half goes from one iteration to the next without waiting for the tensor core. The regions alternate,
+//   region 0: S0(g) -> read -> P1, dS1(g - 1) -> dV dK dQ of (g - 1, 1) -> S0(g + 1) ...
+//   region 1: S1(g) -> read -> P0, dS0(g)     -> dV dK dQ of (g, 0)     -> S1(g + 1) ...
+// so the issue order is [dQ dV dK](g, 0), S1(g + 1), dP0(g + 1), [dQ dV dK](g, 1), S0(g + 2), dP1(g + 1): one wait of the issuer per
+// half and about 830 clocks of products behind it (an mbarrier wait costs the issuer 100 to 150 clocks even when the phase
+// has completed, and the tensor pipe takes about eight instructions ahead: with P-hat and dS-hat announced separately and S^T
+// issued after them the pipe drained at each of four waits per half, and the compute warps waited 1100 to 1700 of an
+// iteration's 3800 clocks for their scores). Half 0 runs ahead by up to one iteration.
+// Every wait is bounded (sm100.cuh).
 // Item epilogue: the compute warpgroups read dV (warpgroup 0) / dK (warpgroup 1) out of tensor memory, release the
 // accumulators to the next item's products, and write their rows through the finished item's K / V tile buffers (dead by
 // then) with TMA stores, 64 columns at a time; only then may the producer refill those buffers (two items ahead).
 // FL_MODE_FP4 (the mixed route): S^T_x is recomputed at the forward's precision, K4 Q4_x^T with
 // kind::mxf4nvf4.block_scale.scale_vec::4X on the NVFP4 copies; everything after P' is the E4M3 path above. The 16 scale
-// columns of that product (tcgen05.cp of the K and Q atoms) are parked in the half's own dP^T columns: they are free
-// once the previous dQ^T_x has been read out, and the dP^T_x product that overwrites them is issued right after S^T_x
-// (the tensor pipe runs in issue order). The second half's Q scales are columns 2, 3 of each atom.
+// columns of that product (tcgen05.cp of the K and Q atoms) are parked in dP^T columns whose dQ^T has been read out and whose
+// next dP^T is issued right behind the S^T (the tensor pipe runs in issue order). The second half's Q scales are columns
+// 2, 3 of each atom.
 // VAR = 1 (FL_A_DQ_ROWLOCAL, the reference's ds_dq_rowlocal="all", flash_bwd_sm100_fp4.py:3637-3642): the dQ side of
 // dS-hat gets its own codes with one exponent per (query row, 32-key block) instead of sharing the 32 x 32 block's.
 // VAR = 2 (FL_A_TOKEN_LOCAL + row-local, flash_bwd_sm100_fp4.py:152-158): every token of Q, K, V, dO carries its own
@@ -95,12 +105,12 @@ struct BTile {
   int n_m;    // number of query tiles that see it
 };
 
-// barriers; [2] = one per half, stage or buffer
-enum { BB_KV = 0, BB_KVE = 2, BB_QFULL = 4, BB_QEMPTY = 6, BB_S = 8, BB_DP = 10, BB_P = 12, BB_DS = 14, BB_EX = 16,
-       BB_DQF = 18, BB_DQE = 20, BB_EP = 22, BB_EPI = 24, BB_R1 = 26, BB_R2 = 27, BB_ACC = 28, BB_ACCFREE = 29,
-       BB_COUNT = 30 };
+// barriers; [2] = one per half, stage or buffer, [3] = one per stage of the score operand's ring
+enum { BB_KV = 0, BB_KVE = 2, BB_AFULL = 4, BB_AEMPTY = 7, BB_BFULL = 10, BB_BEMPTY = 12, BB_S = 14, BB_DP = 16, BB_GRANT = 18,
+       BB_DS = 20, BB_DQF = 22, BB_DQE = 24, BB_EPI = 26, BB_R1 = 28, BB_R2 = 29, BB_ACC = 30, BB_ACCFREE = 31, BB_SDR = 32,
+       BB_COUNT = 33 };
 // TMEM columns; the per-half regions are at + 64 * x
-enum { TC_S = 0, TO_P = 0, TO_DS = 16, TO_SFA_P = 32, TO_SFB_DO = 36, TO_SFA_DK = 40, TO_SFB_Q = 44, TO_SFA_DQ = 48,
+enum { TC_S = 0, TO_P = 0, TO_DS = 16, TO_SFA_P = 32, TO_SFB_DO = 36, TO_SFB_Q = 40, TO_SFA_DQ = 44, TO_SFA_DK = 48,
        TO_SFB_DQ = 52, TC_DV = 128, TC_DP = 256, TC_DK = 384 };
 
 // bits of the warp's largest |v| (the f32 form of the instruction is faster than masking the sign and reducing integers:
@@ -109,11 +119,6 @@ __device__ __forceinline__ uint32_t warp_max_abs_f32(float v) {
   float r;
   asm volatile("redux.sync.max.abs.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
   return __float_as_uint(r);
-}
-__device__ __forceinline__ uint32_t warp_max_u32(uint32_t v) {
-  uint32_t r;
-  asm volatile("redux.sync.max.u32 %0, %1, 0xffffffff;" : "=r"(r) : "r"(v));
-  return r;
 }
 template <int N>
 __device__ __forceinline__ void reg_alloc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -127,6 +132,8 @@ __device__ __forceinline__ float4 lds128(uint32_t addr) {
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
+__device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts8(uint32_t addr, uint32_t v) { asm volatile("st.shared.b8 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 // 448 * 2^(e - 127) >= amax for the returned UE8M0 byte (bits = the non-negative float's pattern), clamped to [1, 254]
 __device__ __forceinline__ uint32_t exp448(uint32_t bits) {
   const int e = (int)((bits + 0x00200000u) >> 23) - 8;
@@ -191,6 +198,39 @@ __device__ __forceinline__ void st_release_gpu(int32_t* ptr, int v) {
   asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(ptr), "r"(v) : "memory");
 }
 
+// Shared memory of one CTA (dynamic, from a 1024-byte boundary; the kernel has no static shared memory, so that the 8-bit route
+// at d = 128 fits the 227 KB to the byte).
+struct BwdMisc {
+  uint64_t bars[BB_COUNT];
+  uint32_t tmem_base;
+  int abort;
+  BTile tile[2];            // the items in flight (written by the producer, item k in slot k & 1)
+};
+template <int D, bool FP4>
+struct BwdSmem {
+  static constexpr int TILE = 128 * D;
+  static constexpr int A_TILE = FP4 ? 8192 : TILE;                  // the score operand: Q, or its NVFP4 copy
+  static constexpr bool EPI2 = D == 128 && !FP4;                    // a second way out for the gradient rows, see the item epilogue
+  static constexpr int K = 0;                                       // 2 buffers (items alternate)
+  static constexpr int V = K + 2 * TILE;                            // 2 buffers
+  static constexpr int DO = V + 2 * TILE;                           // 2 stages
+  static constexpr int A = DO + 2 * TILE;                           // 3 stages
+  static constexpr int Q = FP4 ? A + 3 * A_TILE : A;                // FP4: the E4M3 Q tiles (dK), 2 stages; else the A ring
+  static constexpr int DS = Q + (FP4 ? 2 : 3) * TILE;               // per half: 128 key rows x 64 query bytes, 64 B swizzle
+  static constexpr int DQ = DS + 2 * 8192;                          // per half: 128 head-dim rows x 64 queries f16, 128 B swizzle
+  static constexpr int OUT = DQ + 2 * 16384;                        // gradient rows' way out: EPI2 or d = 64, 2 x 16 KB
+  static constexpr int K4 = OUT + ((EPI2 || D == 64) ? 2 * 16384 : 0);   // FP4: NVFP4 K tiles, 2 x 8 KB
+  static constexpr int SF = K4 + (FP4 ? 2 * 8192 : 0);              // FP4: scale atoms, K 2 x 1 KB then Q 3 x 1 KB
+  static constexpr int VEC = SF + (FP4 ? 5 * 1024 : 0);             // 2 stages x {lse_log2[128], D''[128]}
+  // per half three scale atoms of 512 bytes (dK's A side, dQ's query side, P-hat's), written by the compute warps and copied by
+  // the issuer. EPI2: inside the half's own part of OUT, in use only between an item's last product and the next item's first dS.
+  static constexpr int ATOM_STRIDE = EPI2 ? 16384 : 1536;
+  static constexpr int ATOMS = EPI2 ? OUT : VEC + 2048;
+  static constexpr int MISC = EPI2 ? VEC + 2048 : ATOMS + 2 * ATOM_STRIDE;
+  static constexpr int BYTES = MISC + 1024;
+  static_assert(sizeof(BwdMisc) <= 1024 && BYTES <= 227 * 1024);
+};
+
 // FULL: the variants that also serve the rarer call forms (deterministic dQ order, per-query-row pre-scale, packed
 // outputs, the dK mantissa factor), each behind a run-time check of its pointer. A template flag, so that the kernels
 // of the plain calls carry none of that code: the loop is sensitive to every register and instruction added to it.
@@ -201,68 +241,60 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                      const __grid_constant__ CUtensorMap tm_acc, const __grid_constant__ CUtensorMap tm_q4,
                      const __grid_constant__ CUtensorMap tm_k4, const __grid_constant__ CUtensorMap tm_dk,
                      const __grid_constant__ CUtensorMap tm_dv, const BwdParams p) {
+  using SM = BwdSmem<D, FP4>;
   constexpr int TILE_BYTES = 128 * D;
   constexpr uint64_t OP_SWZ = (D == 128) ? SWZ_128 : SWZ_64;     // operand tiles: rows of D bytes
   constexpr uint32_t OP_SBO = 8 * D;
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sK = smem;                                  // 2 buffers (items alternate)
-  uint8_t* sV = sK + 2 * TILE_BYTES;                   // 2 buffers
-  uint8_t* sQ = sV + 2 * TILE_BYTES;                   // 2 stages
-  uint8_t* sDO = sQ + 2 * TILE_BYTES;                  // 2 stages
-  uint8_t* sDS = sDO + 2 * TILE_BYTES;                 // per half: 128 key rows x 64 query bytes, 64 B swizzle
-  uint8_t* sDQ = sDS + 2 * 8192;                       // per half: 128 head-dim rows x 64 queries f16, 128 B swizzle
-  float* sVec = reinterpret_cast<float*>(sDQ + 2 * 16384);   // 2 stages x {lse_log2[128], D''[128]}
-  // d = 64 only: the gradient rows' way out (2 x 16 KB; at d = 128 the finished item's K / V buffers serve)
-  uint8_t* sOut64 = reinterpret_cast<uint8_t*>(sVec) + 2048;
-  // FP4 only: NVFP4 K tiles (2 x 8 KB), Q4 stages (2 x 8 KB), scale atoms K 2 x 1 KB + Q 2 x 1 KB
-  uint8_t* sK4 = sOut64 + (D == 64 ? 2 * 16384 : 0);
-  uint8_t* sQ4 = sK4 + 2 * 8192;
-  uint8_t* sSF = sQ4 + 2 * 8192;
-  // d = 128, 8-bit route: a second way out for the gradient rows (2 x 16 KB), see the item epilogue
-  constexpr bool EPI2 = (D == 128) && !FP4;
-  uint8_t* sOut2 = sOut64;
-  __shared__ __align__(8) uint64_t bars[BB_COUNT];
-  __shared__ uint32_t tmem_base_s;
-  __shared__ int abort_s;
-  __shared__ BTile tile_s[2];                          // the items in flight (written by the producer, item k in slot k & 1)
-  __shared__ uint32_t sE[2][4];                        // [half][key block] = exponent bytes of the half's two query blocks
-  __shared__ uint32_t sEP[2][128];                     // VAR 2: [half][key row] = P-hat exponent bytes of the two query blocks
-  __shared__ __align__(4) uint8_t sEQ[2][64][4];       // VAR >= 1: [half][query][key block] = dQ-side dS-hat exponents
+  constexpr bool EPI2 = SM::EPI2;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  BwdMisc& misc = *reinterpret_cast<BwdMisc*>(smem + SM::MISC);
+  uint64_t* const bars = misc.bars;
+  BTile* const tile_s = misc.tile;
   constexpr bool RL = VAR >= 1, TL = VAR == 2;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (smem_u32(smem) & 1023) {           // (never the case without static shared memory; the swizzles depend on it)
+    if (threadIdx.x == 0 && p.ctl.status) atomicCAS(p.ctl.status, 0, FL_DEV_WAIT_TIMEOUT | 63);
+    return;
+  }
+  // (the warp index through a shuffle: the compiler then knows that it is the same in all lanes)
+  const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
   const int G = gridDim.x, cta = blockIdx.x;
   const int grp = p.h / p.h_kv;
 
   if (tid == 13 * 32) {
-    abort_s = 0;
+    misc.abort = 0;
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars[BB_KV + i], 1); mbar_init(&bars[BB_KVE + i], 2);      // released by one thread of each compute warpgroup
-      mbar_init(&bars[BB_QFULL + i], 1); mbar_init(&bars[BB_QEMPTY + i], 1);
+      mbar_init(&bars[BB_BFULL + i], 1); mbar_init(&bars[BB_BEMPTY + i], 1);
       mbar_init(&bars[BB_S + i], 1); mbar_init(&bars[BB_DP + i], 1);
-      mbar_init(&bars[BB_P + i], 4); mbar_init(&bars[BB_DS + i], 4); mbar_init(&bars[BB_EX + i], 4);      // one arrival per warp
+      mbar_init(&bars[BB_GRANT + i], 4); mbar_init(&bars[BB_DS + i], 4);      // one arrival per warp
       mbar_init(&bars[BB_DQF + i], 1); mbar_init(&bars[BB_DQE + i], 4);
-      mbar_init(&bars[BB_EP + i], 4); mbar_init(&bars[BB_EPI + i], 4);
+      mbar_init(&bars[BB_EPI + i], 4);
     }
+    for (int i = 0; i < 3; ++i) { mbar_init(&bars[BB_AFULL + i], 1); mbar_init(&bars[BB_AEMPTY + i], 1); }
     mbar_init(&bars[BB_R1], 4);
     mbar_init(&bars[BB_R2], 4);
     mbar_init(&bars[BB_ACC], 1);
     mbar_init(&bars[BB_ACCFREE], 8);
+    mbar_init(&bars[BB_SDR], 4);
     fence_barrier_init();
     tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v); tma_prefetch_desc(&tm_do);
     tma_prefetch_desc(&tm_acc); tma_prefetch_desc(&tm_dk); tma_prefetch_desc(&tm_dv);
     if (FP4) { tma_prefetch_desc(&tm_q4); tma_prefetch_desc(&tm_k4); }
   }
   if (warp == 0) {
-    tmem_alloc(&tmem_base_s, 512);
+    tmem_alloc(&misc.tmem_base, 512);
     tmem_relinquish();
+  }
+  if (!EPI2) {      // (atom bytes that nobody writes are scale 1; with EPI2 no product looks at them)
+    for (int i = tid; i < 2 * SM::ATOM_STRIDE / 4; i += 512) reinterpret_cast<uint32_t*>(smem + SM::ATOMS)[i] = 0x7F7F7F7Fu;
+    fence_proxy_async();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base_s;
-  volatile int* abortp = &abort_s;
+  const uint32_t tmem = misc.tmem_base;
+  volatile int* abortp = &misc.abort;
   // (a status word already set by an earlier launch is not looked at: a kernel that runs after one that gave up does no harm)
 
   if (warp >= 12) reg_dealloc<80>();     // register budget per warpgroup: 176 / 176 / 80 / 80 (x 128 threads = 64 K)
@@ -283,33 +315,36 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         tile_s[kb] = t;
         if (t.nk > 0) {
           mbar_arrive_expect_tx(&bars[BB_KV + kb], 2 * TILE_BYTES + (FP4 ? 8192 + 1024 : 0));
-          tma_load_4d(sK + kb * TILE_BYTES, &tm_k, &bars[BB_KV + kb], 0, t.hkv, t.k0, t.bat);
-          tma_load_4d(sV + kb * TILE_BYTES, &tm_v, &bars[BB_KV + kb], 0, t.hkv, t.k0, t.bat);
+          tma_load_4d(smem + SM::K + kb * TILE_BYTES, &tm_k, &bars[BB_KV + kb], 0, t.hkv, t.k0, t.bat);
+          tma_load_4d(smem + SM::V + kb * TILE_BYTES, &tm_v, &bars[BB_KV + kb], 0, t.hkv, t.k0, t.bat);
           if (FP4) {
-            tma_load_4d(sK4 + kb * 8192, &tm_k4, &bars[BB_KV + kb], 0, t.hkv, t.k0, t.bat);
-            bulk_load(sSF + kb * 1024, p.sfk4 + (((size_t)t.bat * p.h_kv + t.hkv) * (p.s_k / 128) + t.k0 / 128) * 1024, 1024,
-                      &bars[BB_KV + kb]);
+            tma_load_4d(smem + SM::K4 + kb * 8192, &tm_k4, &bars[BB_KV + kb], 0, t.hkv, t.k0, t.bat);
+            bulk_load(smem + SM::SF + kb * 1024, p.sfk4 + (((size_t)t.bat * p.h_kv + t.hkv) * (p.s_k / 128) + t.k0 / 128) * 1024,
+                      1024, &bars[BB_KV + kb]);
           }
         } else {
           mbar_arrive(&bars[BB_KV + kb]);  // an empty tile slot: the phase still completes, every role moves on
         }
         const int n_it = t.n_m * grp;
+        int head = t.hkv * grp, m = t.m_lo;
         for (int it = 0; it < n_it; ++it, ++gi) {
-          const int st = gi & 1;
-          const int head = t.hkv * grp + it / t.n_m, m = t.m_lo + it % t.n_m;
-          if (gi >= 2 && !(ok = mbar_wait(&bars[BB_QEMPTY + st], ((gi >> 1) - 1) & 1, p.ctl, abortp, 10))) break;
-          mbar_arrive_expect_tx(&bars[BB_QFULL + st], 2 * TILE_BYTES + 1024 + (FP4 ? 8192 + 1024 : 0));
-          tma_load_4d(sQ + st * TILE_BYTES, &tm_q, &bars[BB_QFULL + st], 0, head, t.q0 + m * 128, t.bat);
-          if (FP4) {
-            tma_load_4d(sQ4 + st * 8192, &tm_q4, &bars[BB_QFULL + st], 0, head, t.q0 + m * 128, t.bat);
-            bulk_load(sSF + 2048 + st * 1024,
-                      p.sfq4 + (((size_t)t.bat * p.h + head) * (p.s_q / 128) + (t.q0 + m * 128) / 128) * 1024, 1024,
-                      &bars[BB_QFULL + st]);
-          }
-          tma_load_4d(sDO + st * TILE_BYTES, &tm_do, &bars[BB_QFULL + st], 0, head, t.q0 + m * 128, t.bat);
-          const size_t ro = ((size_t)t.bat * p.h + head) * p.s_q + t.q0 + m * 128;
-          bulk_load(sVec + st * 256, p.lse_log2 + ro, 512, &bars[BB_QFULL + st]);
-          bulk_load(sVec + st * 256 + 128, p.d_rows + ro, 512, &bars[BB_QFULL + st]);
+          // ring A: the scores' query operand, one tile further ahead than ring B (dO, the row vectors, FP4: the E4M3 Q)
+          const int sa = gi % 3, ra = gi / 3, sb = gi & 1, rb = gi >> 1;
+          const int qrow = t.q0 + m * 128;
+          const size_t ro = ((size_t)t.bat * p.h + head) * p.s_q + qrow;
+          if (gi >= 3 && !(ok = mbar_wait(&bars[BB_AEMPTY + sa], (ra - 1) & 1, p.ctl, abortp, 10))) break;
+          mbar_arrive_expect_tx(&bars[BB_AFULL + sa], SM::A_TILE + (FP4 ? 1024 : 0));
+          tma_load_4d(smem + SM::A + sa * SM::A_TILE, FP4 ? &tm_q4 : &tm_q, &bars[BB_AFULL + sa], 0, head, qrow, t.bat);
+          if (FP4)
+            bulk_load(smem + SM::SF + 2048 + sa * 1024, p.sfq4 + (((size_t)t.bat * p.h + head) * (p.s_q / 128) + qrow / 128) * 1024,
+                      1024, &bars[BB_AFULL + sa]);
+          if (gi >= 2 && !(ok = mbar_wait(&bars[BB_BEMPTY + sb], (rb - 1) & 1, p.ctl, abortp, 10))) break;
+          mbar_arrive_expect_tx(&bars[BB_BFULL + sb], TILE_BYTES + 1024 + (FP4 ? TILE_BYTES : 0));
+          if (FP4) tma_load_4d(smem + SM::Q + sb * TILE_BYTES, &tm_q, &bars[BB_BFULL + sb], 0, head, qrow, t.bat);
+          tma_load_4d(smem + SM::DO + sb * TILE_BYTES, &tm_do, &bars[BB_BFULL + sb], 0, head, qrow, t.bat);
+          bulk_load(smem + SM::VEC + sb * 1024, p.lse_log2 + ro, 512, &bars[BB_BFULL + sb]);
+          bulk_load(smem + SM::VEC + sb * 1024 + 512, p.d_rows + ro, 512, &bars[BB_BFULL + sb]);
+          if (++m == t.m_lo + t.n_m) { m = t.m_lo; ++head; }
         }
       }
     }
@@ -319,14 +354,13 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     // lane issues. Descriptors are built once; the loops only add byte offsets.
     constexpr uint32_t ID_N64 = idesc_f8(128, 64, 0, 0);
     const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
-    const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), q_addr = smem_u32(sQ), do_addr = smem_u32(sDO),
-                   ds_addr = smem_u32(sDS);
-    const uint64_t dQ0 = smem_desc(q_addr, 16, OP_SBO, OP_SWZ), dDO0 = smem_desc(do_addr, 16, OP_SBO, OP_SWZ),
-                   dDS_A = smem_desc(ds_addr, 8192, 512, SWZ_64),   // d = 64: dS-hat as A, next M block 8 KB further
-                   dDS0 = smem_desc(ds_addr, 16, 512, SWZ_64);
-    const uint32_t k4_addr = smem_u32(sK4);
-    const uint64_t dQ40 = smem_desc(smem_u32(sQ4), 16, 512, SWZ_64), dSF0 = smem_desc(smem_u32(sSF), 0, 128, SWZ_NONE);
-    int gi = 0;
+    const uint32_t base = smem_u32(smem);
+    const uint64_t dA0 = FP4 ? smem_desc(base + SM::A, 16, 512, SWZ_64) : smem_desc(base + SM::A, 16, OP_SBO, OP_SWZ),
+                   dQ0 = smem_desc(base + SM::Q, 16, OP_SBO, OP_SWZ), dDO0 = smem_desc(base + SM::DO, 16, OP_SBO, OP_SWZ),
+                   dDS_A = smem_desc(base + SM::DS, 8192, 512, SWZ_64),   // d = 64: dS-hat as A, next M block 8 KB further
+                   dDS0 = smem_desc(base + SM::DS, 16, 512, SWZ_64),
+                   dSF0 = smem_desc(base + SM::SF, 0, 128, SWZ_NONE), dAT0 = smem_desc(base + SM::ATOMS, 0, 128, SWZ_NONE);
+    int gi = 0, sdr = 0;                   // iterations so far; uses of BB_SDR so far
     bool ok = true;
     for (int k = 0; ok; ++k) {
       const int L = bwd_item(k, G, cta, p.zigzag);
@@ -334,96 +368,121 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[BB_KV + kb], (k >> 1) & 1, p.ctl, abortp, 20))) break;
       const int n_it = tile_s[kb].n_m * grp;
-      const int n_steps = 2 * n_it;
-      const uint64_t dK_k = smem_desc(k_addr + kb * TILE_BYTES, 16, OP_SBO, OP_SWZ),
-                     dV_k = smem_desc(v_addr + kb * TILE_BYTES, 16, OP_SBO, OP_SWZ),
-                     dK4 = smem_desc(k4_addr + kb * 8192, 16, 512, SWZ_64);
-      for (int t = 0; ok && t <= n_steps; ++t) {
-        if (t < n_steps) {
-          // ---- front end of step t: S^T_x and dP^T_x
-          const int g = gi + (t >> 1), x = t & 1, st = g & 1;
-          if (x == 0 && !(ok = mbar_wait(&bars[BB_QFULL + st], (g >> 1) & 1, p.ctl, abortp, 21))) break;
-          tc_fence_after();
-          const uint64_t qx = desc_adv(dQ0, st * TILE_BYTES + x * 64 * D), dox = desc_adv(dDO0, st * TILE_BYTES + x * 64 * D);
+      const uint64_t dK_k = smem_desc(base + SM::K + kb * TILE_BYTES, 16, OP_SBO, OP_SWZ),
+                     dV_k = smem_desc(base + SM::V + kb * TILE_BYTES, 16, OP_SBO, OP_SWZ),
+                     dK4 = smem_desc(base + SM::K4 + kb * 8192, 16, 512, SWZ_64);
+      // S^T_x of iteration g. FP4: the scale columns stand in `park` (free tensor memory)
+      auto issue_s = [&](int g, int x, uint32_t park) -> bool {
+        const int st = g % 3;
+        // (the second half finds the stage loaded: the first half's product of the same iteration was issued before)
+        if (x == 0 && !mbar_wait(&bars[BB_AFULL + st], (g / 3) & 1, p.ctl, abortp, 21)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+          const uint64_t ax = desc_adv(dA0, st * SM::A_TILE + x * (SM::A_TILE / 2));
           if (FP4) {
-            // the scale columns go into the half's dP^T region: its previous dQ^T must have been read out first
-            if (g > 0 && !(ok = mbar_wait(&bars[BB_DQE + x], (g - 1) & 1, p.ctl, abortp, 22))) break;
-            tc_fence_after();
-          }
-          if (elect_one()) {
-            if (FP4) {
-              const uint32_t park = tm + TC_DP + 64 * x;
-              const uint64_t q4x = desc_adv(dQ40, st * 8192 + x * 4096);
 #pragma unroll
-              for (int kk = 0; kk < 2; ++kk) {
-                tmem_cp_sf_atom(park + 4 * kk, desc_adv(dSF0, kb * 1024 + 512 * kk));
-                tmem_cp_sf_atom(park + 8 + 4 * kk, desc_adv(dSF0, 2048 + st * 1024 + 512 * kk));
-              }
-#pragma unroll
-              for (int kk = 0; kk < 2; ++kk)   // K = 64 elements = 32 bytes per instruction
-                umma_nvf4_ss(tm + TC_S + 64 * x, desc_adv(dK4, 32 * kk), desc_adv(q4x, 32 * kk),
-                             idesc_bs(128, 64, 1, 1, 0, 0, 0, 0, 0), park + 4 * kk, park + 8 + 4 * kk + 2 * x, kk > 0);
-            } else {
-#pragma unroll
-              for (int kk = 0; kk < D / 32; ++kk)
-                umma_f8_ss(tm + TC_S + 64 * x, desc_adv(dK_k, 32 * kk), desc_adv(qx, 32 * kk), ID_N64, kk > 0);
+            for (int kk = 0; kk < 2; ++kk) {
+              tmem_cp_sf_atom(park + 4 * kk, desc_adv(dSF0, kb * 1024 + 512 * kk));
+              tmem_cp_sf_atom(park + 8 + 4 * kk, desc_adv(dSF0, 2048 + st * 1024 + 512 * kk));
             }
-            tc_commit(&bars[BB_S + x]);
-          }
-          __syncwarp();
-          // the half's dP^T columns hold its previous dQ^T until the reduction warps have read it
-          if (!FP4 && g > 0 && !(ok = mbar_wait(&bars[BB_DQE + x], (g - 1) & 1, p.ctl, abortp, 22))) break;
-          tc_fence_after();
-          if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk)   // K = 64 elements = 32 bytes per instruction
+              umma_nvf4_ss(tm + TC_S + 64 * x, desc_adv(dK4, 32 * kk), desc_adv(ax, 32 * kk),
+                           idesc_bs(128, 64, 1, 1, 0, 0, 0, 0, 0), park + 4 * kk, park + 8 + 4 * kk + 2 * x, kk > 0);
+          } else {
 #pragma unroll
             for (int kk = 0; kk < D / 32; ++kk)
-              umma_f8_ss(tm + TC_DP + 64 * x, desc_adv(dV_k, 32 * kk), desc_adv(dox, 32 * kk), ID_N64, kk > 0);
-            tc_commit(&bars[BB_DP + x]);
+              umma_f8_ss(tm + TC_S + 64 * x, desc_adv(dK_k, 32 * kk), desc_adv(ax, 32 * kk), ID_N64, kk > 0);
           }
-          __syncwarp();
+          tc_commit(&bars[BB_S + x]);
         }
-        if (t >= 1) {
-          // ---- back end of step t - 1: dV, dK, dQ^T of half y
-          const int tb = t - 1, g = gi + (tb >> 1), y = tb & 1, st = g & 1;
-          const uint32_t sx = tm + TC_S + 64 * y;
-          const uint64_t qy = desc_adv(dQ0, st * TILE_BYTES + y * 64 * D), doy = desc_adv(dDO0, st * TILE_BYTES + y * 64 * D);
-          const uint32_t accum = tb > 0;
-          // the first products of an item overwrite dV / dK: the previous item's rows must have left tensor memory
-          if (tb == 0 && k > 0 && !(ok = mbar_wait(&bars[BB_ACCFREE], (k - 1) & 1, p.ctl, abortp, 25))) break;
-          if (!(ok = mbar_wait(&bars[BB_P + y], g & 1, p.ctl, abortp, 23))) break;
-          tc_fence_after();
-          if (elect_one()) {
+        __syncwarp();
+        return true;
+      };
+      // the half's dP^T columns hold its previous dQ^T until the reduction warps have read it (iteration g - 1)
+      auto dq_read = [&](int g, int x) -> bool { return g == 0 || mbar_wait(&bars[BB_DQE + x], (g - 1) & 1, p.ctl, abortp, 22); };
+      auto issue_dp = [&](int g, int x) -> bool {
+        const int st = g & 1;
+        if (x == 0 && !mbar_wait(&bars[BB_BFULL + st], (g >> 1) & 1, p.ctl, abortp, 27)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+          const uint64_t dox = desc_adv(dDO0, st * TILE_BYTES + x * 64 * D);
 #pragma unroll
-            for (int kk = 0; kk < 2; ++kk)     // K = 64 queries: two instructions of 32
-              umma_mxf8_ts(tm + TC_DV, sx + TO_P + 8 * kk, desc_adv(doy, kk * 32 * D),
-                           idesc_bs(128, D, 0, 0, 0, 1, 1, kk, kk), sx + TO_SFA_P, sx + TO_SFB_DO, accum | kk);
-          }
-          __syncwarp();
-          if (!(ok = mbar_wait(&bars[BB_DS + y], g & 1, p.ctl, abortp, 24))) break;
-          tc_fence_after();
-          if (elect_one()) {
-#pragma unroll
-            for (int kk = 0; kk < 2; ++kk)
-              umma_mxf8_ts(tm + TC_DK, sx + TO_DS + 8 * kk, desc_adv(qy, kk * 32 * D),
-                           idesc_bs(128, D, 0, 0, 0, 1, 1, kk, kk), sx + TO_SFA_DK, sx + TO_SFB_Q, accum | kk);
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {   // K = 128 keys
-              if (D == 128)      // A = K tile (M = head dim), B = dS-hat half (N = 64 queries)
-                umma_mxf8_ss(tm + TC_DP + 64 * y, desc_adv(dK_k, kk * 32 * D), desc_adv(dDS0, y * 8192 + kk * 2048),
-                             idesc_bs(128, 64, 0, 0, 1, 1, 1, kk, kk), sx + TO_SFA_DQ, sx + TO_SFB_DQ, kk > 0);
-              else               // A = dS-hat half (M = 64 queries + 64 unused rows), B = K tile (N = head dim)
-                umma_mxf8_ss(tm + TC_DP + 64 * y, desc_adv(dDS_A, y * 8192 + kk * 2048), desc_adv(dK_k, kk * 32 * D),
-                             idesc_bs(128, 64, 0, 0, 1, 1, 1, kk, kk), sx + TO_SFB_DQ, sx + TO_SFA_DQ, kk > 0);
-            }
-            tc_commit(&bars[BB_DQF + y]);
-            if (y == 1) tc_commit(&bars[BB_QEMPTY + st]);
-          }
-          __syncwarp();
+          for (int kk = 0; kk < D / 32; ++kk)
+            umma_f8_ss(tm + TC_DP + 64 * x, desc_adv(dV_k, 32 * kk), desc_adv(dox, 32 * kk), ID_N64, kk > 0);
+          tc_commit(&bars[BB_DP + x]);
         }
+        __syncwarp();
+        return true;
+      };
+      // dQ^T_x, dV, dK of iteration g (P-hat and dS-hat of half x stand in the other half's region); dQ^T first: the reduction
+      // warps read it while the rest runs, and dP^T_x of the next iteration takes its columns
+      auto issue_grads = [&](int g, int x, bool first) -> bool {
+        if (!mbar_wait(&bars[BB_DS + x], g & 1, p.ctl, abortp, 24)) return false;
+        tc_fence_after();
+        if (elect_one()) {
+          const int sa = g % 3, sb = g & 1;
+          const uint32_t ro = tm + TC_S + 64 * (1 - x);
+          const uint64_t qx = desc_adv(dQ0, (FP4 ? sb : sa) * TILE_BYTES + x * 64 * D), dox = desc_adv(dDO0, sb * TILE_BYTES + x * 64 * D);
+          const uint64_t at = desc_adv(dAT0, x * SM::ATOM_STRIDE);
+          const uint32_t accum = first ? 0u : 1u;
+          tmem_cp_sf_atom(ro + TO_SFB_DQ, desc_adv(at, 512));
+          tmem_cp_sf_atom(ro + TO_SFA_DK, at);
+          if (TL) tmem_cp_sf_atom(ro + TO_SFA_P, desc_adv(at, 1024));
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) {   // K = 128 keys
+            if (D == 128)      // A = K tile (M = head dim), B = dS-hat half (N = 64 queries)
+              umma_mxf8_ss(tm + TC_DP + 64 * x, desc_adv(dK_k, kk * 32 * D), desc_adv(dDS0, x * 8192 + kk * 2048),
+                           idesc_bs(128, 64, 0, 0, 1, 1, 1, kk, kk), ro + TO_SFA_DQ, ro + TO_SFB_DQ, kk > 0);
+            else               // A = dS-hat half (M = 64 queries + 64 unused rows), B = K tile (N = head dim)
+              umma_mxf8_ss(tm + TC_DP + 64 * x, desc_adv(dDS_A, x * 8192 + kk * 2048), desc_adv(dK_k, kk * 32 * D),
+                           idesc_bs(128, 64, 0, 0, 1, 1, 1, kk, kk), ro + TO_SFB_DQ, ro + TO_SFA_DQ, kk > 0);
+          }
+          tc_commit(&bars[BB_DQF + x]);
+#pragma unroll
+          for (int kk = 0; kk < 2; ++kk)     // K = 64 queries: two instructions of 32
+            umma_mxf8_ts(tm + TC_DV, ro + TO_P + 8 * kk, desc_adv(dox, kk * 32 * D),
+                         idesc_bs(128, D, 0, 0, 0, 1, 1, kk, kk), ro + TO_SFA_P, ro + TO_SFB_DO, accum | kk);
+#pragma unroll
+          for (int kk = 0; kk < 2; ++kk)
+            umma_mxf8_ts(tm + TC_DK, ro + TO_DS + 8 * kk, desc_adv(qx, kk * 32 * D),
+                         idesc_bs(128, D, 0, 0, 0, 1, 1, kk, kk), ro + TO_SFA_DK, ro + TO_SFB_Q, accum | kk);
+          if (x == 1) { tc_commit(&bars[BB_AEMPTY + sa]); tc_commit(&bars[BB_BEMPTY + sb]); }
+        }
+        __syncwarp();
+        return true;
+      };
+      const uint32_t park0 = tm + TC_DP, park1 = tm + TC_DP + 64;
+      if (n_it > 0) {
+        // the item's first products; they run while the compute warpgroups write the previous item's rows
+        if (!(ok = dq_read(gi, 0) && issue_s(gi, 0, park0) && issue_dp(gi, 0))) break;
+        if (!(ok = dq_read(gi, 1) && issue_s(gi, 1, park1))) break;
+        if (!FP4 && !(ok = issue_dp(gi, 1))) break;
+        if (n_it > 1) {      // S0 of the second iteration: once the first one's scores are in registers
+          if (!(ok = mbar_wait(&bars[BB_SDR], sdr & 1, p.ctl, abortp, 26))) break;
+          ++sdr;
+          if (!(ok = issue_s(gi + 1, 0, park1))) break;
+        }
+        if (FP4 && !(ok = issue_dp(gi, 1))) break;
+      }
+      for (int j = 0; ok && j < n_it; ++j) {
+        const int g = gi + j;
+        // the first products of an item overwrite dV / dK: the previous item's rows must have left tensor memory
+        if (j == 0 && k > 0 && !(ok = mbar_wait(&bars[BB_ACCFREE], (k - 1) & 1, p.ctl, abortp, 25))) break;
+        if (!(ok = issue_grads(g, 0, j == 0))) break;
+        // (P0 and dS0 stood where S1(g) had been: their arrival says that those scores have been read; likewise below)
+        if (j + 1 < n_it) {
+          if (FP4) { if (!(ok = dq_read(g + 1, 0) && issue_s(g + 1, 1, park0) && issue_dp(g + 1, 0))) break; }
+          else if (!(ok = issue_s(g + 1, 1, 0) && dq_read(g + 1, 0) && issue_dp(g + 1, 0))) break;
+        }
+        if (!(ok = issue_grads(g, 1, false))) break;
+        if (FP4 && j + 1 < n_it && !(ok = dq_read(g + 1, 1))) break;
+        if (j + 2 < n_it && !(ok = issue_s(g + 2, 0, park1))) break;
+        if (j + 1 < n_it && !(ok = (FP4 || dq_read(g + 1, 1)) && issue_dp(g + 1, 1))) break;
       }
       if (!ok) break;
       // an item without query tiles issues nothing, but its accumulator hand-over still takes place once
-      if (n_steps == 0 && k > 0 && !(ok = mbar_wait(&bars[BB_ACCFREE], (k - 1) & 1, p.ctl, abortp, 25))) break;
+      if (n_it == 0 && k > 0 && !(ok = mbar_wait(&bars[BB_ACCFREE], (k - 1) & 1, p.ctl, abortp, 25))) break;
       if (elect_one()) tc_commit(&bars[BB_ACC]);       // every product of the item has completed when this arrives
       __syncwarp();
       gi += n_it;
@@ -451,7 +510,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         if (!(ok = mbar_wait(&bars[BB_R1], gt & 1, p.ctl, abortp, 41))) break;
         if (!(ok = mbar_wait(&bars[BB_DQF + y], g & 1, p.ctl, abortp, 40))) break;
         tc_fence_after();
-        const uint32_t rowp = smem_u32(sDQ) + y * 16384 + r * 128;
+        const uint32_t rowp = smem_u32(smem) + SM::DQ + y * 16384 + r * 128;
         // d = 128: thread = head-dim row of dQ^T, 64 query columns. d = 64: thread = query row (the first 64 lanes; the
         // other two warps hold the product's unused rows), 64 head-dim columns. Either way 64 f16 = one 128-byte row.
         if (D == 128 || warp < 10) {
@@ -480,8 +539,8 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const bool det = FULL && p.dq_order != nullptr;
         if (!det) {
           if (tid == 256) {
-            if (D == 128) tma_reduce_add_4d(&tm_acc, sDQ + y * 16384, T.q0 + m * 128 + 64 * y, 0, head, T.bat);
-            else tma_reduce_add_4d(&tm_acc, sDQ + y * 16384, 0, T.q0 + m * 128 + 64 * y, head, T.bat);
+            if (D == 128) tma_reduce_add_4d(&tm_acc, smem + SM::DQ + y * 16384, T.q0 + m * 128 + 64 * y, 0, head, T.bat);
+            else tma_reduce_add_4d(&tm_acc, smem + SM::DQ + y * 16384, 0, T.q0 + m * 128 + 64 * y, head, T.bat);
             tma_store_commit();
           }
         } else if (warp == 8) {                 // (the whole warp stays converged: lane 0 works, the others follow its result)
@@ -506,8 +565,8 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             go = __shfl_sync(0xFFFFFFFFu, go, 0);
           }
           if (go && lane == 0) {
-            if (D == 128) tma_reduce_add_4d(&tm_acc, sDQ + y * 16384, T.q0 + m * 128 + 64 * y, 0, head, T.bat);
-            else tma_reduce_add_4d(&tm_acc, sDQ + y * 16384, 0, T.q0 + m * 128 + 64 * y, head, T.bat);
+            if (D == 128) tma_reduce_add_4d(&tm_acc, smem + SM::DQ + y * 16384, T.q0 + m * 128 + 64 * y, 0, head, T.bat);
+            else tma_reduce_add_4d(&tm_acc, smem + SM::DQ + y * 16384, 0, T.q0 + m * 128 + 64 * y, head, T.bat);
             tma_store_commit();
             if (order) {
               tma_store_wait<0>();                // the addition has completed, not only read its source
@@ -531,9 +590,14 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     const int r = wq * 32 + lane;                    // key row of the tile = TMEM lane
     const uint32_t lane_base = tmem + ((uint32_t)(wq * 32) << 16);
     const uint32_t t_sx = lane_base + TC_S + 64 * x, t_dpx = lane_base + TC_DP + 64 * x;
-    const uint32_t ds_row = smem_u32(sDS) + x * 8192 + r * 64;
+    const uint32_t t_ox = lane_base + TC_S + 64 * (1 - x);           // where P-hat, dS-hat and the scale columns go
+    const uint32_t ds_row = smem_u32(smem) + SM::DS + x * 8192 + r * 64;
+    // this thread's words of the scale atoms (row r of a 128-row atom: word (r % 32) * 4 + r / 32; query rows 0..63 likewise)
+    const uint32_t at = smem_u32(smem) + SM::ATOMS + x * SM::ATOM_STRIDE;
+    const uint32_t at_row = at + lane * 16 + wq * 4, at_q = at + 512 + lane * 16 + wq;
     bool ok = true;
     int gi = 0, epi = 0;                             // iterations so far; uses of the epilogue barrier so far
+    int cg = 0;                                      // grants used so far
     int pending_kve = -1;                            // the K / V buffer whose gradient stores are still to be confirmed
     for (int k = 0; ok; ++k) {
       const int L = bwd_item(k, G, cta, p.zigzag);
@@ -544,8 +608,8 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       // this item's buffers are released); otherwise a register copy
       const BTile Tcopy = tile_s[kb];
       const BTile& T = TL ? tile_s[kb] : Tcopy;
-      const int hkv = T.hkv, n_m = T.n_m, m_lo = T.m_lo;
-      const int n_it = n_m * grp;
+      const int hkv = T.hkv;
+      const int n_it = T.n_m * grp;
       const int krel = T.krel + r;
       const bool key_valid = r < T.nv;
       const size_t bh_k = (size_t)T.bat * p.h_kv + hkv;
@@ -561,44 +625,51 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           ek_word |= ((__float_as_uint(p.fac_k[bh_k * (p.s_k / 32) + T.k0 / 32 + kbk]) >> 23) & 0xFF) << (8 * kbk);
       }
       const int vis_from = p.win_r >= 0 ? (krel - T.off - p.win_r) : 0;    // queries in [vis_from, vis_to] see this key
-      const int vis_to = p.win_l >= 0 ? (krel - T.off + p.win_l) : 0x7FFFFFFF;
-      for (int it = 0; it < n_it; ++it) {
-        const int g = gi + it, st = g & 1, u = g >> 1;
-        const int head = hkv * grp + it / n_m, m = m_lo + it % n_m;
-        if (it == 1 && pending_kve >= 0) {
-          // the previous item's gradient stores have long read their shared-memory source: its K / V buffer goes back
-          if (r == 0) { tma_store_wait_read<0>(); mbar_arrive(&bars[BB_KVE + pending_kve]); }
-          pending_kve = -1;
+      const int vis_to = min(p.win_l >= 0 ? (krel - T.off + p.win_l) : 0x7FFFFFFF, T.sq - 1);
+      // one iteration's scalars: the half's two 32-query factors of Q and dO, the query tile's pre-scale. Loaded an iteration
+      // ahead: the tensor core's results are waiting when an iteration begins, so nothing else would hide their latency.
+      int head = hkv * grp, m = T.m_lo;
+      float2 fq_n = {1.f, 1.f}, fd_n = {1.f, 1.f};
+      float bsc_n = 1.f;
+      const bool pre_rows = FULL && p.dq_scale_rows != nullptr;
+      auto load_scalars = [&]() {
+        if (!TL) {
+          const size_t o = ((size_t)T.bat * p.h + head) * (p.s_q / 32) + (T.q0 + m * 128) / 32 + 2 * x;
+          fq_n = __ldg(reinterpret_cast<const float2*>(p.fac_q + o));
+          fd_n = __ldg(reinterpret_cast<const float2*>(p.fac_do + o));
         }
+        if (!pre_rows) bsc_n = __ldg(p.dq_scale + (size_t)T.bat * (p.s_q / 128) + T.q0 / 128 + m);
+      };
+      if (n_it > 0) load_scalars();
+      for (int it = 0; it < n_it; ++it) {
+        const int g = gi + it, st = g & 1;
         const size_t bh_q = (size_t)T.bat * p.h + head;
-        const int qb0 = (T.q0 + m * 128) / 32 + 2 * x;                     // first of the half's two 32-query blocks
-        const float fq0 = TL ? 1.f : p.fac_q[bh_q * (p.s_q / 32) + qb0], fq1 = TL ? 1.f : p.fac_q[bh_q * (p.s_q / 32) + qb0 + 1];
-        const float fd0 = TL ? 1.f : p.fac_do[bh_q * (p.s_q / 32) + qb0], fd1 = TL ? 1.f : p.fac_do[bh_q * (p.s_q / 32) + qb0 + 1];
         // token-local: the 64 per-query factors of the half (same addresses for every thread: broadcast loads)
         const float4* fq_vec = reinterpret_cast<const float4*>(p.fac_q + (TL ? bh_q * p.s_q + T.q0 + m * 128 + 64 * x : 0));
         const float4* fdo_vec = reinterpret_cast<const float4*>(p.fac_do + (TL ? bh_q * p.s_q + T.q0 + m * 128 + 64 * x : 0));
         // the f16 pre-scale: one power of two per query tile (folded into K's exponent bytes below), or one per query row
         // (folded into the dQ side's B scale bytes, whose lanes are the queries)
-        const bool pre_rows = FULL && p.dq_scale_rows != nullptr;
-        const float bsc = pre_rows ? 1.0f : p.dq_scale[(size_t)T.bat * (p.s_q / 128) + T.q0 / 128 + m];
+        const float bsc = bsc_n;
         [[maybe_unused]] uint32_t lq0 = 0, lq1 = 0;
         if (pre_rows) {
           const float* rp = p.dq_scale_rows + (size_t)T.bat * p.s_q + T.q0 + m * 128 + 64 * x;
-          lq0 = ((uint32_t)((int)((__float_as_uint(rp[lane]) >> 23) & 0xFF) - 127) & 0xFF) * 0x01010101u;
-          lq1 = ((uint32_t)((int)((__float_as_uint(rp[32 + lane]) >> 23) & 0xFF) - 127) & 0xFF) * 0x01010101u;
+          lq0 = (uint32_t)((int)((__float_as_uint(rp[lane]) >> 23) & 0xFF) - 127);
+          lq1 = (uint32_t)((int)((__float_as_uint(rp[32 + lane]) >> 23) & 0xFF) - 127);
         }
         // FP4: the block scales of S were applied by the tensor core; only the softmax scale remains
-        const float c[2] = {FP4 ? p.scale_log2 : fk * fq0, FP4 ? p.scale_log2 : fk * fq1}, b8[2] = {fv8 * fd0, fv8 * fd1};
-        // token-local: fq0 = fq1 = fd0 = fd1 = 1, i.e. unit scale bytes for the Q and dO operands
-        const uint32_t eq2 = ((__float_as_uint(fq0) >> 23) & 0xFF) | (((__float_as_uint(fq1) >> 23) & 0xFF) << 8);
-        const uint32_t edo2 = ((__float_as_uint(fd0) >> 23) & 0xFF) | (((__float_as_uint(fd1) >> 23) & 0xFF) << 8);
+        const float c[2] = {FP4 ? p.scale_log2 : fk * fq_n.x, FP4 ? p.scale_log2 : fk * fq_n.y}, b8[2] = {fv8 * fd_n.x, fv8 * fd_n.y};
+        // token-local: fq = fd = 1, i.e. unit scale bytes for the Q and dO operands
+        const uint32_t eq2 = ((__float_as_uint(fq_n.x) >> 23) & 0xFF) | (((__float_as_uint(fq_n.y) >> 23) & 0xFF) << 8);
+        const uint32_t edo2 = ((__float_as_uint(fd_n.x) >> 23) & 0xFF) | (((__float_as_uint(fd_n.y) >> 23) & 0xFF) << 8);
         // K's exponent bytes with the power-of-two f16 pre-scale of this query tile folded in (A scale of dQ^T)
         const uint32_t lb = (uint32_t)((int)((__float_as_uint(bsc) >> 23) & 0xFF) - 127) & 0xFF;
         const uint32_t ekb_word = __vadd4(ek_word, lb * 0x01010101u);
-        if (!(ok = mbar_wait(&bars[BB_QFULL + st], u & 1, p.ctl, abortp, 30))) break;   // lse / D'' vectors visible
-        const uint32_t v_lse = smem_u32(sVec) + (st * 256 + 64 * x) * 4, v_dpp = v_lse + 512;
         const int q_first = m * 128 + 64 * x;                              // document-relative query of column 0
-        const bool full = key_valid && (q_first >= vis_from) && (q_first + 63 <= vis_to) && (q_first + 64 <= T.sq);
+        const bool full = key_valid && (q_first >= vis_from) && (q_first + 63 <= vis_to);
+        if (++m == T.m_lo + T.n_m) { m = T.m_lo; ++head; }                  // (the next iteration's from here on)
+        if (it + 1 < n_it) load_scalars();
+        if (!(ok = mbar_wait(&bars[BB_BFULL + st], (g >> 1) & 1, p.ctl, abortp, 30))) break;   // lse / D'' vectors visible
+        const uint32_t v_lse = smem_u32(smem) + SM::VEC + st * 1024 + 256 * x, v_dpp = v_lse + 512;
 
         // ---- P' = 2^(s c - lse2)
         if (!(ok = mbar_wait(&bars[BB_S + x], g & 1, p.ctl, abortp, 31))) break;
@@ -607,8 +678,14 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         FL_TMEM_LD_32(t_sx, pv);
         FL_TMEM_LD_32(t_sx + 32, (pv + 32));
         tc_wait_ld();
+        // the scores are in registers: this region may take the other half's P-hat and dS-hat (half 0's iteration waits for S1 of
+        // the same iteration; half 1's for S0 of the next one, which is issued before, or of this one where that was the last)
+        tc_fence_before();
+        if (x == 1 || it > 0 || n_it == 1) mbar_arrive_warp(&bars[BB_GRANT + (1 - x)]);
+        if (x == 0 && it == 0 && n_it > 1) mbar_arrive_warp(&bars[BB_SDR]);
         float pf[64];
-        [[maybe_unused]] uint32_t pw_sc[SC ? 16 : 1];
+        [[maybe_unused]] uint32_t pw_ep = 0;
+        uint32_t pw[16];                  // P-hat's codes, kept until the region they go to is free
         if constexpr (SC) {
           // soft cap: x = cap_a tanh(s c cap_b); P-hat is taken from P' right here, and what stays in pf is
           // P' (1 - tanh^2), the factor dS needs (the reference's score_mod_bwd, flash_attn/cute/utils.py:178-187)
@@ -625,10 +702,10 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
               df[e] = fmaf(-th, th, 1.0f);
               if (!full) {
                 const int qi = q_first + 4 * j4 + e;
-                pp[e] = (key_valid && qi >= vis_from && qi <= vis_to && qi < T.sq) ? pp[e] : 0.f;
+                pp[e] = (key_valid && qi >= vis_from && qi <= vis_to) ? pp[e] : 0.f;
               }
             }
-            pw_sc[j4] = cvt_e4m3x4(pp[0], pp[1], pp[2], pp[3]);
+            pw[j4] = cvt_e4m3x4(pp[0], pp[1], pp[2], pp[3]);
 #pragma unroll
             for (int e = 0; e < 4; ++e) pf[4 * j4 + e] = pp[e] * df[e];
           }
@@ -637,42 +714,35 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           for (int j4 = 0; j4 < 16; ++j4) {
             const float4 l4 = lds128(v_lse + 16 * j4);
             const float cc = c[j4 >> 3];
+            // t = lse2 - s c (token-local: c = f_K f_Q(query)), two columns per instruction; P' = 2^-t
+            uint64_t c01, c23;
             if (TL) {
-              // t = lse2 - s f_K f_Q(query), two columns per instruction
               const float4 f4 = __ldg(fq_vec + j4);
               const uint64_t nfk2 = pack2(-fk, -fk);
-              float t0, t1, t2, t3;
-              unpack2(fma2(pack2(__uint_as_float(pv[4 * j4 + 0]), __uint_as_float(pv[4 * j4 + 1])),
-                           mul2(pack2(f4.x, f4.y), nfk2), pack2(l4.x, l4.y)), t0, t1);
-              unpack2(fma2(pack2(__uint_as_float(pv[4 * j4 + 2]), __uint_as_float(pv[4 * j4 + 3])),
-                           mul2(pack2(f4.z, f4.w), nfk2), pack2(l4.z, l4.w)), t2, t3);
-              pf[4 * j4 + 0] = ex2_neg(t0);
-              pf[4 * j4 + 1] = ex2_neg(t1);
-              pf[4 * j4 + 2] = ex2_neg(t2);
-              pf[4 * j4 + 3] = ex2_neg(t3);
+              c01 = mul2(pack2(f4.x, f4.y), nfk2);
+              c23 = mul2(pack2(f4.z, f4.w), nfk2);
             } else {
-              // two columns per instruction: t = lse2 - s c, P' = 2^-t
-              const uint64_t nc2 = pack2(-cc, -cc);
-              float t0, t1, t2, t3;
-              unpack2(fma2(pack2(__uint_as_float(pv[4 * j4 + 0]), __uint_as_float(pv[4 * j4 + 1])), nc2, pack2(l4.x, l4.y)), t0, t1);
-              unpack2(fma2(pack2(__uint_as_float(pv[4 * j4 + 2]), __uint_as_float(pv[4 * j4 + 3])), nc2, pack2(l4.z, l4.w)), t2, t3);
-              pf[4 * j4 + 0] = ex2_neg(t0);
-              pf[4 * j4 + 1] = ex2_neg(t1);
-              pf[4 * j4 + 2] = ex2_neg(t2);
-              pf[4 * j4 + 3] = ex2_neg(t3);
+              c01 = c23 = pack2(-cc, -cc);
             }
+            float t0, t1, t2, t3;
+            unpack2(fma2(pack2(__uint_as_float(pv[4 * j4 + 0]), __uint_as_float(pv[4 * j4 + 1])), c01, pack2(l4.x, l4.y)), t0, t1);
+            unpack2(fma2(pack2(__uint_as_float(pv[4 * j4 + 2]), __uint_as_float(pv[4 * j4 + 3])), c23, pack2(l4.z, l4.w)), t2, t3);
+            pf[4 * j4 + 0] = ex2_neg(t0);
+            pf[4 * j4 + 1] = ex2_neg(t1);
+            pf[4 * j4 + 2] = ex2_neg(t2);
+            pf[4 * j4 + 3] = ex2_neg(t3);
           }
         }
         if (!SC && !full) {      // diagonal / tail tiles only
 #pragma unroll
           for (int j = 0; j < 64; ++j) {
             const int qi = q_first + j;
-            pf[j] = (key_valid && qi >= vis_from && qi <= vis_to && qi < T.sq) ? pf[j] : 0.f;
+            pf[j] = (key_valid && qi >= vis_from && qi <= vis_to) ? pf[j] : 0.f;
           }
         }
         if (TL) {
           // block-scaled P-hat carrying f_dO(query): one exponent per (this key row, 32 queries)
-          uint32_t pw[16], ep[2];
+          uint32_t ep[2];
 #pragma unroll
           for (int qh = 0; qh < 2; ++qh) {
             float t[32];
@@ -696,29 +766,24 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
               pw[qh * 8 + w] = cvt_e4m3x4(a0, a1, a2, a3);
             }
           }
-          FL_TMEM_ST_16(t_sx + TO_P, pw);
-          // every lane quadrant holds the whole A scale tile: column = key block, lane = row of the block
-          sEP[x][r] = ep[0] | (ep[1] << 8);
-          mbar_arrive_warp(&bars[BB_EP + x]);
-          if (!(ok = mbar_wait(&bars[BB_EP + x], g & 1, p.ctl, abortp, 37))) break;
-          uint32_t sf[8] = {sEP[x][lane], sEP[x][32 + lane], sEP[x][64 + lane], sEP[x][96 + lane],
-                            0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu};
-          FL_TMEM_ST_8(t_sx + TO_SFA_P, sf);
-        } else {
-          uint32_t pw[16];
+          // (this atom's last reader, the dV product of the iteration before, has completed when dP^T has, which is waited for below;
+          // the words are kept in registers until then)
+          pw_ep = ep[0] | (ep[1] << 8);
+        } else if constexpr (!SC) {
 #pragma unroll
-          for (int w = 0; w < 16; ++w) {
-            if constexpr (SC) pw[w] = pw_sc[w];
-            else pw[w] = cvt_e4m3x4(pf[4 * w], pf[4 * w + 1], pf[4 * w + 2], pf[4 * w + 3]);
-          }
-          FL_TMEM_ST_16(t_sx + TO_P, pw);
-          // scale tiles of the dV product: A = 1, B = dO's exponent per 32 queries (bytes = the half's two K steps)
-          uint32_t sf[8] = {0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, edo2, edo2, edo2, edo2};
-          FL_TMEM_ST_8(t_sx + TO_SFA_P, sf);
+          for (int w = 0; w < 16; ++w) pw[w] = cvt_e4m3x4(pf[4 * w], pf[4 * w + 1], pf[4 * w + 2], pf[4 * w + 3]);
         }
-        tc_wait_st();
-        tc_fence_before();
-        mbar_arrive_warp(&bars[BB_P + x]);
+        if (it == 0 && pending_kve >= 0) {
+          // the previous item's gradient stores have long read their shared-memory source: its K / V buffer goes back (and, where
+          // the scale atoms share the way out's memory, the whole warpgroup has to know)
+          if (r == 0) { tma_store_wait_read<0>(); mbar_arrive(&bars[BB_KVE + pending_kve]); }
+          pending_kve = -1;
+          if (EPI2) {
+            mbar_arrive_warp(&bars[BB_EPI + x]);
+            if (!(ok = mbar_wait(&bars[BB_EPI + x], epi & 1, p.ctl, abortp, 38))) break;
+            ++epi;
+          }
+        }
 
         // ---- dS = P' (b dP + D''), block exponent per (this warp's 32 keys, 32 queries)
         if (!(ok = mbar_wait(&bars[BB_DP + x], g & 1, p.ctl, abortp, 32))) break;
@@ -760,8 +825,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
               am = fmax3_abs(fmax3_abs(am, pf[j], pf[j + 1]), pf[j + 2], pf[j + 3]);
             }
           }
-          const uint32_t wm = warp_max_u32(__float_as_uint(am));          // non-negative floats order as integers
-          ebyte[qh] = exp448(wm);                                          // 448 * 2^(e-127) >= amax
+          ebyte[qh] = exp448(warp_max_abs_f32(am));                        // 448 * 2^(e-127) >= amax
         }
         if (!full) {      // diagonal / tail tiles only
           // masked entries hold P' = 0, but their dP^T or D'' may come from rows outside the document (padding or whatever
@@ -770,11 +834,16 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #pragma unroll
           for (int j = 0; j < 64; ++j) {
             const int qi = q_first + j;
-            pf[j] = (key_valid && qi >= vis_from && qi <= vis_to && qi < T.sq) ? pf[j] : 0.f;
+            pf[j] = (key_valid && qi >= vis_from && qi <= vis_to) ? pf[j] : 0.f;
           }
         }
-        if (lane == 0) sE[x][wq] = ebyte[0] | (ebyte[1] << 8);
-        if (!RL) mbar_arrive_warp(&bars[BB_EX + x]);
+        // dK's A scales: row = key; bytes = the half's two query blocks
+        sts32(at_row, ebyte[0] | (ebyte[1] << 8));
+        if (TL) sts32(at_row + 1024, pw_ep);
+        if (!RL) {          // dQ's query-side scales: row = query; byte = this warp's key block (+ the row's pre-scale)
+          sts8(at_q, ebyte[0] + lq0);
+          sts8(at_q + 4, ebyte[1] + lq1);
+        }
         uint32_t dsw[16];
 #pragma unroll
         for (int qh = 0; qh < 2; ++qh) {
@@ -796,7 +865,21 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             }
           }
         }
-        FL_TMEM_ST_16(t_sx + TO_DS, dsw);
+        // the other half's scores must have left the region (long since, when the halves run half an iteration apart)
+        if (x == 0 || it + 1 < n_it || n_it == 1) {
+          if (!(ok = mbar_wait(&bars[BB_GRANT + x], cg & 1, p.ctl, abortp, 36))) break;
+          ++cg;
+          tc_fence_after();
+        }
+        FL_TMEM_ST_16(t_ox + TO_P, pw);
+        FL_TMEM_ST_16(t_ox + TO_DS, dsw);
+        {
+          // dV: A = 1 (token-local: the issuer's copy of P-hat's atom follows), B = dO's exponent per 32 queries (bytes = the
+          // half's two K steps); dK: B = Q's exponents; dQ^T: A[head-dim lane] = K's exponents (+ pre-scale) per key block
+          uint32_t sf[16] = {0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, edo2, edo2, edo2, edo2,
+                             eq2, eq2, eq2, eq2, ekb_word, ekb_word, ekb_word, ekb_word};
+          FL_TMEM_ST_16(t_ox + TO_SFA_P, sf);
+        }
         if (RL) {
           // the dQ side's own codes: one exponent per (query, this warp's 32 keys); token-local: they carry f_K(key)
           // per column: t = the exponent field of 2^(e - 119), e the UE8M0 byte with 448 * 2^(e - 127) >= amax, floored
@@ -817,40 +900,15 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             }
             dsw[w] = cvt_e4m3x4(v[0], v[1], v[2], v[3]);
           }
-          sEQ[x][lane][wq] = (uint8_t)((mine[0] >> 23) - 8);
-          sEQ[x][32 + lane][wq] = (uint8_t)((mine[1] >> 23) - 8);
-          mbar_arrive_warp(&bars[BB_EX + x]);
+          sts8(at_q, ((mine[0] >> 23) - 8) + lq0);
+          sts8(at_q + 4, ((mine[1] >> 23) - 8) + lq1);
         }
         // the dQ^T product's MN-major B operand: row = key, 64 bytes = 4 chunks of 16 B, 64 B swizzle
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4)
           sts128(ds_row + ((q4 ^ ((r >> 1) & 3)) << 4), dsw[4 * q4], dsw[4 * q4 + 1], dsw[4 * q4 + 2], dsw[4 * q4 + 3]);
-        if (!(ok = mbar_wait(&bars[BB_EX + x], g & 1, p.ctl, abortp, 36))) break;
-        {
-          // dK:   A[key lane, column = key block]  bytes = the half's two query blocks;  B = Q's exponents
-          // dQ^T: A[head-dim lane] = K's exponents (+ pre-scale) per key block; B[query lane, column = query block of
-          //       the half] bytes = the four key blocks
-          const uint32_t e0 = sE[x][0], e1 = sE[x][1], e2 = sE[x][2], e3 = sE[x][3];
-          uint32_t sf[16];
-          sf[0] = e0; sf[1] = e1; sf[2] = e2; sf[3] = e3;
-          sf[4] = sf[5] = sf[6] = sf[7] = eq2;
-          sf[8] = sf[9] = sf[10] = sf[11] = ekb_word;
-          if (RL) {   // B[query lane, column = query block] bytes = that query's exponents over the four key blocks
-            sf[12] = *reinterpret_cast<const uint32_t*>(&sEQ[x][lane][0]);
-            sf[13] = *reinterpret_cast<const uint32_t*>(&sEQ[x][32 + lane][0]);
-          } else {
-            sf[12] = (e0 & 0xFF) | ((e1 & 0xFF) << 8) | ((e2 & 0xFF) << 16) | ((e3 & 0xFF) << 24);
-            sf[13] = ((e0 >> 8) & 0xFF) | (((e1 >> 8) & 0xFF) << 8) | (((e2 >> 8) & 0xFF) << 16) | (((e3 >> 8) & 0xFF) << 24);
-          }
-          if constexpr (FULL) {
-            sf[12] = __vadd4(sf[12], lq0);
-            sf[13] = __vadd4(sf[13], lq1);
-          }
-          sf[14] = sf[15] = 0x7F7F7F7Fu;
-          FL_TMEM_ST_16(t_sx + TO_SFA_DK, sf);
-        }
         tc_wait_st();
-        fence_proxy_async();             // the dS-hat tile in shared memory is read by the tensor core (async proxy)
+        fence_proxy_async();             // the dS-hat tile and the atoms in shared memory are read by the tensor core (async proxy)
         tc_fence_before();
         mbar_arrive_warp(&bars[BB_DS + x]);
       }
@@ -921,8 +979,8 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           if (!(ok = mbar_wait(&bars[BB_EPI + x], epi & 1, p.ctl, abortp, 38))) break;
           ++epi;
         }
-        uint8_t* stage0 = (D == 128) ? ((x == 0 ? sK : sV) + kb * TILE_BYTES) : (sOut64 + x * 16384);
-        uint8_t* stage1 = EPI2 ? (sOut2 + x * 16384) : stage0;
+        uint8_t* stage0 = smem + ((D == 128) ? ((x == 0 ? SM::K : SM::V) + kb * TILE_BYTES) : (SM::OUT + x * 16384));
+        uint8_t* stage1 = EPI2 ? (smem + SM::OUT + x * 16384) : stage0;
         const CUtensorMap* tm_out = (x == 0) ? &tm_dv : &tm_dk;
         // packed output: the key tile is slot T.k0 / 128 of the aligned buffer; its rows go to the packed rows out_row ..
         // + out_n of the caller's tensor: a full slot as TMA stores, a document's last rows row by row
@@ -985,7 +1043,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     // the shared-memory sources of the last stores must outlive the copies (the writes complete with the grid)
     if (r == 0) tma_store_wait_read<0>();
   }
-  if (abort_s) {
+  if (misc.abort) {
     for (int it = 0; it < 200; ++it) __nanosleep(1000);
   }
   tc_fence_before();
@@ -1066,8 +1124,7 @@ extern "C" int fl_bwd(const fl_attn_args* a, void* stream) {
   p.n_items = (int)n_items;
   p.zigzag = (p.causal && !a->doc_start) ? 1 : 0;
   const int grid = (int)(n_items < sm_count() ? n_items : sm_count());     // one persistent CTA per SM
-  const int smem = 8 * 128 * a->d + 2 * 8192 + 2 * 16384 + 2048 + ((a->d == 64 || !fp4) ? 2 * 16384 : 0) + 1024 +
-                   (fp4 ? 4 * 8192 + 4 * 1024 : 0);
+  const int smem = a->d == 64 ? BwdSmem<64, false>::BYTES : fp4 ? BwdSmem<128, true>::BYTES : BwdSmem<128, false>::BYTES;
   auto launch = [&](auto kern) -> int {
     if (int e = set_smem(kern, smem, "fl_bwd: cudaFuncSetAttribute")) return e;
     kern<<<grid, 512, smem, (cudaStream_t)stream>>>(mq, mk, mv, mdo, macc, mq4, mk4, mdk, mdv, p);

@@ -333,10 +333,10 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
-// max(a, |b|, |c|)
+// max(|a|, |b|, |c|) (a NaN does not take part)
 __device__ __forceinline__ float fmax3_abs(float a, float b, float c) {
   float d;
-  asm("{\n\t.reg .f32 x, y;\n\tabs.f32 x, %2;\n\tabs.f32 y, %3;\n\tmax.f32 %0, %1, x, y;\n\t}" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
 // 2^(-x)
