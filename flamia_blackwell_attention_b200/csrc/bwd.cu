@@ -24,7 +24,8 @@
 //   A = dS-hat (shared memory, MN-major; its second 64-row block is whatever follows in memory and only fills the
 //   unused rows 64..127 of the result) and B = the K tile; rows = queries, accumulator layout (b, h, s, d)
 //   warps 0-3 compute half 0, warps 4-7 compute half 1 (thread = key row = TMEM lane, 64 query columns)
-//   warps 8-11 dQ reduction (thread = head-dim row)      warp 12 UMMA issuer      warp 13 TMA producer
+//   warps 8-11 dQ reduction (thread = head-dim row)      warp 13 TMA producer
+//   warp 12 UMMA issuer of dQ^T, dV, dK                  warp 14 UMMA issuer of S^T, dP^T
 // TMEM: [0,64) / [64,128) S^T_x; [128,256) dV; [256,320) / [320,384) dP^T_x, then dQ^T_x; [384,512) dK.
 // P-hat, dS-hat and the scale tiles of a half go to the OTHER half's S^T columns (P-hat +0, dS-hat +16, scale tiles +32..+56): the
 // compute warps read all 64 scores of a row into registers at once, so their own S^T columns take the next scores while they
@@ -106,9 +107,10 @@ struct BTile {
 };
 
 // barriers; [2] = one per half, stage or buffer, [3] = one per stage of the score operand's ring
-enum { BB_KV = 0, BB_KVE = 2, BB_AFULL = 4, BB_AEMPTY = 7, BB_BFULL = 10, BB_BEMPTY = 12, BB_S = 14, BB_DP = 16, BB_GRANT = 18,
-       BB_DS = 20, BB_DQF = 22, BB_DQE = 24, BB_EPI = 26, BB_R1 = 28, BB_R2 = 29, BB_ACC = 30, BB_ACCFREE = 31, BB_SDR = 32,
-       BB_COUNT = 33 };
+// (B ring: [stage][half])
+enum { BB_KV = 0, BB_KVE = 2, BB_AFULL = 4, BB_AEMPTY = 7, BB_BFULL = 10, BB_BEMPTY = 14, BB_S = 18, BB_DP = 20, BB_GRANT = 22,
+       BB_DS = 24, BB_DQF = 26, BB_DQE = 28, BB_EPI = 30, BB_R1 = 32, BB_R2 = 33, BB_ACC = 34, BB_ACCFREE = 35, BB_SDR = 36,
+       BB_COUNT = 37 };
 // TMEM columns; the per-half regions are at + 64 * x
 enum { TC_S = 0, TO_P = 0, TO_DS = 16, TO_SFA_P = 32, TO_SFB_DO = 36, TO_SFB_Q = 40, TO_SFA_DQ = 44, TO_SFA_DK = 48,
        TO_SFB_DQ = 52, TC_DV = 128, TC_DP = 256, TC_DK = 384 };
@@ -205,12 +207,16 @@ struct BwdMisc {
   uint32_t tmem_base;
   int abort;
   BTile tile[2];            // the items in flight (written by the producer, item k in slot k & 1)
+  // ring B's scalars [stage][half]: Q's and dO's factors of the half's two 32-query blocks, then the query tile's pre-scale. Read
+  // from global memory by the producer: a load that misses in a compute warp stalls it at its next scoreboard wait (every
+  // second iteration, by 700 clocks), whatever the distance to the value's use.
+  alignas(16) float scal[2][2][8];
 };
-template <int D, bool FP4>
+template <int D, bool FP4, bool TL>
 struct BwdSmem {
   static constexpr int TILE = 128 * D;
   static constexpr int A_TILE = FP4 ? 8192 : TILE;                  // the score operand: Q, or its NVFP4 copy
-  static constexpr bool EPI2 = D == 128 && !FP4;                    // a second way out for the gradient rows, see the item epilogue
+  static constexpr bool EPI2 = D == 128 && !FP4 && !TL;             // a second way out for the gradient rows, see the item epilogue
   static constexpr int K = 0;                                       // 2 buffers (items alternate)
   static constexpr int V = K + 2 * TILE;                            // 2 buffers
   static constexpr int DO = V + 2 * TILE;                           // 2 stages
@@ -221,12 +227,13 @@ struct BwdSmem {
   static constexpr int OUT = DQ + 2 * 16384;                        // gradient rows' way out: EPI2 or d = 64, 2 x 16 KB
   static constexpr int K4 = OUT + ((EPI2 || D == 64) ? 2 * 16384 : 0);   // FP4: NVFP4 K tiles, 2 x 8 KB
   static constexpr int SF = K4 + (FP4 ? 2 * 8192 : 0);              // FP4: scale atoms, K 2 x 1 KB then Q 3 x 1 KB
-  static constexpr int VEC = SF + (FP4 ? 5 * 1024 : 0);             // 2 stages x {lse_log2[128], D''[128]}
+  static constexpr int VEC = SF + (FP4 ? 5 * 1024 : 0);             // 2 stages x 2 halves x {lse_log2[64], D''[64]; TL: f_Q[64], f_dO[64]}
+  static constexpr int VEC_HALF = TL ? 1024 : 512;
   // per half three scale atoms of 512 bytes (dK's A side, dQ's query side, P-hat's), written by the compute warps and copied by
   // the issuer. EPI2: inside the half's own part of OUT, in use only between an item's last product and the next item's first dS.
   static constexpr int ATOM_STRIDE = EPI2 ? 16384 : 1536;
-  static constexpr int ATOMS = EPI2 ? OUT : VEC + 2048;
-  static constexpr int MISC = EPI2 ? VEC + 2048 : ATOMS + 2 * ATOM_STRIDE;
+  static constexpr int ATOMS = EPI2 ? OUT : VEC + 4 * VEC_HALF;
+  static constexpr int MISC = EPI2 ? VEC + 4 * VEC_HALF : ATOMS + 2 * ATOM_STRIDE;
   static constexpr int BYTES = MISC + 1024;
   static_assert(sizeof(BwdMisc) <= 1024 && BYTES <= 227 * 1024);
 };
@@ -241,7 +248,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                      const __grid_constant__ CUtensorMap tm_acc, const __grid_constant__ CUtensorMap tm_q4,
                      const __grid_constant__ CUtensorMap tm_k4, const __grid_constant__ CUtensorMap tm_dk,
                      const __grid_constant__ CUtensorMap tm_dv, const BwdParams p) {
-  using SM = BwdSmem<D, FP4>;
+  using SM = BwdSmem<D, FP4, VAR == 2>;
   constexpr int TILE_BYTES = 128 * D;
   constexpr uint64_t OP_SWZ = (D == 128) ? SWZ_128 : SWZ_64;     // operand tiles: rows of D bytes
   constexpr uint32_t OP_SBO = 8 * D;
@@ -265,7 +272,8 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     misc.abort = 0;
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars[BB_KV + i], 1); mbar_init(&bars[BB_KVE + i], 2);      // released by one thread of each compute warpgroup
-      mbar_init(&bars[BB_BFULL + i], 1); mbar_init(&bars[BB_BEMPTY + i], 1);
+      mbar_init(&bars[BB_BFULL + 2 * i], 1); mbar_init(&bars[BB_BEMPTY + 2 * i], 1);
+      mbar_init(&bars[BB_BFULL + 2 * i + 1], 1); mbar_init(&bars[BB_BEMPTY + 2 * i + 1], 1);
       mbar_init(&bars[BB_S + i], 1); mbar_init(&bars[BB_DP + i], 1);
       mbar_init(&bars[BB_GRANT + i], 4); mbar_init(&bars[BB_DS + i], 4);      // one arrival per warp
       mbar_init(&bars[BB_DQF + i], 1); mbar_init(&bars[BB_DQE + i], 4);
@@ -328,39 +336,60 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const int n_it = t.n_m * grp;
         int head = t.hkv * grp, m = t.m_lo;
         for (int it = 0; it < n_it; ++it, ++gi) {
-          // ring A: the scores' query operand, one tile further ahead than ring B (dO, the row vectors, FP4: the E4M3 Q)
+          // ring A: the scores' query operand, three stages of a whole query tile. Ring B: dO, the row vectors, FP4: the E4M3 Q; two
+          // stages in halves of 64 queries, each given back when its half is done: a whole period to load the next one in
+          // (as whole tiles it was half a period, less than a load takes)
           const int sa = gi % 3, ra = gi / 3, sb = gi & 1, rb = gi >> 1;
           const int qrow = t.q0 + m * 128;
           const size_t ro = ((size_t)t.bat * p.h + head) * p.s_q + qrow;
+          float4 fq = {1.f, 1.f, 1.f, 1.f}, fd = {1.f, 1.f, 1.f, 1.f};       // token-local: unit block factors
+          float bsc = 1.f;
+          if (!TL) {
+            fq = __ldg(reinterpret_cast<const float4*>(p.fac_q + ro / 32));
+            fd = __ldg(reinterpret_cast<const float4*>(p.fac_do + ro / 32));
+          }
+          if (!(FULL && p.dq_scale_rows)) bsc = __ldg(p.dq_scale + (size_t)t.bat * (p.s_q / 128) + qrow / 128);
           if (gi >= 3 && !(ok = mbar_wait(&bars[BB_AEMPTY + sa], (ra - 1) & 1, p.ctl, abortp, 10))) break;
           mbar_arrive_expect_tx(&bars[BB_AFULL + sa], SM::A_TILE + (FP4 ? 1024 : 0));
           tma_load_4d(smem + SM::A + sa * SM::A_TILE, FP4 ? &tm_q4 : &tm_q, &bars[BB_AFULL + sa], 0, head, qrow, t.bat);
           if (FP4)
             bulk_load(smem + SM::SF + 2048 + sa * 1024, p.sfq4 + (((size_t)t.bat * p.h + head) * (p.s_q / 128) + qrow / 128) * 1024,
                       1024, &bars[BB_AFULL + sa]);
-          if (gi >= 2 && !(ok = mbar_wait(&bars[BB_BEMPTY + sb], (rb - 1) & 1, p.ctl, abortp, 10))) break;
-          mbar_arrive_expect_tx(&bars[BB_BFULL + sb], TILE_BYTES + 1024 + (FP4 ? TILE_BYTES : 0));
-          if (FP4) tma_load_4d(smem + SM::Q + sb * TILE_BYTES, &tm_q, &bars[BB_BFULL + sb], 0, head, qrow, t.bat);
-          tma_load_4d(smem + SM::DO + sb * TILE_BYTES, &tm_do, &bars[BB_BFULL + sb], 0, head, qrow, t.bat);
-          bulk_load(smem + SM::VEC + sb * 1024, p.lse_log2 + ro, 512, &bars[BB_BFULL + sb]);
-          bulk_load(smem + SM::VEC + sb * 1024 + 512, p.d_rows + ro, 512, &bars[BB_BFULL + sb]);
+          for (int x = 0; x < 2; ++x) {
+            uint64_t* const full = &bars[BB_BFULL + 2 * sb + x];
+            if (gi >= 2 && !(ok = mbar_wait(&bars[BB_BEMPTY + 2 * sb + x], (rb - 1) & 1, p.ctl, abortp, 10))) break;
+            float* const sc = misc.scal[sb][x];
+            *reinterpret_cast<float4*>(sc) = x == 0 ? make_float4(fq.x, fq.y, fd.x, fd.y) : make_float4(fq.z, fq.w, fd.z, fd.w);
+            sc[4] = bsc;
+            mbar_arrive_expect_tx(full, TILE_BYTES / 2 + SM::VEC_HALF + (FP4 ? TILE_BYTES / 2 : 0));
+            const int half = sb * TILE_BYTES + x * (TILE_BYTES / 2), vec = SM::VEC + (2 * sb + x) * SM::VEC_HALF;
+            bulk_load(smem + vec, p.lse_log2 + ro + 64 * x, 256, full);
+            tma_load_4d(smem + SM::DO + half, &tm_do, full, 0, head, qrow + 64 * x, t.bat);
+            if (FP4) tma_load_4d(smem + SM::Q + half, &tm_q, full, 0, head, qrow + 64 * x, t.bat);
+            bulk_load(smem + vec + 256, p.d_rows + ro + 64 * x, 256, full);
+            if (TL) {
+              bulk_load(smem + vec + 512, p.fac_q + ro + 64 * x, 256, full);
+              bulk_load(smem + vec + 768, p.fac_do + ro + 64 * x, 256, full);
+            }
+          }
+          if (!ok) break;
           if (++m == t.m_lo + t.n_m) { m = t.m_lo; ++head; }
         }
       }
     }
   } else if (warp == 12) {
-    // =================================================================== UMMA issuer
+    // =================================================================== UMMA issuer of the gradient products
     // The whole warp stays converged through the waits and the descriptor arithmetic (warp-uniform values); one elected
-    // lane issues. Descriptors are built once; the loops only add byte offsets.
-    constexpr uint32_t ID_N64 = idesc_f8(128, 64, 0, 0);
+    // lane issues. Descriptors are built once; the loops only add byte offsets. Two warps issue (this one dQ^T, dV, dK; warp 14
+    // S^T, dP^T): alone, one warp's waits and descriptor moves took longer than the products. Each loop exists once, with the
+    // half as a run-time value: the roles' loops share the instruction cache.
     const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
     const uint32_t base = smem_u32(smem);
-    const uint64_t dA0 = FP4 ? smem_desc(base + SM::A, 16, 512, SWZ_64) : smem_desc(base + SM::A, 16, OP_SBO, OP_SWZ),
-                   dQ0 = smem_desc(base + SM::Q, 16, OP_SBO, OP_SWZ), dDO0 = smem_desc(base + SM::DO, 16, OP_SBO, OP_SWZ),
-                   dDS_A = smem_desc(base + SM::DS, 8192, 512, SWZ_64),   // d = 64: dS-hat as A, next M block 8 KB further
-                   dDS0 = smem_desc(base + SM::DS, 16, 512, SWZ_64),
-                   dSF0 = smem_desc(base + SM::SF, 0, 128, SWZ_NONE), dAT0 = smem_desc(base + SM::ATOMS, 0, 128, SWZ_NONE);
-    int gi = 0, sdr = 0;                   // iterations so far; uses of BB_SDR so far
+    const uint64_t dQ0 = smem_desc(base + SM::Q, 16, OP_SBO, OP_SWZ), dDO0 = smem_desc(base + SM::DO, 16, OP_SBO, OP_SWZ),
+                   dDS0 = D == 128 ? smem_desc(base + SM::DS, 16, 512, SWZ_64)
+                                   : smem_desc(base + SM::DS, 8192, 512, SWZ_64),   // d = 64: dS-hat as A, next M block 8 KB further
+                   dAT0 = smem_desc(base + SM::ATOMS, 0, 128, SWZ_NONE), dK0 = smem_desc(base + SM::K, 16, OP_SBO, OP_SWZ);
+    int gi = 0;
     bool ok = true;
     for (int k = 0; ok; ++k) {
       const int L = bwd_item(k, G, cta, p.zigzag);
@@ -368,123 +397,133 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[BB_KV + kb], (k >> 1) & 1, p.ctl, abortp, 20))) break;
       const int n_it = tile_s[kb].n_m * grp;
-      const uint64_t dK_k = smem_desc(base + SM::K + kb * TILE_BYTES, 16, OP_SBO, OP_SWZ),
-                     dV_k = smem_desc(base + SM::V + kb * TILE_BYTES, 16, OP_SBO, OP_SWZ),
-                     dK4 = smem_desc(base + SM::K4 + kb * 8192, 16, 512, SWZ_64);
-      // S^T_x of iteration g. FP4: the scale columns stand in `park` (free tensor memory)
-      auto issue_s = [&](int g, int x, uint32_t park) -> bool {
-        const int st = g % 3;
-        // (the second half finds the stage loaded: the first half's product of the same iteration was issued before)
-        if (x == 0 && !mbar_wait(&bars[BB_AFULL + st], (g / 3) & 1, p.ctl, abortp, 21)) return false;
+      const uint64_t dK_k = desc_adv(dK0, kb * TILE_BYTES);
+      // the first products of an item overwrite dV / dK: the previous item's rows must have left tensor memory (an item without
+      // query tiles issues nothing, but its accumulator hand-over still takes place once)
+      if (k > 0 && !(ok = mbar_wait(&bars[BB_ACCFREE], (k - 1) & 1, p.ctl, abortp, 25))) break;
+#pragma unroll 1
+      for (int t = 0; t < 2 * n_it; ++t) {
+        const int g = gi + (t >> 1), x = t & 1, sa = g % 3, sb = g & 1;
+        // dQ^T_x, dV, dK of iteration g (P-hat and dS-hat of half x stand in the other half's region); dQ^T first: the reduction
+        // warps read it while the rest runs, and dP^T_x of the next iteration takes its columns
+        const uint32_t ro = tm + TC_S + 64 * (1 - x), t_dq = tm + TC_DP + 64 * x;
+        const uint64_t qx = desc_adv(dQ0, (FP4 ? sb : sa) * TILE_BYTES + x * 64 * D), dox = desc_adv(dDO0, sb * TILE_BYTES + x * 64 * D),
+                       at = desc_adv(dAT0, x * SM::ATOM_STRIDE), dsx = desc_adv(dDS0, x * 8192);
+        uint64_t* const b_free = &bars[BB_BEMPTY + 2 * sb + x];
+        if (!(ok = mbar_wait(&bars[BB_DS + x], g & 1, p.ctl, abortp, 24))) break;
         tc_fence_after();
         if (elect_one()) {
-          const uint64_t ax = desc_adv(dA0, st * SM::A_TILE + x * (SM::A_TILE / 2));
-          if (FP4) {
-#pragma unroll
-            for (int kk = 0; kk < 2; ++kk) {
-              tmem_cp_sf_atom(park + 4 * kk, desc_adv(dSF0, kb * 1024 + 512 * kk));
-              tmem_cp_sf_atom(park + 8 + 4 * kk, desc_adv(dSF0, 2048 + st * 1024 + 512 * kk));
-            }
-#pragma unroll
-            for (int kk = 0; kk < 2; ++kk)   // K = 64 elements = 32 bytes per instruction
-              umma_nvf4_ss(tm + TC_S + 64 * x, desc_adv(dK4, 32 * kk), desc_adv(ax, 32 * kk),
-                           idesc_bs(128, 64, 1, 1, 0, 0, 0, 0, 0), park + 4 * kk, park + 8 + 4 * kk + 2 * x, kk > 0);
-          } else {
-#pragma unroll
-            for (int kk = 0; kk < D / 32; ++kk)
-              umma_f8_ss(tm + TC_S + 64 * x, desc_adv(dK_k, 32 * kk), desc_adv(ax, 32 * kk), ID_N64, kk > 0);
-          }
-          tc_commit(&bars[BB_S + x]);
-        }
-        __syncwarp();
-        return true;
-      };
-      // the half's dP^T columns hold its previous dQ^T until the reduction warps have read it (iteration g - 1)
-      auto dq_read = [&](int g, int x) -> bool { return g == 0 || mbar_wait(&bars[BB_DQE + x], (g - 1) & 1, p.ctl, abortp, 22); };
-      auto issue_dp = [&](int g, int x) -> bool {
-        const int st = g & 1;
-        if (x == 0 && !mbar_wait(&bars[BB_BFULL + st], (g >> 1) & 1, p.ctl, abortp, 27)) return false;
-        tc_fence_after();
-        if (elect_one()) {
-          const uint64_t dox = desc_adv(dDO0, st * TILE_BYTES + x * 64 * D);
-#pragma unroll
-          for (int kk = 0; kk < D / 32; ++kk)
-            umma_f8_ss(tm + TC_DP + 64 * x, desc_adv(dV_k, 32 * kk), desc_adv(dox, 32 * kk), ID_N64, kk > 0);
-          tc_commit(&bars[BB_DP + x]);
-        }
-        __syncwarp();
-        return true;
-      };
-      // dQ^T_x, dV, dK of iteration g (P-hat and dS-hat of half x stand in the other half's region); dQ^T first: the reduction
-      // warps read it while the rest runs, and dP^T_x of the next iteration takes its columns
-      auto issue_grads = [&](int g, int x, bool first) -> bool {
-        if (!mbar_wait(&bars[BB_DS + x], g & 1, p.ctl, abortp, 24)) return false;
-        tc_fence_after();
-        if (elect_one()) {
-          const int sa = g % 3, sb = g & 1;
-          const uint32_t ro = tm + TC_S + 64 * (1 - x);
-          const uint64_t qx = desc_adv(dQ0, (FP4 ? sb : sa) * TILE_BYTES + x * 64 * D), dox = desc_adv(dDO0, sb * TILE_BYTES + x * 64 * D);
-          const uint64_t at = desc_adv(dAT0, x * SM::ATOM_STRIDE);
-          const uint32_t accum = first ? 0u : 1u;
           tmem_cp_sf_atom(ro + TO_SFB_DQ, desc_adv(at, 512));
           tmem_cp_sf_atom(ro + TO_SFA_DK, at);
           if (TL) tmem_cp_sf_atom(ro + TO_SFA_P, desc_adv(at, 1024));
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {   // K = 128 keys
             if (D == 128)      // A = K tile (M = head dim), B = dS-hat half (N = 64 queries)
-              umma_mxf8_ss(tm + TC_DP + 64 * x, desc_adv(dK_k, kk * 32 * D), desc_adv(dDS0, x * 8192 + kk * 2048),
-                           idesc_bs(128, 64, 0, 0, 1, 1, 1, kk, kk), ro + TO_SFA_DQ, ro + TO_SFB_DQ, kk > 0);
+              umma_mxf8_ss(t_dq, desc_adv(dK_k, kk * 32 * D), desc_adv(dsx, kk * 2048), idesc_bs(128, 64, 0, 0, 1, 1, 1, kk, kk),
+                           ro + TO_SFA_DQ, ro + TO_SFB_DQ, kk > 0);
             else               // A = dS-hat half (M = 64 queries + 64 unused rows), B = K tile (N = head dim)
-              umma_mxf8_ss(tm + TC_DP + 64 * x, desc_adv(dDS_A, x * 8192 + kk * 2048), desc_adv(dK_k, kk * 32 * D),
-                           idesc_bs(128, 64, 0, 0, 1, 1, 1, kk, kk), ro + TO_SFB_DQ, ro + TO_SFA_DQ, kk > 0);
+              umma_mxf8_ss(t_dq, desc_adv(dsx, kk * 2048), desc_adv(dK_k, kk * 32 * D), idesc_bs(128, 64, 0, 0, 1, 1, 1, kk, kk),
+                           ro + TO_SFB_DQ, ro + TO_SFA_DQ, kk > 0);
           }
           tc_commit(&bars[BB_DQF + x]);
 #pragma unroll
           for (int kk = 0; kk < 2; ++kk)     // K = 64 queries: two instructions of 32
             umma_mxf8_ts(tm + TC_DV, ro + TO_P + 8 * kk, desc_adv(dox, kk * 32 * D),
-                         idesc_bs(128, D, 0, 0, 0, 1, 1, kk, kk), ro + TO_SFA_P, ro + TO_SFB_DO, accum | kk);
+                         idesc_bs(128, D, 0, 0, 0, 1, 1, kk, kk), ro + TO_SFA_P, ro + TO_SFB_DO, t | kk);
 #pragma unroll
           for (int kk = 0; kk < 2; ++kk)
             umma_mxf8_ts(tm + TC_DK, ro + TO_DS + 8 * kk, desc_adv(qx, kk * 32 * D),
-                         idesc_bs(128, D, 0, 0, 0, 1, 1, kk, kk), ro + TO_SFA_DK, ro + TO_SFB_Q, accum | kk);
-          if (x == 1) { tc_commit(&bars[BB_AEMPTY + sa]); tc_commit(&bars[BB_BEMPTY + sb]); }
+                         idesc_bs(128, D, 0, 0, 0, 1, 1, kk, kk), ro + TO_SFA_DK, ro + TO_SFB_Q, t | kk);
+          tc_commit(b_free);
+          if (x == 1) tc_commit(&bars[BB_AEMPTY + sa]);
         }
         __syncwarp();
-        return true;
-      };
-      const uint32_t park0 = tm + TC_DP, park1 = tm + TC_DP + 64;
-      if (n_it > 0) {
-        // the item's first products; they run while the compute warpgroups write the previous item's rows
-        if (!(ok = dq_read(gi, 0) && issue_s(gi, 0, park0) && issue_dp(gi, 0))) break;
-        if (!(ok = dq_read(gi, 1) && issue_s(gi, 1, park1))) break;
-        if (!FP4 && !(ok = issue_dp(gi, 1))) break;
-        if (n_it > 1) {      // S0 of the second iteration: once the first one's scores are in registers
-          if (!(ok = mbar_wait(&bars[BB_SDR], sdr & 1, p.ctl, abortp, 26))) break;
-          ++sdr;
-          if (!(ok = issue_s(gi + 1, 0, park1))) break;
-        }
-        if (FP4 && !(ok = issue_dp(gi, 1))) break;
-      }
-      for (int j = 0; ok && j < n_it; ++j) {
-        const int g = gi + j;
-        // the first products of an item overwrite dV / dK: the previous item's rows must have left tensor memory
-        if (j == 0 && k > 0 && !(ok = mbar_wait(&bars[BB_ACCFREE], (k - 1) & 1, p.ctl, abortp, 25))) break;
-        if (!(ok = issue_grads(g, 0, j == 0))) break;
-        // (P0 and dS0 stood where S1(g) had been: their arrival says that those scores have been read; likewise below)
-        if (j + 1 < n_it) {
-          if (FP4) { if (!(ok = dq_read(g + 1, 0) && issue_s(g + 1, 1, park0) && issue_dp(g + 1, 0))) break; }
-          else if (!(ok = issue_s(g + 1, 1, 0) && dq_read(g + 1, 0) && issue_dp(g + 1, 0))) break;
-        }
-        if (!(ok = issue_grads(g, 1, false))) break;
-        if (FP4 && j + 1 < n_it && !(ok = dq_read(g + 1, 1))) break;
-        if (j + 2 < n_it && !(ok = issue_s(g + 2, 0, park1))) break;
-        if (j + 1 < n_it && !(ok = (FP4 || dq_read(g + 1, 1)) && issue_dp(g + 1, 1))) break;
       }
       if (!ok) break;
-      // an item without query tiles issues nothing, but its accumulator hand-over still takes place once
-      if (n_it == 0 && k > 0 && !(ok = mbar_wait(&bars[BB_ACCFREE], (k - 1) & 1, p.ctl, abortp, 25))) break;
       if (elect_one()) tc_commit(&bars[BB_ACC]);       // every product of the item has completed when this arrives
       __syncwarp();
+      gi += n_it;
+    }
+  } else if (warp == 14) {
+    // =================================================================== UMMA issuer of the score products
+    // Step t of an item (y = t & 1, j = t >> 1) follows the gradient products of (j, y) and issues S^T_{1-y} of iteration
+    // j + 1 + y and dP^T_y of iteration j + 1; steps -3 to -1 are the item's first products, which run while the compute
+    // warpgroups write the previous item's rows.
+    constexpr uint32_t ID_N64 = idesc_f8(128, 64, 0, 0);
+    const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
+    const uint32_t base = smem_u32(smem);
+    const uint64_t dA0 = FP4 ? smem_desc(base + SM::A, 16, 512, SWZ_64) : smem_desc(base + SM::A, 16, OP_SBO, OP_SWZ),
+                   dDO0 = smem_desc(base + SM::DO, 16, OP_SBO, OP_SWZ), dSF0 = smem_desc(base + SM::SF, 0, 128, SWZ_NONE),
+                   dK0 = FP4 ? smem_desc(base + SM::K4, 16, 512, SWZ_64) : smem_desc(base + SM::K, 16, OP_SBO, OP_SWZ),
+                   dV0 = smem_desc(base + SM::V, 16, OP_SBO, OP_SWZ);
+    int gi = 0, sdr = 0;                   // iterations so far; uses of BB_SDR so far
+    bool ok = true;
+    for (int k = 0; ok; ++k) {
+      const int L = bwd_item(k, G, cta, p.zigzag);
+      if (L >= p.n_items) break;
+      const int kb = k & 1;
+      if (!(ok = mbar_wait(&bars[BB_KV + kb], (k >> 1) & 1, p.ctl, abortp, 21))) break;
+      const int n_it = tile_s[kb].n_m * grp;
+      const uint64_t dK_k = desc_adv(dK0, kb * (FP4 ? 8192 : TILE_BYTES)), dV_k = desc_adv(dV0, kb * TILE_BYTES);
+#pragma unroll 1
+      for (int t = -3; t < 2 * n_it - 2; ++t) {
+        const int y = t & 1, j = t >> 1;
+        const bool do_s = j + 1 + y < n_it, do_p = j + 1 >= 0 && j + 1 < n_it;
+        const int gs = gi + j + 1 + y, gp = gi + j + 1, xs = 1 - y;
+        // the half's dP^T columns hold its previous dQ^T until the reduction warps have read it. FP4: the 16 scale columns of S^T
+        // stand in them, too
+        auto dq_read = [&](int g) -> bool { return g == 0 || mbar_wait(&bars[BB_DQE + y], (g - 1) & 1, p.ctl, abortp, 22); };
+        // The region S^T goes to: its last user were the gradient products of (j, y) (their completion also says that the scores
+        // before have been read: the P-hat that took their place waited for that); at an item's start those of the item
+        // before, and for half 0's second tile its own first scores.
+        if (t != -2) {
+          const int gl = t >= 0 ? gi + j : gi - 1;
+          if (t == -1) { if (do_s && !(ok = mbar_wait(&bars[BB_SDR], sdr++ & 1, p.ctl, abortp, 26))) break; }
+          else if (gl >= 0 && !(ok = mbar_wait(&bars[BB_BEMPTY + 2 * (gl & 1) + y], (gl >> 1) & 1, p.ctl, abortp, 28))) break;
+        }
+        if (FP4 && !(ok = dq_read(t == -3 ? gi : gp))) break;
+        if (do_s) {
+          const int st = gs % 3;
+          // (the second half finds the stage loaded: the first half's product of the same iteration was issued before)
+          if (xs == 0 && !(ok = mbar_wait(&bars[BB_AFULL + st], (gs / 3) & 1, p.ctl, abortp, 21))) break;
+          tc_fence_after();
+          const uint64_t ax = desc_adv(dA0, st * SM::A_TILE + xs * (SM::A_TILE / 2));
+          const uint32_t t_s = tm + TC_S + 64 * xs, park = tm + TC_DP + 64 * y;
+          const uint64_t sfk = desc_adv(dSF0, kb * 1024), sfq = desc_adv(dSF0, 2048 + st * 1024);
+          if (elect_one()) {
+            if (FP4) {
+#pragma unroll
+              for (int kk = 0; kk < 2; ++kk) {
+                tmem_cp_sf_atom(park + 4 * kk, desc_adv(sfk, 512 * kk));
+                tmem_cp_sf_atom(park + 8 + 4 * kk, desc_adv(sfq, 512 * kk));
+              }
+#pragma unroll
+              for (int kk = 0; kk < 2; ++kk)   // K = 64 elements = 32 bytes per instruction
+                umma_nvf4_ss(t_s, desc_adv(dK_k, 32 * kk), desc_adv(ax, 32 * kk), idesc_bs(128, 64, 1, 1, 0, 0, 0, 0, 0), park + 4 * kk,
+                             park + 8 + 4 * kk + 2 * xs, kk > 0);
+            } else {
+#pragma unroll
+              for (int kk = 0; kk < D / 32; ++kk) umma_f8_ss(t_s, desc_adv(dK_k, 32 * kk), desc_adv(ax, 32 * kk), ID_N64, kk > 0);
+            }
+            tc_commit(&bars[BB_S + xs]);
+          }
+          __syncwarp();
+        }
+        if (do_p) {
+          const int st = gp & 1;
+          if (!FP4 && !(ok = dq_read(gp))) break;
+          if (!(ok = mbar_wait(&bars[BB_BFULL + 2 * st + y], (gp >> 1) & 1, p.ctl, abortp, 27))) break;
+          tc_fence_after();
+          const uint64_t doy = desc_adv(dDO0, st * TILE_BYTES + y * 64 * D);
+          if (elect_one()) {
+#pragma unroll
+            for (int kk = 0; kk < D / 32; ++kk)
+              umma_f8_ss(tm + TC_DP + 64 * y, desc_adv(dV_k, 32 * kk), desc_adv(doy, 32 * kk), ID_N64, kk > 0);
+            tc_commit(&bars[BB_DP + y]);
+          }
+          __syncwarp();
+        }
+      }
       gi += n_it;
     }
   } else if (warp >= 8 && warp < 12) {
@@ -626,50 +665,33 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       }
       const int vis_from = p.win_r >= 0 ? (krel - T.off - p.win_r) : 0;    // queries in [vis_from, vis_to] see this key
       const int vis_to = min(p.win_l >= 0 ? (krel - T.off + p.win_l) : 0x7FFFFFFF, T.sq - 1);
-      // one iteration's scalars: the half's two 32-query factors of Q and dO, the query tile's pre-scale. Loaded an iteration
-      // ahead: the tensor core's results are waiting when an iteration begins, so nothing else would hide their latency.
-      int head = hkv * grp, m = T.m_lo;
-      float2 fq_n = {1.f, 1.f}, fd_n = {1.f, 1.f};
-      float bsc_n = 1.f;
-      const bool pre_rows = FULL && p.dq_scale_rows != nullptr;
-      auto load_scalars = [&]() {
-        if (!TL) {
-          const size_t o = ((size_t)T.bat * p.h + head) * (p.s_q / 32) + (T.q0 + m * 128) / 32 + 2 * x;
-          fq_n = __ldg(reinterpret_cast<const float2*>(p.fac_q + o));
-          fd_n = __ldg(reinterpret_cast<const float2*>(p.fac_do + o));
-        }
-        if (!pre_rows) bsc_n = __ldg(p.dq_scale + (size_t)T.bat * (p.s_q / 128) + T.q0 / 128 + m);
-      };
-      if (n_it > 0) load_scalars();
+      int m = T.m_lo;
       for (int it = 0; it < n_it; ++it) {
         const int g = gi + it, st = g & 1;
-        const size_t bh_q = (size_t)T.bat * p.h + head;
-        // token-local: the 64 per-query factors of the half (same addresses for every thread: broadcast loads)
-        const float4* fq_vec = reinterpret_cast<const float4*>(p.fac_q + (TL ? bh_q * p.s_q + T.q0 + m * 128 + 64 * x : 0));
-        const float4* fdo_vec = reinterpret_cast<const float4*>(p.fac_do + (TL ? bh_q * p.s_q + T.q0 + m * 128 + 64 * x : 0));
+        const int q_first = m * 128 + 64 * x;                              // document-relative query of column 0
+        const bool full = key_valid && (q_first >= vis_from) && (q_first + 63 <= vis_to);
+        if (++m == T.m_lo + T.n_m) m = T.m_lo;                              // (the next iteration's from here on)
+        if (!(ok = mbar_wait(&bars[BB_BFULL + 2 * st + x], (g >> 1) & 1, p.ctl, abortp, 30))) break;   // row vectors and scalars visible
+        const uint32_t v_lse = smem_u32(smem) + SM::VEC + (2 * st + x) * SM::VEC_HALF, v_dpp = v_lse + 256;
+        [[maybe_unused]] const uint32_t v_fq = v_lse + 512, v_fdo = v_lse + 768;      // token-local: the 64 per-query factors of the half
         // the f16 pre-scale: one power of two per query tile (folded into K's exponent bytes below), or one per query row
         // (folded into the dQ side's B scale bytes, whose lanes are the queries)
-        const float bsc = bsc_n;
+        const float4 sc4 = lds128(smem_u32(misc.scal[st][x]));
+        const float bsc = misc.scal[st][x][4];
         [[maybe_unused]] uint32_t lq0 = 0, lq1 = 0;
-        if (pre_rows) {
-          const float* rp = p.dq_scale_rows + (size_t)T.bat * p.s_q + T.q0 + m * 128 + 64 * x;
+        if (FULL && p.dq_scale_rows) {
+          const float* rp = p.dq_scale_rows + (size_t)T.bat * p.s_q + T.q0 + q_first;
           lq0 = (uint32_t)((int)((__float_as_uint(rp[lane]) >> 23) & 0xFF) - 127);
           lq1 = (uint32_t)((int)((__float_as_uint(rp[32 + lane]) >> 23) & 0xFF) - 127);
         }
         // FP4: the block scales of S were applied by the tensor core; only the softmax scale remains
-        const float c[2] = {FP4 ? p.scale_log2 : fk * fq_n.x, FP4 ? p.scale_log2 : fk * fq_n.y}, b8[2] = {fv8 * fd_n.x, fv8 * fd_n.y};
-        // token-local: fq = fd = 1, i.e. unit scale bytes for the Q and dO operands
-        const uint32_t eq2 = ((__float_as_uint(fq_n.x) >> 23) & 0xFF) | (((__float_as_uint(fq_n.y) >> 23) & 0xFF) << 8);
-        const uint32_t edo2 = ((__float_as_uint(fd_n.x) >> 23) & 0xFF) | (((__float_as_uint(fd_n.y) >> 23) & 0xFF) << 8);
+        const float c[2] = {FP4 ? p.scale_log2 : fk * sc4.x, FP4 ? p.scale_log2 : fk * sc4.y}, b8[2] = {fv8 * sc4.z, fv8 * sc4.w};
+        // token-local: unit scale bytes for the Q and dO operands
+        const uint32_t eq2 = ((__float_as_uint(sc4.x) >> 23) & 0xFF) | (((__float_as_uint(sc4.y) >> 23) & 0xFF) << 8);
+        const uint32_t edo2 = ((__float_as_uint(sc4.z) >> 23) & 0xFF) | (((__float_as_uint(sc4.w) >> 23) & 0xFF) << 8);
         // K's exponent bytes with the power-of-two f16 pre-scale of this query tile folded in (A scale of dQ^T)
         const uint32_t lb = (uint32_t)((int)((__float_as_uint(bsc) >> 23) & 0xFF) - 127) & 0xFF;
         const uint32_t ekb_word = __vadd4(ek_word, lb * 0x01010101u);
-        const int q_first = m * 128 + 64 * x;                              // document-relative query of column 0
-        const bool full = key_valid && (q_first >= vis_from) && (q_first + 63 <= vis_to);
-        if (++m == T.m_lo + T.n_m) { m = T.m_lo; ++head; }                  // (the next iteration's from here on)
-        if (it + 1 < n_it) load_scalars();
-        if (!(ok = mbar_wait(&bars[BB_BFULL + st], (g >> 1) & 1, p.ctl, abortp, 30))) break;   // lse / D'' vectors visible
-        const uint32_t v_lse = smem_u32(smem) + SM::VEC + st * 1024 + 256 * x, v_dpp = v_lse + 512;
 
         // ---- P' = 2^(s c - lse2)
         if (!(ok = mbar_wait(&bars[BB_S + x], g & 1, p.ctl, abortp, 31))) break;
@@ -717,7 +739,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             // t = lse2 - s c (token-local: c = f_K f_Q(query)), two columns per instruction; P' = 2^-t
             uint64_t c01, c23;
             if (TL) {
-              const float4 f4 = __ldg(fq_vec + j4);
+              const float4 f4 = lds128(v_fq + 16 * j4);
               const uint64_t nfk2 = pack2(-fk, -fk);
               c01 = mul2(pack2(f4.x, f4.y), nfk2);
               c23 = mul2(pack2(f4.z, f4.w), nfk2);
@@ -733,7 +755,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             pf[4 * j4 + 3] = ex2_neg(t3);
           }
         }
-        if (!SC && !full) {      // diagonal / tail tiles only
+        if (!SC && __builtin_expect(!full, 0)) {      // diagonal / tail tiles only
 #pragma unroll
           for (int j = 0; j < 64; ++j) {
             const int qi = q_first + j;
@@ -749,7 +771,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             float am = 0.f;
 #pragma unroll
             for (int j4 = 0; j4 < 8; ++j4) {
-              const float4 f4 = __ldg(fdo_vec + qh * 8 + j4);
+              const float4 f4 = lds128(v_fdo + 16 * (qh * 8 + j4));
               const int j = qh * 32 + 4 * j4;
               unpack2(mul2(pack2(pf[j + 0], pf[j + 1]), pack2(f4.x, f4.y)), t[4 * j4 + 0], t[4 * j4 + 1]);
               unpack2(mul2(pack2(pf[j + 2], pf[j + 3]), pack2(f4.z, f4.w)), t[4 * j4 + 2], t[4 * j4 + 3]);
@@ -801,8 +823,8 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             const int j = qh * 32 + 4 * j4;
             if (TL) {
               // b = f_V(key) f_dO(query) per column; the dK side's maximum carries f_Q(query)
-              const float4 f4 = __ldg(fdo_vec + qh * 8 + j4);
-              const float4 q4 = __ldg(fq_vec + qh * 8 + j4);
+              const float4 f4 = lds128(v_fdo + 16 * (qh * 8 + j4));
+              const float4 q4 = lds128(v_fq + 16 * (qh * 8 + j4));
               const uint64_t fv2 = pack2(fv8, fv8);
               const uint64_t u01 = fma2(pack2(__uint_as_float(pv[j + 0]), __uint_as_float(pv[j + 1])),
                                         mul2(pack2(f4.x, f4.y), fv2), pack2(d4.x, d4.y));
@@ -827,7 +849,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           }
           ebyte[qh] = exp448(warp_max_abs_f32(am));                        // 448 * 2^(e-127) >= amax
         }
-        if (!full) {      // diagonal / tail tiles only
+        if (__builtin_expect(!full, 0)) {      // diagonal / tail tiles only
           // masked entries hold P' = 0, but their dP^T or D'' may come from rows outside the document (padding or whatever
           // the buffer held: possibly Inf / NaN), and 0 * NaN is NaN: select again after the multiply. (The maxima above
           // ignore NaN, so the block exponents are those of the visible entries.)
@@ -854,7 +876,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             const uint64_t inv2 = pack2(inv, inv);
             float a0, a1, a2, a3;
             if (TL) {
-              const float4 f4 = __ldg(fq_vec + qh * 8 + w);      // f_Q(query) 2^(127 - e): powers of two, exact, in range
+              const float4 f4 = lds128(v_fq + 16 * (qh * 8 + w));      // f_Q(query) 2^(127 - e): powers of two, exact, in range
               unpack2(mul2(pack2(pf[j0], pf[j0 + 1]), mul2(pack2(f4.x, f4.y), inv2)), a0, a1);
               unpack2(mul2(pack2(pf[j0 + 2], pf[j0 + 3]), mul2(pack2(f4.z, f4.w), inv2)), a2, a3);
               dsw[qh * 8 + w] = cvt_e4m3x4(a0, a1, a2, a3);
@@ -1072,10 +1094,11 @@ extern "C" int fl_bwd(const fl_attn_args* a, void* stream) {
   if (a->seqused_k && a->doc_start) return FL_ERR_UNSUPPORTED;      // documents carry their own lengths
   CUtensorMap mq, mk, mv, mdo, macc, mq4, mk4, mdk, mdv;
   int rc;
-  if ((rc = make_rows_map(&mq, a->q_codes, a->b, a->s_q, a->h, a->d, 128))) return rc;
+  // (boxes of 64 query rows where a half tile is loaded at a time)
+  if ((rc = make_rows_map(&mq, a->q_codes, a->b, a->s_q, a->h, a->d, fp4 ? 64 : 128))) return rc;
   if ((rc = make_rows_map(&mk, a->k_codes, a->b, a->s_k, a->h_kv, a->d, 128))) return rc;
   if ((rc = make_rows_map(&mv, a->v_codes, a->b, a->s_k, a->h_kv, a->d, 128))) return rc;
-  if ((rc = make_rows_map(&mdo, a->do_codes, a->b, a->s_q, a->h, a->d, 128))) return rc;
+  if ((rc = make_rows_map(&mdo, a->do_codes, a->b, a->s_q, a->h, a->d, 64))) return rc;
   if (a->d == 128) rc = make_acc_t_map_16(&macc, a->dq_acc, a->b, a->h, a->d, a->s_q);
   else rc = make_acc_map_16(&macc, a->dq_acc, a->b, a->h, a->s_q, a->d, 64);       // (b, h, s, d): boxes of 64 query rows
   if (rc) return rc;
@@ -1124,7 +1147,8 @@ extern "C" int fl_bwd(const fl_attn_args* a, void* stream) {
   p.n_items = (int)n_items;
   p.zigzag = (p.causal && !a->doc_start) ? 1 : 0;
   const int grid = (int)(n_items < sm_count() ? n_items : sm_count());     // one persistent CTA per SM
-  const int smem = a->d == 64 ? BwdSmem<64, false>::BYTES : fp4 ? BwdSmem<128, true>::BYTES : BwdSmem<128, false>::BYTES;
+  const int smem = a->d == 64 ? BwdSmem<64, false, false>::BYTES : fp4 ? BwdSmem<128, true, false>::BYTES
+                   : tl ? BwdSmem<128, false, true>::BYTES : BwdSmem<128, false, false>::BYTES;
   auto launch = [&](auto kern) -> int {
     if (int e = set_smem(kern, smem, "fl_bwd: cudaFuncSetAttribute")) return e;
     kern<<<grid, 512, smem, (cudaStream_t)stream>>>(mq, mk, mv, mdo, macc, mq4, mk4, mdk, mdv, p);

@@ -73,7 +73,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // Bounded wait. `abort` is a CTA-shared int; `site` identifies the wait for the status word.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const DevCtl& ctl, volatile int* abort,
                                           int site) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (__builtin_expect(mbar_try_wait(bar, parity), 1)) return true;
   long long t0 = clock64();
   uint32_t spins = 0;
   while (!mbar_try_wait(bar, parity)) {
@@ -298,7 +298,10 @@ __host__ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t l
 // A descriptor whose start address is `bytes` further (bytes % 16 == 0; the 14-bit address field must not wrap, which
 // holds for offsets inside one CTA's shared memory window below 256 KB). The UMMA issuer is a single thread whose own
 // instruction latency bounds the tensor pipe's issue rate, so descriptors are built once and only advanced in loops.
-__host__ __device__ __forceinline__ uint64_t desc_adv(uint64_t d, uint32_t bytes) { return d + (uint64_t)(bytes >> 4); }
+// (a 32-bit addition: the upper word stays as it is)
+__host__ __device__ __forceinline__ uint64_t desc_adv(uint64_t d, uint32_t bytes) {
+  return (d & 0xFFFFFFFF00000000ull) | (uint32_t)((uint32_t)d + (bytes >> 4));
+}
 // Instruction descriptor, kind::f8f6f4 with E4M3 x E4M3 -> F32.
 __host__ __device__ constexpr uint32_t idesc_f8(int M, int N, int a_mn_major, int b_mn_major) {
   return (1u << 4) | ((uint32_t)a_mn_major << 15) | ((uint32_t)b_mn_major << 16) | ((uint32_t)(N >> 3) << 17) |
