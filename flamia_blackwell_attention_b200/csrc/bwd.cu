@@ -355,6 +355,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           if (FP4)
             bulk_load(smem + SM::SF + 2048 + sa * 1024, p.sfq4 + (((size_t)t.bat * p.h + head) * (p.s_q / 128) + qrow / 128) * 1024,
                       1024, &bars[BB_AFULL + sa]);
+#pragma unroll 1
           for (int x = 0; x < 2; ++x) {
             uint64_t* const full = &bars[BB_BFULL + 2 * sb + x];
             if (gi >= 2 && !(ok = mbar_wait(&bars[BB_BEMPTY + 2 * sb + x], (rb - 1) & 1, p.ctl, abortp, 10))) break;
@@ -540,9 +541,11 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       if (!(ok = mbar_wait(&bars[BB_KV + kb], (k >> 1) & 1, p.ctl, abortp, 43))) break;
       const BTile T = tile_s[kb];
       const int n_it = T.n_m * grp;
+      int head = T.hkv * grp, m = T.m_lo;
+#pragma unroll 1
       for (int t = 0; t < 2 * n_it; ++t, ++gt) {
         const int it = t >> 1, y = t & 1, g = gi + it;
-        const int head = T.hkv * grp + it / T.n_m, m = T.m_lo + it % T.n_m;
+        if (t > 0 && y == 0 && ++m == T.m_lo + T.n_m) { m = T.m_lo; ++head; }
         // the staging buffer of this half was last read by the reduction of step gt - 2
         if (tid == 256) tma_store_wait_read<1>();
         mbar_arrive_warp(&bars[BB_R1]);
@@ -553,7 +556,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // d = 128: thread = head-dim row of dQ^T, 64 query columns. d = 64: thread = query row (the first 64 lanes; the
         // other two warps hold the product's unused rows), 64 head-dim columns. Either way 64 f16 = one 128-byte row.
         if (D == 128 || warp < 10) {
-#pragma unroll
+#pragma unroll 1
           for (int cc = 0; cc < 2; ++cc) {
             uint32_t v[32];
             FL_TMEM_LD_32(lane_base + TC_DP + 64 * y + 32 * cc, v);
@@ -670,6 +673,16 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const int g = gi + it, st = g & 1;
         const int q_first = m * 128 + 64 * x;                              // document-relative query of column 0
         const bool full = key_valid && (q_first >= vis_from) && (q_first + 63 <= vis_to);
+        // which of the half's queries see this key, a bit each (tested bit by bit the mask takes a third of the instructions that
+        // comparisons take, and they stand in the loop whether they run or not)
+        uint32_t see[2];
+        {
+          const int lo = max(vis_from - q_first, 0), n = key_valid ? max(min(vis_to - q_first + 1, 64) - lo, 0) : 0;
+          const uint64_t b = lo < 64 && n > 0 ? (~0ull >> (64 - n)) << lo : 0ull;
+          see[0] = (uint32_t)b;
+          see[1] = (uint32_t)(b >> 32);
+        }
+        auto visible = [&](int j) { return (see[j >> 5] & (1u << (j & 31))) != 0; };
         if (++m == T.m_lo + T.n_m) m = T.m_lo;                              // (the next iteration's from here on)
         if (!(ok = mbar_wait(&bars[BB_BFULL + 2 * st + x], (g >> 1) & 1, p.ctl, abortp, 30))) break;   // row vectors and scalars visible
         const uint32_t v_lse = smem_u32(smem) + SM::VEC + (2 * st + x) * SM::VEC_HALF, v_dpp = v_lse + 256;
@@ -722,10 +735,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
               const float th = tanh_fast(__uint_as_float(pv[4 * j4 + e]) * (cc * p.cap_b));
               pp[e] = ex2(fmaf(p.cap_a, th, -l[e]));
               df[e] = fmaf(-th, th, 1.0f);
-              if (!full) {
-                const int qi = q_first + 4 * j4 + e;
-                pp[e] = (key_valid && qi >= vis_from && qi <= vis_to) ? pp[e] : 0.f;
-              }
+              if (!full) pp[e] = visible(4 * j4 + e) ? pp[e] : 0.f;
             }
             pw[j4] = cvt_e4m3x4(pp[0], pp[1], pp[2], pp[3]);
 #pragma unroll
@@ -755,12 +765,9 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             pf[4 * j4 + 3] = ex2_neg(t3);
           }
         }
-        if (!SC && __builtin_expect(!full, 0)) {      // diagonal / tail tiles only
+        if (!SC && !full) {      // diagonal / tail tiles only
 #pragma unroll
-          for (int j = 0; j < 64; ++j) {
-            const int qi = q_first + j;
-            pf[j] = (key_valid && qi >= vis_from && qi <= vis_to) ? pf[j] : 0.f;
-          }
+          for (int j = 0; j < 64; ++j) pf[j] = visible(j) ? pf[j] : 0.f;
         }
         if (TL) {
           // block-scaled P-hat carrying f_dO(query): one exponent per (this key row, 32 queries)
@@ -849,15 +856,12 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           }
           ebyte[qh] = exp448(warp_max_abs_f32(am));                        // 448 * 2^(e-127) >= amax
         }
-        if (__builtin_expect(!full, 0)) {      // diagonal / tail tiles only
+        if (!full) {      // diagonal / tail tiles only
           // masked entries hold P' = 0, but their dP^T or D'' may come from rows outside the document (padding or whatever
           // the buffer held: possibly Inf / NaN), and 0 * NaN is NaN: select again after the multiply. (The maxima above
           // ignore NaN, so the block exponents are those of the visible entries.)
 #pragma unroll
-          for (int j = 0; j < 64; ++j) {
-            const int qi = q_first + j;
-            pf[j] = (key_valid && qi >= vis_from && qi <= vis_to) ? pf[j] : 0.f;
-          }
+          for (int j = 0; j < 64; ++j) pf[j] = visible(j) ? pf[j] : 0.f;
         }
         // dK's A scales: row = key; bytes = the half's two query blocks
         sts32(at_row, ebyte[0] | (ebyte[1] << 8));
@@ -945,48 +949,43 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // dV carries 2^8 (P'), dK the softmax scale (and the mantissa of a Q factor that is no power of two)
         const float mult = (x == 0) ? 0.00390625f : p.softmax_scale * ((FULL && p.dk_mult) ? p.dk_mult[bh_k] : 1.0f);
         const float mk = key_valid ? mult : 0.f;       // rows past the end of the document store zeros
-        uint32_t v[D];
-        if (n_it > 0) {                  // (CTA-uniform: the tensor-memory loads are warp-collective)
+        // dK of rotated operands: (y H / sqrt(128)) * signs. The butterfly runs in small loops over tensor memory (levels 1 .. 16
+        // inside blocks of 32 columns, then levels 32 and 64 across them on eight columns of each block at a time): unrolled over
+        // a row of registers it was 900 instructions, which pushed the main loops out of the instruction cache at every item.
+        const bool rot = D == 128 && x == 1 && p.had_dk;
+        if (rot && n_it > 0) {
+#pragma unroll 1
+          for (int cc = 0; cc < 4; ++cc) {
+            uint32_t v[32];
+            FL_TMEM_LD_32(t_acc + 32 * cc, v);
+            tc_wait_ld();
+            uint64_t Y[16];
 #pragma unroll
-          for (int cc = 0; cc < D / 32; ++cc) FL_TMEM_LD_32(t_acc + 32 * cc, (v + 32 * cc));   // all loads in flight, one wait
-          tc_wait_ld();
-        } else {                         // no query tile saw this key tile
+            for (int i = 0; i < 16; ++i) {            // level 1: the two halves of a pair
+              const float a = __uint_as_float(v[2 * i]), b2 = __uint_as_float(v[2 * i + 1]);
+              Y[i] = pack2(a + b2, a - b2);
+            }
 #pragma unroll
-          for (int e = 0; e < D; ++e) v[e] = 0;
-        }
-        // the accumulators are in registers: the next item's products may overwrite them
-        tc_fence_before();
-        mbar_arrive_warp(&bars[BB_ACCFREE]);
-        // pairs of neighbouring columns in one 64-bit register: every step below is one instruction per pair
-        uint64_t Y[D / 2];
-        if (D == 128 && x == 1 && p.had_dk) {       // dK of rotated operands: (y H / sqrt(128)) * signs
+            for (int hs = 1; hs < 16; hs <<= 1) {     // levels 2 .. 16: whole pairs
 #pragma unroll
-          for (int i = 0; i < D / 2; ++i) {         // butterfly level 1: the two halves of a pair
-            const float a = __uint_as_float(v[2 * i]), b2 = __uint_as_float(v[2 * i + 1]);
-            Y[i] = pack2(a + b2, a - b2);
-          }
-#pragma unroll
-          for (int hs = 1; hs < D / 2; hs <<= 1) {  // levels 2 .. D / 2: whole pairs
-#pragma unroll
-            for (int i = 0; i < D / 2; ++i) {
-              if ((i & hs) == 0) {
-                const uint64_t a = Y[i], b2 = Y[i + hs];
-                Y[i] = add2(a, b2);
-                Y[i + hs] = sub2(a, b2);
+              for (int i = 0; i < 16; ++i) {
+                if ((i & hs) == 0) {
+                  const uint64_t a = Y[i], b2 = Y[i + hs];
+                  Y[i] = add2(a, b2);
+                  Y[i + hs] = sub2(a, b2);
+                }
               }
             }
-          }
-          constexpr uint32_t NEG[4] = {0x10D2E03Eu, 0xE0D9F0E2u, 0x45809F07u, 0x75954FEDu};
-          const float cp = 0.08838834764831845f * mk, cn = -cp;
 #pragma unroll
-          for (int i = 0; i < D / 2; ++i) {
-            const bool n0 = (NEG[(2 * i) >> 5] >> ((2 * i) & 31)) & 1, n1 = (NEG[(2 * i + 1) >> 5] >> ((2 * i + 1) & 31)) & 1;
-            Y[i] = mul2(Y[i], pack2(n0 ? cn : cp, n1 ? cn : cp));
+            for (int i = 0; i < 16; ++i) {
+              float a, b2;
+              unpack2(Y[i], a, b2);
+              v[2 * i] = __float_as_uint(a);
+              v[2 * i + 1] = __float_as_uint(b2);
+            }
+            FL_TMEM_ST_32(t_acc + 32 * cc, v);
           }
-        } else {
-          const uint64_t mk2 = pack2(mk, mk);
-#pragma unroll
-          for (int i = 0; i < D / 2; ++i) Y[i] = mul2(pack2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), mk2);
+          tc_wait_st();
         }
         // rows -> shared memory (boxes of 64 elements, 128 B swizzle) -> one TMA store per box: a thread's own row
         // written straight to global memory costs 32 separate 128-byte lines per warp instruction. At d = 128 the first
@@ -1013,42 +1012,81 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         }
         const bool by_rows = FULL && p.slot_src && out_n < 128;   // (CTA-uniform)
         uint16_t* out_base = reinterpret_cast<uint16_t*>(x == 0 ? p.dv : p.dk);
+        const uint32_t srow0 = smem_u32(stage0) + r * 128, srow1 = smem_u32(stage1) + r * 128;
+        const float cs = rot ? 0.08838834764831845f * mk : mk;
+        constexpr int NB = D / 32, PASSES = EPI2 ? 1 : D / 64;      // 32-column blocks; a pass writes the boxes that fit
+#pragma unroll 1
+        for (int pass = 0; pass < PASSES; ++pass) {
+#pragma unroll 1
+          for (int c8 = 0; c8 < 4; ++c8) {           // eight columns of every block
+            uint32_t v[NB][8];
 #pragma unroll
-        for (int pass = 0; pass < D / 64; ++pass) {
-          uint8_t* stage = pass == 0 ? stage0 : stage1;
-          const uint32_t srow = smem_u32(stage) + r * 128;
+            for (int b2 = 0; b2 < NB; ++b2) {
+              if (n_it > 0) FL_TMEM_LD_8(t_acc + 32 * b2 + 8 * c8, v[b2]);     // (CTA-uniform: the loads are warp-collective)
+              else {
 #pragma unroll
-          for (int c8 = 0; c8 < 8; ++c8) {
-            uint32_t w[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              float a, b2;
-              unpack2(Y[32 * pass + 4 * c8 + e], a, b2);
-              if (p.out_f16) {
-                __half2 hh = __floats2half2_rn(a, b2);
-                w[e] = *reinterpret_cast<uint32_t*>(&hh);
-              } else {
-                w[e] = pack_bf16x2(a, b2);
+                for (int e = 0; e < 8; ++e) v[b2][e] = 0;              // no query tile saw this key tile
               }
             }
-            if (by_rows) {
-              if (r < out_n && 64 * pass + 8 * c8 < p.d_out)
-                *reinterpret_cast<uint4*>(out_base + ((size_t)(out_row + r) * p.h_kv + hkv) * p.d_out + 64 * pass + 8 * c8) =
-                    make_uint4(w[0], w[1], w[2], w[3]);
-            } else {
-              sts128(srow + ((c8 ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+            tc_wait_ld();
+            if (c8 == 3 && pass + 1 == PASSES) {     // the accumulators are in registers: the next item's products may overwrite them
+              tc_fence_before();
+              mbar_arrive_warp(&bars[BB_ACCFREE]);
+            }
+            uint64_t Y[NB][4];
+#pragma unroll
+            for (int b2 = 0; b2 < NB; ++b2)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) Y[b2][e] = pack2(__uint_as_float(v[b2][2 * e]), __uint_as_float(v[b2][2 * e + 1]));
+            if (D == 128 && rot) {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const uint64_t a0 = add2(Y[0][e], Y[1][e]), a1 = sub2(Y[0][e], Y[1][e]), a2 = add2(Y[NB - 2][e], Y[NB - 1][e]),
+                               a3 = sub2(Y[NB - 2][e], Y[NB - 1][e]);
+                Y[0][e] = add2(a0, a2);
+                Y[1][e] = add2(a1, a3);
+                Y[NB - 2][e] = sub2(a0, a2);
+                Y[NB - 1][e] = sub2(a1, a3);
+              }
+            }
+#pragma unroll
+            for (int b2 = 0; b2 < NB; ++b2) {
+              if (!EPI2 && (b2 >> 1) != pass) continue;
+              constexpr uint32_t NEG[4] = {0x10D2E03Eu, 0xE0D9F0E2u, 0x45809F07u, 0x75954FEDu};
+              const uint32_t neg = rot ? NEG[b2 & 3] >> (8 * c8) : 0u;
+              uint32_t w[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float c0 = __uint_as_float(__float_as_uint(cs) ^ ((neg << (31 - 2 * e)) & 0x80000000u)),
+                            c1 = __uint_as_float(__float_as_uint(cs) ^ ((neg << (30 - 2 * e)) & 0x80000000u));
+                float a, b3;
+                unpack2(mul2(Y[b2][e], pack2(c0, c1)), a, b3);
+                if (p.out_f16) {
+                  __half2 hh = __floats2half2_rn(a, b3);
+                  w[e] = *reinterpret_cast<uint32_t*>(&hh);
+                } else {
+                  w[e] = pack_bf16x2(a, b3);
+                }
+              }
+              const int ch = 4 * b2 + c8;            // 16-byte chunk of the row
+              if (by_rows) {
+                if (r < out_n && 8 * ch < p.d_out)
+                  *reinterpret_cast<uint4*>(out_base + ((size_t)(out_row + r) * p.h_kv + hkv) * p.d_out + 8 * ch) =
+                      make_uint4(w[0], w[1], w[2], w[3]);
+              } else {
+                sts128((b2 < 2 ? srow0 : srow1) + (((ch & 7) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+              }
             }
           }
           if (by_rows) continue;
-          const bool last = pass + 1 == D / 64;
-          if (EPI2 && !last) continue;                    // both boxes are announced together
+          const bool last = pass + 1 == PASSES;
           fence_proxy_async();
           mbar_arrive_warp(&bars[BB_EPI + x]);            // the warpgroup's four warps have written their rows
           if (!(ok = mbar_wait(&bars[BB_EPI + x], epi & 1, p.ctl, abortp, 38))) break;
           ++epi;
           if (r == 0 && out_n == 128) {
-            if (EPI2) tma_store_4d(tm_out, stage0, 0, hkv, out_row, T.bat);
-            tma_store_4d(tm_out, stage, 64 * pass, hkv, out_row, T.bat);
+            tma_store_4d(tm_out, stage0, 64 * pass, hkv, out_row, T.bat);
+            if (EPI2) tma_store_4d(tm_out, stage1, 64, hkv, out_row, T.bat);
             tma_store_commit();
             if (!last) tma_store_wait_read<0>();          // the one buffer is written again by the next pass
           }
@@ -1137,8 +1175,7 @@ extern "C" int fl_bwd(const fl_attn_args* a, void* stream) {
   p.win_r = p.causal ? 0 : a->window_right_p1 - 1;
   p.out_f16 = (a->flags & FL_A_OUT_F16) ? 1 : 0;
   p.had_dk = (a->flags & FL_A_HAD_DK) ? 1 : 0;
-  p.ctl.status = a->status;
-  p.ctl.wait_cycles = a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles;
+  p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);
   const int ntile = a->doc_start ? (a->s_k / 128 + a->n_docs) : a->s_k / 128;
   const int nb = a->doc_start ? 1 : a->b;
   p.n_tile = ntile;

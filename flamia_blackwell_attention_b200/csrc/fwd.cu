@@ -729,8 +729,7 @@ extern "C" int fl_fwd(const fl_attn_args* a, void* stream) {
   p.win_l = a->window_left_p1 - 1;
   p.win_r = p.causal ? 0 : a->window_right_p1 - 1;
   p.out_f16 = (a->flags & FL_A_OUT_F16) ? 1 : 0;
-  p.ctl.status = a->status;
-  p.ctl.wait_cycles = a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles;
+  p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);
   // packed documents: at most one extra 256-row block per document beyond total / 256
   const int nblk = a->doc_start ? (a->s_q / 256 + a->n_docs + 1) : (a->s_q + 255) / 256;
   const int nb = a->doc_start ? 1 : a->b;

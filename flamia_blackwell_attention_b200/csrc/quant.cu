@@ -880,8 +880,7 @@ static int quant_rows(const fl_quant_args* const* args, int n, cudaStream_t st) 
   p.n_ops = n; p.n_tiles = (int)tiles;
   p.slot_src = a->slot_src; p.slot_rows = a->slot_rows;
   p.in_f16 = a->in_f16;
-  p.ctl.status = a->status;
-  p.ctl.wait_cycles = a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles;
+  p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);
   int rc;
   if (a->d == 64) rc = launch_quant_rows<0, 64>(maps, p, st);
   else if (mode == 6) rc = launch_quant_rows<6, 128>(maps, p, st);
@@ -916,8 +915,7 @@ extern "C" int fl_quant_blocks(const fl_quant_args* a, void* stream) {
   p.token_local = (a->flags & FL_Q_TOKEN_LOCAL) ? 1 : 0;
   p.in_f16 = a->in_f16;
   p.lse_shift = a->lse_shift; p.d_multiplier = a->d_multiplier;
-  p.ctl.status = a->status;
-  p.ctl.wait_cycles = a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles;
+  p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);
   CUtensorMap mx, mo;
   int rc;
   if ((rc = make_rows_map_16(&mx, a->x, a->b, packed ? a->src_rows : a->s, a->h, d_src, 128))) return rc;

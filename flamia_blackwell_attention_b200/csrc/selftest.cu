@@ -222,8 +222,7 @@ extern "C" int fl_selftest_mma(int32_t which, const uint8_t* a, const uint8_t* b
   }
   SelfTestParams p;
   p.a = a; p.b = b; p.sfa = sfa; p.sfb = sfb; p.d = d; p.which = which;
-  p.ctl.status = status;
-  p.ctl.wait_cycles = wait_cycles > 0 ? wait_cycles : kDefaultWaitCycles;
+  p.ctl = dev_ctl(status, wait_cycles > 0 ? wait_cycles : kDefaultWaitCycles);
   const int smem = 32768 + 2048 + 1024;
   if (cudaFuncSetAttribute(selftest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return FL_ERR_CUDA;

@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(128) dq_post_t128_kernel(const __grid_constant
   if (head_mult) mult *= head_mult[(size_t)bat * h + head];
   const float sc = (per_row ? post[(size_t)bat * s + t0 + tid] : post[(size_t)bat * (s / 128) + tile]) * mult;   // thread = token
   __syncthreads();
-  const DevCtl ctl = {nullptr, kDefaultWaitCycles};
+  const DevCtl ctl = dev_ctl(nullptr, kDefaultWaitCycles);
   bool ok = mbar_wait(&bar, 0, ctl, &abort_s, 60);
   ok = __syncthreads_and(ok ? 1 : 0) != 0;
   if (ok) {
