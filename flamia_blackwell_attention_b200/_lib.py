@@ -61,6 +61,9 @@ EXPORTS = {
     "fl_dq_post_packed": (i32, [vp, vp, f32, vp, i32, i32, i32, i32, i32, vp, vp, vp]),
     "fl_dq_prescale_rows": (i32, [vp, vp, vp, i32, i32, f32, vp, vp, vp]),
     "fl_doc_tables": (i32, [vp, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp]),
+    "fl_doc_work": (i32, [vp, vp, i32, i32, i32, i32, i32, i32, vp, vp, vp]),
+    "fl_fwd_work": (i32, [C.POINTER(AttnArgs), vp, vp]),
+    "fl_bwd_work": (i32, [C.POINTER(AttnArgs), vp, vp]),
     "fl_unpack_lse": (i32, [vp, vp, vp, i32, i32, i32, i32, vp, vp]),
     "fl_pack_rows": (i32, [vp, vp, vp, i32, i32, vp]),
     "fl_unpack_rows": (i32, [vp, vp, vp, i32, i32, vp]),

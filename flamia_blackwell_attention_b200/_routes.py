@@ -125,6 +125,7 @@ def state_spec(plan, n_docs=0, dtype=torch.bfloat16, capacity=None):
         spec += [((b,), i32)]
     if docs:
         spec += [((n,), i32), ((n,), i32)] + ([] if sh.aligned_varlen else [((cap,), i32), ((cap // 128,), i32), ((cap // 128,), i32)])
+        spec += [((4 + 9 * (cap // 128),), i32)]                  # the kernels' work lists
     return spec
 
 

@@ -86,6 +86,10 @@ struct BwdParams {
   int win_l, win_r;      // sliding window sides, -1 = unlimited (causal: the right side is 0)
   int out_f16;
   int had_dk;
+  const int4* work;      // documents: the backward entries of fl_doc_work's list, or null
+  const int4* work_head;
+  FastDiv div_item, div_h;   // items per (causal: key tile; otherwise: kv head), kv heads
+  int grp;               // query heads per kv head
   int n_items;           // work items: key tiles x kv heads x batch rows (documents: tile slots x kv heads)
   int n_tile;            // key tiles per batch row (documents: tile slots of the packed buffer)
   int zigzag;            // deal the items out in zigzag rounds (causal: they are ordered longest first)
@@ -151,23 +155,28 @@ __device__ __forceinline__ int bwd_item(int k, int G, int c, int zigzag) {
 // Work item L -> its key tile. Causal: tiles slowest, so that the item index orders the items longest first (a key tile
 // near the start of the sequence is seen by the most query tiles). Otherwise tiles fastest: the CTAs that run at the same
 // time work on one head and share its Q / dO tiles in L2.
+template <bool DOCS>
 __device__ __forceinline__ void bwd_decode(const BwdParams& p, int L, BTile& t) {
-  if (p.doc_start == nullptr) {
-    int tile, rem;
-    if (p.causal) { tile = L / (p.h_kv * p.b); rem = L % (p.h_kv * p.b); }
-    else { tile = L % p.n_tile; rem = L / p.n_tile; }
-    t.hkv = rem % p.h_kv; t.bat = rem / p.h_kv;
+  if (!DOCS || p.doc_start == nullptr) {
+    const int q = p.div_item.div(L), rq = L - q * p.div_item.d;
+    const int tile = p.causal ? q : rq, rem = p.causal ? rq : q;
+    t.bat = p.div_h.div(rem); t.hkv = rem - t.bat * p.h_kv;
     t.k0 = tile * 128; t.nk = min(128, p.s_k - t.k0); t.krel = t.k0; t.q0 = 0; t.sq = p.s_q; t.off = p.s_k - p.s_q;
     t.nv = p.seqused_k ? min(t.nk, p.seqused_k[t.bat] - t.k0) : t.nk;
   } else {
     // documents sit at 128-aligned starts of one packed batch entry; tile slot x -> (document, key tile of it)
-    int x = L / p.h_kv, dsel = -1, len = 0, st = 0;
-    t.hkv = L % p.h_kv;
-    for (int dI = 0; dI < p.n_docs; ++dI) {
-      doc_entry(p.doc_start, p.doc_len, dI, p.s_k, p.ctl.status, st, len);
-      const int nb = (len + 127) / 128;
-      if (x < nb) { dsel = dI; break; }
-      x -= nb;
+    int x = p.div_h.div(L), dsel = -1, len = 0, st = 0;
+    t.hkv = L - x * p.h_kv;
+    if (p.work) {          // longest first; checked when the list was made
+      const int4 e = __ldg(p.work + x);
+      st = e.x; len = e.y; x = e.z; dsel = 0;
+    } else {
+      for (int dI = 0; dI < p.n_docs; ++dI) {
+        doc_entry(p.doc_start, p.doc_len, dI, p.s_k, p.ctl.status, st, len);
+        const int nb = (len + 127) / 128;
+        if (x < nb) { dsel = dI; break; }
+        x -= nb;
+      }
     }
     if (dsel < 0) { t.nk = 0; t.bat = 0; t.k0 = 0; t.krel = 0; t.q0 = 0; t.sq = 0; t.off = 0; }
     else { t.bat = 0; t.k0 = st + x * 128; t.nk = min(128, len - x * 128); t.krel = x * 128; t.q0 = st; t.sq = len; t.off = 0; }
@@ -266,7 +275,8 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   // (the warp index through a shuffle: the compiler then knows that it is the same in all lanes)
   const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
   const int G = gridDim.x, cta = blockIdx.x;
-  const int grp = p.h / p.h_kv;
+  const int grp = p.grp;
+  const int n_items = FULL && p.work ? __ldg(p.work_head).y * p.h_kv : p.n_items;
 
   if (tid == 13 * 32) {
     misc.abort = 0;
@@ -313,13 +323,13 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       bool ok = true;
       for (int k = 0; ok; ++k) {
         const int L = bwd_item(k, G, cta, p.zigzag);
-        if (L >= p.n_items) break;
+        if (L >= n_items) break;
         const int kb = k & 1;
         // the buffers of item k - 2 (and its slot of tile_s) are free once both compute warpgroups have written its
         // gradient rows out of them
         if (k >= 2 && !(ok = mbar_wait(&bars[BB_KVE + kb], ((k >> 1) - 1) & 1, p.ctl, abortp, 11))) break;
         BTile t;
-        bwd_decode(p, L, t);
+        bwd_decode<FULL>(p, L, t);
         tile_s[kb] = t;
         if (t.nk > 0) {
           mbar_arrive_expect_tx(&bars[BB_KV + kb], 2 * TILE_BYTES + (FP4 ? 8192 + 1024 : 0));
@@ -394,7 +404,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     bool ok = true;
     for (int k = 0; ok; ++k) {
       const int L = bwd_item(k, G, cta, p.zigzag);
-      if (L >= p.n_items) break;
+      if (L >= n_items) break;
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[BB_KV + kb], (k >> 1) & 1, p.ctl, abortp, 20))) break;
       const int n_it = tile_s[kb].n_m * grp;
@@ -461,7 +471,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     bool ok = true;
     for (int k = 0; ok; ++k) {
       const int L = bwd_item(k, G, cta, p.zigzag);
-      if (L >= p.n_items) break;
+      if (L >= n_items) break;
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[BB_KV + kb], (k >> 1) & 1, p.ctl, abortp, 21))) break;
       const int n_it = tile_s[kb].n_m * grp;
@@ -536,7 +546,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     int gi = 0, gt = 0;                     // iterations and half steps so far, over all items
     for (int k = 0; ok; ++k) {
       const int L = bwd_item(k, G, cta, p.zigzag);
-      if (L >= p.n_items) break;
+      if (L >= n_items) break;
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[BB_KV + kb], (k >> 1) & 1, p.ctl, abortp, 43))) break;
       const BTile T = tile_s[kb];
@@ -597,8 +607,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
               const long long t_start = clock64();
               while (ld_acquire_gpu(order) != rank) {
                 if (*abortp || clock64() - t_start > p.ctl.wait_cycles) {
-                  if (p.ctl.status) atomicCAS(p.ctl.status, 0, FL_DEV_WAIT_TIMEOUT | 44);
-                  *abortp = 1;
+                  if (!*abortp) *abortp = 44;
                   go = 0;
                   break;
                 }
@@ -643,7 +652,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     int pending_kve = -1;                            // the K / V buffer whose gradient stores are still to be confirmed
     for (int k = 0; ok; ++k) {
       const int L = bwd_item(k, G, cta, p.zigzag);
-      if (L >= p.n_items) break;
+      if (L >= n_items) break;
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[BB_KV + kb], (k >> 1) & 1, p.ctl, abortp, 39))) break;
       // token-local variant: short of registers, so the tile is read from its slot where needed (the slot stays valid until
@@ -675,8 +684,8 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const bool full = key_valid && (q_first >= vis_from) && (q_first + 63 <= vis_to);
         // which of the half's queries see this key, a bit each (tested bit by bit the mask takes a third of the instructions that
         // comparisons take, and they stand in the loop whether they run or not)
-        uint32_t see[2];
-        {
+        uint32_t see[2] = {0u, 0u};
+        if (!full) {
           const int lo = max(vis_from - q_first, 0), n = key_valid ? max(min(vis_to - q_first + 1, 64) - lo, 0) : 0;
           const uint64_t b = lo < 64 && n > 0 ? (~0ull >> (64 - n)) << lo : 0ull;
           see[0] = (uint32_t)b;
@@ -986,6 +995,31 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             FL_TMEM_ST_32(t_acc + 32 * cc, v);
           }
           tc_wait_st();
+#pragma unroll 1
+          for (int c8 = 0; c8 < 4; ++c8) {           // levels 32 and 64: eight columns of every block
+            uint32_t v[4][8];
+#pragma unroll
+            for (int b2 = 0; b2 < 4; ++b2) FL_TMEM_LD_8(t_acc + 32 * b2 + 8 * c8, v[b2]);
+            tc_wait_ld();
+#pragma unroll
+            for (int e = 0; e < 8; e += 2) {
+              uint64_t y[4];
+#pragma unroll
+              for (int b2 = 0; b2 < 4; ++b2) y[b2] = pack2(__uint_as_float(v[b2][e]), __uint_as_float(v[b2][e + 1]));
+              const uint64_t a0 = add2(y[0], y[1]), a1 = sub2(y[0], y[1]), a2 = add2(y[2], y[3]), a3 = sub2(y[2], y[3]);
+              const uint64_t z[4] = {add2(a0, a2), add2(a1, a3), sub2(a0, a2), sub2(a1, a3)};
+#pragma unroll
+              for (int b2 = 0; b2 < 4; ++b2) {
+                float f0, f1;
+                unpack2(z[b2], f0, f1);
+                v[b2][e] = __float_as_uint(f0);
+                v[b2][e + 1] = __float_as_uint(f1);
+              }
+            }
+#pragma unroll
+            for (int b2 = 0; b2 < 4; ++b2) FL_TMEM_ST_8(t_acc + 32 * b2 + 8 * c8, v[b2]);
+          }
+          tc_wait_st();
         }
         // rows -> shared memory (boxes of 64 elements, 128 B swizzle) -> one TMA store per box: a thread's own row
         // written straight to global memory costs 32 separate 128-byte lines per warp instruction. At d = 128 the first
@@ -1014,89 +1048,84 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         uint16_t* out_base = reinterpret_cast<uint16_t*>(x == 0 ? p.dv : p.dk);
         const uint32_t srow0 = smem_u32(stage0) + r * 128, srow1 = smem_u32(stage1) + r * 128;
         const float cs = rot ? 0.08838834764831845f * mk : mk;
-        constexpr int NB = D / 32, PASSES = EPI2 ? 1 : D / 64;      // 32-column blocks; a pass writes the boxes that fit
-#pragma unroll 1
-        for (int pass = 0; pass < PASSES; ++pass) {
-#pragma unroll 1
-          for (int c8 = 0; c8 < 4; ++c8) {           // eight columns of every block
-            uint32_t v[NB][8];
-#pragma unroll
-            for (int b2 = 0; b2 < NB; ++b2) {
-              if (n_it > 0) FL_TMEM_LD_8(t_acc + 32 * b2 + 8 * c8, v[b2]);     // (CTA-uniform: the loads are warp-collective)
-              else {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) v[b2][e] = 0;              // no query tile saw this key tile
-              }
-            }
+        // 32 columns of the row: scaled (with the rotation's signs), as 16 words of two 16-bit values
+        auto block = [&](int cc, uint32_t* w) {
+          uint32_t v[32];
+          if (n_it > 0) {                  // (CTA-uniform: the tensor-memory loads are warp-collective)
+            FL_TMEM_LD_32(t_acc + 32 * cc, v);
             tc_wait_ld();
-            if (c8 == 3 && pass + 1 == PASSES) {     // the accumulators are in registers: the next item's products may overwrite them
-              tc_fence_before();
-              mbar_arrive_warp(&bars[BB_ACCFREE]);
-            }
-            uint64_t Y[NB][4];
+          } else {                         // no query tile saw this key tile
 #pragma unroll
-            for (int b2 = 0; b2 < NB; ++b2)
+            for (int e = 0; e < 32; ++e) v[e] = 0;
+          }
+          const uint32_t neg = !rot ? 0u : cc == 0 ? 0x10D2E03Eu : cc == 1 ? 0xE0D9F0E2u : cc == 2 ? 0x45809F07u : 0x75954FEDu;
 #pragma unroll
-              for (int e = 0; e < 4; ++e) Y[b2][e] = pack2(__uint_as_float(v[b2][2 * e]), __uint_as_float(v[b2][2 * e + 1]));
-            if (D == 128 && rot) {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const uint64_t a0 = add2(Y[0][e], Y[1][e]), a1 = sub2(Y[0][e], Y[1][e]), a2 = add2(Y[NB - 2][e], Y[NB - 1][e]),
-                               a3 = sub2(Y[NB - 2][e], Y[NB - 1][e]);
-                Y[0][e] = add2(a0, a2);
-                Y[1][e] = add2(a1, a3);
-                Y[NB - 2][e] = sub2(a0, a2);
-                Y[NB - 1][e] = sub2(a1, a3);
-              }
-            }
-#pragma unroll
-            for (int b2 = 0; b2 < NB; ++b2) {
-              if (!EPI2 && (b2 >> 1) != pass) continue;
-              constexpr uint32_t NEG[4] = {0x10D2E03Eu, 0xE0D9F0E2u, 0x45809F07u, 0x75954FEDu};
-              const uint32_t neg = rot ? NEG[b2 & 3] >> (8 * c8) : 0u;
-              uint32_t w[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float c0 = __uint_as_float(__float_as_uint(cs) ^ ((neg << (31 - 2 * e)) & 0x80000000u)),
-                            c1 = __uint_as_float(__float_as_uint(cs) ^ ((neg << (30 - 2 * e)) & 0x80000000u));
-                float a, b3;
-                unpack2(mul2(Y[b2][e], pack2(c0, c1)), a, b3);
-                if (p.out_f16) {
-                  __half2 hh = __floats2half2_rn(a, b3);
-                  w[e] = *reinterpret_cast<uint32_t*>(&hh);
-                } else {
-                  w[e] = pack_bf16x2(a, b3);
-                }
-              }
-              const int ch = 4 * b2 + c8;            // 16-byte chunk of the row
-              if (by_rows) {
-                if (r < out_n && 8 * ch < p.d_out)
-                  *reinterpret_cast<uint4*>(out_base + ((size_t)(out_row + r) * p.h_kv + hkv) * p.d_out + 8 * ch) =
-                      make_uint4(w[0], w[1], w[2], w[3]);
-              } else {
-                sts128((b2 < 2 ? srow0 : srow1) + (((ch & 7) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
-              }
+          for (int e = 0; e < 16; ++e) {
+            const float c0 = __uint_as_float(__float_as_uint(cs) ^ ((neg << (31 - 2 * e)) & 0x80000000u)),
+                        c1 = __uint_as_float(__float_as_uint(cs) ^ ((neg << (30 - 2 * e)) & 0x80000000u));
+            float f0, f1;
+            unpack2(mul2(pack2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1])), pack2(c0, c1)), f0, f1);
+            if (p.out_f16) {
+              __half2 hh = __floats2half2_rn(f0, f1);
+              w[e] = *reinterpret_cast<uint32_t*>(&hh);
+            } else {
+              w[e] = pack_bf16x2(f0, f1);
             }
           }
-          if (by_rows) continue;
-          const bool last = pass + 1 == PASSES;
+        };
+        auto write = [&](int cc, const uint32_t* w) {
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) {
+            const int ch = 4 * cc + q4;            // 16-byte chunk of the row
+            if (by_rows) {
+              if (r < out_n && 8 * ch < p.d_out)
+                *reinterpret_cast<uint4*>(out_base + ((size_t)(out_row + r) * p.h_kv + hkv) * p.d_out + 8 * ch) =
+                    make_uint4(w[4 * q4], w[4 * q4 + 1], w[4 * q4 + 2], w[4 * q4 + 3]);
+            } else {
+              sts128((cc < 2 ? srow0 : srow1) + (((ch & 7) ^ (r & 7)) << 4), w[4 * q4], w[4 * q4 + 1], w[4 * q4 + 2], w[4 * q4 + 3]);
+            }
+          }
+        };
+        // (the first box's rows, or both boxes' where the second has a buffer of its own)
+#pragma unroll 1
+        for (int cc = 0; cc < (EPI2 ? 4 : 2); ++cc) {
+          uint32_t w[16];
+          block(cc, w);
+          write(cc, w);
+        }
+        // one buffer for two boxes: the second box's words wait in registers, so that the accumulators are free all the same
+        constexpr bool HOLD = D == 128 && !EPI2;
+        [[maybe_unused]] uint32_t held[HOLD ? 32 : 1];
+        if constexpr (HOLD) {
+          block(2, held);
+          block(3, held + 16);
+        }
+        tc_fence_before();
+        mbar_arrive_warp(&bars[BB_ACCFREE]);         // the next item's products may overwrite the accumulators
+        auto announce = [&](int pass) -> bool {      // the warpgroup's four warps have written their rows: out with them
           fence_proxy_async();
-          mbar_arrive_warp(&bars[BB_EPI + x]);            // the warpgroup's four warps have written their rows
-          if (!(ok = mbar_wait(&bars[BB_EPI + x], epi & 1, p.ctl, abortp, 38))) break;
+          mbar_arrive_warp(&bars[BB_EPI + x]);
+          if (!mbar_wait(&bars[BB_EPI + x], epi & 1, p.ctl, abortp, 38)) return false;
           ++epi;
           if (r == 0 && out_n == 128) {
             tma_store_4d(tm_out, stage0, 64 * pass, hkv, out_row, T.bat);
             if (EPI2) tma_store_4d(tm_out, stage1, 64, hkv, out_row, T.bat);
             tma_store_commit();
-            if (!last) tma_store_wait_read<0>();          // the one buffer is written again by the next pass
           }
-          if (!last) {
+          return true;
+        };
+        if (!by_rows && !(ok = announce(0))) break;
+        if constexpr (HOLD) {
+          if (!by_rows) {
+            if (r == 0) tma_store_wait_read<0>();
             mbar_arrive_warp(&bars[BB_EPI + x]);
             if (!(ok = mbar_wait(&bars[BB_EPI + x], epi & 1, p.ctl, abortp, 38))) break;
             ++epi;
           }
+          write(2, held);
+          write(3, held + 16);
+          if (!by_rows && !(ok = announce(1))) break;
         }
-        if (!ok) break;
         pending_kve = kb;
       }
     }
@@ -1108,12 +1137,13 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) report_abort(p.ctl, abortp);
   if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
 }  // namespace fl
 
-extern "C" int fl_bwd(const fl_attn_args* a, void* stream) {
+static int bwd_launch(const fl_attn_args* a, const void* work, void* stream) {
   using namespace fl;
   if (!a || !a->q_codes || !a->k_codes || !a->v_codes || !a->do_codes || !a->status) return FL_ERR_BAD_ARG;
   if (!a->fac_q || !a->fac_k || !a->fac_v || !a->fac_do || !a->lse_log2 || !a->d_rows || !a->dq_acc || (!a->dq_scale && !a->dq_scale_rows) ||
@@ -1176,13 +1206,19 @@ extern "C" int fl_bwd(const fl_attn_args* a, void* stream) {
   p.out_f16 = (a->flags & FL_A_OUT_F16) ? 1 : 0;
   p.had_dk = (a->flags & FL_A_HAD_DK) ? 1 : 0;
   p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);
-  const int ntile = a->doc_start ? (a->s_k / 128 + a->n_docs) : a->s_k / 128;
+  const int ntile = a->doc_start && !work ? (a->s_k / 128 + a->n_docs) : a->s_k / 128;
   const int nb = a->doc_start ? 1 : a->b;
   p.n_tile = ntile;
   const long long n_items = (long long)ntile * a->h_kv * nb;
   if (n_items > 0x3FFFFFFF) return FL_ERR_TOO_LARGE;
   p.n_items = (int)n_items;
-  p.zigzag = (p.causal && !a->doc_start) ? 1 : 0;
+  p.zigzag = ((p.causal && !a->doc_start) || work) ? 1 : 0;
+  if (work && !a->doc_start) return FL_ERR_BAD_ARG;
+  p.work_head = (const int4*)work;
+  p.work = work ? p.work_head + 1 + a->s_k / 128 : nullptr;
+  p.div_item = FastDiv(a->doc_start ? 1 : p.causal ? a->h_kv * a->b : ntile);
+  p.div_h = FastDiv(a->h_kv);
+  p.grp = a->h / a->h_kv;
   const int grid = (int)(n_items < sm_count() ? n_items : sm_count());     // one persistent CTA per SM
   const int smem = a->d == 64 ? BwdSmem<64, false, false>::BYTES : fp4 ? BwdSmem<128, true, false>::BYTES
                    : tl ? BwdSmem<128, false, true>::BYTES : BwdSmem<128, false, false>::BYTES;
@@ -1194,7 +1230,7 @@ extern "C" int fl_bwd(const fl_attn_args* a, void* stream) {
   const bool det = a->dq_order != nullptr;
   if (det && (sc || rl || tl)) return FL_ERR_UNSUPPORTED;     // ordered dQ: the default dS-hat route only
   // the lean kernels serve the plain calls; any of the rarer forms takes the full variant of the same kernel
-  const bool full = det || a->dq_scale_rows || a->slot_src || a->dk_mult;
+  const bool full = det || a->dq_scale_rows || a->doc_start || a->dk_mult;
 #define FL_BWD_LAUNCH(D_, FP4_, VAR_, SC_) \
   (full ? launch(bwd_kernel_pipelined<D_, FP4_, VAR_, SC_, true>) : launch(bwd_kernel_pipelined<D_, FP4_, VAR_, SC_, false>))
   if (sc) {
@@ -1212,4 +1248,10 @@ extern "C" int fl_bwd(const fl_attn_args* a, void* stream) {
 #undef FL_BWD_LAUNCH
   if (rc) return rc;
   return launch_result("fl_bwd: kernel launch");
+}
+
+extern "C" int fl_bwd(const fl_attn_args* a, void* stream) { return bwd_launch(a, nullptr, stream); }
+
+extern "C" int fl_bwd_work(const fl_attn_args* a, const int32_t* work, void* stream) {
+  return work ? bwd_launch(a, work, stream) : fl::FL_ERR_BAD_ARG;
 }

@@ -38,6 +38,19 @@ int set_smem(void (*kern)(A...), int bytes, const char* where) {
 // multiprocessors of the current device (cached per device): the size of a persistent grid
 int sm_count();
 
+// Division of n < 2^31 by a divisor known at launch: one multiplication (m = floor(2^(31 + l) / d) + 1 with 2^(l - 1) < d <= 2^l; the
+// error n (m d - 2^(31 + l)) stays below 2^(31 + l)).
+struct FastDiv {
+  uint32_t m;
+  int l, d;
+  FastDiv() = default;
+  explicit FastDiv(int div) : d(div) {
+    for (l = 0; (1ll << l) < div; ++l) {}
+    m = (uint32_t)((1ull << (31 + l)) / (uint32_t)div + 1);
+  }
+  __device__ __forceinline__ int div(int n) const { return (int)(((uint64_t)(uint32_t)n * m) >> (31 + l)); }
+};
+
 static constexpr long long kDefaultWaitCycles = 1ll << 31;
 
 }  // namespace fl

@@ -75,6 +75,8 @@ struct FwdParams {
   int causal;
   int win_l, win_r;      // sliding window sides, -1 = unlimited (causal: the right side is 0)
   int out_f16;
+  const int4* work;      // documents: the list of fl_doc_work, or null
+  FastDiv div_item, div_h, div_grp;   // items per (causal: row block; otherwise: head), query heads, group size
   int n_items;           // work items: 256-row blocks x heads x batch rows (documents: block slots x heads)
   int n_blk;             // blocks per batch row (documents: block slots of the packed buffer)
   int zigzag;            // deal the items out in zigzag rounds (causal: they are ordered longest first)
@@ -84,6 +86,7 @@ struct FwdParams {
 struct Tile {
   int bat;    // batch coordinate of the tensor maps (0 for packed documents)
   int head;   // query head
+  int hkv;    // its kv head
   int q0;     // first query row (row index inside the batch entry)
   int nq;     // valid query rows of this item (<= 256; 0 = an empty block slot)
   int k0;     // first key row this item loads (row index inside the batch entry)
@@ -115,32 +118,37 @@ __device__ __forceinline__ int fwd_item(int k, int G, int c, int zigzag) {
 // Work item L -> its block. Causal: blocks slowest and last block first, so that the item index orders the items longest
 // first; heads fastest, so the query heads of a kv group run together and share its K / V tiles in L2. Otherwise blocks
 // fastest: neighbours share their K / V tiles in L2 and every block costs the same.
+template <bool DOCS>
 __device__ __forceinline__ void fwd_decode(const FwdParams& p, int L, Tile& t) {
-  if (p.doc_start == nullptr) {
-    int blk, rem;
-    if (p.causal) { blk = p.n_blk - 1 - L / (p.h * p.b); rem = L % (p.h * p.b); }
-    else { blk = L % p.n_blk; rem = L / p.n_blk; }
-    t.head = rem % p.h; t.bat = rem / p.h;
+  if (!DOCS || p.doc_start == nullptr) {
+    const int q = p.div_item.div(L), rq = L - q * p.div_item.d;
+    const int blk = p.causal ? p.n_blk - 1 - q : rq, rem = p.causal ? rq : q;
+    t.bat = p.div_h.div(rem); t.head = rem - t.bat * p.h;
     t.q0 = blk * 256; t.nq = min(256, p.s_q - t.q0); t.k0 = 0; t.sk = p.s_k;
     if (p.seqused_k) t.sk = max(0, min(p.s_k, p.seqused_k[t.bat]));      // keys past it are masked like a document's end
     t.off = p.s_k - p.s_q; t.qrel = t.q0;
   } else {
     // documents sit at 128-aligned starts of one packed batch entry; block slot x -> (document, 256-row block)
-    int x = L / p.h, dsel = -1, blk = 0, len = 0, st = 0;
-    t.head = L % p.h;
-    for (int dI = 0; dI < p.n_docs; ++dI) {
-      doc_entry(p.doc_start, p.doc_len, dI, p.s_q, p.ctl.status, st, len);
-      const int nb = (len + 255) / 256;
-      if (x < nb) { dsel = dI; blk = x; break; }
-      x -= nb;
+    int x = p.div_h.div(L), dsel = -1, blk = 0, len = 0, st = 0;
+    t.head = L - x * p.h;
+    if (p.work) {          // longest first; checked when the list was made
+      const int4 e = __ldg(p.work + 1 + x);
+      st = e.x; len = e.y; blk = e.z; dsel = 0;
+    } else {
+      for (int dI = 0; dI < p.n_docs; ++dI) {
+        doc_entry(p.doc_start, p.doc_len, dI, p.s_q, p.ctl.status, st, len);
+        const int nb = (len + 255) / 256;
+        if (x < nb) { dsel = dI; blk = p.causal ? nb - 1 - x : x; break; }
+        x -= nb;
+      }
     }
     if (dsel < 0) { t.nq = 0; t.bat = 0; t.q0 = 0; t.k0 = 0; t.sk = 0; t.off = 0; t.qrel = 0; }
     else {
-      if (p.causal) blk = (len + 255) / 256 - 1 - blk;
       t.bat = 0; t.q0 = st + blk * 256; t.nq = min(256, len - blk * 256); t.k0 = st; t.sk = len; t.off = 0;
       t.qrel = blk * 256;
     }
   }
+  t.hkv = p.div_grp.div(t.head);
   // left window: the first key any row of this block can see; both stages start at that key tile
   t.kofs = 0;
   if (p.win_l >= 0 && t.nq > 0) t.kofs = (max(0, t.qrel + t.off - p.win_l) / 128) * 128;
@@ -181,7 +189,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = gridDim.x, cta = blockIdx.x;
-  const int grp = p.h / p.h_kv;
+  const int n_items = FULL && p.work ? __ldg(p.work).x * p.h : p.n_items;
 
   if (tid == 8 * 32) {
     abort_s = 0;
@@ -222,15 +230,15 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       bool ok = true;
       for (int k = 0; ok; ++k) {
         const int L = fwd_item(k, G, cta, p.zigzag);
-        if (L >= p.n_items) break;
+        if (L >= n_items) break;
         const int kb = k & 1;
         // the Q buffer of item k - 2 (and its slot of tile_s) is free once both softmax warpgroups have written its
         // output rows out of it
         if (k >= 2 && !(ok = mbar_wait(&bars[B_QE + kb], ((k >> 1) - 1) & 1, p.ctl, abortp, 12))) break;
         Tile t;
-        fwd_decode(p, L, t);
+        fwd_decode<FULL>(p, L, t);
         tile_s[kb] = t;
-        const int hkv = t.head / grp;
+        const int hkv = t.hkv;
         if (t.nq > 0) {
           const bool two = t.nq > 128;
           mbar_arrive_expect_tx(&bars[B_Q + kb], 2 * OP_BYTES + (FP4 ? (two ? 2048 : 1024) : 0));
@@ -276,7 +284,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     bool ok = true;
     for (int k = 0; ok; ++k) {
       const int L = fwd_item(k, G, cta, p.zigzag);
-      if (L >= p.n_items) break;
+      if (L >= n_items) break;
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[B_Q + kb], (k >> 1) & 1, p.ctl, abortp, 20))) break;
       const int n0 = tile_s[kb].n[0], n1 = tile_s[kb].n[1];
@@ -400,11 +408,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     bool ok = true;
     for (int k = 0; ok; ++k) {
       const int L = fwd_item(k, G, cta, p.zigzag);
-      if (L >= p.n_items) break;
+      if (L >= n_items) break;
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[B_Q + kb], (k >> 1) & 1, p.ctl, abortp, 36))) break;
       const Tile T = tile_s[kb];
-      const int head = T.head, hkv = head / grp;
+      const int head = T.head, hkv = T.hkv;
       const int n_i = T.n[i];
       const int qrow = T.q0 + 128 * i + r;              // row inside the batch entry
       const int qrel = T.qrel + 128 * i + r;            // row inside the document
@@ -682,12 +690,13 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) report_abort(p.ctl, abortp);
   if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
 }  // namespace fl
 
-extern "C" int fl_fwd(const fl_attn_args* a, void* stream) {
+static int fwd_launch(const fl_attn_args* a, const void* work, void* stream) {
   using namespace fl;
   if (!a || !a->q_codes || !a->k_codes || !a->v_codes || !a->out || !a->status) return FL_ERR_BAD_ARG;
   if (!a->fac_q || !a->fac_k || !a->fac_v) return FL_ERR_BAD_ARG;
@@ -731,13 +740,18 @@ extern "C" int fl_fwd(const fl_attn_args* a, void* stream) {
   p.out_f16 = (a->flags & FL_A_OUT_F16) ? 1 : 0;
   p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);
   // packed documents: at most one extra 256-row block per document beyond total / 256
-  const int nblk = a->doc_start ? (a->s_q / 256 + a->n_docs + 1) : (a->s_q + 255) / 256;
+  const int nblk = work ? a->s_q / 128 : a->doc_start ? (a->s_q / 256 + a->n_docs + 1) : (a->s_q + 255) / 256;
   const int nb = a->doc_start ? 1 : a->b;
   p.n_blk = nblk;
   const long long n_items = (long long)nblk * a->h * nb;
   if (n_items > 0x3FFFFFFF) return FL_ERR_TOO_LARGE;
   p.n_items = (int)n_items;
-  p.zigzag = (p.causal && !a->doc_start) ? 1 : 0;
+  p.zigzag = ((p.causal && !a->doc_start) || work) ? 1 : 0;
+  p.work = (const int4*)work;
+  if (work && !a->doc_start) return FL_ERR_BAD_ARG;
+  p.div_item = FastDiv(a->doc_start ? 1 : p.causal ? a->h * a->b : nblk);
+  p.div_h = FastDiv(a->h);
+  p.div_grp = FastDiv(a->h / a->h_kv);
   const int grid = (int)(n_items < sm_count() ? n_items : sm_count());     // one persistent CTA per SM
   const int smem = 4 * Q_STRIDE + 2 * KV_STAGES * 128 * a->d + 1024 + (fp4 ? 4096 + KV_STAGES * 1024 : 0);
   cudaStream_t st = (cudaStream_t)stream;
@@ -750,8 +764,8 @@ extern "C" int fl_fwd(const fl_attn_args* a, void* stream) {
   if (sc && tl) return FL_ERR_UNSUPPORTED;
   p.cap_a = sc ? a->softcap * 1.4426950408889634f : 0.f;
   p.cap_b = sc ? 1.0f / p.cap_a : 0.f;
-  // the lean kernels serve the plain calls; packed outputs and the output-row factor take the full variant
-  const bool full = a->slot_src != nullptr || a->o_mult != nullptr;
+  // the lean kernels serve the plain calls; documents, packed outputs and the output-row factor take the full variant
+  const bool full = a->doc_start != nullptr || a->o_mult != nullptr;
 #define FL_FWD_LAUNCH(D_, FP4_, TL_, GF_, SC_) \
   (full ? launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, true>) : launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, false>))
   if (sc) {
@@ -769,4 +783,10 @@ extern "C" int fl_fwd(const fl_attn_args* a, void* stream) {
 #undef FL_FWD_LAUNCH
   if (rc) return rc;
   return launch_result("fl_fwd: kernel launch");
+}
+
+extern "C" int fl_fwd(const fl_attn_args* a, void* stream) { return fwd_launch(a, nullptr, stream); }
+
+extern "C" int fl_fwd_work(const fl_attn_args* a, const int32_t* work, void* stream) {
+  return work ? fwd_launch(a, work, stream) : fl::FL_ERR_BAD_ARG;
 }

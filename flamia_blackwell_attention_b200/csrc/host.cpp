@@ -174,7 +174,7 @@ struct Workspace {
 // rows of every 128-row slot), and the kernels write the caller's packed rows themselves. aligned: the caller's rows are
 // the buffer's rows already.
 struct Docs {
-  Tensor start, len, row_map, slot_src, slot_rows;
+  Tensor start, len, row_map, slot_src, slot_rows, work;
   int64_t capacity = 0;
   bool aligned = false;
 };
@@ -375,7 +375,15 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> forward(int64_t handle, const Te
     check(fl_token_aux(ptr<float>(vq.token_factors), n, ptr<float>(tok), ptr<float>(tok) + n, st), "fl_token_aux");
     a.tok_lg_v = ptr<float>(tok); a.tok_rcp_v = ptr<float>(tok) + n;
   }
-  check(fl_fwd(&a, st), "fl_fwd");
+  if (has_docs) {          // which blocks exist, longest first
+    docs.work = empty({FL_DOC_WORK_INTS(docs.capacity)}, at::kInt, dev);
+    check(fl_doc_work(a.doc_start, a.doc_len, a.n_docs, (int32_t)docs.capacity, a.window_left_p1, a.window_right_p1, p.causal,
+                      p.deterministic, ptr<int32_t>(docs.work), stp, st),
+          "fl_doc_work");
+    check(fl_fwd_work(&a, ptr<int32_t>(docs.work), st), "fl_fwd_work");
+  } else {
+    check(fl_fwd(&a, st), "fl_fwd");
+  }
 
   std::vector<Tensor> state;
   state.reserve(20);
@@ -391,6 +399,7 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> forward(int64_t handle, const Te
   if (has_docs) {
     state.push_back(docs.start); state.push_back(docs.len);
     if (repacked) { state.push_back(docs.row_map); state.push_back(docs.slot_src); state.push_back(docs.slot_rows); }
+    state.push_back(docs.work);
     if (docs.aligned) {
       lse_user = lse.select(0, 0);            // (h, total_q): the caller's rows are the kernels' rows
     } else if (p.return_lse) {
@@ -442,7 +451,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
   if (p.fp4) { a.q4 = ptr<uint8_t>(next()); a.sfq4 = ptr<uint8_t>(next()); a.k4 = ptr<uint8_t>(next()); a.sfk4 = ptr<uint8_t>(next()); }
   if (p.token_local) { a.fac_q = ptr<float>(next()); a.fac_k = ptr<float>(next()); a.fac_v = ptr<float>(next()); }
   if (p.seqused_k) a.seqused_k = ptr<int32_t>(next());
-  const int32_t *slot_src = nullptr, *slot_rows = nullptr;
+  const int32_t *slot_src = nullptr, *slot_rows = nullptr, *work = nullptr;
   const int64_t total = p.varlen ? p.tot_q : p.b * p.s_q;
   if (has_docs) {
     a.doc_start = ptr<int32_t>(next());
@@ -453,6 +462,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
       slot_src = ptr<int32_t>(next()); slot_rows = ptr<int32_t>(next());
       a.slot_src = slot_src; a.slot_rows = slot_rows; a.out_rows = (int32_t)total;
     }
+    work = ptr<int32_t>(next());
   }
   int32_t* stp = ptr<int32_t>(status);
   const bool rows = p.prescale == 2;
@@ -516,7 +526,8 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
   a.dk_mult = ptr<float>(dk_mult);
   if (p.deterministic) a.dq_order = ptr<int32_t>(ws.at(w_order));
   a.status = stp;
-  check(fl_bwd(&a, st), "fl_bwd");
+  if (work) check(fl_bwd_work(&a, work, st), "fl_bwd_work");
+  else check(fl_bwd(&a, st), "fl_bwd");
   check(fl_dq_post_cols(g.zero_acc, ps, rows, ptr<float>(dq_mult), a.softmax_scale, ptr<void>(dq), (int32_t)sh.b, (int32_t)sh.s_q,
                         (int32_t)p.h, (int32_t)p.d, (int32_t)p.d_call, had8, f16, slot_src, slot_rows, st),
         "fl_dq_post_cols");

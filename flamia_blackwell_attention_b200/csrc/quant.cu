@@ -486,6 +486,7 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
   // a CTA that gave up must not exit while loads into its shared memory may still land
   if (abort_s) {
     for (int i = 0; i < 200; ++i) __nanosleep(1000);
+    if (tid == 0) report_abort(p.ctl, abortp);
   }
 }
 
@@ -796,6 +797,7 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
   if (tid == 0) tma_store_wait_read<0>();
   if (abort_s) {
     for (int i = 0; i < 200; ++i) __nanosleep(1000);
+    if (tid == 0) report_abort(p.ctl, abortp);
   }
 }
 

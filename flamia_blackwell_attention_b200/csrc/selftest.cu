@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(128) selftest_kernel(const __grid_constant__ C
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) report_abort(p.ctl, &abort_s);
   if (warp == 0) tmem_dealloc(tmem, 512);
 }
 

@@ -247,6 +247,17 @@ int fl_bwd_static_acc(const fl_attn_args* args, const float* post_scale, float m
 int fl_doc_tables(const int32_t* cu, int32_t n_docs, int32_t fixed_len, int32_t total, int32_t capacity, int32_t* start, int32_t* len,
                   int32_t* row_map, int32_t* slot_src, int32_t* slot_rows, void* stream);
 
+/* Work lists of packed documents for fl_fwd_work / fl_bwd_work, in one launch: which blocks exist, longest first (ordered != 0: in
+ * document order, which the ordered dQ reduction needs). work: FL_DOC_WORK_INTS(capacity) ints, 16-byte aligned. Masks as in
+ * fl_attn_args. status: takes FL_DEV_BAD_TABLE for a table entry that does not fit, or NULL. The counterpart of the reference's
+ * packed scheduler (flash_attn/cute/lp_varlen.py). */
+#define FL_DOC_WORK_INTS(capacity) (4 + 9 * ((capacity) / 128))
+int fl_doc_work(const int32_t* doc_start, const int32_t* doc_len, int32_t n_docs, int32_t capacity, int32_t window_left_p1,
+                int32_t window_right_p1, int32_t causal, int32_t ordered, int32_t* work, int32_t* status, void* stream);
+/* fl_fwd / fl_bwd on packed documents with their work lists: the same results */
+int fl_fwd_work(const fl_attn_args* args, const int32_t* work, void* stream);
+int fl_bwd_work(const fl_attn_args* args, const int32_t* work, void* stream);
+
 /* The live rows of the aligned buffer's LSE (h, capacity) in the caller's rows: packed row g goes to out[g / seq][head][g % seq]
  * (packed documents: seq = total, out is (h, total); batch rows run as documents: seq = s, out is (b, h, s)). */
 int fl_unpack_lse(const float* lse, const int32_t* slot_src, const int32_t* slot_rows, int32_t capacity, int32_t h, int32_t seq,

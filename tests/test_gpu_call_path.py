@@ -37,7 +37,7 @@ def test_one_launch_quantiser_equals_single_launches(entry, d, dtype, form):
         q, k, v, _ = (t[0].to(dt).cuda() for t in attention_inputs(1, sum(LENS), h, hk, d, seed=3))
         cu = torch.tensor([0] + list(torch.tensor(LENS).cumsum(0)), dtype=torch.int32, device="cuda")
         _, _, st = _state(entry, q, k, v, [cu, cu], cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=max(LENS), max_seqlen_k=max(LENS))
-        slots, base = (st[-3], st[-2], st[-4].numel()), 1
+        slots, base = (st[-4], st[-3], st[-5].numel()), 1
     pad = lambda t: torch.nn.functional.pad(t, (0, dp - d))      # noqa: E731
     want = [K.quantize_fp8_blocks(pad(t), legacy_kernel=True, packed_slots=slots, output_tile_stats=i > 0, **(rot if i < 2 else {}))
             for i, t in enumerate((q, k, v))]
@@ -60,7 +60,7 @@ def test_document_tables_in_one_launch(lens):
     q, k, v, _ = (t[0].cuda() for t in attention_inputs(1, total, 2, 1, 64, seed=4))
     c = cu.cuda()
     _, lse, st = _state("fp8", q, k, v, [c, c], cu_seqlens_q=c, cu_seqlens_k=c, max_seqlen_q=max(lens), max_seqlen_k=max(lens), return_lse=True)
-    for name, t in zip(("start", "len", "row_map", "slot_src", "slot_rows"), st[-6:-1]):
+    for name, t in zip(("start", "len", "row_map", "slot_src", "slot_rows"), st[-7:-2]):
         assert torch.equal(t.cpu(), getattr(ref, name)), name
     rows = ref.row_map.cuda().long()
     assert torch.equal(lse[:, rows[rows >= 0]], st[0][0][:, rows >= 0])
@@ -78,3 +78,28 @@ def test_dq_prescale_of_many_tiles(b, h, hk, nt, causal):
         bound = 8.0 * do[:, :, q_sl, 1].amax((1, 2)).sqrt() * v[:, :, k_sl, 1].amax((1, 2)).sqrt() * k[:, :, k_sl, 0].amax((1, 2))
         want = torch.exp2(torch.floor(torch.log2(65504.0 / bound)))
         assert torch.equal(ks[:, t], want) and torch.equal(ps[:, t], 1.0 / want)
+
+
+@pytest.mark.parametrize("lens,kw", [(LENS, {}), ([1] * 1100 + [700], {}), ([5000, 3, 1300], dict(window_size=(400, 0))),
+                                     ([640, 128, 256], dict(deterministic=True))])
+def test_work_list_changes_nothing(lens, kw):
+    """Documents through fl_doc_work's lists (several chunks of its scan, equal costs, a window, document order) against the kernel's
+    own walk over the document table: O and LSE bit for bit, every pair exactly once."""
+    from flamia_blackwell_attention_b200 import kernels as K
+    h, hk, d = 3, 1, 128
+    total = sum(lens)
+    q, k, v, _ = (t[0].cuda() for t in attention_inputs(1, total, h, hk, d, seed=6))
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device="cuda")
+    out, _, st = _state("fp8", q, k, v, [cu, cu], cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=max(lens), max_seqlen_k=max(lens), **kw)
+    start, length, row_map, slot_src, slot_rows, work = st[-7:-1]
+    n_f, n_b = work[:2].tolist()
+    tiles = row_map.numel() // 128
+    pairs = work[4:4 + 8 * tiles].view(2, tiles, 4)
+    for part, rows, n in ((pairs[0], 256, n_f), (pairs[1], 128, n_b)):
+        got = sorted((s, m, b) for s, m, b, _ in part[:n].tolist())
+        assert got == sorted((s, m, b) for s, m in zip(start.tolist(), length.tolist()) for b in range((m + rows - 1) // rows))
+    ops = [dict(codes=st[1 + 2 * i].view(torch.uint8), fac=st[2 + 2 * i]) for i in range(3)]
+    want, lse, _ = K.attn_fwd(*ops, causal=True, softmax_scale=d ** -0.5, window=kw.get("window_size"),
+                              packed_out=(slot_src, slot_rows, total), doc_start=start, doc_len=length)
+    live = row_map >= 0
+    assert torch.equal(out, want[0]) and torch.equal(st[0][0][:, live], lse[0][:, live])
