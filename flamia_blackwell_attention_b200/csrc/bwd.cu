@@ -649,6 +649,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     bool ok = true;
     int gi = 0, epi = 0;                             // iterations so far; uses of the epilogue barrier so far
     int cg = 0;                                      // grants used so far
+    constexpr int QW = RL ? 32 : 64, NP = 64 / QW;   // queries per pass, passes
     int pending_kve = -1;                            // the K / V buffer whose gradient stores are still to be confirmed
     for (int k = 0; ok; ++k) {
       const int L = bwd_item(k, G, cta, p.zigzag);
@@ -691,11 +692,9 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           see[0] = (uint32_t)b;
           see[1] = (uint32_t)(b >> 32);
         }
-        auto visible = [&](int j) { return (see[j >> 5] & (1u << (j & 31))) != 0; };
         if (++m == T.m_lo + T.n_m) m = T.m_lo;                              // (the next iteration's from here on)
         if (!(ok = mbar_wait(&bars[BB_BFULL + 2 * st + x], (g >> 1) & 1, p.ctl, abortp, 30))) break;   // row vectors and scalars visible
-        const uint32_t v_lse = smem_u32(smem) + SM::VEC + (2 * st + x) * SM::VEC_HALF, v_dpp = v_lse + 256;
-        [[maybe_unused]] const uint32_t v_fq = v_lse + 512, v_fdo = v_lse + 768;      // token-local: the 64 per-query factors of the half
+        const uint32_t v_vec = smem_u32(smem) + SM::VEC + (2 * st + x) * SM::VEC_HALF;
         // the f16 pre-scale: one power of two per query tile (folded into K's exponent bytes below), or one per query row
         // (folded into the dQ side's B scale bytes, whose lanes are the queries)
         const float4 sc4 = lds128(smem_u32(misc.scal[st][x]));
@@ -707,7 +706,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           lq1 = (uint32_t)((int)((__float_as_uint(rp[32 + lane]) >> 23) & 0xFF) - 127);
         }
         // FP4: the block scales of S were applied by the tensor core; only the softmax scale remains
-        const float c[2] = {FP4 ? p.scale_log2 : fk * sc4.x, FP4 ? p.scale_log2 : fk * sc4.y}, b8[2] = {fv8 * sc4.z, fv8 * sc4.w};
+        const float cq[2] = {FP4 ? p.scale_log2 : fk * sc4.x, FP4 ? p.scale_log2 : fk * sc4.y}, bq[2] = {fv8 * sc4.z, fv8 * sc4.w};
         // token-local: unit scale bytes for the Q and dO operands
         const uint32_t eq2 = ((__float_as_uint(sc4.x) >> 23) & 0xFF) | (((__float_as_uint(sc4.y) >> 23) & 0xFF) << 8);
         const uint32_t edo2 = ((__float_as_uint(sc4.z) >> 23) & 0xFF) | (((__float_as_uint(sc4.w) >> 23) & 0xFF) << 8);
@@ -715,190 +714,253 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const uint32_t lb = (uint32_t)((int)((__float_as_uint(bsc) >> 23) & 0xFF) - 127) & 0xFF;
         const uint32_t ekb_word = __vadd4(ek_word, lb * 0x01010101u);
 
-        // ---- P' = 2^(s c - lse2)
+        // The 64 queries are worked on QW at a time: all of them in the plain variants; 32 in a rolled loop where the row-local dQ
+        // side's code would not fit the instruction cache twice (token-local: 74 KB of code, of it 35 KB in this loop).
+        uint32_t pw[16], dsw[16];         // P-hat's and dS-hat's codes, kept until the region they go to is free
+        uint32_t epw = 0, ebw = 0;        // exponent bytes of the two query blocks: token-local P-hat's, dS-hat's
         if (!(ok = mbar_wait(&bars[BB_S + x], g & 1, p.ctl, abortp, 31))) break;
         tc_fence_after();
-        uint32_t pv[64];
-        FL_TMEM_LD_32(t_sx, pv);
-        FL_TMEM_LD_32(t_sx + 32, (pv + 32));
-        tc_wait_ld();
-        // the scores are in registers: this region may take the other half's P-hat and dS-hat (half 0's iteration waits for S1 of
-        // the same iteration; half 1's for S0 of the next one, which is issued before, or of this one where that was the last)
-        tc_fence_before();
-        if (x == 1 || it > 0 || n_it == 1) mbar_arrive_warp(&bars[BB_GRANT + (1 - x)]);
-        if (x == 0 && it == 0 && n_it > 1) mbar_arrive_warp(&bars[BB_SDR]);
-        float pf[64];
-        [[maybe_unused]] uint32_t pw_ep = 0;
-        uint32_t pw[16];                  // P-hat's codes, kept until the region they go to is free
-        if constexpr (SC) {
-          // soft cap: x = cap_a tanh(s c cap_b); P-hat is taken from P' right here, and what stays in pf is
-          // P' (1 - tanh^2), the factor dS needs (the reference's score_mod_bwd, flash_attn/cute/utils.py:178-187)
-#pragma unroll
-          for (int j4 = 0; j4 < 16; ++j4) {
-            const float4 l4 = lds128(v_lse + 16 * j4);
-            const float cc = c[j4 >> 3];
-            const float l[4] = {l4.x, l4.y, l4.z, l4.w};
-            float pp[4], df[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float th = tanh_fast(__uint_as_float(pv[4 * j4 + e]) * (cc * p.cap_b));
-              pp[e] = ex2(fmaf(p.cap_a, th, -l[e]));
-              df[e] = fmaf(-th, th, 1.0f);
-              if (!full) pp[e] = visible(4 * j4 + e) ? pp[e] : 0.f;
-            }
-            pw[j4] = cvt_e4m3x4(pp[0], pp[1], pp[2], pp[3]);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) pf[4 * j4 + e] = pp[e] * df[e];
+#pragma unroll 1
+        for (int ps = 0; ps < NP; ++ps) {
+          const uint32_t v_lse = v_vec + 4 * QW * ps, v_dpp = v_lse + 256;
+          [[maybe_unused]] const uint32_t v_fq = v_lse + 512, v_fdo = v_lse + 768;      // token-local: the per-query factors
+          // ---- P' = 2^(s c - lse2)
+          uint32_t pv[QW];
+          FL_TMEM_LD_32(t_sx + QW * ps, pv);
+          if constexpr (QW == 64) FL_TMEM_LD_32(t_sx + 32, (pv + 32));
+          tc_wait_ld();
+          if (NP == 1 || ps + 1 == NP) {
+            // the scores are in registers: this region may take the other half's P-hat and dS-hat (half 0's iteration waits for S1 of
+            // the same iteration; half 1's for S0 of the next one, which is issued before, or of this one where that was the last)
+            tc_fence_before();
+            if (x == 1 || it > 0 || n_it == 1) mbar_arrive_warp(&bars[BB_GRANT + (1 - x)]);
+            if (x == 0 && it == 0 && n_it > 1) mbar_arrive_warp(&bars[BB_SDR]);
           }
-        } else {
+          // the pass's factors per 32 queries
+          const float c[2] = {NP == 1 || ps == 0 ? cq[0] : cq[1], cq[1]}, b8[2] = {NP == 1 || ps == 0 ? bq[0] : bq[1], bq[1]};
+          const uint32_t seen[2] = {NP == 1 || ps == 0 ? see[0] : see[1], see[1]};
+          auto visible = [&](int j) { return (seen[j >> 5] & (1u << (j & 31))) != 0; };
+          float pf[QW];
+          uint32_t pn[QW / 4], dn[QW / 4];      // this pass's codes
+          if constexpr (SC) {
+            // soft cap: x = cap_a tanh(s c cap_b); P-hat is taken from P' right here, and what stays in pf is
+            // P' (1 - tanh^2), the factor dS needs (the reference's score_mod_bwd, flash_attn/cute/utils.py:178-187)
 #pragma unroll
-          for (int j4 = 0; j4 < 16; ++j4) {
-            const float4 l4 = lds128(v_lse + 16 * j4);
-            const float cc = c[j4 >> 3];
-            // t = lse2 - s c (token-local: c = f_K f_Q(query)), two columns per instruction; P' = 2^-t
-            uint64_t c01, c23;
-            if (TL) {
-              const float4 f4 = lds128(v_fq + 16 * j4);
-              const uint64_t nfk2 = pack2(-fk, -fk);
-              c01 = mul2(pack2(f4.x, f4.y), nfk2);
-              c23 = mul2(pack2(f4.z, f4.w), nfk2);
-            } else {
-              c01 = c23 = pack2(-cc, -cc);
+            for (int j4 = 0; j4 < QW / 4; ++j4) {
+              const float4 l4 = lds128(v_lse + 16 * j4);
+              const float cc = c[j4 >> 3];
+              const float l[4] = {l4.x, l4.y, l4.z, l4.w};
+              float pp[4], df[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float th = tanh_fast(__uint_as_float(pv[4 * j4 + e]) * (cc * p.cap_b));
+                pp[e] = ex2(fmaf(p.cap_a, th, -l[e]));
+                df[e] = fmaf(-th, th, 1.0f);
+                if (!full) pp[e] = visible(4 * j4 + e) ? pp[e] : 0.f;
+              }
+              pn[j4] = cvt_e4m3x4(pp[0], pp[1], pp[2], pp[3]);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) pf[4 * j4 + e] = pp[e] * df[e];
             }
-            float t0, t1, t2, t3;
-            unpack2(fma2(pack2(__uint_as_float(pv[4 * j4 + 0]), __uint_as_float(pv[4 * j4 + 1])), c01, pack2(l4.x, l4.y)), t0, t1);
-            unpack2(fma2(pack2(__uint_as_float(pv[4 * j4 + 2]), __uint_as_float(pv[4 * j4 + 3])), c23, pack2(l4.z, l4.w)), t2, t3);
-            pf[4 * j4 + 0] = ex2_neg(t0);
-            pf[4 * j4 + 1] = ex2_neg(t1);
-            pf[4 * j4 + 2] = ex2_neg(t2);
-            pf[4 * j4 + 3] = ex2_neg(t3);
+          } else {
+#pragma unroll
+            for (int j4 = 0; j4 < QW / 4; ++j4) {
+              const float4 l4 = lds128(v_lse + 16 * j4);
+              const float cc = c[j4 >> 3];
+              // t = lse2 - s c (token-local: c = f_K f_Q(query)), two columns per instruction; P' = 2^-t
+              uint64_t c01, c23;
+              if (TL) {
+                const float4 f4 = lds128(v_fq + 16 * j4);
+                const uint64_t nfk2 = pack2(-fk, -fk);
+                c01 = mul2(pack2(f4.x, f4.y), nfk2);
+                c23 = mul2(pack2(f4.z, f4.w), nfk2);
+              } else {
+                c01 = c23 = pack2(-cc, -cc);
+              }
+              float t0, t1, t2, t3;
+              unpack2(fma2(pack2(__uint_as_float(pv[4 * j4 + 0]), __uint_as_float(pv[4 * j4 + 1])), c01, pack2(l4.x, l4.y)), t0, t1);
+              unpack2(fma2(pack2(__uint_as_float(pv[4 * j4 + 2]), __uint_as_float(pv[4 * j4 + 3])), c23, pack2(l4.z, l4.w)), t2, t3);
+              pf[4 * j4 + 0] = ex2_neg(t0);
+              pf[4 * j4 + 1] = ex2_neg(t1);
+              pf[4 * j4 + 2] = ex2_neg(t2);
+              pf[4 * j4 + 3] = ex2_neg(t3);
+            }
           }
-        }
-        if (!SC && !full) {      // diagonal / tail tiles only
+          if (!SC && !full) {      // diagonal / tail tiles only
 #pragma unroll
-          for (int j = 0; j < 64; ++j) pf[j] = visible(j) ? pf[j] : 0.f;
-        }
-        if (TL) {
-          // block-scaled P-hat carrying f_dO(query): one exponent per (this key row, 32 queries)
-          uint32_t ep[2];
+            for (int j = 0; j < QW; ++j) pf[j] = visible(j) ? pf[j] : 0.f;
+          }
+          if (TL) {
+            // block-scaled P-hat carrying f_dO(query): one exponent per (this key row, 32 queries). (Its atom's last reader, the dV
+            // product of the iteration before, has completed when dP^T has: the bytes are written after the passes.)
 #pragma unroll
-          for (int qh = 0; qh < 2; ++qh) {
-            float t[32];
+            for (int qh = 0; qh < QW / 32; ++qh) {
+              float t[32];
+              float am = 0.f;
+#pragma unroll
+              for (int j4 = 0; j4 < 8; ++j4) {
+                const float4 f4 = lds128(v_fdo + 16 * (qh * 8 + j4));
+                const int j = qh * 32 + 4 * j4;
+                unpack2(mul2(pack2(pf[j + 0], pf[j + 1]), pack2(f4.x, f4.y)), t[4 * j4 + 0], t[4 * j4 + 1]);
+                unpack2(mul2(pack2(pf[j + 2], pf[j + 3]), pack2(f4.z, f4.w)), t[4 * j4 + 2], t[4 * j4 + 3]);
+                am = fmax3_abs(fmax3_abs(am, t[4 * j4], t[4 * j4 + 1]), t[4 * j4 + 2], t[4 * j4 + 3]);   // all >= 0
+              }
+              const uint32_t ep = exp448(__float_as_uint(am));
+              epw = __byte_perm(epw, ep, 0x0041);          // (the first block's byte moves down)
+              const float inv = pow2_inv(ep);
+              const uint64_t inv2 = pack2(inv, inv);
+#pragma unroll
+              for (int w = 0; w < 8; ++w) {
+                float a0, a1, a2, a3;
+                unpack2(mul2(pack2(t[4 * w], t[4 * w + 1]), inv2), a0, a1);
+                unpack2(mul2(pack2(t[4 * w + 2], t[4 * w + 3]), inv2), a2, a3);
+                pn[qh * 8 + w] = cvt_e4m3x4(a0, a1, a2, a3);
+              }
+            }
+          } else if constexpr (!SC) {
+#pragma unroll
+            for (int w = 0; w < QW / 4; ++w) pn[w] = cvt_e4m3x4(pf[4 * w], pf[4 * w + 1], pf[4 * w + 2], pf[4 * w + 3]);
+          }
+          if (NP == 1 || ps == 0) {
+            if (it == 0 && pending_kve >= 0) {
+              // the previous item's gradient stores have long read their shared-memory source: its K / V buffer goes back (and, where
+              // the scale atoms share the way out's memory, the whole warpgroup has to know)
+              if (r == 0) { tma_store_wait_read<0>(); mbar_arrive(&bars[BB_KVE + pending_kve]); }
+              pending_kve = -1;
+              if (EPI2) {
+                mbar_arrive_warp(&bars[BB_EPI + x]);
+                if (!(ok = mbar_wait(&bars[BB_EPI + x], epi & 1, p.ctl, abortp, 38))) break;
+                ++epi;
+              }
+            }
+            if (!(ok = mbar_wait(&bars[BB_DP + x], g & 1, p.ctl, abortp, 32))) break;
+            tc_fence_after();
+          }
+
+          // ---- dS = P' (b dP + D''), block exponent per (this warp's 32 keys, 32 queries)
+          FL_TMEM_LD_32(t_dpx + QW * ps, pv);
+          if constexpr (QW == 64) FL_TMEM_LD_32(t_dpx + 32, (pv + 32));
+          tc_wait_ld();
+          uint32_t ebyte[QW / 32];
+#pragma unroll
+          for (int qh = 0; qh < QW / 32; ++qh) {
             float am = 0.f;
 #pragma unroll
             for (int j4 = 0; j4 < 8; ++j4) {
-              const float4 f4 = lds128(v_fdo + 16 * (qh * 8 + j4));
+              const float4 d4 = lds128(v_dpp + 16 * (qh * 8 + j4));
               const int j = qh * 32 + 4 * j4;
-              unpack2(mul2(pack2(pf[j + 0], pf[j + 1]), pack2(f4.x, f4.y)), t[4 * j4 + 0], t[4 * j4 + 1]);
-              unpack2(mul2(pack2(pf[j + 2], pf[j + 3]), pack2(f4.z, f4.w)), t[4 * j4 + 2], t[4 * j4 + 3]);
-              am = fmax3_abs(fmax3_abs(am, t[4 * j4], t[4 * j4 + 1]), t[4 * j4 + 2], t[4 * j4 + 3]);   // all >= 0
+              if (TL) {
+                // b = f_V(key) f_dO(query) per column; the dK side's maximum and codes carry f_Q(query) (kept in pv)
+                const float4 f4 = lds128(v_fdo + 16 * (qh * 8 + j4));
+                const float4 q4 = lds128(v_fq + 16 * (qh * 8 + j4));
+                const uint64_t fv2 = pack2(fv8, fv8);
+                const uint64_t u01 = fma2(pack2(__uint_as_float(pv[j + 0]), __uint_as_float(pv[j + 1])),
+                                          mul2(pack2(f4.x, f4.y), fv2), pack2(d4.x, d4.y));
+                const uint64_t u23 = fma2(pack2(__uint_as_float(pv[j + 2]), __uint_as_float(pv[j + 3])),
+                                          mul2(pack2(f4.z, f4.w), fv2), pack2(d4.z, d4.w));
+                const uint64_t p01 = mul2(pack2(pf[j + 0], pf[j + 1]), u01), p23 = mul2(pack2(pf[j + 2], pf[j + 3]), u23);
+                unpack2(p01, pf[j + 0], pf[j + 1]);
+                unpack2(p23, pf[j + 2], pf[j + 3]);
+                float w0, w1, w2, w3;
+                unpack2(mul2(p01, pack2(q4.x, q4.y)), w0, w1);
+                unpack2(mul2(p23, pack2(q4.z, q4.w)), w2, w3);
+                am = fmax3_abs(fmax3_abs(am, w0, w1), w2, w3);
+                pv[j] = __float_as_uint(w0); pv[j + 1] = __float_as_uint(w1);
+                pv[j + 2] = __float_as_uint(w2); pv[j + 3] = __float_as_uint(w3);
+              } else {
+                // two columns per instruction
+                const uint64_t b2 = pack2(b8[qh], b8[qh]);
+                const uint64_t u01 = fma2(pack2(__uint_as_float(pv[j + 0]), __uint_as_float(pv[j + 1])), b2, pack2(d4.x, d4.y));
+                const uint64_t u23 = fma2(pack2(__uint_as_float(pv[j + 2]), __uint_as_float(pv[j + 3])), b2, pack2(d4.z, d4.w));
+                unpack2(mul2(pack2(pf[j + 0], pf[j + 1]), u01), pf[j + 0], pf[j + 1]);
+                unpack2(mul2(pack2(pf[j + 2], pf[j + 3]), u23), pf[j + 2], pf[j + 3]);
+                am = fmax3_abs(fmax3_abs(am, pf[j], pf[j + 1]), pf[j + 2], pf[j + 3]);
+              }
             }
-            ep[qh] = exp448(__float_as_uint(am));
-            const float inv = pow2_inv(ep[qh]);
-            const uint64_t inv2 = pack2(inv, inv);
+            ebyte[qh] = exp448(warp_max_abs_f32(am));                        // 448 * 2^(e-127) >= amax
+          }
+          if (!full) {      // diagonal / tail tiles only
+            // masked entries hold P' = 0, but their dP^T or D'' may come from rows outside the document (padding or whatever
+            // the buffer held: possibly Inf / NaN), and 0 * NaN is NaN: select again after the multiply. (The maxima above
+            // ignore NaN, so the block exponents are those of the visible entries.)
+#pragma unroll
+            for (int j = 0; j < QW; ++j) {
+              pf[j] = visible(j) ? pf[j] : 0.f;
+              if (TL) pv[j] = visible(j) ? pv[j] : 0u;
+            }
+          }
+#pragma unroll
+          for (int qh = 0; qh < QW / 32; ++qh) {
+            ebw = __byte_perm(ebw, ebyte[qh], 0x0041);     // (as epw)
+            const float inv = pow2_inv(ebyte[qh]);                           // 2^(127 - e)
 #pragma unroll
             for (int w = 0; w < 8; ++w) {
+              const int j0 = qh * 32 + 4 * w;
+              const uint64_t inv2 = pack2(inv, inv);
+              auto ds = [&](int j) { return TL ? __uint_as_float(pv[j]) : pf[j]; };
               float a0, a1, a2, a3;
-              unpack2(mul2(pack2(t[4 * w], t[4 * w + 1]), inv2), a0, a1);
-              unpack2(mul2(pack2(t[4 * w + 2], t[4 * w + 3]), inv2), a2, a3);
-              pw[qh * 8 + w] = cvt_e4m3x4(a0, a1, a2, a3);
+              unpack2(mul2(pack2(ds(j0), ds(j0 + 1)), inv2), a0, a1);
+              unpack2(mul2(pack2(ds(j0 + 2), ds(j0 + 3)), inv2), a2, a3);
+              dn[qh * 8 + w] = cvt_e4m3x4(a0, a1, a2, a3);
             }
           }
-          // (this atom's last reader, the dV product of the iteration before, has completed when dP^T has, which is waited for below;
-          // the words are kept in registers until then)
-          pw_ep = ep[0] | (ep[1] << 8);
-        } else if constexpr (!SC) {
 #pragma unroll
-          for (int w = 0; w < 16; ++w) pw[w] = cvt_e4m3x4(pf[4 * w], pf[4 * w + 1], pf[4 * w + 2], pf[4 * w + 3]);
-        }
-        if (it == 0 && pending_kve >= 0) {
-          // the previous item's gradient stores have long read their shared-memory source: its K / V buffer goes back (and, where
-          // the scale atoms share the way out's memory, the whole warpgroup has to know)
-          if (r == 0) { tma_store_wait_read<0>(); mbar_arrive(&bars[BB_KVE + pending_kve]); }
-          pending_kve = -1;
-          if (EPI2) {
-            mbar_arrive_warp(&bars[BB_EPI + x]);
-            if (!(ok = mbar_wait(&bars[BB_EPI + x], epi & 1, p.ctl, abortp, 38))) break;
-            ++epi;
+          for (int w = 0; w < 16; ++w) {                   // this pass's codes become the last ones
+            pw[w] = w + QW / 4 < 16 ? pw[(w + QW / 4) & 15] : pn[(w + QW / 4) & (QW / 4 - 1)];
+            dsw[w] = w + QW / 4 < 16 ? dsw[(w + QW / 4) & 15] : dn[(w + QW / 4) & (QW / 4 - 1)];
           }
-        }
-
-        // ---- dS = P' (b dP + D''), block exponent per (this warp's 32 keys, 32 queries)
-        if (!(ok = mbar_wait(&bars[BB_DP + x], g & 1, p.ctl, abortp, 32))) break;
-        tc_fence_after();
-        FL_TMEM_LD_32(t_dpx, pv);
-        FL_TMEM_LD_32(t_dpx + 32, (pv + 32));
-        tc_wait_ld();
-        uint32_t ebyte[2];
+          if constexpr (RL) {
+            // the dQ side's own codes: one exponent per (query, this warp's 32 keys); token-local: they carry f_K(key). Per column:
+            // s = the bits of 2^-7 amax rounded up to the next 448 2^k, floored so that the UE8M0 byte is at least 1; the bits of
+            // 2^(127 - e) are its exponent field inverted. (Integer and min / max instructions issue at half rate: the fewer per
+            // column the better.) The columns' values are the same in all lanes; lane = query keeps its own by a selection tree
+            // over the lane's bits (one select per column instead of a comparison and a select).
+            uint32_t tree[5];
 #pragma unroll
-        for (int qh = 0; qh < 2; ++qh) {
-          float am = 0.f;
+            for (int w = 0; w < 8; ++w) {
+              float v[4];
+              uint32_t iv[4];
 #pragma unroll
-          for (int j4 = 0; j4 < 8; ++j4) {
-            const float4 d4 = lds128(v_dpp + 16 * (qh * 8 + j4));
-            const int j = qh * 32 + 4 * j4;
-            if (TL) {
-              // b = f_V(key) f_dO(query) per column; the dK side's maximum carries f_Q(query)
-              const float4 f4 = lds128(v_fdo + 16 * (qh * 8 + j4));
-              const float4 q4 = lds128(v_fq + 16 * (qh * 8 + j4));
-              const uint64_t fv2 = pack2(fv8, fv8);
-              const uint64_t u01 = fma2(pack2(__uint_as_float(pv[j + 0]), __uint_as_float(pv[j + 1])),
-                                        mul2(pack2(f4.x, f4.y), fv2), pack2(d4.x, d4.y));
-              const uint64_t u23 = fma2(pack2(__uint_as_float(pv[j + 2]), __uint_as_float(pv[j + 3])),
-                                        mul2(pack2(f4.z, f4.w), fv2), pack2(d4.z, d4.w));
-              const uint64_t p01 = mul2(pack2(pf[j + 0], pf[j + 1]), u01), p23 = mul2(pack2(pf[j + 2], pf[j + 3]), u23);
-              unpack2(p01, pf[j + 0], pf[j + 1]);
-              unpack2(p23, pf[j + 2], pf[j + 3]);
-              float w0, w1, w2, w3;
-              unpack2(mul2(p01, pack2(q4.x, q4.y)), w0, w1);
-              unpack2(mul2(p23, pack2(q4.z, q4.w)), w2, w3);
-              am = fmax3_abs(fmax3_abs(am, w0, w1), w2, w3);
-            } else {
-              // two columns per instruction
-              const uint64_t b2 = pack2(b8[qh], b8[qh]);
-              const uint64_t u01 = fma2(pack2(__uint_as_float(pv[j + 0]), __uint_as_float(pv[j + 1])), b2, pack2(d4.x, d4.y));
-              const uint64_t u23 = fma2(pack2(__uint_as_float(pv[j + 2]), __uint_as_float(pv[j + 3])), b2, pack2(d4.z, d4.w));
-              unpack2(mul2(pack2(pf[j + 0], pf[j + 1]), u01), pf[j + 0], pf[j + 1]);
-              unpack2(mul2(pack2(pf[j + 2], pf[j + 3]), u23), pf[j + 2], pf[j + 3]);
-              am = fmax3_abs(fmax3_abs(am, pf[j], pf[j + 1]), pf[j + 2], pf[j + 3]);
+              for (int e = 0; e < 4; ++e) {
+                const float a = TL ? pf[4 * w + e] * fk_true : pf[4 * w + e];
+                const int sb = __viaddmax_s32((int)warp_max_abs_f32(a), 0x00200000 - 0x03800000, 2 << 23);
+                iv[e] = ~(uint32_t)sb & 0x7F800000u;
+                v[e] = a * __uint_as_float(iv[e]);
+              }
+              dn[w] = cvt_e4m3x4(v[0], v[1], v[2], v[3]);
+              uint32_t n = (lane & 2) ? ((lane & 1) ? iv[3] : iv[2]) : ((lane & 1) ? iv[1] : iv[0]);
+              if (w & 1) {
+                n = (lane & 4) ? n : tree[0];
+                if ((w & 3) == 3) {
+                  n = (lane & 8) ? n : tree[1];
+                  if (w == 7) tree[3] = (lane & 16) ? n : tree[2];
+                  else tree[2] = n;
+                } else {
+                  tree[1] = n;
+                }
+              } else {
+                tree[0] = n;
+              }
             }
-          }
-          ebyte[qh] = exp448(warp_max_abs_f32(am));                        // 448 * 2^(e-127) >= amax
-        }
-        if (!full) {      // diagonal / tail tiles only
-          // masked entries hold P' = 0, but their dP^T or D'' may come from rows outside the document (padding or whatever
-          // the buffer held: possibly Inf / NaN), and 0 * NaN is NaN: select again after the multiply. (The maxima above
-          // ignore NaN, so the block exponents are those of the visible entries.)
+            // UE8M0 byte e: 2^(127 - e) has the exponent field 254 - e
+            sts8(at_q + 4 * ps, 254u - (tree[3] >> 23) + (ps == 0 ? lq0 : lq1));
 #pragma unroll
-          for (int j = 0; j < 64; ++j) pf[j] = visible(j) ? pf[j] : 0.f;
+            for (int q4 = 0; q4 < 2; ++q4)
+              sts128(ds_row + (((2 * ps + q4) ^ ((r >> 1) & 3)) << 4), dn[4 * q4], dn[4 * q4 + 1], dn[4 * q4 + 2], dn[4 * q4 + 3]);
+          }
         }
+        if (!ok) break;
         // dK's A scales: row = key; bytes = the half's two query blocks
-        sts32(at_row, ebyte[0] | (ebyte[1] << 8));
-        if (TL) sts32(at_row + 1024, pw_ep);
-        if (!RL) {          // dQ's query-side scales: row = query; byte = this warp's key block (+ the row's pre-scale)
-          sts8(at_q, ebyte[0] + lq0);
-          sts8(at_q + 4, ebyte[1] + lq1);
-        }
-        uint32_t dsw[16];
+        sts32(at_row, ebw);
+        if (TL) sts32(at_row + 1024, epw);
+        if constexpr (!RL) {
+          // dQ's query-side scales: row = query; byte = this warp's key block (+ the row's pre-scale)
+          sts8(at_q, (ebw & 0xFF) + lq0);
+          sts8(at_q + 4, (ebw >> 8) + lq1);
+          // the dQ^T product's MN-major B operand: row = key, 64 bytes = 4 chunks of 16 B, 64 B swizzle
 #pragma unroll
-        for (int qh = 0; qh < 2; ++qh) {
-          const float inv = pow2_inv(ebyte[qh]);                           // 2^(127 - e)
-#pragma unroll
-          for (int w = 0; w < 8; ++w) {
-            const int j0 = qh * 32 + 4 * w;
-            const uint64_t inv2 = pack2(inv, inv);
-            float a0, a1, a2, a3;
-            if (TL) {
-              const float4 f4 = lds128(v_fq + 16 * (qh * 8 + w));      // f_Q(query) 2^(127 - e): powers of two, exact, in range
-              unpack2(mul2(pack2(pf[j0], pf[j0 + 1]), mul2(pack2(f4.x, f4.y), inv2)), a0, a1);
-              unpack2(mul2(pack2(pf[j0 + 2], pf[j0 + 3]), mul2(pack2(f4.z, f4.w), inv2)), a2, a3);
-              dsw[qh * 8 + w] = cvt_e4m3x4(a0, a1, a2, a3);
-            } else {
-              unpack2(mul2(pack2(pf[j0], pf[j0 + 1]), inv2), a0, a1);
-              unpack2(mul2(pack2(pf[j0 + 2], pf[j0 + 3]), inv2), a2, a3);
-              dsw[qh * 8 + w] = cvt_e4m3x4(a0, a1, a2, a3);
-            }
-          }
+          for (int q4 = 0; q4 < 4; ++q4)
+            sts128(ds_row + ((q4 ^ ((r >> 1) & 3)) << 4), dsw[4 * q4], dsw[4 * q4 + 1], dsw[4 * q4 + 2], dsw[4 * q4 + 3]);
         }
         // the other half's scores must have left the region (long since, when the halves run half an iteration apart)
         if (x == 0 || it + 1 < n_it || n_it == 1) {
@@ -915,33 +977,6 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                              eq2, eq2, eq2, eq2, ekb_word, ekb_word, ekb_word, ekb_word};
           FL_TMEM_ST_16(t_ox + TO_SFA_P, sf);
         }
-        if (RL) {
-          // the dQ side's own codes: one exponent per (query, this warp's 32 keys); token-local: they carry f_K(key)
-          // per column: t = the exponent field of 2^(e - 119), e the UE8M0 byte with 448 * 2^(e - 127) >= amax, floored
-          // at e = 1; 2^(127 - e) is then the field 262 - (e + 8). (Integer and min / max instructions issue at half rate:
-          // the fewer per column the better.)
-          uint32_t mine[2] = {9u << 23, 9u << 23};
-#pragma unroll
-          for (int w = 0; w < 16; ++w) {
-            float v[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const int j = 4 * w + e;
-              const float a = TL ? pf[j] * fk_true : pf[j];
-              const uint32_t wm = warp_max_abs_f32(a);
-              const uint32_t t = max((wm + 0x00200000u) & 0x7F800000u, 9u << 23);
-              if (lane == (j & 31)) mine[j >> 5] = t;
-              v[e] = a * __uint_as_float(0x83000000u - t);
-            }
-            dsw[w] = cvt_e4m3x4(v[0], v[1], v[2], v[3]);
-          }
-          sts8(at_q, ((mine[0] >> 23) - 8) + lq0);
-          sts8(at_q + 4, ((mine[1] >> 23) - 8) + lq1);
-        }
-        // the dQ^T product's MN-major B operand: row = key, 64 bytes = 4 chunks of 16 B, 64 B swizzle
-#pragma unroll
-        for (int q4 = 0; q4 < 4; ++q4)
-          sts128(ds_row + ((q4 ^ ((r >> 1) & 3)) << 4), dsw[4 * q4], dsw[4 * q4 + 1], dsw[4 * q4 + 2], dsw[4 * q4 + 3]);
         tc_wait_st();
         fence_proxy_async();             // the dS-hat tile and the atoms in shared memory are read by the tensor core (async proxy)
         tc_fence_before();
