@@ -484,9 +484,15 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         const int kb0 = T.kofs + j * 128;                       // document-relative key of column 0
         const bool need_mask = (kb0 + 127 > col_limit) || (kb0 < col_first);    // only on boundary tiles
         if (need_mask) {   // scale first, then mask: the factor product may underflow to zero and 0 * inf is NaN
+          // a bit per column (the code stands in the loop whether it runs or not, and bits take half the instructions)
+          const int lo = col_first - kb0, hi = col_limit - kb0;      // visible: lo <= column <= hi
 #pragma unroll
-          for (int e = 0; e < 128; ++e)
-            s[e] = (kb0 + e > col_limit || kb0 + e < col_first) ? -INFINITY : s[e] * c[e >> 5];
+          for (int kbk = 0; kbk < 4; ++kbk) {
+            const int l = min(max(lo - 32 * kbk, 0), 32), n = min(max(hi - 32 * kbk + 1, 0), 32);
+            const uint32_t see = (uint32_t)((1ull << n) - 1) & ~(uint32_t)((1ull << l) - 1);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) s[32 * kbk + e] = (see & (1u << e)) ? s[32 * kbk + e] * c[kbk] : -INFINITY;
+          }
 #pragma unroll
           for (int kbk = 0; kbk < 4; ++kbk) c[kbk] = 1.f;
         }
@@ -621,58 +627,56 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       }
       const bool by_rows = FULL && p.slot_src && out_n < 128;    // (warpgroup-uniform)
 #pragma unroll 1
-      for (int pass = 0; pass < D / 64; ++pass) {
+      for (int cc = 0; cc < D / 32; ++cc) {              // 32 columns at a time, a box of 64 per store
+        uint32_t ov[32];
+        if (n_i > 0) {                   // (warpgroup-uniform: the tensor-memory loads are warp-collective)
+          FL_TMEM_LD_32(t_o + 32 * cc, ov);
+          tc_wait_ld();
+        } else {
 #pragma unroll
-        for (int cc = 0; cc < 2; ++cc) {
-          uint32_t ov[32];
-          if (n_i > 0) {                 // (warpgroup-uniform: the tensor-memory loads are warp-collective)
-            FL_TMEM_LD_32(t_o + 64 * pass + 32 * cc, ov);
-            tc_wait_ld();
-          } else {
+          for (int e = 0; e < 32; ++e) ov[e] = 0;
+        }
 #pragma unroll
-            for (int e = 0; e < 32; ++e) ov[e] = 0;
-          }
+        for (int q4 = 0; q4 < 4; ++q4) {
+          uint32_t w[4];
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
-            uint32_t w[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              // rows past the end of the document store zeros (a select: what tensor memory holds there is arbitrary)
-              float a, b2;
-              unpack2(mul2(pack2(__uint_as_float(ov[8 * q4 + 2 * e]), __uint_as_float(ov[8 * q4 + 2 * e + 1])),
-                           pack2(inv_l, inv_l)), a, b2);
-              a = row_valid ? a : 0.f;
-              b2 = row_valid ? b2 : 0.f;
-              if (p.out_f16) {
-                __half2 hh = __floats2half2_rn(a, b2);
-                w[e] = *reinterpret_cast<uint32_t*>(&hh);
-              } else {
-                w[e] = pack_bf16x2(a, b2);
-              }
-            }
-            if (by_rows) {
-              if (r < out_n && 64 * pass + 8 * (cc * 4 + q4) < p.d_out)
-                *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) +
-                                          ((size_t)(out_row + r) * p.h + head) * p.d_out + 64 * pass + 8 * (cc * 4 + q4)) =
-                    make_uint4(w[0], w[1], w[2], w[3]);
+          for (int e = 0; e < 4; ++e) {
+            // rows past the end of the document store zeros (a select: what tensor memory holds there is arbitrary)
+            float a, b2;
+            unpack2(mul2(pack2(__uint_as_float(ov[8 * q4 + 2 * e]), __uint_as_float(ov[8 * q4 + 2 * e + 1])),
+                         pack2(inv_l, inv_l)), a, b2);
+            if (p.out_f16) {
+              __half2 hh = __floats2half2_rn(a, b2);
+              w[e] = *reinterpret_cast<uint32_t*>(&hh);
             } else {
-              fwd_sts128(srow + (((cc * 4 + q4) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+              w[e] = pack_bf16x2(a, b2);
             }
+            w[e] = row_valid ? w[e] : 0u;
+          }
+          const int ch = 4 * cc + q4;                    // 16-byte chunk of the row
+          if (by_rows) {
+            if (r < out_n && 8 * ch < p.d_out)
+              *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) +
+                                        ((size_t)(out_row + r) * p.h + head) * p.d_out + 8 * ch) = make_uint4(w[0], w[1], w[2], w[3]);
+          } else {
+            fwd_sts128(srow + (((ch & 7) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
           }
         }
-        if (by_rows) continue;
+        if (by_rows || !(cc & 1)) continue;
         fence_proxy_async();
         mbar_arrive_warp(&bars[B_EPI + i]);             // the warpgroup's four warps have written their rows
         if (!(ok = mbar_wait(&bars[B_EPI + i], epi & 1, p.ctl, abortp, 38))) break;
         ++epi;
         if (r == 0 && out_n == 128) {
-          tma_store_4d(&tm_o, stage, 64 * pass, head, out_row, T.bat);
+          tma_store_4d(&tm_o, stage, 32 * (cc - 1), head, out_row, T.bat);
           tma_store_commit();
           tma_store_wait_read<0>();      // the shared-memory source must outlive the copy; the writes complete with the grid
         }
-        mbar_arrive_warp(&bars[B_EPI + i]);             // the buffer has been read: the next pass / the producer may take it
-        if (!(ok = mbar_wait(&bars[B_EPI + i], epi & 1, p.ctl, abortp, 38))) break;
-        ++epi;
+        if (cc + 1 < D / 32) {
+          mbar_arrive_warp(&bars[B_EPI + i]);           // the buffer has been read: the next box may take it
+          if (!(ok = mbar_wait(&bars[B_EPI + i], epi & 1, p.ctl, abortp, 38))) break;
+          ++epi;
+        }
       }
       if (!ok) break;
       if (row_valid && p.lse) {
