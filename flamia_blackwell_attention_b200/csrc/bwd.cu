@@ -23,9 +23,9 @@
 //   d = 64: block-scaled products need M = 128, so the product is taken the other way round, dQ_x = dS-hat_x K with
 //   A = dS-hat (shared memory, MN-major; its second 64-row block is whatever follows in memory and only fills the
 //   unused rows 64..127 of the result) and B = the K tile; rows = queries, accumulator layout (b, h, s, d)
-//   warps 0-3 compute half 0, warps 4-7 compute half 1 (thread = key row = TMEM lane, 64 query columns)
-//   warps 8-11 dQ reduction (thread = head-dim row)      warp 13 TMA producer
-//   warp 12 UMMA issuer of dQ^T, dV, dK                  warp 14 UMMA issuer of S^T, dP^T
+//   compute warpgroups: two, one per half (64 queries each), or four of 32 queries (bwd_qw); thread = key row = TMEM lane
+//   four warps of dQ reduction (thread = head-dim row), one TMA producer warp
+//   three UMMA issuer warps: dQ^T, dV, dK | S^T | dP^T
 // TMEM: [0,64) / [64,128) S^T_x; [128,256) dV; [256,320) / [320,384) dP^T_x, then dQ^T_x; [384,512) dK.
 // P-hat, dS-hat and the scale tiles of a half go to the OTHER half's S^T columns (P-hat +0, dS-hat +16, scale tiles +32..+56): the
 // compute warps read all 64 scores of a row into registers at once, so their own S^T columns take the next scores while they
@@ -113,8 +113,8 @@ struct BTile {
 // barriers; [2] = one per half, stage or buffer, [3] = one per stage of the score operand's ring
 // (B ring: [stage][half])
 enum { BB_KV = 0, BB_KVE = 2, BB_AFULL = 4, BB_AEMPTY = 7, BB_BFULL = 10, BB_BEMPTY = 14, BB_S = 18, BB_DP = 20, BB_GRANT = 22,
-       BB_DS = 24, BB_DQF = 26, BB_DQE = 28, BB_EPI = 30, BB_R1 = 32, BB_R2 = 33, BB_ACC = 34, BB_ACCFREE = 35, BB_SDR = 36,
-       BB_COUNT = 37 };
+       BB_DS = 24, BB_DQF = 26, BB_DQE = 28, BB_EPI = 30, BB_R1 = 34, BB_R2 = 35, BB_ACC = 36, BB_ACCFREE = 37, BB_SDR = 38,
+       BB_EPX = 39, BB_ROT = 41, BB_COUNT = 42 };
 // TMEM columns; the per-half regions are at + 64 * x
 enum { TC_S = 0, TO_P = 0, TO_DS = 16, TO_SFA_P = 32, TO_SFB_DO = 36, TO_SFB_Q = 40, TO_SFA_DQ = 44, TO_SFA_DK = 48,
        TO_SFB_DQ = 52, TC_DV = 128, TC_DP = 256, TC_DK = 384 };
@@ -247,11 +247,18 @@ struct BwdSmem {
   static_assert(sizeof(BwdMisc) <= 1024 && BYTES <= 227 * 1024);
 };
 
+// Queries per compute warpgroup, and with them the number of compute warpgroups. Two of 64 queries are enough where an iteration
+// is a chain of hand-overs (four lost 6 % to narrower loads and more arrivals). The row-local dQ side adds a warp reduction per
+// column: two warps a scheduler no longer cover its latencies, four of 32 queries do (b2 s4096 h16/4, one B200: row-local
+// 379 -> 292 us, token-local 456 -> 420), and the code of one query block is half as long (59 KB instead of 61 with a rolled loop).
+constexpr int bwd_qw(int var) { return var >= 1 ? 32 : 64; }
+constexpr int bwd_threads(int var) { return (128 / bwd_qw(var) + 2) * 128; }     // + the dQ reduction, + issuers and producer
+
 // FULL: the variants that also serve the rarer call forms (deterministic dQ order, per-query-row pre-scale, packed
 // outputs, the dK mantissa factor), each behind a run-time check of its pointer. A template flag, so that the kernels
 // of the plain calls carry none of that code: the loop is sensitive to every register and instruction added to it.
 template <int D, bool FP4, int VAR, bool SC, bool FULL = false>
-__global__ void __launch_bounds__(512, 1)
+__global__ void __launch_bounds__(bwd_threads(VAR), 1)
 bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                      const __grid_constant__ CUtensorMap tm_acc, const __grid_constant__ CUtensorMap tm_q4,
@@ -267,6 +274,8 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   uint64_t* const bars = misc.bars;
   BTile* const tile_s = misc.tile;
   constexpr bool RL = VAR >= 1, TL = VAR == 2;
+  constexpr int QW = bwd_qw(VAR), NQ = QW / 32, NWG = 128 / QW;      // queries, query blocks per warpgroup; warpgroups
+  constexpr int W_RED = 4 * NWG, W_GRAD = W_RED + 4, W_PROD = W_RED + 5, W_S = W_RED + 6, W_DP = W_RED + 7;    // warps
 
   if (smem_u32(smem) & 1023) {           // (never the case without static shared memory; the swizzles depend on it)
     if (threadIdx.x == 0 && p.ctl.status) atomicCAS(p.ctl.status, 0, FL_DEV_WAIT_TIMEOUT | 63);
@@ -278,23 +287,25 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const int grp = p.grp;
   const int n_items = FULL && p.work ? __ldg(p.work_head).y * p.h_kv : p.n_items;
 
-  if (tid == 13 * 32) {
+  if (tid == W_PROD * 32) {
     misc.abort = 0;
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&bars[BB_KV + i], 1); mbar_init(&bars[BB_KVE + i], 2);      // released by one thread of each compute warpgroup
+      mbar_init(&bars[BB_KV + i], 1); mbar_init(&bars[BB_KVE + i], NWG);      // released by one thread of each compute warpgroup
       mbar_init(&bars[BB_BFULL + 2 * i], 1); mbar_init(&bars[BB_BEMPTY + 2 * i], 1);
       mbar_init(&bars[BB_BFULL + 2 * i + 1], 1); mbar_init(&bars[BB_BEMPTY + 2 * i + 1], 1);
       mbar_init(&bars[BB_S + i], 1); mbar_init(&bars[BB_DP + i], 1);
-      mbar_init(&bars[BB_GRANT + i], 4); mbar_init(&bars[BB_DS + i], 4);      // one arrival per warp
+      mbar_init(&bars[BB_GRANT + i], 2 * NWG); mbar_init(&bars[BB_DS + i], 2 * NWG);      // one arrival per warp of the half
       mbar_init(&bars[BB_DQF + i], 1); mbar_init(&bars[BB_DQE + i], 4);
-      mbar_init(&bars[BB_EPI + i], 4);
+      mbar_init(&bars[BB_EPI + i], 4); mbar_init(&bars[BB_EPI + 2 + i], 4);      // [warpgroup]
+      mbar_init(&bars[BB_EPX + i], EPI2 ? 2 * NWG : 1);
     }
     for (int i = 0; i < 3; ++i) { mbar_init(&bars[BB_AFULL + i], 1); mbar_init(&bars[BB_AEMPTY + i], 1); }
     mbar_init(&bars[BB_R1], 4);
     mbar_init(&bars[BB_R2], 4);
     mbar_init(&bars[BB_ACC], 1);
-    mbar_init(&bars[BB_ACCFREE], 8);
-    mbar_init(&bars[BB_SDR], 4);
+    mbar_init(&bars[BB_ACCFREE], 4 * NWG);
+    mbar_init(&bars[BB_SDR], 2 * NWG);
+    mbar_init(&bars[BB_ROT], 8);
     fence_barrier_init();
     tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v); tma_prefetch_desc(&tm_do);
     tma_prefetch_desc(&tm_acc); tma_prefetch_desc(&tm_dk); tma_prefetch_desc(&tm_dv);
@@ -305,7 +316,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     tmem_relinquish();
   }
   if (!EPI2) {      // (atom bytes that nobody writes are scale 1; with EPI2 no product looks at them)
-    for (int i = tid; i < 2 * SM::ATOM_STRIDE / 4; i += 512) reinterpret_cast<uint32_t*>(smem + SM::ATOMS)[i] = 0x7F7F7F7Fu;
+    for (int i = tid; i < 2 * SM::ATOM_STRIDE / 4; i += bwd_threads(VAR)) reinterpret_cast<uint32_t*>(smem + SM::ATOMS)[i] = 0x7F7F7F7Fu;
     fence_proxy_async();
   }
   tc_fence_before();
@@ -315,8 +326,9 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   volatile int* abortp = &misc.abort;
   // (a status word already set by an earlier launch is not looked at: a kernel that runs after one that gave up does no harm)
 
-  if (warp >= 12) reg_dealloc<80>();     // register budget per warpgroup: 176 / 176 / 80 / 80 (x 128 threads = 64 K)
-  if (warp == 13) {
+  // registers per warpgroup: 2 x 176 + 2 x 80 (= the launch's 512 x 128 / 128), or 4 x 96 + 2 x 48 (= 768 x 80 / 128)
+  if (warp >= W_RED) reg_dealloc<NWG == 2 ? 80 : 48>();
+  if (warp == W_PROD) {
     // =================================================================== TMA producer
     if (lane == 0) {
       int gi = 0;                          // query-tile iterations issued so far, over all items
@@ -388,11 +400,11 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         }
       }
     }
-  } else if (warp == 12) {
+  } else if (warp == W_GRAD) {
     // =================================================================== UMMA issuer of the gradient products
     // The whole warp stays converged through the waits and the descriptor arithmetic (warp-uniform values); one elected
-    // lane issues. Descriptors are built once; the loops only add byte offsets. Two warps issue (this one dQ^T, dV, dK; warp 14
-    // S^T, dP^T): alone, one warp's waits and descriptor moves took longer than the products. Each loop exists once, with the
+    // lane issues. Descriptors are built once; the loops only add byte offsets. Three warps issue (this one dQ^T, dV, dK; the
+    // others S^T and dP^T): alone, one warp's waits and descriptor moves took longer than the products. Each loop exists once, with the
     // half as a run-time value: the roles' loops share the instruction cache.
     const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
     const uint32_t base = smem_u32(smem);
@@ -455,11 +467,14 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       __syncwarp();
       gi += n_it;
     }
-  } else if (warp == 14) {
+  } else if (warp == W_S || (!FP4 && warp == W_DP)) {
     // =================================================================== UMMA issuer of the score products
     // Step t of an item (y = t & 1, j = t >> 1) follows the gradient products of (j, y) and issues S^T_{1-y} of iteration
     // j + 1 + y and dP^T_y of iteration j + 1; steps -3 to -1 are the item's first products, which run while the compute
-    // warpgroups write the previous item's rows.
+    // warpgroups write the previous item's rows. One warp issues S^T, one dP^T: dP^T_y goes out as soon as dQ^T_y has been read
+    // out of its columns (the longest chain of an iteration: dS -> dQ^T -> read -> dP^T -> dS), whatever S^T waits for. FP4: one
+    // warp, S^T first, because its scale columns stand in dP^T's.
+    const bool role_s = FP4 || warp == W_S, role_p = FP4 || warp == W_DP;
     constexpr uint32_t ID_N64 = idesc_f8(128, 64, 0, 0);
     const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
     const uint32_t base = smem_u32(smem);
@@ -479,7 +494,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #pragma unroll 1
       for (int t = -3; t < 2 * n_it - 2; ++t) {
         const int y = t & 1, j = t >> 1;
-        const bool do_s = j + 1 + y < n_it, do_p = j + 1 >= 0 && j + 1 < n_it;
+        const bool do_s = role_s && j + 1 + y < n_it, do_p = role_p && j + 1 >= 0 && j + 1 < n_it;
         const int gs = gi + j + 1 + y, gp = gi + j + 1, xs = 1 - y;
         // the half's dP^T columns hold its previous dQ^T until the reduction warps have read it. FP4: the 16 scale columns of S^T
         // stand in them, too
@@ -487,7 +502,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // The region S^T goes to: its last user were the gradient products of (j, y) (their completion also says that the scores
         // before have been read: the P-hat that took their place waited for that); at an item's start those of the item
         // before, and for half 0's second tile its own first scores.
-        if (t != -2) {
+        if (role_s && t != -2) {
           const int gl = t >= 0 ? gi + j : gi - 1;
           if (t == -1) { if (do_s && !(ok = mbar_wait(&bars[BB_SDR], sdr++ & 1, p.ctl, abortp, 26))) break; }
           else if (gl >= 0 && !(ok = mbar_wait(&bars[BB_BEMPTY + 2 * (gl & 1) + y], (gl >> 1) & 1, p.ctl, abortp, 28))) break;
@@ -537,8 +552,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       }
       gi += n_it;
     }
-  } else if (warp >= 8 && warp < 12) {
-    reg_dealloc<80>();
+  } else if (warp >= W_RED && warp < W_GRAD) {
     // =================================================================== dQ reduction (thread = head-dim row)
     const int r = tid & 127;
     const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
@@ -557,7 +571,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const int it = t >> 1, y = t & 1, g = gi + it;
         if (t > 0 && y == 0 && ++m == T.m_lo + T.n_m) { m = T.m_lo; ++head; }
         // the staging buffer of this half was last read by the reduction of step gt - 2
-        if (tid == 256) tma_store_wait_read<1>();
+        if (tid == W_RED * 32) tma_store_wait_read<1>();
         mbar_arrive_warp(&bars[BB_R1]);
         if (!(ok = mbar_wait(&bars[BB_R1], gt & 1, p.ctl, abortp, 41))) break;
         if (!(ok = mbar_wait(&bars[BB_DQF + y], g & 1, p.ctl, abortp, 40))) break;
@@ -565,37 +579,53 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const uint32_t rowp = smem_u32(smem) + SM::DQ + y * 16384 + r * 128;
         // d = 128: thread = head-dim row of dQ^T, 64 query columns. d = 64: thread = query row (the first 64 lanes; the
         // other two warps hold the product's unused rows), 64 head-dim columns. Either way 64 f16 = one 128-byte row.
-        if (D == 128 || warp < 10) {
-#pragma unroll 1
-          for (int cc = 0; cc < 2; ++cc) {
-            uint32_t v[32];
-            FL_TMEM_LD_32(lane_base + TC_DP + 64 * y + 32 * cc, v);
-            tc_wait_ld();
+        if (D == 128 || warp < W_RED + 2) {
+          uint32_t v[64], w[32];
+          auto narrow = [&](int n) {
 #pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4) {     // 8 f16 = 16 bytes per chunk; 128 B swizzle by the row
-              uint32_t w[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                __half2 hh = __floats2half2_rn(__uint_as_float(v[8 * q4 + 2 * e]), __uint_as_float(v[8 * q4 + 2 * e + 1]));
-                w[e] = *reinterpret_cast<uint32_t*>(&hh);
-              }
-              sts128(rowp + (((cc * 4 + q4) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+            for (int e = 0; e < 32; ++e) {
+              if (e >= n) continue;
+              __half2 hh = __floats2half2_rn(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));
+              w[e] = *reinterpret_cast<uint32_t*>(&hh);
             }
+          };
+          const uint32_t t_dq = lane_base + TC_DP + 64 * y;
+          if constexpr (NWG == 2) {
+            FL_TMEM_LD_32(t_dq, v);
+            FL_TMEM_LD_32(t_dq + 32, (v + 32));
+            tc_wait_ld();
+          } else {                             // (48 registers: half the columns at a time)
+            FL_TMEM_LD_32(t_dq, v);
+            tc_wait_ld();
+            narrow(16);
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4)     // 8 f16 = 16 bytes per chunk; 128 B swizzle by the row
+              sts128(rowp + ((q4 ^ (r & 7)) << 4), w[4 * q4], w[4 * q4 + 1], w[4 * q4 + 2], w[4 * q4 + 3]);
+            FL_TMEM_LD_32(t_dq + 32, v);
+            tc_wait_ld();
           }
+          tc_fence_before();                   // the columns go back (to dP^T) before the rows are stored
+          mbar_arrive_warp(&bars[BB_DQE + y]);
+          narrow(NWG == 2 ? 32 : 16);
+          constexpr int Q0 = NWG == 2 ? 0 : 4;
+#pragma unroll
+          for (int q4 = Q0; q4 < 8; ++q4)
+            sts128(rowp + ((q4 ^ (r & 7)) << 4), w[4 * (q4 - Q0)], w[4 * (q4 - Q0) + 1], w[4 * (q4 - Q0) + 2], w[4 * (q4 - Q0) + 3]);
+        } else {
+          tc_fence_before();
+          mbar_arrive_warp(&bars[BB_DQE + y]);
         }
-        tc_fence_before();
-        mbar_arrive_warp(&bars[BB_DQE + y]);
         fence_proxy_async();
         mbar_arrive_warp(&bars[BB_R2]);
         if (!(ok = mbar_wait(&bars[BB_R2], gt & 1, p.ctl, abortp, 42))) break;
         const bool det = FULL && p.dq_order != nullptr;
         if (!det) {
-          if (tid == 256) {
+          if (tid == W_RED * 32) {
             if (D == 128) tma_reduce_add_4d(&tm_acc, smem + SM::DQ + y * 16384, T.q0 + m * 128 + 64 * y, 0, head, T.bat);
             else tma_reduce_add_4d(&tm_acc, smem + SM::DQ + y * 16384, 0, T.q0 + m * 128 + 64 * y, head, T.bat);
             tma_store_commit();
           }
-        } else if (warp == 8) {                 // (the whole warp stays converged: lane 0 works, the others follow its result)
+        } else if (warp == W_RED) {              // (the whole warp stays converged: lane 0 works, the others follow its result)
           int go = 1;
           int32_t* order = nullptr;
           int rank = 0;
@@ -632,37 +662,36 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       }
       gi += n_it;
     }
-    if (tid == 256) tma_store_wait<0>();
-  } else if (warp < 8) {
-    reg_alloc<176>();
-    // =================================================================== compute (thread = key row, 64 query columns)
-    const int x = warp >> 2;                         // the half this warpgroup owns
+    if (tid == W_RED * 32) tma_store_wait<0>();
+  } else if (warp < W_RED) {
+    reg_alloc<NWG == 2 ? 176 : 96>();
+    // =================================================================== compute (thread = key row, QW query columns)
+    const int x = warp / (2 * NWG);                  // the half this warpgroup works for
+    const int qb = NWG == 2 ? 0 : (warp >> 2) & 1;   // its first 32-query block of the half
     const int wq = warp & 3;                         // lane quadrant = 32-key block of the tile
     const int r = wq * 32 + lane;                    // key row of the tile = TMEM lane
     const uint32_t lane_base = tmem + ((uint32_t)(wq * 32) << 16);
-    const uint32_t t_sx = lane_base + TC_S + 64 * x, t_dpx = lane_base + TC_DP + 64 * x;
+    const uint32_t t_sx = lane_base + TC_S + 64 * x + 32 * qb, t_dpx = lane_base + TC_DP + 64 * x + 32 * qb;
     const uint32_t t_ox = lane_base + TC_S + 64 * (1 - x);           // where P-hat, dS-hat and the scale columns go
     const uint32_t ds_row = smem_u32(smem) + SM::DS + x * 8192 + r * 64;
-    // this thread's words of the scale atoms (row r of a 128-row atom: word (r % 32) * 4 + r / 32; query rows 0..63 likewise)
+    // this thread's bytes of the scale atoms (row r of a 128-row atom: word (r % 32) * 4 + r / 32; query rows 0..63 likewise)
     const uint32_t at = smem_u32(smem) + SM::ATOMS + x * SM::ATOM_STRIDE;
-    const uint32_t at_row = at + lane * 16 + wq * 4, at_q = at + 512 + lane * 16 + wq;
+    const uint32_t at_row = at + lane * 16 + wq * 4 + qb, at_q = at + 512 + lane * 16 + 4 * qb + wq;
+    uint64_t* const bar_epi = &bars[BB_EPI + (warp >> 2)];
     bool ok = true;
-    int gi = 0, epi = 0;                             // iterations so far; uses of the epilogue barrier so far
+    int gi = 0, epi = 0, epx = 0;                    // iterations so far; uses of the epilogue barriers so far
+    [[maybe_unused]] int n_rot = 0;                                   // rotated items so far
     int cg = 0;                                      // grants used so far
-    constexpr int QW = RL ? 32 : 64, NP = 64 / QW;   // queries per pass, passes
     int pending_kve = -1;                            // the K / V buffer whose gradient stores are still to be confirmed
     for (int k = 0; ok; ++k) {
       const int L = bwd_item(k, G, cta, p.zigzag);
       if (L >= n_items) break;
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[BB_KV + kb], (k >> 1) & 1, p.ctl, abortp, 39))) break;
-      // token-local variant: short of registers, so the tile is read from its slot where needed (the slot stays valid until
-      // this item's buffers are released); otherwise a register copy
       const BTile Tcopy = tile_s[kb];
-      const BTile& T = TL ? tile_s[kb] : Tcopy;
+      const BTile& T = NWG == 4 ? tile_s[kb] : Tcopy;
       const int hkv = T.hkv;
       const int n_it = T.n_m * grp;
-      const int krel = T.krel + r;
       const bool key_valid = r < T.nv;
       const size_t bh_k = (size_t)T.bat * p.h_kv + hkv;
       const int kblk = (T.k0 + r) / 32;
@@ -676,291 +705,233 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         for (int kbk = 0; kbk < 4; ++kbk)
           ek_word |= ((__float_as_uint(p.fac_k[bh_k * (p.s_k / 32) + T.k0 / 32 + kbk]) >> 23) & 0xFF) << (8 * kbk);
       }
-      const int vis_from = p.win_r >= 0 ? (krel - T.off - p.win_r) : 0;    // queries in [vis_from, vis_to] see this key
-      const int vis_to = min(p.win_l >= 0 ? (krel - T.off + p.win_l) : 0x7FFFFFFF, T.sq - 1);
-      int m = T.m_lo;
-      for (int it = 0; it < n_it; ++it) {
+      const int krel = T.krel + r - T.off;
+  const int vis_from = p.win_r >= 0 ? krel - p.win_r : 0;    // queries in [vis_from, vis_to] see this key
+  const int vis_to = min(p.win_l >= 0 ? krel + p.win_l : 0x7FFFFFFF, T.sq - 1);
+  int m = T.m_lo;
+  for (int it = 0; it < n_it; ++it) {
         const int g = gi + it, st = g & 1;
-        const int q_first = m * 128 + 64 * x;                              // document-relative query of column 0
-        const bool full = key_valid && (q_first >= vis_from) && (q_first + 63 <= vis_to);
-        // which of the half's queries see this key, a bit each (tested bit by bit the mask takes a third of the instructions that
+        const int q_first = m * 128 + 64 * x + 32 * qb;                    // document-relative query of column 0
+        const bool full = key_valid && (q_first >= vis_from) && (q_first + QW - 1 <= vis_to);
+        // which of the queries see this key, a bit each (tested bit by bit the mask takes a third of the instructions that
         // comparisons take, and they stand in the loop whether they run or not)
         uint32_t see[2] = {0u, 0u};
         if (!full) {
-          const int lo = max(vis_from - q_first, 0), n = key_valid ? max(min(vis_to - q_first + 1, 64) - lo, 0) : 0;
-          const uint64_t b = lo < 64 && n > 0 ? (~0ull >> (64 - n)) << lo : 0ull;
+          const int lo = max(vis_from - q_first, 0), n = key_valid ? max(min(vis_to - q_first + 1, QW) - lo, 0) : 0;
+          const uint64_t b = lo < QW && n > 0 ? (~0ull >> (64 - n)) << lo : 0ull;
           see[0] = (uint32_t)b;
           see[1] = (uint32_t)(b >> 32);
         }
         if (++m == T.m_lo + T.n_m) m = T.m_lo;                              // (the next iteration's from here on)
+        auto visible = [&](int j) { return (see[j >> 5] & (1u << (j & 31))) != 0; };
         if (!(ok = mbar_wait(&bars[BB_BFULL + 2 * st + x], (g >> 1) & 1, p.ctl, abortp, 30))) break;   // row vectors and scalars visible
-        const uint32_t v_vec = smem_u32(smem) + SM::VEC + (2 * st + x) * SM::VEC_HALF;
-        // the f16 pre-scale: one power of two per query tile (folded into K's exponent bytes below), or one per query row
-        // (folded into the dQ side's B scale bytes, whose lanes are the queries)
+        const uint32_t v_lse = smem_u32(smem) + SM::VEC + (2 * st + x) * SM::VEC_HALF + 128 * qb, v_dpp = v_lse + 256;
+        [[maybe_unused]] const uint32_t v_fq = v_lse + 512, v_fdo = v_lse + 768;      // token-local: the per-query factors
         const float4 sc4 = lds128(smem_u32(misc.scal[st][x]));
-        const float bsc = misc.scal[st][x][4];
-        [[maybe_unused]] uint32_t lq0 = 0, lq1 = 0;
-        if (FULL && p.dq_scale_rows) {
-          const float* rp = p.dq_scale_rows + (size_t)T.bat * p.s_q + T.q0 + q_first;
-          lq0 = (uint32_t)((int)((__float_as_uint(rp[lane]) >> 23) & 0xFF) - 127);
-          lq1 = (uint32_t)((int)((__float_as_uint(rp[32 + lane]) >> 23) & 0xFF) - 127);
+        const float sc[5] = {sc4.x, sc4.y, sc4.z, sc4.w, misc.scal[st][x][4]};
+        const uint32_t edo2 = ((__float_as_uint(sc[2]) >> 23) & 0xFF) | (((__float_as_uint(sc[3]) >> 23) & 0xFF) << 8);
+        const uint32_t eq2 = ((__float_as_uint(sc[0]) >> 23) & 0xFF) | (((__float_as_uint(sc[1]) >> 23) & 0xFF) << 8);
+        const uint32_t lb = (uint32_t)((int)((__float_as_uint(sc[4]) >> 23) & 0xFF) - 127) & 0xFF;
+        const uint32_t ekb_word = __vadd4(ek_word, lb * 0x01010101u);
+        uint32_t lq[NQ];                           // a pre-scale per query row: folded into the dQ side's B scale bytes
+#pragma unroll
+        for (int qh = 0; qh < NQ; ++qh) {
+          lq[qh] = 0;
+          if (FULL && p.dq_scale_rows)
+            lq[qh] = (uint32_t)((int)((__float_as_uint(p.dq_scale_rows[(size_t)T.bat * p.s_q + T.q0 + q_first + 32 * qh + lane]) >> 23) & 0xFF) - 127);
         }
         // FP4: the block scales of S were applied by the tensor core; only the softmax scale remains
-        const float cq[2] = {FP4 ? p.scale_log2 : fk * sc4.x, FP4 ? p.scale_log2 : fk * sc4.y}, bq[2] = {fv8 * sc4.z, fv8 * sc4.w};
-        // token-local: unit scale bytes for the Q and dO operands
-        const uint32_t eq2 = ((__float_as_uint(sc4.x) >> 23) & 0xFF) | (((__float_as_uint(sc4.y) >> 23) & 0xFF) << 8);
-        const uint32_t edo2 = ((__float_as_uint(sc4.z) >> 23) & 0xFF) | (((__float_as_uint(sc4.w) >> 23) & 0xFF) << 8);
-        // K's exponent bytes with the power-of-two f16 pre-scale of this query tile folded in (A scale of dQ^T)
-        const uint32_t lb = (uint32_t)((int)((__float_as_uint(bsc) >> 23) & 0xFF) - 127) & 0xFF;
-        const uint32_t ekb_word = __vadd4(ek_word, lb * 0x01010101u);
+        float c[NQ], b8[NQ];
+#pragma unroll
+        for (int qh = 0; qh < NQ; ++qh) {
+          c[qh] = FP4 ? p.scale_log2 : fk * (qb ? sc[1] : sc[qh]);
+          b8[qh] = fv8 * (qb ? sc[3] : sc[2 + qh]);
+        }
 
-        // The 64 queries are worked on QW at a time: all of them in the plain variants; 32 in a rolled loop where the row-local dQ
-        // side's code would not fit the instruction cache twice (token-local: 74 KB of code, of it 35 KB in this loop).
-        uint32_t pw[16], dsw[16];         // P-hat's and dS-hat's codes, kept until the region they go to is free
-        uint32_t epw = 0, ebw = 0;        // exponent bytes of the two query blocks: token-local P-hat's, dS-hat's
+        // ---- P' = 2^(s c - lse2)
         if (!(ok = mbar_wait(&bars[BB_S + x], g & 1, p.ctl, abortp, 31))) break;
         tc_fence_after();
-#pragma unroll 1
-        for (int ps = 0; ps < NP; ++ps) {
-          const uint32_t v_lse = v_vec + 4 * QW * ps, v_dpp = v_lse + 256;
-          [[maybe_unused]] const uint32_t v_fq = v_lse + 512, v_fdo = v_lse + 768;      // token-local: the per-query factors
-          // ---- P' = 2^(s c - lse2)
-          uint32_t pv[QW];
-          FL_TMEM_LD_32(t_sx + QW * ps, pv);
-          if constexpr (QW == 64) FL_TMEM_LD_32(t_sx + 32, (pv + 32));
-          tc_wait_ld();
-          if (NP == 1 || ps + 1 == NP) {
-            // the scores are in registers: this region may take the other half's P-hat and dS-hat (half 0's iteration waits for S1 of
-            // the same iteration; half 1's for S0 of the next one, which is issued before, or of this one where that was the last)
-            tc_fence_before();
-            if (x == 1 || it > 0 || n_it == 1) mbar_arrive_warp(&bars[BB_GRANT + (1 - x)]);
-            if (x == 0 && it == 0 && n_it > 1) mbar_arrive_warp(&bars[BB_SDR]);
-          }
-          // the pass's factors per 32 queries
-          const float c[2] = {NP == 1 || ps == 0 ? cq[0] : cq[1], cq[1]}, b8[2] = {NP == 1 || ps == 0 ? bq[0] : bq[1], bq[1]};
-          const uint32_t seen[2] = {NP == 1 || ps == 0 ? see[0] : see[1], see[1]};
-          auto visible = [&](int j) { return (seen[j >> 5] & (1u << (j & 31))) != 0; };
-          float pf[QW];
-          uint32_t pn[QW / 4], dn[QW / 4];      // this pass's codes
-          if constexpr (SC) {
-            // soft cap: x = cap_a tanh(s c cap_b); P-hat is taken from P' right here, and what stays in pf is
-            // P' (1 - tanh^2), the factor dS needs (the reference's score_mod_bwd, flash_attn/cute/utils.py:178-187)
+        uint32_t pv[QW];
+        FL_TMEM_LD_32(t_sx, pv);
+        if constexpr (NQ == 2) FL_TMEM_LD_32(t_sx + 32, (pv + 32));
+        tc_wait_ld();
+        // the scores are in registers: this region may take the other half's P-hat and dS-hat (half 0's iteration waits for S1 of
+        // the same iteration; half 1's for S0 of the next one, which is issued before, or of this one where that was the last)
+        tc_fence_before();
+        if (x == 1 || it > 0 || n_it == 1) mbar_arrive_warp(&bars[BB_GRANT + (1 - x)]);
+        if (x == 0 && it == 0 && n_it > 1) mbar_arrive_warp(&bars[BB_SDR]);
+        float pf[QW];
+        uint32_t pw[QW / 4];                   // P-hat's codes, kept until the region they go to is free
+        [[maybe_unused]] uint32_t ep = 0;
+        if constexpr (SC) {
+          // soft cap: x = cap_a tanh(s c cap_b); P-hat is taken from P' right here, and what stays in pf is
+          // P' (1 - tanh^2), the factor dS needs (the reference's score_mod_bwd, flash_attn/cute/utils.py:178-187)
 #pragma unroll
-            for (int j4 = 0; j4 < QW / 4; ++j4) {
-              const float4 l4 = lds128(v_lse + 16 * j4);
-              const float cc = c[j4 >> 3];
-              const float l[4] = {l4.x, l4.y, l4.z, l4.w};
-              float pp[4], df[4];
+          for (int j4 = 0; j4 < QW / 4; ++j4) {
+            const float4 l4 = lds128(v_lse + 16 * j4);
+            const float l[4] = {l4.x, l4.y, l4.z, l4.w};
+            float pp[4], df[4];
 #pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float th = tanh_fast(__uint_as_float(pv[4 * j4 + e]) * (cc * p.cap_b));
-                pp[e] = ex2(fmaf(p.cap_a, th, -l[e]));
-                df[e] = fmaf(-th, th, 1.0f);
-                if (!full) pp[e] = visible(4 * j4 + e) ? pp[e] : 0.f;
-              }
-              pn[j4] = cvt_e4m3x4(pp[0], pp[1], pp[2], pp[3]);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) pf[4 * j4 + e] = pp[e] * df[e];
+            for (int e = 0; e < 4; ++e) {
+              const float th = tanh_fast(__uint_as_float(pv[4 * j4 + e]) * (c[j4 >> 3] * p.cap_b));
+              pp[e] = ex2(fmaf(p.cap_a, th, -l[e]));
+              df[e] = fmaf(-th, th, 1.0f);
+              if (!full) pp[e] = visible(4 * j4 + e) ? pp[e] : 0.f;
             }
-          } else {
+            pw[j4] = cvt_e4m3x4(pp[0], pp[1], pp[2], pp[3]);
 #pragma unroll
-            for (int j4 = 0; j4 < QW / 4; ++j4) {
-              const float4 l4 = lds128(v_lse + 16 * j4);
-              const float cc = c[j4 >> 3];
-              // t = lse2 - s c (token-local: c = f_K f_Q(query)), two columns per instruction; P' = 2^-t
-              uint64_t c01, c23;
-              if (TL) {
-                const float4 f4 = lds128(v_fq + 16 * j4);
-                const uint64_t nfk2 = pack2(-fk, -fk);
-                c01 = mul2(pack2(f4.x, f4.y), nfk2);
-                c23 = mul2(pack2(f4.z, f4.w), nfk2);
-              } else {
-                c01 = c23 = pack2(-cc, -cc);
-              }
-              float t0, t1, t2, t3;
-              unpack2(fma2(pack2(__uint_as_float(pv[4 * j4 + 0]), __uint_as_float(pv[4 * j4 + 1])), c01, pack2(l4.x, l4.y)), t0, t1);
-              unpack2(fma2(pack2(__uint_as_float(pv[4 * j4 + 2]), __uint_as_float(pv[4 * j4 + 3])), c23, pack2(l4.z, l4.w)), t2, t3);
-              pf[4 * j4 + 0] = ex2_neg(t0);
-              pf[4 * j4 + 1] = ex2_neg(t1);
-              pf[4 * j4 + 2] = ex2_neg(t2);
-              pf[4 * j4 + 3] = ex2_neg(t3);
-            }
+            for (int e = 0; e < 4; ++e) pf[4 * j4 + e] = pp[e] * df[e];
           }
-          if (!SC && !full) {      // diagonal / tail tiles only
+        } else {
+#pragma unroll
+          for (int j4 = 0; j4 < QW / 4; ++j4) {
+            const float4 l4 = lds128(v_lse + 16 * j4);
+            // t = lse2 - s c (token-local: c = f_K f_Q(query)), two columns per instruction; P' = 2^-t
+            uint64_t c01, c23;
+            if (TL) {
+              const float4 f4 = lds128(v_fq + 16 * j4);
+              const uint64_t nfk2 = pack2(-fk, -fk);
+              c01 = mul2(pack2(f4.x, f4.y), nfk2);
+              c23 = mul2(pack2(f4.z, f4.w), nfk2);
+            } else {
+              c01 = c23 = pack2(-c[j4 >> 3], -c[j4 >> 3]);
+            }
+            float t0, t1, t2, t3;
+            unpack2(fma2(pack2(__uint_as_float(pv[4 * j4 + 0]), __uint_as_float(pv[4 * j4 + 1])), c01, pack2(l4.x, l4.y)), t0, t1);
+            unpack2(fma2(pack2(__uint_as_float(pv[4 * j4 + 2]), __uint_as_float(pv[4 * j4 + 3])), c23, pack2(l4.z, l4.w)), t2, t3);
+            pf[4 * j4 + 0] = ex2_neg(t0);
+            pf[4 * j4 + 1] = ex2_neg(t1);
+            pf[4 * j4 + 2] = ex2_neg(t2);
+            pf[4 * j4 + 3] = ex2_neg(t3);
+          }
+          if (!full) {      // diagonal / tail tiles only
 #pragma unroll
             for (int j = 0; j < QW; ++j) pf[j] = visible(j) ? pf[j] : 0.f;
           }
-          if (TL) {
+          if constexpr (TL) {
+            static_assert(!TL || QW == 32, "one query block per warpgroup");
             // block-scaled P-hat carrying f_dO(query): one exponent per (this key row, 32 queries). (Its atom's last reader, the dV
-            // product of the iteration before, has completed when dP^T has: the bytes are written after the passes.)
-#pragma unroll
-            for (int qh = 0; qh < QW / 32; ++qh) {
-              float t[32];
-              float am = 0.f;
-#pragma unroll
-              for (int j4 = 0; j4 < 8; ++j4) {
-                const float4 f4 = lds128(v_fdo + 16 * (qh * 8 + j4));
-                const int j = qh * 32 + 4 * j4;
-                unpack2(mul2(pack2(pf[j + 0], pf[j + 1]), pack2(f4.x, f4.y)), t[4 * j4 + 0], t[4 * j4 + 1]);
-                unpack2(mul2(pack2(pf[j + 2], pf[j + 3]), pack2(f4.z, f4.w)), t[4 * j4 + 2], t[4 * j4 + 3]);
-                am = fmax3_abs(fmax3_abs(am, t[4 * j4], t[4 * j4 + 1]), t[4 * j4 + 2], t[4 * j4 + 3]);   // all >= 0
-              }
-              const uint32_t ep = exp448(__float_as_uint(am));
-              epw = __byte_perm(epw, ep, 0x0041);          // (the first block's byte moves down)
-              const float inv = pow2_inv(ep);
-              const uint64_t inv2 = pack2(inv, inv);
-#pragma unroll
-              for (int w = 0; w < 8; ++w) {
-                float a0, a1, a2, a3;
-                unpack2(mul2(pack2(t[4 * w], t[4 * w + 1]), inv2), a0, a1);
-                unpack2(mul2(pack2(t[4 * w + 2], t[4 * w + 3]), inv2), a2, a3);
-                pn[qh * 8 + w] = cvt_e4m3x4(a0, a1, a2, a3);
-              }
-            }
-          } else if constexpr (!SC) {
-#pragma unroll
-            for (int w = 0; w < QW / 4; ++w) pn[w] = cvt_e4m3x4(pf[4 * w], pf[4 * w + 1], pf[4 * w + 2], pf[4 * w + 3]);
-          }
-          if (NP == 1 || ps == 0) {
-            if (it == 0 && pending_kve >= 0) {
-              // the previous item's gradient stores have long read their shared-memory source: its K / V buffer goes back (and, where
-              // the scale atoms share the way out's memory, the whole warpgroup has to know)
-              if (r == 0) { tma_store_wait_read<0>(); mbar_arrive(&bars[BB_KVE + pending_kve]); }
-              pending_kve = -1;
-              if (EPI2) {
-                mbar_arrive_warp(&bars[BB_EPI + x]);
-                if (!(ok = mbar_wait(&bars[BB_EPI + x], epi & 1, p.ctl, abortp, 38))) break;
-                ++epi;
-              }
-            }
-            if (!(ok = mbar_wait(&bars[BB_DP + x], g & 1, p.ctl, abortp, 32))) break;
-            tc_fence_after();
-          }
-
-          // ---- dS = P' (b dP + D''), block exponent per (this warp's 32 keys, 32 queries)
-          FL_TMEM_LD_32(t_dpx + QW * ps, pv);
-          if constexpr (QW == 64) FL_TMEM_LD_32(t_dpx + 32, (pv + 32));
-          tc_wait_ld();
-          uint32_t ebyte[QW / 32];
-#pragma unroll
-          for (int qh = 0; qh < QW / 32; ++qh) {
+            // product of the iteration before, has completed when dP^T has: the byte is written below.)
+            float t[32];
             float am = 0.f;
 #pragma unroll
             for (int j4 = 0; j4 < 8; ++j4) {
-              const float4 d4 = lds128(v_dpp + 16 * (qh * 8 + j4));
-              const int j = qh * 32 + 4 * j4;
-              if (TL) {
-                // b = f_V(key) f_dO(query) per column; the dK side's maximum and codes carry f_Q(query) (kept in pv)
-                const float4 f4 = lds128(v_fdo + 16 * (qh * 8 + j4));
-                const float4 q4 = lds128(v_fq + 16 * (qh * 8 + j4));
-                const uint64_t fv2 = pack2(fv8, fv8);
-                const uint64_t u01 = fma2(pack2(__uint_as_float(pv[j + 0]), __uint_as_float(pv[j + 1])),
-                                          mul2(pack2(f4.x, f4.y), fv2), pack2(d4.x, d4.y));
-                const uint64_t u23 = fma2(pack2(__uint_as_float(pv[j + 2]), __uint_as_float(pv[j + 3])),
-                                          mul2(pack2(f4.z, f4.w), fv2), pack2(d4.z, d4.w));
-                const uint64_t p01 = mul2(pack2(pf[j + 0], pf[j + 1]), u01), p23 = mul2(pack2(pf[j + 2], pf[j + 3]), u23);
-                unpack2(p01, pf[j + 0], pf[j + 1]);
-                unpack2(p23, pf[j + 2], pf[j + 3]);
-                float w0, w1, w2, w3;
-                unpack2(mul2(p01, pack2(q4.x, q4.y)), w0, w1);
-                unpack2(mul2(p23, pack2(q4.z, q4.w)), w2, w3);
-                am = fmax3_abs(fmax3_abs(am, w0, w1), w2, w3);
-                pv[j] = __float_as_uint(w0); pv[j + 1] = __float_as_uint(w1);
-                pv[j + 2] = __float_as_uint(w2); pv[j + 3] = __float_as_uint(w3);
-              } else {
-                // two columns per instruction
-                const uint64_t b2 = pack2(b8[qh], b8[qh]);
-                const uint64_t u01 = fma2(pack2(__uint_as_float(pv[j + 0]), __uint_as_float(pv[j + 1])), b2, pack2(d4.x, d4.y));
-                const uint64_t u23 = fma2(pack2(__uint_as_float(pv[j + 2]), __uint_as_float(pv[j + 3])), b2, pack2(d4.z, d4.w));
-                unpack2(mul2(pack2(pf[j + 0], pf[j + 1]), u01), pf[j + 0], pf[j + 1]);
-                unpack2(mul2(pack2(pf[j + 2], pf[j + 3]), u23), pf[j + 2], pf[j + 3]);
-                am = fmax3_abs(fmax3_abs(am, pf[j], pf[j + 1]), pf[j + 2], pf[j + 3]);
-              }
+              const float4 f4 = lds128(v_fdo + 16 * j4);
+              const int j = 4 * j4;
+              unpack2(mul2(pack2(pf[j + 0], pf[j + 1]), pack2(f4.x, f4.y)), t[j + 0], t[j + 1]);
+              unpack2(mul2(pack2(pf[j + 2], pf[j + 3]), pack2(f4.z, f4.w)), t[j + 2], t[j + 3]);
+              am = fmax3_abs(fmax3_abs(am, t[j], t[j + 1]), t[j + 2], t[j + 3]);   // all >= 0
             }
-            ebyte[qh] = exp448(warp_max_abs_f32(am));                        // 448 * 2^(e-127) >= amax
-          }
-          if (!full) {      // diagonal / tail tiles only
-            // masked entries hold P' = 0, but their dP^T or D'' may come from rows outside the document (padding or whatever
-            // the buffer held: possibly Inf / NaN), and 0 * NaN is NaN: select again after the multiply. (The maxima above
-            // ignore NaN, so the block exponents are those of the visible entries.)
-#pragma unroll
-            for (int j = 0; j < QW; ++j) {
-              pf[j] = visible(j) ? pf[j] : 0.f;
-              if (TL) pv[j] = visible(j) ? pv[j] : 0u;
-            }
-          }
-#pragma unroll
-          for (int qh = 0; qh < QW / 32; ++qh) {
-            ebw = __byte_perm(ebw, ebyte[qh], 0x0041);     // (as epw)
-            const float inv = pow2_inv(ebyte[qh]);                           // 2^(127 - e)
+            ep = exp448(__float_as_uint(am));
+            const float inv = pow2_inv(ep);
+            const uint64_t inv2 = pack2(inv, inv);
 #pragma unroll
             for (int w = 0; w < 8; ++w) {
-              const int j0 = qh * 32 + 4 * w;
-              const uint64_t inv2 = pack2(inv, inv);
-              auto ds = [&](int j) { return TL ? __uint_as_float(pv[j]) : pf[j]; };
               float a0, a1, a2, a3;
-              unpack2(mul2(pack2(ds(j0), ds(j0 + 1)), inv2), a0, a1);
-              unpack2(mul2(pack2(ds(j0 + 2), ds(j0 + 3)), inv2), a2, a3);
-              dn[qh * 8 + w] = cvt_e4m3x4(a0, a1, a2, a3);
+              unpack2(mul2(pack2(t[4 * w], t[4 * w + 1]), inv2), a0, a1);
+              unpack2(mul2(pack2(t[4 * w + 2], t[4 * w + 3]), inv2), a2, a3);
+              pw[w] = cvt_e4m3x4(a0, a1, a2, a3);
             }
-          }
+          } else {
 #pragma unroll
-          for (int w = 0; w < 16; ++w) {                   // this pass's codes become the last ones
-            pw[w] = w + QW / 4 < 16 ? pw[(w + QW / 4) & 15] : pn[(w + QW / 4) & (QW / 4 - 1)];
-            dsw[w] = w + QW / 4 < 16 ? dsw[(w + QW / 4) & 15] : dn[(w + QW / 4) & (QW / 4 - 1)];
-          }
-          if constexpr (RL) {
-            // the dQ side's own codes: one exponent per (query, this warp's 32 keys); token-local: they carry f_K(key). Per column:
-            // s = the bits of 2^-7 amax rounded up to the next 448 2^k, floored so that the UE8M0 byte is at least 1; the bits of
-            // 2^(127 - e) are its exponent field inverted. (Integer and min / max instructions issue at half rate: the fewer per
-            // column the better.) The columns' values are the same in all lanes; lane = query keeps its own by a selection tree
-            // over the lane's bits (one select per column instead of a comparison and a select).
-            uint32_t tree[5];
-#pragma unroll
-            for (int w = 0; w < 8; ++w) {
-              float v[4];
-              uint32_t iv[4];
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float a = TL ? pf[4 * w + e] * fk_true : pf[4 * w + e];
-                const int sb = __viaddmax_s32((int)warp_max_abs_f32(a), 0x00200000 - 0x03800000, 2 << 23);
-                iv[e] = ~(uint32_t)sb & 0x7F800000u;
-                v[e] = a * __uint_as_float(iv[e]);
-              }
-              dn[w] = cvt_e4m3x4(v[0], v[1], v[2], v[3]);
-              uint32_t n = (lane & 2) ? ((lane & 1) ? iv[3] : iv[2]) : ((lane & 1) ? iv[1] : iv[0]);
-              if (w & 1) {
-                n = (lane & 4) ? n : tree[0];
-                if ((w & 3) == 3) {
-                  n = (lane & 8) ? n : tree[1];
-                  if (w == 7) tree[3] = (lane & 16) ? n : tree[2];
-                  else tree[2] = n;
-                } else {
-                  tree[1] = n;
-                }
-              } else {
-                tree[0] = n;
-              }
-            }
-            // UE8M0 byte e: 2^(127 - e) has the exponent field 254 - e
-            sts8(at_q + 4 * ps, 254u - (tree[3] >> 23) + (ps == 0 ? lq0 : lq1));
-#pragma unroll
-            for (int q4 = 0; q4 < 2; ++q4)
-              sts128(ds_row + (((2 * ps + q4) ^ ((r >> 1) & 3)) << 4), dn[4 * q4], dn[4 * q4 + 1], dn[4 * q4 + 2], dn[4 * q4 + 3]);
+            for (int w = 0; w < QW / 4; ++w) pw[w] = cvt_e4m3x4(pf[4 * w], pf[4 * w + 1], pf[4 * w + 2], pf[4 * w + 3]);
           }
         }
-        if (!ok) break;
-        // dK's A scales: row = key; bytes = the half's two query blocks
-        sts32(at_row, ebw);
-        if (TL) sts32(at_row + 1024, epw);
-        if constexpr (!RL) {
-          // dQ's query-side scales: row = query; byte = this warp's key block (+ the row's pre-scale)
-          sts8(at_q, (ebw & 0xFF) + lq0);
-          sts8(at_q + 4, (ebw >> 8) + lq1);
-          // the dQ^T product's MN-major B operand: row = key, 64 bytes = 4 chunks of 16 B, 64 B swizzle
+        if (it == 0 && pending_kve >= 0) {
+          // the previous item's gradient stores have long read their shared-memory source: its K / V buffer goes back (and, where
+          // the scale atoms share the way out's memory, every warp of the half has to know)
+          if (r == 0) { tma_store_wait_read<0>(); mbar_arrive(&bars[BB_KVE + pending_kve]); }
+          pending_kve = -1;
+          if (EPI2) {
+            mbar_arrive_warp(&bars[BB_EPX + x]);
+            if (!(ok = mbar_wait(&bars[BB_EPX + x], epx & 1, p.ctl, abortp, 38))) break;
+            ++epx;
+          }
+        }
+
+        // ---- dS = P' (b dP + D''), block exponent per (this warp's 32 keys, 32 queries)
+        if (!(ok = mbar_wait(&bars[BB_DP + x], g & 1, p.ctl, abortp, 32))) break;
+        tc_fence_after();
+        FL_TMEM_LD_32(t_dpx, pv);
+        if constexpr (NQ == 2) FL_TMEM_LD_32(t_dpx + 32, (pv + 32));
+        tc_wait_ld();
+        uint32_t ebyte[NQ];
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4)
-            sts128(ds_row + ((q4 ^ ((r >> 1) & 3)) << 4), dsw[4 * q4], dsw[4 * q4 + 1], dsw[4 * q4 + 2], dsw[4 * q4 + 3]);
+        for (int qh = 0; qh < NQ; ++qh) {
+        float am = 0.f;
+#pragma unroll
+        for (int j4 = 8 * qh; j4 < 8 * qh + 8; ++j4) {
+          const float4 d4 = lds128(v_dpp + 16 * j4);
+          const int j = 4 * j4;
+          if (TL) {
+            // b = f_V(key) f_dO(query) per column; the dK side's maximum and codes carry f_Q(query) (kept in pv)
+            const float4 f4 = lds128(v_fdo + 16 * j4);
+            const float4 q4 = lds128(v_fq + 16 * j4);
+            const uint64_t fv2 = pack2(fv8, fv8);
+            const uint64_t u01 = fma2(pack2(__uint_as_float(pv[j + 0]), __uint_as_float(pv[j + 1])),
+                                      mul2(pack2(f4.x, f4.y), fv2), pack2(d4.x, d4.y));
+            const uint64_t u23 = fma2(pack2(__uint_as_float(pv[j + 2]), __uint_as_float(pv[j + 3])),
+                                      mul2(pack2(f4.z, f4.w), fv2), pack2(d4.z, d4.w));
+            const uint64_t p01 = mul2(pack2(pf[j + 0], pf[j + 1]), u01), p23 = mul2(pack2(pf[j + 2], pf[j + 3]), u23);
+            unpack2(p01, pf[j + 0], pf[j + 1]);
+            unpack2(p23, pf[j + 2], pf[j + 3]);
+            float w0, w1, w2, w3;
+            unpack2(mul2(p01, pack2(q4.x, q4.y)), w0, w1);
+            unpack2(mul2(p23, pack2(q4.z, q4.w)), w2, w3);
+            am = fmax3_abs(fmax3_abs(am, w0, w1), w2, w3);
+            pv[j] = __float_as_uint(w0); pv[j + 1] = __float_as_uint(w1);
+            pv[j + 2] = __float_as_uint(w2); pv[j + 3] = __float_as_uint(w3);
+          } else {
+            // two columns per instruction
+            const uint64_t b2 = pack2(b8[qh], b8[qh]);
+            const uint64_t u01 = fma2(pack2(__uint_as_float(pv[j + 0]), __uint_as_float(pv[j + 1])), b2, pack2(d4.x, d4.y));
+            const uint64_t u23 = fma2(pack2(__uint_as_float(pv[j + 2]), __uint_as_float(pv[j + 3])), b2, pack2(d4.z, d4.w));
+            unpack2(mul2(pack2(pf[j + 0], pf[j + 1]), u01), pf[j + 0], pf[j + 1]);
+            unpack2(mul2(pack2(pf[j + 2], pf[j + 3]), u23), pf[j + 2], pf[j + 3]);
+            am = fmax3_abs(fmax3_abs(am, pf[j], pf[j + 1]), pf[j + 2], pf[j + 3]);
+          }
+        }
+        ebyte[qh] = exp448(warp_max_abs_f32(am));                          // 448 * 2^(e-127) >= amax
+        }
+        if (!full) {      // diagonal / tail tiles only
+          // masked entries hold P' = 0, but their dP^T or D'' may come from rows outside the document (padding or whatever
+          // the buffer held: possibly Inf / NaN), and 0 * NaN is NaN: select again after the multiply. (The maxima above
+          // ignore NaN, so the block exponents are those of the visible entries.)
+#pragma unroll
+          for (int j = 0; j < QW; ++j) {
+            pf[j] = visible(j) ? pf[j] : 0.f;
+            if (TL) pv[j] = visible(j) ? pv[j] : 0u;
+          }
+        }
+        // dK's A scales: row = key; bytes = the half's two query blocks
+        if constexpr (NQ == 2) sts32(at_row, ebyte[0] | (ebyte[1] << 8));
+        else sts8(at_row, ebyte[0]);
+        if (TL) sts8(at_row + 1024, ep);
+        uint32_t dsw[QW / 4];
+#pragma unroll
+        for (int qh = 0; qh < NQ; ++qh) {
+          const float inv = pow2_inv(ebyte[qh]);                           // 2^(127 - e)
+          const uint64_t inv2 = pack2(inv, inv);
+          auto ds = [&](int j) { return TL ? __uint_as_float(pv[j]) : pf[j]; };
+#pragma unroll
+          for (int w = 8 * qh; w < 8 * qh + 8; ++w) {
+            float a0, a1, a2, a3;
+            unpack2(mul2(pack2(ds(4 * w), ds(4 * w + 1)), inv2), a0, a1);
+            unpack2(mul2(pack2(ds(4 * w + 2), ds(4 * w + 3)), inv2), a2, a3);
+            dsw[w] = cvt_e4m3x4(a0, a1, a2, a3);
+          }
+        }
+        // the dQ^T product's MN-major B operand: row = key, 64 bytes = 4 chunks of 16 B, 64 B swizzle
+        auto ds_rows = [&]() {
+#pragma unroll
+          for (int q4 = 0; q4 < 2 * NQ; ++q4)
+            sts128(ds_row + (((2 * qb + q4) ^ ((r >> 1) & 3)) << 4), dsw[4 * q4], dsw[4 * q4 + 1], dsw[4 * q4 + 2], dsw[4 * q4 + 3]);
+        };
+        if constexpr (!RL) {
+          // dQ's query-side scales: row = query; byte = this warp's key block
+#pragma unroll
+          for (int qh = 0; qh < NQ; ++qh) sts8(at_q + 4 * qh, ebyte[qh] + lq[qh]);
+          ds_rows();
         }
         // the other half's scores must have left the region (long since, when the halves run half an iteration apart)
         if (x == 0 || it + 1 < n_it || n_it == 1) {
@@ -968,14 +939,59 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           ++cg;
           tc_fence_after();
         }
-        FL_TMEM_ST_16(t_ox + TO_P, pw);
-        FL_TMEM_ST_16(t_ox + TO_DS, dsw);
         {
           // dV: A = 1 (token-local: the issuer's copy of P-hat's atom follows), B = dO's exponent per 32 queries (bytes = the
-          // half's two K steps); dK: B = Q's exponents; dQ^T: A[head-dim lane] = K's exponents (+ pre-scale) per key block
+          // half's two K steps); dK: B = Q's exponents; dQ^T: A[head-dim lane] = K's exponents per key block with the power-of-two
+          // f16 pre-scale of the query tile folded in
           uint32_t sf[16] = {0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, edo2, edo2, edo2, edo2,
                              eq2, eq2, eq2, eq2, ekb_word, ekb_word, ekb_word, ekb_word};
-          FL_TMEM_ST_16(t_ox + TO_SFA_P, sf);
+          if constexpr (NQ == 2) {
+            FL_TMEM_ST_16(t_ox + TO_P, pw);
+            FL_TMEM_ST_16(t_ox + TO_DS, dsw);
+            FL_TMEM_ST_16(t_ox + TO_SFA_P, sf);
+          } else {
+            FL_TMEM_ST_8(t_ox + TO_P + 8 * qb, pw);
+            FL_TMEM_ST_8(t_ox + TO_DS + 8 * qb, dsw);
+            if (qb == 0) FL_TMEM_ST_8(t_ox + TO_SFA_P, sf);
+            else FL_TMEM_ST_8(t_ox + TO_SFB_Q, (sf + 8));
+          }
+        }
+        if constexpr (RL) {
+          static_assert(!RL || QW == 32, "one query block per warpgroup");
+          // the dQ side's own codes: one exponent per (query, this warp's 32 keys); token-local: they carry f_K(key). Per column:
+          // s = the bits of 2^-7 amax rounded up to the next 448 2^k, floored so that the UE8M0 byte is at least 1; the bits of
+          // 2^(127 - e) are its exponent field inverted. (Integer and min / max instructions issue at half rate: the fewer per
+          // column the better.) The columns' values are the same in all lanes; lane = query keeps its own by a selection tree
+          // over the lane's bits (one select per column instead of a comparison and a select).
+          uint32_t tree[4];
+#pragma unroll
+          for (int w = 0; w < 8; ++w) {
+            float v[4];
+            uint32_t iv[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float a = TL ? pf[4 * w + e] * fk_true : pf[4 * w + e];
+              const int sb = __viaddmax_s32((int)warp_max_abs_f32(a), 0x00200000 - 0x03800000, 2 << 23);
+              iv[e] = ~(uint32_t)sb & 0x7F800000u;
+              v[e] = a * __uint_as_float(iv[e]);
+            }
+            dsw[w] = cvt_e4m3x4(v[0], v[1], v[2], v[3]);
+            uint32_t n = (lane & 2) ? ((lane & 1) ? iv[3] : iv[2]) : ((lane & 1) ? iv[1] : iv[0]);
+            if (w & 1) {
+              n = (lane & 4) ? n : tree[0];
+              if ((w & 3) == 3) {
+                n = (lane & 8) ? n : tree[1];
+                if (w == 7) tree[3] = (lane & 16) ? n : tree[2];
+                else tree[2] = n;
+              } else {
+                tree[1] = n;
+              }
+            } else {
+              tree[0] = n;
+            }
+          }
+          sts8(at_q, 254u - (tree[3] >> 23) + lq[0]);   // UE8M0 byte e: 2^(127 - e) has the exponent field 254 - e
+          ds_rows();
         }
         tc_wait_st();
         fence_proxy_async();             // the dS-hat tile and the atoms in shared memory are read by the tensor core (async proxy)
@@ -985,7 +1001,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       if (!ok) break;
       gi += n_it;
 
-      // ---- item epilogue: warpgroup 0 writes dV, warpgroup 1 writes dK (full rows)
+      // ---- item epilogue: the warpgroups of half 0 write dV, those of half 1 dK (four warpgroups: half of the columns each)
       if (!(ok = mbar_wait(&bars[BB_ACC], k & 1, p.ctl, abortp, 33))) break;
       tc_fence_after();
       {
@@ -993,15 +1009,16 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // dV carries 2^8 (P'), dK the softmax scale (and the mantissa of a Q factor that is no power of two)
         const float mult = (x == 0) ? 0.00390625f : p.softmax_scale * ((FULL && p.dk_mult) ? p.dk_mult[bh_k] : 1.0f);
         const float mk = key_valid ? mult : 0.f;       // rows past the end of the document store zeros
-        // dK of rotated operands: (y H / sqrt(128)) * signs. The butterfly runs in small loops over tensor memory (levels 1 .. 16
-        // inside blocks of 32 columns, then levels 32 and 64 across them on eight columns of each block at a time): unrolled over
-        // a row of registers it was 900 instructions, which pushed the main loops out of the instruction cache at every item.
-        const bool rot = D == 128 && x == 1 && p.had_dk;
-        if (rot && n_it > 0) {
+        // dK of rotated operands: (y H / sqrt(128)) * signs. Levels 1 .. 16 of the butterfly inside the warpgroup's blocks of 32
+        // columns, in place in tensor memory, then (all blocks done) levels 32 and 64 across the blocks on the way out, eight
+        // columns at a time. Small loops: unrolled over a row of registers it was 900 instructions, which pushed the main loops
+        // out of the instruction cache at every item.
+        const bool rot = D == 128 && x == 1 && p.had_dk && n_it > 0;
+        if (rot) {
 #pragma unroll 1
-          for (int cc = 0; cc < 4; ++cc) {
+          for (int cc = 0; cc < 8 / NWG; ++cc) {
             uint32_t v[32];
-            FL_TMEM_LD_32(t_acc + 32 * cc, v);
+            FL_TMEM_LD_32(t_acc + 64 * qb + 32 * cc, v);
             tc_wait_ld();
             uint64_t Y[16];
 #pragma unroll
@@ -1027,50 +1044,30 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
               v[2 * i] = __float_as_uint(a);
               v[2 * i + 1] = __float_as_uint(b2);
             }
-            FL_TMEM_ST_32(t_acc + 32 * cc, v);
+            FL_TMEM_ST_32(t_acc + 64 * qb + 32 * cc, v);
           }
           tc_wait_st();
-#pragma unroll 1
-          for (int c8 = 0; c8 < 4; ++c8) {           // levels 32 and 64: eight columns of every block
-            uint32_t v[4][8];
-#pragma unroll
-            for (int b2 = 0; b2 < 4; ++b2) FL_TMEM_LD_8(t_acc + 32 * b2 + 8 * c8, v[b2]);
-            tc_wait_ld();
-#pragma unroll
-            for (int e = 0; e < 8; e += 2) {
-              uint64_t y[4];
-#pragma unroll
-              for (int b2 = 0; b2 < 4; ++b2) y[b2] = pack2(__uint_as_float(v[b2][e]), __uint_as_float(v[b2][e + 1]));
-              const uint64_t a0 = add2(y[0], y[1]), a1 = sub2(y[0], y[1]), a2 = add2(y[2], y[3]), a3 = sub2(y[2], y[3]);
-              const uint64_t z[4] = {add2(a0, a2), add2(a1, a3), sub2(a0, a2), sub2(a1, a3)};
-#pragma unroll
-              for (int b2 = 0; b2 < 4; ++b2) {
-                float f0, f1;
-                unpack2(z[b2], f0, f1);
-                v[b2][e] = __float_as_uint(f0);
-                v[b2][e + 1] = __float_as_uint(f1);
-              }
-            }
-#pragma unroll
-            for (int b2 = 0; b2 < 4; ++b2) FL_TMEM_ST_8(t_acc + 32 * b2 + 8 * c8, v[b2]);
+          if constexpr (NWG == 4) {
+            tc_fence_before();
+            mbar_arrive_warp(&bars[BB_ROT]);
+            if (!(ok = mbar_wait(&bars[BB_ROT], n_rot & 1, p.ctl, abortp, 37))) break;
+            ++n_rot;
+            tc_fence_after();
           }
-          tc_wait_st();
         }
         // rows -> shared memory (boxes of 64 elements, 128 B swizzle) -> one TMA store per box: a thread's own row
         // written straight to global memory costs 32 separate 128-byte lines per warp instruction. At d = 128 the first
-        // box goes through the finished item's K (warpgroup 0) / V (warpgroup 1) buffer: every product that read it has
-        // completed. The second box has a buffer of its own where shared memory allows (the 8-bit route), so that both
-        // stores are issued together and nobody waits for them here: the thread that issued them confirms that they have
-        // read their source, and only then hands the K / V buffer back to the producer, one query tile into the next item.
+        // box goes through the finished item's K (dV) / V (dK) buffer: every product that read it has completed. The second box
+        // has a buffer of its own where shared memory allows (the plain 8-bit route); otherwise it follows in the first one's.
+        // Nobody waits for the stores here: the thread that issued one confirms that it has read its source, and only then
+        // hands the K / V buffer back to the producer, one query tile into the next item.
         if (pending_kve >= 0) {          // (an item with fewer than two query tiles came in between)
           if (r == 0) { tma_store_wait_read<0>(); mbar_arrive(&bars[BB_KVE + pending_kve]); }
           pending_kve = -1;
-          mbar_arrive_warp(&bars[BB_EPI + x]);
-          if (!(ok = mbar_wait(&bars[BB_EPI + x], epi & 1, p.ctl, abortp, 38))) break;
+          mbar_arrive_warp(bar_epi);
+          if (!(ok = mbar_wait(bar_epi, epi & 1, p.ctl, abortp, 38))) break;
           ++epi;
         }
-        uint8_t* stage0 = smem + ((D == 128) ? ((x == 0 ? SM::K : SM::V) + kb * TILE_BYTES) : (SM::OUT + x * 16384));
-        uint8_t* stage1 = EPI2 ? (smem + SM::OUT + x * 16384) : stage0;
         const CUtensorMap* tm_out = (x == 0) ? &tm_dv : &tm_dk;
         // packed output: the key tile is slot T.k0 / 128 of the aligned buffer; its rows go to the packed rows out_row ..
         // + out_n of the caller's tensor: a full slot as TMA stores, a document's last rows row by row
@@ -1081,86 +1078,131 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         }
         const bool by_rows = FULL && p.slot_src && out_n < 128;   // (CTA-uniform)
         uint16_t* out_base = reinterpret_cast<uint16_t*>(x == 0 ? p.dv : p.dk);
-        const uint32_t srow0 = smem_u32(stage0) + r * 128, srow1 = smem_u32(stage1) + r * 128;
         const float cs = rot ? 0.08838834764831845f * mk : mk;
-        // 32 columns of the row: scaled (with the rotation's signs), as 16 words of two 16-bit values
-        auto block = [&](int cc, uint32_t* w) {
-          uint32_t v[32];
-          if (n_it > 0) {                  // (CTA-uniform: the tensor-memory loads are warp-collective)
-            FL_TMEM_LD_32(t_acc + 32 * cc, v);
-            tc_wait_ld();
-          } else {                         // no query tile saw this key tile
+        // eight columns of both 32-column blocks of a box, finished, as words of two 16-bit values
+        auto octets = [&](int bx, int c8, uint32_t (&w)[2][4]) {
+          uint32_t v[2][8];
 #pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] = 0;
+          for (int b2 = 0; b2 < 2; ++b2) {
+            if (n_it > 0) FL_TMEM_LD_8(t_acc + (rot ? 0 : 64 * bx) + 32 * b2 + 8 * c8, v[b2]);   // (CTA-uniform: warp-collective loads)
+            else {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) v[b2][e] = 0;              // no query tile saw this key tile
+            }
           }
-          const uint32_t neg = !rot ? 0u : cc == 0 ? 0x10D2E03Eu : cc == 1 ? 0xE0D9F0E2u : cc == 2 ? 0x45809F07u : 0x75954FEDu;
+          uint64_t Y[2][4];
+          if (D == 128 && rot) {
+            uint32_t u[2][8];
+            FL_TMEM_LD_8(t_acc + 64 + 8 * c8, u[0]);
+            FL_TMEM_LD_8(t_acc + 96 + 8 * c8, u[1]);
+            tc_wait_ld();
+            const float sg = bx == 0 ? 1.0f : -1.0f;
+            const uint64_t sg2 = pack2(sg, sg);
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            const float c0 = __uint_as_float(__float_as_uint(cs) ^ ((neg << (31 - 2 * e)) & 0x80000000u)),
-                        c1 = __uint_as_float(__float_as_uint(cs) ^ ((neg << (30 - 2 * e)) & 0x80000000u));
-            float f0, f1;
-            unpack2(mul2(pack2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1])), pack2(c0, c1)), f0, f1);
-            if (p.out_f16) {
-              __half2 hh = __floats2half2_rn(f0, f1);
-              w[e] = *reinterpret_cast<uint32_t*>(&hh);
-            } else {
-              w[e] = pack_bf16x2(f0, f1);
+            for (int e = 0; e < 4; ++e) {
+              const uint64_t l0 = pack2(__uint_as_float(v[0][2 * e]), __uint_as_float(v[0][2 * e + 1])),
+                             l1 = pack2(__uint_as_float(v[1][2 * e]), __uint_as_float(v[1][2 * e + 1])),
+                             h0 = pack2(__uint_as_float(u[0][2 * e]), __uint_as_float(u[0][2 * e + 1])),
+                             h1 = pack2(__uint_as_float(u[1][2 * e]), __uint_as_float(u[1][2 * e + 1]));
+              Y[0][e] = fma2(add2(h0, h1), sg2, add2(l0, l1));       // (the products are exact)
+              Y[1][e] = fma2(sub2(h0, h1), sg2, sub2(l0, l1));
+            }
+          } else {
+            tc_wait_ld();
+#pragma unroll
+            for (int b2 = 0; b2 < 2; ++b2)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) Y[b2][e] = pack2(__uint_as_float(v[b2][2 * e]), __uint_as_float(v[b2][2 * e + 1]));
+          }
+#pragma unroll
+          for (int b2 = 0; b2 < 2; ++b2) {
+            const uint32_t neg = !rot ? 0u : (bx == 0 ? (b2 == 0 ? 0x10D2E03Eu : 0xE0D9F0E2u) : (b2 == 0 ? 0x45809F07u : 0x75954FEDu)) >> (8 * c8);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float c0 = __uint_as_float(__float_as_uint(cs) ^ ((neg << (31 - 2 * e)) & 0x80000000u)),
+                          c1 = __uint_as_float(__float_as_uint(cs) ^ ((neg << (30 - 2 * e)) & 0x80000000u));
+              float f0, f1;
+              unpack2(mul2(Y[b2][e], pack2(c0, c1)), f0, f1);
+              if (p.out_f16) {
+                __half2 hh = __floats2half2_rn(f0, f1);
+                w[b2][e] = *reinterpret_cast<uint32_t*>(&hh);
+              } else {
+                w[b2][e] = pack_bf16x2(f0, f1);
+              }
             }
           }
         };
-        auto write = [&](int cc, const uint32_t* w) {
+        auto stage_of = [&](int bx) -> uint8_t* {
+          return smem + (D == 64 || (EPI2 && bx == 1) ? SM::OUT + x * 16384 : (x == 0 ? SM::K : SM::V) + kb * TILE_BYTES);
+        };
+        auto put = [&](int bx, int c8, const uint32_t (&w)[2][4]) {
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
-            const int ch = 4 * cc + q4;            // 16-byte chunk of the row
+          for (int b2 = 0; b2 < 2; ++b2) {
+            const int ch = 8 * bx + 4 * b2 + c8;     // 16-byte chunk of the row
             if (by_rows) {
               if (r < out_n && 8 * ch < p.d_out)
                 *reinterpret_cast<uint4*>(out_base + ((size_t)(out_row + r) * p.h_kv + hkv) * p.d_out + 8 * ch) =
-                    make_uint4(w[4 * q4], w[4 * q4 + 1], w[4 * q4 + 2], w[4 * q4 + 3]);
+                    make_uint4(w[b2][0], w[b2][1], w[b2][2], w[b2][3]);
             } else {
-              sts128((cc < 2 ? srow0 : srow1) + (((ch & 7) ^ (r & 7)) << 4), w[4 * q4], w[4 * q4 + 1], w[4 * q4 + 2], w[4 * q4 + 3]);
+              sts128(smem_u32(stage_of(bx)) + r * 128 + (((ch & 7) ^ (r & 7)) << 4), w[b2][0], w[b2][1], w[b2][2], w[b2][3]);
             }
           }
         };
-        // (the first box's rows, or both boxes' where the second has a buffer of its own)
-#pragma unroll 1
-        for (int cc = 0; cc < (EPI2 ? 4 : 2); ++cc) {
-          uint32_t w[16];
-          block(cc, w);
-          write(cc, w);
-        }
-        // one buffer for two boxes: the second box's words wait in registers, so that the accumulators are free all the same
-        constexpr bool HOLD = D == 128 && !EPI2;
-        [[maybe_unused]] uint32_t held[HOLD ? 32 : 1];
-        if constexpr (HOLD) {
-          block(2, held);
-          block(3, held + 16);
-        }
-        tc_fence_before();
-        mbar_arrive_warp(&bars[BB_ACCFREE]);         // the next item's products may overwrite the accumulators
-        auto announce = [&](int pass) -> bool {      // the warpgroup's four warps have written their rows: out with them
+        auto announce = [&](int bx) -> bool {        // the warpgroup's four warps have written their rows: out with them
+          if (by_rows) return true;
           fence_proxy_async();
-          mbar_arrive_warp(&bars[BB_EPI + x]);
-          if (!mbar_wait(&bars[BB_EPI + x], epi & 1, p.ctl, abortp, 38)) return false;
+          mbar_arrive_warp(bar_epi);
+          if (!mbar_wait(bar_epi, epi & 1, p.ctl, abortp, 38)) return false;
           ++epi;
           if (r == 0 && out_n == 128) {
-            tma_store_4d(tm_out, stage0, 64 * pass, hkv, out_row, T.bat);
-            if (EPI2) tma_store_4d(tm_out, stage1, 64, hkv, out_row, T.bat);
+            tma_store_4d(tm_out, stage_of(bx), 64 * bx, hkv, out_row, T.bat);
             tma_store_commit();
           }
           return true;
         };
-        if (!by_rows && !(ok = announce(0))) break;
-        if constexpr (HOLD) {
-          if (!by_rows) {
-            if (r == 0) tma_store_wait_read<0>();
-            mbar_arrive_warp(&bars[BB_EPI + x]);
-            if (!(ok = mbar_wait(&bars[BB_EPI + x], epi & 1, p.ctl, abortp, 38))) break;
-            ++epi;
+        auto free_acc = [&]() {                      // the accumulators are in registers: the next item's products may overwrite them
+          tc_fence_before();
+          mbar_arrive_warp(&bars[BB_ACCFREE]);
+        };
+        // One buffer for both boxes: two warpgroups take turns (four), or the second box's words wait in registers (two).
+        constexpr bool IN_TURN = D == 128 && !EPI2, HOLD = IN_TURN && NWG == 2;
+        constexpr int N_BOX = NWG == 4 || HOLD ? 1 : D / 64;
+#pragma unroll 1
+        for (int bx = qb; bx < qb + N_BOX; ++bx) {
+          if (IN_TURN && NWG == 4 && bx == 1 && !by_rows) {      // the first box has been read
+            if (!(ok = mbar_wait(&bars[BB_EPX + x], epx & 1, p.ctl, abortp, 38))) break;
+            ++epx;
           }
-          write(2, held);
-          write(3, held + 16);
-          if (!by_rows && !(ok = announce(1))) break;
+#pragma unroll 1
+          for (int c8 = 0; c8 < 4; ++c8) {
+            uint32_t w[2][4];
+            octets(bx, c8, w);
+            if (!HOLD && c8 == 3 && bx + 1 == qb + N_BOX) free_acc();
+            put(bx, c8, w);
+          }
+          [[maybe_unused]] uint32_t held[HOLD ? 4 : 1][2][4];
+          if constexpr (HOLD) {
+#pragma unroll
+            for (int c8 = 0; c8 < 4; ++c8) octets(1, c8, held[c8]);
+            free_acc();
+          }
+          if (!(ok = announce(bx))) break;
+          if constexpr (HOLD) {
+            if (!by_rows) {
+              if (r == 0) tma_store_wait_read<0>();
+              mbar_arrive_warp(bar_epi);
+              if (!(ok = mbar_wait(bar_epi, epi & 1, p.ctl, abortp, 38))) break;
+              ++epi;
+            }
+#pragma unroll
+            for (int c8 = 0; c8 < 4; ++c8) put(1, c8, held[c8]);
+            if (!(ok = announce(1))) break;
+          } else if (IN_TURN && bx == 0 && r == 0 && !by_rows) {
+            tma_store_wait_read<0>();
+            mbar_arrive(&bars[BB_EPX + x]);
+          }
         }
+        if (!ok) break;
         pending_kve = kb;
       }
     }
@@ -1259,7 +1301,7 @@ static int bwd_launch(const fl_attn_args* a, const void* work, void* stream) {
                    : tl ? BwdSmem<128, false, true>::BYTES : BwdSmem<128, false, false>::BYTES;
   auto launch = [&](auto kern) -> int {
     if (int e = set_smem(kern, smem, "fl_bwd: cudaFuncSetAttribute")) return e;
-    kern<<<grid, 512, smem, (cudaStream_t)stream>>>(mq, mk, mv, mdo, macc, mq4, mk4, mdk, mdv, p);
+    kern<<<grid, bwd_threads(rl || tl ? 1 : 0), smem, (cudaStream_t)stream>>>(mq, mk, mv, mdo, macc, mq4, mk4, mdk, mdv, p);
     return FL_OK;
   };
   const bool det = a->dq_order != nullptr;
