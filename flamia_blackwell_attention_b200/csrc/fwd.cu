@@ -411,21 +411,25 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       if (L >= n_items) break;
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[B_Q + kb], (k >> 1) & 1, p.ctl, abortp, 36))) break;
-      const Tile T = tile_s[kb];
-      const int head = T.head, hkv = T.hkv;
+      const Tile& T = tile_s[kb];                       // (valid until this item's Q buffer is released)
       const int n_i = T.n[i];
-      const int qrow = T.q0 + 128 * i + r;              // row inside the batch entry
-      const int qrel = T.qrel + 128 * i + r;            // row inside the document
-      const bool row_valid = (128 * i + r) < T.nq;
-      const size_t bh_q = (size_t)T.bat * p.h + head, bh_k = (size_t)T.bat * p.h_kv + hkv;
-      const float fq = !row_valid ? 0.f
-                       : FP4     ? p.scale_log2
-                       : TL      ? p.fac_q[bh_q * p.s_q + qrow] * p.scale_log2
-                                 : p.fac_q[bh_q * (p.s_q / 32) + qrow / 32] * p.scale_log2;
+      const size_t bh_k = (size_t)T.bat * p.h_kv + T.hkv;
+      float fq;
+      int col_limit, col_first;                         // last and first visible key of this row, counted from the item's first key
+      {
+        const int qrow = T.q0 + 128 * i + r;            // row inside the batch entry
+        const int qrel = T.qrel + 128 * i + r;          // row inside the document
+        const size_t bh_q = (size_t)T.bat * p.h + T.head;
+        fq = (128 * i + r) >= T.nq ? 0.f
+             : FP4                ? p.scale_log2
+             : TL                 ? p.fac_q[bh_q * p.s_q + qrow] * p.scale_log2
+                                  : p.fac_q[bh_q * (p.s_q / 32) + qrow / 32] * p.scale_log2;
+        col_limit = (p.win_r >= 0 ? min(qrel + T.off + p.win_r, T.sk - 1) : T.sk - 1) - T.kofs;
+        col_first = (p.win_l >= 0 ? qrel + T.off - p.win_l : 0) - T.kofs;
+      }
       const float* fk_row = p.fac_k + bh_k * (p.s_k / 32) + T.k0 / 32;
       const float* fv_row = p.fac_v + bh_k * (p.s_k / 32) + T.k0 / 32;
-      const int col_limit = p.win_r >= 0 ? min(qrel + T.off + p.win_r, T.sk - 1) : T.sk - 1;   // last visible key of this row
-      const int col_first = p.win_l >= 0 ? qrel + T.off - p.win_l : 0;                          // first visible key
+      [[maybe_unused]] const size_t tok0 = bh_k * p.s_k + T.k0;       // token-local: the item's first key in the tables
       constexpr float P_OFF = GF ? P_LOG2_448 : P_LOG2_OFFSET;
 
       float m_used = -INFINITY, l_sum = 0.f;
@@ -441,9 +445,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         // token-local: the tile's 128 per-key factors (same addresses for every thread: broadcast loads through L1;
         // staging them in shared memory was twice as slow: 384 broadcast reads per thread and tile saturate the
         // shared-memory port that the tensor core's operand reads also go through)
-        const float4* fk4 = reinterpret_cast<const float4*>(p.fac_k + (TL ? bh_k * p.s_k + T.k0 + j * 128 : 0));
-        const float4* lg4 = reinterpret_cast<const float4*>(TL ? p.tok_lg_v + bh_k * p.s_k + T.k0 + j * 128 : p.fac_v);
-        const float4* rc4 = reinterpret_cast<const float4*>(TL ? p.tok_rcp_v + bh_k * p.s_k + T.k0 + j * 128 : p.fac_v);
+        const float4* fk4 = reinterpret_cast<const float4*>(p.fac_k + (TL ? tok0 + j * 128 : 0));
+        const float4* lg4 = reinterpret_cast<const float4*>(TL ? p.tok_lg_v + tok0 + j * 128 : p.fac_v);
+        const float4* rc4 = reinterpret_cast<const float4*>(TL ? p.tok_rcp_v + tok0 + j * 128 : p.fac_v);
         if (TL) {
           sfv = 0x7F7F7F7Fu;
 #pragma unroll
@@ -481,7 +485,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 #pragma unroll
           for (int kbk = 0; kbk < 4; ++kbk) c[kbk] = 1.f;
         }
-        const int kb0 = T.kofs + j * 128;                       // document-relative key of column 0
+        const int kb0 = j * 128;                                // key of column 0, as the limits
         const bool need_mask = (kb0 + 127 > col_limit) || (kb0 < col_first);    // only on boundary tiles
         if (need_mask) {   // scale first, then mask: the factor product may underflow to zero and 0 * inf is NaN
           // a bit per column (the code stands in the loop whether it runs or not, and bits take half the instructions)
@@ -613,8 +617,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         ++cd;
       }
       tc_fence_after();
+      const int head = T.head, qrow = T.q0 + 128 * i + r;
+      const bool row_valid = (128 * i + r) < T.nq;
       const bool stage_present = T.nq > 128 * i;        // (warpgroup-uniform) an absent stage's rows belong to someone else
-      const float inv_l = ((l_sum > 0.f) ? 1.0f / l_sum : 0.f) * ((FULL && p.o_mult) ? p.o_mult[bh_k] : 1.0f);
+      const float inv_l = ((l_sum > 0.f) ? 1.0f / l_sum : 0.f) * ((FULL && p.o_mult) ? p.o_mult[T.bat * p.h_kv + T.hkv] : 1.0f);
       uint8_t* stage = sQ + (2 * kb + i) * Q_STRIDE;
       const uint32_t srow = smem_u32(stage) + r * 128;
       // packed output: this stage's 128 rows are slot (T.q0 + 128 i) / 128 of the aligned buffer; they go to the packed
@@ -682,7 +688,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       if (row_valid && p.lse) {
         // l carries 2^P_OFF: lse = ln2 * (m - P_OFF + log2 l)
         float v = (l_sum > 0.f) ? (m_used - P_OFF + lg2(l_sum)) * 0.6931471805599453f : -INFINITY;
-        p.lse[bh_q * p.s_q + qrow] = v;
+        p.lse[((size_t)T.bat * p.h + head) * p.s_q + qrow] = v;
       }
       tc_fence_before();                 // this stage's output has left tensor memory before the next item's P-hat is announced
       if (r == 0) mbar_arrive(&bars[B_QE + kb]);
