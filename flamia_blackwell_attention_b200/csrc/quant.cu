@@ -499,7 +499,14 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
 // (tests/test_gpu_quant.py compares them).
 // One launch takes up to three operands (Q, K and V of a call): their tiles form one list, so that a short call pays one
 // launch instead of three and a long one has one tail instead of three.
+// What bounds it is latency, not traffic: a warp works through its rows alone (load, butterfly, maximum, codes), so the CTAs that
+// share an SM have to cover each other. Three of them (d = 128: 168 registers a thread) instead of two need the codes to leave
+// through the tile's own input buffer, whose rows every thread has read for itself; four at d = 64.
+// One B200, before -> after: Q K V of b4 s4096 h16 d128 rotated 63.5 -> 56.5 us (traffic alone: 46), with NVFP4 copies 86 -> 82,
+// 8 x 1000 x 12 heads at d = 64 18.3 -> 14.8.
 static constexpr int QR_STAGES = 2;
+constexpr int qr_ctas(int d) { return d == 128 ? 3 : 4; }
+constexpr int qr_smem(int d) { return QR_STAGES * QT * d * 2 + (d == 128 ? 0 : 2 * QT * d) + 1024; }
 
 struct QuantOperand {
   uint8_t* e_tab;         // outputs as in QuantParams; the codes leave through the operand's tensor map
@@ -528,7 +535,7 @@ struct QuantRowsMaps {
 // MODE as in the four-lane kernel: bit 0 = the E4M3 codes are of the rotated row, bit 1 = also the NVFP4 copy, bit 2 =
 // rotate only the NVFP4 copy. PK: packed source.
 template <int MODE, int D, bool PK>
-__global__ void __launch_bounds__(128, 2)
+__global__ void __launch_bounds__(128, qr_ctas(D))
 quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_constant__ QuantRowsParams p) {
   static_assert(D == 128 || (D == 64 && MODE == 0), "head_dim 64 has no rotation and no NVFP4 copy");
   constexpr int QR_TILE_B = QT * D * 2;            // one 16-bit input tile (boxes of 64 columns: 128-byte rows)
@@ -536,7 +543,9 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
   constexpr bool ROT = (MODE & 1) != 0, NV4 = (MODE & 2) != 0, ROT4 = (MODE & 4) != 0;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* s_out = smem + QR_STAGES * QR_TILE_B;   // two code tiles (128 rows x 128 B, 128 B swizzle)
+  constexpr bool OWN = D == 128;                   // the codes leave through the first box of the tile's own input buffer
+  uint8_t* s_out = smem + (OWN ? 0 : QR_STAGES * QR_TILE_B);   // two code tiles (128 rows x D bytes)
+  constexpr int OUT_STRIDE = OWN ? QR_TILE_B : QR_CODE_B;
   __shared__ __align__(8) uint64_t full[QR_STAGES];
   __shared__ float s_wmax[2][4], s_wsq[2][4];
   __shared__ int abort_s;
@@ -584,6 +593,11 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
     const bool live = !PK || r < p.slot_rows[tile];     // packed source: rows past the slot's document read as zero
     bool ok = mbar_wait(&full[st], (it / QR_STAGES) & 1, p.ctl, abortp, 51);
 
+    // the previous tile's buffer: filled again once its codes have left it (the store was issued a tile ago)
+    if (OWN && tid == 0 && it > 0) {
+      tma_store_wait_read<0>();
+      if (L + (QR_STAGES - 1) * G < p.n_tiles) issue(L + (QR_STAGES - 1) * G, st ^ 1);
+    }
     // ---- the row: D / 8 chunks of 8 elements (element 8 g + e in chunk g), rotation signs applied to the raw bits
     float x[D];
     auto load_row = [&](bool signs) {
@@ -746,7 +760,7 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
     // ---- codes -> this tile's staging buffer (rows of D bytes, the swizzle of that width)
     {
       const uint64_t inv2 = pack2(inv, inv);
-      const uint32_t orow = smem_u32(s_out + par * QR_CODE_B) + r * D;
+      const uint32_t orow = smem_u32(s_out + par * OUT_STRIDE) + r * D;
       const int swz = D == 128 ? (r & 7) : ((r >> 1) & 3);
 #pragma unroll
       for (int c = 0; c < D / 16; ++c) {            // 16 codes per 16-byte chunk
@@ -764,13 +778,13 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
     }
     fence_proxy_async();
     // the store of the previous tile has read its staging buffer (the other one): the next tile may write it
-    if (tid == 0) tma_store_wait_read<0>();
+    if (!OWN && tid == 0) tma_store_wait_read<0>();
     // every thread has read the stage and written its codes; a wait that ran out leaves the loop here, all threads together
     ok = __syncthreads_and(ok ? 1 : 0) != 0;
     if (!ok) break;
     if (tid == 0) {
-      if (L + QR_STAGES * G < p.n_tiles) issue(L + QR_STAGES * G, st);
-      tma_store_4d(&maps.c[oi], s_out + par * QR_CODE_B, 0, head, t0, bat);
+      if (!OWN && L + QR_STAGES * G < p.n_tiles) issue(L + QR_STAGES * G, st);
+      tma_store_4d(&maps.c[oi], s_out + par * OUT_STRIDE, 0, head, t0, bat);
       tma_store_commit();
     }
     // ---- side tables
@@ -803,8 +817,8 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
 
 template <int MODE, int D>
 static int launch_quant_rows(const QuantRowsMaps& maps, const QuantRowsParams& p, cudaStream_t st) {
-  const int smem = QR_STAGES * QT * D * 2 + 2 * QT * D + 1024;
-  const int grid = min(p.n_tiles, sm_count() * 2);
+  const int smem = qr_smem(D);
+  const int grid = min(p.n_tiles, sm_count() * qr_ctas(D));
   auto launch = [&](auto kern) -> int {
     if (int rc = set_smem(kern, smem, "fl_quant_blocks: cudaFuncSetAttribute")) return rc;
     kern<<<grid, 128, smem, st>>>(maps, p);
