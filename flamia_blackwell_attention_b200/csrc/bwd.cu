@@ -285,7 +285,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;
   const int G = gridDim.x, cta = blockIdx.x;
   const int grp = p.grp;
-  const int n_items = FULL && p.work ? __ldg(p.work_head).y * p.h_kv : p.n_items;
+  int n_items = p.n_items;
 
   if (tid == W_PROD * 32) {
     misc.abort = 0;
@@ -310,6 +310,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v); tma_prefetch_desc(&tm_do);
     tma_prefetch_desc(&tm_acc); tma_prefetch_desc(&tm_dk); tma_prefetch_desc(&tm_dv);
     if (FP4) { tma_prefetch_desc(&tm_q4); tma_prefetch_desc(&tm_k4); }
+    grid_dependency();                     // (the others wait at the barrier below)
   }
   if (warp == 0) {
     tmem_alloc(&misc.tmem_base, 512);
@@ -322,6 +323,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (FULL && p.work) n_items = *reinterpret_cast<const volatile int*>(&p.work_head->y) * p.h_kv;
   const uint32_t tmem = misc.tmem_base;
   volatile int* abortp = &misc.abort;
   // (a status word already set by an earlier launch is not looked at: a kernel that runs after one that gave up does no harm)
@@ -1301,7 +1303,7 @@ static int bwd_launch(const fl_attn_args* a, const void* work, void* stream) {
                    : tl ? BwdSmem<128, false, true>::BYTES : BwdSmem<128, false, false>::BYTES;
   auto launch = [&](auto kern) -> int {
     if (int e = set_smem(kern, smem, "fl_bwd: cudaFuncSetAttribute")) return e;
-    kern<<<grid, bwd_threads(rl || tl ? 1 : 0), smem, (cudaStream_t)stream>>>(mq, mk, mv, mdo, macc, mq4, mk4, mdk, mdv, p);
+    launch_after(kern, grid, bwd_threads(rl || tl ? 1 : 0), smem, (cudaStream_t)stream, mq, mk, mv, mdo, macc, mq4, mk4, mdk, mdv, p);
     return FL_OK;
   };
   const bool det = a->dq_order != nullptr;

@@ -195,7 +195,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = gridDim.x, cta = blockIdx.x;
-  const int n_items = FULL && p.work ? __ldg(p.work).x * p.h : p.n_items;
 
   if (tid == 8 * 32) {
     abort_s = 0;
@@ -218,6 +217,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     }
     fence_barrier_init();
     tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v); tma_prefetch_desc(&tm_o);
+    grid_dependency();                     // (the others wait at the barrier below)
   }
   if (warp == 0) {
     tmem_alloc(&tmem_base_s, 512);
@@ -226,6 +226,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  const int n_items = FULL && p.work ? *reinterpret_cast<const volatile int*>(&p.work->x) * p.h : p.n_items;
   const uint32_t tmem = tmem_base_s;
   volatile int* abortp = &abort_s;
   // (a status word already set by an earlier launch is not looked at: a kernel that runs after one that gave up does no harm)
@@ -861,7 +862,7 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   auto launch = [&](auto kern) -> int {
     if (int e = set_smem(kern, smem, "fl_fwd: cudaFuncSetAttribute")) return e;
-    kern<<<grid, 384, smem, st>>>(mq, mk, mv, mo, p);
+    launch_after(kern, grid, 384, smem, st, mq, mk, mv, mo, p);
     return FL_OK;
   };
   const bool sc = a->softcap > 0.f;

@@ -137,6 +137,7 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     fence_barrier_init();
     tma_prefetch_desc(&tm_x);
     if (PRO) tma_prefetch_desc(&tm_o);
+    grid_dependency();
     for (int i = 0; i < QSTAGES; ++i)
       if (blockIdx.x + i * G < p.n_tiles) issue(blockIdx.x + i * G, i);
   }
@@ -148,6 +149,7 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     for (int k = 0; k < 4; ++k) s_sign[qq][j][k] = (((m >> (2 * k)) & 1) << 15) | (((m >> (2 * k + 1)) & 1) << 31);
   }
   __syncthreads();
+  grid_dependency();
 
   // raw 16-byte chunk j of this thread's row (global chunk 4 j + q) from a staged tile
   bool row_live = true;                          // packed source: false for the rows of a slot past its document's end
@@ -573,10 +575,12 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
     abort_s = 0;
     for (int i = 0; i < QR_STAGES; ++i) mbar_init(&full[i], 1);
     fence_barrier_init();
+    grid_dependency();
     for (int i = 0; i < QR_STAGES; ++i)
       if (blockIdx.x + i * G < p.n_tiles) issue(blockIdx.x + i * G, i);
   }
   __syncthreads();
+  grid_dependency();
 
   int it = 0;
   for (int L = blockIdx.x; L < p.n_tiles; L += G, ++it) {
@@ -821,7 +825,7 @@ static int launch_quant_rows(const QuantRowsMaps& maps, const QuantRowsParams& p
   const int grid = min(p.n_tiles, sm_count() * qr_ctas(D));
   auto launch = [&](auto kern) -> int {
     if (int rc = set_smem(kern, smem, "fl_quant_blocks: cudaFuncSetAttribute")) return rc;
-    kern<<<grid, 128, smem, st>>>(maps, p);
+    launch_after(kern, grid, 128, smem, st, maps, p);
     return FL_OK;
   };
   return p.slot_src ? launch(quant_rows_kernel<MODE, D, true>) : launch(quant_rows_kernel<MODE, D, false>);
@@ -835,7 +839,7 @@ static int launch_quant_pk(const CUtensorMap& mx, const CUtensorMap& mo, const Q
   if (int rc = set_smem(kern, smem, "fl_quant_blocks: cudaFuncSetAttribute")) return rc;
   const int per_sm = (PRO || want_t) ? 1 : 2;
   const int grid = min(p.n_tiles, sm_count() * per_sm);
-  kern<<<grid, QTHREADS, smem, st>>>(mx, mo, p);
+  launch_after(kern, grid, QTHREADS, smem, st, mx, mo, p);
   return FL_OK;
 }
 

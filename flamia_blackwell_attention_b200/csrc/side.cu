@@ -19,7 +19,7 @@ __device__ __forceinline__ float pow2_floor_clamped(float x, int lo, int hi) {
 __global__ void dq_prescale_kernel(const float* __restrict__ st_do, const float* __restrict__ st_v,
                                    const float* __restrict__ st_k, int h, int h_kv, int nt_q, int nt_k, int causal_local,
                                    float unit, float* kernel_scale, float* post_scale) {
-  const int bq = blockIdx.y, t = blockIdx.x, tid = threadIdx.x;
+  const int bq = blockIdx.y + grid_dependency(), t = blockIdx.x, tid = threadIdx.x;
   const int q_lo = causal_local ? t : 0, q_hi = causal_local ? t + 1 : nt_q;
   const int k_lo = 0, k_hi = causal_local ? min(t + 1 + max(nt_k - nt_q, 0), nt_k) : nt_k;
   float dn = 0.f, vn = 0.f, km = 0.f;
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(128) dq_post_rows64_kernel(const __half* __res
                                                              const int32_t* __restrict__ slot_src,
                                                              const int32_t* __restrict__ slot_rows) {
   constexpr int D = 64, CPR = D / 8;
-  const int tile = blockIdx.x, head = blockIdx.y, bat = blockIdx.z, tid = threadIdx.x;
+  const int tile = blockIdx.x + grid_dependency(), head = blockIdx.y, bat = blockIdx.z, tid = threadIdx.x;
   const int t0 = tile * 128;
   if (head_mult) mult *= head_mult[(size_t)bat * h + head];
   const __half* src = acc + (((size_t)bat * h + head) * s + t0) * D;
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(128) dq_post_t128_kernel(const __grid_constant
   uint8_t* s_out = sm + 32768;         // 128 token rows x (256 + 16) B
   __shared__ __align__(8) uint64_t bar;
   __shared__ int abort_s;
-  const int tile = blockIdx.x, head = blockIdx.y, bat = blockIdx.z, tid = threadIdx.x;
+  const int tile = blockIdx.x + grid_dependency(), head = blockIdx.y, bat = blockIdx.z, tid = threadIdx.x;
   const int t0 = tile * 128;
   if (tid == 0) {
     abort_s = 0;
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(DT_THREADS) doc_tables_kernel(const int32_t* _
                                                                 int32_t* __restrict__ slot_src, int32_t* __restrict__ slot_rows) {
   __shared__ int s_warp[DT_THREADS / 32];
   __shared__ int s_src[DT_SLOTS], s_rows[DT_SLOTS];      // first source row of the slot, real rows from there
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x + grid_dependency(), lane = tid & 31, warp = tid >> 5;
   const int slot0 = blockIdx.x * DT_SLOTS, n_slots = min(DT_SLOTS, capacity / 128 - slot0);
   if (tid < DT_SLOTS) { s_src[tid] = -1; s_rows[tid] = 0; }
   auto doc_len = [&](int i) { return cu ? cu[i + 1] - cu[i] : fixed_len; };
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(DW_THREADS) doc_work_kernel(const int32_t* __r
                                                               int n_docs, int capacity, int win_l, int win_r, int ordered,
                                                               int4* __restrict__ work, int* status) {
   __shared__ int s_bin[2][DW_BINS], s_warp[2][32], s_mark[32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x + grid_dependency(), lane = tid & 31, warp = tid >> 5;
   const int T = capacity / 128;
   int* mark = reinterpret_cast<int*>(work + 1 + 2 * T);
   for (int t = tid; t < T; t += DW_THREADS) mark[t] = -1;
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(DW_THREADS) doc_work_kernel(const int32_t* __r
 __global__ void __launch_bounds__(128) unpack_lse_kernel(const float* __restrict__ lse, const int32_t* __restrict__ slot_src,
                                                          const int32_t* __restrict__ slot_rows, int capacity, int h, int seq,
                                                          float* __restrict__ out) {
-  const int slot = blockIdx.x, head = blockIdx.y, r = threadIdx.x;
+  const int slot = blockIdx.x + grid_dependency(), head = blockIdx.y, r = threadIdx.x;
   if (slot_src[slot] < 0 || r >= slot_rows[slot]) return;
   const int g = slot_src[slot] + r;
   out[((size_t)(g / seq) * h + head) * seq + g % seq] = lse[(size_t)head * capacity + slot * 128 + r];
@@ -486,7 +486,7 @@ extern "C" int fl_dq_prescale(const float* stats_do, const float* stats_v, const
   if (!stats_do || !stats_v || !stats_k || !kernel_scale || !post_scale || b <= 0 || nt_q <= 0 || nt_k <= 0)
     return FL_ERR_BAD_ARG;
   const int threads = causal_local ? 128 : 1024;
-  dq_prescale_kernel<<<dim3(causal_local ? nt_q : 1, b), threads, 0, (cudaStream_t)stream>>>(stats_do, stats_v, stats_k, h, h_kv, nt_q, nt_k,
+  launch_after(dq_prescale_kernel, dim3(causal_local ? nt_q : 1, b), threads, 0, (cudaStream_t)stream, stats_do, stats_v, stats_k, h, h_kv, nt_q, nt_k,
                                                                       causal_local, unit, kernel_scale, post_scale);
   return launch_result("fl_dq_prescale: kernel launch");
 }
@@ -510,10 +510,10 @@ static int dq_post_launch(const void* dq_acc, const float* post_scale, float mul
     if (rc) return rc;
     const int sm = 32768 + 128 * 272 + 1024;
     if (int e = set_smem(dq_post_t128_kernel, sm, "fl_dq_post: cudaFuncSetAttribute")) return e;
-    dq_post_t128_kernel<<<grid, 128, sm, st>>>(macc, post_scale, (uint16_t*)dq, s, h, d_out, mult, unrotate, out_f16, per_row,
+    launch_after(dq_post_t128_kernel, grid, 128, sm, st, macc, post_scale, (uint16_t*)dq, s, h, d_out, mult, unrotate, out_f16, per_row,
                                                head_mult, slot_src, slot_rows);
   } else {
-    dq_post_rows64_kernel<<<grid, 128, 0, st>>>((const __half*)dq_acc, post_scale, (uint16_t*)dq, s, h, d_out, mult, out_f16,
+    launch_after(dq_post_rows64_kernel, grid, 128, 0, st, (const __half*)dq_acc, post_scale, (uint16_t*)dq, s, h, d_out, mult, out_f16,
                                                 per_row, head_mult, slot_src, slot_rows);
   }
   return launch_result("fl_dq_post: kernel launch");
@@ -561,7 +561,7 @@ extern "C" int fl_dq_prescale_rows(const float* row_do, float* row_v, float* row
 namespace fl {
 // lg = log2 f, rcp = 1 / f for power-of-two factors: exponent-field arithmetic, exact
 __global__ void token_aux_kernel(const float* __restrict__ f, long long n, float* __restrict__ lg, float* __restrict__ rcp) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x + grid_dependency();
   if (i >= n) return;
   const uint32_t bits = __float_as_uint(f[i]) & 0x7F800000u;
   lg[i] = (float)((int)(bits >> 23) - 127);
@@ -573,7 +573,7 @@ extern "C" int fl_token_aux(const float* factors, int64_t n, float* lg, float* r
   using namespace fl;
   if (!factors || !lg || !rcp || n <= 0) return FL_ERR_BAD_ARG;
   if ((n + 255) / 256 > 0x7FFFFFFF) return FL_ERR_TOO_LARGE;
-  token_aux_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(factors, (long long)n, lg, rcp);
+  launch_after(token_aux_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, factors, (long long)n, lg, rcp);
   return launch_result("fl_token_aux: kernel launch");
 }
 
@@ -594,7 +594,7 @@ extern "C" int fl_doc_tables(const int32_t* cu, int32_t n_docs, int32_t fixed_le
       (!cu && (fixed_len <= 0 || (long long)fixed_len * n_docs > total)))
     return FL_ERR_BAD_ARG;
   const int grid = (capacity / 128 + DT_SLOTS - 1) / DT_SLOTS;
-  doc_tables_kernel<<<grid, DT_THREADS, 0, (cudaStream_t)stream>>>(cu, n_docs, fixed_len, total, capacity, start, len, row_map, slot_src,
+  launch_after(doc_tables_kernel, grid, DT_THREADS, 0, (cudaStream_t)stream, cu, n_docs, fixed_len, total, capacity, start, len, row_map, slot_src,
                                                                    slot_rows);
   return launch_result("fl_doc_tables: kernel launch");
 }
@@ -603,7 +603,7 @@ extern "C" int fl_doc_work(const int32_t* doc_start, const int32_t* doc_len, int
                            int32_t window_right_p1, int32_t causal, int32_t ordered, int32_t* work, int32_t* status, void* stream) {
   using namespace fl;
   if (!doc_start || !doc_len || !work || n_docs <= 0 || capacity <= 0 || (capacity % 128)) return FL_ERR_BAD_ARG;
-  doc_work_kernel<<<1, DW_THREADS, 0, (cudaStream_t)stream>>>(doc_start, doc_len, n_docs, capacity, window_left_p1 - 1,
+  launch_after(doc_work_kernel, 1, DW_THREADS, 0, (cudaStream_t)stream, doc_start, doc_len, n_docs, capacity, window_left_p1 - 1,
                                                               causal ? 0 : window_right_p1 - 1, ordered, (int4*)work, status);
   return launch_result("fl_doc_work: kernel launch");
 }
@@ -613,7 +613,7 @@ extern "C" int fl_unpack_lse(const float* lse, const int32_t* slot_src, const in
   using namespace fl;
   if (!lse || !slot_src || !slot_rows || !out || capacity <= 0 || (capacity % 128) || h <= 0 || seq <= 0 || total % seq) return FL_ERR_BAD_ARG;
   if (h > 65535) return FL_ERR_TOO_LARGE;
-  unpack_lse_kernel<<<dim3(capacity / 128, h), 128, 0, (cudaStream_t)stream>>>(lse, slot_src, slot_rows, capacity, h, seq, out);
+  launch_after(unpack_lse_kernel, dim3(capacity / 128, h), 128, 0, (cudaStream_t)stream, lse, slot_src, slot_rows, capacity, h, seq, out);
   return launch_result("fl_unpack_lse: kernel launch");
 }
 
