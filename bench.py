@@ -201,7 +201,7 @@ def measure_route(fn, route, causal, tensors, args, world, dist, K, clock_gpu=No
     for _ in range(W):
         step()
     barrier()
-    # ---- the timed steps replay one captured step (8 launches): no host launch gaps
+    # ---- the timed steps replay one captured step (6 launches): no host launch gaps
     run_step, mode = step, "eager"
     if not args.no_graph:
         try:
@@ -338,7 +338,7 @@ def main():
             fn(pq, pk, pv, causal=causal).backward(pg)
         torch.cuda.synchronize()
         F.check_status()
-        print(json.dumps({"profile_case": f"b2 s{S} h{H} d{D}", "steps": args.warmup + args.steps, "launches_per_step": 8}))
+        print(json.dumps({"profile_case": f"b2 s{S} h{H} d{D}", "steps": args.warmup + args.steps, "launches_per_step": 6}))
         return
     W = max(args.warmup, 3)
 
@@ -486,7 +486,7 @@ def main():
                     "copy_probe": {"h2d_gbs_slowest_rank": h2d_gbs, "d2h_gbs_slowest_rank": d2h_gbs,
                                    "what": "pinned cudaMemcpyAsync of the same buffers, both directions at once on every "
                                            "rank, no kernels: the ceiling of the end-to-end figure"}},
-            "gpu_launches": 8 * n_timed,
+            "gpu_launches": 6 * n_timed,
             "clocks": top["clocks"],
             "status_word": 0,
         }
