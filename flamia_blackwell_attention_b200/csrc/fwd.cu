@@ -31,10 +31,6 @@
 //   warps 4-7   softmax stage 1                                               warp 9  UMMA issuer
 //   warps 10-11 idle: they complete the third warpgroup, which hands its registers to the softmax warpgroups
 //   (setmaxnreg 216 / 216 / 72 of a 168-register launch: a softmax thread keeps 128 scores and 32 packed words live)
-// Token-local: steps of 64 keys instead of 128, two score buffers per stage (S0a S0b S1a S1b) and an issuer per stage (warps 9, 10):
-// the scores of the next step are ready when a step ends, and a thread holds 64 scores instead of 128. With 128 its per-key tables
-// made it spill; there is hardly an L1 left beside 200 KB of shared memory. (b2 s4096 h16/4, one B200: 228 -> 196 us. The other
-// variants, which do not spill, lose 5 to 9 %: they pay the hand-overs of a step twice.)
 // TMEM (512 columns): S0 [0,128) S1 [128,256) O0 [256,384) O1 [384,512); P-hat overlays columns [0,32) of its S, the
 // P.V scale factors columns [32,40).
 // Output rows leave through the finished item's own Q tile buffer (dead once the stage's last product has completed): 64
@@ -53,7 +49,6 @@ static constexpr int Q_STRIDE = 16384;            // bytes between Q tile buffer
 static constexpr float P_LOG2_OFFSET = 4.0f;      // row frame: P-hat = 2^(x - m + 4) keeps small probabilities out of E4M3 subnormals
 static constexpr float P_LOG2_448 = 8.807354922057604f;   // group frame: the row maximum sits at 448 before the group bias
 static constexpr long long STAGE_SKEW_CLOCKS = 2000;   // about half a softmax period; see the UMMA issuer's prologue
-static constexpr long long STEP_SKEW_CLOCKS = 500;      // the same for steps of 64 keys
 static constexpr float RESCALE_THRESHOLD = 4.0f;  // the running maximum is refreshed only when it grew by more than this
 
 struct FwdParams {
@@ -99,13 +94,13 @@ struct Tile {
   int off;    // causal alignment: key j (document-relative) is visible to query i iff j <= i + off
   int qrel;   // document-relative index of row q0
   int kofs;   // document-relative key of the first key row this item loads (a multiple of 128; > 0 under a left window)
-  int n[2];   // steps of KS keys stage 0 / 1 walks: keys [kofs, kmax_i), n_i = ceil((kmax_i - kofs) / KS)
+  int n[2];   // key tiles stage 0 / 1 walks: keys [kofs, kmax_i), n_i = ceil((kmax_i - kofs) / 128)
 };
 
 // barrier indices
 enum { B_Q = 0, B_QE = 2, B_KFULL = 4, B_KEMPTY = B_KFULL + KV_STAGES, B_VFULL = B_KEMPTY + KV_STAGES,
-       B_VEMPTY = B_VFULL + KV_STAGES, B_SFULL = B_VEMPTY + KV_STAGES, B_PFULL = B_SFULL + 4, B_PVDONE = B_PFULL + 4,
-       B_SDRAIN = B_PVDONE + 2, B_EPI = B_SDRAIN + 2, B_COUNT = B_EPI + 2 };      // S and P: [stage][buffer]
+       B_VEMPTY = B_VFULL + KV_STAGES, B_SFULL = B_VEMPTY + KV_STAGES, B_PFULL = B_SFULL + 2, B_PVDONE = B_PFULL + 2,
+       B_SDRAIN = B_PVDONE + 2, B_EPI = B_SDRAIN + 2, B_COUNT = B_EPI + 2 };
 
 template <int N>
 __device__ __forceinline__ void fwd_reg_alloc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -123,7 +118,7 @@ __device__ __forceinline__ int fwd_item(int k, int G, int c, int zigzag) {
 // Work item L -> its block. Causal: blocks slowest and last block first, so that the item index orders the items longest
 // first; heads fastest, so the query heads of a kv group run together and share its K / V tiles in L2. Otherwise blocks
 // fastest: neighbours share their K / V tiles in L2 and every block costs the same.
-template <bool DOCS, int KS>
+template <bool DOCS>
 __device__ __forceinline__ void fwd_decode(const FwdParams& p, int L, Tile& t) {
   if (!DOCS || p.doc_start == nullptr) {
     const int q = p.div_item.div(L), rq = L - q * p.div_item.d;
@@ -163,7 +158,7 @@ __device__ __forceinline__ void fwd_decode(const FwdParams& p, int L, Tile& t) {
     const int rows = min(128, t.nq - 128 * i);             // valid rows of the stage (<= 0: stage absent)
     int kmax = t.sk;
     if (p.win_r >= 0) kmax = min(t.sk, t.qrel + 128 * i + rows + t.off + p.win_r);
-    t.n[i] = (rows > 0 && kmax > t.kofs) ? (kmax - t.kofs + KS - 1) / KS : 0;
+    t.n[i] = (rows > 0 && kmax > t.kofs) ? (kmax - t.kofs + 127) / 128 : 0;
   }
 }
 
@@ -174,7 +169,6 @@ __global__ void __launch_bounds__(384, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
            const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const FwdParams p) {
   constexpr int TILE_BYTES = 128 * D;
-  constexpr int KS = TL ? 64 : 128, NB = 128 / KS, NG = KS / 32;      // keys per step, score buffers per stage, 32-key groups
   constexpr uint64_t SWZ = (D == 128) ? SWZ_128 : SWZ_64;
   constexpr uint32_t SBO = 8 * D;                       // bytes between 8-row groups
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -200,20 +194,18 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     abort_s = 0;
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars[B_Q + i], 1);
-      mbar_init(&bars[B_QE + i], TL ? 4 : 2);    // released by one thread of each softmax warpgroup (and by both issuers)
-      for (int rg = 0; rg < 2; ++rg) {
-        mbar_init(&bars[B_SFULL + 2 * i + rg], 1);
-        mbar_init(&bars[B_PFULL + 2 * i + rg], 4);      // one arrival per softmax warp
-      }
+      mbar_init(&bars[B_QE + i], 2);         // released by one thread of each softmax warpgroup
+      mbar_init(&bars[B_SFULL + i], 1);
+      mbar_init(&bars[B_PFULL + i], 4);      // one arrival per softmax warp
       mbar_init(&bars[B_PVDONE + i], 1);
       mbar_init(&bars[B_SDRAIN + i], 4);
       mbar_init(&bars[B_EPI + i], 4);
     }
     for (int i = 0; i < KV_STAGES; ++i) {
       mbar_init(&bars[B_KFULL + i], 1);
-      mbar_init(&bars[B_KEMPTY + i], NB);      // one release per issuer
+      mbar_init(&bars[B_KEMPTY + i], 1);
       mbar_init(&bars[B_VFULL + i], 1);
-      mbar_init(&bars[B_VEMPTY + i], NB);
+      mbar_init(&bars[B_VEMPTY + i], 1);
     }
     fence_barrier_init();
     tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v); tma_prefetch_desc(&tm_o);
@@ -245,7 +237,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         // output rows out of it
         if (k >= 2 && !(ok = mbar_wait(&bars[B_QE + kb], ((k >> 1) - 1) & 1, p.ctl, abortp, 12))) break;
         Tile t;
-        fwd_decode<FULL, KS>(p, L, t);
+        fwd_decode<FULL>(p, L, t);
         tile_s[kb] = t;
         const int hkv = t.hkv;
         if (t.nq > 0) {
@@ -259,7 +251,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         } else {
           mbar_arrive(&bars[B_Q + kb]);    // an empty block slot: the phase still completes, every role moves on
         }
-        const int n_max = (max(t.n[0], t.n[1]) + NB - 1) / NB;      // key tiles
+        const int n_max = max(t.n[0], t.n[1]);
         for (int j = 0; j < n_max; ++j, ++gj) {
           const int st = gj % KV_STAGES, ph = (gj / KV_STAGES) & 1;
           if (gj >= KV_STAGES && !(ok = mbar_wait(&bars[B_KEMPTY + st], ph ^ 1, p.ctl, abortp, 10))) break;
@@ -275,7 +267,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         }
       }
     }
-  } else if (!TL && warp == 9) {
+  } else if (warp == 9) {
     // =================================================================== UMMA issuer
     // The whole warp stays converged through the waits and the descriptor arithmetic (warp-uniform values); one elected
     // lane issues. Descriptors are built once; the loops only add byte offsets.
@@ -341,7 +333,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         if (n0 > 0) {
           if (!o1 && !(ok = drained(0))) break;
           if (FP4) tc_fence_after();
-          if (elect_one()) { issue_s(0, st0, o1); tc_commit(&bars[B_SFULL]); }
+          if (elect_one()) { issue_s(0, st0, o1); tc_commit(&bars[B_SFULL + 0]); }
           __syncwarp();
           ++cs0;
         }
@@ -355,7 +347,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         if (n1 > 0) {
           if (!o1 && !(ok = drained(1))) break;
           if (FP4) tc_fence_after();
-          if (elect_one()) { issue_s(1, st0, o1); tc_commit(&bars[B_SFULL + 2]); }
+          if (elect_one()) { issue_s(1, st0, o1); tc_commit(&bars[B_SFULL + 1]); }
           __syncwarp();
           ++cs1;
         }
@@ -375,7 +367,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           if (j >= n_i) continue;
           // P-hat(j) of stage i belongs to the stage's latest S product (number cs_i - 1)
           const int ci = i == 0 ? cs0 : cs1;
-          if (!(ok = mbar_wait(&bars[B_PFULL + 2 * i], (ci - 1) & 1, p.ctl, abortp, 23 + i))) break;
+          if (!(ok = mbar_wait(&bars[B_PFULL + i], (ci - 1) & 1, p.ctl, abortp, 23 + i))) break;
           tc_fence_after();
           // P.V(j) completes before S(j + 1) does (issue order), which the softmax threads wait for anyway: a
           // separate completion signal is needed only after the stage's last tile (each commit costs the issuer ~60 clocks)
@@ -389,7 +381,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             }
             if (!(ok = drained(i))) break;
             if (FP4) tc_fence_after();
-            if (elect_one()) { issue_s(i, stn, false); tc_commit(&bars[B_SFULL + 2 * i]); }
+            if (elect_one()) { issue_s(i, stn, false); tc_commit(&bars[B_SFULL + i]); }
             __syncwarp();
             if (i == 0) ++cs0; else ++cs1;
           }
@@ -404,91 +396,14 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       }
       gj += nmax;
     }
-  } else if (TL && (warp == 9 || warp == 10)) {
-    // =================================================================== UMMA issuers (one per stage)
-    // The whole warp stays converged through the waits and the descriptor arithmetic (warp-uniform values); one elected
-    // lane issues. Descriptors are built once; the loops only add byte offsets.
-    const int i = __shfl_sync(0xFFFFFFFFu, warp - 9, 0);
-    constexpr uint32_t ID_S = idesc_f8(128, 64, 0, 0);
-    const uint32_t tm = __shfl_sync(0xFFFFFFFFu, tmem, 0);
-    const uint32_t t_si = tm + 128 * i, t_oi = tm + 256 + 128 * i;
-    const uint32_t q_addr = smem_u32(sQ) + i * Q_STRIDE, k_addr = smem_u32(sK), v_addr = smem_u32(sV);
-    const uint64_t dq0 = smem_desc(q_addr, 16, SBO, SWZ), dk0 = smem_desc(k_addr, 16, SBO, SWZ), dv0 = smem_desc(v_addr, 16, SBO, SWZ);
-    int gj = 0;                            // key tiles consumed so far, over all items
-    int cs = 0;                            // S products issued so far (the buffer is its parity)
-    bool ok = true;
-    for (int k = 0; ok; ++k) {
-      const int L = fwd_item(k, G, cta, p.zigzag);
-      if (L >= n_items) break;
-      const int kb = k & 1;
-      if (!(ok = mbar_wait(&bars[B_Q + kb], (k >> 1) & 1, p.ctl, abortp, 20))) break;
-      const int n = tile_s[kb].n[i], n_tiles = (max(tile_s[kb].n[0], tile_s[kb].n[1]) + 1) / 2;      // steps; key tiles
-      // Start the second stage about half a step after the first: the two softmax warpgroups share each scheduler's
-      // transcendental unit, which saturates when their exponential phases coincide and idles while both do something else.
-      if (k == 0 && i == 1) {
-        const long long t_skew = clock64();
-        while (clock64() - t_skew < STEP_SKEW_CLOCKS) {}
-      }
-      // Turn t: P.V of step t, then S of step t + 2 into the buffer that held P-hat(t) (the pipe runs in issue order);
-      // turns -2 and -1 are the item's first two products, which run while the softmax warps write the previous item's rows.
-#pragma unroll 1
-      for (int t = -2; t < n; ++t) {
-        if (t >= 0) {
-          const int st = (gj + (t >> 1)) % KV_STAGES;
-          const int cp = cs - min(2, n - t);             // the step's number over all items
-          const int rg = cp & 1;
-          if (!(t & 1) && !(ok = mbar_wait(&bars[B_VFULL + st], ((gj + (t >> 1)) / KV_STAGES) & 1, p.ctl, abortp, 22))) break;
-          if (!(ok = mbar_wait(&bars[B_PFULL + 2 * i + rg], (cp >> 1) & 1, p.ctl, abortp, 23))) break;
-          tc_fence_after();
-          if (elect_one()) {
-            const uint64_t b = desc_adv(dv0, st * TILE_BYTES + (t & 1) * (TILE_BYTES / 2));
-            const uint32_t ts = t_si + 64 * rg;
-#pragma unroll
-            for (int kk = 0; kk < 2; ++kk)   // 32 keys per instruction: 32 rows of the V tile (MN-major operand)
-              umma_mxf8_ts(t_oi, ts + 8 * kk, desc_adv(b, kk * 32 * D), idesc_bs(128, D, 0, 0, 0, 1, 1, kk, kk), ts + 16, ts + 20,
-                           t > 0 || kk > 0);
-            tc_commit(&bars[B_PVDONE + i]);
-            if ((t & 1) || t + 1 == n) tc_commit(&bars[B_VEMPTY + st]);
-          }
-          __syncwarp();
-        }
-        const int u = t + 2;
-        if (u < n) {
-          const int st = (gj + (u >> 1)) % KV_STAGES, rg = cs & 1;
-          if (!(u & 1) && !(ok = mbar_wait(&bars[B_KFULL + st], ((gj + (u >> 1)) / KV_STAGES) & 1, p.ctl, abortp, 21))) break;
-          tc_fence_after();
-          if (elect_one()) {
-            const uint64_t a = desc_adv(dq0, 2 * kb * Q_STRIDE), b = desc_adv(dk0, st * TILE_BYTES + (u & 1) * (TILE_BYTES / 2));
-            const uint32_t ts = t_si + 64 * rg;
-#pragma unroll
-            for (int kk = 0; kk < D / 32; ++kk) umma_f8_ss(ts, desc_adv(a, 32 * kk), desc_adv(b, 32 * kk), ID_S, kk > 0);
-            tc_commit(&bars[B_SFULL + 2 * i + rg]);
-            if ((u & 1) || u + 1 == n) tc_commit(&bars[B_KEMPTY + st]);
-          }
-          __syncwarp();
-          ++cs;
-        }
-      }
-      if (!ok) break;
-      mbar_arrive_warp(&bars[B_QE + kb]);      // (the slot of tile_s may be written again)
-      // tiles only the other stage uses: this one's releases follow their arrival (so that they count for the right phase)
-      for (int j = (n + 1) / 2; j < n_tiles; ++j) {
-        const int st = (gj + j) % KV_STAGES, ph = ((gj + j) / KV_STAGES) & 1;
-        if (!(ok = mbar_wait(&bars[B_KFULL + st], ph, p.ctl, abortp, 24))) break;
-        mbar_arrive_warp(&bars[B_KEMPTY + st]);
-        if (!(ok = mbar_wait(&bars[B_VFULL + st], ph, p.ctl, abortp, 25))) break;
-        mbar_arrive_warp(&bars[B_VEMPTY + st]);
-      }
-      gj += n_tiles;
-    }
   } else if (warp < 8) {
     // =================================================================== softmax + correction + epilogue
     fwd_reg_alloc<216>();
     const int i = warp >> 2;                          // stage
     const int r = tid & 127;                          // row of the stage = TMEM lane
-    const uint32_t t_s0 = tmem + 128 * i + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t t_s = tmem + 128 * i + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t t_o = tmem + 256 + 128 * i + ((uint32_t)((warp & 3) * 32) << 16);
-    int cs = 0;                                       // steps of this stage so far, over all items
+    int cs = 0;                                       // tiles of this stage so far, over all items
     int cd = 0;                                       // items of this stage that ended with a P.V so far
     int epi = 0, gfn = 0;                             // uses of the epilogue barrier / group-frame scale atoms so far
     bool ok = true;
@@ -520,43 +435,41 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 
       float m_used = -INFINITY, l_sum = 0.f;
       for (int j = 0; j < n_i; ++j, ++cs) {
-        const int rg = NB == 2 ? cs & 1 : 0;
-        const uint32_t t_s = t_s0 + 64 * rg;
-        float c[NG];
+        float c[4];
         uint32_t sfv = 0;
 #pragma unroll
-        for (int kbk = 0; kbk < NG; ++kbk) {
+        for (int kbk = 0; kbk < 4; ++kbk) {
           if (TL) continue;
-          c[kbk] = FP4 ? fq : fq * fk_row[j * NG + kbk];      // FP4: the block scales were applied by the tensor core
-          sfv |= ((__float_as_uint(fv_row[j * NG + kbk]) >> 23) & 0xFF) << (8 * kbk);
+          c[kbk] = FP4 ? fq : fq * fk_row[j * 4 + kbk];      // FP4: the block scales were applied by the tensor core
+          sfv |= ((__float_as_uint(fv_row[j * 4 + kbk]) >> 23) & 0xFF) << (8 * kbk);
         }
-        // token-local: the step's 64 per-key factors (same addresses for every thread: broadcast loads through L1;
-        // staging them in shared memory was twice as slow: 384 broadcast reads per thread and 128 keys saturate the
+        // token-local: the tile's 128 per-key factors (same addresses for every thread: broadcast loads through L1;
+        // staging them in shared memory was twice as slow: 384 broadcast reads per thread and tile saturate the
         // shared-memory port that the tensor core's operand reads also go through)
-        const float4* fk4 = reinterpret_cast<const float4*>(p.fac_k + (TL ? tok0 + j * KS : 0));
-        const float4* lg4 = reinterpret_cast<const float4*>(TL ? p.tok_lg_v + tok0 + j * KS : p.fac_v);
-        const float4* rc4 = reinterpret_cast<const float4*>(TL ? p.tok_rcp_v + tok0 + j * KS : p.fac_v);
+        const float4* fk4 = reinterpret_cast<const float4*>(p.fac_k + (TL ? tok0 + j * 128 : 0));
+        const float4* lg4 = reinterpret_cast<const float4*>(TL ? p.tok_lg_v + tok0 + j * 128 : p.fac_v);
+        const float4* rc4 = reinterpret_cast<const float4*>(TL ? p.tok_rcp_v + tok0 + j * 128 : p.fac_v);
         if (TL) {
           sfv = 0x7F7F7F7Fu;
 #pragma unroll
-          for (int kbk = 0; kbk < NG; ++kbk) c[kbk] = 1.f;
+          for (int kbk = 0; kbk < 4; ++kbk) c[kbk] = 1.f;
         }
-        if (!(ok = mbar_wait(&bars[B_SFULL + 2 * i + rg], (cs / NB) & 1, p.ctl, abortp, 30 + i))) break;
+        if (!(ok = mbar_wait(&bars[B_SFULL + i], cs & 1, p.ctl, abortp, 30 + i))) break;
         tc_fence_after();
-        uint32_t su[KS];
+        uint32_t su[128];
 #pragma unroll
-        for (int cc = 0; cc < NG; ++cc) FL_TMEM_LD_32(t_s + 32 * cc, (su + 32 * cc));
+        for (int cc = 0; cc < 4; ++cc) FL_TMEM_LD_32(t_s + 32 * cc, (su + 32 * cc));
         tc_wait_ld();
         if (FP4) {      // the scores are in registers: this S region may take the other stage's scale columns
           tc_fence_before();
           mbar_arrive_warp(&bars[B_SDRAIN + i]);
         }
-        float s[KS];
+        float s[128];
 #pragma unroll
-        for (int e = 0; e < KS; ++e) s[e] = __uint_as_float(su[e]);
+        for (int e = 0; e < 128; ++e) s[e] = __uint_as_float(su[e]);
         if (TL) {   // y = s f_Q f_K(key) scale + log2 f_V(key)
 #pragma unroll
-          for (int e4 = 0; e4 < KS / 4; ++e4) {
+          for (int e4 = 0; e4 < 32; ++e4) {
             // two columns per instruction; log2 f_V comes from a table (derived here it cost three integer instructions
             // per score on loops that are issue-bound)
             const float4 k4 = __ldg(fk4 + e4), l4 = __ldg(lg4 + e4);
@@ -569,29 +482,29 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         }
         if (SC) {   // soft cap: the capped score in log2 units; the factors are used up here
 #pragma unroll
-          for (int e = 0; e < KS; ++e) s[e] = p.cap_a * tanh_fast(s[e] * (c[e >> 5] * p.cap_b));
+          for (int e = 0; e < 128; ++e) s[e] = p.cap_a * tanh_fast(s[e] * (c[e >> 5] * p.cap_b));
 #pragma unroll
-          for (int kbk = 0; kbk < NG; ++kbk) c[kbk] = 1.f;
+          for (int kbk = 0; kbk < 4; ++kbk) c[kbk] = 1.f;
         }
-        const int kb0 = j * KS;                                // key of column 0, as the limits
-        const bool need_mask = (kb0 + KS - 1 > col_limit) || (kb0 < col_first);    // only on boundary tiles
+        const int kb0 = j * 128;                                // key of column 0, as the limits
+        const bool need_mask = (kb0 + 127 > col_limit) || (kb0 < col_first);    // only on boundary tiles
         if (need_mask) {   // scale first, then mask: the factor product may underflow to zero and 0 * inf is NaN
           // a bit per column (the code stands in the loop whether it runs or not, and bits take half the instructions)
           const int lo = col_first - kb0, hi = col_limit - kb0;      // visible: lo <= column <= hi
 #pragma unroll
-          for (int kbk = 0; kbk < NG; ++kbk) {
+          for (int kbk = 0; kbk < 4; ++kbk) {
             const int l = min(max(lo - 32 * kbk, 0), 32), n = min(max(hi - 32 * kbk + 1, 0), 32);
             const uint32_t see = (uint32_t)((1ull << n) - 1) & ~(uint32_t)((1ull << l) - 1);
 #pragma unroll
             for (int e = 0; e < 32; ++e) s[32 * kbk + e] = (see & (1u << e)) ? s[32 * kbk + e] * c[kbk] : -INFINITY;
           }
 #pragma unroll
-          for (int kbk = 0; kbk < NG; ++kbk) c[kbk] = 1.f;
+          for (int kbk = 0; kbk < 4; ++kbk) c[kbk] = 1.f;
         }
         float mx = -INFINITY;
-        float gm[NG];                                            // the 32-key groups' maxima (scaled)
+        float gm[4];                                             // the four 32-key groups' maxima (scaled)
 #pragma unroll
-        for (int kbk = 0; kbk < NG; ++kbk) {
+        for (int kbk = 0; kbk < 4; ++kbk) {
           // eight independent chains of three-input maxima, then a tree: a serial chain would cost its latency 31 times
           float a[8];
 #pragma unroll
@@ -610,11 +523,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         }
         if (j > 0 && __any_sync(0xFFFFFFFFu, refresh)) {
           // rescale this row of O in tensor memory once the previous P.V has finished
-          // P.V(j - 1) has completed: S(j), which this thread has read, was issued after it. Two buffers: P.V(j - 2) has.
-          if (NB == 2) {
-            if (!(ok = mbar_wait(&bars[B_PVDONE + i], (cs - 1) & 1, p.ctl, abortp, 32 + i))) break;
-            tc_fence_after();
-          }
+          // P.V(j - 1) has completed: S(j), which this thread has read, was issued after it
 #pragma unroll 1
           for (int cc = 0; cc < D / 32; ++cc) {
             uint32_t ov[32];
@@ -627,21 +536,21 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         }
         const float mb = (m_used == -INFINITY) ? 0.f : (m_used - P_OFF);
         // group frame: per 32 keys the exponent argument is lowered by the group's own integer bias
-        float gb[NG] = {};
+        float gb[4] = {0.f, 0.f, 0.f, 0.f};
         uint32_t sfp = 0x7F7F7F7Fu;
         if (GF) {
           sfp = 0;
 #pragma unroll
-          for (int kbk = 0; kbk < NG; ++kbk) {
+          for (int kbk = 0; kbk < 4; ++kbk) {
             gb[kbk] = ceilf(fmaxf(gm[kbk] - mb, -100.0f) - P_LOG2_448);
             sfp |= ((uint32_t)(127 + (int)gb[kbk]) & 0xFF) << (8 * kbk);
           }
         }
         float ps[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};     // independent partial sums (group frame: two per group)
         [[maybe_unused]] uint64_t ps2[4] = {0ull, 0ull, 0ull, 0ull};  // the same as packed pairs (default route)
-        uint32_t pw[KS / 4];
+        uint32_t pw[32];
 #pragma unroll
-        for (int w = 0; w < KS / 4; ++w) {
+        for (int w = 0; w < 32; ++w) {
           const float cw = c[w >> 3];
           const float mbw = GF ? mb + gb[w >> 3] : mb;
           // exponent arguments: two columns per instruction
@@ -671,7 +580,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           pw[w] = cvt_e4m3x4(p0, p1, p2, p3);
         }
         float psum;
-        if constexpr (GF) {   // each group's sum weighs 2^bias_g
+        if (GF) {   // each group's sum weighs 2^bias_g
           float pg[4];
 #pragma unroll
           for (int kbk = 0; kbk < 4; ++kbk) unpack2(ps2[kbk], ps[2 * kbk], ps[2 * kbk + 1]);
@@ -685,8 +594,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           psum = ((ps[0] + ps[1]) + (ps[2] + ps[3])) + ((ps[4] + ps[5]) + (ps[6] + ps[7]));
         }
         l_sum = fmaf(l_sum, alpha, psum);
-        if constexpr (NB == 2) FL_TMEM_ST_16(t_s, pw);
-        else FL_TMEM_ST_32(t_s, pw);
+        FL_TMEM_ST_32(t_s, pw);
         if (GF) {
           // the A scale tile (every lane quadrant holds all 128 rows' exponent words: lane = row % 32, column = row / 32)
           // is copied from this atom by the issuer; only the B scale columns are stored from here
@@ -694,21 +602,19 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           ++gfn;
           fence_proxy_async();             // the atom is read by tcgen05.cp (async proxy)
           uint32_t sf[8] = {0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, sfv, sfv, sfv, sfv};
-          FL_TMEM_ST_8(t_s + KS / 4, sf);
+          FL_TMEM_ST_8(t_s + 32, sf);
         } else {
           uint32_t sf[8] = {0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, sfv, sfv, sfv, sfv};
-          FL_TMEM_ST_8(t_s + KS / 4, sf);
+          FL_TMEM_ST_8(t_s + 32, sf);
         }
-        // (two buffers: the last step but one's P.V has completed before the last one's can: a parity tells two phases apart, not three)
-        if (NB == 2 && j > 0 && j + 1 == n_i && !(ok = mbar_wait(&bars[B_PVDONE + i], (cs - 1) & 1, p.ctl, abortp, 32 + i))) break;
         tc_wait_st();
         tc_fence_before();
-        mbar_arrive_warp(&bars[B_PFULL + 2 * i + rg]);
+        mbar_arrive_warp(&bars[B_PFULL + i]);
       }
       if (!ok) break;
       // ---- item epilogue: O / l -> bf16 rows through this stage's Q tile buffer, LSE
       if (n_i > 0) {
-        if (!(ok = mbar_wait(&bars[B_PVDONE + i], (NB == 2 ? cs - 1 : cd) & 1, p.ctl, abortp, 34 + i))) break;
+        if (!(ok = mbar_wait(&bars[B_PVDONE + i], cd & 1, p.ctl, abortp, 34 + i))) break;
         ++cd;
       }
       tc_fence_after();

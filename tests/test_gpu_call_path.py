@@ -103,22 +103,3 @@ def test_work_list_changes_nothing(lens, kw):
                               packed_out=(slot_src, slot_rows, total), doc_start=start, doc_len=length)
     live = row_map >= 0
     assert torch.equal(out, want[0]) and torch.equal(st[0][0][:, live], lse[0][:, live])
-
-
-@pytest.mark.parametrize("sq,h,used,window", [(128, 1, [1], None), (128, 2, [64, 65], None), (256, 2, [63, 192, 129], None), (384, 2, [320, 256], None),
-                                              (256, 160, [320, 64], None), (384, 2, [384], (130, 20)), (512, 160, [512], (40, 0))])
-def test_token_local_forward_in_steps_of_64_keys(sq, h, used, window):
-    """Per-token scales: one step, odd and even numbers of steps, stages of different lengths, an absent second stage, several items
-    per CTA (160 heads) with the score buffers' parity carried over. Bound: E4M3 P-hat, as in test_gpu_fwd."""
-    from flamia_blackwell_attention_b200 import kernels as K
-    from oracle import attention_oracle as A
-    b, sk = len(used), (max(used) + 127) // 128 * 128
-    q, k, v, _ = attention_inputs(b, max(sq, sk), h, 1, 128, seed=9)
-    q, k, v = q[:, :sq], k[:, :sk], v[:, :sk]
-    ops = [K.quantize_fp8_blocks(t.cuda(), token_local_exponents=True) for t in (q, k, v)]
-    su = torch.tensor(used, dtype=torch.int32)
-    out, lse, st = K.attn_fwd(*ops, causal=False, softmax_scale=128 ** -0.5, token_local=True, window=window, seqused_k=su.cuda())
-    assert K.read_status(st) == 0
-    ref = A.qdq_attention(q, k, v, token_local=True, window=window, seqused_k=su)
-    assert A.accuracy(out.cpu(), ref[0])["rel_l2"] < 3.2e-2
-    assert (lse.cpu() - ref[1].reshape(lse.shape)).abs().max() < 2e-3
