@@ -708,10 +708,10 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           ek_word |= ((__float_as_uint(p.fac_k[bh_k * (p.s_k / 32) + T.k0 / 32 + kbk]) >> 23) & 0xFF) << (8 * kbk);
       }
       const int krel = T.krel + r - T.off;
-  const int vis_from = p.win_r >= 0 ? krel - p.win_r : 0;    // queries in [vis_from, vis_to] see this key
-  const int vis_to = min(p.win_l >= 0 ? krel + p.win_l : 0x7FFFFFFF, T.sq - 1);
-  int m = T.m_lo;
-  for (int it = 0; it < n_it; ++it) {
+      const int vis_from = p.win_r >= 0 ? krel - p.win_r : 0;    // queries in [vis_from, vis_to] see this key
+      const int vis_to = min(p.win_l >= 0 ? krel + p.win_l : 0x7FFFFFFF, T.sq - 1);
+      int m = T.m_lo;
+      for (int it = 0; it < n_it; ++it) {
         const int g = gi + it, st = g & 1;
         const int q_first = m * 128 + 64 * x + 32 * qb;                    // document-relative query of column 0
         const bool full = key_valid && (q_first >= vis_from) && (q_first + QW - 1 <= vis_to);
