@@ -72,6 +72,12 @@ EXPORTS = {
     "fl_last_cuda_error": (i32, [C.c_char_p, i32]),
 }
 
+def window_p1(side) -> int:
+    """A side of a sliding window (None = unlimited) as the ABI takes it: side + 1, 0 = unlimited. A side beyond any sequence is cut to
+    what the kernels' 32-bit positions can be added to."""
+    return 0 if side is None else min(int(side), 1 << 30) + 1
+
+
 _lib = None
 
 

@@ -33,7 +33,7 @@ def _plan_facts(plan) -> dict:
                 need_bwd=bw.kernel != "none", p_group=f.p_hat_frame == "group", seqused_k=f.seqused_k, varlen=sh.varlen,
                 aligned=sh.aligned_varlen, ragged=f.ragged_documents, return_lse=f.return_lse, deterministic=bw.deterministic,
                 rowlocal=bw.ds_dq_rowlocal == "all", prescale={"row": 0, "causal_tile": 1, "causal_row": 2}[bw.dq_prescale],
-                window_left_p1=0 if win[0] is None else win[0] + 1, window_right_p1=0 if win[1] is None else win[1] + 1,
+                window_left_p1=L.window_p1(win[0]), window_right_p1=L.window_p1(win[1]),
                 softcap=f.softcap, softmax_scale=plan.softmax_scale, b=sh.b, s_q=sh.s_q, s_k=sh.s_k, h=sh.h, h_kv=sh.h_kv, d=sh.d,
                 tot_q=sh.tot_q, d_call=plan.pad_from or sh.d)
 

@@ -1280,8 +1280,8 @@ static int bwd_launch(const fl_attn_args* a, const void* work, void* stream) {
   p.cap_a = sc ? a->softcap * 1.4426950408889634f : 0.f;
   p.cap_b = sc ? 1.0f / p.cap_a : 0.f;
   p.causal = (a->flags & FL_A_CAUSAL) ? 1 : 0;
-  p.win_l = a->window_left_p1 - 1;
-  p.win_r = p.causal ? 0 : a->window_right_p1 - 1;
+  p.win_l = window_side(a->window_left_p1);
+  p.win_r = p.causal ? 0 : window_side(a->window_right_p1);
   p.out_f16 = (a->flags & FL_A_OUT_F16) ? 1 : 0;
   p.had_dk = (a->flags & FL_A_HAD_DK) ? 1 : 0;
   p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);

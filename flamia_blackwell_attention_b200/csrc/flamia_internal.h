@@ -71,6 +71,10 @@ struct FastDiv {
   __device__ __forceinline__ int div(int n) const { return (int)(((uint64_t)(uint32_t)n * m) >> (31 + l)); }
 };
 
+// A side of a sliding window (ABI: side + 1, 0 = unlimited) as the kernels take it: -1 = unlimited. A side beyond any sequence is cut,
+// so that the kernels' sums of a position and a side stay inside 32 bits.
+inline int window_side(int32_t p1) { return p1 <= 0 ? -1 : p1 - 1 < (1 << 30) ? p1 - 1 : (1 << 30); }
+
 static constexpr long long kDefaultWaitCycles = 1ll << 31;
 
 }  // namespace fl

@@ -746,8 +746,8 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream) {
   p.b = a->b; p.s_q = a->s_q; p.s_k = a->s_k; p.h = a->h; p.h_kv = a->h_kv; p.d_out = d_out;
   p.scale_log2 = a->softmax_scale * 1.4426950408889634f;
   p.causal = (a->flags & FL_A_CAUSAL) ? 1 : 0;
-  p.win_l = a->window_left_p1 - 1;
-  p.win_r = p.causal ? 0 : a->window_right_p1 - 1;
+  p.win_l = window_side(a->window_left_p1);
+  p.win_r = p.causal ? 0 : window_side(a->window_right_p1);
   p.out_f16 = (a->flags & FL_A_OUT_F16) ? 1 : 0;
   p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);
   // packed documents: at most one extra 256-row block per document beyond total / 256

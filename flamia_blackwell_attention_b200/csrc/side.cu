@@ -603,8 +603,8 @@ extern "C" int fl_doc_work(const int32_t* doc_start, const int32_t* doc_len, int
                            int32_t window_right_p1, int32_t causal, int32_t ordered, int32_t* work, int32_t* status, void* stream) {
   using namespace fl;
   if (!doc_start || !doc_len || !work || n_docs <= 0 || capacity <= 0 || (capacity % 128)) return FL_ERR_BAD_ARG;
-  launch_after(doc_work_kernel, 1, DW_THREADS, 0, (cudaStream_t)stream, doc_start, doc_len, n_docs, capacity, window_left_p1 - 1,
-                                                              causal ? 0 : window_right_p1 - 1, ordered, (int4*)work, status);
+  launch_after(doc_work_kernel, 1, DW_THREADS, 0, (cudaStream_t)stream, doc_start, doc_len, n_docs, capacity,
+               window_side(window_left_p1), causal ? 0 : window_side(window_right_p1), ordered, (int4*)work, status);
   return launch_result("fl_doc_work: kernel launch");
 }
 

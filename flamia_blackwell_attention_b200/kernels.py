@@ -157,8 +157,7 @@ def attn_args(q, k, v, *, causal, softmax_scale, mode=L.FL_MODE_FP8, flags=0, st
     a.status = L.ptr(status)
     a.wait_cycles = int(wait_cycles)
     if window is not None:      # (left, right), None = unlimited; stored as window + 1 (0 = unlimited)
-        a.window_left_p1 = 0 if window[0] is None else int(window[0]) + 1
-        a.window_right_p1 = 0 if window[1] is None else int(window[1]) + 1
+        a.window_left_p1, a.window_right_p1 = L.window_p1(window[0]), L.window_p1(window[1])
     a.seqused_k = L.ptr(seqused_k)      # batched form: (b,) int32 valid keys per batch row, or None
     a.softcap = float(softcap or 0.0)
     return a
