@@ -541,6 +541,10 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           const int st = gp & 1;
           if (!FP4 && !(ok = dq_read(gp))) break;
           if (!(ok = mbar_wait(&bars[BB_BFULL + 2 * st + y], (gp >> 1) & 1, p.ctl, abortp, 27))) break;
+          // Half 1's P-hat and dS-hat go to the region that the products of (gp - 1, 1) read last. Otherwise the grant of the scores in
+          // between says that they have (S^T is issued behind them); an item's last iteration has none, and dP^T waits in their
+          // stead. (Waiting in the compute warps cost the 8-bit kernel 2 %: b4 s4096 h16 step 917 -> 931 us; here 909 -> 912, within noise.)
+          if (y == 1 && j >= 0 && j + 2 == n_it && !(ok = mbar_wait(&bars[BB_BEMPTY + 2 * (st ^ 1) + 1], ((gp - 1) >> 1) & 1, p.ctl, abortp, 29))) break;
           tc_fence_after();
           const uint64_t doy = desc_adv(dDO0, st * TILE_BYTES + y * 64 * D);
           if (elect_one()) {

@@ -22,3 +22,21 @@ def test_window_longer_than_any_sequence(s, window, same):
     x = [t.cuda() for t in attention_inputs(2, s, 2, 1, 64, seed=11)]
     for a, b in zip(_step(F.flash_attn_fp8, *x, window_size=window), _step(F.flash_attn_fp8, *x, window_size=same)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("entry,d,opts", [("fp8", 128, {}), ("fp8", 64, {}), ("fp4", 128, {}), ("fp8", 128, dict(ds_dq_rowlocal="all")),
+                                          ("fp8", 128, dict(operand_scaling="token_local", ds_dq_rowlocal="all"))])
+@pytest.mark.parametrize("s,hk,causal", [(128, 4, False), (256, 4, True), (384, 2, False)])
+def test_dk_dv_of_items_with_few_query_tiles(entry, d, opts, s, hk, causal):
+    """Every key tile's dK and dV are sums in a fixed order, so they repeat bit for bit; items of one to six query tiles, where an
+    item's first and last iteration (whose hand-overs differ) are most of them, and several items a CTA."""
+    import flamia_blackwell_attention_b200 as F
+    fn = F.flash_attn_fp8 if entry == "fp8" else F.flash_attn_fp4
+    kw = dict(options=(F.FP8AttnOptions if entry == "fp8" else F.FP4AttnOptions)(**opts)) if opts else {}
+    q, k, v, do = (t.cuda() for t in attention_inputs(128, s, 4, hk, d, seed=12))
+    q, k, v = (t.requires_grad_(True) for t in (q, k, v))
+    first = None
+    for _ in range(10):
+        dk, dv = torch.autograd.grad(fn(q, k, v, causal=causal, **kw), (k, v), do)
+        first = first or (dk, dv)
+        assert torch.equal(dk, first[0]) and torch.equal(dv, first[1])
