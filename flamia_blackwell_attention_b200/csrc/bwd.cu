@@ -275,6 +275,13 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   BTile* const tile_s = misc.tile;
   constexpr bool RL = VAR >= 1, TL = VAR == 2;
   constexpr int QW = bwd_qw(VAR), NQ = QW / 32, NWG = 128 / QW;      // queries, query blocks per warpgroup; warpgroups
+  // Who gives a K / V buffer and its slot of tile_s back: the compute warps (gradient rows written, slot no longer read), each warp of
+  // the reduction and each issuer (slot read; an item without query tiles does not hold these up, and an ordered dQ can keep the
+  // reduction behind). One thread a compute warpgroup is enough where the warps work on a copy of the slot (two warpgroups; what
+  // they write through the buffer is stored behind a barrier of the warpgroup) and is kept for the plain 8-bit route (every warp: b4 s4096 h16 914 -> 930 us);
+  // the others are faster with an arrival per warp, spills go (d = 64 b8 s1000 209 -> 201 us, token scales b2 s8192 4900 -> 4350).
+  constexpr bool KVE_EACH = !(NWG == 2 && SM::EPI2);
+  constexpr int N_KVE = (KVE_EACH ? 4 * NWG : NWG) + 4 + (FP4 ? 2 : 3);
   constexpr int W_RED = 4 * NWG, W_GRAD = W_RED + 4, W_PROD = W_RED + 5, W_S = W_RED + 6, W_DP = W_RED + 7;    // warps
 
   if (smem_u32(smem) & 1023) {           // (never the case without static shared memory; the swizzles depend on it)
@@ -290,7 +297,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   if (tid == W_PROD * 32) {
     misc.abort = 0;
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&bars[BB_KV + i], 1); mbar_init(&bars[BB_KVE + i], NWG);      // released by one thread of each compute warpgroup
+      mbar_init(&bars[BB_KV + i], 1); mbar_init(&bars[BB_KVE + i], N_KVE);
       mbar_init(&bars[BB_BFULL + 2 * i], 1); mbar_init(&bars[BB_BEMPTY + 2 * i], 1);
       mbar_init(&bars[BB_BFULL + 2 * i + 1], 1); mbar_init(&bars[BB_BEMPTY + 2 * i + 1], 1);
       mbar_init(&bars[BB_S + i], 1); mbar_init(&bars[BB_DP + i], 1);
@@ -339,8 +346,8 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const int L = bwd_item(k, G, cta, p.zigzag);
         if (L >= n_items) break;
         const int kb = k & 1;
-        // the buffers of item k - 2 (and its slot of tile_s) are free once both compute warpgroups have written its
-        // gradient rows out of them
+        // the buffers of item k - 2 (and its slot of tile_s) are free once the compute warpgroups have written its
+        // gradient rows out of them and every other role has read the slot
         if (k >= 2 && !(ok = mbar_wait(&bars[BB_KVE + kb], ((k >> 1) - 1) & 1, p.ctl, abortp, 11))) break;
         BTile t;
         bwd_decode<FULL>(p, L, t);
@@ -422,6 +429,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[BB_KV + kb], (k >> 1) & 1, p.ctl, abortp, 20))) break;
       const int n_it = tile_s[kb].n_m * grp;
+      mbar_arrive_warp(&bars[BB_KVE + kb]);
       const uint64_t dK_k = desc_adv(dK0, kb * TILE_BYTES);
       // the first products of an item overwrite dV / dK: the previous item's rows must have left tensor memory (an item without
       // query tiles issues nothing, but its accumulator hand-over still takes place once)
@@ -492,6 +500,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[BB_KV + kb], (k >> 1) & 1, p.ctl, abortp, 21))) break;
       const int n_it = tile_s[kb].n_m * grp;
+      mbar_arrive_warp(&bars[BB_KVE + kb]);
       const uint64_t dK_k = desc_adv(dK0, kb * (FP4 ? 8192 : TILE_BYTES)), dV_k = desc_adv(dV0, kb * TILE_BYTES);
 #pragma unroll 1
       for (int t = -3; t < 2 * n_it - 2; ++t) {
@@ -570,6 +579,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[BB_KV + kb], (k >> 1) & 1, p.ctl, abortp, 43))) break;
       const BTile T = tile_s[kb];
+      mbar_arrive_warp(&bars[BB_KVE + kb]);
       const int n_it = T.n_m * grp;
       int head = T.hkv * grp, m = T.m_lo;
 #pragma unroll 1
@@ -689,6 +699,11 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     [[maybe_unused]] int n_rot = 0;                                   // rotated items so far
     int cg = 0;                                      // grants used so far
     int pending_kve = -1;                            // the K / V buffer whose gradient stores are still to be confirmed
+    auto free_kv = [&](int buf) {
+      if (r == 0) tma_store_wait_read<0>();
+      if (KVE_EACH) mbar_arrive_warp(&bars[BB_KVE + buf]);
+      else if (r == 0) mbar_arrive(&bars[BB_KVE + buf]);
+    };
     for (int k = 0; ok; ++k) {
       const int L = bwd_item(k, G, cta, p.zigzag);
       if (L >= n_items) break;
@@ -846,7 +861,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         if (it == 0 && pending_kve >= 0) {
           // the previous item's gradient stores have long read their shared-memory source: its K / V buffer goes back (and, where
           // the scale atoms share the way out's memory, every warp of the half has to know)
-          if (r == 0) { tma_store_wait_read<0>(); mbar_arrive(&bars[BB_KVE + pending_kve]); }
+          free_kv(pending_kve);
           pending_kve = -1;
           if (EPI2) {
             mbar_arrive_warp(&bars[BB_EPX + x]);
@@ -1068,7 +1083,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         // Nobody waits for the stores here: the thread that issued one confirms that it has read its source, and only then
         // hands the K / V buffer back to the producer, one query tile into the next item.
         if (pending_kve >= 0) {          // (an item with fewer than two query tiles came in between)
-          if (r == 0) { tma_store_wait_read<0>(); mbar_arrive(&bars[BB_KVE + pending_kve]); }
+          free_kv(pending_kve);
           pending_kve = -1;
           mbar_arrive_warp(bar_epi);
           if (!(ok = mbar_wait(bar_epi, epi & 1, p.ctl, abortp, 38))) break;

@@ -40,3 +40,22 @@ def test_dk_dv_of_items_with_few_query_tiles(entry, d, opts, s, hk, causal):
         dk, dv = torch.autograd.grad(fn(q, k, v, causal=causal, **kw), (k, v), do)
         first = first or (dk, dv)
         assert torch.equal(dk, first[0]) and torch.equal(dv, first[1])
+
+
+@pytest.mark.parametrize("causal", [False, True])
+def test_key_tiles_that_no_query_sees(causal):
+    """seqused_k far below s_k: most key tiles are items without query tiles, many in a row for each CTA, beside an ordered dQ whose
+    reduction is still waiting for its turn. Bit for bit the same again; dense: bit for bit the call on the keys in use alone."""
+    import flamia_blackwell_attention_b200 as F
+    b, s, used = 2, 4096, 256
+    q, k, v, do = (t.cuda() for t in attention_inputs(b, s, 8, 8, 128, seed=13))
+    k[:, used:], v[:, used:] = 0, 0                      # (the f16 pre-scale of dQ is sized from all keys)
+    su = torch.full((b,), used, dtype=torch.int32, device="cuda")
+    first = _step(F.flash_attn_fp8, q, k, v, do, causal=causal, seqused_k=su)
+    for x, y in zip(first, _step(F.flash_attn_fp8, q, k, v, do, causal=causal, seqused_k=su)):
+        assert torch.equal(x, y)
+    assert not first[2][:, used:].any() and not first[3][:, used:].any()
+    if not causal:
+        out, dq, dk, dv = _step(F.flash_attn_fp8, q, k[:, :used], v[:, :used], do)
+        assert torch.equal(out, first[0]) and torch.equal(dq, first[1])
+        assert torch.equal(dk, first[2][:, :used]) and torch.equal(dv, first[3][:, :used])
