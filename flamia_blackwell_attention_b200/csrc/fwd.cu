@@ -194,7 +194,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     abort_s = 0;
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars[B_Q + i], 1);
-      mbar_init(&bars[B_QE + i], 2);         // released by one thread of each softmax warpgroup
+      mbar_init(&bars[B_QE + i], 9);         // released by each softmax warp and by the issuer: all of them read the slot of tile_s
       mbar_init(&bars[B_SFULL + i], 1);
       mbar_init(&bars[B_PFULL + i], 4);      // one arrival per softmax warp
       mbar_init(&bars[B_PVDONE + i], 1);
@@ -234,7 +234,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         if (L >= n_items) break;
         const int kb = k & 1;
         // the Q buffer of item k - 2 (and its slot of tile_s) is free once both softmax warpgroups have written its
-        // output rows out of it
+        // output rows out of it and everyone has read the slot
         if (k >= 2 && !(ok = mbar_wait(&bars[B_QE + kb], ((k >> 1) - 1) & 1, p.ctl, abortp, 12))) break;
         Tile t;
         fwd_decode<FULL>(p, L, t);
@@ -289,6 +289,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[B_Q + kb], (k >> 1) & 1, p.ctl, abortp, 20))) break;
       const int n0 = tile_s[kb].n[0], n1 = tile_s[kb].n[1];
+      mbar_arrive_warp(&bars[B_QE + kb]);
       const int nmax = max(n0, n1);
       // issue_s(i, st): S of stage i against the K tile in ring slot st
       auto issue_s = [&](int i, int st, bool park_o1) {
@@ -692,7 +693,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         p.lse[((size_t)T.bat * p.h + head) * p.s_q + qrow] = v;
       }
       tc_fence_before();                 // this stage's output has left tensor memory before the next item's P-hat is announced
-      if (r == 0) mbar_arrive(&bars[B_QE + kb]);
+      mbar_arrive_warp(&bars[B_QE + kb]);  // (the thread that stored the rows has seen them read)
     }
   }
   // ---- common exit: nothing of this CTA may still be in flight when tensor memory is released

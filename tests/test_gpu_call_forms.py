@@ -59,3 +59,24 @@ def test_key_tiles_that_no_query_sees(causal):
         out, dq, dk, dv = _step(F.flash_attn_fp8, q, k[:, :used], v[:, :used], do)
         assert torch.equal(out, first[0]) and torch.equal(dq, first[1])
         assert torch.equal(dk, first[2][:, :used]) and torch.equal(dv, first[3][:, :used])
+
+
+@pytest.mark.parametrize("entry", ["fp8", "fp4"])
+def test_documents_of_a_pack_equal_their_own_calls(entry):
+    """Several short items per CTA, most of them partly filled (rows stored one by one): O and LSE of every document bit for bit those of
+    a call on that document alone, time after time."""
+    import flamia_blackwell_attention_b200 as F
+    fn = F.flash_attn_fp8 if entry == "fp8" else F.flash_attn_fp4
+    lens = [1, 300, 77, 128, 129, 256, 5, 640, 31, 200] * 4
+    edges = [0] + list(torch.tensor(lens).cumsum(0))
+    q, k, v, _ = (t[0].cuda() for t in attention_inputs(1, sum(lens), 16, 16, 128, seed=14))
+
+    def call(lo, hi, cu):
+        cu = torch.tensor(cu, dtype=torch.int32, device="cuda")
+        return fn(q[lo:hi], k[lo:hi], v[lo:hi], causal=True, cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=640, max_seqlen_k=640, return_lse=True)
+    alone = [call(lo, hi, [0, hi - lo]) for lo, hi in zip(edges[:10], edges[1:11])]
+    for _ in range(5):
+        out, lse = call(0, edges[-1], edges)
+        for i in range(10):
+            lo, hi = edges[i], edges[i + 1]
+            assert torch.equal(out[lo:hi], alone[i][0]) and torch.equal(lse[:, lo:hi], alone[i][1]), i
