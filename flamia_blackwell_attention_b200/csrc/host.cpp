@@ -406,6 +406,7 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> forward(int64_t handle, const Te
       // the kernels' LSE has the aligned buffer's rows; its live rows go to the caller's: (h, total) in packed order, or
       // (b, h, s) for batch rows that ran as documents
       lse_user = p.varlen ? empty({p.h, total}, at::kFloat, dev) : empty({p.b, p.h, p.s_q}, at::kFloat, dev);
+      if (p.varlen) lse_user.zero_();         // (rows that no document covers read as zeros)
       check(fl_unpack_lse(ptr<float>(lse), ptr<int32_t>(docs.slot_src), ptr<int32_t>(docs.slot_rows), (int32_t)docs.capacity,
                           (int32_t)p.h, (int32_t)(p.varlen ? total : p.s_q), (int32_t)total, ptr<float>(lse_user), st),
             "fl_unpack_lse");

@@ -80,3 +80,18 @@ def test_documents_of_a_pack_equal_their_own_calls(entry):
         for i in range(10):
             lo, hi = edges[i], edges[i + 1]
             assert torch.equal(out[lo:hi], alone[i][0]) and torch.equal(lse[:, lo:hi], alone[i][1]), i
+
+
+@pytest.mark.parametrize("first,last", [(0, 700), (64, 764)])
+def test_lse_of_rows_that_no_document_covers(first, last):
+    """A token buffer longer than its documents: their LSE rows are those of the exact pack, the others zeros."""
+    import flamia_blackwell_attention_b200 as F
+    q, k, v, _ = (t[0].cuda() for t in attention_inputs(1, 900, 2, 2, 64, seed=15))
+    kw = dict(causal=True, max_seqlen_q=400, max_seqlen_k=400, return_lse=True)
+    cu = torch.tensor([first, first + 300, last], dtype=torch.int32, device="cuda")
+    own = cu - first
+    del [torch.full((2, 900), float("nan"), device="cuda") for _ in range(64)][:]      # (what the allocator hands out next)
+    lse = F.flash_attn_fp8(q, k, v, cu_seqlens_q=cu, cu_seqlens_k=cu, **kw)[1]
+    want = F.flash_attn_fp8(*(t[first:last] for t in (q, k, v)), cu_seqlens_q=own, cu_seqlens_k=own, **kw)[1]
+    assert torch.equal(lse[:, first:last], want)
+    assert not lse[:, :first].any() and not lse[:, last:].any()
