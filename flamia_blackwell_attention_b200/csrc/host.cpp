@@ -185,6 +185,10 @@ Docs docs_of(const Plan& p, const Tensor& q, at::TensorList t, cudaStream_t st) 
   if (t.size() == 6) {                        // precomputed maps: cu, start, len, row_map, slot_src, slot_rows
     d.start = t[1]; d.len = t[2]; d.row_map = t[3]; d.slot_src = t[4]; d.slot_rows = t[5];
     d.capacity = t[3].numel();
+    for (const Tensor& x : t) TORCH_CHECK(x.scalar_type() == at::kInt && x.is_contiguous(), "document maps are contiguous int32 tables");
+    TORCH_CHECK(d.start.numel() == d.len.numel() && d.capacity % 128 == 0 && d.slot_src.numel() == d.capacity / 128 &&
+                    d.slot_rows.numel() == d.capacity / 128,
+                "document maps: start / len of one size, slot_src / slot_rows one entry per 128 rows of row_map");
     return d;
   }
   if (p.varlen && p.aligned) {
@@ -192,6 +196,7 @@ Docs docs_of(const Plan& p, const Tensor& q, at::TensorList t, cudaStream_t st) 
     d.aligned = true;
     d.start = t[0].slice(0, 0, t[0].size(0) - 1).to(at::kInt).contiguous();
     d.len = t[2].to(at::kInt).contiguous();
+    TORCH_CHECK(d.len.numel() == d.start.numel(), "aligned documents: one seqused entry per document");
     d.capacity = p.tot_q;
     return d;
   }
@@ -298,6 +303,11 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> forward(int64_t handle, const Te
                                                         at::TensorList docs_in) {
   const Plan& p = plan_at(handle);
   TORCH_CHECK(q_.is_cuda() && k_.is_cuda() && v_.is_cuda(), "q, k, v must be CUDA tensors: this library has no CPU path");
+  // (the kernels take plain pointers: a host tensor's or another device's would be followed)
+  TORCH_CHECK(k_.device() == q_.device() && v_.device() == q_.device(), "q, k, v must be on one device; got ", q_.device(), ", ",
+              k_.device(), ", ", v_.device());
+  for (const Tensor& t : docs_in)
+    TORCH_CHECK(t.device() == q_.device(), "cu_seqlens / seqused / document maps must be on q's device ", q_.device(), "; got ", t.device());
   const c10::cuda::CUDAGuard guard(q_.device());
   const auto dev = q_.device();
   const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
@@ -310,6 +320,8 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> forward(int64_t handle, const Te
   if (p.seqused_k) {                          // batched form: docs = [seqused_k]
     TORCH_CHECK(docs_in.size() == 1, "docs is [seqused_k]");
     seqused = docs_in[0];
+    TORCH_CHECK(seqused.scalar_type() == at::kInt && seqused.numel() == p.b && seqused.is_contiguous(),
+                "seqused_k is an int32 tensor of shape (batch,)");
   }
   Docs docs;
   const bool has_docs = p.varlen || p.ragged;
@@ -441,6 +453,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
     return state[i++];
   };
   const Tensor &out = next(), &lse = next();
+  TORCH_CHECK(out.device() == dout.device(), "dout is on ", dout.device(), ", the output on ", out.device());
   const Tensor &qc = next(), &qf = next(), &kc = next(), &kf = next(), &vc = next(), &vf = next();
   const Tensor& status = next();
   const Tensor &kstats = next(), &vstats = next();

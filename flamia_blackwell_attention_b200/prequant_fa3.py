@@ -30,6 +30,8 @@ def _validate(q, k, v, descs, proxies):
         if not isinstance(t, torch.Tensor) or t.dtype != torch.float8_e4m3fn:
             _fail(32, TypeError, f"flash_attn_fp8 with q_descale / k_descale / v_descale takes q, k, v as "
                                  f"torch.float8_e4m3fn codes; {n} is {getattr(t, 'dtype', type(t).__name__)}")
+        if t.device != q.device:
+            _fail(32, ValueError, f"q, k, v codes must be on one device; {n} is on {t.device}, q on {q.device}")
         if t.requires_grad:
             _fail(32, ValueError, f"E4M3 {n} requires grad: PyTorch would cast its gradient to E4M3. Pass detached codes "
                                   "and grad_proxies=(q, k, v)")
@@ -105,6 +107,8 @@ def flash_attn_fp8_prequant(resolve, q, k, v, q_descale, k_descale, v_descale, g
     qd, kd, vd = (d.to(torch.float32).contiguous() for d in (q_descale, k_descale, v_descale))
     su_k = kw.get("seqused_k")
     su_k = su_k.contiguous() if plan.fwd.seqused_k else None
+    if su_k is not None and su_k.device != q.device:
+        _fail("B9", ValueError, f"seqused_k must be on the codes' device {q.device}; got {su_k.device}")
     pq, pk, pv = grad_proxies if want_grad else (None, None, None)
     out, lse = _PrequantAttn.apply(pq, pk, pv, q.contiguous(), k.contiguous(), v.contiguous(), qd, kd, vd, plan, su_k)
     return (out, lse) if return_lse else out

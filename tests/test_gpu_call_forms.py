@@ -95,3 +95,36 @@ def test_lse_of_rows_that_no_document_covers(first, last):
     want = F.flash_attn_fp8(*(t[first:last] for t in (q, k, v)), cu_seqlens_q=own, cu_seqlens_k=own, **kw)[1]
     assert torch.equal(lse[:, first:last], want)
     assert not lse[:, :first].any() and not lse[:, last:].any()
+
+
+def test_tables_on_another_device_are_refused():
+    """Host tensors (cu_seqlens, seqused_*, maps, k) and tables of another type or size are an error before the first launch."""
+    import flamia_blackwell_attention_b200 as F
+    from flamia_blackwell_attention_b200 import _op
+    q = torch.randn(384, 2, 64, device="cuda", dtype=torch.bfloat16)
+    cu, su = torch.tensor([0, 128, 384], dtype=torch.int32), torch.tensor([100, 256], dtype=torch.int32)
+    packed = dict(cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=256, max_seqlen_k=256)
+    aligned = dict(packed, cu_seqlens_q=cu.cuda())
+    aligned["cu_seqlens_k"] = aligned["cu_seqlens_q"]
+    for kw in (packed, dict(aligned, seqused_q=su, seqused_k=su)):
+        with pytest.raises(RuntimeError, match="on q's device"):
+            F.flash_attn_fp8(q, q, q, **kw)
+    long = su.cuda().repeat(2)
+    with pytest.raises(RuntimeError, match="one seqused entry per document"):
+        F.flash_attn_fp8(q, q, q, **dict(aligned, seqused_q=long, seqused_k=long))
+    q4 = q.view(3, 128, 2, 64)
+    with pytest.raises(RuntimeError, match="on q's device"):
+        F.flash_attn_fp8(q4, q4, q4, seqused_k=torch.tensor([128, 5, 7], dtype=torch.int32))
+    with pytest.raises(RuntimeError, match="must be CUDA tensors"):
+        F.flash_attn_fp8(q4, q4.cpu(), q4)
+    q8, one = q4.to(torch.float8_e4m3fn), torch.ones(3, 2, device="cuda")
+    pre = dict(q_descale=one, k_descale=one, v_descale=one)
+    with pytest.raises(ValueError, match="one device"):
+        F.flash_attn_fp8(q8, q8, q8.cpu(), **pre)
+    with pytest.raises(ValueError, match="codes' device"):
+        F.flash_attn_fp8(q8, q8, q8, seqused_k=torch.tensor([128, 5, 7], dtype=torch.int32), **pre)
+    maps = F.DocMaps.from_cu_seqlens(cu).to("cuda")
+    pid = _op.register_plan(F.resolve_fp8(q, q, q, **packed))
+    for bad in (lambda t: t[:4] + [t[4][:-1], t[5]], lambda t: [x.long() for x in t]):
+        with pytest.raises(RuntimeError, match="document maps"):
+            torch.ops.lowbit_attn.fp8(q, q, q, bad(maps.tensors()), pid, 0)
