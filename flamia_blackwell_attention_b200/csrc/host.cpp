@@ -155,6 +155,13 @@ T* ptr(void* p) {
   return reinterpret_cast<T*>(p);
 }
 
+// An operand's rows as the quantisers read them. Zero-padded head dims are served at any start address (they used to be copied for their
+// zero columns); the tensor maps want 16-byte alignment, and an odd view is copied. The kernels' own head dims refuse it.
+Tensor rows_of(const Plan& p, const Tensor& x) {
+  const Tensor c = x.contiguous();
+  return p.d_call != p.d && reinterpret_cast<uintptr_t>(c.const_data_ptr()) % 16 ? c.clone() : c;
+}
+
 // Temporaries of one call carved out of one allocation (256-byte aligned pieces): sizes first, pointers afterwards.
 struct Workspace {
   size_t size = 0;
@@ -311,7 +318,7 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> forward(int64_t handle, const Te
   const c10::cuda::CUDAGuard guard(q_.device());
   const auto dev = q_.device();
   const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-  const Tensor q = q_.contiguous(), k = k_.contiguous(), v = v_.contiguous();
+  const Tensor q = rows_of(p, q_), k = rows_of(p, k_), v = rows_of(p, v_);
   TORCH_CHECK(q.numel() == (p.varlen ? p.tot_q : p.b * p.s_q) * p.h * p.d_call &&
                   k.numel() == (p.varlen ? p.tot_q : p.b * p.s_k) * p.h_kv * p.d_call &&
                   v.numel() == k.numel() && k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(),
@@ -443,7 +450,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
   const c10::cuda::CUDAGuard guard(dout_.device());
   const auto dev = dout_.device();
   const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-  const Tensor dout = dout_.contiguous();
+  const Tensor dout = rows_of(p, dout_);
   const bool has_docs = capacity >= 0, repacked = has_docs && !aligned;
   const Shapes sh = shapes_of(p, capacity);
   TORCH_CHECK(dout.numel() == (p.varlen ? p.tot_q : p.b * p.s_q) * p.h * p.d_call, "dout does not have the shape of the output");

@@ -128,3 +128,21 @@ def test_tables_on_another_device_are_refused():
     for bad in (lambda t: t[:4] + [t[4][:-1], t[5]], lambda t: [x.long() for x in t]):
         with pytest.raises(RuntimeError, match="document maps"):
             torch.ops.lowbit_attn.fp8(q, q, q, bad(maps.tensors()), pid, 0)
+
+
+@pytest.mark.parametrize("d", [16, 48, 80, 96])
+@pytest.mark.parametrize("form", ["batched", "ragged", "packed"])
+def test_padded_head_dims_at_any_address(d, form):
+    """Inputs and an output gradient that start two bytes past an aligned address: bit for bit the aligned call."""
+    import flamia_blackwell_attention_b200 as F
+    x = [t.cuda() for t in attention_inputs(2, 250 if form == "ragged" else 256, 4, 2, d, seed=16)]
+    kw = dict(causal=True)
+    if form == "packed":
+        cu = torch.tensor([0, 77, 512], dtype=torch.int32, device="cuda")
+        x, kw = [t.flatten(0, 1) for t in x], dict(kw, cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=435, max_seqlen_k=435)
+
+    def odd(t):
+        y = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape)
+        return y.copy_(t)
+    for a, b in zip(_step(F.flash_attn_fp8, *map(odd, x), **kw), _step(F.flash_attn_fp8, *x, **kw)):
+        assert torch.equal(a, b)
