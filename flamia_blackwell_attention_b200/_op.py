@@ -95,7 +95,8 @@ for _e in ("fp8", "fp4"):
 
 def op_apply(entry, handle, q, k, v, docs_tensors):
     """Runs the registered op of the entry on a registered plan; returns (out, lse)."""
-    if torch.compiler.is_compiling():
+    # (the native call goes to the dispatcher directly: traced programs, __torch_function__ subclasses and modes need the op itself)
+    if torch.compiler.is_compiling() or torch.overrides.has_torch_function((q, k, v)):
         out, lse, _state = getattr(torch.ops.lowbit_attn, entry)(q, k, v, list(docs_tensors), handle, 0)
         return out, lse
     return L.host().run(entry == "fp4", handle, q, k, v, docs_tensors)

@@ -1,6 +1,7 @@
 """The call path's host side, without a GPU."""
 import pytest
 import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
 
 import flamia_blackwell_attention_b200 as F
 from flamia_blackwell_attention_b200 import _op
@@ -14,3 +15,18 @@ def test_window_sides_reach_the_kernels_whole(side):
     facts = _op._plan_facts(F.resolve_fp8(q, q, q, window_size=(side, side)))
     for name in ("window_left_p1", "window_right_p1"):
         assert min(side, 256) < facts[name] <= 2 ** 30 + 1
+
+
+def test_torch_function_modes_see_the_op():
+    calls = []
+
+    class Mode(torch.overrides.TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            calls.append(str(func))
+            return func(*args, **(kwargs or {}))
+    with FakeTensorMode():
+        q = torch.empty(1, 256, 2, 128, dtype=torch.bfloat16, device="cuda")
+        with Mode():
+            F.flash_attn_fp8(q, q, q)
+            F.flash_attn_fp4(q, q, q)
+    assert "lowbit_attn.fp8" in calls and "lowbit_attn.fp4" in calls

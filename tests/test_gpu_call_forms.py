@@ -146,3 +146,18 @@ def test_padded_head_dims_at_any_address(d, form):
         return y.copy_(t)
     for a, b in zip(_step(F.flash_attn_fp8, *map(odd, x), **kw), _step(F.flash_attn_fp8, *x, **kw)):
         assert torch.equal(a, b)
+
+
+def test_tensor_subclass_goes_through_the_op():
+    import flamia_blackwell_attention_b200 as F
+    seen = []
+
+    class Sub(torch.Tensor):
+        @classmethod
+        def __torch_function__(cls, func, types, args=(), kwargs=None):
+            seen.append(getattr(func, "__name__", ""))
+            return super().__torch_function__(func, types, args, kwargs or {})
+    q, k, v, _ = (t.cuda() for t in attention_inputs(1, 256, 2, 2, 64, seed=17))
+    out = F.flash_attn_fp8(q.as_subclass(Sub), k, v, causal=True)
+    assert type(out) is Sub and "fp8" in seen
+    assert torch.equal(out.as_subclass(torch.Tensor), F.flash_attn_fp8(q, k, v, causal=True))
