@@ -580,15 +580,18 @@ std::tuple<Tensor, Tensor, Tensor> bwd_cuda(const Tensor& dout, at::TensorList s
   return backward(e.plan, e.capacity, e.aligned, dout, state, Tensor(), Tensor());
 }
 
-// O and the LSE are the node's outputs; the state (codes, tables) is saved beside them and leaves the op as plain tensors.
+// O is the node's output; the LSE (no gradient) and the state (codes, tables) are saved beside it and leave the op as plain tensors.
 struct Call {
   at::TensorList docs;
   int64_t plan, docs_id;
+  Tensor* lse;
   std::vector<Tensor>* state;
 };
 template <bool FP4>
 struct AttnNode : public torch::autograd::Function<AttnNode<FP4>> {
-  static variable_list forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, Call c) {
+  // compiled autograd may trace backward(): it reads nothing but its inputs, the saved tensors and two saved numbers
+  static constexpr bool is_traceable = true;
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, Call c) {
     at::AutoDispatchBelowADInplaceOrView below;
     auto [out, lse, state] = fwd_op<FP4>().call(q, k, v, c.docs, c.plan, c.docs_id);
     const Plan& p = plan_at(c.plan);
@@ -603,9 +606,9 @@ struct AttnNode : public torch::autograd::Function<AttnNode<FP4>> {
     ctx->saved_data["entry"] = entry_of(c.plan, !has_docs ? -1 : repacked ? state[0].size(2) : p.tot_q, has_docs && p.aligned);
     ctx->saved_data["repacked"] = repacked;
     ctx->set_materialize_grads(false);
-    ctx->mark_non_differentiable({lse});
+    *c.lse = std::move(lse);
     *c.state = std::move(state);
-    return {out, lse};
+    return out;
   }
   static variable_list backward(torch::autograd::AutogradContext* ctx, variable_list grads) {
     if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor(), Tensor()};
@@ -624,8 +627,8 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> fwd_autograd(const Tensor& q, co
     return fwd_op<FP4>().call(q, k, v, docs, plan, docs_id);
   }
   std::vector<Tensor> state;
-  variable_list o = AttnNode<FP4>::apply(q, k, v, Call{docs, plan, docs_id, &state});
-  return {o[0], o[1], std::move(state)};
+  Tensor lse, out = AttnNode<FP4>::apply(q, k, v, Call{docs, plan, docs_id, &lse, &state});
+  return {std::move(out), std::move(lse), std::move(state)};
 }
 
 TORCH_LIBRARY_IMPL(lowbit_attn, CUDA, m) {

@@ -161,3 +161,26 @@ def test_tensor_subclass_goes_through_the_op():
     out = F.flash_attn_fp8(q.as_subclass(Sub), k, v, causal=True)
     assert type(out) is Sub and "fp8" in seen
     assert torch.equal(out.as_subclass(torch.Tensor), F.flash_attn_fp8(q, k, v, causal=True))
+
+
+@pytest.mark.parametrize("form", ["batched", "packed", "aligned", "ragged"])
+def test_compiled_autograd(form):
+    """A backward traced by compiled autograd, after an eager forward and after a traced one: the eager gradients."""
+    import flamia_blackwell_attention_b200 as F
+    x, kw = [t.cuda() for t in attention_inputs(2, 250 if form == "ragged" else 256, 2, 2, 128, seed=18)], dict(causal=True)
+    if form in ("packed", "aligned"):
+        cu = torch.tensor([0, 128, 512], dtype=torch.int32, device="cuda")
+        x, kw = [t.flatten(0, 1) for t in x], dict(kw, cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=384, max_seqlen_k=384)
+        if form == "aligned":
+            su = torch.tensor([100, 384], dtype=torch.int32, device="cuda")
+            kw.update(seqused_q=su, seqused_k=su)
+    want = _step(F.flash_attn_fp8, *x, **kw)
+    fn = lambda q, k, v: F.flash_attn_fp8(q, k, v, deterministic=True, **kw)      # noqa: E731
+    for forward in (fn, torch.compile(fn, backend="aot_eager")):
+        torch._dynamo.reset()
+        q, k, v = (t.detach().requires_grad_(True) for t in x[:3])
+        with torch._dynamo.config.patch(compiled_autograd=True):
+            out = forward(q, k, v)
+            torch.compile(lambda: out.backward(x[3]), backend="aot_eager")()
+        for a, b in zip((out.detach(), q.grad, k.grad, v.grad), want):
+            assert torch.equal(a, b)
