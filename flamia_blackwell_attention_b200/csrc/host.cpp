@@ -182,11 +182,16 @@ struct Workspace {
 // the buffer's rows already.
 struct Docs {
   Tensor start, len, row_map, slot_src, slot_rows, work;
+  Tensor all;                // pooled: one buffer of the five tables
   int64_t capacity = 0;
   bool aligned = false;
+  void split(int64_t n) {
+    const auto parts = all.split_with_sizes({n, n, capacity, capacity / 128, capacity / 128});
+    start = parts[0]; len = parts[1]; row_map = parts[2]; slot_src = parts[3]; slot_rows = parts[4];
+  }
 };
 
-Docs docs_of(const Plan& p, const Tensor& q, at::TensorList t, cudaStream_t st) {
+Docs docs_of(const Plan& p, const Tensor& q, at::TensorList t, bool pooled, cudaStream_t st) {
   Docs d;
   const auto dev = q.device();
   if (t.size() == 6) {                        // precomputed maps: cu, start, len, row_map, slot_src, slot_rows
@@ -212,9 +217,13 @@ Docs docs_of(const Plan& p, const Tensor& q, at::TensorList t, cudaStream_t st) 
   const int64_t n = p.varlen ? t[0].size(0) - 1 : p.b, total = p.varlen ? p.tot_q : p.b * p.s_q;
   d.capacity = (total + 127 * n + 127) / 128 * 128;
   const int64_t slots = d.capacity / 128;
-  const Tensor all = empty({2 * n + d.capacity + 2 * slots}, at::kInt, dev);
-  const auto parts = all.split_with_sizes({n, n, d.capacity, slots, slots});
-  d.start = parts[0]; d.len = parts[1]; d.row_map = parts[2]; d.slot_src = parts[3]; d.slot_rows = parts[4];
+  if (pooled) {
+    d.all = empty({2 * n + d.capacity + 2 * slots}, at::kInt, dev);
+    d.split(n);
+  } else {
+    d.start = empty({n}, at::kInt, dev); d.len = empty({n}, at::kInt, dev); d.row_map = empty({d.capacity}, at::kInt, dev);
+    d.slot_src = empty({slots}, at::kInt, dev); d.slot_rows = empty({slots}, at::kInt, dev);
+  }
   const Tensor cu = p.varlen ? t[0].to(at::kInt).contiguous() : Tensor();
   check(fl_doc_tables(ptr<int32_t>(cu), (int32_t)n, (int32_t)(p.varlen ? 0 : p.s_q), (int32_t)total, (int32_t)d.capacity,
                       ptr<int32_t>(d.start), ptr<int32_t>(d.len), ptr<int32_t>(d.row_map), ptr<int32_t>(d.slot_src),
@@ -229,14 +238,21 @@ struct Quantised {
   fl_quant_args args = {};
 };
 
-// Tensors of one call over one allocation: every tensor object of its own costs an allocator round trip of about half a
-// microsecond, a view made directly a fifth of that. Two passes over the same requests: sizes first, then the tensors.
+// Tensors of one call over one buffer: every tensor object of its own costs an allocator round trip of about half a microsecond, a
+// view made directly a fifth of that. Two passes over the same requests: sizes first, then the tensors. Such tensors stay inside a
+// call: what autograd saves is the buffer, and the registered op, whose outputs may not share memory, has tensors of their own.
 class Pool {
  public:
-  explicit Pool(at::Device dev) : dev_(dev) {}
+  Pool() = default;
+  Pool(Tensor buf, bool traced) : buf_(std::move(buf)), traced_(traced) {}       // a buffer made before (the same requests again)
   void add(at::IntArrayRef sizes, at::ScalarType dt) { size_ = round(size_ + bytes(sizes, dt)); }
-  void allocate() { buf_ = empty({(int64_t)size_}, at::kByte, dev_); size_ = 0; }
+  const Tensor& allocate(at::Device dev) { buf_ = empty({(int64_t)size_}, at::kByte, dev); size_ = 0; return buf_; }
   Tensor take(at::IntArrayRef sizes, at::ScalarType dt) {
+    if (traced_) {
+      Tensor t = buf_.narrow(0, (int64_t)size_, (int64_t)bytes(sizes, dt)).view(dt).view(sizes);
+      size_ = round(size_ + bytes(sizes, dt));
+      return t;
+    }
     Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(buf_.storage()), buf_.key_set(), c10::scalarTypeToTypeMeta(dt));
     t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
     t.unsafeGetTensorImpl()->set_storage_offset((int64_t)(size_ / c10::elementSize(dt)));
@@ -247,9 +263,9 @@ class Pool {
  private:
   static size_t round(size_t n) { return (n + 255) & ~size_t(255); }
   static size_t bytes(at::IntArrayRef sizes, at::ScalarType dt) { return (size_t)c10::multiply_integers(sizes) * c10::elementSize(dt); }
-  at::Device dev_;
   size_t size_ = 0;
   Tensor buf_;
+  bool traced_ = false;      // through operators, for a program that records them
 };
 
 struct Shapes {            // the kernels' view of the call: one batch entry of `capacity` rows under documents
@@ -304,10 +320,46 @@ void attn_common(fl_attn_args& a, const Plan& p, const Shapes& sh, bool f16) {
   a.softcap = (float)p.softcap;
 }
 
-// Returns (out, lse, state): out / lse in the caller's layout, state = the tensors the backward needs in the order of
-// _routes.py::state_spec (without O, and without the LSE where that is the op's output), the entry handle last.
-std::tuple<Tensor, Tensor, std::vector<Tensor>> forward(int64_t handle, const Tensor& q_, const Tensor& k_, const Tensor& v_,
-                                                        at::TensorList docs_in) {
+// One call's tensors: the results in the caller's layout and what the backward needs.
+struct State {
+  Tensor out, lse_user;
+  Tensor lse;                // of the kernels: the caller's, except under documents
+  Quantised q, k, v;
+  Tensor buf;                // pooled: the buffer of the three operands' tensors
+  Tensor status, k_rows, v_rows, seqused;
+  Docs docs;
+};
+
+template <typename Make>
+void operand_tensors(State& s, const Plan& p, const Shapes& sh, Make make) {
+  const bool stats = p.need_bwd && p.prescale != 2;     // per tile (prescale == 2: per token instead, k_rows / v_rows)
+  quantised_tensors(s.q, p, sh.b, sh.s_q, p.h, true, false, make);
+  quantised_tensors(s.k, p, sh.b, sh.s_k, p.h_kv, true, stats, make);
+  quantised_tensors(s.v, p, sh.b, sh.s_k, p.h_kv, false, stats, make);
+}
+
+// The tensors of a call in the order of _routes.py::state_spec, without O and the LSE.
+std::vector<Tensor> state_list(const Plan& p, const State& s) {
+  std::vector<Tensor> state;
+  state.reserve(22);
+  for (const Quantised* x : {&s.q, &s.k, &s.v}) { state.push_back(x->codes); state.push_back(x->fac); }
+  state.push_back(s.status);
+  const bool rows = p.prescale == 2;
+  if (p.need_bwd) { state.push_back(rows ? s.k_rows : s.k.tile_stats); state.push_back(rows ? s.v_rows : s.v.tile_stats); }
+  if (p.fp4) { state.push_back(s.q.x4); state.push_back(s.q.sf4); state.push_back(s.k.x4); state.push_back(s.k.sf4); }
+  if (p.token_local)
+    for (const Quantised* x : {&s.q, &s.k, &s.v}) state.push_back(x->token_factors);
+  if (p.seqused_k) state.push_back(s.seqused);
+  if (p.varlen || p.ragged) {
+    state.push_back(s.docs.start); state.push_back(s.docs.len);
+    if (!s.docs.aligned) { state.push_back(s.docs.row_map); state.push_back(s.docs.slot_src); state.push_back(s.docs.slot_rows); }
+    state.push_back(s.docs.work);
+  }
+  return state;
+}
+
+// pooled: the operands' tensors (and document tables made here) are views of one buffer each, s.buf and s.docs.all.
+State forward(int64_t handle, const Tensor& q_, const Tensor& k_, const Tensor& v_, at::TensorList docs_in, bool pooled) {
   const Plan& p = plan_at(handle);
   TORCH_CHECK(q_.is_cuda() && k_.is_cuda() && v_.is_cuda(), "q, k, v must be CUDA tensors: this library has no CPU path");
   // (the kernels take plain pointers: a host tensor's or another device's would be followed)
@@ -323,40 +375,40 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> forward(int64_t handle, const Te
                   k.numel() == (p.varlen ? p.tot_q : p.b * p.s_k) * p.h_kv * p.d_call &&
                   v.numel() == k.numel() && k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(),
               "q, k, v do not have the shapes and types of their plan");
-  Tensor seqused;
+  State S;
+  Tensor& seqused = S.seqused;
   if (p.seqused_k) {                          // batched form: docs = [seqused_k]
     TORCH_CHECK(docs_in.size() == 1, "docs is [seqused_k]");
     seqused = docs_in[0];
     TORCH_CHECK(seqused.scalar_type() == at::kInt && seqused.numel() == p.b && seqused.is_contiguous(),
                 "seqused_k is an int32 tensor of shape (batch,)");
   }
-  Docs docs;
+  Docs& docs = S.docs;
   const bool has_docs = p.varlen || p.ragged;
-  if (has_docs) docs = docs_of(p, q, docs_in, st);
+  if (has_docs) docs = docs_of(p, q, docs_in, pooled, st);
   const Docs* dp = has_docs ? &docs : nullptr;
   const bool repacked = has_docs && !docs.aligned;
   const Shapes sh = shapes_of(p, has_docs ? docs.capacity : -1);
-  const Tensor status = status_word(dev);
+  const Tensor status = S.status = status_word(dev);
   int32_t* stp = ptr<int32_t>(status);
   const bool f16 = q.scalar_type() == at::kHalf;
 
   const bool rows = p.need_bwd && p.prescale == 2;      // per-token K / V statistics instead of per-tile ones
-  Tensor k_rows, v_rows;
+  Tensor &k_rows = S.k_rows, &v_rows = S.v_rows;
   if (rows) {
-    const Tensor both = at::zeros({2, sh.b, sh.s_k}, at::TensorOptions().dtype(at::kFloat).device(dev));
-    k_rows = both.select(0, 0); v_rows = both.select(0, 1);
+    k_rows = at::zeros({sh.b, sh.s_k}, at::TensorOptions().dtype(at::kFloat).device(dev));
+    v_rows = at::zeros_like(k_rows);
   }
-  const bool stats = p.need_bwd && !rows;
-  Quantised qq, kq, vq;
-  Pool pool(dev);
-  auto tensors = [&](auto make) {
-    quantised_tensors(qq, p, sh.b, sh.s_q, p.h, true, false, make);
-    quantised_tensors(kq, p, sh.b, sh.s_k, p.h_kv, true, stats, make);
-    quantised_tensors(vq, p, sh.b, sh.s_k, p.h_kv, false, stats, make);
-  };
-  tensors([&](std::initializer_list<int64_t> sz, at::ScalarType dt) { pool.add(sz, dt); return Tensor(); });
-  pool.allocate();
-  tensors([&](std::initializer_list<int64_t> sz, at::ScalarType dt) { return pool.take(sz, dt); });
+  using Sizes = std::initializer_list<int64_t>;
+  if (pooled) {
+    Pool pool;
+    operand_tensors(S, p, sh, [&](Sizes sz, at::ScalarType dt) { pool.add(sz, dt); return Tensor(); });
+    S.buf = pool.allocate(dev);
+    operand_tensors(S, p, sh, [&](Sizes sz, at::ScalarType dt) { return pool.take(sz, dt); });
+  } else {
+    operand_tensors(S, p, sh, [&](Sizes sz, at::ScalarType dt) { return empty(sz, dt, dev); });
+  }
+  Quantised &qq = S.q, &kq = S.k, &vq = S.v;
   quantise_args(qq, p, q, sh.b, sh.s_q, p.h, true, dp, Tensor(), 0, stp);
   // max |K_j| of the codes' values; where those are rotated, the rotation-invariant 2-norm bounds it
   quantise_args(kq, p, k, sh.b, sh.s_k, p.h_kv, true, dp, k_rows, p.hadamard && !p.fp4 ? 3 : 2, stp);
@@ -366,8 +418,8 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> forward(int64_t handle, const Te
   // O has the caller's rows: under repacked documents the kernel writes the packed rows itself. On the aligned form the
   // kernel writes the rows of its documents only, and the padding rows read as zeros. (The LSE of repacked documents keeps
   // the aligned buffer's rows; its padding rows are never used: the backward selects zero wherever a row is no document's.)
-  Tensor out = empty(q.sizes(), q.scalar_type(), dev);
-  Tensor lse = empty({sh.b, p.h, sh.s_q}, at::kFloat, dev);
+  Tensor& out = S.out = empty(q.sizes(), q.scalar_type(), dev);
+  Tensor& lse = S.lse = empty({sh.b, p.h, sh.s_q}, at::kFloat, dev);
   if (has_docs && docs.aligned) { out.zero_(); lse.zero_(); }
   fl_attn_args a = {};
   attn_common(a, p, sh, f16);
@@ -404,21 +456,8 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> forward(int64_t handle, const Te
     check(fl_fwd(&a, st), "fl_fwd");
   }
 
-  std::vector<Tensor> state;
-  state.reserve(20);
-  if (repacked) state.push_back(lse);
-  for (const Quantised* x : {&qq, &kq, &vq}) { state.push_back(x->codes); state.push_back(x->fac); }
-  state.push_back(status);
-  if (p.need_bwd) { state.push_back(rows ? k_rows : kq.tile_stats); state.push_back(rows ? v_rows : vq.tile_stats); }
-  if (p.fp4) { state.push_back(qq.x4); state.push_back(qq.sf4); state.push_back(kq.x4); state.push_back(kq.sf4); }
-  if (p.token_local)
-    for (const Quantised* x : {&qq, &kq, &vq}) state.push_back(x->token_factors);
-  if (p.seqused_k) state.push_back(seqused);
-  Tensor lse_user = lse;
+  Tensor& lse_user = S.lse_user = lse;
   if (has_docs) {
-    state.push_back(docs.start); state.push_back(docs.len);
-    if (repacked) { state.push_back(docs.row_map); state.push_back(docs.slot_src); state.push_back(docs.slot_rows); }
-    state.push_back(docs.work);
     if (docs.aligned) {
       lse_user = lse.select(0, 0);            // (h, total_q): the caller's rows are the kernels' rows
     } else if (p.return_lse) {
@@ -433,12 +472,8 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> forward(int64_t handle, const Te
       lse_user = empty({0}, at::kFloat, dev);
     }
   }
-  // the entry handle rides along as a 0-d tensor, so that the backward op needs no object beside its tensors
-  Tensor entry = at::empty({}, at::TensorOptions().dtype(at::kLong));
-  *entry.mutable_data_ptr<int64_t>() = entry_of(handle, has_docs ? docs.capacity : -1, has_docs && docs.aligned);
-  state.push_back(entry);
   check_status_if_asked(dev);
-  return {out, lse_user, std::move(state)};
+  return S;
 }
 
 // ---------------------------------------------------------------------------------------------------- backward
@@ -573,7 +608,16 @@ const c10::TypedOperatorHandle<BwdSig>& bwd_op() {
 
 std::tuple<Tensor, Tensor, std::vector<Tensor>> fwd_cuda(const Tensor& q, const Tensor& k, const Tensor& v, at::TensorList docs,
                                                          int64_t plan, int64_t /*docs_id*/) {
-  return forward(plan, q, k, v, docs);
+  const Plan& p = plan_at(plan);
+  State s = forward(plan, q, k, v, docs, false);
+  std::vector<Tensor> state = state_list(p, s);
+  const bool has_docs = p.varlen || p.ragged;
+  if (has_docs && !p.aligned) state.insert(state.begin(), s.lse);       // (otherwise the kernels' LSE is the op's output)
+  // the entry handle rides along as a 0-d tensor, so that the backward op needs no object beside its tensors
+  Tensor entry = at::empty({}, at::TensorOptions().dtype(at::kLong));
+  *entry.mutable_data_ptr<int64_t>() = entry_of(plan, has_docs ? s.docs.capacity : -1, has_docs && s.docs.aligned);
+  state.push_back(entry);
+  return {s.out, s.lse_user, std::move(state)};
 }
 std::tuple<Tensor, Tensor, Tensor> bwd_cuda(const Tensor& dout, at::TensorList state, int64_t entry) {
   const Entry e = entry_at(entry);
@@ -631,6 +675,67 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> fwd_autograd(const Tensor& q, co
   return {std::move(out), std::move(lse), std::move(state)};
 }
 
+// Nothing between the caller and the CUDA kernels wants to see the op: no dispatch mode, fake or wrapped tensor, transform or tracer.
+bool direct(std::initializer_list<const Tensor*> ts) {
+  static const c10::DispatchKeySet known =
+      c10::DispatchKeySet({c10::DispatchKey::CUDA, c10::DispatchKey::AutogradCUDA, c10::DispatchKey::ADInplaceOrView,
+                           c10::DispatchKey::BackendSelect}) |
+      c10::autocast_dispatch_keyset;
+  const auto tls = c10::impl::tls_local_dispatch_key_set();
+  c10::DispatchKeySet ks = tls.included_;
+  for (const Tensor* t : ts) ks = ks | t->key_set();
+  return ((ks - tls.excluded_).raw_repr() & ~known.raw_repr()) == 0;
+}
+
+// The node of a call that went to the kernels directly. It saves the call's buffers whole and makes the tensors in them again: a
+// saved tensor can be offloaded, resized or freed without touching another.
+struct DirectNode : public torch::autograd::Function<DirectNode> {
+  static constexpr bool is_traceable = true;         // (as AttnNode; traced, the views and the op are recorded)
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, Call c) {
+    at::AutoDispatchBelowADInplaceOrView below;
+    State s = ::forward(c.plan, q, k, v, c.docs, true);
+    const Docs& d = s.docs;
+    const bool made = d.all.defined();               // (then the tables are views of it)
+    ctx->save_for_backward({s.out, s.lse, s.buf, s.status, s.k_rows, s.v_rows, s.seqused, made ? Tensor() : d.start,
+                            made ? Tensor() : d.len, made ? Tensor() : d.row_map, made ? Tensor() : d.slot_src,
+                            made ? Tensor() : d.slot_rows, d.all, d.work});
+    ctx->saved_data["plan"] = c.plan;
+    ctx->set_materialize_grads(false);
+    *c.lse = std::move(s.lse_user);
+    return s.out;
+  }
+  static variable_list backward(torch::autograd::AutogradContext* ctx, variable_list grads) {
+    if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor(), Tensor()};
+    const int64_t plan = ctx->saved_data["plan"].toInt();
+    const Plan& p = plan_at(plan);
+    const variable_list t = ctx->get_saved_variables();
+    State s;
+    s.status = t[3]; s.k_rows = t[4]; s.v_rows = t[5]; s.seqused = t[6];
+    Docs& d = s.docs;
+    d.start = t[7]; d.len = t[8]; d.row_map = t[9]; d.slot_src = t[10]; d.slot_rows = t[11]; d.all = t[12]; d.work = t[13];
+    const bool has_docs = p.varlen || p.ragged;
+    d.aligned = has_docs && p.aligned;
+    d.capacity = !has_docs ? -1 : d.aligned ? p.tot_q : t[1].size(2);          // (repacked documents: the kernels' LSE, (1, h, capacity))
+    if (d.all.defined()) d.split((d.all.numel() - d.capacity - d.capacity / 128 * 2) / 2);
+    // (a backward that records a graph of its own meets the op, too: it has no derivative, and says so)
+    const bool plain = !at::GradMode::is_enabled() && direct({&grads[0], &t[0], &t[2]});
+    Pool pool(t[2], !plain);
+    operand_tensors(s, p, shapes_of(p, d.capacity), [&](std::initializer_list<int64_t> sz, at::ScalarType dt) { return pool.take(sz, dt); });
+    std::vector<Tensor> state = state_list(p, s);
+    state.insert(state.begin(), {t[0], t[1]});
+    Tensor dq, dk, dv;
+    if (plain) {
+      at::AutoDispatchBelowADInplaceOrView below;
+      RECORD_FUNCTION(p.fp4 ? "lowbit_attn::fp4_bwd" : "lowbit_attn::fp8_bwd", c10::ArrayRef<const c10::IValue>{});
+      std::tie(dq, dk, dv) = ::backward(plan, d.capacity, d.aligned, grads[0], state, Tensor(), Tensor());
+    } else {
+      const auto& op = p.fp4 ? bwd_op<true>() : bwd_op<false>();
+      std::tie(dq, dk, dv) = op.call(grads[0].contiguous(), state, entry_of(plan, d.capacity, d.aligned));
+    }
+    return {dq, dk, dv, Tensor()};
+  }
+};
+
 TORCH_LIBRARY_IMPL(lowbit_attn, CUDA, m) {
   m.impl("fp8", fwd_cuda);
   m.impl("fp4", fwd_cuda);
@@ -644,7 +749,7 @@ TORCH_LIBRARY_IMPL(lowbit_attn, Autograd, m) {
 
 // ---------------------------------------------------------------------------------------------------- Python
 // run(fp4, plan, q, k, v, docs) -> (out, lse): the registered op on a resolved plan, without going through torch.ops (whose
-// argument matching alone costs more than the C++ side of a call)
+// argument matching alone costs more than the C++ side of a call), and without the op where nothing would see it
 PyObject* py_run(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 6 && PyTuple_Check(args[5]), "run(fp4, plan, q, k, v, docs)");
@@ -661,9 +766,21 @@ PyObject* py_run(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Tensor out, lse;
   {
     pybind11::gil_scoped_release nogil;
-    const auto& op = fp4 ? fwd_op<true>() : fwd_op<false>();
-    std::vector<Tensor> state;
-    std::tie(out, lse, state) = op.call(q, k, v, docs, plan, 0);
+    if (direct({&q, &k, &v})) {
+      RECORD_FUNCTION(fp4 ? "lowbit_attn::fp4" : "lowbit_attn::fp8", c10::ArrayRef<const c10::IValue>{});
+      if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) {
+        out = DirectNode::apply(q, k, v, Call{docs, plan, 0, &lse, nullptr});
+      } else {
+        at::AutoDispatchBelowADInplaceOrView below;
+        State s = forward(plan, q, k, v, docs, true);
+        out = std::move(s.out);
+        lse = std::move(s.lse_user);
+      }
+    } else {
+      const auto& op = fp4 ? fwd_op<true>() : fwd_op<false>();
+      std::vector<Tensor> state;
+      std::tie(out, lse, state) = op.call(q, k, v, docs, plan, 0);
+    }
   }
   PyObject* t = PyTuple_New(2);
   PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(out)));

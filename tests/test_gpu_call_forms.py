@@ -184,3 +184,96 @@ def test_compiled_autograd(form):
             torch.compile(lambda: out.backward(x[3]), backend="aot_eager")()
         for a, b in zip((out.detach(), q.grad, k.grad, v.grad), want):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("form", ["batched", "fp4", "rows", "packed", "ragged"])
+def test_state_tensors_have_a_storage_each(form):
+    """What the op returns shares no memory, as its schema says."""
+    import flamia_blackwell_attention_b200 as F
+    import flamia_blackwell_attention_b200.interface_bwd_fp4 as switches
+    from flamia_blackwell_attention_b200 import _op
+    entry = "fp4" if form == "fp4" else "fp8"
+    x = torch.randn(*((600, 2, 128) if form == "packed" else (2, 300 if form == "ragged" else 256, 2, 128)), device="cuda", dtype=torch.bfloat16)
+    kw, docs, was = dict(causal=True), [], (switches.DQ_CAUSAL_PRESCALE, switches.DQ_CAUSAL_GRANULARITY)
+    if form == "packed":
+        cu = torch.tensor([0, 128, 600], dtype=torch.int32, device="cuda")
+        kw.update(cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=472, max_seqlen_k=472)
+        docs = [cu, cu]
+    try:
+        if form == "rows":
+            switches.DQ_CAUSAL_PRESCALE, switches.DQ_CAUSAL_GRANULARITY = True, "row"
+        plan = (F.resolve_fp4 if entry == "fp4" else F.resolve_fp8)(x.requires_grad_(True), x, x, **kw)
+    finally:
+        switches.DQ_CAUSAL_PRESCALE, switches.DQ_CAUSAL_GRANULARITY = was
+    assert plan.bwd.dq_prescale == ("causal_row" if form == "rows" else "row")
+    out, lse, state = getattr(torch.ops.lowbit_attn, entry)(x, x, x, docs, _op.register_plan(plan), 0)
+    every = [t for t in (out, lse, *state) if t.numel()]
+    assert len({t.untyped_storage().data_ptr() for t in every}) == len(every)
+
+
+FORMS = ["batched", "fp4", "seqused", "token", "packed", "maps", "aligned", "ragged", "padded"]
+
+
+def _form(form):
+    """(function, (q, k, v, do), keyword arguments) of one call per form of the saved state."""
+    import flamia_blackwell_attention_b200 as F
+    s, d = 250 if form == "ragged" else 256, 80 if form == "padded" else 128
+    x, kw = [t.cuda() for t in attention_inputs(2, s, 2, 2, d, seed=19)], dict(causal=True)
+    cu = torch.tensor([0, 128, 512], dtype=torch.int32, device="cuda")
+    if form in ("packed", "aligned", "maps"):
+        x = [t.flatten(0, 1) for t in x]
+        kw.update(dict(doc_maps=F.DocMaps.from_cu_seqlens(cu.cpu()).to("cuda")) if form == "maps" else
+                  dict(cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=384, max_seqlen_k=384))
+    if form == "aligned":
+        kw.update(seqused_q=(su := torch.tensor([100, 384], dtype=torch.int32, device="cuda")), seqused_k=su)
+    if form == "seqused":
+        kw.update(seqused_k=torch.tensor([256, 100], dtype=torch.int32, device="cuda"))
+    if form == "token":
+        kw.update(options=F.FP8AttnOptions(operand_scaling="token_local", ds_dq_rowlocal="all"))
+    else:
+        kw.update(deterministic=True)
+    return (F.flash_attn_fp4 if form == "fp4" else F.flash_attn_fp8), x, kw
+
+
+def _same(got, want, form):
+    for i, (a, b) in enumerate(zip(got, want)):
+        # (without deterministic=True the two key tiles' f16 partial sums of dQ may be added in either order: two roundings of 2^-11)
+        assert torch.equal(a, b) or (form == "token" and i == 1 and (a - b).float().norm() <= 2 ** -10 * b.float().norm())
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_saved_tensors_have_a_storage_each_and_can_be_moved(form):
+    fn, x, kw = _form(form)
+    q, k, v = (t.detach().requires_grad_(True) for t in x[:3])
+    out = fn(q, k, v, **kw)
+    want = (out.detach(), *torch.autograd.grad(out, (q, k, v), x[3]))
+    held = []
+
+    def pack(t):
+        held.append(t.untyped_storage().data_ptr())
+        return t.cpu()
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+        out = fn(q, k, v, **kw)
+    assert len(set(held)) == len(held) >= 4
+    _same((out.detach(), *torch.autograd.grad(out, (q, k, v), x[3])), want, form)
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_mode_around_either_pass_sees_the_op(form):
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+    fn, x, kw = _form(form)
+    q, k, v = (t.detach().requires_grad_(True) for t in x[:3])
+    name, runs = f"lowbit_attn.{'fp4' if form == 'fp4' else 'fp8'}", []
+    for around in ((), ("fwd",), ("bwd",), ("fwd", "bwd")):
+        seen = []
+        with Mode() if "fwd" in around else torch.enable_grad():
+            out = fn(q, k, v, **kw)
+        with Mode() if "bwd" in around else torch.enable_grad():
+            runs.append((out.detach(), *torch.autograd.grad(out, (q, k, v), x[3])))
+        assert (f"{name}.default" in seen) == ("fwd" in around) and (f"{name}_bwd.default" in seen) == ("bwd" in around)
+        _same(runs[-1], runs[0], form)
