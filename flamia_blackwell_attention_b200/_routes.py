@@ -111,7 +111,7 @@ def state_spec(plan, n_docs=0, dtype=torch.bfloat16, capacity=None):
     o_rows = s_q
     if docs and not sh.aligned_varlen:      # repacked documents: O has the caller's packed rows
         o_rows = sh.tot_q if sh.varlen else sh.b * sh.s_q
-    spec = [((b, o_rows, h, plan.pad_from or d), dtype), ((b, h, s_q), f32),                                    # O, LSE of the kernels
+    spec = [((b, o_rows, h, plan.pad_from or d), dtype), ((b, h, s_q), f32),                   # O, LSE of the kernels
             ((b, s_q, h, d), f8), ((b, h, s_q // 32), f32), ((b, s_k, hk, d), f8), ((b, hk, s_k // 32), f32),
             ((b, s_k, hk, d), f8), ((b, hk, s_k // 32), f32), ((1,), i32)]                     # codes, factors, status
     if need_bwd:      # K / V statistics of the f16 dQ pre-scale: per 128-row tile and head, or per token

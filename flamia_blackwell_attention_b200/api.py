@@ -22,8 +22,8 @@ __all__ = ["flash_attn_fp4", "flash_attn_fp8"]
 _REPACK_WARNED = False
 REPACK_WARNING = (
     "flash_attn_{entry} got cu_seqlens_q / cu_seqlens_k without seqused_q / seqused_k. No tensor is copied (the kernels "
-    "read and write the packed rows in place), but the document tables are rebuilt on the device on every call (one "
-    "small launch) and the intermediates take a padded buffer of up to 127 extra rows per document. Build the tables "
+    "read and write the packed rows in place), but the document tables are rebuilt on the device on every call (one small "
+    "launch before the quantiser) and the intermediates take a padded buffer of up to 127 extra rows per document. Build the tables "
     "once with DocMaps.from_cu_seqlens(...) and pass doc_maps=, or lay the documents out at starts that are multiples of "
     "128 and pass the true lengths as seqused_q / seqused_k. (Warned once.)")
 
@@ -125,17 +125,12 @@ def _run(call, q, k, v, cu_q, cu_k, su_q, su_k, return_lse, doc_maps=None):
         _REPACK_WARNED = True
         warnings.warn(REPACK_WARNING.format(entry=plan.entry), UserWarning, stacklevel=3)
     if doc_maps is not None:
-        docs = tuple(doc_maps.tensors())    # cu, start, len, row_map, slot_src, slot_rows: nothing is computed per call
+        docs = tuple(doc_maps.tensors())    # cu, start, len, row_map, slot_src, slot_rows: per call only the work lists are made
     else:
         docs = tuple(t for t in (cu_q, cu_k, su_q, su_k) if t is not None) if sh.varlen else \
             ((su_k.contiguous(),) if plan.fwd.seqused_k else ())
     out, lse = _op.op_apply(plan.entry, call.handle, q, k, v, docs)
-    if return_lse:
-        if lse.numel() == 0:
-            _fail("B8", ValueError, "return_lse is served on the batched and the aligned varlen forms, not under "
-                                    "repacked documents")
-        return out, lse
-    return out
+    return (out, lse) if return_lse else out
 
 
 _COMMON_NAMES = ("softmax_scale", "causal", "window_size", "softcap", "score_mod", "score_mod_bwd", "mask_mod", "cu_seqlens_q",

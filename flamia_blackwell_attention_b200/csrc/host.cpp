@@ -6,6 +6,9 @@
 //   forward   1 quantiser launch (Q, K [rotated], V) + 1 forward kernel
 //   backward  1 fused prologue (dO quantiser + D + shifted LSE + zeroed accumulator) + 1 pre-scale + 1 main kernel
 //             + 1 dQ postprocess
+//   also      packed documents: the work lists before the forward, with cu_seqlens the tables before the quantiser, with return_lse
+//             the LSE's way back (a zero fill and a launch); per-token scales: a quantiser launch per operand and V's tables;
+//             per-row pre-scale, ordered dQ: zero fills of their tables, copies of the statistics
 //
 // Why native: the same sequence in Python (ctypes structures, a Python autograd node, one tensor object per table) held a
 // small call (b1 s512 h4 d64, forward and backward) at 600 us of host time for about 60 us of kernels. No host
@@ -514,7 +517,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
     const Tensor& len = next();
     a.doc_len = ptr<int32_t>(len); a.n_docs = (int32_t)len.numel();
     if (repacked) {
-      next();                                  // the row map: the kernels work from the slot tables
+      next();                                  // the row map (part of the op's state; the kernels work from the slot tables)
       slot_src = ptr<int32_t>(next()); slot_rows = ptr<int32_t>(next());
       a.slot_src = slot_src; a.slot_rows = slot_rows; a.out_rows = (int32_t)total;
     }

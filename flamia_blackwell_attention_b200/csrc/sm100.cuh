@@ -2,7 +2,8 @@
 // TMEM load / store / copy), shared-memory and instruction descriptors, and the bounded-wait protocol.
 //
 // Every wait in this library is bounded: a spin that exceeds its cycle budget raises the CTA's abort flag and returns false;
-// the caller unwinds to the common exit where TMEM is released and the kernel's global status word takes a code. A kernel therefore always terminates and the host reads the status word through fl_read_status().
+// the caller unwinds to the common exit where TMEM is released and the kernel's global status word takes a code. A kernel
+// therefore always terminates and the host reads the status word through fl_read_status().
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>

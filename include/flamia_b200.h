@@ -264,7 +264,8 @@ int fl_unpack_lse(const float* lse, const int32_t* slot_src, const int32_t* slot
                   int32_t total, float* out, void* stream);
 
 /* Row gather / scatter between a packed (total, h, d) tensor and its 128-aligned repacked buffer.
- * Replaces flash_attn/cute/lp_varlen.py:421 pack_rows / unpack_rows. row_map[i] = source row of padded row i or -1. */
+ * Replaces flash_attn/cute/lp_varlen.py:421 pack_rows / unpack_rows. row_map[i] = source row of padded row i or -1.
+ * For hosts that keep a padded copy; this library's own calls read and write packed rows in place. */
 int fl_pack_rows(const void* src, void* dst, const int32_t* row_map, int32_t n_dst_rows, int32_t row_bytes, void* stream);
 int fl_unpack_rows(const void* src, void* dst, const int32_t* row_map, int32_t n_src_rows, int32_t row_bytes,
                    void* stream);
