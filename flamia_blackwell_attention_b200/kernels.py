@@ -165,12 +165,12 @@ def attn_args(q, k, v, *, causal, softmax_scale, mode=L.FL_MODE_FP8, flags=0, st
 
 def attn_fwd(q, k, v, *, causal, softmax_scale, out_dtype=torch.bfloat16, mode=L.FL_MODE_FP8, status=None,
              doc_start=None, doc_len=None, wait_cycles=0, token_local=False, window=None, p_group=False, seqused_k=None,
-             softcap=0.0, o_mult=None, packed_out=None):
+             softcap=0.0, o_mult=None, packed_out=None, work=None):
     """Forward kernel on quantised operands. Returns (out (b, s_q, h, d), lse (b, h, s_q) float32, status).
     p_group: group-frame P-hat (one UE8M0 exponent per query row and 32 keys) instead of the row frame.
     o_mult: (b, h_kv) f32 factor on the output rows (the mantissa of a V factor that is no power of two).
     packed_out = (slot_src, slot_rows, total): documents; out is (1, total, h, d) with the documents stored back to back
-    (the kernel writes the caller's packed rows itself); lse keeps the aligned buffer's rows."""
+    (the kernel writes the caller's packed rows itself); lse keeps the aligned buffer's rows. work: the documents' work lists (doc_work)."""
     qc = q["codes"]
     b, s_q, h, d = qc.shape
     dev = qc.device
@@ -196,7 +196,7 @@ def attn_fwd(q, k, v, *, causal, softmax_scale, out_dtype=torch.bfloat16, mode=L
     if token_local:     # log2 f_V and 1 / f_V per key, which the forward applies to every score
         lg, rcp = token_aux(v["token_factors"])
         a.tok_lg_v, a.tok_rcp_v = L.ptr(lg), L.ptr(rcp)
-    L.check(L.load().fl_fwd(C.byref(a), _stream()), "fl_fwd")
+    L.check(L.load().fl_fwd(C.byref(a), _stream()) if work is None else L.load().fl_fwd_work(C.byref(a), L.ptr(work), _stream()), "fl_fwd")
     return out, lse, status
 
 
@@ -281,11 +281,11 @@ def code_stats(codes, descale):
 def attn_bwd(q, k, v, do, *, lse_log2, d_rows, dq_acc, dq_scale, causal, softmax_scale, out_dtype=torch.bfloat16,
              mode=L.FL_MODE_FP8, had_dk=False, status=None, doc_start=None, doc_len=None, wait_cycles=0,
              token_local=False, dq_rowlocal=False, window=None, seqused_k=None, softcap=0.0, dq_order=None,
-             dq_scale_rows=None, dk_mult=None, packed_out=None):
+             dq_scale_rows=None, dk_mult=None, packed_out=None, work=None):
     """Backward main kernel on quantised operands. q / k / v / do: quantiser outputs (codes, fac). Adds the pre-scaled
     dQ partials into the f16 accumulator dq_acc of b * h * s_q * d elements ((b, h, d, s_q) at d = 128, (b, h, s_q, d)
     at d = 64) and returns (dk, dv, status), each (b, s_k, h_kv, d). dq_order: a zeroed (b, h, s_q / 128, 2) int32 table
-    makes the key tiles add their partial sums in ascending key order (bitwise reproducible dQ)."""
+    makes the key tiles add their partial sums in ascending key order (bitwise reproducible dQ; work lists then have to be ordered)."""
     kc = k["codes"]
     b, s_k, h_kv, d = kc.shape
     dev = kc.device
@@ -313,7 +313,7 @@ def attn_bwd(q, k, v, do, *, lse_log2, d_rows, dq_acc, dq_scale, causal, softmax
     if dq_order is not None:
         assert dq_order.dtype == torch.int32 and dq_order.numel() == b * q["codes"].shape[2] * (q["codes"].shape[1] // 128) * 2
         a.dq_order = L.ptr(dq_order)
-    L.check(L.load().fl_bwd(C.byref(a), _stream()), "fl_bwd")
+    L.check(L.load().fl_bwd(C.byref(a), _stream()) if work is None else L.load().fl_bwd_work(C.byref(a), L.ptr(work), _stream()), "fl_bwd")
     return dk, dv, status
 
 

@@ -84,7 +84,8 @@ def test_dq_prescale_of_many_tiles(b, h, hk, nt, causal):
                                      ([640, 128, 256], dict(deterministic=True))])
 def test_work_list_changes_nothing(lens, kw):
     """Documents through fl_doc_work's lists (several chunks of its scan, equal costs, a window, document order) against the kernel's
-    own walk over the document table: O and LSE bit for bit, every pair exactly once."""
+    own walk over the document table: O, LSE, dK and dV bit for bit (with an ordered dQ its accumulator, too), every pair exactly
+    once, in document order or longest first."""
     from flamia_blackwell_attention_b200 import kernels as K
     h, hk, d = 3, 1, 128
     total = sum(lens)
@@ -103,3 +104,34 @@ def test_work_list_changes_nothing(lens, kw):
                               packed_out=(slot_src, slot_rows, total), doc_start=start, doc_len=length)
     live = row_map >= 0
     assert torch.equal(out, want[0]) and torch.equal(st[0][0][:, live], lse[0][:, live])
+    # the order of the lists: as the documents lie (the ordered dQ waits for entries before it), or no block before a longer one
+    left = kw["window_size"][0] if "window_size" in kw else max(lens)
+    for part, rows, n in ((pairs[0], 256, n_f), (pairs[1], 128, n_b)):
+        raw = [tuple(e[:3]) for e in part[:n].tolist()]
+        if kw.get("deterministic"):
+            assert raw == sorted((s, m, b) for s, m, b in raw)
+            continue
+        cost = []
+        for _, m, b in raw:
+            if rows == 256:      # key tiles of both halves of the block, from the window's first key on
+                lo = max(0, b * 256 - left) // 128 * 128
+                cost.append(sum((min(m, b * 256 + i + 128) - lo + 127) // 128 for i in (0, 128) if b * 256 + i < m))
+            else:                # query tiles from the diagonal to the window's last one
+                cost.append(min((m + 127) // 128, (min(m, b * 128 + 128) - 1 + left) // 128 + 1) - b)
+        assert cost == sorted(cost, reverse=True)
+    # the backward, both ways, from the same operands
+    docs = dict(doc_start=start, doc_len=length)
+    g = attention_inputs(1, total, h, hk, d, seed=6)[3][0].cuda()
+    res = []
+    for lists in (None, work):
+        acc = torch.empty(1, h, row_map.numel(), d, dtype=torch.float16, device="cuda")
+        gq = K.quantize_fp8_blocks(g, packed_slots=(slot_src, slot_rows, row_map.numel()), compute_d_with_output=out, shifted_log2_lse_from=st[0],
+                                   log2_lse_shift=8.0, d_multiplier=-2.0 ** -8, zero_accumulator=acc, output_tile_stats=True)
+        ks, _ = K.dq_prescale(gq["tile_stats"], st[9], st[8])
+        order = torch.zeros(1, h, tiles, 2, dtype=torch.int32, device="cuda") if kw.get("deterministic") else None
+        dk, dv, status = K.attn_bwd(*ops, gq, lse_log2=gq["lse_log2"], d_rows=gq["D"], dq_acc=acc, dq_scale=ks, causal=True, softmax_scale=d ** -0.5,
+                                    window=kw.get("window_size"), packed_out=(slot_src, slot_rows, total), dq_order=order, work=lists, **docs)
+        assert K.read_status(status) == 0
+        res.append((dk, dv) + ((acc,) if kw.get("deterministic") else ()))
+    for a, b in zip(*res):
+        assert torch.equal(a, b)
