@@ -151,32 +151,31 @@ NCU_BWD_TRAFFIC_B2 = {"fp8": 163.8e6, "fp4": 221.8e6}
 
 def kernel_calls(q, k, v, g, causal, fp4):
     """The kernel-level calls of one fwd+bwd step on the default route, in order, as (name, function, args, keywords), each run
-    once here for the next ones' operands: the launches of the public call."""
+    once here for the next ones' operands: the six launches of the public call, with the options of its plan."""
     import torch
+    import flamia_blackwell_attention_b200 as F
     from flamia_blackwell_attention_b200 import kernels as K, _lib as L
     b, s, h, d = q.shape
-    sm = 1.0 / math.sqrt(d)
+    plan = (F.resolve_fp4 if fp4 else F.resolve_fp8)(q, k, v, causal=causal)
+    sm, rot, group = plan.softmax_scale, plan.fwd.qk_hadamard, plan.fwd.p_hat_frame == "group"
     mode = L.FL_MODE_FP4 if fp4 else L.FL_MODE_FP8
     calls = []
 
     def call(f, *a, **kw):
         calls.append((f.__name__, f, a, kw))
         return f(*a, **kw)
-    qk = dict(apply_hadamard_rotation=True, hadamard_rotation_scope="nvfp4_copy" if fp4 else "all", also_make_nvfp4_copy=fp4,
-              output_exponent_table=False)
     status = K.new_status(q.device)
-    qq = call(K.quantize_fp8_blocks, q, status=status, **qk)
-    kq = call(K.quantize_fp8_blocks, k, status=status, output_tile_stats=True, **qk)
-    vq = call(K.quantize_fp8_blocks, v, status=status, output_tile_stats=True, output_exponent_table=False)
+    qq, kq, vq = call(K.quantize_qkv, q, k, v, status=status, output_tile_stats=True, output_exponent_table=False,
+                      apply_hadamard_rotation=rot, hadamard_rotation_scope="nvfp4_copy" if fp4 else "all", also_make_nvfp4_copy=fp4)
     out, lse, _ = call(K.attn_fwd, qq, kq, vq, causal=causal, softmax_scale=sm, out_dtype=q.dtype, mode=mode, status=status,
-                       p_group=fp4)
+                       p_group=group)
     acc = torch.empty(b, h, s, d, dtype=torch.float16, device=q.device)
     gq = call(K.quantize_fp8_blocks, g, compute_d_with_output=out, shifted_log2_lse_from=lse, log2_lse_shift=8.0,
               d_multiplier=-2.0 ** -8, zero_accumulator=acc, output_tile_stats=True, status=status, output_exponent_table=False)
     ks, ps = call(K.dq_prescale, gq["tile_stats"], vq["tile_stats"], kq["tile_stats"])
     call(K.attn_bwd, qq, kq, vq, gq, lse_log2=gq["lse_log2"], d_rows=gq["D"], dq_acc=acc, dq_scale=ks, causal=causal,
-         softmax_scale=sm, out_dtype=q.dtype, mode=mode, had_dk=not fp4, status=status)
-    call(K.dq_post, acc, ps, sm, b=b, s=s, h=h, d=d, unrotate=not fp4, out_dtype=q.dtype)
+         softmax_scale=sm, out_dtype=q.dtype, mode=mode, had_dk=rot and not fp4, status=status)
+    call(K.dq_post, acc, ps, sm, b=b, s=s, h=h, d=d, unrotate=rot and not fp4, out_dtype=q.dtype)
     return calls
 
 
@@ -240,8 +239,8 @@ def measure_route(fn, route, causal, tensors, args, world, dist, K, clock_gpu=No
     per = {}
     labels = []
     n_rep = 10
-    for idx, (name, f, a, kw) in enumerate(calls):
-        label = name if name != "quantize_fp8_blocks" else "quant_" + ("q", "k", "v", "do")[min(sum(1 for c in calls[:idx] if c[0] == name), 3)]
+    for name, f, a, kw in calls:
+        label = {"quantize_qkv": "quant_qkv", "quantize_fp8_blocks": "quant_do"}.get(name, name)
         gk = torch.cuda.CUDAGraph()
         keep = []
         with torch.cuda.graph(gk):

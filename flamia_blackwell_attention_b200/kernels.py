@@ -48,6 +48,29 @@ def quantize_fp8_blocks(x, *, apply_hadamard_rotation=False, hadamard_rotation_s
     hadamard_rotation_scope: "all" (codes and NVFP4 copy of the rotated rows) | "nvfp4_copy" (only the NVFP4 copy).
     row_stat = (kind, table): table (b, s) f32, zero on entry, takes per token the maximum over the heads of the row's
     "sumsq" | "amax" | "norm2" (the statistics of the per-query-row causal dQ pre-scale)."""
+    kw = dict(locals())
+    a, out, _keep = _quant_args(kw.pop("x"), **kw)
+    L.check(L.load().fl_quant_blocks(C.byref(a), _stream()), "fl_quant_blocks")
+    return out
+
+
+def quantize_qkv(q, k, v, *, output_tile_stats=False, status=None, output_exponent_table=True, **qk):
+    """Q, K and V of one forward call in one launch (fl_quant_qkv): (q, k, v) outputs as of three quantize_fp8_blocks calls. qk: what
+    Q and K ask for (rotation, NVFP4 copy); output_tile_stats: of K and V."""
+    common = dict(status=status, output_exponent_table=output_exponent_table)
+    (qa, qo, _), (ka, ko, _), (va, vo, _) = [_quant_args(x, **common, **kw) for x, kw in (
+        (q, qk), (k, dict(qk, output_tile_stats=output_tile_stats)), (v, dict(output_tile_stats=output_tile_stats)))]
+    L.check(L.load().fl_quant_qkv(C.byref(qa), C.byref(ka), C.byref(va), _stream()), "fl_quant_qkv")
+    return qo, ko, vo
+
+
+def _quant_args(x, *, apply_hadamard_rotation=False, hadamard_rotation_scope="all", token_local_exponents=False,
+                make_channel_major_copy=False, output_exponent_table=True, output_token_block_factors=True,
+                output_sf_atoms=False, also_make_nvfp4_copy=False, compute_d_with_output=None,
+                shifted_log2_lse_from=None, log2_lse_shift=0.0, d_multiplier=1.0, zero_accumulator=None,
+                output_tile_stats=False, status=None, wait_cycles=0, packed_slots=None, row_stat=None,
+                legacy_kernel=False):
+    """(QuantArgs, outputs, what has to live until the launch) of one operand."""
     _require_cuda(x, "x")
     if x.dtype not in (torch.bfloat16, torch.float16):
         raise TypeError("x must be bf16 or f16")
@@ -96,7 +119,7 @@ def quantize_fp8_blocks(x, *, apply_hadamard_rotation=False, hadamard_rotation_s
         out["x4"] = torch.empty(b, s, h, d // 2, **u8)
         out["sf4_raw"] = torch.empty(b, h, s // 128, d // 64, 32, 4, 4, **u8)
         a.x4, a.sf4 = L.ptr(out["x4"]), L.ptr(out["sf4_raw"])
-    keep = []
+    keep = [x]
     if compute_d_with_output is not None:
         o = compute_d_with_output.contiguous()
         if packed_slots is not None and o.numel() == x.numel():      # the forward output has x's packed rows
@@ -127,11 +150,10 @@ def quantize_fp8_blocks(x, *, apply_hadamard_rotation=False, hadamard_rotation_s
         a.row_stat, a.row_stat_kind = L.ptr(table), {"sumsq": 1, "amax": 2, "norm2": 3}[kind]
     a.lse_shift, a.d_multiplier = float(log2_lse_shift), float(d_multiplier)
     a.status, a.wait_cycles = L.ptr(status), int(wait_cycles)      # status: the call's device status word or None
-    L.check(L.load().fl_quant_blocks(C.byref(a), _stream()), "fl_quant_blocks")
     out["codes"] = out["codes"].view(torch.float8_e4m3fn)
     if "codes_t" in out:
         out["codes_t"] = out["codes_t"].view(torch.float8_e4m3fn)
-    return out
+    return a, out, keep
 
 
 def attn_args(q, k, v, *, causal, softmax_scale, mode=L.FL_MODE_FP8, flags=0, status=None, doc_start=None, doc_len=None,
