@@ -25,6 +25,7 @@
 #include <torch/csrc/utils/pybind.h>
 #include <torch/library.h>
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <deque>
@@ -614,6 +615,8 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> fwd_cuda(const Tensor& q, const 
   const Plan& p = plan_at(plan);
   State s = forward(plan, q, k, v, docs, false);
   std::vector<Tensor> state = state_list(p, s);
+  for (Tensor& t : state)                     // (nor do an op's outputs share memory with its inputs: the tables it was given)
+    if (std::any_of(docs.begin(), docs.end(), [&](const Tensor& d) { return t.is_alias_of(d); })) t = t.clone();
   const bool has_docs = p.varlen || p.ragged;
   if (has_docs && !p.aligned) state.insert(state.begin(), s.lse);       // (otherwise the kernels' LSE is the op's output)
   // the entry handle rides along as a 0-d tensor, so that the backward op needs no object beside its tensors

@@ -186,19 +186,24 @@ def test_compiled_autograd(form):
             assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("form", ["batched", "fp4", "rows", "packed", "ragged"])
+@pytest.mark.parametrize("form", ["batched", "fp4", "rows", "packed", "maps", "aligned", "seqused", "ragged"])
 def test_state_tensors_have_a_storage_each(form):
-    """What the op returns shares no memory, as its schema says."""
+    """What the op returns shares no memory, with its inputs neither, as its schema says."""
     import flamia_blackwell_attention_b200 as F
     import flamia_blackwell_attention_b200.interface_bwd_fp4 as switches
     from flamia_blackwell_attention_b200 import _op
     entry = "fp4" if form == "fp4" else "fp8"
-    x = torch.randn(*((600, 2, 128) if form == "packed" else (2, 300 if form == "ragged" else 256, 2, 128)), device="cuda", dtype=torch.bfloat16)
+    packed = form in ("packed", "maps", "aligned")
+    x = torch.randn(*((640, 2, 128) if packed else (2, 300 if form == "ragged" else 256, 2, 128)), device="cuda", dtype=torch.bfloat16)
     kw, docs, was = dict(causal=True), [], (switches.DQ_CAUSAL_PRESCALE, switches.DQ_CAUSAL_GRANULARITY)
-    if form == "packed":
-        cu = torch.tensor([0, 128, 600], dtype=torch.int32, device="cuda")
-        kw.update(cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=472, max_seqlen_k=472)
-        docs = [cu, cu]
+    if packed:
+        cu = torch.tensor([0, 128, 640], dtype=torch.int32, device="cuda")
+        kw.update(cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=512, max_seqlen_k=512)
+        docs = [cu, cu] if form != "maps" else F.DocMaps.from_cu_seqlens(cu.cpu()).to("cuda").tensors()
+    if form in ("aligned", "seqused"):
+        su = torch.tensor([100, 200], dtype=torch.int32, device="cuda")
+        kw.update(seqused_k=su, **(dict(seqused_q=su) if packed else {}))
+        docs = docs + [su, su] if packed else [su]
     try:
         if form == "rows":
             switches.DQ_CAUSAL_PRESCALE, switches.DQ_CAUSAL_GRANULARITY = True, "row"
@@ -208,7 +213,8 @@ def test_state_tensors_have_a_storage_each(form):
     assert plan.bwd.dq_prescale == ("causal_row" if form == "rows" else "row")
     out, lse, state = getattr(torch.ops.lowbit_attn, entry)(x, x, x, docs, _op.register_plan(plan), 0)
     every = [t for t in (out, lse, *state) if t.numel()]
-    assert len({t.untyped_storage().data_ptr() for t in every}) == len(every)
+    held = {t.untyped_storage().data_ptr() for t in every}
+    assert len(held) == len(every) and not held & {t.untyped_storage().data_ptr() for t in (x, *docs)}
 
 
 FORMS = ["batched", "fp4", "seqused", "token", "packed", "maps", "aligned", "ragged", "padded"]
