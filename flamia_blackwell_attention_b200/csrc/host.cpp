@@ -653,7 +653,7 @@ struct AttnNode : public torch::autograd::Function<AttnNode<FP4>> {
     ctx->save_for_backward(std::move(saved));
     // the capacity of the aligned buffer is in the shapes: repacked documents keep its LSE (1, h, capacity) first
     const bool has_docs = p.varlen || p.ragged, repacked = has_docs && !p.aligned;
-    ctx->saved_data["entry"] = entry_of(c.plan, !has_docs ? -1 : repacked ? state[0].size(2) : p.tot_q, has_docs && p.aligned);
+    ctx->saved_data["entry"] = entry_of(c.plan, !has_docs ? -1 : repacked ? state[0].sym_size(2).guard_int(__FILE__, __LINE__) : p.tot_q, has_docs && p.aligned);
     ctx->saved_data["repacked"] = repacked;
     ctx->set_materialize_grads(false);
     *c.lse = std::move(lse);
@@ -721,8 +721,8 @@ struct DirectNode : public torch::autograd::Function<DirectNode> {
     d.start = t[7]; d.len = t[8]; d.row_map = t[9]; d.slot_src = t[10]; d.slot_rows = t[11]; d.all = t[12]; d.work = t[13];
     const bool has_docs = p.varlen || p.ragged;
     d.aligned = has_docs && p.aligned;
-    d.capacity = !has_docs ? -1 : d.aligned ? p.tot_q : t[1].size(2);          // (repacked documents: the kernels' LSE, (1, h, capacity))
-    if (d.all.defined()) d.split((d.all.numel() - d.capacity - d.capacity / 128 * 2) / 2);
+    d.capacity = !has_docs ? -1 : d.aligned ? p.tot_q : t[1].sym_size(2).guard_int(__FILE__, __LINE__);   // (repacked documents: the kernels' LSE, (1, h, capacity))
+    if (d.all.defined()) d.split((d.all.sym_numel().guard_int(__FILE__, __LINE__) - d.capacity - d.capacity / 128 * 2) / 2);
     // (a backward that records a graph of its own meets the op, too: it has no derivative, and says so)
     const bool plain = !at::GradMode::is_enabled() && direct({&grads[0], &t[0], &t[2]});
     Pool pool(t[2], !plain);

@@ -174,15 +174,29 @@ def test_compiled_autograd(form):
         if form == "aligned":
             su = torch.tensor([100, 384], dtype=torch.int32, device="cuda")
             kw.update(seqused_q=su, seqused_k=su)
-    want = _step(F.flash_attn_fp8, *x, **kw)
-    fn = lambda q, k, v: F.flash_attn_fp8(q, k, v, deterministic=True, **kw)      # noqa: E731
-    for forward in (fn, torch.compile(fn, backend="aot_eager")):
+    for traced in (False, True):
         torch._dynamo.reset()
+        for kw["causal"] in (True, False):               # (the same shapes, another plan: not the first one's trace again)
+            fn = lambda q, k, v: F.flash_attn_fp8(q, k, v, deterministic=True, **kw)      # noqa: E731
+            q, k, v = (t.detach().requires_grad_(True) for t in x[:3])
+            with torch._dynamo.config.patch(compiled_autograd=True):
+                out = (torch.compile(fn, backend="aot_eager") if traced else fn)(q, k, v)
+                torch.compile(lambda: out.backward(x[3]), backend="aot_eager")()
+            for a, b in zip((out.detach(), q.grad, k.grad, v.grad), _step(F.flash_attn_fp8, *x, **kw)):
+                assert torch.equal(a, b)
+
+
+def test_compiled_autograd_with_maps_of_several_sizes():
+    """One plan, buffers of other sizes from call to call (what makes a trace take sizes as symbols)."""
+    import flamia_blackwell_attention_b200 as F
+    x = [t.flatten(0, 1).cuda() for t in attention_inputs(2, 256, 2, 2, 64, seed=20)]
+    for size in (512, 640, 896, 1024):
+        maps = F.DocMaps.from_cu_seqlens(torch.tensor([0, 128, 512]), padded_size=size).to("cuda")
         q, k, v = (t.detach().requires_grad_(True) for t in x[:3])
         with torch._dynamo.config.patch(compiled_autograd=True):
-            out = forward(q, k, v)
+            out = F.flash_attn_fp8(q, k, v, causal=True, deterministic=True, doc_maps=maps)
             torch.compile(lambda: out.backward(x[3]), backend="aot_eager")()
-        for a, b in zip((out.detach(), q.grad, k.grad, v.grad), want):
+        for a, b in zip((out.detach(), q.grad, k.grad, v.grad), _step(F.flash_attn_fp8, *x, causal=True, doc_maps=maps)):
             assert torch.equal(a, b)
 
 
