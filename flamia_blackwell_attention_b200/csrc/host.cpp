@@ -496,10 +496,10 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
   size_t i = 0;
   auto next = [&]() -> const Tensor& {
     TORCH_CHECK(i < state.size(), "the saved state of the forward is incomplete");
+    TORCH_CHECK(state[i].device() == dev, "the saved state of the forward must be on dout's device ", dev, "; got ", state[i].device());
     return state[i++];
   };
   const Tensor &out = next(), &lse = next();
-  TORCH_CHECK(out.device() == dout.device(), "dout is on ", dout.device(), ", the output on ", out.device());
   const Tensor &qc = next(), &qf = next(), &kc = next(), &kf = next(), &vc = next(), &vf = next();
   const Tensor& status = next();
   const Tensor &kstats = next(), &vstats = next();

@@ -278,6 +278,16 @@ def test_saved_tensors_have_a_storage_each_and_can_be_moved(form):
     _same((out.detach(), *torch.autograd.grad(out, (q, k, v), x[3])), want, form)
 
 
+@pytest.mark.parametrize("form", ["batched", "packed"])
+def test_saved_tensors_left_on_the_host_are_refused(form):
+    fn, x, kw = _form(form)
+    q, k, v = (t.detach().requires_grad_(True) for t in x[:3])
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu(), lambda t: t):
+        out = fn(q, k, v, **kw)
+    with pytest.raises(RuntimeError, match="on dout's device"):
+        torch.autograd.grad(out, (q, k, v), x[3])
+
+
 @pytest.mark.parametrize("form", FORMS)
 def test_mode_around_either_pass_sees_the_op(form):
     from torch.utils._python_dispatch import TorchDispatchMode
