@@ -57,6 +57,8 @@ struct FwdParams {
   const float* fac_v;
   const float* tok_lg_v;   // token-local: log2 f_V(key) and 1 / f_V(key), (b, h_kv, s_k)
   const float* tok_rcp_v;
+  const uint32_t* tok_kv;  // token-local, narrow tables of fl_token_tables: f_K (upper half) and log2 f_V as bfloat16 bits, and
+  const uint16_t* tok_r16; // 1 / f_V, (b, h_kv, s_k)
   const uint8_t* sfq4;   // FL_MODE_FP4: E4M3 scale atoms of the NVFP4 Q / K copies, 1 KB per 128-row tile at d = 128
   const uint8_t* sfk4;
   float* lse;
@@ -164,10 +166,15 @@ __device__ __forceinline__ void fwd_decode(const FwdParams& p, int L, Tile& t) {
 
 // FULL: the variants that also serve packed outputs and the output-row factor, each behind a run-time check of its
 // pointer. A template flag, so that the kernels of the plain calls carry none of that code (-2 % kernel time).
-template <int D, bool FP4, bool TL, bool GF, bool SC, bool FULL = false>
+// TLV (token-local): 1 = the per-key factors come from three float tables, 2 = from the narrow ones. What bounds these kernels is the
+// load path: a broadcast load of 16 bytes returns 512 to a warp, and three float tables are 96 of them per 128 keys, the narrow ones
+// 48 (all values are powers of two or small integers: bfloat16 holds them exactly, a shift or a mask takes each one out again, and
+// the results are the same bits). b2 s8192 h32/8 d128 causal, one B200: 1725 -> 1475 us. 1 serves callers of fl_fwd with their own tables.
+template <int D, bool FP4, int TLV, bool GF, bool SC, bool FULL = false>
 __global__ void __launch_bounds__(384, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
            const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const FwdParams p) {
+  constexpr bool TL = TLV != 0;
   constexpr int TILE_BYTES = 128 * D;
   constexpr uint64_t SWZ = (D == 128) ? SWZ_128 : SWZ_64;
   constexpr uint32_t SBO = 8 * D;                       // bytes between 8-row groups
@@ -447,9 +454,13 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         // token-local: the tile's 128 per-key factors (same addresses for every thread: broadcast loads through L1;
         // staging them in shared memory was twice as slow: 384 broadcast reads per thread and tile saturate the
         // shared-memory port that the tensor core's operand reads also go through)
-        const float4* fk4 = reinterpret_cast<const float4*>(p.fac_k + (TL ? tok0 + j * 128 : 0));
-        const float4* lg4 = reinterpret_cast<const float4*>(TL ? p.tok_lg_v + tok0 + j * 128 : p.fac_v);
-        const float4* rc4 = reinterpret_cast<const float4*>(TL ? p.tok_rcp_v + tok0 + j * 128 : p.fac_v);
+        const float4* fk4 = reinterpret_cast<const float4*>(p.fac_k + (TLV == 1 ? tok0 + j * 128 : 0));
+        const float4* lg4 = reinterpret_cast<const float4*>(TLV == 1 ? p.tok_lg_v + tok0 + j * 128 : p.fac_v);
+        const float4* rc4 = reinterpret_cast<const float4*>(TLV == 1 ? p.tok_rcp_v + tok0 + j * 128 : p.fac_v);
+        const uint4* kv4 = reinterpret_cast<const uint4*>(p.tok_kv + (TLV == 2 ? tok0 + j * 128 : 0));
+        const uint4* rc8 = reinterpret_cast<const uint4*>(p.tok_r16 + (TLV == 2 ? tok0 + j * 128 : 0));
+        auto upper = [](uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); };
+        auto lower = [](uint32_t w) { return __uint_as_float(w << 16); };
         if (TL) {
           sfv = 0x7F7F7F7Fu;
 #pragma unroll
@@ -473,7 +484,15 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           for (int e4 = 0; e4 < 32; ++e4) {
             // two columns per instruction; log2 f_V comes from a table (derived here it cost three integer instructions
             // per score on loops that are issue-bound)
-            const float4 k4 = __ldg(fk4 + e4), l4 = __ldg(lg4 + e4);
+            float4 k4, l4;
+            if (TLV == 2) {
+              const uint4 kv = __ldg(kv4 + e4);
+              k4 = make_float4(upper(kv.x), upper(kv.y), upper(kv.z), upper(kv.w));
+              l4 = make_float4(lower(kv.x), lower(kv.y), lower(kv.z), lower(kv.w));
+            } else {
+              k4 = __ldg(fk4 + e4);
+              l4 = __ldg(lg4 + e4);
+            }
             const uint64_t fq2 = pack2(fq, fq);
             unpack2(fma2(pack2(s[4 * e4 + 0], s[4 * e4 + 1]), mul2(pack2(k4.x, k4.y), fq2), pack2(l4.x, l4.y)),
                     s[4 * e4 + 0], s[4 * e4 + 1]);
@@ -550,6 +569,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         float ps[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};     // independent partial sums (group frame: two per group)
         [[maybe_unused]] uint64_t ps2[4] = {0ull, 0ull, 0ull, 0ull};  // the same as packed pairs (default route)
         uint32_t pw[32];
+        [[maybe_unused]] uint4 rc = {0u, 0u, 0u, 0u};
 #pragma unroll
         for (int w = 0; w < 32; ++w) {
           const float cw = c[w >> 3];
@@ -570,7 +590,14 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             p3 = ex2(a3);
           }
           if (TL) {     // the row sum is that of the probabilities: take f_V(key) back out
-            const float4 r4 = __ldg(rc4 + w);
+            float4 r4;
+            if (TLV == 2) {      // eight keys a load
+              if (!(w & 1)) rc = __ldg(rc8 + (w >> 1));
+              const uint32_t a = w & 1 ? rc.z : rc.x, b = w & 1 ? rc.w : rc.y;
+              r4 = make_float4(lower(a), upper(a), lower(b), upper(b));
+            } else {
+              r4 = __ldg(rc4 + w);
+            }
             ps2[w & 3] = fma2(pack2(p0, p1), pack2(r4.x, r4.y), ps2[w & 3]);
             ps2[w & 3] = fma2(pack2(p2, p3), pack2(r4.z, r4.w), ps2[w & 3]);
           } else if (GF) {  // packed: (p0 + p2, p1 + p3) into the group's pair accumulator
@@ -708,7 +735,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 
 }  // namespace fl
 
-static int fwd_launch(const fl_attn_args* a, const void* work, void* stream) {
+static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, const uint32_t* tok_kv = nullptr,
+                      const uint16_t* tok_r16 = nullptr) {
   using namespace fl;
   if (!a || !a->q_codes || !a->k_codes || !a->v_codes || !a->out || !a->status) return FL_ERR_BAD_ARG;
   if (!a->fac_q || !a->fac_k || !a->fac_v) return FL_ERR_BAD_ARG;
@@ -719,7 +747,7 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream) {
   if (fp4 && (!a->q4 || !a->k4 || !a->sfq4 || !a->sfk4)) return FL_ERR_BAD_ARG;
   const bool tl = (a->flags & FL_A_TOKEN_LOCAL) != 0, gf = (a->flags & FL_A_P_GROUP) != 0;
   if (tl && (a->doc_start || a->mode != FL_MODE_FP8)) return FL_ERR_UNSUPPORTED;   // token-local: batched 8-bit route
-  if (tl && (!a->tok_lg_v || !a->tok_rcp_v)) return FL_ERR_BAD_ARG;                 // tables of fl_token_aux over V's factors
+  if (tl && !tok_kv && (!a->tok_lg_v || !a->tok_rcp_v)) return FL_ERR_BAD_ARG;      // tables of fl_token_aux over V's factors
   if (gf && (tl || a->d != 128)) return FL_ERR_UNSUPPORTED;                        // group frame: d = 128, block factors
   if (a->h <= 0 || a->h_kv <= 0 || a->h % a->h_kv) return FL_ERR_BAD_ARG;
   if ((a->s_q % 128) || (a->s_k % 128) || a->s_q <= 0 || a->s_k <= 0 || a->b <= 0) return FL_ERR_BAD_ARG;
@@ -737,7 +765,7 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream) {
   FwdParams p;
   p.fac_q = a->fac_q; p.fac_k = a->fac_k; p.fac_v = a->fac_v; p.lse = a->lse;
   p.sfq4 = a->sfq4; p.sfk4 = a->sfk4;
-  p.tok_lg_v = a->tok_lg_v; p.tok_rcp_v = a->tok_rcp_v;
+  p.tok_lg_v = a->tok_lg_v; p.tok_rcp_v = a->tok_rcp_v; p.tok_kv = tok_kv; p.tok_r16 = tok_r16;
   p.doc_start = a->doc_start; p.doc_len = a->doc_len; p.n_docs = a->n_docs;
   p.seqused_k = a->seqused_k;
   p.o_mult = a->o_mult;
@@ -781,16 +809,17 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream) {
 #define FL_FWD_LAUNCH(D_, FP4_, TL_, GF_, SC_) \
   (full ? launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, true>) : launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, false>))
   if (sc) {
-    if (fp4) rc = gf ? FL_FWD_LAUNCH(128, true, false, true, true) : FL_FWD_LAUNCH(128, true, false, false, true);
-    else if (a->d == 128) rc = gf ? FL_FWD_LAUNCH(128, false, false, true, true) : FL_FWD_LAUNCH(128, false, false, false, true);
-    else rc = FL_FWD_LAUNCH(64, false, false, false, true);
+    if (fp4) rc = gf ? FL_FWD_LAUNCH(128, true, 0, true, true) : FL_FWD_LAUNCH(128, true, 0, false, true);
+    else if (a->d == 128) rc = gf ? FL_FWD_LAUNCH(128, false, 0, true, true) : FL_FWD_LAUNCH(128, false, 0, false, true);
+    else rc = FL_FWD_LAUNCH(64, false, 0, false, true);
   } else if (fp4) {
-    rc = gf ? FL_FWD_LAUNCH(128, true, false, true, false) : FL_FWD_LAUNCH(128, true, false, false, false);
+    rc = gf ? FL_FWD_LAUNCH(128, true, 0, true, false) : FL_FWD_LAUNCH(128, true, 0, false, false);
   } else if (a->d == 128) {
-    rc = tl ? FL_FWD_LAUNCH(128, false, true, false, false)
-            : (gf ? FL_FWD_LAUNCH(128, false, false, true, false) : FL_FWD_LAUNCH(128, false, false, false, false));
+    rc = tl ? (tok_kv ? FL_FWD_LAUNCH(128, false, 2, false, false) : FL_FWD_LAUNCH(128, false, 1, false, false))
+            : (gf ? FL_FWD_LAUNCH(128, false, 0, true, false) : FL_FWD_LAUNCH(128, false, 0, false, false));
   } else {
-    rc = tl ? FL_FWD_LAUNCH(64, false, true, false, false) : FL_FWD_LAUNCH(64, false, false, false, false);
+    rc = tl ? (tok_kv ? FL_FWD_LAUNCH(64, false, 2, false, false) : FL_FWD_LAUNCH(64, false, 1, false, false))
+            : FL_FWD_LAUNCH(64, false, 0, false, false);
   }
 #undef FL_FWD_LAUNCH
   if (rc) return rc;
@@ -801,4 +830,11 @@ extern "C" int fl_fwd(const fl_attn_args* a, void* stream) { return fwd_launch(a
 
 extern "C" int fl_fwd_work(const fl_attn_args* a, const int32_t* work, void* stream) {
   return work ? fwd_launch(a, work, stream) : fl::FL_ERR_BAD_ARG;
+}
+
+extern "C" int fl_fwd_tokens(const fl_attn_args* a, const uint32_t* kv, const uint16_t* rcp, void* stream) {
+  using namespace fl;
+  if (!a || !kv || !rcp || !(a->flags & FL_A_TOKEN_LOCAL)) return FL_ERR_BAD_ARG;
+  if ((reinterpret_cast<uintptr_t>(kv) | reinterpret_cast<uintptr_t>(rcp)) & 15) return FL_ERR_BAD_ARG;     // read 16 bytes at a time
+  return fwd_launch(a, nullptr, stream, kv, rcp);
 }

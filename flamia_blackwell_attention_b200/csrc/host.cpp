@@ -444,11 +444,11 @@ State forward(int64_t handle, const Tensor& q_, const Tensor& k_, const Tensor& 
     a.slot_src = ptr<int32_t>(docs.slot_src); a.slot_rows = ptr<int32_t>(docs.slot_rows); a.out_rows = (int32_t)total;
   }
   Tensor tok;
-  if (p.token_local) {     // log2 f_V and 1 / f_V per key, which the forward applies to every score
+  if (p.token_local) {     // f_K, log2 f_V and 1 / f_V per key, which the forward applies to every score
     const int64_t n = vq.token_factors.numel();
-    tok = empty({2, n}, at::kFloat, dev);
-    check(fl_token_aux(ptr<float>(vq.token_factors), n, ptr<float>(tok), ptr<float>(tok) + n, st), "fl_token_aux");
-    a.tok_lg_v = ptr<float>(tok); a.tok_rcp_v = ptr<float>(tok) + n;
+    tok = empty({3 * n}, at::kShort, dev);
+    check(fl_token_tables(ptr<float>(kq.token_factors), ptr<float>(vq.token_factors), n, ptr<uint32_t>(tok), ptr<uint16_t>(tok) + 2 * n, st),
+          "fl_token_tables");
   }
   if (has_docs) {          // which blocks exist, longest first
     docs.work = empty({FL_DOC_WORK_INTS(docs.capacity)}, at::kInt, dev);
@@ -456,6 +456,8 @@ State forward(int64_t handle, const Tensor& q_, const Tensor& k_, const Tensor& 
                       p.deterministic, ptr<int32_t>(docs.work), stp, st),
           "fl_doc_work");
     check(fl_fwd_work(&a, ptr<int32_t>(docs.work), st), "fl_fwd_work");
+  } else if (p.token_local) {
+    check(fl_fwd_tokens(&a, ptr<uint32_t>(tok), ptr<uint16_t>(tok) + 2 * vq.token_factors.numel(), st), "fl_fwd_tokens");
   } else {
     check(fl_fwd(&a, st), "fl_fwd");
   }

@@ -577,6 +577,28 @@ extern "C" int fl_token_aux(const float* factors, int64_t n, float* lg, float* r
   return launch_result("fl_token_aux: kernel launch");
 }
 
+namespace fl {
+// the same for the forward's narrow tables: f_K and log2 f_V as two bfloat16 in a word, 1 / f_V as one (exact: powers of two, and
+// integers below 128; 1 / 2^127 gives 0 as above)
+__global__ void token_tables_kernel(const float* __restrict__ fk, const float* __restrict__ fv, long long n, uint32_t* __restrict__ kv,
+                                    uint16_t* __restrict__ rcp) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x + grid_dependency();
+  if (i >= n) return;
+  const uint32_t bits = __float_as_uint(fv[i]) & 0x7F800000u;
+  const uint32_t lg = __float_as_uint((float)((int)(bits >> 23) - 127));
+  kv[i] = (__float_as_uint(fk[i]) & 0xFFFF0000u) | (lg >> 16);
+  rcp[i] = (uint16_t)(((254u << 23) - bits) >> 16);
+}
+}  // namespace fl
+
+extern "C" int fl_token_tables(const float* factors_k, const float* factors_v, int64_t n, uint32_t* kv, uint16_t* rcp, void* stream) {
+  using namespace fl;
+  if (!factors_k || !factors_v || !kv || !rcp || n <= 0) return FL_ERR_BAD_ARG;
+  if ((n + 255) / 256 > 0x7FFFFFFF) return FL_ERR_TOO_LARGE;
+  launch_after(token_tables_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, factors_k, factors_v, (long long)n, kv, rcp);
+  return launch_result("fl_token_tables: kernel launch");
+}
+
 extern "C" int fl_code_stats(const void* codes, const float* descale, int32_t b, int32_t s, int32_t h, int32_t d,
                              float* tile_stats, void* stream) {
   using namespace fl;

@@ -222,6 +222,12 @@ int fl_code_stats(const void* codes, const float* descale, int32_t b, int32_t s,
  * fl_attn_args.tok_lg_v / tok_rcp_v. The reference keeps such per-token rows in its (6, b, h, s) token table
  * (flash_attn/cute/lowprec/_routes.py:749-755). */
 int fl_token_aux(const float* factors, int64_t n, float* lg, float* rcp, void* stream);
+
+/* The per-key tables of the token-local forward in half the width: kv[i] = f_K (upper half) and log2 f_V (lower half) as bfloat16
+ * bits, rcp[i] = 1 / f_V as bfloat16 bits, (b, h_kv, s_k) each, 16-byte aligned; all exact. fl_fwd_tokens is fl_fwd with
+ * FL_A_TOKEN_LOCAL on these tables instead of args->tok_lg_v / tok_rcp_v (which are not read): the same results. */
+int fl_token_tables(const float* factors_k, const float* factors_v, int64_t n, uint32_t* kv, uint16_t* rcp, void* stream);
+int fl_fwd_tokens(const fl_attn_args* args, const uint32_t* kv, const uint16_t* rcp, void* stream);
 /* fl_dq_post_rows: post_scale_rows is (b, s), one value per query row. */
 int fl_dq_post_rows(const void* dq_acc, const float* post_scale_rows, float mult, void* dq, int32_t b, int32_t s,
                     int32_t h, int32_t d, int32_t unrotate, int32_t out_f16, void* stream);
