@@ -48,6 +48,8 @@ EXPORTS = {
     "fl_abi_version": (i32, []),
     "fl_quant_blocks": (i32, [C.POINTER(QuantArgs), vp]),
     "fl_quant_qkv": (i32, [C.POINTER(QuantArgs), C.POINTER(QuantArgs), C.POINTER(QuantArgs), vp]),
+    "fl_quant_qkv_work": (i32, [C.POINTER(QuantArgs), C.POINTER(QuantArgs), C.POINTER(QuantArgs), vp, vp, i32, i32, i32, i32, i32, i32, vp,
+                               vp]),
     "fl_fwd": (i32, [C.POINTER(AttnArgs), vp]),
     "fl_bwd": (i32, [C.POINTER(AttnArgs), vp]),
     "fl_dq_prescale": (i32, [vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp, vp, vp]),

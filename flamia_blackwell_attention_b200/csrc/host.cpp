@@ -417,7 +417,15 @@ State forward(int64_t handle, const Tensor& q_, const Tensor& k_, const Tensor& 
   // max |K_j| of the codes' values; where those are rotated, the rotation-invariant 2-norm bounds it
   quantise_args(kq, p, k, sh.b, sh.s_k, p.h_kv, true, dp, k_rows, p.hadamard && !p.fp4 ? 3 : 2, stp);
   quantise_args(vq, p, v, sh.b, sh.s_k, p.h_kv, false, dp, v_rows, 1, stp);
-  check(fl_quant_qkv(&qq.args, &kq.args, &vq.args, st), "fl_quant_qkv");
+  if (has_docs) {          // with them, which blocks exist, longest first
+    docs.work = empty({FL_DOC_WORK_INTS(docs.capacity)}, at::kInt, dev);
+    check(fl_quant_qkv_work(&qq.args, &kq.args, &vq.args, ptr<int32_t>(docs.start), ptr<int32_t>(docs.len), (int32_t)docs.len.numel(),
+                            (int32_t)docs.capacity, p.window_left_p1, p.window_right_p1, p.causal, p.deterministic,
+                            ptr<int32_t>(docs.work), st),
+          "fl_quant_qkv_work");
+  } else {
+    check(fl_quant_qkv(&qq.args, &kq.args, &vq.args, st), "fl_quant_qkv");
+  }
 
   // O has the caller's rows: under repacked documents the kernel writes the packed rows itself. On the aligned form the
   // kernel writes the rows of its documents only, and the padding rows read as zeros. (The LSE of repacked documents keeps
@@ -450,11 +458,7 @@ State forward(int64_t handle, const Tensor& q_, const Tensor& k_, const Tensor& 
     check(fl_token_tables(ptr<float>(kq.token_factors), ptr<float>(vq.token_factors), n, ptr<uint32_t>(tok), ptr<uint16_t>(tok) + 2 * n, st),
           "fl_token_tables");
   }
-  if (has_docs) {          // which blocks exist, longest first
-    docs.work = empty({FL_DOC_WORK_INTS(docs.capacity)}, at::kInt, dev);
-    check(fl_doc_work(a.doc_start, a.doc_len, a.n_docs, (int32_t)docs.capacity, a.window_left_p1, a.window_right_p1, p.causal,
-                      p.deterministic, ptr<int32_t>(docs.work), stp, st),
-          "fl_doc_work");
+  if (has_docs) {
     check(fl_fwd_work(&a, ptr<int32_t>(docs.work), st), "fl_fwd_work");
   } else if (p.token_local) {
     check(fl_fwd_tokens(&a, ptr<uint32_t>(tok), ptr<uint16_t>(tok) + 2 * vq.token_factors.numel(), st), "fl_fwd_tokens");

@@ -14,6 +14,7 @@
 // the same order of operations as a one-thread-per-row butterfly, hence the same bits. The butterflies run as packed
 // f32x2 instructions on register pairs (chunk j, chunk j + 2): one issue slot per two additions, same rounding.
 // Bound: HBM (2 B read + 1 B written per element, plus the optional copies).
+#include "doc_work.cuh"
 #include "flamia_internal.h"
 
 namespace fl {
@@ -528,6 +529,7 @@ struct QuantRowsParams {
   const int32_t* slot_src;   // packed source, see QuantParams
   const int32_t* slot_rows;
   int in_f16;
+  DocWork docs;              // packed source: the documents' work lists, made by block 0 while the others quantise (work null: none)
   DevCtl ctl;
 };
 struct QuantRowsMaps {
@@ -553,7 +555,13 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
   __shared__ int abort_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r = tid;                               // token row of the tile
-  const int G = gridDim.x;
+  if (PK && p.docs.work && blockIdx.x == 0) {
+    static_assert(DOC_WORK_INTS * 4 <= QR_STAGES * QR_TILE_B);
+    grid_dependency();
+    doc_work<128>(p.docs, reinterpret_cast<int*>(smem), p.ctl.status);
+    return;
+  }
+  const int G = gridDim.x - (PK && p.docs.work ? 1 : 0), cta = blockIdx.x - (PK && p.docs.work ? 1 : 0);
   volatile int* abortp = &abort_s;
 
   auto operand_of = [&](int L) { return (p.n_ops > 1 && L >= p.op[1].first) ? ((p.n_ops > 2 && L >= p.op[2].first) ? 2 : 1) : 0; };
@@ -577,13 +585,13 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
     fence_barrier_init();
     grid_dependency();
     for (int i = 0; i < QR_STAGES; ++i)
-      if (blockIdx.x + i * G < p.n_tiles) issue(blockIdx.x + i * G, i);
+      if (cta + i * G < p.n_tiles) issue(cta + i * G, i);
   }
   __syncthreads();
   grid_dependency();
 
   int it = 0;
-  for (int L = blockIdx.x; L < p.n_tiles; L += G, ++it) {
+  for (int L = cta; L < p.n_tiles; L += G, ++it) {
     const int st = it % QR_STAGES, par = it & 1;
     const int oi = operand_of(L);
     const QuantOperand& op = p.op[oi];
@@ -822,7 +830,7 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
 template <int MODE, int D>
 static int launch_quant_rows(const QuantRowsMaps& maps, const QuantRowsParams& p, cudaStream_t st) {
   const int smem = qr_smem(D);
-  const int grid = min(p.n_tiles, sm_count() * qr_ctas(D));
+  const int grid = min(p.n_tiles + (p.docs.work ? 1 : 0), sm_count() * qr_ctas(D));
   auto launch = [&](auto kern) -> int {
     if (int rc = set_smem(kern, smem, "fl_quant_blocks: cudaFuncSetAttribute")) return rc;
     launch_after(kern, grid, 128, smem, st, maps, p);
@@ -877,7 +885,7 @@ static int quant_mode(const fl_quant_args* a) {
   return ((a->flags & FL_Q_HADAMARD) ? 1 : 0) | (a->x4 ? 2 : 0);
 }
 
-static int quant_rows(const fl_quant_args* const* args, int n, cudaStream_t st) {
+static int quant_rows(const fl_quant_args* const* args, int n, cudaStream_t st, const DocWork& docs = {}) {
   QuantRowsMaps maps;
   QuantRowsParams p = {};
   int mode = 0;
@@ -900,6 +908,7 @@ static int quant_rows(const fl_quant_args* const* args, int n, cudaStream_t st) 
   p.n_ops = n; p.n_tiles = (int)tiles;
   p.slot_src = a->slot_src; p.slot_rows = a->slot_rows;
   p.in_f16 = a->in_f16;
+  p.docs = docs;
   p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);
   int rc;
   if (a->d == 64) rc = launch_quant_rows<0, 64>(maps, p, st);
@@ -958,17 +967,40 @@ extern "C" int fl_quant_blocks(const fl_quant_args* a, void* stream) {
   return launch_result("fl_quant_blocks: kernel launch");
 }
 
+namespace fl {
+// do the three go as one launch of the one-thread-per-row kernel?
+static bool one_launch(const fl_quant_args* q, const fl_quant_args* k, const fl_quant_args* v) {
+  const int mq = quant_mode(q), mk = quant_mode(k), mv = quant_mode(v);
+  return rows_kernel_serves(q) && rows_kernel_serves(k) && rows_kernel_serves(v) && mq == mk && mv == 0 && q->d == k->d && q->d == v->d &&
+         q->in_f16 == k->in_f16 && q->in_f16 == v->in_f16 && q->slot_src == k->slot_src && q->slot_src == v->slot_src;
+}
+}  // namespace fl
+
 extern "C" int fl_quant_qkv(const fl_quant_args* q, const fl_quant_args* k, const fl_quant_args* v, void* stream) {
   using namespace fl;
   const fl_quant_args* a[3] = {q, k, v};
   for (const fl_quant_args* x : a)
     if (int rc = check_quant_args(x)) return rc;
-  const int mq = quant_mode(q), mk = quant_mode(k), mv = quant_mode(v);
-  const bool one = rows_kernel_serves(q) && rows_kernel_serves(k) && rows_kernel_serves(v) && mq == mk && mv == 0 && q->d == k->d &&
-                   q->d == v->d && q->in_f16 == k->in_f16 && q->in_f16 == v->in_f16 && q->slot_src == k->slot_src &&
-                   q->slot_src == v->slot_src;
-  if (one) return quant_rows(a, 3, (cudaStream_t)stream);
+  if (one_launch(q, k, v)) return quant_rows(a, 3, (cudaStream_t)stream);
   for (const fl_quant_args* x : a)
     if (int rc = fl_quant_blocks(x, stream)) return rc;
   return FL_OK;
+}
+
+extern "C" int fl_quant_qkv_work(const fl_quant_args* q, const fl_quant_args* k, const fl_quant_args* v, const int32_t* doc_start,
+                                 const int32_t* doc_len, int32_t n_docs, int32_t capacity, int32_t window_left_p1,
+                                 int32_t window_right_p1, int32_t causal, int32_t ordered, int32_t* work, void* stream) {
+  using namespace fl;
+  const fl_quant_args* a[3] = {q, k, v};
+  for (const fl_quant_args* x : a)
+    if (int rc = check_quant_args(x)) return rc;
+  if (!doc_start || !doc_len || !work || n_docs <= 0 || capacity <= 0 || (capacity % 128)) return FL_ERR_BAD_ARG;
+  // One block of 128 threads walks the table and the buffer tiles, eight times as many turns as 1024 threads take: as long as that is
+  // a few dozen turns it hides behind the quantiser (75 tiles: 7 us less a call, above), beyond a launch of its own is the shorter way.
+  if (one_launch(q, k, v) && q->slot_src && n_docs <= 4096 && capacity <= 4096 * 128)
+    return quant_rows(a, 3, (cudaStream_t)stream,
+                      DocWork{doc_start, doc_len, n_docs, capacity, window_side(window_left_p1), causal ? 0 : window_side(window_right_p1),
+                              ordered, (int4*)work});
+  if (int rc = fl_quant_qkv(q, k, v, stream)) return rc;
+  return fl_doc_work(doc_start, doc_len, n_docs, capacity, window_left_p1, window_right_p1, causal, ordered, work, q->status, stream);
 }

@@ -1,4 +1,5 @@
 // HBM-bound side kernels of the backward: f16 dQ pre-scale table, dQ postprocess, packed-row gather / scatter.
+#include "doc_work.cuh"
 #include "flamia_internal.h"
 
 namespace fl {
@@ -324,128 +325,10 @@ __global__ void __launch_bounds__(DT_THREADS) doc_tables_kernel(const int32_t* _
   }
 }
 
-// Work lists of packed documents: the (document, block) pairs that exist, longest first, for the forward (256-row blocks) and the
-// backward (128-key tiles). Entry = {document start, document length, block of it, 0}; header {forward entries, backward entries};
-// capacity / 128 places per list, then capacity / 128 ints of scratch. Without them the attention kernels search the document
-// table once per item, one document after the other (a packed batch of thousands of short documents spent its time there), and
-// walk the documents in their order: a long document at the end left most of the chip idle.
-// One CTA; thread = 128-row tile of the buffer: documents leave their number at their first tile, a prefix maximum spreads it, a
-// counting sort over the cost (key / query tiles visited; 1023 = that or more) places the pairs. ordered: the pairs keep their
-// order (the ordered dQ reduction waits for earlier entries).
-static constexpr int DW_THREADS = 1024, DW_BINS = 1024;
-__global__ void __launch_bounds__(DW_THREADS) doc_work_kernel(const int32_t* __restrict__ doc_start, const int32_t* __restrict__ doc_len,
-                                                              int n_docs, int capacity, int win_l, int win_r, int ordered,
-                                                              int4* __restrict__ work, int* status) {
-  __shared__ int s_bin[2][DW_BINS], s_warp[2][32], s_mark[32];
-  const int tid = threadIdx.x + grid_dependency(), lane = tid & 31, warp = tid >> 5;
-  const int T = capacity / 128;
-  int* mark = reinterpret_cast<int*>(work + 1 + 2 * T);
-  for (int t = tid; t < T; t += DW_THREADS) mark[t] = -1;
-  for (int i = tid; i < DW_BINS; i += DW_THREADS) { s_bin[0][i] = 0; s_bin[1][i] = 0; }
-  __syncthreads();
-  for (int i = tid; i < n_docs; i += DW_THREADS) {
-    int st, len;
-    doc_entry(doc_start, doc_len, i, capacity, status, st, len);
-    if (len > 0) mark[st / 128] = i;
-  }
-  __syncthreads();
-  auto block_exclusive = [&](int v, int (*sums)[32], int which, int& total) {   // exclusive sum over the block (two barriers)
-    int inc = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-      if (lane >= o) inc += u;
-    }
-    if (lane == 31) sums[which][warp] = inc;
-    __syncthreads();
-    int before = 0;
-    total = 0;
-    for (int w = 0; w < DW_THREADS / 32; ++w) { before += w < warp ? sums[which][w] : 0; total += sums[which][w]; }
-    __syncthreads();
-    return before + inc - v;
-  };
-  // a tile's document (from the last mark at or before it), its pairs and their costs
-  struct Pair { int st, len, rel, cf, cb; };
-  auto pair_of = [&](int t, int doc, Pair& q) -> bool {
-    if (t >= T || doc < 0) return false;
-    int st, len;
-    doc_entry(doc_start, doc_len, doc, capacity, nullptr, st, len);
-    const int rel = t * 128 - st;
-    if (rel < 0 || rel >= len) return false;
-    q.st = st; q.len = len; q.rel = rel; q.cf = 0;
-    if (!(rel & 255)) {                             // a forward block starts here
-      const int nq = min(256, len - rel), k_lo = win_l >= 0 ? max(0, rel - win_l) / 128 * 128 : 0;
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int rows = min(128, nq - 128 * i);
-        const int k_hi = win_r >= 0 ? min(len, rel + 128 * i + rows + win_r) : len;
-        if (rows > 0) q.cf += (k_hi - k_lo + 127) / 128;
-      }
-    }
-    int m_hi = (len + 127) / 128, m_lo = 0;
-    if (win_r >= 0 && rel > win_r) m_lo = (rel - win_r) / 128;
-    if (win_l >= 0) m_hi = min(m_hi, (rel + min(128, len - rel) - 1 + win_l) / 128 + 1);
-    q.cb = max(1, m_hi - m_lo);
-    return true;
-  };
-  auto bin_of = [](int cost) { return DW_BINS - 1 - min(cost, DW_BINS - 1); };
-  int carry = -1;                                   // the last mark of the tiles before this chunk
-  for (int t0 = 0; t0 < T; t0 += DW_THREADS) {
-    const int t = t0 + tid;
-    int m = (t < T && mark[t] >= 0) ? t : -1;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xFFFFFFFFu, m, o);
-      if (lane >= o) m = max(m, u);
-    }
-    if (lane == 31) s_mark[warp] = m;
-    __syncthreads();
-    int all = carry;
-    for (int w = 0; w < DW_THREADS / 32; ++w) { if (w < warp) m = max(m, s_mark[w]); all = max(all, s_mark[w]); }
-    m = max(m, carry);
-    const int doc = m >= 0 ? mark[m] : -1;
-    __syncthreads();                                // (a tile with a mark keeps it; the others take the document's number)
-    if (t < T) mark[t] = doc;
-    carry = all;
-    Pair q;
-    if (!ordered && pair_of(t, doc, q)) {
-      if (q.cf) atomicAdd(&s_bin[0][bin_of(q.cf)], 1);
-      atomicAdd(&s_bin[1][bin_of(q.cb)], 1);
-    }
-    __syncthreads();
-  }
-  int n[2] = {0, 0};
-  if (!ordered) {
-#pragma unroll
-    for (int l = 0; l < 2; ++l) {                   // (DW_BINS == DW_THREADS)
-      const int v = s_bin[l][tid];
-      const int at = block_exclusive(v, s_warp, l, n[l]);
-      s_bin[l][tid] = at;
-    }
-    __syncthreads();
-  }
-  for (int t0 = 0; t0 < T; t0 += DW_THREADS) {
-    const int t = t0 + tid;
-    Pair q;
-    const bool live = pair_of(t, t < T ? mark[t] : -1, q);
-    int at[2];
-    if (ordered) {
-#pragma unroll
-      for (int l = 0; l < 2; ++l) {
-        int total;
-        at[l] = n[l] + block_exclusive(live && (l || q.cf), s_warp, l, total);
-        n[l] += total;
-      }
-    } else if (live) {
-      at[0] = q.cf ? atomicAdd(&s_bin[0][bin_of(q.cf)], 1) : 0;
-      at[1] = atomicAdd(&s_bin[1][bin_of(q.cb)], 1);
-    }
-    if (live) {
-      if (q.cf) work[1 + at[0]] = make_int4(q.st, q.len, q.rel / 256, 0);
-      work[1 + T + at[1]] = make_int4(q.st, q.len, q.rel / 128, 0);
-    }
-  }
-  if (tid == 0) work[0] = make_int4(n[0], n[1], 0, 0);
+__global__ void __launch_bounds__(1024) doc_work_kernel(const DocWork w, int* status) {
+  __shared__ int sm[DOC_WORK_INTS];
+  grid_dependency();
+  doc_work<1024>(w, sm, status);
 }
 
 // The live rows of the aligned buffer's LSE (h, capacity) to the caller's rows: packed row g = seq * k + i goes to
@@ -625,8 +508,10 @@ extern "C" int fl_doc_work(const int32_t* doc_start, const int32_t* doc_len, int
                            int32_t window_right_p1, int32_t causal, int32_t ordered, int32_t* work, int32_t* status, void* stream) {
   using namespace fl;
   if (!doc_start || !doc_len || !work || n_docs <= 0 || capacity <= 0 || (capacity % 128)) return FL_ERR_BAD_ARG;
-  launch_after(doc_work_kernel, 1, DW_THREADS, 0, (cudaStream_t)stream, doc_start, doc_len, n_docs, capacity,
-               window_side(window_left_p1), causal ? 0 : window_side(window_right_p1), ordered, (int4*)work, status);
+  launch_after(doc_work_kernel, 1, 1024, 0, (cudaStream_t)stream,
+               DocWork{doc_start, doc_len, n_docs, capacity, window_side(window_left_p1), causal ? 0 : window_side(window_right_p1), ordered,
+                       (int4*)work},
+               status);
   return launch_result("fl_doc_work: kernel launch");
 }
 

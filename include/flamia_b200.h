@@ -260,6 +260,11 @@ int fl_doc_tables(const int32_t* cu, int32_t n_docs, int32_t fixed_len, int32_t 
 #define FL_DOC_WORK_INTS(capacity) (4 + 9 * ((capacity) / 128))
 int fl_doc_work(const int32_t* doc_start, const int32_t* doc_len, int32_t n_docs, int32_t capacity, int32_t window_left_p1,
                 int32_t window_right_p1, int32_t causal, int32_t ordered, int32_t* work, int32_t* status, void* stream);
+/* fl_quant_qkv and fl_doc_work of one call (status: q->status): the lists are made by a block of the quantiser's launch where the three
+ * operands go as one launch. */
+int fl_quant_qkv_work(const fl_quant_args* q, const fl_quant_args* k, const fl_quant_args* v, const int32_t* doc_start,
+                      const int32_t* doc_len, int32_t n_docs, int32_t capacity, int32_t window_left_p1, int32_t window_right_p1,
+                      int32_t causal, int32_t ordered, int32_t* work, void* stream);
 /* fl_fwd / fl_bwd on packed documents with their work lists: the same results */
 int fl_fwd_work(const fl_attn_args* args, const int32_t* work, void* stream);
 int fl_bwd_work(const fl_attn_args* args, const int32_t* work, void* stream);
