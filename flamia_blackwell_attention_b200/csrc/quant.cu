@@ -20,8 +20,13 @@
 namespace fl {
 
 static constexpr int QT = 128;        // tokens per tile
-static constexpr int QTHREADS = 512;  // four lanes per token
 static constexpr int QSTAGES = 3;
+// Threads (four lanes per token) and with them the tokens of a step: a whole tile, or half of one in the prologue. Its two input tiles
+// and 127 registers a thread left room for one block of 512 threads an SM, which waited for itself at every tile's barriers (3.3 us a
+// tile, a third of it work); two blocks of 256 that take a tile in two steps cover each other.
+// One B200, launch alone: b4 s4096 h16 d128 46 -> 40.7 us, b1 s32768 h16 88 -> 77, b2 s8192 h32 token scales 90 -> 77, b2 s2048 h16 d96
+// 15.7 -> 14.2; the smallest calls lose: b1 s512 h4 d64 5.4 -> 6.1.
+constexpr int q_threads(bool pro) { return pro ? 256 : 512; }
 
 struct QuantParams {
   const float* lse;       // (b, h, s) or null
@@ -85,20 +90,22 @@ __device__ __forceinline__ float2 e4m3x2_to_f32(uint16_t v) {
 // MODE bits: 1 = the E4M3 codes are of the rotated rows, 2 = also write the NVFP4 copy, 4 = rotate only the NVFP4 copy
 // PK: packed source (slot tables); a template flag, so that the batched form pays nothing for it
 template <int D, int MODE, bool PRO, bool PK>
-__global__ void __launch_bounds__(QTHREADS, PRO ? 1 : 2)
+__global__ void __launch_bounds__(q_threads(PRO), 2)
 quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_o,
                     const QuantParams p) {
   constexpr bool ROT = (MODE & 1) != 0, NV4 = (MODE & 2) != 0, ROT4 = (MODE & 4) != 0;
   constexpr int NJ = D / 32;                     // 16-byte chunks per lane
   constexpr int NE = 8 * NJ;                     // elements per lane
-  constexpr int TILE_B = QT * D * 2;             // bytes of one 16-bit input tile
+  constexpr int QTHREADS = q_threads(PRO), ROWS = QTHREADS / 4, STEPS = QT / ROWS;     // tokens of a step, steps of a tile
+  constexpr int TILE_B = ROWS * D * 2;           // bytes of one 16-bit input tile (of a step)
   constexpr int STAGE_B = PRO ? 2 * TILE_B : TILE_B;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* s_codes = smem + QSTAGES * STAGE_B;   // channel-major copy only (present when codes_t is asked for)
   __shared__ __align__(8) uint64_t full[QSTAGES];
-  __shared__ float s_wmax[2][16];                // per-warp (8 rows) maximum, double-buffered by tile parity
-  __shared__ float s_wsq[2][16];                 // per-warp maximum row sum of squares
+  // per-warp (8 rows) maximum and largest row sum of squares, by step: a tile's last step reads those of both, while a warp
+  // that is ahead may write the next one's
+  __shared__ float s_wmax[4][QTHREADS / 32], s_wsq[4][QTHREADS / 32];
   __shared__ __align__(16) uint32_t s_sign[4][4][4];   // [lane of the row][chunk][word]: sign bits of the rotation
   __shared__ int abort_s;
 
@@ -106,17 +113,20 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
   // lane -> (row of the warp's eight, lane of the row). The two rows of a quarter warp differ in bit 2, so that with
   // the 128-byte swizzle their 16-byte chunks fall into different bank groups (conflict-free 128-bit loads).
   const int q = lane & 3;
-  const int r = warp * 8 + ((lane >> 2) & 1) * 4 + (lane >> 3);      // token row of the tile
+  const int rs = warp * 8 + ((lane >> 2) & 1) * 4 + (lane >> 3);     // token row of the step
   const int G = gridDim.x;
   const int ntile = p.s / QT;
   volatile int* abortp = &abort_s;
 
-  auto issue = [&](int L, int st) {              // one thread: the loads of linear tile L into stage st
+  auto issue = [&](int n) {                      // one thread: the loads of this block's step n
+    const int L = blockIdx.x + n / STEPS * G, half = n % STEPS * ROWS, st = n % QSTAGES;
+    if (L >= p.n_tiles) return;
     const int head = L % p.h, tile = (L / p.h) % ntile, bat = L / (p.h * ntile);
     uint8_t* dst = smem + st * STAGE_B;
     // packed source (documents stored back to back): the slot's rows start at an arbitrary row of the (1, total, h, d)
     // tensor; only the innermost TMA coordinate has an alignment rule. An empty slot loads nothing of x.
-    const int xrow = PK ? p.slot_src[tile] : tile * QT;
+    int xrow = PK ? p.slot_src[tile] : tile * QT;
+    if (!PK || xrow >= 0) xrow += half;
     mbar_arrive_expect_tx(&full[st], (xrow >= 0 ? TILE_B : 0) + ((PRO && (xrow >= 0 || !(PK && p.o_packed))) ? TILE_B : 0));
     if (xrow >= 0) {
       tma_load_4d(dst, &tm_x, &full[st], 0, head, xrow, bat);
@@ -125,7 +135,7 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     if (PRO) {
       // (packed source: the forward output has the packed rows too; an empty slot's stage keeps what it held, and its
       // rows read as zero below)
-      const int orow = (PK && p.o_packed) ? xrow : tile * QT;
+      const int orow = (PK && p.o_packed) ? xrow : tile * QT + half;
       if (orow >= 0) {
         tma_load_4d(dst + TILE_B, &tm_o, &full[st], 0, head, orow, bat);
         if (D == 128) tma_load_4d(dst + TILE_B + TILE_B / 2, &tm_o, &full[st], 64, head, orow, bat);
@@ -139,8 +149,7 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     tma_prefetch_desc(&tm_x);
     if (PRO) tma_prefetch_desc(&tm_o);
     grid_dependency();
-    for (int i = 0; i < QSTAGES; ++i)
-      if (blockIdx.x + i * G < p.n_tiles) issue(blockIdx.x + i * G, i);
+    for (int n = 0; n < QSTAGES; ++n) issue(n);
   }
   if ((ROT || ROT4) && tid < 16) {               // sign words: bit 15 / 31 of word k = sign of element 2 k / 2 k + 1
     constexpr uint32_t NEG[4] = {0x10D2E03Eu, 0xE0D9F0E2u, 0x45809F07u, 0x75954FEDu};
@@ -157,7 +166,7 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
   auto lds_chunk = [&](uint32_t tile_addr, int j) -> uint4 {
     const int g = 4 * j + q;
     const uint32_t box = (D == 128) ? (uint32_t)(g >> 3) * (TILE_B / 2) : 0u;
-    return lds_u4(tile_addr + box + r * 128 + (((g & 7) ^ (r & 7)) << 4));
+    return lds_u4(tile_addr + box + rs * 128 + (((g & 7) ^ (rs & 7)) << 4));
   };
   // the same for a chunk of x: rows that do not belong to the slot's document (or an empty slot, whose stage holds
   // whatever was there) read as zero
@@ -242,22 +251,26 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     for (int j = 0; j < NJ; ++j) to_f32(lds_chunk_x(tile_addr, j), y + 8 * j);
   };
 
-  int it = 0;
-  for (int L = blockIdx.x; L < p.n_tiles; L += G, ++it) {
-    const int st = it % QSTAGES, par = it & 1;
+  int it = 0;                                    // steps so far
+  for (int L = blockIdx.x; L < p.n_tiles; it % STEPS == STEPS - 1 ? L += G : 0, ++it) {
+    const int st = it % QSTAGES, par = it & 3, step = it % STEPS;
+    const bool whole = step == STEPS - 1;          // with this step the tile's maxima are complete
+    const int r = step * ROWS + rs;                // token row of the tile
     const int head = L % p.h, tile = (L / p.h) % ntile, bat = L / (p.h * ntile);
     const int t0 = tile * QT;
     const size_t row_off = (((size_t)bat * p.s + t0 + r) * p.h + head) * D;     // this row in a (b, s, h, D) tensor
     const size_t bh = (size_t)bat * p.h + head;
     const size_t ri = bh * p.s + t0 + r;
     const uint32_t tile_addr = smem_u32(smem + st * STAGE_B);
+    const float lse_row = q == 0 && p.lse && p.lse_log2 ? p.lse[ri] : 0.f;
+    const int live_rows = PK ? p.slot_rows[tile] : QT;     // (before the wait, which covers the load)
     bool ok = mbar_wait(&full[st], (it / QSTAGES) & 1, p.ctl, abortp, 50);
-    if (PK) row_live = r < p.slot_rows[tile];
+    if (PK) row_live = r < live_rows;
 
     if (p.zero_acc) {   // this tile's share of the accumulator: 128 * D f16 = 32 D 16-byte chunks, contiguous
-      uint4* z = reinterpret_cast<uint4*>(p.zero_acc + (bh * p.s + t0) * D);
+      uint4* z = reinterpret_cast<uint4*>(p.zero_acc + (bh * p.s + t0 + step * ROWS) * D);
       const uint4 zero = make_uint4(0, 0, 0, 0);
-      for (int i = tid; i < QT * D / 8; i += QTHREADS) z[i] = zero;
+      for (int i = tid; i < ROWS * D / 8; i += QTHREADS) z[i] = zero;
     }
 
     // NVFP4 copy of y: per 16 along d (two neighbouring lanes): SF = E4M3_rn(amax * f32(1/6)); codes = E2M1_rn(ftz(y * m)),
@@ -361,11 +374,15 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     // threads together.
     ok = __syncthreads_and(ok ? 1 : 0) != 0;
     if (!ok) break;
-    if (tid == 0 && L + QSTAGES * G < p.n_tiles) issue(L + QSTAGES * G, st);
+    if (tid == 0) issue(it + QSTAGES);
 
-    const float* wm = s_wmax[par];
-    const int blk = r >> 5;                                         // 32-token block of the tile
-    const float bmax = fmaxf(fmaxf(wm[4 * blk], wm[4 * blk + 1]), fmaxf(wm[4 * blk + 2], wm[4 * blk + 3]));
+    // the maximum of 32-token block b of the tile (of this step's or, in the last step, any)
+    auto block_max = [&](int b) -> float {
+      const float* wm = s_wmax[(it - step + b * 32 / ROWS) & 3] + b * 4 % (QTHREADS / 32);
+      return fmaxf(fmaxf(wm[0], wm[1]), fmaxf(wm[2], wm[3]));
+    };
+    const int blk = r >> 5;                                         // this row's
+    const float bmax = block_max(blk);
     const uint32_t bbyte = ue8m0_byte(bmax);
     const bool tl = p.token_local != 0;
     const uint32_t tbyte = tl ? ue8m0_byte(amax) : bbyte;
@@ -431,38 +448,43 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       if (q == 0 && p.d_out) p.d_out[ri] = __fmul_rn(w1, p.d_multiplier);
     }
     if (p.lse && p.lse_log2 && q == 0) {
-      const float l = p.lse[ri];
+      const float l = lse_row;
       p.lse_log2[ri] = __fsub_rn((l == -INFINITY) ? 0.f : __fmul_rn(l, 1.4426950408889634f), p.lse_shift);
     }
 
     // ---- side tables
-    const uint32_t b0 = ue8m0_byte(fmaxf(fmaxf(wm[0], wm[1]), fmaxf(wm[2], wm[3])));
-    const uint32_t b1 = ue8m0_byte(fmaxf(fmaxf(wm[4], wm[5]), fmaxf(wm[6], wm[7])));
-    const uint32_t b2 = ue8m0_byte(fmaxf(fmaxf(wm[8], wm[9]), fmaxf(wm[10], wm[11])));
-    const uint32_t b3 = ue8m0_byte(fmaxf(fmaxf(wm[12], wm[13]), fmaxf(wm[14], wm[15])));
-    if ((tid & 127) == 0) {                          // one thread per 32-token block (tid 128 k: row 32 k, lane 0 of it)
-      if (p.e_tab) {
-        uint8_t* e = p.e_tab + (bh * (p.s / 32) + tile * 4 + blk) * (D / 32);
+    if ((tid & 127) == 0 && p.e_tab) {               // one thread per 32-token block (tid 128 k: row 32 k, lane 0 of it)
+      uint8_t* e = p.e_tab + (bh * (p.s / 32) + tile * 4 + blk) * (D / 32);
 #pragma unroll
-        for (int g = 0; g < D / 32; ++g) e[g] = (uint8_t)bbyte;
-      }
-      if (p.fac) {
-        const uint32_t tm = max(max(b0, b1), max(b2, b3));
-        const uint32_t e0 = bbyte ? bbyte : tm;
-        p.fac[bh * (p.s / 32) + tile * 4 + blk] = e0 ? pow2_from_field((int)e0) : 1.0f;
-      }
+      for (int g = 0; g < D / 32; ++g) e[g] = (uint8_t)bbyte;
+    }
+    uint32_t b0 = 0, b1 = 0, b2 = 0, b3 = 0;         // the tile's four exponents
+    if (whole && (tid < 4 || p.sf_dim)) {
+      b0 = ue8m0_byte(block_max(0));
+      b1 = ue8m0_byte(block_max(1));
+      b2 = ue8m0_byte(block_max(2));
+      b3 = ue8m0_byte(block_max(3));
+    }
+    if (whole && tid < 4 && p.fac) {
+      const uint32_t tm = max(max(b0, b1), max(b2, b3)), own = tid == 0 ? b0 : tid == 1 ? b1 : tid == 2 ? b2 : b3;
+      const uint32_t e0 = own ? own : tm;
+      p.fac[bh * (p.s / 32) + tile * 4 + tid] = e0 ? pow2_from_field((int)e0) : 1.0f;
     }
     if (q == 0) {
       if (p.token_factors) p.token_factors[ri] = tbyte ? scale : 1.0f;
       if (p.sf_tok)
         *reinterpret_cast<uint32_t*>(p.sf_tok + (bh * ntile + tile) * 512 + (r & 31) * 16 + (r >> 5) * 4) = tbyte * 0x01010101u;
     }
-    if (p.sf_dim && tid < 128)
+    if (whole && p.sf_dim && tid < 128)
       *reinterpret_cast<uint32_t*>(p.sf_dim + (bh * ntile + tile) * 512 + tid * 4) = b0 | (b1 << 8) | (b2 << 16) | (b3 << 24);
-    if (p.tile_stats && tid == 0) {
+    if (whole && p.tile_stats && tid == 0) {
       float a = 0.f, sq = 0.f;
 #pragma unroll
-      for (int w = 0; w < 16; ++w) { a = fmaxf(a, wm[w]); sq = fmaxf(sq, s_wsq[par][w]); }
+      for (int w = 0; w < 16; ++w) {
+        const int at = (it - step + w * 8 / ROWS) & 3, ws = w % (QTHREADS / 32);
+        a = fmaxf(a, s_wmax[at][ws]);
+        sq = fmaxf(sq, s_wsq[at][ws]);
+      }
       p.tile_stats[(bh * ntile + tile) * 2] = a;
       p.tile_stats[(bh * ntile + tile) * 2 + 1] = sq;
     }
@@ -473,6 +495,7 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
 #pragma unroll
       for (int j = 0; j < NJ; ++j)
         *reinterpret_cast<uint2*>(s_codes + r * CROWB + (4 * j + q) * 8) = make_uint2(cw[2 * j], cw[2 * j + 1]);
+      if (!whole) continue;
       __syncthreads();
       for (int i = tid; i < D * 8; i += QTHREADS) {  // (channel, 16-token group)
         const int c = i >> 3, rg = (i & 7) * 16;
@@ -552,6 +575,7 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
   constexpr int OUT_STRIDE = OWN ? QR_TILE_B : QR_CODE_B;
   __shared__ __align__(8) uint64_t full[QR_STAGES];
   __shared__ float s_wmax[2][4], s_wsq[2][4];
+  __shared__ __align__(16) uint4 s_zero[PK ? 8 : 1];           // what the rows past a slot's document read
   __shared__ int abort_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r = tid;                               // token row of the tile
@@ -579,6 +603,7 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
       if (D == 128) tma_load_4d(dst + QR_TILE_B / 2, &maps.x[o], &full[st], 64, head, xrow, bat);
     }
   };
+  if (PK && tid < 8) s_zero[tid] = make_uint4(0, 0, 0, 0);
   if (tid == 0) {
     abort_s = 0;
     for (int i = 0; i < QR_STAGES; ++i) mbar_init(&full[i], 1);
@@ -612,13 +637,13 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
     }
     // ---- the row: D / 8 chunks of 8 elements (element 8 g + e in chunk g), rotation signs applied to the raw bits
     float x[D];
+    // (one select of the row's address; of the loaded words it was 64: 16384 packed tokens h16/16 68 -> 66 us, lists included)
+    const uint32_t row_at = PK && !live ? smem_u32(s_zero) : tile_addr + r * 128, box_at = PK && !live ? 0u : (uint32_t)(QR_TILE_B / 2);
     auto load_row = [&](bool signs) {
       constexpr uint32_t NEG[4] = {0x10D2E03Eu, 0xE0D9F0E2u, 0x45809F07u, 0x75954FEDu};
 #pragma unroll
       for (int g = 0; g < D / 8; ++g) {
-        const uint32_t box = (uint32_t)(g >> 3) * (QR_TILE_B / 2);
-        uint4 v = lds_u4(tile_addr + box + r * 128 + (((g & 7) ^ (r & 7)) << 4));
-        if (PK && !live) v = make_uint4(0, 0, 0, 0);
+        const uint4 v = lds_u4(row_at + (g >> 3) * box_at + (((g & 7) ^ (r & 7)) << 4));
         uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -841,13 +866,12 @@ static int launch_quant_rows(const QuantRowsMaps& maps, const QuantRowsParams& p
 
 template <int D, int MODE, bool PRO, bool PK>
 static int launch_quant_pk(const CUtensorMap& mx, const CUtensorMap& mo, const QuantParams& p, bool want_t, cudaStream_t st) {
-  constexpr int TILE_B = QT * D * 2;
-  const int smem = QSTAGES * (PRO ? 2 : 1) * TILE_B + 1024 + (want_t ? QT * (D + 16) : 0);
+  const int smem = QSTAGES * (PRO ? 2 : 1) * (q_threads(PRO) / 4 * D * 2) + 1024 + (want_t ? QT * (D + 16) : 0);
   auto kern = quant_blocks_kernel<D, MODE, PRO, PK>;
   if (int rc = set_smem(kern, smem, "fl_quant_blocks: cudaFuncSetAttribute")) return rc;
-  const int per_sm = (PRO || want_t) ? 1 : 2;
+  const int per_sm = want_t ? 1 : 2;
   const int grid = min(p.n_tiles, sm_count() * per_sm);
-  launch_after(kern, grid, QTHREADS, smem, st, mx, mo, p);
+  launch_after(kern, grid, q_threads(PRO), smem, st, mx, mo, p);
   return FL_OK;
 }
 
@@ -947,9 +971,10 @@ extern "C" int fl_quant_blocks(const fl_quant_args* a, void* stream) {
   p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);
   CUtensorMap mx, mo;
   int rc;
-  if ((rc = make_rows_map_16(&mx, a->x, a->b, packed ? a->src_rows : a->s, a->h, d_src, 128))) return rc;
+  const int box = q_threads(pro) / 4;          // rows of a step
+  if ((rc = make_rows_map_16(&mx, a->x, a->b, packed ? a->src_rows : a->s, a->h, d_src, box))) return rc;
   p.o_packed = (packed && (a->flags & FL_Q_O_PACKED)) ? 1 : 0;
-  if ((rc = make_rows_map_16(&mo, pro ? a->o : a->x, a->b, p.o_packed ? a->src_rows : a->s, a->h, d_src, 128))) return rc;
+  if ((rc = make_rows_map_16(&mo, pro ? a->o : a->x, a->b, p.o_packed ? a->src_rows : a->s, a->h, d_src, box))) return rc;
   const bool wt = a->codes_t != nullptr;
   if (a->d == 64) {
     if (pro) rc = launch_quant<64, 0, true>(mx, mo, p, wt, st);
@@ -996,7 +1021,8 @@ extern "C" int fl_quant_qkv_work(const fl_quant_args* q, const fl_quant_args* k,
     if (int rc = check_quant_args(x)) return rc;
   if (!doc_start || !doc_len || !work || n_docs <= 0 || capacity <= 0 || (capacity % 128)) return FL_ERR_BAD_ARG;
   // One block of 128 threads walks the table and the buffer tiles, eight times as many turns as 1024 threads take: as long as that is
-  // a few dozen turns it hides behind the quantiser (75 tiles: 7 us less a call, above), beyond a launch of its own is the shorter way.
+  // a few dozen turns it hides behind the quantiser (75 tiles: 7 us less a call, above). The line is a bound, not a crossing point:
+  // both sides were measured at 62 to 140 tiles only.
   if (one_launch(q, k, v) && q->slot_src && n_docs <= 4096 && capacity <= 4096 * 128)
     return quant_rows(a, 3, (cudaStream_t)stream,
                       DocWork{doc_start, doc_len, n_docs, capacity, window_side(window_left_p1), causal ? 0 : window_side(window_right_p1),
