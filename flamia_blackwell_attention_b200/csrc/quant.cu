@@ -5,7 +5,7 @@
 // staging :262-300) and the fused NVFP4 copy (flash_attn/cute/quant/_fp8_nvfp4.py:121-158). Outputs are byte-identical to
 // the reference's eager definitions (tests/cute/quant_reference.py:714-798, 270-369).
 //
-// Persistent CTAs (512 threads) walk the (128-token tile, head) pairs of the tensor, heads fastest, so the CTAs running
+// Persistent CTAs (512 threads, the prologue 256) walk the (128-token tile, head) pairs of the tensor, heads fastest, so the CTAs running
 // at any moment read one contiguous stretch of the (b, s, h, d) input. Each CTA keeps STAGES tiles in flight: one thread
 // issues the TMA loads of tile t + STAGES (plain cp.async.bulk.tensor, never multicast) as soon as every thread has read
 // tile t out of its stage, so the memory system stays busy while the butterflies and conversions of the current tile run.
