@@ -5,8 +5,8 @@
 // staging :262-300) and the fused NVFP4 copy (flash_attn/cute/quant/_fp8_nvfp4.py:121-158). Outputs are byte-identical to
 // the reference's eager definitions (tests/cute/quant_reference.py:714-798, 270-369).
 //
-// Persistent CTAs (512 threads, the prologue 256) walk the (128-token tile, head) pairs of the tensor, heads fastest, so the CTAs running
-// at any moment read one contiguous stretch of the (b, s, h, d) input. Each CTA keeps STAGES tiles in flight: one thread
+// Persistent CTAs walk the (128-token tile, head) pairs of the tensor, heads fastest, so the CTAs running at any moment read one
+// contiguous stretch of the (b, s, h, d) input. Each CTA keeps STAGES tiles in flight: one thread
 // issues the TMA loads of tile t + STAGES (plain cp.async.bulk.tensor, never multicast) as soon as every thread has read
 // tile t out of its stage, so the memory system stays busy while the butterflies and conversions of the current tile run.
 // Four lanes share a token row: lane q of the row holds the 16-byte chunks c = 4 j + q (8 elements each); element index
@@ -21,12 +21,11 @@ namespace fl {
 
 static constexpr int QT = 128;        // tokens per tile
 static constexpr int QSTAGES = 3;
-// Threads (four lanes per token) and with them the tokens of a step: a whole tile, or half of one in the prologue. Its two input tiles
-// and 127 registers a thread left room for one block of 512 threads an SM, which waited for itself at every tile's barriers (3.3 us a
-// tile, a third of it work); two blocks of 256 that take a tile in two steps cover each other.
-// One B200, launch alone: b4 s4096 h16 d128 46 -> 40.7 us, b1 s32768 h16 88 -> 77, b2 s8192 h32 token scales 90 -> 77, b2 s2048 h16 d96
-// 15.7 -> 14.2; the smallest calls lose: b1 s512 h4 d64 5.4 -> 6.1.
-constexpr int q_threads(bool pro) { return pro ? 256 : 512; }
+// Threads (four lanes per token) and with them the steps of a tile: one of 512 threads, or in the prologue also two of 256. Its two
+// input tiles and 127 registers a thread leave room for one block of 512 threads an SM, which waits for itself at every tile's
+// barriers; two of 256 cover each other (prologue_steps() says when).
+constexpr int q_threads(int steps) { return 512 / steps; }
+constexpr int q_blocks(bool pro, int steps) { return pro && steps == 1 ? 1 : 2; }      // an SM
 
 struct QuantParams {
   const float* lse;       // (b, h, s) or null
@@ -89,14 +88,14 @@ __device__ __forceinline__ float2 e4m3x2_to_f32(uint16_t v) {
 
 // MODE bits: 1 = the E4M3 codes are of the rotated rows, 2 = also write the NVFP4 copy, 4 = rotate only the NVFP4 copy
 // PK: packed source (slot tables); a template flag, so that the batched form pays nothing for it
-template <int D, int MODE, bool PRO, bool PK>
-__global__ void __launch_bounds__(q_threads(PRO), 2)
+template <int D, int MODE, bool PRO, int STEPS, bool PK>
+__global__ void __launch_bounds__(q_threads(STEPS), q_blocks(PRO, STEPS))
 quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_o,
                     const QuantParams p) {
   constexpr bool ROT = (MODE & 1) != 0, NV4 = (MODE & 2) != 0, ROT4 = (MODE & 4) != 0;
   constexpr int NJ = D / 32;                     // 16-byte chunks per lane
   constexpr int NE = 8 * NJ;                     // elements per lane
-  constexpr int QTHREADS = q_threads(PRO), ROWS = QTHREADS / 4, STEPS = QT / ROWS;     // tokens of a step, steps of a tile
+  constexpr int QTHREADS = q_threads(STEPS), ROWS = QT / STEPS;     // tokens of a step
   constexpr int TILE_B = ROWS * D * 2;           // bytes of one 16-bit input tile (of a step)
   constexpr int STAGE_B = PRO ? 2 * TILE_B : TILE_B;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -458,17 +457,20 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
 #pragma unroll
       for (int g = 0; g < D / 32; ++g) e[g] = (uint8_t)bbyte;
     }
+    // factors: in the prologue's one-step form by the thread that holds the block's exponent (d = 64: 13.6 -> 13.1 us at 8 x 1024 x 12
+    // heads), else by the tile's first four threads
+    constexpr bool OWN_FAC = PRO && STEPS == 1;
     uint32_t b0 = 0, b1 = 0, b2 = 0, b3 = 0;         // the tile's four exponents
-    if (whole && (tid < 4 || p.sf_dim)) {
+    if (OWN_FAC || (whole && (tid < 4 || p.sf_dim))) {
       b0 = ue8m0_byte(block_max(0));
       b1 = ue8m0_byte(block_max(1));
       b2 = ue8m0_byte(block_max(2));
       b3 = ue8m0_byte(block_max(3));
     }
-    if (whole && tid < 4 && p.fac) {
-      const uint32_t tm = max(max(b0, b1), max(b2, b3)), own = tid == 0 ? b0 : tid == 1 ? b1 : tid == 2 ? b2 : b3;
+    if ((OWN_FAC ? (tid & 127) == 0 : whole && tid < 4) && p.fac) {
+      const uint32_t tm = max(max(b0, b1), max(b2, b3)), own = OWN_FAC ? bbyte : tid == 0 ? b0 : tid == 1 ? b1 : tid == 2 ? b2 : b3;
       const uint32_t e0 = own ? own : tm;
-      p.fac[bh * (p.s / 32) + tile * 4 + tid] = e0 ? pow2_from_field((int)e0) : 1.0f;
+      p.fac[bh * (p.s / 32) + tile * 4 + (OWN_FAC ? blk : tid)] = e0 ? pow2_from_field((int)e0) : 1.0f;
     }
     if (q == 0) {
       if (p.token_factors) p.token_factors[ri] = tbyte ? scale : 1.0f;
@@ -864,21 +866,32 @@ static int launch_quant_rows(const QuantRowsMaps& maps, const QuantRowsParams& p
   return p.slot_src ? launch(quant_rows_kernel<MODE, D, true>) : launch(quant_rows_kernel<MODE, D, false>);
 }
 
-template <int D, int MODE, bool PRO, bool PK>
+template <int D, int MODE, bool PRO, int STEPS, bool PK>
 static int launch_quant_pk(const CUtensorMap& mx, const CUtensorMap& mo, const QuantParams& p, bool want_t, cudaStream_t st) {
-  const int smem = QSTAGES * (PRO ? 2 : 1) * (q_threads(PRO) / 4 * D * 2) + 1024 + (want_t ? QT * (D + 16) : 0);
-  auto kern = quant_blocks_kernel<D, MODE, PRO, PK>;
+  const int smem = QSTAGES * (PRO ? 2 : 1) * (QT / STEPS * D * 2) + 1024 + (want_t ? QT * (D + 16) : 0);
+  auto kern = quant_blocks_kernel<D, MODE, PRO, STEPS, PK>;
   if (int rc = set_smem(kern, smem, "fl_quant_blocks: cudaFuncSetAttribute")) return rc;
-  const int per_sm = want_t ? 1 : 2;
+  const int per_sm = want_t ? 1 : q_blocks(PRO, STEPS);
   const int grid = min(p.n_tiles, sm_count() * per_sm);
-  launch_after(kern, grid, q_threads(PRO), smem, st, mx, mo, p);
+  launch_after(kern, grid, q_threads(STEPS), smem, st, mx, mo, p);
   return FL_OK;
 }
 
-template <int D, int MODE, bool PRO>
+template <int D, int MODE, bool PRO, int STEPS = 1>
 static int launch_quant(const CUtensorMap& mx, const CUtensorMap& mo, const QuantParams& p, bool want_t, cudaStream_t st) {
-  return p.slot_src ? launch_quant_pk<D, MODE, PRO, true>(mx, mo, p, want_t, st)
-                    : launch_quant_pk<D, MODE, PRO, false>(mx, mo, p, want_t, st);
+  return p.slot_src ? launch_quant_pk<D, MODE, PRO, STEPS, true>(mx, mo, p, want_t, st)
+                    : launch_quant_pk<D, MODE, PRO, STEPS, false>(mx, mo, p, want_t, st);
+}
+
+// Steps of a prologue tile. Two where both of an SM's blocks have tiles. One where there is no more than a tile an SM, or where in the
+// last round most SMs have one tile only, which a block of 256 then works through with nothing beside it.
+// One B200 (148 SMs), one head, launch in a row, one step / two steps, us at d = 64 (d = 128): 16 tiles 3.4 / 4.1 (4.2 / 4.9), 148 tiles
+// 3.6 / 4.3 (4.4 / 5.1), 296 tiles 5.6 / 5.0 (6.9 / 6.5), 390 tiles 7.5 / 7.8 (9.6 / 9.7), 407 to 444 tiles 7.5 / 8.7 (9.6 / 11.1), 592 tiles
+// 9.5 / 9.0 (12.1 / 11.5), 666 tiles 11.5 / 11.5 (14.8 / 14.4), 740 tiles 11.5 / 12.6 (15.1 / 16.3), 1184 tiles 17.3 / 16.7 (26.3 / 25.4);
+// b4 s4096 h16 d128 41.9 / 43.3, behind a write of O 47.2 / 45.1.
+static int prologue_steps(long long n_tiles) {
+  const int sms = sm_count(), rest = (int)(n_tiles % (2 * sms));
+  return rest > sms || rest == 0 || (n_tiles > 3 * sms && rest <= sms * 2 / 3) ? 2 : 1;
 }
 
 static int quant_cols(const fl_quant_args* a) { return (a->flags >> 16) > 0 ? (a->flags >> 16) : a->d; }
@@ -971,16 +984,16 @@ extern "C" int fl_quant_blocks(const fl_quant_args* a, void* stream) {
   p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);
   CUtensorMap mx, mo;
   int rc;
-  const int box = q_threads(pro) / 4;          // rows of a step
+  const bool wt = a->codes_t != nullptr;
+  const int steps = pro ? prologue_steps(n_tiles) : 1, box = QT / steps;          // rows of a step
   if ((rc = make_rows_map_16(&mx, a->x, a->b, packed ? a->src_rows : a->s, a->h, d_src, box))) return rc;
   p.o_packed = (packed && (a->flags & FL_Q_O_PACKED)) ? 1 : 0;
   if ((rc = make_rows_map_16(&mo, pro ? a->o : a->x, a->b, p.o_packed ? a->src_rows : a->s, a->h, d_src, box))) return rc;
-  const bool wt = a->codes_t != nullptr;
   if (a->d == 64) {
-    if (pro) rc = launch_quant<64, 0, true>(mx, mo, p, wt, st);
+    if (pro) rc = steps == 2 ? launch_quant<64, 0, true, 2>(mx, mo, p, wt, st) : launch_quant<64, 0, true>(mx, mo, p, wt, st);
     else rc = nv4 ? launch_quant<64, 2, false>(mx, mo, p, wt, st) : launch_quant<64, 0, false>(mx, mo, p, wt, st);
   } else if (pro) {
-    rc = launch_quant<128, 0, true>(mx, mo, p, wt, st);
+    rc = steps == 2 ? launch_quant<128, 0, true, 2>(mx, mo, p, wt, st) : launch_quant<128, 0, true>(mx, mo, p, wt, st);
   } else if (rot4) {
     rc = launch_quant<128, 6, false>(mx, mo, p, wt, st);
   } else if (rot) {
