@@ -261,8 +261,9 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     const size_t bh = (size_t)bat * p.h + head;
     const size_t ri = bh * p.s + t0 + r;
     const uint32_t tile_addr = smem_u32(smem + st * STAGE_B);
-    const float lse_row = q == 0 && p.lse && p.lse_log2 ? p.lse[ri] : 0.f;
-    const int live_rows = PK ? p.slot_rows[tile] : QT;     // (before the wait, which covers the load)
+    // before the wait, which covers the loads (the LSE in the prologue alone: b2 s8192 h32 token scales 42.0 -> 41.0 us)
+    const float lse_row = PRO && q == 0 && p.lse && p.lse_log2 ? p.lse[ri] : 0.f;
+    const int live_rows = PK ? p.slot_rows[tile] : QT;
     bool ok = mbar_wait(&full[st], (it / QSTAGES) & 1, p.ctl, abortp, 50);
     if (PK) row_live = r < live_rows;
 
@@ -447,7 +448,7 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       if (q == 0 && p.d_out) p.d_out[ri] = __fmul_rn(w1, p.d_multiplier);
     }
     if (p.lse && p.lse_log2 && q == 0) {
-      const float l = lse_row;
+      const float l = PRO ? lse_row : p.lse[ri];
       p.lse_log2[ri] = __fsub_rn((l == -INFINITY) ? 0.f : __fmul_rn(l, 1.4426950408889634f), p.lse_shift);
     }
 
@@ -888,8 +889,10 @@ static int launch_quant(const CUtensorMap& mx, const CUtensorMap& mo, const Quan
 // One B200 (148 SMs), one head, launch in a row, one step / two steps, us at d = 64 (d = 128): 16 tiles 3.4 / 4.1 (4.2 / 4.9), 148 tiles
 // 3.6 / 4.3 (4.4 / 5.1), 296 tiles 5.6 / 5.0 (6.9 / 6.5), 390 tiles 7.5 / 7.8 (9.6 / 9.7), 407 to 444 tiles 7.5 / 8.7 (9.6 / 11.1), 592 tiles
 // 9.5 / 9.0 (12.1 / 11.5), 666 tiles 11.5 / 11.5 (14.8 / 14.4), 740 tiles 11.5 / 12.6 (15.1 / 16.3), 1184 tiles 17.3 / 16.7 (26.3 / 25.4);
-// b4 s4096 h16 d128 41.9 / 43.3, behind a write of O 47.2 / 45.1.
-static int prologue_steps(long long n_tiles) {
+// b4 s4096 h16 d128 41.9 / 43.3, behind a write of O 47.2 / 45.1. One with the channel-major copy, whose staging rows leave room for one
+// block an SM at d = 128 (b4 s4096 h16, one step / two: 79 / 90 us, at d = 64 48 / 64).
+static int prologue_steps(long long n_tiles, bool want_t) {
+  if (want_t) return 1;
   const int sms = sm_count(), rest = (int)(n_tiles % (2 * sms));
   return rest > sms || rest == 0 || (n_tiles > 3 * sms && rest <= sms * 2 / 3) ? 2 : 1;
 }
@@ -985,7 +988,7 @@ extern "C" int fl_quant_blocks(const fl_quant_args* a, void* stream) {
   CUtensorMap mx, mo;
   int rc;
   const bool wt = a->codes_t != nullptr;
-  const int steps = pro ? prologue_steps(n_tiles) : 1, box = QT / steps;          // rows of a step
+  const int steps = pro ? prologue_steps(n_tiles, wt) : 1, box = QT / steps;          // rows of a step
   if ((rc = make_rows_map_16(&mx, a->x, a->b, packed ? a->src_rows : a->s, a->h, d_src, box))) return rc;
   p.o_packed = (packed && (a->flags & FL_Q_O_PACKED)) ? 1 : 0;
   if ((rc = make_rows_map_16(&mo, pro ? a->o : a->x, a->b, p.o_packed ? a->src_rows : a->s, a->h, d_src, box))) return rc;

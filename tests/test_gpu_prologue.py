@@ -49,6 +49,16 @@ def test_launch_shape(d, rounds, extra, threads, tmp_path):
     assert _threads(lambda: _prologue(x, o, lse), tmp_path) == [(threads, 1, 1)]
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("tiles", [1, 160, 1000])
+def test_channel_major_copy_takes_a_tile_at_once(tiles, d, tmp_path):
+    from flamia_blackwell_attention_b200 import kernels as K
+    x, o, lse = _inputs(1, 128 * tiles, 1, d)
+    got = []
+    assert _threads(lambda: got.append(_prologue(x, o, lse, make_channel_major_copy=True)), tmp_path) == [(512, 1, 1)]
+    _equal(got[0], K.quantize_fp8_blocks(x, make_channel_major_copy=True), ("codes", "codes_t", "fac"), "plain")
+
+
 def _equal(got, want, keys, what):
     for k in keys:
         a, b = (t[k].contiguous().view(torch.uint8) for t in (got, want))
