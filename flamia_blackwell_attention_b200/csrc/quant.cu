@@ -1015,6 +1015,24 @@ static bool one_launch(const fl_quant_args* q, const fl_quant_args* k, const fl_
   return rows_kernel_serves(q) && rows_kernel_serves(k) && rows_kernel_serves(v) && mq == mk && mv == 0 && q->d == k->d && q->d == v->d &&
          q->in_f16 == k->in_f16 && q->in_f16 == v->in_f16 && q->slot_src == k->slot_src && q->slot_src == v->slot_src;
 }
+
+// Work lists: does a block of the quantiser's launch make them in the time that a launch of their own would take? Its 128 threads take
+// eight times as many turns over documents and tiles as the 1024 there. Up to 1536 of these it always does (2560 where the documents
+// are few or short), beyond where the quantiser beside it has work enough: tiles of 64 columns for each tile of the buffer, more of them
+// where full tiles of many documents load the memory (a buffer sized for any division has empty tiles between). Above 4096 it was not
+// measured. One B200, quantiser with the lists / with the launch, us:
+// d = 64, documents of a tile: 75 tiles h16/4 7 us less; 1536 h1/1 30.9 / 31.6; 2048 h1/1 48 / 38, h4/1 64 / 62, h4/2 74 / 78; 3000 h1/1
+//   74 / 53, h4/2 115 / 110, h6/2 131 / 132; 4096 h1/1 104 / 71, h4/2 158 / 147, h6/2 180 / 179;
+// documents of 32 rows: 2048 h1/1 33 / 34; 3000 h2/1 62 / 59, h4/1 76 / 79; 4096 h2/1 92 / 79, h4/1 110 / 106, h4/2 125 / 137;
+// d = 128: 2048 h1/1 61 / 71; 3000 h1/1 98 / 99; 4096 h1/1 136 / 131, h2/1 158 / 169, with NVFP4 copies h1/1 152 / 170;
+// whole forward calls with cu_seqlens (twice as many tiles as documents, each of a tile), d = 64: 1000 documents h1/1 62 / 70, 1500 h1/1
+//   101 / 97, h4/1 236 / 243, 2040 h1/1 137 / 126, h4/1 323 / 327.
+static bool lists_hide(const fl_quant_args* q, const fl_quant_args* k, const fl_quant_args* v, int n_docs, int tiles) {
+  const int most = max(n_docs, tiles);
+  const float full = min((float)n_docs, q->src_rows / 128.f) * min(1.f, (float)n_docs / tiles);
+  const float col = q->d == 128 ? 2.75f : 1.f, score = q->x4 ? 3.75f : col;      // a tile's time in tiles of 64 columns
+  return most <= 1536 || (most <= 2560 && full <= 1100) || (most <= 4096 && score * (q->h + k->h) + col * v->h >= 3.9f + full * (6.f / 4096));
+}
 }  // namespace fl
 
 extern "C" int fl_quant_qkv(const fl_quant_args* q, const fl_quant_args* k, const fl_quant_args* v, void* stream) {
@@ -1036,10 +1054,7 @@ extern "C" int fl_quant_qkv_work(const fl_quant_args* q, const fl_quant_args* k,
   for (const fl_quant_args* x : a)
     if (int rc = check_quant_args(x)) return rc;
   if (!doc_start || !doc_len || !work || n_docs <= 0 || capacity <= 0 || (capacity % 128)) return FL_ERR_BAD_ARG;
-  // One block of 128 threads walks the table and the buffer tiles, eight times as many turns as 1024 threads take: as long as that is
-  // a few dozen turns it hides behind the quantiser (75 tiles: 7 us less a call, above). The line is a bound, not a crossing point:
-  // both sides were measured at 62 to 140 tiles only.
-  if (one_launch(q, k, v) && q->slot_src && n_docs <= 4096 && capacity <= 4096 * 128)
+  if (one_launch(q, k, v) && q->slot_src && lists_hide(q, k, v, n_docs, capacity / 128))
     return quant_rows(a, 3, (cudaStream_t)stream,
                       DocWork{doc_start, doc_len, n_docs, capacity, window_side(window_left_p1), causal ? 0 : window_side(window_right_p1),
                               ordered, (int4*)work});

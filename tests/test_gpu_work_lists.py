@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from inputs import attention_inputs
+from launches import launches
 from test_gpu_call_path import _state
 
 pytestmark = pytest.mark.gpu
@@ -14,7 +15,9 @@ pytestmark = pytest.mark.gpu
     ([1] * 127 + [128 * 130], {}),                                     # more tiles than threads, a document over several chunks
     ([700, 3, 1300, 129], dict(window_size=(200, 0))),
     ([640, 128, 256], dict(deterministic=True)),                       # document order
-    ([1] * 4096, {}),                                                  # the most documents that the quantiser's block takes
+    ([1] * 1536, {}),                                                  # the most documents that the quantiser's block takes at one head
+    ([1] * 1537, {}),
+    ([1] * 4096, {}),
     ([1] * 4097, {}),
 ])
 def test_lists_equal_those_of_their_own_launch(lens, kw):
@@ -34,3 +37,19 @@ def test_lists_equal_those_of_their_own_launch(lens, kw):
         assert sorted(a) == sorted(b)              # (equal costs may change places, except in document order)
         if kw.get("deterministic"):
             assert a == b
+
+
+@pytest.mark.parametrize("docs,rows,h,d,own", [
+    (1536, 128, 1, 64, False), (1537, 128, 1, 64, True), (2048, 128, 4, 64, True), (2048, 128, 6, 64, False), (4096, 128, 6, 64, True),
+    (4096, 128, 8, 64, False), (4097, 128, 8, 64, True),
+    (2200, 64, 1, 64, False), (2300, 64, 1, 64, True), (2561, 1, 1, 64, True), (4096, 1, 2, 64, False), (4096, 32, 2, 64, True),
+    (3000, 128, 1, 128, True), (2048, 128, 1, 128, False), (4096, 128, 2, 128, False),
+])
+def test_long_lists_of_few_heads_are_a_launch_of_their_own(docs, rows, h, d, own, tmp_path):
+    import flamia_blackwell_attention_b200 as F
+    n = docs * rows
+    q, k, v = (torch.zeros(n, i, d, dtype=torch.bfloat16, device="cuda") for i in (h, 1, 1))
+    maps = F.DocMaps.from_cu_seqlens(torch.arange(0, n + 1, rows, dtype=torch.int32), padded_size=docs * 128).to("cuda")
+    with torch.no_grad():
+        names = [name for name, _, _ in launches(lambda: F.flash_attn_fp8(q, k, v, causal=True, doc_maps=maps), tmp_path)]
+    assert any("quant_rows" in name for name in names) and any("doc_work" in name for name in names) == own, names
