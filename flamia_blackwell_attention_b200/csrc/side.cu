@@ -461,8 +461,8 @@ extern "C" int fl_token_aux(const float* factors, int64_t n, float* lg, float* r
 }
 
 namespace fl {
-// the same for the forward's narrow tables: f_K and log2 f_V as two bfloat16 in a word, 1 / f_V as one (exact: powers of two, and
-// integers below 128; 1 / 2^127 gives 0 as above)
+// the same for the forward's narrow tables: f_K and log2 f_V as two bfloat16 in a word, 1 / f_V as one. Of power-of-two factors all
+// exact (powers of two, and integers below 128; 1 / 2^127 gives 0 as above); other factors lose the bits that bfloat16 does not have.
 __global__ void token_tables_kernel(const float* __restrict__ fk, const float* __restrict__ fv, long long n, uint32_t* __restrict__ kv,
                                     uint16_t* __restrict__ rcp) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x + grid_dependency();
