@@ -167,10 +167,11 @@ __device__ __forceinline__ void fwd_decode(const FwdParams& p, int L, Tile& t) {
 // FULL: the variants that also serve packed outputs and the output-row factor, each behind a run-time check of its
 // pointer. A template flag, so that the kernels of the plain calls carry none of that code (-2 % kernel time).
 // TLV (token-local): 1 = the per-key factors come from three float tables, 2 = from the narrow ones. What bounds these kernels is the
-// load path: a broadcast load of 16 bytes returns 512 to a warp, and three float tables are 96 of them per 128 keys, the narrow ones
-// 48 (the quantiser's factors are powers of two, their logarithms small integers: bfloat16 holds them exactly, a shift or a mask takes
-// each one out again, and the results are the same bits). b2 s8192 h32/8 d128 causal, one B200: 1725 -> 1475 us. 1 serves callers of
-// fl_fwd with tables of their own, whose factors may be any numbers.
+// wait for the table loads (long scoreboard 3.0 of the 9.0 clocks a warp takes to an instruction, no pipe above half): a broadcast load
+// of 16 bytes returns 512 to a warp, and three float tables are 96 of them per 128 keys, the narrow ones 48 (the quantiser's factors
+// are powers of two, their logarithms small integers: bfloat16 holds them exactly, a shift or a mask takes each one out again, and the
+// results are the same bits; long scoreboard 1.5 of 6.4). b2 s8192 h32/8 d128 causal, one B200: 1725 -> 1475 us. 1 serves callers of
+// fl_fwd with tables of their own, in 32 bits.
 template <int D, bool FP4, int TLV, bool GF, bool SC, bool FULL = false>
 __global__ void __launch_bounds__(384, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,

@@ -225,8 +225,8 @@ int fl_token_aux(const float* factors, int64_t n, float* lg, float* rcp, void* s
 
 /* The per-key tables of the token-local forward in half the width: kv[i] = f_K (upper half) and log2 f_V (lower half) as bfloat16
  * bits, rcp[i] = 1 / f_V as bfloat16 bits, (b, h_kv, s_k) each, 16-byte aligned. For power-of-two factors
- * (fl_quant_args.token_factors), which these hold exactly; of other factors only f_K's upper 16 bits and f_V's exponent are kept:
- * take fl_fwd with float tables for them. fl_fwd_tokens is fl_fwd with FL_A_TOKEN_LOCAL on these tables instead of
+ * (fl_quant_args.token_factors), which these hold exactly; of another f_K the upper 16 bits are kept (fl_fwd reads all 32), of another
+ * f_V the exponent. fl_fwd_tokens is fl_fwd with FL_A_TOKEN_LOCAL on these tables instead of
  * args->tok_lg_v / tok_rcp_v (which are not read): the same results. */
 int fl_token_tables(const float* factors_k, const float* factors_v, int64_t n, uint32_t* kv, uint16_t* rcp, void* stream);
 int fl_fwd_tokens(const fl_attn_args* args, const uint32_t* kv, const uint16_t* rcp, void* stream);
