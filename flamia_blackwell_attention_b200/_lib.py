@@ -71,6 +71,7 @@ EXPORTS = {
     "fl_token_tables": (i32, [vp, vp, C.c_int64, vp, vp, vp]),
     "fl_fwd_tokens": (i32, [C.POINTER(AttnArgs), vp, vp, vp]),
     "fl_dq_post_cols": (i32, [vp, vp, i32, vp, f32, vp, i32, i32, i32, i32, i32, i32, i32, vp, vp, vp]),
+    "fl_dq_post_trim": (i32, [vp, vp, f32, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp]),
     "fl_dq_post_packed": (i32, [vp, vp, f32, vp, i32, i32, i32, i32, i32, vp, vp, vp]),
     "fl_dq_prescale_rows": (i32, [vp, vp, vp, i32, i32, f32, vp, vp, vp]),
     "fl_doc_tables": (i32, [vp, i32, i32, i32, i32, vp, vp, vp, vp, vp, vp]),

@@ -97,20 +97,16 @@ def state_spec(plan, n_docs=0, dtype=torch.bfloat16, capacity=None):
     tl = f.operand_scaling == "token_local"
     need_bwd = plan.bwd.kernel != "none"
     f8, u8, f32, i32 = torch.float8_e4m3fn, torch.uint8, torch.float32, torch.int32
-    docs = sh.varlen or f.ragged_documents
+    docs = sh.varlen
     if docs:
-        if sh.aligned_varlen:
-            n, cap = n_docs, sh.tot_q
-        else:
-            n, tot = (n_docs, sh.tot_q) if sh.varlen else (sh.b, sh.b * sh.s_q)
-            cap = capacity if capacity is not None else ((tot + 127 * n + 127) // 128) * 128
+        n, cap = n_docs, sh.tot_q
+        if not sh.aligned_varlen:
+            cap = capacity if capacity is not None else ((sh.tot_q + 127 * n + 127) // 128) * 128
         b, s_q, s_k = 1, cap, cap
-    else:
-        b, s_q, s_k = sh.b, sh.s_q, sh.s_k
+    else:                                   # batch rows of whole tiles
+        b, s_q, s_k = sh.b, (sh.s_q + 127) // 128 * 128, (sh.s_k + 127) // 128 * 128
     h, hk, d = sh.h, sh.h_kv, sh.d
-    o_rows = s_q
-    if docs and not sh.aligned_varlen:      # repacked documents: O has the caller's packed rows
-        o_rows = sh.tot_q if sh.varlen else sh.b * sh.s_q
+    o_rows = sh.tot_q if docs else sh.s_q   # (the caller's)
     spec = [((b, o_rows, h, plan.pad_from or d), dtype), ((b, h, s_q), f32),                   # O, LSE of the kernels
             ((b, s_q, h, d), f8), ((b, h, s_q // 32), f32), ((b, s_k, hk, d), f8), ((b, hk, s_k // 32), f32),
             ((b, s_k, hk, d), f8), ((b, hk, s_k // 32), f32), ((1,), i32)]                     # codes, factors, status

@@ -78,6 +78,7 @@ struct BwdParams {
   int32_t* dq_order;     // deterministic dQ: (b, h, s_q / 128, 2) counters, zero on entry, or null
   int n_docs;
   int b, s_q, s_k, h, h_kv;
+  int q_len, k_len;      // batched form: a batch row's queries and keys (s_q, s_k, or fewer where those are rounded up to whole tiles)
   int d_out;             // columns of a gradient row (D, or fewer: zero-padded head dims)
   float scale_log2;
   float softmax_scale;
@@ -161,7 +162,7 @@ __device__ __forceinline__ void bwd_decode(const BwdParams& p, int L, BTile& t) 
     const int q = p.div_item.div(L), rq = L - q * p.div_item.d;
     const int tile = p.causal ? q : rq, rem = p.causal ? rq : q;
     t.bat = p.div_h.div(rem); t.hkv = rem - t.bat * p.h_kv;
-    t.k0 = tile * 128; t.nk = min(128, p.s_k - t.k0); t.krel = t.k0; t.q0 = 0; t.sq = p.s_q; t.off = p.s_k - p.s_q;
+    t.k0 = tile * 128; t.nk = min(128, p.k_len - t.k0); t.krel = t.k0; t.q0 = 0; t.sq = p.q_len; t.off = p.k_len - p.q_len;
     t.nv = p.seqused_k ? min(t.nk, p.seqused_k[t.bat] - t.k0) : t.nk;
   } else {
     // documents sit at 128-aligned starts of one packed batch entry; tile slot x -> (document, key tile of it)
@@ -1258,6 +1259,10 @@ static int bwd_launch(const fl_attn_args* a, const void* work, void* stream) {
   if ((a->s_q % 128) || (a->s_k % 128) || a->s_q <= 0 || a->s_k <= 0 || a->b <= 0) return FL_ERR_BAD_ARG;
   if (a->doc_start && (a->b != 1 || a->n_docs <= 0 || !a->doc_len || a->s_q != a->s_k)) return FL_ERR_BAD_ARG;
   if (a->seqused_k && a->doc_start) return FL_ERR_UNSUPPORTED;      // documents carry their own lengths
+  // batch rows of fewer rows than the whole tiles of the intermediates
+  const bool trim = a->out_rows > 0 && !a->doc_start;
+  if (trim && (a->s_q != a->s_k || a->out_rows > a->s_q || a->out_rows <= a->s_q - 128)) return FL_ERR_BAD_ARG;
+  const int k_len = trim ? a->out_rows : a->s_k;
   CUtensorMap mq, mk, mv, mdo, macc, mq4, mk4, mdk, mdv;
   int rc;
   // (boxes of 64 query rows where a half tile is loaded at a time)
@@ -1277,8 +1282,8 @@ static int bwd_launch(const fl_attn_args* a, const void* work, void* stream) {
   // a box that reaches past a row's last column (zero-padded head dims) stores the columns inside only
   const int d_out = (a->flags >> 16) > 0 ? (a->flags >> 16) : a->d;
   if (d_out > a->d || d_out % 8) return FL_ERR_BAD_ARG;
-  if ((rc = make_rows_map_16(&mdk, a->dk, a->b, a->slot_src ? a->out_rows : a->s_k, a->h_kv, d_out, 128))) return rc;
-  if ((rc = make_rows_map_16(&mdv, a->dv, a->b, a->slot_src ? a->out_rows : a->s_k, a->h_kv, d_out, 128))) return rc;
+  if ((rc = make_rows_map_16(&mdk, a->dk, a->b, a->slot_src ? a->out_rows : k_len, a->h_kv, d_out, 128))) return rc;
+  if ((rc = make_rows_map_16(&mdv, a->dv, a->b, a->slot_src ? a->out_rows : k_len, a->h_kv, d_out, 128))) return rc;
   BwdParams p;
   p.fac_q = a->fac_q; p.fac_k = a->fac_k; p.fac_v = a->fac_v; p.fac_do = a->fac_do; p.lse_log2 = a->lse_log2;
   p.d_rows = a->d_rows; p.dq_scale = a->dq_scale; p.dq_scale_rows = a->dq_scale_rows; p.dk = a->dk; p.dv = a->dv;
@@ -1292,6 +1297,7 @@ static int bwd_launch(const fl_attn_args* a, const void* work, void* stream) {
   p.seqused_k = a->seqused_k;
   p.dq_order = a->dq_order;
   p.b = a->b; p.s_q = a->s_q; p.s_k = a->s_k; p.h = a->h; p.h_kv = a->h_kv; p.d_out = d_out;
+  p.q_len = trim ? k_len : a->s_q; p.k_len = k_len;
   p.softmax_scale = a->softmax_scale;
   p.scale_log2 = a->softmax_scale * 1.4426950408889634f;
   const bool sc = a->softcap > 0.f;

@@ -78,6 +78,7 @@ struct FwdParams {
   float* part;                // split schedule: the partial results
   int n_docs;
   int b, s_q, s_k, h, h_kv;
+  int q_len, k_len;      // batched form: a batch row's queries and keys (s_q, s_k, or fewer where those are rounded up to whole tiles)
   int d_out;             // columns of an output row (D, or fewer: zero-padded head dims)
   float scale_log2;
   float cap_a, cap_b;    // soft cap c: x = cap_a tanh(s * factor * cap_b) in log2 units, cap_a = c log2 e, cap_b = 1 / cap_a
@@ -149,9 +150,9 @@ __device__ __forceinline__ void fwd_decode(const FwdParams& p, int L, Tile& t) {
     const int q = p.div_item.div(L), rq = L - q * p.div_item.d;
     const int blk = p.causal ? p.n_blk - 1 - q : rq, rem = p.causal ? rq : q;
     t.bat = p.div_h.div(rem); t.head = rem - t.bat * p.h;
-    t.q0 = blk * 256; t.nq = min(256, p.s_q - t.q0); t.k0 = 0; t.sk = p.s_k;
-    if (p.seqused_k) t.sk = max(0, min(p.s_k, p.seqused_k[t.bat]));      // keys past it are masked like a document's end
-    t.off = p.s_k - p.s_q; t.qrel = t.q0;
+    t.q0 = blk * 256; t.nq = min(256, p.q_len - t.q0); t.k0 = 0; t.sk = p.k_len;
+    if (p.seqused_k) t.sk = max(0, min(p.k_len, p.seqused_k[t.bat]));    // keys past it are masked like a document's end
+    t.off = p.k_len - p.q_len; t.qrel = t.q0;
   } else {
     // documents sit at 128-aligned starts of one packed batch entry; block slot x -> (document, 256-row block)
     int x = p.div_h.div(L), dsel = -1, blk = 0, len = 0, st = 0;
@@ -877,7 +878,7 @@ __global__ void __launch_bounds__(128) fwd_merge_kernel(const FwdParams p, const
     }
   }
   const float inv = l > 0.f ? 1.0f / l : 0.f;
-  const size_t qrow = (size_t)t.bat * p.s_q + t.q0 + row;
+  const size_t qrow = (size_t)t.bat * p.q_len + t.q0 + row;
   uint16_t* const out = reinterpret_cast<uint16_t*>(p.out) + (qrow * p.h + t.head) * p.d_out;
 #pragma unroll
   for (int e = 0; e < N; e += 2) {
@@ -919,6 +920,10 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, con
   if ((a->s_q % 128) || (a->s_k % 128) || a->s_q <= 0 || a->s_k <= 0 || a->b <= 0) return FL_ERR_BAD_ARG;
   if (a->doc_start && (a->b != 1 || a->n_docs <= 0 || !a->doc_len || a->s_q != a->s_k)) return FL_ERR_BAD_ARG;
   if (a->seqused_k && a->doc_start) return FL_ERR_UNSUPPORTED;      // documents carry their own lengths
+  // batch rows of fewer rows than the whole tiles of the intermediates
+  const bool trim = a->out_rows > 0 && !a->doc_start;
+  if (trim && (a->s_q != a->s_k || a->out_rows > a->s_q || a->out_rows <= a->s_q - 128)) return FL_ERR_BAD_ARG;
+  const int q_len = trim ? a->out_rows : a->s_q;
   CUtensorMap mq, mk, mv, mo;
   int rc;
   if ((rc = make_rows_map(&mq, fp4 ? a->q4 : a->q_codes, a->b, a->s_q, a->h, fp4 ? a->d / 2 : a->d, 128))) return rc;
@@ -927,7 +932,7 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, con
   // a box that reaches past a row's last column (zero-padded head dims) stores the columns inside only
   const int d_out = (a->flags >> 16) > 0 ? (a->flags >> 16) : a->d;
   if (d_out > a->d || d_out % 8) return FL_ERR_BAD_ARG;
-  if ((rc = make_rows_map_16(&mo, a->out, a->b, a->slot_src ? a->out_rows : a->s_q, a->h, d_out, 128))) return rc;
+  if ((rc = make_rows_map_16(&mo, a->out, a->b, a->slot_src ? a->out_rows : q_len, a->h, d_out, 128))) return rc;
   FwdParams p;
   p.fac_q = a->fac_q; p.fac_k = a->fac_k; p.fac_v = a->fac_v; p.lse = a->lse;
   p.sfq4 = a->sfq4; p.sfk4 = a->sfk4;
@@ -939,6 +944,7 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, con
   p.slot_src = a->slot_src; p.slot_rows = a->slot_rows; p.out = a->out;
   if (a->slot_src && (!a->doc_start || !a->slot_rows || a->out_rows <= 0)) return FL_ERR_BAD_ARG;
   p.b = a->b; p.s_q = a->s_q; p.s_k = a->s_k; p.h = a->h; p.h_kv = a->h_kv; p.d_out = d_out;
+  p.q_len = q_len; p.k_len = trim ? q_len : a->s_k;
   p.scale_log2 = a->softmax_scale * 1.4426950408889634f;
   p.causal = (a->flags & FL_A_CAUSAL) ? 1 : 0;
   p.win_l = window_side(a->window_left_p1);
@@ -946,7 +952,7 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, con
   p.out_f16 = (a->flags & FL_A_OUT_F16) ? 1 : 0;
   p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);
   // packed documents: at most one extra 256-row block per document beyond total / 256
-  const int nblk = work ? a->s_q / 128 : a->doc_start ? (a->s_q / 256 + a->n_docs + 1) : (a->s_q + 255) / 256;
+  const int nblk = work ? a->s_q / 128 : a->doc_start ? (a->s_q / 256 + a->n_docs + 1) : (q_len + 255) / 256;
   const int nb = a->doc_start ? 1 : a->b;
   p.n_blk = nblk;
   const long long n_items = (long long)nblk * a->h * nb;
@@ -1036,12 +1042,13 @@ extern "C" int fl_fwd_split_plan(const fl_attn_args* a, int32_t ctas, fl_split* 
   // (under a left window the first key tile of a row is not that of its item; with token factors and outlier channels, where the running
   // maximum is refreshed again and again, pieces would frame some rows otherwise than whole items: 2.5e-2 on gradients)
   if (a->window_left_p1 > 0 || (a->flags & FL_A_TOKEN_LOCAL)) return FL_OK;
-  const int n_blk = (a->s_q + 255) / 256, off = a->s_k - a->s_q;
+  const int s_q = a->out_rows > 0 ? a->out_rows : a->s_q, s_k = a->out_rows > 0 ? a->out_rows : a->s_k;
+  const int n_blk = (s_q + 255) / 256, off = s_k - s_q;
   const bool causal = a->flags & FL_A_CAUSAL;
   const int win_r = causal ? 0 : window_side(a->window_right_p1);
   auto tiles = [&](int blk) {            // as fwd_decode
-    const int q0 = blk * 256, nq = std::min(256, a->s_q - q0);
-    const int to = win_r >= 0 ? std::min<int64_t>(a->s_k, (int64_t)q0 + nq + off + win_r) : a->s_k;
+    const int q0 = blk * 256, nq = std::min(256, s_q - q0);
+    const int to = win_r >= 0 ? std::min<int64_t>(s_k, (int64_t)q0 + nq + off + win_r) : s_k;
     return to > 0 ? (to + 127) / 128 : 0;
   };
   std::vector<int> n(n_blk);

@@ -215,7 +215,7 @@ Docs docs_of(const Plan& p, const Tensor& q, at::TensorList t, bool pooled, cuda
                 "document maps: start / len of one size, slot_src / slot_rows one entry per 128 rows of row_map");
     return d;
   }
-  if (p.varlen && p.aligned) {
+  if (p.aligned) {
     TORCH_CHECK(t.size() == 4, "aligned documents: cu_seqlens_q, cu_seqlens_k, seqused_q, seqused_k");
     d.aligned = true;
     d.start = t[0].slice(0, 0, t[0].size(0) - 1).to(at::kInt).contiguous();
@@ -224,9 +224,9 @@ Docs docs_of(const Plan& p, const Tensor& q, at::TensorList t, bool pooled, cuda
     d.capacity = p.tot_q;
     return d;
   }
-  // cu_seqlens, or batch rows of one length that is no multiple of 128: the tables in one launch
-  TORCH_CHECK(!p.varlen || t.size() >= 1, "packed documents: cu_seqlens");
-  const int64_t n = p.varlen ? t[0].size(0) - 1 : p.b, total = p.varlen ? p.tot_q : p.b * p.s_q;
+  // cu_seqlens: the tables in one launch
+  TORCH_CHECK(t.size() >= 1, "packed documents: cu_seqlens");
+  const int64_t n = t[0].size(0) - 1, total = p.tot_q;
   d.capacity = (total + 127 * n + 127) / 128 * 128;
   const int64_t slots = d.capacity / 128;
   if (pooled) {
@@ -236,8 +236,8 @@ Docs docs_of(const Plan& p, const Tensor& q, at::TensorList t, bool pooled, cuda
     d.start = empty({n}, at::kInt, dev); d.len = empty({n}, at::kInt, dev); d.row_map = empty({d.capacity}, at::kInt, dev);
     d.slot_src = empty({slots}, at::kInt, dev); d.slot_rows = empty({slots}, at::kInt, dev);
   }
-  const Tensor cu = p.varlen ? t[0].to(at::kInt).contiguous() : Tensor();
-  check(fl_doc_tables(ptr<int32_t>(cu), (int32_t)n, (int32_t)(p.varlen ? 0 : p.s_q), (int32_t)total, (int32_t)d.capacity,
+  const Tensor cu = t[0].to(at::kInt).contiguous();
+  check(fl_doc_tables(ptr<int32_t>(cu), (int32_t)n, 0, (int32_t)total, (int32_t)d.capacity,
                       ptr<int32_t>(d.start), ptr<int32_t>(d.len), ptr<int32_t>(d.row_map), ptr<int32_t>(d.slot_src),
                       ptr<int32_t>(d.slot_rows), st),
         "fl_doc_tables");
@@ -280,11 +280,11 @@ class Pool {
   bool traced_ = false;      // through operators, for a program that records them
 };
 
-struct Shapes {            // the kernels' view of the call: one batch entry of `capacity` rows under documents
+struct Shapes {            // the kernels' view of the call: one batch entry of `capacity` rows under documents, batch rows of whole tiles
   int64_t b, s_q, s_k;
 };
 Shapes shapes_of(const Plan& p, int64_t capacity) {
-  return capacity >= 0 ? Shapes{1, capacity, capacity} : Shapes{p.b, p.s_q, p.s_k};
+  return capacity >= 0 ? Shapes{1, capacity, capacity} : Shapes{p.b, (p.s_q + 127) / 128 * 128, (p.s_k + 127) / 128 * 128};
 }
 
 // The outputs of one operand's quantiser: `make` allocates (or sizes) a tensor.
@@ -316,6 +316,8 @@ void quantise_args(Quantised& o, const Plan& p, const Tensor& x, int64_t b, int6
   if (docs && !docs->aligned) {
     a.slot_src = ptr<int32_t>(docs->slot_src); a.slot_rows = ptr<int32_t>(docs->slot_rows);
     a.src_rows = (int32_t)(x.numel() / (heads * p.d_call));
+  } else if (p.ragged) {
+    a.src_rows = (int32_t)p.s_q;
   }
   if (row_stat.defined()) { a.row_stat = ptr<float>(row_stat); a.row_stat_kind = row_stat_kind; }
   a.status = status;
@@ -330,6 +332,7 @@ void attn_common(fl_attn_args& a, const Plan& p, const Shapes& sh, bool f16) {
             (p.d_call != p.d ? FL_A_COLS(p.d_call) : 0);
   a.window_left_p1 = p.window_left_p1; a.window_right_p1 = p.window_right_p1;
   a.softcap = (float)p.softcap;
+  if (p.ragged) a.out_rows = (int32_t)p.s_q;
 }
 
 // One call's tensors: the results in the caller's layout and what the backward needs.
@@ -362,7 +365,7 @@ std::vector<Tensor> state_list(const Plan& p, const State& s) {
   if (p.token_local)
     for (const Quantised* x : {&s.q, &s.k, &s.v}) state.push_back(x->token_factors);
   if (p.seqused_k) state.push_back(s.seqused);
-  if (p.varlen || p.ragged) {
+  if (p.varlen) {
     state.push_back(s.docs.start); state.push_back(s.docs.len);
     if (!s.docs.aligned) { state.push_back(s.docs.row_map); state.push_back(s.docs.slot_src); state.push_back(s.docs.slot_rows); }
     state.push_back(s.docs.work);
@@ -383,6 +386,7 @@ State forward(int64_t handle, const Tensor& q_, const Tensor& k_, const Tensor& 
   const auto dev = q_.device();
   const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
   const Tensor q = rows_of(p, q_), k = rows_of(p, k_), v = rows_of(p, v_);
+  TORCH_CHECK(!p.ragged || p.s_q == p.s_k, "batch rows that are no whole tiles: s_q must equal s_k");
   TORCH_CHECK(q.numel() == (p.varlen ? p.tot_q : p.b * p.s_q) * p.h * p.d_call &&
                   k.numel() == (p.varlen ? p.tot_q : p.b * p.s_k) * p.h_kv * p.d_call &&
                   v.numel() == k.numel() && k.scalar_type() == q.scalar_type() && v.scalar_type() == q.scalar_type(),
@@ -396,7 +400,7 @@ State forward(int64_t handle, const Tensor& q_, const Tensor& k_, const Tensor& 
                 "seqused_k is an int32 tensor of shape (batch,)");
   }
   Docs& docs = S.docs;
-  const bool has_docs = p.varlen || p.ragged;
+  const bool has_docs = p.varlen;
   if (has_docs) docs = docs_of(p, q, docs_in, pooled, st);
   const Docs* dp = has_docs ? &docs : nullptr;
   const bool repacked = has_docs && !docs.aligned;
@@ -455,7 +459,7 @@ State forward(int64_t handle, const Tensor& q_, const Tensor& k_, const Tensor& 
   if (has_docs) {
     a.doc_start = ptr<int32_t>(docs.start); a.doc_len = ptr<int32_t>(docs.len); a.n_docs = (int32_t)docs.len.numel();
   }
-  const int64_t total = p.varlen ? p.tot_q : p.b * p.s_q;
+  const int64_t total = p.tot_q;
   if (repacked) {
     a.slot_src = ptr<int32_t>(docs.slot_src); a.slot_rows = ptr<int32_t>(docs.slot_rows); a.out_rows = (int32_t)total;
   }
@@ -484,16 +488,17 @@ State forward(int64_t handle, const Tensor& q_, const Tensor& k_, const Tensor& 
     if (docs.aligned) {
       lse_user = lse.select(0, 0);            // (h, total_q): the caller's rows are the kernels' rows
     } else if (p.return_lse) {
-      // the kernels' LSE has the aligned buffer's rows; its live rows go to the caller's: (h, total) in packed order, or
-      // (b, h, s) for batch rows that ran as documents
-      lse_user = p.varlen ? empty({p.h, total}, at::kFloat, dev) : empty({p.b, p.h, p.s_q}, at::kFloat, dev);
-      if (p.varlen) lse_user.zero_();         // (rows that no document covers read as zeros)
+      // the kernels' LSE has the aligned buffer's rows; its live rows go to the caller's: (h, total) in packed order
+      lse_user = empty({p.h, total}, at::kFloat, dev);
+      lse_user.zero_();                       // (rows that no document covers read as zeros)
       check(fl_unpack_lse(ptr<float>(lse), ptr<int32_t>(docs.slot_src), ptr<int32_t>(docs.slot_rows), (int32_t)docs.capacity,
-                          (int32_t)p.h, (int32_t)(p.varlen ? total : p.s_q), (int32_t)total, ptr<float>(lse_user), st),
+                          (int32_t)p.h, (int32_t)total, (int32_t)total, ptr<float>(lse_user), st),
             "fl_unpack_lse");
     } else {
       lse_user = empty({0}, at::kFloat, dev);
     }
+  } else if (p.ragged) {                      // (the kernels' LSE has whole tiles of rows)
+    lse_user = p.return_lse ? lse.narrow(2, 0, p.s_q).contiguous() : empty({0}, at::kFloat, dev);
   }
   check_status_if_asked(dev);
   return S;
@@ -531,7 +536,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
   if (p.token_local) { a.fac_q = ptr<float>(next()); a.fac_k = ptr<float>(next()); a.fac_v = ptr<float>(next()); }
   if (p.seqused_k) a.seqused_k = ptr<int32_t>(next());
   const int32_t *slot_src = nullptr, *slot_rows = nullptr, *work = nullptr;
-  const int64_t total = p.varlen ? p.tot_q : p.b * p.s_q;
+  const int64_t total = p.tot_q;
   if (has_docs) {
     a.doc_start = ptr<int32_t>(next());
     const Tensor& len = next();
@@ -576,6 +581,8 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
   if (repacked) {
     g.slot_src = slot_src; g.slot_rows = slot_rows; g.src_rows = (int32_t)total;
     g.flags |= FL_Q_O_PACKED;                  // the forward output has the packed rows
+  } else if (p.ragged) {
+    g.src_rows = (int32_t)p.s_q;
   }
   check(fl_quant_blocks(&g, st), "fl_quant_blocks");
 
@@ -607,7 +614,12 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
   a.status = stp;
   if (work) check(fl_bwd_work(&a, work, st), "fl_bwd_work");
   else check(fl_bwd(&a, st), "fl_bwd");
-  check(fl_dq_post_cols(g.zero_acc, ps, rows, ptr<float>(dq_mult), a.softmax_scale, ptr<void>(dq), (int32_t)sh.b, (int32_t)sh.s_q,
+  if (p.ragged)
+    check(fl_dq_post_trim(g.zero_acc, ps, a.softmax_scale, ptr<void>(dq), (int32_t)sh.b, (int32_t)sh.s_q, (int32_t)p.s_q, (int32_t)p.h,
+                          (int32_t)p.d, (int32_t)p.d_call, had8, f16, st),
+          "fl_dq_post_trim");
+  else
+    check(fl_dq_post_cols(g.zero_acc, ps, rows, ptr<float>(dq_mult), a.softmax_scale, ptr<void>(dq), (int32_t)sh.b, (int32_t)sh.s_q,
                         (int32_t)p.h, (int32_t)p.d, (int32_t)p.d_call, had8, f16, slot_src, slot_rows, st),
         "fl_dq_post_cols");
   check_status_if_asked(dev);
@@ -636,8 +648,8 @@ std::tuple<Tensor, Tensor, std::vector<Tensor>> fwd_cuda(const Tensor& q, const 
   std::vector<Tensor> state = state_list(p, s);
   for (Tensor& t : state)                     // (nor do an op's outputs share memory with its inputs: the tables it was given)
     if (std::any_of(docs.begin(), docs.end(), [&](const Tensor& d) { return t.is_alias_of(d); })) t = t.clone();
-  const bool has_docs = p.varlen || p.ragged;
-  if (has_docs && !p.aligned) state.insert(state.begin(), s.lse);       // (otherwise the kernels' LSE is the op's output)
+  const bool has_docs = p.varlen;
+  if ((has_docs && !p.aligned) || p.ragged) state.insert(state.begin(), s.lse);       // (otherwise the kernels' LSE is the op's output)
   // the entry handle rides along as a 0-d tensor, so that the backward op needs no object beside its tensors
   Tensor entry = at::empty({}, at::TensorOptions().dtype(at::kLong));
   *entry.mutable_data_ptr<int64_t>() = entry_of(plan, has_docs ? s.docs.capacity : -1, has_docs && s.docs.aligned);
@@ -670,10 +682,11 @@ struct AttnNode : public torch::autograd::Function<AttnNode<FP4>> {
     saved.push_back(lse);
     saved.insert(saved.end(), state.begin(), state.end() - 1);     // (the entry handle is kept as a number)
     ctx->save_for_backward(std::move(saved));
-    // the capacity of the aligned buffer is in the shapes: repacked documents keep its LSE (1, h, capacity) first
-    const bool has_docs = p.varlen || p.ragged, repacked = has_docs && !p.aligned;
+    // the capacity of the aligned buffer is in the shapes: repacked documents keep its LSE (1, h, capacity) first (as do batch rows that
+    // are no whole tiles)
+    const bool has_docs = p.varlen, repacked = has_docs && !p.aligned;
     ctx->saved_data["entry"] = entry_of(c.plan, !has_docs ? -1 : repacked ? state[0].sym_size(2).guard_int(__FILE__, __LINE__) : p.tot_q, has_docs && p.aligned);
-    ctx->saved_data["repacked"] = repacked;
+    ctx->saved_data["own_lse"] = repacked || p.ragged;
     ctx->set_materialize_grads(false);
     *c.lse = std::move(lse);
     *c.state = std::move(state);
@@ -682,7 +695,7 @@ struct AttnNode : public torch::autograd::Function<AttnNode<FP4>> {
   static variable_list backward(torch::autograd::AutogradContext* ctx, variable_list grads) {
     if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor(), Tensor()};
     variable_list state = ctx->get_saved_variables();
-    if (ctx->saved_data["repacked"].toBool()) state.erase(state.begin() + 1);      // the kernels' own LSE follows the caller's
+    if (ctx->saved_data["own_lse"].toBool()) state.erase(state.begin() + 1);      // the kernels' own LSE follows the caller's
     auto [dq, dk, dv] = bwd_op<FP4>().call(grads[0].contiguous(), state, ctx->saved_data["entry"].toInt());
     return {dq, dk, dv, Tensor()};
   }
@@ -738,7 +751,7 @@ struct DirectNode : public torch::autograd::Function<DirectNode> {
     s.status = t[3]; s.k_rows = t[4]; s.v_rows = t[5]; s.seqused = t[6];
     Docs& d = s.docs;
     d.start = t[7]; d.len = t[8]; d.row_map = t[9]; d.slot_src = t[10]; d.slot_rows = t[11]; d.all = t[12]; d.work = t[13];
-    const bool has_docs = p.varlen || p.ragged;
+    const bool has_docs = p.varlen;
     d.aligned = has_docs && p.aligned;
     d.capacity = !has_docs ? -1 : d.aligned ? p.tot_q : t[1].sym_size(2).guard_int(__FILE__, __LINE__);   // (repacked documents: the kernels' LSE, (1, h, capacity))
     if (d.all.defined()) d.split((d.all.sym_numel().guard_int(__FILE__, __LINE__) - d.capacity - d.capacity / 128 * 2) / 2);

@@ -899,6 +899,9 @@ static int prologue_steps(long long n_tiles, bool want_t) {
 
 static int quant_cols(const fl_quant_args* a) { return (a->flags >> 16) > 0 ? (a->flags >> 16) : a->d; }
 
+// rows of a batch row of x (the outputs have a->s): the tensor maps read the missing ones as zeros
+static int quant_src_rows(const fl_quant_args* a) { return a->src_rows > 0 ? a->src_rows : a->s; }
+
 static int check_quant_args(const fl_quant_args* a) {
   if (!a || !a->x || !a->codes) return FL_ERR_BAD_ARG;
   if (a->b <= 0 || a->s <= 0 || a->h <= 0 || (a->s % 128) != 0) return FL_ERR_BAD_ARG;
@@ -911,6 +914,7 @@ static int check_quant_args(const fl_quant_args* a) {
   if ((long long)a->b * (a->s / 128) * a->h > 0x7FFFFFFF) return FL_ERR_TOO_LARGE;
   if (a->row_stat && (a->row_stat_kind < 1 || a->row_stat_kind > 3)) return FL_ERR_BAD_ARG;
   if (a->slot_src && (!a->slot_rows || a->b != 1 || a->src_rows <= 0)) return FL_ERR_BAD_ARG;
+  if (!a->slot_src && a->src_rows != 0 && (a->src_rows > a->s || a->src_rows <= a->s - 128)) return FL_ERR_BAD_ARG;
   return FL_OK;
 }
 
@@ -940,7 +944,7 @@ static int quant_rows(const fl_quant_args* const* args, int n, cudaStream_t st, 
     o.s = a->s; o.h = a->h; o.first = (int)tiles; o.plain = m == 0;
     tiles += (long long)a->b * (a->s / 128) * a->h;
     int rc;
-    if ((rc = make_rows_map_16(&maps.x[i], a->x, a->b, a->slot_src ? a->src_rows : a->s, a->h, quant_cols(a), 128))) return rc;
+    if ((rc = make_rows_map_16(&maps.x[i], a->x, a->b, quant_src_rows(a), a->h, quant_cols(a), 128))) return rc;
     if ((rc = make_rows_map(&maps.c[i], a->codes, a->b, a->s, a->h, a->d, 128))) return rc;
   }
   if (tiles > 0x7FFFFFFF) return FL_ERR_TOO_LARGE;
@@ -989,9 +993,9 @@ extern "C" int fl_quant_blocks(const fl_quant_args* a, void* stream) {
   int rc;
   const bool wt = a->codes_t != nullptr;
   const int steps = pro ? prologue_steps(n_tiles, wt) : 1, box = QT / steps;          // rows of a step
-  if ((rc = make_rows_map_16(&mx, a->x, a->b, packed ? a->src_rows : a->s, a->h, d_src, box))) return rc;
+  if ((rc = make_rows_map_16(&mx, a->x, a->b, quant_src_rows(a), a->h, d_src, box))) return rc;
   p.o_packed = (packed && (a->flags & FL_Q_O_PACKED)) ? 1 : 0;
-  if ((rc = make_rows_map_16(&mo, pro ? a->o : a->x, a->b, p.o_packed ? a->src_rows : a->s, a->h, d_src, box))) return rc;
+  if ((rc = make_rows_map_16(&mo, pro ? a->o : a->x, a->b, !packed || p.o_packed ? quant_src_rows(a) : a->s, a->h, d_src, box))) return rc;
   if (a->d == 64) {
     if (pro) rc = steps == 2 ? launch_quant<64, 0, true, 2>(mx, mo, p, wt, st) : launch_quant<64, 0, true>(mx, mo, p, wt, st);
     else rc = nv4 ? launch_quant<64, 2, false>(mx, mo, p, wt, st) : launch_quant<64, 0, false>(mx, mo, p, wt, st);

@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(1024) dq_prescale_rows_kernel(const float* __r
 // ------------------------------------------------------------------------------------------------ dQ postprocess
 // dq[b, q, h, :] = cast(f32(acc) * post[b, q / 128] * mult), optionally rotated back: (y H_128 / sqrt(128)) * signs in the
 // quantiser's butterfly order. Replaces the reference's DQPostprocess (flash_attn/cute/dq_postprocess_cute.py:46-124).
-// HBM-bound: 2 B read + 2 B written per element.
+// HBM-bound: 2 B read + 2 B written per element. rows: a batch row's rows of dq (s, or fewer where s is rounded up to whole tiles).
 __device__ __forceinline__ uint32_t cvt_out2(float a, float b, int out_f16) {
   if (out_f16) { __half2 hh = __floats2half2_rn(a, b); return *reinterpret_cast<uint32_t*>(&hh); }
   return pack_bf16x2(a, b);
@@ -107,7 +107,7 @@ __device__ __forceinline__ uint32_t cvt_out2(float a, float b, int out_f16) {
 
 // head dim 64: the accumulator is (b, h, s, 64); a straight scaled copy into the (b, s, h, 64) gradient
 __global__ void __launch_bounds__(128) dq_post_rows64_kernel(const __half* __restrict__ acc, const float* __restrict__ post,
-                                                             uint16_t* __restrict__ dq, int s, int h, int d_out, float mult,
+                                                             uint16_t* __restrict__ dq, int s, int rows, int h, int d_out, float mult,
                                                              int out_f16, int per_row, const float* __restrict__ head_mult,
                                                              const int32_t* __restrict__ slot_src,
                                                              const int32_t* __restrict__ slot_rows) {
@@ -118,8 +118,8 @@ __global__ void __launch_bounds__(128) dq_post_rows64_kernel(const __half* __res
   const __half* src = acc + (((size_t)bat * h + head) * s + t0) * D;
   const float sc_tile = per_row ? 0.f : post[(size_t)bat * (s / 128) + tile] * mult;
   // packed output: the tile's rows go to the packed rows slot_src[tile] .. + slot_rows[tile] of dq
-  const int n_rows = slot_src ? (slot_src[tile] >= 0 ? min(slot_rows[tile], 128) : 0) : 128;
-  uint16_t* dst = dq + (((size_t)bat * s + (slot_src ? (n_rows ? slot_src[tile] : 0) : t0)) * h + head) * d_out;
+  const int n_rows = slot_src ? (slot_src[tile] >= 0 ? min(slot_rows[tile], 128) : 0) : min(rows - t0, 128);
+  uint16_t* dst = dq + (((size_t)bat * rows + (slot_src ? (n_rows ? slot_src[tile] : 0) : t0)) * h + head) * d_out;
   const size_t row_stride = (size_t)h * d_out;
   for (int i = tid; i < 128 * CPR; i += 128) {
     const int r = i / CPR, c = i % CPR;
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(128) dq_post_rows64_kernel(const __half* __res
 // as coalesced 16-byte stores.
 __global__ void __launch_bounds__(128) dq_post_t128_kernel(const __grid_constant__ CUtensorMap tm_acc,
                                                            const float* __restrict__ post, uint16_t* __restrict__ dq,
-                                                           int s, int h, int d_out, float mult, int unrotate, int out_f16,
+                                                           int s, int rows, int h, int d_out, float mult, int unrotate, int out_f16,
                                                            int per_row, const float* __restrict__ head_mult,
                                                            const int32_t* __restrict__ slot_src,
                                                            const int32_t* __restrict__ slot_rows) {
@@ -223,8 +223,8 @@ __global__ void __launch_bounds__(128) dq_post_t128_kernel(const __grid_constant
     }
     __syncthreads();
     // packed output: the tile's rows go to the packed rows slot_src[tile] .. + slot_rows[tile] of dq
-    const int n_rows = slot_src ? (slot_src[tile] >= 0 ? min(slot_rows[tile], 128) : 0) : 128;
-    uint16_t* dst = dq + (((size_t)bat * s + (slot_src ? (n_rows ? slot_src[tile] : 0) : t0)) * h + head) * d_out;
+    const int n_rows = slot_src ? (slot_src[tile] >= 0 ? min(slot_rows[tile], 128) : 0) : min(rows - t0, 128);
+    uint16_t* dst = dq + (((size_t)bat * rows + (slot_src ? (n_rows ? slot_src[tile] : 0) : t0)) * h + head) * d_out;
     const size_t row_stride = (size_t)h * d_out;
     for (int i = tid; i < 128 * CPR; i += 128) {
       const int r = i / CPR, c = i % CPR;
@@ -378,13 +378,15 @@ extern "C" int fl_dq_prescale(const float* stats_do, const float* stats_v, const
 // transposed dQ tiles), (b, h, s, d) for head_dim 64.
 static int dq_post_launch(const void* dq_acc, const float* post_scale, float mult, void* dq, int32_t b, int32_t s,
                           int32_t h, int32_t d, int32_t unrotate, int32_t out_f16, int per_row, const float* head_mult,
-                          void* stream, const int32_t* slot_src = nullptr, const int32_t* slot_rows = nullptr, int d_out = 0) {
+                          void* stream, const int32_t* slot_src = nullptr, const int32_t* slot_rows = nullptr, int d_out = 0, int rows = 0) {
   using namespace fl;
   if (!dq_acc || !post_scale || !dq || b <= 0 || s <= 0 || (s % 128) || h <= 0) return FL_ERR_BAD_ARG;
   if ((d != 64 && d != 128) || (unrotate && d != 128)) return FL_ERR_UNSUPPORTED;
   if (h > 65535 || b > 65535) return FL_ERR_TOO_LARGE;
   if (d_out == 0) d_out = d;
   if (d_out < 0 || d_out > d || d_out % 8) return FL_ERR_BAD_ARG;
+  if (rows == 0) rows = s;
+  if (rows < 0 || rows > s || rows <= s - 128) return FL_ERR_BAD_ARG;
   dim3 grid(s / 128, h, b);
   cudaStream_t st = (cudaStream_t)stream;
   if (d == 128) {
@@ -393,10 +395,10 @@ static int dq_post_launch(const void* dq_acc, const float* post_scale, float mul
     if (rc) return rc;
     const int sm = 32768 + 128 * 272 + 1024;
     if (int e = set_smem(dq_post_t128_kernel, sm, "fl_dq_post: cudaFuncSetAttribute")) return e;
-    launch_after(dq_post_t128_kernel, grid, 128, sm, st, macc, post_scale, (uint16_t*)dq, s, h, d_out, mult, unrotate, out_f16, per_row,
+    launch_after(dq_post_t128_kernel, grid, 128, sm, st, macc, post_scale, (uint16_t*)dq, s, rows, h, d_out, mult, unrotate, out_f16, per_row,
                                                head_mult, slot_src, slot_rows);
   } else {
-    launch_after(dq_post_rows64_kernel, grid, 128, 0, st, (const __half*)dq_acc, post_scale, (uint16_t*)dq, s, h, d_out, mult, out_f16,
+    launch_after(dq_post_rows64_kernel, grid, 128, 0, st, (const __half*)dq_acc, post_scale, (uint16_t*)dq, s, rows, h, d_out, mult, out_f16,
                                                 per_row, head_mult, slot_src, slot_rows);
   }
   return launch_result("fl_dq_post: kernel launch");
@@ -431,6 +433,11 @@ extern "C" int fl_dq_post_cols(const void* dq_acc, const float* post_scale, int3
   if (slot_src && (!slot_rows || b != 1 || per_row || head_mult)) return fl::FL_ERR_BAD_ARG;
   return dq_post_launch(dq_acc, post_scale, mult, dq, b, s, h, d, unrotate, out_f16, per_row ? 1 : 0, head_mult, stream, slot_src,
                         slot_rows, d_out);
+}
+
+extern "C" int fl_dq_post_trim(const void* dq_acc, const float* post_scale, float mult, void* dq, int32_t b, int32_t s, int32_t rows, int32_t h,
+                               int32_t d, int32_t d_out, int32_t unrotate, int32_t out_f16, void* stream) {
+  return dq_post_launch(dq_acc, post_scale, mult, dq, b, s, h, d, unrotate, out_f16, 0, nullptr, stream, nullptr, nullptr, d_out, rows);
 }
 
 extern "C" int fl_dq_prescale_rows(const float* row_do, float* row_v, float* row_k, int32_t b, int32_t s, float unit,

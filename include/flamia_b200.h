@@ -64,7 +64,8 @@ typedef struct fl_quant_args {
   /* Packed source (documents stored back to back, b = 1): x is (src_rows, h, d) and the outputs are the 128-aligned buffer
    * of s rows; slot_src[i] = first row of x that goes to rows [128 i, 128 i + 128) of the outputs (-1: the slot is
    * empty), slot_rows[i] = how many of them are real (the others quantise as zeros). Replaces the row gather of
-   * flash_attn/cute/lp_docmaps.py (the quantisers read Q / K / V / dO through the row map). NULL = x has the outputs' rows. */
+   * flash_attn/cute/lp_docmaps.py (the quantisers read Q / K / V / dO through the row map). NULL = x has the outputs' rows, or, with
+   * src_rows > 0, that many of each batch row's (s: those rounded up to whole tiles; the missing rows, of o too, read as zeros). */
   const int32_t* slot_src;
   const int32_t* slot_rows;
   int32_t src_rows;
@@ -162,7 +163,9 @@ typedef struct fl_attn_args {
    * of fl_quant_args.slot_src on the way out): out (forward) and dk, dv (backward) are (out_rows, heads, d) with the
    * documents stored back to back; slot_src[i] = the packed row of row 128 i of the aligned buffer the kernels work in
    * (-1: an empty slot), slot_rows[i] = how many rows of that slot are real. A full slot leaves as one TMA store, a
-   * document's last rows as row stores. NULL = the outputs have the aligned buffer's rows. lse keeps those rows. */
+   * document's last rows as row stores. NULL = the outputs have the aligned buffer's rows. lse keeps those rows.
+   * Batched form: out_rows > 0 is the number of queries and keys of a batch row where s_q = s_k is that rounded up to whole tiles:
+   * out, dk and dv are (b, out_rows, heads, d), every intermediate and lse have s_q rows. */
   const int32_t* slot_src;
   const int32_t* slot_rows;
   int32_t out_rows;
@@ -230,6 +233,9 @@ int fl_dq_post_packed(const void* dq_acc, const float* post_scale, float mult, v
 int fl_dq_post_cols(const void* dq_acc, const float* post_scale, int32_t per_row, const float* head_mult, float mult, void* dq,
                     int32_t b, int32_t s, int32_t h, int32_t d, int32_t d_out, int32_t unrotate, int32_t out_f16,
                     const int32_t* slot_src, const int32_t* slot_rows, void* stream);
+/* fl_dq_post_trim: dq has rows <= s rows per batch row (s: those rounded up to whole tiles) of d_out columns. */
+int fl_dq_post_trim(const void* dq_acc, const float* post_scale, float mult, void* dq, int32_t b, int32_t s, int32_t rows, int32_t h, int32_t d,
+                    int32_t d_out, int32_t unrotate, int32_t out_f16, void* stream);
 /* Tile statistics of E4M3 codes times a factor per (batch row, head): tile_stats (b, h, s/128, 2) = the largest
  * magnitude and the largest row sum of squares of codes * descale[b, h] per 128-row tile, the figures the quantiser
  * writes for operands it quantises itself (the reference sizes the f16 dQ pre-scale of pre-quantised inputs from one

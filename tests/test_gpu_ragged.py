@@ -1,0 +1,42 @@
+"""Batch rows that are no whole tiles, as batch rows: against the same rows as packed documents, bit for bit."""
+import warnings
+
+import pytest
+import torch
+
+from inputs import attention_inputs
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("b,s,h,hk,d,dtype,kw", [
+    (1, 1, 1, 1, 128, "bfloat16", dict(causal=True)),
+    (3, 127, 2, 1, 64, "float16", dict(causal=False)),
+    (2, 129, 4, 2, 128, "bfloat16", dict(causal=True)),             # one row in the last tile
+    (2, 257, 2, 2, 96, "bfloat16", dict(causal=True)),              # and in the last block of 256
+    (2, 383, 2, 1, 80, "float16", dict(causal=False)),
+    (2, 640 + 31, 3, 1, 64, "bfloat16", dict(causal=True, window_size=(200, 0))),
+    (2, 500, 2, 2, 128, "bfloat16", dict(causal=False, window_size=(60, 130))),
+    (2, 300, 2, 1, 128, "bfloat16", dict(causal=True, softcap=20.0)),
+    (2, 300, 2, 1, 128, "float16", dict(causal=True, deterministic=True)),
+])
+def test_batch_rows_equal_documents(b, s, h, hk, d, dtype, kw):
+    """dQ to the rounding of its f16 sums, which come in arrival order with a pre-scale per batch row instead of one (the bound of
+    test_gpu_full_size.py for the same)."""
+    import flamia_blackwell_attention_b200 as F
+    x = [t.to(getattr(torch, dtype)).cuda() for t in attention_inputs(b, s, h, hk, d, seed=21)]
+
+    def step(q, k, v, g, **more):
+        q, k, v = (t.detach().clone().requires_grad_(True) for t in (q, k, v))
+        out, lse = F.flash_attn_fp8(q, k, v, return_lse=True, **kw, **more)
+        return (out.detach(), lse, *torch.autograd.grad(out, (q, k, v), g))
+    o, lse, dq, dk, dv = step(*x)
+    cu = torch.arange(0, b * s + 1, s, dtype=torch.int32, device="cuda")
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        po, plse, pdq, pdk, pdv = step(*(t.flatten(0, 1) for t in x), cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=s, max_seqlen_k=s)
+    assert torch.equal(lse, plse.view(h, b, s).transpose(0, 1))
+    for got, want in ((o, po), (dk, pdk), (dv, pdv)):
+        assert torch.equal(got, want.view(got.shape))
+    assert float((dq.float() - pdq.view(dq.shape).float()).norm()) <= 8e-3 * float(pdq.float().norm())
+    assert F.check_status() == 0
