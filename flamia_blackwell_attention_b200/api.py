@@ -12,6 +12,7 @@ from typing import Callable, Optional, Tuple
 
 import torch
 
+from . import _lib as L
 from . import _op
 from . import interface_bwd_fp4 as _switches
 from .options import FP4AttnOptions, FP8AttnOptions
@@ -68,9 +69,12 @@ def _resolved(entry, resolve, names, q, k, v, *values) -> _Resolved:
     """The resolved plan of a call; names / values: its keyword arguments in the resolver's names."""
     try:
         # (entry, mode, the module switches the resolver reads, tensor metadata, argument values)
-        key = (entry, torch.is_grad_enabled(), _switches.DQ_CAUSAL_PRESCALE, _switches.DQ_CAUSAL_GRANULARITY,
-               q.shape, q.dtype, q.requires_grad, k.shape, k.dtype, k.requires_grad, v.shape, v.dtype, v.requires_grad,
-               *[x if not isinstance(x, torch.Tensor) else _facts(x) for x in values])
+        key = None if torch.compiler.is_compiling() else \
+            L.host().call_key(q, k, v, entry, _switches.DQ_CAUSAL_PRESCALE, _switches.DQ_CAUSAL_GRANULARITY, *values)
+        if key is None:
+            key = (entry, torch.is_grad_enabled(), _switches.DQ_CAUSAL_PRESCALE, _switches.DQ_CAUSAL_GRANULARITY,
+                   q.shape, q.dtype, q.requires_grad, k.shape, k.dtype, k.requires_grad, v.shape, v.dtype, v.requires_grad,
+                   *[x if not isinstance(x, torch.Tensor) else _facts(x) for x in values])
         hit = _CALLS.get(key)
     except (AttributeError, TypeError):         # not tensors, or an unhashable argument (e.g. a callable object): uncached
         return _resolve(entry, resolve, q, k, v, dict(zip(names, values)))
@@ -133,6 +137,10 @@ def _run(call, q, k, v, cu_q, cu_k, su_q, su_k, return_lse, doc_maps=None):
     return (out, lse) if return_lse else out
 
 
+def _is_e4m3(t):
+    return isinstance(t, torch.Tensor) and t.dtype is torch.float8_e4m3fn
+
+
 _COMMON_NAMES = ("softmax_scale", "causal", "window_size", "softcap", "score_mod", "score_mod_bwd", "mask_mod", "cu_seqlens_q",
                  "cu_seqlens_k", "max_seqlen_q", "max_seqlen_k", "seqused_k", "seqused_q", "deterministic", "return_lse")
 _FP8_NAMES = _COMMON_NAMES + ("qk_hadamard", "q_quantized", "k_quantized", "q_scale_fused", "options")
@@ -163,7 +171,7 @@ def flash_attn_fp8(q, k, v, *, softmax_scale: Optional[float] = None, causal: bo
     if aux_tensors is not None:
         _fail("B3", NotImplementedError, "aux_tensors belong to score_mod / mask_mod, which this library does not take")
     if q_descale is not None or k_descale is not None or v_descale is not None or grad_proxies is not None or \
-            (isinstance(q, torch.Tensor) and q.dtype == torch.float8_e4m3fn):
+            _is_e4m3(q):
         if doc_maps is not None:
             _fail("B7", NotImplementedError, "pre-quantised E4M3 inputs are served on the batched form, not with doc_maps")
         from .prequant_fa3 import flash_attn_fp8_prequant
@@ -197,7 +205,7 @@ def flash_attn_fp4(q, k, v, *, softmax_scale: Optional[float] = None, causal: bo
         cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k = _doc_maps_args(doc_maps, q, cu_seqlens_q, cu_seqlens_k,
                                                                                 seqused_q, seqused_k)
     if q_descale is not None or k_descale is not None or v_descale is not None or \
-            any(isinstance(t, torch.Tensor) and t.dtype == torch.float8_e4m3fn for t in (q, k, v)):
+            _is_e4m3(q) or _is_e4m3(k) or _is_e4m3(v):
         _fail("B7", TypeError, "flash_attn_fp4 takes bf16 / f16 inputs: pre-quantised E4M3 inputs are a flash_attn_fp8 "
                                "feature of the reference and are not built here")
     if aux_tensors is not None:

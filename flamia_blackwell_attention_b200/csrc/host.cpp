@@ -829,6 +829,41 @@ PyObject* py_run(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyMethodDef kRun = {"run", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_run)), METH_FASTCALL,
                     "run(fp4, plan, q, k, v, docs) -> (out, lse)"};
 
+// call_key(q, k, v, *values) -> tuple: what plan resolution may look at, as a key. Tensors as their sizes, type and requires_grad, everything
+// else as it is; None where q, k, v are not plain tensors of known sizes (the caller makes its key from their attributes). In Python the
+// same key (thirty attributes and type tests) was half of the 5 us that a short call spends before it gets here.
+PyObject* py_call_key(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n >= 3, "call_key(q, k, v, *values)");
+  PyObject* key = PyTuple_New(n + 1);
+  PyTuple_SET_ITEM(key, n, PyBool_FromLong(at::GradMode::is_enabled()));
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyObject* item = nullptr;
+    if (PyType_IsSubtype(Py_TYPE(args[i]), reinterpret_cast<PyTypeObject*>(THPVariableClass))) {      // (an isinstance of Tensor takes its metaclass along)
+      const Tensor& t = THPVariable_Unpack(args[i]);
+      const c10::TensorImpl* impl = t.unsafeGetTensorImpl();
+      if (!THPVariable_CheckExact(args[i]) || impl->has_symbolic_sizes_strides() || impl->is_python_dispatch() || t.dim() > 8) {
+        Py_DECREF(key);
+        Py_RETURN_NONE;
+      }
+      int64_t facts[10] = {(int64_t)t.scalar_type() * 2 + t.requires_grad(), t.dim()};
+      for (int64_t d = 0; d < t.dim(); ++d) facts[2 + d] = t.size(d);
+      item = PyBytes_FromStringAndSize(reinterpret_cast<const char*>(facts), (2 + t.dim()) * sizeof(int64_t));
+    } else if (i < 3) {
+      Py_DECREF(key);
+      Py_RETURN_NONE;
+    } else {
+      item = args[i];
+      Py_INCREF(item);
+    }
+    PyTuple_SET_ITEM(key, i, item);
+  }
+  return key;
+  END_HANDLE_TH_ERRORS
+}
+PyMethodDef kCallKey = {"call_key", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_call_key)), METH_FASTCALL,
+                        "call_key(q, k, v, *values) -> tuple or None"};
+
 int64_t register_plan(const pybind11::dict& d) {
   Plan p;
   auto b = [&](const char* n) { return d[n].cast<bool>(); };
@@ -877,5 +912,6 @@ PYBIND11_MODULE(_host, m) {
   m.def("status_word", wrap_pybind_function_no_gil(device_status_word));
   m.def("note_status", wrap_pybind_function_no_gil(note_status));
   m.def("check_status", wrap_pybind_function_no_gil(check_status));
+  m.attr("call_key") = pybind11::reinterpret_steal<pybind11::object>(PyCFunction_NewEx(&kCallKey, nullptr, nullptr));
   m.attr("run") = pybind11::reinterpret_steal<pybind11::object>(PyCFunction_NewEx(&kRun, nullptr, nullptr));
 }
