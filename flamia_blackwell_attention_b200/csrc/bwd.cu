@@ -734,40 +734,55 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       for (int it = 0; it < n_it; ++it) {
         const int g = gi + it, st = g & 1;
         const int q_first = m * 128 + 64 * x + 32 * qb;                    // document-relative query of column 0
-        const bool full = key_valid && (q_first >= vis_from) && (q_first + QW - 1 <= vis_to);
+        bool full = false;
         // which of the queries see this key, a bit each (tested bit by bit the mask takes a third of the instructions that
         // comparisons take, and they stand in the loop whether they run or not)
         uint32_t see[2] = {0u, 0u};
-        if (!full) {
-          const int lo = max(vis_from - q_first, 0), n = key_valid ? max(min(vis_to - q_first + 1, QW) - lo, 0) : 0;
-          const uint64_t b = lo < QW && n > 0 ? (~0ull >> (64 - n)) << lo : 0ull;
-          see[0] = (uint32_t)b;
-          see[1] = (uint32_t)(b >> 32);
-        }
-        if (++m == T.m_lo + T.n_m) m = T.m_lo;                              // (the next iteration's from here on)
+        auto masks = [&]() {
+          full = key_valid && (q_first >= vis_from) && (q_first + QW - 1 <= vis_to);
+          if (!full) {
+            const int lo = max(vis_from - q_first, 0), n = key_valid ? max(min(vis_to - q_first + 1, QW) - lo, 0) : 0;
+            const uint64_t b = lo < QW && n > 0 ? (~0ull >> (64 - n)) << lo : 0ull;
+            see[0] = (uint32_t)b;
+            see[1] = (uint32_t)(b >> 32);
+          }
+          if (++m == T.m_lo + T.n_m) m = T.m_lo;                              // (the next iteration's from here on)
+        };
         auto visible = [&](int j) { return (see[j >> 5] & (1u << (j & 31))) != 0; };
-        if (!(ok = mbar_wait(&bars[BB_BFULL + 2 * st + x], (g >> 1) & 1, p.ctl, abortp, 30))) break;   // row vectors and scalars visible
         const uint32_t v_lse = smem_u32(smem) + SM::VEC + (2 * st + x) * SM::VEC_HALF + 128 * qb, v_dpp = v_lse + 256;
         [[maybe_unused]] const uint32_t v_fq = v_lse + 512, v_fdo = v_lse + 768;      // token-local: the per-query factors
-        const float4 sc4 = lds128(smem_u32(misc.scal[st][x]));
-        const float sc[5] = {sc4.x, sc4.y, sc4.z, sc4.w, misc.scal[st][x][4]};
-        const uint32_t edo2 = ((__float_as_uint(sc[2]) >> 23) & 0xFF) | (((__float_as_uint(sc[3]) >> 23) & 0xFF) << 8);
-        const uint32_t eq2 = ((__float_as_uint(sc[0]) >> 23) & 0xFF) | (((__float_as_uint(sc[1]) >> 23) & 0xFF) << 8);
-        const uint32_t lb = (uint32_t)((int)((__float_as_uint(sc[4]) >> 23) & 0xFF) - 127) & 0xFF;
-        const uint32_t ekb_word = __vadd4(ek_word, lb * 0x01010101u);
-        uint32_t lq[NQ];                           // a pre-scale per query row: folded into the dQ side's B scale bytes
-#pragma unroll
-        for (int qh = 0; qh < NQ; ++qh) {
-          lq[qh] = 0;
-          if (FULL && p.dq_scale_rows)
-            lq[qh] = (uint32_t)((int)((__float_as_uint(p.dq_scale_rows[(size_t)T.bat * p.s_q + T.q0 + q_first + 32 * qh + lane]) >> 23) & 0xFF) - 127);
-        }
-        // FP4: the block scales of S were applied by the tensor core; only the softmax scale remains
+        uint32_t edo2 = 0, eq2 = 0, ekb_word = 0, lq[NQ];
         float c[NQ], b8[NQ];
+        auto row_vectors = [&]() -> bool {         // they are there, and so are the half's scalars
+          if (!mbar_wait(&bars[BB_BFULL + 2 * st + x], (g >> 1) & 1, p.ctl, abortp, 30)) return false;
+          const float4 sc4 = lds128(smem_u32(misc.scal[st][x]));
+          const float sc[5] = {sc4.x, sc4.y, sc4.z, sc4.w, misc.scal[st][x][4]};
+          edo2 = ((__float_as_uint(sc[2]) >> 23) & 0xFF) | (((__float_as_uint(sc[3]) >> 23) & 0xFF) << 8);
+          eq2 = ((__float_as_uint(sc[0]) >> 23) & 0xFF) | (((__float_as_uint(sc[1]) >> 23) & 0xFF) << 8);
+          const uint32_t lb = (uint32_t)((int)((__float_as_uint(sc[4]) >> 23) & 0xFF) - 127) & 0xFF;
+          ekb_word = __vadd4(ek_word, lb * 0x01010101u);
 #pragma unroll
-        for (int qh = 0; qh < NQ; ++qh) {
-          c[qh] = FP4 ? p.scale_log2 : fk * (qb ? sc[1] : sc[qh]);
-          b8[qh] = fv8 * (qb ? sc[3] : sc[2 + qh]);
+          for (int qh = 0; qh < NQ; ++qh) {        // a pre-scale per query row: folded into the dQ side's B scale bytes
+            lq[qh] = 0;
+            if (FULL && p.dq_scale_rows)
+              lq[qh] = (uint32_t)((int)((__float_as_uint(p.dq_scale_rows[(size_t)T.bat * p.s_q + T.q0 + q_first + 32 * qh + lane]) >> 23) & 0xFF) - 127);
+          }
+          // FP4: the block scales of S were applied by the tensor core; only the softmax scale remains
+#pragma unroll
+          for (int qh = 0; qh < NQ; ++qh) {
+            c[qh] = FP4 ? p.scale_log2 : fk * (qb ? sc[1] : sc[qh]);
+            b8[qh] = fv8 * (qb ? sc[3] : sc[2 + qh]);
+          }
+          return true;
+        };
+        // Where the scores are waited for anyway, what they are not needed for stands behind their load from tensor memory, which takes its
+        // time: of an iteration of 3250 clocks the masks took 250 and the row vectors 130 (b4 s4096 h16: 554 -> 544 us, masks alone
+        // 548). Not where registers are short or the order of waits matters more: mixed route masks alone (both: +0.3 %), d = 64 +1 %, token-local
+        // +5 %.
+        constexpr bool LATE_MASK = D == 128 && VAR == 0 && !SC, LATE_VEC = LATE_MASK && !FP4;
+        if constexpr (!LATE_MASK) masks();
+        if constexpr (!LATE_VEC) {
+          if (!(ok = row_vectors())) break;
         }
 
         // ---- P' = 2^(s c - lse2)
@@ -776,6 +791,10 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         uint32_t pv[QW];
         FL_TMEM_LD_32(t_sx, pv);
         if constexpr (NQ == 2) FL_TMEM_LD_32(t_sx + 32, (pv + 32));
+        if constexpr (LATE_MASK) masks();
+        if constexpr (LATE_VEC) {
+          if (!(ok = row_vectors())) break;
+        }
         tc_wait_ld();
         // the scores are in registers: this region may take the other half's P-hat and dS-hat (half 0's iteration waits for S1 of
         // the same iteration; half 1's for S0 of the next one, which is issued before, or of this one where that was the last)
