@@ -609,13 +609,14 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         float gm[4];                                             // the four 32-key groups' maxima (scaled)
 #pragma unroll
         for (int kbk = 0; kbk < 4; ++kbk) {
-          // eight independent chains of three-input maxima, then a tree: a serial chain would cost its latency 31 times
-          float a[8];
+          // a tree of three-input maxima (sixteen instructions, four deep; b4 s4096 h16, against twenty of mixed ones: dense 383 -> 378
+          // us, causal mixed route 227 -> 221)
+          const float* z = s + 32 * kbk;
+          float a[10];
 #pragma unroll
-          for (int t = 0; t < 8; ++t)
-            a[t] = fmaxf(fmax3(s[32 * kbk + 4 * t], s[32 * kbk + 4 * t + 1], s[32 * kbk + 4 * t + 2]), s[32 * kbk + 4 * t + 3]);
-          const float m8 = fmax3(fmax3(a[0], a[1], a[2]), fmax3(a[3], a[4], a[5]), fmaxf(a[6], a[7]));
-          gm[kbk] = m8 * c[kbk];
+          for (int t = 0; t < 10; ++t) a[t] = fmax3(z[3 * t], z[3 * t + 1], z[3 * t + 2]);
+          const float m9 = fmax3(fmax3(a[0], a[1], a[2]), fmax3(a[3], a[4], a[5]), fmax3(a[6], a[7], a[8]));
+          gm[kbk] = fmax3(m9, fmax3(a[9], z[30], z[31]), m9) * c[kbk];
           mx = fmaxf(mx, gm[kbk]);
         }
         // lazy refresh of the running maximum
