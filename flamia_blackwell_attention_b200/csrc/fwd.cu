@@ -33,8 +33,11 @@
 //   (setmaxnreg 216 / 216 / 72 of a 168-register launch: a softmax thread keeps 128 scores and 32 packed words live)
 // TMEM (512 columns): S0 [0,128) S1 [128,256) O0 [256,384) O1 [384,512); P-hat overlays columns [0,32) of its S, the
 // P.V scale factors columns [32,40).
-// Output rows leave through the finished item's own Q tile buffer (dead once the stage's last product has completed): 64
-// columns at a time -> shared memory (128 B swizzle) -> TMA store; only then may the producer refill that Q buffer.
+// Output rows leave through the finished item's own Q tile buffer (dead once the stage's last product has completed) and, at d = 128, a
+// second one of the stage's own: 64 columns each -> shared memory (128 B swizzle) -> TMA store. Nobody waits for the stores: the warp
+// whose thread issued them confirms, a key tile into the next item, that they have read their rows, and only then may the
+// producer refill the Q buffer. (An item's end took a softmax warp 5500 clocks, two tiles' worth, with both boxes through the Q
+// buffer one after the other: b4 s4096 h16 causal 216 -> 215 us, mixed route 221 -> 219, 16 x 384 tokens h12/4 23.3 -> 22.2.)
 // FL_MODE_FP4: all 512 columns are taken, so the 16 scale columns of an S product (Q and K atoms, tcgen05.cp from shared
 // memory) are parked in columns [64,80) of the OTHER stage's S region once that stage's softmax warps have read their
 // latest scores into registers (B_SDRAIN), and in O1 for the two products of the very first key tile of the CTA (nothing
@@ -230,7 +233,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   uint8_t* sQ = smem;                                   // [item buffer 2][stage 2] x Q_STRIDE
   uint8_t* sK = sQ + 4 * Q_STRIDE;                      // KV_STAGES tiles
   uint8_t* sV = sK + KV_STAGES * TILE_BYTES;            // KV_STAGES tiles
-  uint8_t* sSF = sV + KV_STAGES * TILE_BYTES;           // FP4: scale atoms, Q [item buffer 2] x 2 KB then K KV_STAGES x 1 KB
+  uint8_t* sO = sV + KV_STAGES * TILE_BYTES;            // d = 128: [stage 2] x Q_STRIDE, the second box of the output rows
+  uint8_t* sSF = sO + (D == 128 ? 2 * Q_STRIDE : 0);    // FP4: scale atoms, Q [item buffer 2] x 2 KB then K KV_STAGES x 1 KB
   constexpr int SF_K = 4096;                            // offset of the K atoms inside sSF
   constexpr int OP_BYTES = FP4 ? TILE_BYTES / 2 : TILE_BYTES;   // bytes of one Q / K operand tile (4-bit codes: half)
   __shared__ __align__(8) uint64_t bars[B_COUNT];
@@ -477,6 +481,15 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     const uint32_t t_o = tmem + 256 + 128 * i + ((uint32_t)((warp & 3) * 32) << 16);
     int cs = 0;                                       // tiles of this stage so far, over all items
     int cd = 0;                                       // items of this stage that ended with a P.V so far
+    // The Q buffer whose stores warp 0 of the stage has yet to see read. (The second box's buffer is free with it: its next rows are written
+    // behind the barrier of the next item's first box, where that warp arrives after this.)
+    int pend = -1;
+    auto confirm = [&]() {
+      if (pend < 0) return;
+      if (r == 0) tma_store_wait_read<0>();
+      mbar_arrive_warp(&bars[B_QE + pend]);
+      pend = -1;
+    };
     int epi = 0, gfn = 0;                             // uses of the epilogue barrier / group-frame scale atoms so far
     bool ok = true;
     for (int k = 0; ok; ++k) {
@@ -723,8 +736,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         tc_wait_st();
         tc_fence_before();
         mbar_arrive_warp(&bars[B_PFULL + i]);
+        confirm();
       }
       if (!ok) break;
+      confirm();                         // (an item without tiles)
       // ---- item epilogue: O / l -> bf16 rows through this stage's Q tile buffer, LSE
       if (n_i > 0) {
         if (!(ok = mbar_wait(&bars[B_PVDONE + i], cd & 1, p.ctl, abortp, 34 + i))) break;
@@ -758,8 +773,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       const bool row_valid = (128 * i + r) < T.nq;
       const bool stage_present = T.nq > 128 * i;        // (warpgroup-uniform) an absent stage's rows belong to someone else
       const float inv_l = ((l_sum > 0.f) ? 1.0f / l_sum : 0.f) * ((FULL && p.o_mult) ? p.o_mult[T.bat * p.h_kv + T.hkv] : 1.0f);
-      uint8_t* stage = sQ + (2 * kb + i) * Q_STRIDE;
-      const uint32_t srow = smem_u32(stage) + r * 128;
+      auto stage_of = [&](int cc) { return cc < 2 ? sQ + (2 * kb + i) * Q_STRIDE : sO + i * Q_STRIDE; };
       // packed output: this stage's 128 rows are slot (T.q0 + 128 i) / 128 of the aligned buffer; they go to the packed
       // rows out_row .. + out_n of the caller's tensor: a full slot as TMA stores, a document's last rows row by row
       int out_row = T.q0 + 128 * i, out_n = stage_present ? 128 : 0;
@@ -802,7 +816,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
               *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) +
                                         ((size_t)(out_row + r) * p.h + head) * p.d_out + 8 * ch) = make_uint4(w[0], w[1], w[2], w[3]);
           } else {
-            fwd_sts128(srow + (((ch & 7) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
+            fwd_sts128(smem_u32(stage_of(cc)) + r * 128 + (((ch & 7) ^ (r & 7)) << 4), w[0], w[1], w[2], w[3]);
           }
         }
         if (by_rows || !(cc & 1)) continue;
@@ -811,14 +825,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         if (!(ok = mbar_wait(&bars[B_EPI + i], epi & 1, p.ctl, abortp, 38))) break;
         ++epi;
         if (r == 0 && out_n == 128) {
-          tma_store_4d(&tm_o, stage, 32 * (cc - 1), head, out_row, T.bat);
+          tma_store_4d(&tm_o, stage_of(cc), 32 * (cc - 1), head, out_row, T.bat);
           tma_store_commit();
-          tma_store_wait_read<0>();      // the shared-memory source must outlive the copy; the writes complete with the grid
-        }
-        if (cc + 1 < D / 32) {
-          mbar_arrive_warp(&bars[B_EPI + i]);           // the buffer has been read: the next box may take it
-          if (!(ok = mbar_wait(&bars[B_EPI + i], epi & 1, p.ctl, abortp, 38))) break;
-          ++epi;
         }
       }
       if (!ok) break;
@@ -828,8 +836,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         p.lse[((size_t)T.bat * p.h + head) * p.s_q + qrow] = v;
       }
       tc_fence_before();                 // this stage's output has left tensor memory before the next item's P-hat is announced
-      mbar_arrive_warp(&bars[B_QE + kb]);  // (the thread that stored the rows has seen them read)
+      if (warp & 3) mbar_arrive_warp(&bars[B_QE + kb]);
+      else pend = kb;
     }
+    if (r == 0) tma_store_wait_read<0>();   // (shared memory must outlive the copies; the writes complete with the grid)
   }
   // ---- common exit: nothing of this CTA may still be in flight when tensor memory is released
   if (abort_s) {
@@ -975,7 +985,7 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, con
     if (split->at[split->parts] != (uint32_t)p.n_items << FL_SPLIT_TILE_BITS) return FL_ERR_BAD_ARG;
   }
   const int grid = split ? split->parts : (int)(n_items < sm_count() ? n_items : sm_count());     // one persistent CTA per SM
-  const int smem = 4 * Q_STRIDE + 2 * KV_STAGES * 128 * a->d + 1024 + (fp4 ? 4096 + KV_STAGES * 1024 : 0);
+  const int smem = (a->d == 128 ? 6 : 4) * Q_STRIDE + 2 * KV_STAGES * 128 * a->d + 1024 + (fp4 ? 4096 + KV_STAGES * 1024 : 0);
   cudaStream_t st = (cudaStream_t)stream;
   auto launch = [&](auto kern, auto cuts) -> int {
     if (int e = set_smem(kern, smem, "fl_fwd: cudaFuncSetAttribute")) return e;
