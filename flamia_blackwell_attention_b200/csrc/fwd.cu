@@ -622,8 +622,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         float gm[4];                                             // the four 32-key groups' maxima (scaled)
 #pragma unroll
         for (int kbk = 0; kbk < 4; ++kbk) {
-          // a tree of three-input maxima (sixteen instructions, four deep; b4 s4096 h16, against twenty of mixed ones: dense 383 -> 378
-          // us, causal mixed route 227 -> 221)
+          // a tree of three-input maxima (sixteen instructions, four deep; b4 s4096 h16, against twenty of mixed ones: dense 391 -> 386
+          // us, causal mixed route 227 -> 220)
           const float* z = s + 32 * kbk;
           float a[10];
 #pragma unroll
@@ -681,7 +681,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           }
           float p0 = ex2(a0), p1 = ex2(a1);
           float p2, p3;
-          if (w & 1) {    // one pair in four on the FMA pipe (none: +4 % kernel time causal, +8 % dense; three in eight: the same)
+          // Three pairs in eight on the FMA pipe; one in four with token factors, which load it themselves (three: +5 %). b4 s4096 h16
+          // against one in four by a degree-3 polynomial (25 times the error): dense 378 -> 365 us, causal 215 -> 214, mixed route 219 -> 215;
+          // none: +8 % dense, half: +8 %.
+          if (TL ? (w & 1) != 0 : (w & 3) != 0) {
             ex2_poly2(a2, a3, p2, p3);
           } else {
             p2 = ex2(a2);
