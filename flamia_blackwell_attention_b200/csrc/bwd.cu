@@ -221,6 +221,9 @@ struct BwdMisc {
   // from global memory by the producer: a load that misses in a compute warp stalls it at its next scoreboard wait (every
   // second iteration, by 700 clocks), whatever the distance to the value's use.
   alignas(16) float scal[2][2][8];
+  // block factors of the item's four key blocks, K's then V's [slot]: read ahead by the producer for the same reason (from global memory they
+  // stood 700 clocks in front of an item's first scores)
+  alignas(16) float kfac[2][8];
 };
 template <int D, bool FP4, bool TL>
 struct BwdSmem {
@@ -353,6 +356,14 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         BTile t;
         bwd_decode<FULL>(p, L, t);
         tile_s[kb] = t;
+        if (!TL) {
+          const size_t at = ((size_t)t.bat * p.h_kv + t.hkv) * (p.s_k / 32) + t.k0 / 32;
+          float f[8];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) { f[i] = __ldg(p.fac_k + at + i); f[4 + i] = __ldg(p.fac_v + at + i); }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) misc.kfac[kb][i] = f[i];
+        }
         if (t.nk > 0) {
           mbar_arrive_expect_tx(&bars[BB_KV + kb], 2 * TILE_BYTES + (FP4 ? 8192 + 1024 : 0));
           tma_load_4d(smem + SM::K + kb * TILE_BYTES, &tm_k, &bars[BB_KV + kb], 0, t.hkv, t.k0, t.bat);
@@ -716,16 +727,16 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
       const int n_it = T.n_m * grp;
       const bool key_valid = r < T.nv;
       const size_t bh_k = (size_t)T.bat * p.h_kv + hkv;
-      const int kblk = (T.k0 + r) / 32;
+      const float4 kf = lds128(smem_u32(misc.kfac[kb]));
       // token-local: this key's own factors; otherwise its 32-key block's
-      const float fk_true = TL ? p.fac_k[bh_k * p.s_k + T.k0 + r] : p.fac_k[bh_k * (p.s_k / 32) + kblk];
+      const float fk_true = TL ? p.fac_k[bh_k * p.s_k + T.k0 + r] : misc.kfac[kb][wq];
       const float fk = fk_true * p.scale_log2;
-      const float fv8 = (TL ? p.fac_v[bh_k * p.s_k + T.k0 + r] : p.fac_v[bh_k * (p.s_k / 32) + kblk]) * 0.00390625f;   // f_V 2^-8
+      const float fv8 = (TL ? p.fac_v[bh_k * p.s_k + T.k0 + r] : misc.kfac[kb][4 + wq]) * 0.00390625f;   // f_V 2^-8
       uint32_t ek_word = TL ? 0x7F7F7F7Fu : 0u;        // UE8M0 bytes of the tile's four key blocks (unit when token-local)
       if (!TL) {
+        const float k4[4] = {kf.x, kf.y, kf.z, kf.w};
 #pragma unroll
-        for (int kbk = 0; kbk < 4; ++kbk)
-          ek_word |= ((__float_as_uint(p.fac_k[bh_k * (p.s_k / 32) + T.k0 / 32 + kbk]) >> 23) & 0xFF) << (8 * kbk);
+        for (int kbk = 0; kbk < 4; ++kbk) ek_word |= ((__float_as_uint(k4[kbk]) >> 23) & 0xFF) << (8 * kbk);
       }
       const int krel = T.krel + r - T.off;
       const int vis_from = p.win_r >= 0 ? krel - p.win_r : 0;    // queries in [vis_from, vis_to] see this key
