@@ -137,7 +137,8 @@ int make_acc_t_map_16(CUtensorMap* m, const void* base, int b, int heads, int d,
 // A grid of one CTA an SM that takes whole items is as long as its fullest CTA: with fewer items than SMs, or a few rounds of them,
 // much of the chip waits (one round of causal items is twice as long as their mean). The split schedule deals out equal shares of
 // the items' tiles instead, in the items' order: a CTA's share is whole items and a piece of one at either end. Every share W from the
-// smallest that the CTAs can hold upwards is tried, and the best is taken if it beats the whole items by 3 % and a half tile.
+// smallest that the CTAs can hold upwards is tried, and the best is taken if it beats the whole items by 3 % and a half tile. (A tile
+// of a split kernel takes some 5 % longer.)
 int plan_split(const int* n, int runs, long long reps, bool by_kind, int ctas, float overhead, float lead, float merge, float merge_part,
                fl_split* out) {
   out->parts = 0;
@@ -181,10 +182,10 @@ int plan_split(const int* n, int runs, long long reps, bool by_kind, int ctas, f
     return true;
   };
   double best = whole * 0.97 - 0.6;
-  for (double W = std::max(total / ctas, (double)overhead + lead + 2 * MIN_PIECE); W + merge < best; W *= 1.04) {
+  for (double W = std::max(total / ctas, (double)overhead + lead + 2 * MIN_PIECE); W * 1.05 + merge < best; W *= 1.04) {
     int pieces;
     if (!deal(W, pieces) || !pieces) continue;
-    const double cost = W + merge + merge_part * pieces;
+    const double cost = W * 1.05 + merge + merge_part * pieces;
     if (cost < best) { best = cost; *out = cand; }
   }
   return FL_OK;

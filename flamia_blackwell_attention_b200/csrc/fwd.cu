@@ -683,8 +683,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           float p2, p3;
           // Three pairs in eight on the FMA pipe; one in four with token factors, which load it themselves (three: +5 %). b4 s4096 h16
           // against one in four by a degree-3 polynomial (25 times the error): dense 378 -> 365 us, causal 215 -> 214, mixed route 219 -> 215;
-          // none: +8 % dense, half: +8 %.
-          if (TL ? (w & 1) != 0 : (w & 3) != 0) {
+          // none: +8 % dense, half: +8 %. Split schedules: one in four, too (4608 x 18432 h4 119 -> 112).
+          if (TL || SPLIT ? (w & 1) != 0 : (w & 3) != 0) {
             ex2_poly2(a2, a3, p2, p3);
           } else {
             p2 = ex2(a2);
@@ -739,10 +739,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         tc_wait_st();
         tc_fence_before();
         mbar_arrive_warp(&bars[B_PFULL + i]);
-        confirm();
+        if (!SPLIT) confirm();           // (in the loop it costs the split kernel 2 %, whose CTAs have few items)
       }
       if (!ok) break;
-      confirm();                         // (an item without tiles)
+      confirm();                         // (an item without tiles; split schedules)
       // ---- item epilogue: O / l -> bf16 rows through this stage's Q tile buffer, LSE
       if (n_i > 0) {
         if (!(ok = mbar_wait(&bars[B_PVDONE + i], cd & 1, p.ctl, abortp, 34 + i))) break;
@@ -1067,8 +1067,8 @@ extern "C" int fl_fwd_split_plan(const fl_attn_args* a, int32_t ctas, fl_split* 
   };
   std::vector<int> n(n_blk);
   for (int i = 0; i < n_blk; ++i) n[i] = tiles(causal ? n_blk - 1 - i : i);
-  // What an item costs beside its tiles, and the merge, in key tiles of 256 query rows (1.5 us). One B200, whole items / pieces and merge, us:
-  // 512 x 8192 b4 h32/8 199 / 195; 2688 x 43008 h10 503 / 414; 4608 x 18432 h4 218 / 114; 3072 x 6144 h5 76 / 41; 768 x 3072 h4 40 / 20;
-  // 1792 h5 26.9 / 18.9; 8832 h2 mixed route 120 / 46; 6784 h2 d64 80 / 32. 2048 h16 29.5 / 29.9, with a merge of 2.8 tiles still cut.
+  // What an item costs beside its tiles, and the merge, in key tiles of 256 query rows (1.45 us). One B200, whole items / pieces and merge, us:
+  // 4608 x 18432 h4 210 / 112; 3072 x 6144 h5 75 / 41; 768 x 3072 h4 41 / 21; 8832 h2 mixed route 112 / 48; 1792 h5 26 / 19; 6784 h2 d64
+  // 76 / 31; and 512 x 8192 b4 h32/8 194 / 193, 2048 h16 29 / 30, which are not worth it.
   return plan_split(n.data(), n_blk, a->h * (long long)a->b, causal, ctas ? ctas : sm_count(), 1.2f, 0.4f, 3.2f, 0.01f, split);
 }

@@ -65,8 +65,9 @@ FWD = [
 @pytest.mark.parametrize("b,sq,sk,h,hk,d,causal,form", FWD)
 def test_forward_in_pieces(b, sq, sk, h, hk, d, causal, form, share):
     """Every piece frames a row's P-hat as the whole item does (N(0, 1) operands: the first tile's maximum is refreshed by no later one), so
-    the rounded terms are the same and O differs by f32 sums in another order and the last bit of bfloat16 (2^-9), the LSE by a few
-    units of 2^-20 of logarithms up to about 10."""
+    the rounded terms are the same but for one exponential in eight, which the two kernels take by the unit and by the polynomial (3e-6 apart: of
+    1e5 codes five fall on another value, a sixteenth away, 5e-4 of O's norm). O differs by that, f32 sums in another order and the last bit
+    of bfloat16 (2^-9): below 2^-8; the LSE by a few units of 2^-20 of logarithms up to about 10."""
     from flamia_blackwell_attention_b200 import _lib as L, kernels as K
     q, k, v, _ = attention_inputs(b, max(sq, sk), h, hk, d, seed=11)
     q, k, v = q[:, :sq], k[:, :sk], v[:, :sk]
@@ -88,7 +89,7 @@ def test_forward_in_pieces(b, sq, sk, h, hk, d, causal, form, share):
     vis = torch.isfinite(l1)
     assert torch.equal(vis, torch.isfinite(l2))
     assert float((l1[vis] - l2[vis]).abs().max()) < 1e-4
-    assert A.accuracy(o2.float().cpu(), o1.float().cpu())["rel_l2"] < 2.0 ** -9
+    assert A.accuracy(o2.float().cpu(), o1.float().cpu())["rel_l2"] < 2.0 ** -8
     assert float(o2[~vis.permute(0, 2, 1)].abs().max() if (~vis).any() else 0.0) == 0.0
 
 
