@@ -49,6 +49,7 @@ struct QuantParams {
   const int32_t* slot_src;   // packed source: first source row of each 128-row slot of the output (-1: an empty slot), or null
   const int32_t* slot_rows;  // packed source: valid rows of each slot (the rest of the slot reads as zero)
   int n_tiles;            // b * (s / 128) * h
+  int skip_padding;       // host only: mostly_padding
   int token_local;
   int in_f16;
   float lse_shift, d_multiplier;
@@ -87,8 +88,9 @@ __device__ __forceinline__ float2 e4m3x2_to_f32(uint16_t v) {
 }
 
 // MODE bits: 1 = the E4M3 codes are of the rotated rows, 2 = also write the NVFP4 copy, 4 = rotate only the NVFP4 copy
-// PK: packed source (slot tables); a template flag, so that the batched form pays nothing for it
-template <int D, int MODE, bool PRO, int STEPS, bool PK>
+// PK: packed source (slot tables); a template flag, so that the batched form pays nothing for it. 2: a warp whose rows lie past the slot's
+// document writes zeros and does nothing else (mostly_padding says where).
+template <int D, int MODE, bool PRO, int STEPS, int PK>
 __global__ void __launch_bounds__(q_threads(STEPS), q_blocks(PRO, STEPS))
 quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_o,
                     const QuantParams p) {
@@ -266,6 +268,7 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     const int live_rows = PK ? p.slot_rows[tile] : QT;
     bool ok = mbar_wait(&full[st], (it / QSTAGES) & 1, p.ctl, abortp, 50);
     if (PK) row_live = r < live_rows;
+    const bool work = PK != 2 || step * ROWS + warp * 8 < live_rows;
 
     if (p.zero_acc) {   // this tile's share of the accumulator: 128 * D f16 = 32 D 16-byte chunks, contiguous
       uint4* z = reinterpret_cast<uint4*>(p.zero_acc + (bh * p.s + t0 + step * ROWS) * D);
@@ -318,7 +321,10 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     };
 
     float x[NE];
-    if (ROT4) {          // NVFP4 codes of the rotated row, E4M3 codes of the row as read
+    if (!work) {         // (the prologue alone: no rotation, no NVFP4 copy)
+#pragma unroll
+      for (int i = 0; i < NE; ++i) x[i] = 0.f;
+    } else if (ROT4) {          // NVFP4 codes of the rotated row, E4M3 codes of the row as read
       load_rotated(tile_addr, x);
       nvfp4_row(x);
       load_plain(tile_addr, x);
@@ -333,8 +339,8 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     if (PRO) {
 #pragma unroll
       for (int j = 0; j < NJ; ++j) {
-        o_raw[j] = lds_chunk(tile_addr + TILE_B, j);
-        if (PK && p.o_packed && !row_live) o_raw[j] = make_uint4(0, 0, 0, 0);
+        o_raw[j] = make_uint4(0, 0, 0, 0);
+        if (work && !(PK && p.o_packed && !row_live)) o_raw[j] = lds_chunk(tile_addr + TILE_B, j);
       }
     }
 
@@ -406,7 +412,9 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     }
 
     // ---- prologue: D in the fixed tree order (column bits 1 (fma), 2, 3, 0, 6, 5, 4), shifted log2 LSE
-    if (PRO) {
+    if (PRO && !work) {
+      if (q == 0 && p.d_out) p.d_out[ri] = __fmul_rn(0.f, p.d_multiplier);
+    } else if (PRO) {
       float o[NE];
 #pragma unroll
       for (int j = 0; j < NJ; ++j) to_f32(o_raw[j], o + 8 * j);
@@ -554,6 +562,7 @@ struct QuantRowsParams {
   int n_ops, n_tiles;
   const int32_t* slot_src;   // packed source, see QuantParams
   const int32_t* slot_rows;
+  int skip_padding;          // host only: mostly_padding
   int in_f16;
   DocWork docs;              // packed source: the documents' work lists, made by block 0 while the others quantise (work null: none)
   DevCtl ctl;
@@ -562,9 +571,9 @@ struct QuantRowsMaps {
   CUtensorMap x[3], c[3];
 };
 
-// MODE as in the four-lane kernel: bit 0 = the E4M3 codes are of the rotated row, bit 1 = also the NVFP4 copy, bit 2 =
-// rotate only the NVFP4 copy. PK: packed source.
-template <int MODE, int D, bool PK>
+// MODE and PK as in the four-lane kernel: bit 0 = the E4M3 codes are of the rotated row, bit 1 = also the NVFP4 copy, bit 2 =
+// rotate only the NVFP4 copy.
+template <int MODE, int D, int PK>
 __global__ void __launch_bounds__(128, qr_ctas(D))
 quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_constant__ QuantRowsParams p) {
   static_assert(D == 128 || (D == 64 && MODE == 0), "head_dim 64 has no rotation and no NVFP4 copy");
@@ -630,7 +639,9 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
     const uint32_t tile_addr = smem_u32(smem + st * QR_TILE_B);
     const bool plain = MODE == 0 || op.plain;      // (CTA-uniform)
     const bool stats = op.tile_stats || op.row_stat;
-    const bool live = !PK || r < p.slot_rows[tile];     // packed source: rows past the slot's document read as zero
+    const int live_rows = PK ? p.slot_rows[tile] : QT;
+    const bool live = r < live_rows;                    // packed source: rows past the slot's document read as zero
+    const bool work = PK != 2 || warp * 32 < live_rows;
     bool ok = mbar_wait(&full[st], (it / QR_STAGES) & 1, p.ctl, abortp, 51);
 
     // the previous tile's buffer: filled again once its codes have left it (the store was issued a tile ago)
@@ -739,7 +750,18 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
         for (int a = 0; a < D / 64; ++a) *reinterpret_cast<uint32_t*>(atom + a * 512 + (r & 31) * 16 + (r >> 5) * 4) = sfw[a];
       }
     };
-    if (ROT4 && !plain) {          // NVFP4 codes of the rotated row, E4M3 codes of the row as read
+    if (!work) {
+      if (NV4 && !plain) {
+        const uint4 zero = make_uint4(0, 0, 0, 0);
+        uint4* x4row = reinterpret_cast<uint4*>(op.x4 + (((size_t)bat * s + t0 + r) * h + head) * (D / 2));
+#pragma unroll
+        for (int g2 = 0; g2 < D / 32; ++g2) x4row[g2] = zero;
+        if (op.sf4)
+#pragma unroll
+          for (int a = 0; a < D / 64; ++a)
+            *reinterpret_cast<uint32_t*>(op.sf4 + ((bh * ntile + tile) * (D / 64) + a) * 512 + (r & 31) * 16 + (r >> 5) * 4) = 0u;
+      }
+    } else if (ROT4 && !plain) {          // NVFP4 codes of the rotated row, E4M3 codes of the row as read
       load_row(true);
       rotate_row();
       nvfp4_row();
@@ -752,14 +774,14 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
       load_row(false);
       if (NV4 && !plain) nvfp4_row();
     }
-    if (!ROT || ROT4 || plain) {  // subnormal -> zero of the same sign (rotated rows were flushed by their scaling)
+    if (work && (!ROT || ROT4 || plain)) {  // subnormal -> zero of the same sign (rotated rows were flushed by their scaling)
 #pragma unroll
       for (int i = 0; i < D; i += 2) unpack2(mul2_ftz(pack2(x[i], x[i + 1]), pack2(1.0f, 1.0f)), x[i], x[i + 1]);
     }
 
     // ---- the row's maximum and (with the statistics) its sum of squares, in the four-lane kernel's summation order
     float amax = 0.f, sumsq = 0.f;
-    {
+    if (work) {
       float aq[4] = {0.f, 0.f, 0.f, 0.f};          // per quarter q: elements 32 j + 8 q + e
 #pragma unroll
       for (int q = 0; q < 4; ++q)
@@ -804,9 +826,10 @@ quant_rows_kernel(const __grid_constant__ QuantRowsMaps maps, const __grid_const
       const int swz = D == 128 ? (r & 7) : ((r >> 1) & 3);
 #pragma unroll
       for (int c = 0; c < D / 16; ++c) {            // 16 codes per 16-byte chunk
-        uint32_t cw[4];
+        uint32_t cw[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
+          if (!work) continue;
           float a0, a1, a2, a3;
           unpack2(mul2(pack2(x[16 * c + 4 * k], x[16 * c + 4 * k + 1]), inv2), a0, a1);
           unpack2(mul2(pack2(x[16 * c + 4 * k + 2], x[16 * c + 4 * k + 3]), inv2), a2, a3);
@@ -864,10 +887,11 @@ static int launch_quant_rows(const QuantRowsMaps& maps, const QuantRowsParams& p
     launch_after(kern, grid, 128, smem, st, maps, p);
     return FL_OK;
   };
-  return p.slot_src ? launch(quant_rows_kernel<MODE, D, true>) : launch(quant_rows_kernel<MODE, D, false>);
+  return !p.slot_src ? launch(quant_rows_kernel<MODE, D, 0>)
+         : p.skip_padding && p.n_tiles > grid ? launch(quant_rows_kernel<MODE, D, 2>) : launch(quant_rows_kernel<MODE, D, 1>);
 }
 
-template <int D, int MODE, bool PRO, int STEPS, bool PK>
+template <int D, int MODE, bool PRO, int STEPS, int PK>
 static int launch_quant_pk(const CUtensorMap& mx, const CUtensorMap& mo, const QuantParams& p, bool want_t, cudaStream_t st) {
   const int smem = QSTAGES * (PRO ? 2 : 1) * (QT / STEPS * D * 2) + 1024 + (want_t ? QT * (D + 16) : 0);
   auto kern = quant_blocks_kernel<D, MODE, PRO, STEPS, PK>;
@@ -880,8 +904,9 @@ static int launch_quant_pk(const CUtensorMap& mx, const CUtensorMap& mo, const Q
 
 template <int D, int MODE, bool PRO, int STEPS = 1>
 static int launch_quant(const CUtensorMap& mx, const CUtensorMap& mo, const QuantParams& p, bool want_t, cudaStream_t st) {
-  return p.slot_src ? launch_quant_pk<D, MODE, PRO, STEPS, true>(mx, mo, p, want_t, st)
-                    : launch_quant_pk<D, MODE, PRO, STEPS, false>(mx, mo, p, want_t, st);
+  if (!p.slot_src) return launch_quant_pk<D, MODE, PRO, STEPS, 0>(mx, mo, p, want_t, st);
+  if (PRO && p.skip_padding && p.n_tiles > sm_count() * q_blocks(PRO, STEPS)) return launch_quant_pk<D, MODE, PRO, STEPS, PRO ? 2 : 1>(mx, mo, p, want_t, st);
+  return launch_quant_pk<D, MODE, PRO, STEPS, 1>(mx, mo, p, want_t, st);
 }
 
 // Steps of a prologue tile. Two where both of an SM's blocks have tiles. One where there is no more than a tile an SM, or where in the
@@ -929,6 +954,16 @@ static int quant_mode(const fl_quant_args* a) {
   return ((a->flags & FL_Q_HADAMARD) ? 1 : 0) | (a->x4 ? 2 : 0);
 }
 
+// Packed sources: is more than an eighth of the tiles' rows past the end of a document? Then the kernels in which the warps of such rows
+// leave their work out (PK = 2): 352 documents of 30 to 60 rows, h16/16, d = 128, step 869 -> 815 us; 210 of 100 to 200 454 -> 448; 6000
+// rows in documents of 16 to 1024, h16/4, 182.5 -> 181.2. Not where the documents are long (16k rows in 4, 672 -> 677), and not in
+// a launch of one round, which is over before the shorter way pays for the longer code (75 rows h16/8, mixed route, forward 14.4 -> 14.9).
+static bool mostly_padding(const fl_quant_args* const* args, int n) {
+  long long rows = 0, aligned = 0;
+  for (int i = 0; i < n; ++i) rows += (long long)args[i]->src_rows * args[i]->h, aligned += (long long)args[i]->s * args[i]->h;
+  return args[0]->slot_src && 8 * rows < 7 * aligned;
+}
+
 static int quant_rows(const fl_quant_args* const* args, int n, cudaStream_t st, const DocWork& docs = {}) {
   QuantRowsMaps maps;
   QuantRowsParams p = {};
@@ -951,6 +986,7 @@ static int quant_rows(const fl_quant_args* const* args, int n, cudaStream_t st, 
   const fl_quant_args* a = args[0];
   p.n_ops = n; p.n_tiles = (int)tiles;
   p.slot_src = a->slot_src; p.slot_rows = a->slot_rows;
+  p.skip_padding = mostly_padding(args, n);
   p.in_f16 = a->in_f16;
   p.docs = docs;
   p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);
@@ -983,6 +1019,7 @@ extern "C" int fl_quant_blocks(const fl_quant_args* a, void* stream) {
   p.row_stat = (uint32_t*)a->row_stat; p.row_stat_kind = a->row_stat_kind;
   p.b = a->b; p.s = a->s; p.h = a->h; p.n_tiles = (int)n_tiles;
   p.slot_src = a->slot_src; p.slot_rows = a->slot_rows;
+  p.skip_padding = mostly_padding(&a, 1);
   const bool packed = a->slot_src != nullptr;
   const int d_src = quant_cols(a);
   p.token_local = (a->flags & FL_Q_TOKEN_LOCAL) ? 1 : 0;
