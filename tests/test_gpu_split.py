@@ -65,8 +65,8 @@ FWD = [
 @pytest.mark.parametrize("b,sq,sk,h,hk,d,causal,form", FWD)
 def test_forward_in_pieces(b, sq, sk, h, hk, d, causal, form, share):
     """Every piece frames a row's P-hat as the whole item does (N(0, 1) operands: the first tile's maximum is refreshed by no later one), so
-    the rounded terms are the same but for one exponential in eight, which the two kernels take by the unit and by the polynomial (3e-6 apart: of
-    1e5 codes five fall on another value, a sixteenth away, 5e-4 of O's norm). O differs by that, f32 sums in another order and the last bit
+    the rounded terms are the same but for one exponential in four, by polynomials up to 7.5e-5 apart (codes of P-hat are about a
+    twelfth apart: of 1e5 codes some fifteen fall on another value, 1e-3 of O's norm). O differs by that, f32 sums in another order and the last bit
     of bfloat16 (2^-9): below 2^-8; the LSE by a few units of 2^-20 of logarithms up to about 10."""
     from flamia_blackwell_attention_b200 import _lib as L, kernels as K
     q, k, v, _ = attention_inputs(b, max(sq, sk), h, hk, d, seed=11)
