@@ -52,6 +52,10 @@
 // power-of-two factor. Per-key factors are per-thread scalars here, per-query factors are read per element; S and dP
 // take f_K f_Q and f_V f_dO in the elementwise math; dV takes f_dO inside a block-scaled P-hat (one exponent per key row
 // x 32 queries); dK takes f_Q inside its dS-hat codes, dQ takes f_K inside its own; the operand scale tiles are unit.
+// What bounds these kernels are the loads of the per-query tables: each returns 512 bytes to a warp, four clocks of the 2 350 of a half
+// tile, and eight warps took 48 each. VAR = 3 (FL_A_D_PER_FACTOR: D'' comes divided by f_dO, exactly, as f_dO is a power of two) takes
+// 40: P' f_dO, which P-hat needs, is all that dS = (P' f_dO) (f_V dP + D'' / f_dO) needs, too. b2 s8192 h32/8 d128 causal step, one B200:
+// 4062 -> 3923 us, 56 of the 139 from fewer live registers (VAR = 2 has these as well), same bits. VAR = 2 serves callers with D'' as it is.
 #include "flamia_internal.h"
 
 namespace fl {
@@ -269,7 +273,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                      const __grid_constant__ CUtensorMap tm_acc, const __grid_constant__ CUtensorMap tm_q4,
                      const __grid_constant__ CUtensorMap tm_k4, const __grid_constant__ CUtensorMap tm_dk,
                      const __grid_constant__ CUtensorMap tm_dv, const BwdParams p) {
-  using SM = BwdSmem<D, FP4, VAR == 2>;
+  using SM = BwdSmem<D, FP4, (VAR >= 2)>;
   constexpr int TILE_BYTES = 128 * D;
   constexpr uint64_t OP_SWZ = (D == 128) ? SWZ_128 : SWZ_64;     // operand tiles: rows of D bytes
   constexpr uint32_t OP_SBO = 8 * D;
@@ -278,7 +282,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
   BwdMisc& misc = *reinterpret_cast<BwdMisc*>(smem + SM::MISC);
   uint64_t* const bars = misc.bars;
   BTile* const tile_s = misc.tile;
-  constexpr bool RL = VAR >= 1, TL = VAR == 2;
+  constexpr bool RL = VAR >= 1, TL = VAR >= 2, FOLD = VAR == 3;
   constexpr int QW = bwd_qw(VAR), NQ = QW / 32, NWG = 128 / QW;      // queries, query blocks per warpgroup; warpgroups
   // Who gives a K / V buffer and its slot of tile_s back: the compute warps (gradient rows written, slot no longer read), each warp of
   // the reduction and each issuer (slot read; an item without query tiles does not hold these up, and an ordered dQ can keep the
@@ -869,16 +873,18 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           if constexpr (TL) {
             static_assert(!TL || QW == 32, "one query block per warpgroup");
             // block-scaled P-hat carrying f_dO(query): one exponent per (this key row, 32 queries). (Its atom's last reader, the dV
-            // product of the iteration before, has completed when dP^T has: the byte is written below.)
-            float t[32];
+            // product of the iteration before, has completed when dP^T has: the byte is written below.) FOLD: pf keeps the product, else it is
+            // taken again for the codes (32 registers less).
             float am = 0.f;
 #pragma unroll
             for (int j4 = 0; j4 < 8; ++j4) {
               const float4 f4 = lds128(v_fdo + 16 * j4);
               const int j = 4 * j4;
-              unpack2(mul2(pack2(pf[j + 0], pf[j + 1]), pack2(f4.x, f4.y)), t[j + 0], t[j + 1]);
-              unpack2(mul2(pack2(pf[j + 2], pf[j + 3]), pack2(f4.z, f4.w)), t[j + 2], t[j + 3]);
-              am = fmax3_abs(fmax3_abs(am, t[j], t[j + 1]), t[j + 2], t[j + 3]);   // all >= 0
+              float t0, t1, t2, t3;
+              unpack2(mul2(pack2(pf[j + 0], pf[j + 1]), pack2(f4.x, f4.y)), t0, t1);
+              unpack2(mul2(pack2(pf[j + 2], pf[j + 3]), pack2(f4.z, f4.w)), t2, t3);
+              am = fmax3_abs(fmax3_abs(am, t0, t1), t2, t3);   // all >= 0
+              if (FOLD) { pf[j + 0] = t0; pf[j + 1] = t1; pf[j + 2] = t2; pf[j + 3] = t3; }
             }
             ep = exp448(__float_as_uint(am));
             const float inv = pow2_inv(ep);
@@ -886,8 +892,14 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 #pragma unroll
             for (int w = 0; w < 8; ++w) {
               float a0, a1, a2, a3;
-              unpack2(mul2(pack2(t[4 * w], t[4 * w + 1]), inv2), a0, a1);
-              unpack2(mul2(pack2(t[4 * w + 2], t[4 * w + 3]), inv2), a2, a3);
+              uint64_t t01 = pack2(pf[4 * w], pf[4 * w + 1]), t23 = pack2(pf[4 * w + 2], pf[4 * w + 3]);
+              if (!FOLD) {
+                const float4 f4 = lds128(v_fdo + 16 * w);
+                t01 = mul2(t01, pack2(f4.x, f4.y));
+                t23 = mul2(t23, pack2(f4.z, f4.w));
+              }
+              unpack2(mul2(t01, inv2), a0, a1);
+              unpack2(mul2(t23, inv2), a2, a3);
               pw[w] = cvt_e4m3x4(a0, a1, a2, a3);
             }
           } else {
@@ -922,17 +934,21 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           const float4 d4 = lds128(v_dpp + 16 * j4);
           const int j = 4 * j4;
           if (TL) {
-            // b = f_V(key) f_dO(query) per column; the dK side's maximum and codes carry f_Q(query) (kept in pv)
-            const float4 f4 = lds128(v_fdo + 16 * j4);
+            // b = f_V(key) f_dO(query) per column (FOLD: f_dO is in pf, and D'' comes divided by it); the dK side's maximum and codes
+            // carry f_Q(query) (kept in pv), the dQ side's f_K(key)
             const float4 q4 = lds128(v_fq + 16 * j4);
             const uint64_t fv2 = pack2(fv8, fv8);
-            const uint64_t u01 = fma2(pack2(__uint_as_float(pv[j + 0]), __uint_as_float(pv[j + 1])),
-                                      mul2(pack2(f4.x, f4.y), fv2), pack2(d4.x, d4.y));
-            const uint64_t u23 = fma2(pack2(__uint_as_float(pv[j + 2]), __uint_as_float(pv[j + 3])),
-                                      mul2(pack2(f4.z, f4.w), fv2), pack2(d4.z, d4.w));
+            uint64_t b01 = fv2, b23 = fv2;
+            if (!FOLD) {
+              const float4 f4 = lds128(v_fdo + 16 * j4);
+              b01 = mul2(pack2(f4.x, f4.y), fv2);
+              b23 = mul2(pack2(f4.z, f4.w), fv2);
+            }
+            const uint64_t u01 = fma2(pack2(__uint_as_float(pv[j + 0]), __uint_as_float(pv[j + 1])), b01, pack2(d4.x, d4.y));
+            const uint64_t u23 = fma2(pack2(__uint_as_float(pv[j + 2]), __uint_as_float(pv[j + 3])), b23, pack2(d4.z, d4.w));
             const uint64_t p01 = mul2(pack2(pf[j + 0], pf[j + 1]), u01), p23 = mul2(pack2(pf[j + 2], pf[j + 3]), u23);
-            unpack2(p01, pf[j + 0], pf[j + 1]);
-            unpack2(p23, pf[j + 2], pf[j + 3]);
+            unpack2(mul2(p01, pack2(fk_true, fk_true)), pf[j + 0], pf[j + 1]);
+            unpack2(mul2(p23, pack2(fk_true, fk_true)), pf[j + 2], pf[j + 3]);
             float w0, w1, w2, w3;
             unpack2(mul2(p01, pack2(q4.x, q4.y)), w0, w1);
             unpack2(mul2(p23, pack2(q4.z, q4.w)), w2, w3);
@@ -1027,12 +1043,14 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             float v[4];
             uint32_t iv[4];
 #pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = pf[4 * w + e];
+#pragma unroll
             for (int e = 0; e < 4; ++e) {
-              const float a = TL ? pf[4 * w + e] * fk_true : pf[4 * w + e];
-              const int sb = __viaddmax_s32((int)warp_max_abs_f32(a), 0x00200000 - 0x03800000, 2 << 23);
+              const int sb = __viaddmax_s32((int)warp_max_abs_f32(v[e]), 0x00200000 - 0x03800000, 2 << 23);
               iv[e] = ~(uint32_t)sb & 0x7F800000u;
-              v[e] = a * __uint_as_float(iv[e]);
             }
+            unpack2(mul2(pack2(v[0], v[1]), pack2(__uint_as_float(iv[0]), __uint_as_float(iv[1]))), v[0], v[1]);
+            unpack2(mul2(pack2(v[2], v[3]), pack2(__uint_as_float(iv[2]), __uint_as_float(iv[3]))), v[2], v[3]);
             dsw[w] = cvt_e4m3x4(v[0], v[1], v[2], v[3]);
             uint32_t n = (lane & 2) ? ((lane & 1) ? iv[3] : iv[2]) : ((lane & 1) ? iv[1] : iv[0]);
             if (w & 1) {
@@ -1288,7 +1306,8 @@ static int bwd_launch(const fl_attn_args* a, const void* work, void* stream) {
   if (a->mode != FL_MODE_FP8 && a->mode != FL_MODE_FP4) return FL_ERR_UNSUPPORTED;
   const bool fp4 = a->mode == FL_MODE_FP4;
   if (fp4 && (!a->q4 || !a->k4 || !a->sfq4 || !a->sfk4)) return FL_ERR_BAD_ARG;
-  const bool tl = (a->flags & FL_A_TOKEN_LOCAL) != 0, rl = (a->flags & FL_A_DQ_ROWLOCAL) != 0;
+  const bool tl = (a->flags & FL_A_TOKEN_LOCAL) != 0, rl = (a->flags & FL_A_DQ_ROWLOCAL) != 0, fold = (a->flags & FL_A_D_PER_FACTOR) != 0;
+  if (fold && !tl) return FL_ERR_BAD_ARG;
   if (tl && (!rl || fp4 || a->doc_start)) return FL_ERR_UNSUPPORTED;   // token-local needs the dQ side's own codes
   if (a->d == 64 && (fp4 || rl || tl)) return FL_ERR_UNSUPPORTED;       // d = 64: the default 8-bit route only
   if (a->h <= 0 || a->h_kv <= 0 || a->h % a->h_kv) return FL_ERR_BAD_ARG;
@@ -1381,7 +1400,7 @@ static int bwd_launch(const fl_attn_args* a, const void* work, void* stream) {
   } else if (fp4) {
     rc = rl ? FL_BWD_LAUNCH(128, true, 1, false) : FL_BWD_LAUNCH(128, true, 0, false);
   } else if (tl) {
-    rc = FL_BWD_LAUNCH(128, false, 2, false);
+    rc = fold ? FL_BWD_LAUNCH(128, false, 3, false) : FL_BWD_LAUNCH(128, false, 2, false);
   } else {
     rc = rl ? FL_BWD_LAUNCH(128, false, 1, false) : FL_BWD_LAUNCH(128, false, 0, false);
   }

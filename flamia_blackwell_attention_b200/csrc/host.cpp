@@ -571,7 +571,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
   g.in_f16 = dout.scalar_type() == at::kHalf;
   TORCH_CHECK(dout.scalar_type() == out.scalar_type(), "dout is ", dout.scalar_type(), ", the output ", out.scalar_type());
   if (p.d_call != p.d) g.flags |= FL_Q_COLS(p.d_call);
-  if (p.token_local) { g.flags |= FL_Q_TOKEN_LOCAL; g.token_factors = ptr<float>(ws.at(w_tok)); }
+  if (p.token_local) { g.flags |= FL_Q_TOKEN_LOCAL | FL_Q_D_PER_FACTOR; g.token_factors = ptr<float>(ws.at(w_tok)); }
   g.codes = ptr<uint8_t>(ws.at(w_codes)); g.fac = ptr<float>(ws.at(w_fac));
   g.d_out = ptr<float>(ws.at(w_D)); g.lse_log2 = ptr<float>(ws.at(w_lse)); g.zero_acc = ws.at(w_acc);
   if (!rows) g.tile_stats = ptr<float>(ws.at(w_stats));
@@ -606,7 +606,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
                                                : std::vector<int64_t>{p.b, p.s_k, p.h_kv, p.d_call};
   const Tensor dq = empty(dout.sizes(), out.scalar_type(), dev), dk = empty(kshape, out.scalar_type(), dev),
                dv = empty(kshape, out.scalar_type(), dev);
-  a.flags |= (had8 ? FL_A_HAD_DK : 0) | (p.rowlocal ? FL_A_DQ_ROWLOCAL : 0);
+  a.flags |= (had8 ? FL_A_HAD_DK : 0) | (p.rowlocal ? FL_A_DQ_ROWLOCAL : 0) | (p.token_local ? FL_A_D_PER_FACTOR : 0);
   a.do_codes = g.codes; a.fac_do = p.token_local ? g.token_factors : g.fac;
   a.lse_log2 = g.lse_log2; a.d_rows = g.d_out; a.dq_acc = g.zero_acc;
   a.dk = ptr<void>(dk); a.dv = ptr<void>(dv);

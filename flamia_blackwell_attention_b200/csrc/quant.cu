@@ -50,7 +50,7 @@ struct QuantParams {
   const int32_t* slot_rows;  // packed source: valid rows of each slot (the rest of the slot reads as zero)
   int n_tiles;            // b * (s / 128) * h
   int skip_padding;       // host only: mostly_padding
-  int token_local;
+  int token_local, d_per_factor;
   int in_f16;
   float lse_shift, d_multiplier;
   DevCtl ctl;
@@ -453,7 +453,8 @@ quant_blocks_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       const float w2a = __fadd_rn(w4[0], w4[2]), w2b = __fadd_rn(w4[1], w4[3]);                  // bit 6
       float w1 = __fadd_rn(w2a, w2b);                                                            // bit 5
       w1 = __fadd_rn(w1, __shfl_xor_sync(0xFFFFFFFFu, w1, 2));                                   // bit 4 = lane bit 1
-      if (q == 0 && p.d_out) p.d_out[ri] = __fmul_rn(w1, p.d_multiplier);
+      w1 = __fmul_rn(w1, p.d_multiplier);
+      if (q == 0 && p.d_out) p.d_out[ri] = p.d_per_factor ? __fmul_rn(w1, inv) : w1;     // (a power of two: exact)
     }
     if (p.lse && p.lse_log2 && q == 0) {
       const float l = PRO ? lse_row : p.lse[ri];
@@ -934,6 +935,7 @@ static int check_quant_args(const fl_quant_args* a) {
   if (quant_cols(a) > a->d || quant_cols(a) % 8) return FL_ERR_BAD_ARG;
   if ((a->flags & (FL_Q_HADAMARD | FL_Q_HADAMARD_NVFP4_ONLY)) && a->d != 128) return FL_ERR_UNSUPPORTED;
   if ((a->flags & FL_Q_HADAMARD) && (a->flags & FL_Q_TOKEN_LOCAL)) return FL_ERR_UNSUPPORTED;
+  if ((a->flags & FL_Q_D_PER_FACTOR) && !(a->flags & FL_Q_TOKEN_LOCAL)) return FL_ERR_BAD_ARG;
   if ((a->flags & FL_Q_HADAMARD_NVFP4_ONLY) && !a->x4) return FL_ERR_BAD_ARG;
   if (a->h > 65535 || a->b > 65535) return FL_ERR_TOO_LARGE;
   if ((long long)a->b * (a->s / 128) * a->h > 0x7FFFFFFF) return FL_ERR_TOO_LARGE;
@@ -1023,6 +1025,7 @@ extern "C" int fl_quant_blocks(const fl_quant_args* a, void* stream) {
   const bool packed = a->slot_src != nullptr;
   const int d_src = quant_cols(a);
   p.token_local = (a->flags & FL_Q_TOKEN_LOCAL) ? 1 : 0;
+  p.d_per_factor = (a->flags & FL_Q_D_PER_FACTOR) ? 1 : 0;
   p.in_f16 = a->in_f16;
   p.lse_shift = a->lse_shift; p.d_multiplier = a->d_multiplier;
   p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);

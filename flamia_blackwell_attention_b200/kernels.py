@@ -38,7 +38,7 @@ def quantize_fp8_blocks(x, *, apply_hadamard_rotation=False, hadamard_rotation_s
                         output_sf_atoms=False, also_make_nvfp4_copy=False, compute_d_with_output=None,
                         shifted_log2_lse_from=None, log2_lse_shift=0.0, d_multiplier=1.0, zero_accumulator=None,
                         output_tile_stats=False, status=None, wait_cycles=0, packed_slots=None, row_stat=None,
-                        legacy_kernel=False):
+                        legacy_kernel=False, d_per_factor=False):
     """Token-block MXFP8 quantiser of x (b, s, h, d) bf16 / f16 (s % 128 == 0, d in {64, 128}).
     packed_slots = (slot_src, slot_rows, padded_rows): x is a packed (total, h, d) tensor of documents stored back to back
     and the outputs are those of the 128-aligned buffer (1, padded_rows, h, d): slot_src[i] = first row of x of output
@@ -69,7 +69,7 @@ def _quant_args(x, *, apply_hadamard_rotation=False, hadamard_rotation_scope="al
                 output_sf_atoms=False, also_make_nvfp4_copy=False, compute_d_with_output=None,
                 shifted_log2_lse_from=None, log2_lse_shift=0.0, d_multiplier=1.0, zero_accumulator=None,
                 output_tile_stats=False, status=None, wait_cycles=0, packed_slots=None, row_stat=None,
-                legacy_kernel=False):
+                legacy_kernel=False, d_per_factor=False):
     """(QuantArgs, outputs, what has to live until the launch) of one operand."""
     _require_cuda(x, "x")
     if x.dtype not in (torch.bfloat16, torch.float16):
@@ -94,6 +94,8 @@ def _quant_args(x, *, apply_hadamard_rotation=False, hadamard_rotation_scope="al
         flags |= L.FL_Q_HADAMARD if hadamard_rotation_scope == "all" else L.FL_Q_HADAMARD_NVFP4_ONLY
     if token_local_exponents:
         flags |= L.FL_Q_TOKEN_LOCAL
+    if d_per_factor:        # D divided by the token's factor, for attn_bwd(d_per_factor=True)
+        flags |= L.FL_Q_D_PER_FACTOR
     if legacy_kernel:       # the four-lanes-per-row kernel even where the one-thread-per-row kernel serves (same bits)
         flags |= L.FL_Q_LEGACY
     a.flags = flags
@@ -308,7 +310,7 @@ def code_stats(codes, descale):
 def attn_bwd(q, k, v, do, *, lse_log2, d_rows, dq_acc, dq_scale, causal, softmax_scale, out_dtype=torch.bfloat16,
              mode=L.FL_MODE_FP8, had_dk=False, status=None, doc_start=None, doc_len=None, wait_cycles=0,
              token_local=False, dq_rowlocal=False, window=None, seqused_k=None, softcap=0.0, dq_order=None,
-             dq_scale_rows=None, dk_mult=None, packed_out=None, work=None):
+             dq_scale_rows=None, dk_mult=None, packed_out=None, work=None, d_per_factor=False):
     """Backward main kernel on quantised operands. q / k / v / do: quantiser outputs (codes, fac). Adds the pre-scaled
     dQ partials into the f16 accumulator dq_acc of b * h * s_q * d elements ((b, h, d, s_q) at d = 128, (b, h, s_q, d)
     at d = 64) and returns (dk, dv, status), each (b, s_k, h_kv, d). dq_order: a zeroed (b, h, s_q / 128, 2) int32 table
@@ -322,7 +324,7 @@ def attn_bwd(q, k, v, do, *, lse_log2, d_rows, dq_acc, dq_scale, causal, softmax
     dk = torch.empty(b, rows_out, h_kv, d, dtype=out_dtype, device=dev)
     dv = torch.empty(b, rows_out, h_kv, d, dtype=out_dtype, device=dev)
     flags = (L.FL_A_OUT_F16 if out_dtype == torch.float16 else 0) | (L.FL_A_HAD_DK if had_dk else 0) | \
-        (L.FL_A_DQ_ROWLOCAL if dq_rowlocal else 0)
+        (L.FL_A_DQ_ROWLOCAL if dq_rowlocal else 0) | (L.FL_A_D_PER_FACTOR if d_per_factor else 0)
     a = attn_args(q, k, v, causal=causal, softmax_scale=softmax_scale, mode=mode, flags=flags, status=status,
                   doc_start=doc_start, doc_len=doc_len, wait_cycles=wait_cycles, token_local=token_local, window=window,
                   seqused_k=seqused_k, softcap=softcap)

@@ -25,6 +25,7 @@ extern "C" {
 #define FL_Q_TOKEN_LOCAL 2         /* codes / sf_tok from each token's own exponent */
 #define FL_Q_HADAMARD_NVFP4_ONLY 4 /* rotate only the values of the NVFP4 copy; the E4M3 codes stay unrotated */
 #define FL_Q_O_PACKED 8            /* packed source with the prologue: o has x's packed rows (else the outputs' rows) */
+#define FL_Q_D_PER_FACTOR 32       /* with FL_Q_TOKEN_LOCAL and the prologue: d_out divided by the token's factor */
 #define FL_Q_LEGACY 16             /* keep the four-lanes-per-row kernel where the one-thread-per-row kernel would serve
                                       (the two are bit-identical; for tests that compare them) */
 /* Columns of a row of x and o when they are fewer than d (a multiple of 8; bits 16.. of the flags): the missing columns read
@@ -96,6 +97,7 @@ int fl_quant_qkv(const fl_quant_args* q, const fl_quant_args* k, const fl_quant_
 #define FL_A_HAD_DK 32       /* backward: rotate dK back in the epilogue */
 #define FL_A_COLS(n) ((int32_t)(n) << 16) /* columns of a row of out / dk / dv when they are fewer than d (see FL_Q_COLS) */
 #define FL_A_P_GROUP 64      /* forward: group-frame P-hat (one UE8M0 exponent per query row and 32 keys) instead of the row frame */
+#define FL_A_D_PER_FACTOR 256 /* backward with FL_A_TOKEN_LOCAL: d_rows are divided by f_dO (FL_Q_D_PER_FACTOR): two loads and two products fewer a pair of scores */
 #define FL_A_NO_GRAD 128     /* forward: no backward reads its results (other roundings of P-hat, faster) */
 
 /* One attention problem. Operands are the quantiser's outputs; q / k / v / dO codes are (b, s, heads, d) E4M3. */
