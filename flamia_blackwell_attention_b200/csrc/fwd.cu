@@ -843,7 +843,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         p.lse[((size_t)T.bat * p.h + head) * p.s_q + qrow] = v;
       }
       tc_fence_before();                 // this stage's output has left tensor memory before the next item's P-hat is announced
-      if (warp & 3) mbar_arrive_warp(&bars[B_QE + kb]);
+      if ((warp & 3) || by_rows) mbar_arrive_warp(&bars[B_QE + kb]);     // (by rows: no copy reads the buffer)
       else pend = kb;
     }
     if (r == 0) tma_store_wait_read<0>();   // (shared memory must outlive the copies; the writes complete with the grid)
