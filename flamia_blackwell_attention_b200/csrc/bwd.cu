@@ -779,8 +779,14 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           const float sc[4] = {sc4.x, sc4.y, sc4.z, sc4.w};
           // (the words' sixteen instructions, once in the producer: d = 64 8 x 1024 x 12 93.2 -> 91.7 us, mixed route b4 s4096 h16 503 -> 496)
           const float2 words = *reinterpret_cast<const float2*>(&misc.scal[st][x][4]);
-          eq2 = __float_as_uint(words.x) & 0xFFFF;
-          edo2 = __float_as_uint(words.x) >> 16;
+          if constexpr (SC && D == 128) {        // from the factors (mixed route b5 s1536 h4/1 dense 126 -> 119 us, 8-bit 1 %, d = 64 +0.6 %)
+            auto e8 = [](float f) { return (__float_as_uint(f) >> 23) & 0xFF; };
+            eq2 = e8(sc[0]) | (e8(sc[1]) << 8);
+            edo2 = e8(sc[2]) | (e8(sc[3]) << 8);
+          } else {
+            eq2 = __float_as_uint(words.x) & 0xFFFF;
+            edo2 = __float_as_uint(words.x) >> 16;
+          }
           ekb_word = __vadd4(ek_word, __float_as_uint(words.y));
 #pragma unroll
           for (int qh = 0; qh < NQ; ++qh) {        // a pre-scale per query row: folded into the dQ side's B scale bytes
