@@ -889,7 +889,7 @@ static int launch_quant_rows(const QuantRowsMaps& maps, const QuantRowsParams& p
     return FL_OK;
   };
   return !p.slot_src ? launch(quant_rows_kernel<MODE, D, 0>)
-         : p.skip_padding && p.n_tiles > grid ? launch(quant_rows_kernel<MODE, D, 2>) : launch(quant_rows_kernel<MODE, D, 1>);
+         : p.skip_padding && p.n_tiles > 3 * grid ? launch(quant_rows_kernel<MODE, D, 2>) : launch(quant_rows_kernel<MODE, D, 1>);
 }
 
 template <int D, int MODE, bool PRO, int STEPS, int PK>
@@ -906,7 +906,7 @@ static int launch_quant_pk(const CUtensorMap& mx, const CUtensorMap& mo, const Q
 template <int D, int MODE, bool PRO, int STEPS = 1>
 static int launch_quant(const CUtensorMap& mx, const CUtensorMap& mo, const QuantParams& p, bool want_t, cudaStream_t st) {
   if (!p.slot_src) return launch_quant_pk<D, MODE, PRO, STEPS, 0>(mx, mo, p, want_t, st);
-  if (PRO && p.skip_padding && p.n_tiles > sm_count() * q_blocks(PRO, STEPS)) return launch_quant_pk<D, MODE, PRO, STEPS, PRO ? 2 : 1>(mx, mo, p, want_t, st);
+  if (PRO && p.skip_padding && p.n_tiles > 3 * sm_count() * q_blocks(PRO, STEPS)) return launch_quant_pk<D, MODE, PRO, STEPS, PRO ? 2 : 1>(mx, mo, p, want_t, st);
   return launch_quant_pk<D, MODE, PRO, STEPS, 1>(mx, mo, p, want_t, st);
 }
 
@@ -958,8 +958,9 @@ static int quant_mode(const fl_quant_args* a) {
 
 // Packed sources: is more than an eighth of the tiles' rows past the end of a document? Then the kernels in which the warps of such rows
 // leave their work out (PK = 2): 352 documents of 30 to 60 rows, h16/16, d = 128, step 869 -> 815 us; 210 of 100 to 200 454 -> 448; 6000
-// rows in documents of 16 to 1024, h16/4, 182.5 -> 181.2. Not where the documents are long (16k rows in 4, 672 -> 677), and not in
-// a launch of one round, which is over before the shorter way pays for the longer code (75 rows h16/8, mixed route, forward 14.4 -> 14.9).
+// rows in documents of 16 to 1024, h16/4, 182.5 -> 181.2. Not where the documents are long (16k rows in 4, 672 -> 677), and not in a
+// launch of up to three rounds, which is over before the shorter way pays for the longer code (75 rows h16/8, mixed route, forward 14.4 ->
+// 14.9; 1.1 rounds, prologue, d = 64, 8.4 -> 8.9; 1.2 rounds, rows, 9.7 -> 9.9; 2.7 rounds the same; 3.4 rounds, rows, 30.1 -> 29.4).
 static bool mostly_padding(const fl_quant_args* const* args, int n) {
   long long rows = 0, aligned = 0;
   for (int i = 0; i < n; ++i) rows += (long long)args[i]->src_rows * args[i]->h, aligned += (long long)args[i]->s * args[i]->h;

@@ -1,4 +1,4 @@
-"""Quantiser launches of more tiles than one round, whose warps past a document's end write zeros and do nothing else, against launches
+"""Quantiser launches of more tiles than three rounds, whose warps past a document's end write zeros and do nothing else, against launches
 that treat every row alike, bit for bit."""
 import pytest
 import torch
@@ -32,7 +32,7 @@ LENS = [1, 8, 9, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 300] * 30   
                                                   (64, False, False, "float16"), (128, False, False, "bfloat16")])
 def test_rows_kernel(d, rotate, nvfp4, dtype):
     from flamia_blackwell_attention_b200 import kernels as K
-    x = attention_inputs(1, sum(LENS), 2, 1, d, seed=61)[0][0].to(getattr(torch, dtype)).cuda()
+    x = attention_inputs(1, sum(LENS), 4, 1, d, seed=61)[0][0].to(getattr(torch, dtype)).cuda()
     kw = dict(packed_slots=_slots(LENS), output_tile_stats=True, also_make_nvfp4_copy=nvfp4, apply_hadamard_rotation=rotate,
               hadamard_rotation_scope="nvfp4_copy" if nvfp4 else "all")
     many, plain = K.quantize_fp8_blocks(x, **kw), K.quantize_fp8_blocks(x, legacy_kernel=True, **kw)
@@ -41,9 +41,9 @@ def test_rows_kernel(d, rotate, nvfp4, dtype):
 
 @pytest.mark.parametrize("d,o_packed", [(128, True), (64, True), (128, False)])
 def test_prologue(d, o_packed):
-    """One head more than a round (either form of the prologue) against a head at a time, which is less than one."""
+    """Heads for more than three rounds (either form of the prologue; two heads: of one of them) against a head at a time."""
     from flamia_blackwell_attention_b200 import kernels as K
-    lens = LENS[:96]
+    lens = LENS[:192]
     slots = _slots(lens)
     h, s = 6, slots[2]
     x, o = (t[0].cuda() for t in attention_inputs(1, sum(lens), h, h, d, seed=62)[:2])
