@@ -213,17 +213,13 @@ __device__ __forceinline__ void fwd_cut(const fl_split& s, int cta, int L, Tile&
 
 // FULL: the variants that also serve packed outputs and the output-row factor, each behind a run-time check of its
 // pointer. A template flag, so that the kernels of the plain calls carry none of that code (-2 % kernel time).
-// FINE: calls without gradients (FL_A_NO_GRAD), see the exponentials. With gradients the codes of P-hat stay what the degree-3 polynomial
-// made them: another rounding of P-hat moves D and with it codes of dS by a whole step, which rows of few keys and outlier channels
-// show in full (b2 s8192 h32/8, token factors, one channel in a hundred twenty times as large: dQ by up to 6 times its root mean square,
-// at one value in a million), and it would gain a training step 0.2 to 0.5 %; with token factors it is slower (4062 -> 4089 us a step).
 // TLV (token-local): 1 = the per-key factors come from three float tables, 2 = from the narrow ones. What bounds these kernels is the
 // wait for the table loads (long scoreboard 3.0 of the 9.0 clocks a warp takes to an instruction, no pipe above half): a broadcast load
 // of 16 bytes returns 512 to a warp, and three float tables are 96 of them per 128 keys, the narrow ones 48 (the quantiser's factors
 // are powers of two, their logarithms small integers: bfloat16 holds them exactly, a shift or a mask takes each one out again, and the
 // results are the same bits; long scoreboard 1.5 of 6.4). b2 s8192 h32/8 d128 causal, one B200: 1725 -> 1475 us. 1 serves callers of
 // fl_fwd with tables of their own, in 32 bits.
-template <int D, bool FP4, int TLV, bool GF, bool SC, bool FULL = false, bool SPLIT = false, bool FINE = SPLIT>
+template <int D, bool FP4, int TLV, bool GF, bool SC, bool FULL = false, bool SPLIT = false>
 __global__ void __launch_bounds__(384, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
            const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const FwdParams p,
@@ -685,11 +681,13 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           }
           float p0 = ex2(a0), p1 = ex2(a1);
           float p2, p3;
-          // One pair in four on the FMA pipe, by the degree-3 polynomial; FINE: three in eight, by the degree-4 one (a twenty-fifth of the
-          // error). b4 s4096 h16: dense 378 -> 365 us, causal 215 -> 214, mixed route 219 -> 215 (none: +8 % dense, half: +8 %). Split schedules
-          // keep one in four (4608 x 18432 h4 119 -> 112).
-          if (FINE && !SPLIT ? (w & 3) != 0 : (w & 1) != 0) {
-            ex2_poly2<FINE ? 4 : 3>(a2, a3, p2, p3);
+          // One pair in four on the FMA pipe (b4 s4096 h16, none: +4 % kernel time causal, +8 % dense; half: +8 % dense). Not another share or a
+          // polynomial of another degree for calls without gradients alone (three in eight of degree 4: dense 378 -> 365 us): a call without
+          // gradients returns the bytes of the call with them, as recomputing a layer's activations wants it. Nor for all calls: another
+          // rounding of P-hat moves D and with it codes of dS by a whole step (b2 s8192 h32/8, token factors, one channel in a hundred twenty
+          // times as large: dQ by up to 6 times its root mean square, at one value in a million).
+          if (w & 1) {
+            ex2_poly2(a2, a3, p2, p3);
           } else {
             p2 = ex2(a2);
             p3 = ex2(a3);
@@ -1004,11 +1002,10 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, con
   p.cap_a = sc ? a->softcap * 1.4426950408889634f : 0.f;
   p.cap_b = sc ? 1.0f / p.cap_a : 0.f;
   // the lean kernels serve the plain calls; documents, packed outputs and the output-row factor take the full variant
-  const bool full = a->doc_start != nullptr || a->o_mult != nullptr, fine = (a->flags & FL_A_NO_GRAD) != 0;
+  const bool full = a->doc_start != nullptr || a->o_mult != nullptr;
 #define FL_FWD_LAUNCH(D_, FP4_, TL_, GF_, SC_)                                                                          \
   (split  ? launch(fwd_kernel<D_, FP4_, 0, GF_, SC_, false, true>, Cuts<true>{*split})   \
    : full ? launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, true>, Cuts<false>{})                                         \
-   : fine ? launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, false, false, TL_ == 0 && !SC_>, Cuts<false>{})               \
           : launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, false>, Cuts<false>{}))
   if (sc) {
     if (fp4) rc = gf ? FL_FWD_LAUNCH(128, true, 0, true, true) : FL_FWD_LAUNCH(128, true, 0, false, true);

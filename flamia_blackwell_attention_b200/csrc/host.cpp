@@ -448,7 +448,6 @@ State forward(int64_t handle, const Tensor& q_, const Tensor& k_, const Tensor& 
   fl_attn_args a = {};
   attn_common(a, p, sh, f16);
   if (p.p_group) a.flags |= FL_A_P_GROUP;
-  if (!p.need_bwd) a.flags |= FL_A_NO_GRAD;
   a.q_codes = ptr<uint8_t>(qq.codes); a.k_codes = ptr<uint8_t>(kq.codes); a.v_codes = ptr<uint8_t>(vq.codes);
   a.fac_q = ptr<float>(p.token_local ? qq.token_factors : qq.fac);
   a.fac_k = ptr<float>(p.token_local ? kq.token_factors : kq.fac);

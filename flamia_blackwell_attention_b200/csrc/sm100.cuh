@@ -412,26 +412,17 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
 }
 // 2^x for two arguments on the FMA pipe instead of the transcendental unit (one warp instruction per 8 clocks and
 // scheduler, shared by the two softmax warpgroups): n = round(x) through the 1.5 * 2^23 trick, f = x - n in [-0.5, 0.5],
-// 2^f by a polynomial of DEGREE 3 (weighted least-squares fit of the relative error on Chebyshev nodes: max 7.5e-5) or 4
-// (2.7e-6), then n is added into the exponent field. Arguments below -126 give 2^-126.
-template <int DEGREE>
+// 2^f by a degree-3 polynomial (weighted least-squares fit of the relative error on Chebyshev nodes: max 7.5e-5),
+// then n is added into the exponent field. Arguments below -126 give 2^-126.
 __device__ __forceinline__ void ex2_poly2(float x0, float x1, float& r0, float& r1) {
   constexpr float MAGIC = 12582912.f;
   const uint64_t x = pack2(fmaxf(x0, -126.f), fmaxf(x1, -126.f));
   const uint64_t xr = add2(x, pack2(MAGIC, MAGIC));
   const uint64_t n = add2(xr, pack2(-MAGIC, -MAGIC));
   const uint64_t f = fma2(n, pack2(-1.f, -1.f), x);
-  uint64_t p;
-  if (DEGREE == 3) {
-    p = fma2(f, pack2(0.0551716685295105f, 0.0551716685295105f), pack2(0.2426111251115799f, 0.2426111251115799f));
-    p = fma2(p, f, pack2(0.6932609677314758f, 0.6932609677314758f));
-    p = fma2(p, f, pack2(0.9999280571937561f, 0.9999280571937561f));
-  } else {
-    p = fma2(f, pack2(0.009570087306201458f, 0.009570087306201458f), pack2(0.05591785907745361f, 0.05591785907745361f));
-    p = fma2(p, f, pack2(0.2402474582195282f, 0.2402474582195282f));
-    p = fma2(p, f, pack2(0.6931217908859253f, 0.6931217908859253f));
-    p = fma2(p, f, pack2(0.9999992847442627f, 0.9999992847442627f));
-  }
+  uint64_t p = fma2(f, pack2(0.0551716685295105f, 0.0551716685295105f), pack2(0.2426111251115799f, 0.2426111251115799f));
+  p = fma2(p, f, pack2(0.6932609677314758f, 0.6932609677314758f));
+  p = fma2(p, f, pack2(0.9999280571937561f, 0.9999280571937561f));
   float a0, a1, b0, b1;
   unpack2(p, a0, a1);
   unpack2(xr, b0, b1);

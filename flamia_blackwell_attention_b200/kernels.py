@@ -189,13 +189,13 @@ def attn_args(q, k, v, *, causal, softmax_scale, mode=L.FL_MODE_FP8, flags=0, st
 
 def attn_fwd(q, k, v, *, causal, softmax_scale, out_dtype=torch.bfloat16, mode=L.FL_MODE_FP8, status=None,
              doc_start=None, doc_len=None, wait_cycles=0, token_local=False, window=None, p_group=False, seqused_k=None,
-             softcap=0.0, o_mult=None, packed_out=None, work=None, split=None, no_grad=False):
+             softcap=0.0, o_mult=None, packed_out=None, work=None, split=None):
     """Forward kernel on quantised operands. Returns (out (b, s_q, h, d), lse (b, h, s_q) float32, status).
     p_group: group-frame P-hat (one UE8M0 exponent per query row and 32 keys) instead of the row frame.
     o_mult: (b, h_kv) f32 factor on the output rows (the mantissa of a V factor that is no power of two).
     packed_out = (slot_src, slot_rows, total): documents; out is (1, total, h, d) with the documents stored back to back
     (the kernel writes the caller's packed rows itself); lse keeps the aligned buffer's rows. work: the documents' work lists (doc_work).
-    split: a schedule (_lib.Split) that deals out the items' key tiles instead of whole items. no_grad: no backward reads the results."""
+    split: a schedule (_lib.Split) that deals out the items' key tiles instead of whole items."""
     qc = q["codes"]
     b, s_q, h, d = qc.shape
     dev = qc.device
@@ -208,8 +208,8 @@ def attn_fwd(q, k, v, *, causal, softmax_scale, out_dtype=torch.bfloat16, mode=L
         alloc(b, s_q, h, d, dtype=out_dtype, device=dev)
     lse = alloc(b, h, s_q, dtype=torch.float32, device=dev)
     a = attn_args(q, k, v, causal=causal, softmax_scale=softmax_scale, mode=mode,
-                  flags=(L.FL_A_OUT_F16 if out_dtype == torch.float16 else 0) | (L.FL_A_P_GROUP if p_group else 0) |
-                  (L.FL_A_NO_GRAD if no_grad else 0), status=status, doc_start=doc_start,
+                  flags=(L.FL_A_OUT_F16 if out_dtype == torch.float16 else 0) | (L.FL_A_P_GROUP if p_group else 0),
+                  status=status, doc_start=doc_start,
                   doc_len=doc_len, wait_cycles=wait_cycles, token_local=token_local, window=window, seqused_k=seqused_k,
                   softcap=softcap)
     a.out, a.lse = L.ptr(out), L.ptr(lse)

@@ -98,7 +98,6 @@ int fl_quant_qkv(const fl_quant_args* q, const fl_quant_args* k, const fl_quant_
 #define FL_A_COLS(n) ((int32_t)(n) << 16) /* columns of a row of out / dk / dv when they are fewer than d (see FL_Q_COLS) */
 #define FL_A_P_GROUP 64      /* forward: group-frame P-hat (one UE8M0 exponent per query row and 32 keys) instead of the row frame */
 #define FL_A_D_PER_FACTOR 256 /* backward with FL_A_TOKEN_LOCAL: d_rows are divided by f_dO (FL_Q_D_PER_FACTOR): two loads and two products fewer a pair of scores */
-#define FL_A_NO_GRAD 128     /* forward: no backward reads its results (other roundings of P-hat, faster) */
 
 /* One attention problem. Operands are the quantiser's outputs; q / k / v / dO codes are (b, s, heads, d) E4M3. */
 typedef struct fl_attn_args {
