@@ -45,13 +45,6 @@ class AttnArgs(C.Structure):
                [(n, i32) for n in ("window_left_p1", "window_right_p1")] + [("seqused_k", vp), ("softcap", f32), ("dq_order", vp), ("dq_scale_rows", vp), ("o_mult", vp), ("dk_mult", vp), ("slot_src", vp), ("slot_rows", vp), ("out_rows", i32), ("tok_lg_v", vp), ("tok_rcp_v", vp)]
 
 
-SPLIT_MAX, SPLIT_TILE_BITS = 160, 12
-
-
-class Split(C.Structure):
-    _fields_ = [("parts", i32), ("at", C.c_uint32 * (SPLIT_MAX + 1))]
-
-
 EXPORTS = {
     "fl_abi_version": (i32, []),
     "fl_quant_blocks": (i32, [C.POINTER(QuantArgs), vp]),
@@ -59,8 +52,6 @@ EXPORTS = {
     "fl_quant_qkv_work": (i32, [C.POINTER(QuantArgs), C.POINTER(QuantArgs), C.POINTER(QuantArgs), vp, vp, i32, i32, i32, i32, i32, i32, vp,
                                vp]),
     "fl_fwd": (i32, [C.POINTER(AttnArgs), vp]),
-    "fl_fwd_split_plan": (i32, [C.POINTER(AttnArgs), i32, C.POINTER(Split)]),
-    "fl_fwd_split": (i32, [C.POINTER(AttnArgs), C.POINTER(Split), vp, vp]),
     "fl_bwd": (i32, [C.POINTER(AttnArgs), vp]),
     "fl_dq_prescale": (i32, [vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp, vp, vp]),
     "fl_bwd_static_acc": (i32, [C.POINTER(AttnArgs), vp, f32, vp, vp]),

@@ -6,9 +6,6 @@
 
 #include "flamia_internal.h"
 
-#include <algorithm>
-#include <vector>
-
 namespace fl {
 
 EncodeTiledFn get_encode_tiled() {
@@ -132,63 +129,6 @@ int make_acc_t_map_16(CUtensorMap* m, const void* base, int b, int heads, int d,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? FL_OK : cuda_fail(10000 + (int)r, "cuTensorMapEncodeTiled");
-}
-
-// A grid of one CTA an SM that takes whole items is as long as its fullest CTA: with fewer items than SMs, or a few rounds of them,
-// much of the chip waits (one round of causal items is twice as long as their mean). The split schedule deals out equal shares of
-// the items' tiles instead, in the items' order: a CTA's share is whole items and a piece of one at either end. Every share W from the
-// smallest that the CTAs can hold upwards is tried, and the best is taken if it beats the whole items by 3 % and a half tile. (A tile
-// of a split kernel takes some 5 % longer.)
-int plan_split(const int* n, int runs, long long reps, bool by_kind, int ctas, float overhead, float lead, float merge, float merge_part,
-               fl_split* out) {
-  out->parts = 0;
-  const long long items = runs * reps;
-  constexpr int MAX_TILES = (1 << FL_SPLIT_TILE_BITS) - 1, MIN_PIECE = 2;
-  if (ctas < 2 || ctas > FL_SPLIT_MAX || items > 8ll * ctas) return FL_OK;      // (many rounds: at most a few per cent to gain)
-  auto tiles = [&](long long i) { return n[by_kind ? i / reps : i % runs]; };
-  double total = 0;
-  std::vector<double> load(ctas, 0.0);
-  for (long long i = 0; i < items; ++i) {
-    const int t = tiles(i), k = (int)(i / ctas), c = (int)(i % ctas);
-    if (t > MAX_TILES) return FL_OK;
-    total += t + overhead;
-    load[by_kind && (k & 1) ? ctas - 1 - c : c] += t + overhead;
-  }
-  double whole = 0;
-  for (double l : load) whole = std::max(whole, l);
-  fl_split cand;
-  // shares of at most W: false where the CTAs do not hold all items. pieces: partial results
-  auto deal = [&](double W, int& pieces) -> bool {
-    int c = 0;
-    double l = 0;
-    pieces = 0;
-    cand.at[0] = 0;
-    for (long long i = 0; i < items; ++i) {
-      int t0 = 0;
-      for (const int t = tiles(i);;) {
-        const int rest = t - t0;
-        const double fix = overhead + (t0 ? lead : 0.f);
-        if (l + fix + rest <= W || (l == 0 && rest < 2 * MIN_PIECE)) { l += fix + rest; pieces += t0 > 0; break; }
-        int take = std::min((int)(W - l - fix), rest - MIN_PIECE);
-        if (take < MIN_PIECE && l == 0) take = MIN_PIECE;
-        if (take >= MIN_PIECE) { t0 += take; ++pieces; }
-        if (++c >= ctas) return false;
-        cand.at[c] = (uint32_t)i << FL_SPLIT_TILE_BITS | (uint32_t)t0;
-        l = 0;
-      }
-    }
-    cand.parts = c + 1;
-    cand.at[c + 1] = (uint32_t)items << FL_SPLIT_TILE_BITS;
-    return true;
-  };
-  double best = whole * 0.97 - 0.6;
-  for (double W = std::max(total / ctas, (double)overhead + lead + 2 * MIN_PIECE); W * 1.05 + merge < best; W *= 1.04) {
-    int pieces;
-    if (!deal(W, pieces) || !pieces) continue;
-    const double cost = W * 1.05 + merge + merge_part * pieces;
-    if (cost < best) { best = cost; *out = cand; }
-  }
-  return FL_OK;
 }
 
 }  // namespace fl

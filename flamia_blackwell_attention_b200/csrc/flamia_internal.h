@@ -75,13 +75,6 @@ struct FastDiv {
 // so that the kernels' sums of a position and a side stay inside 32 bits.
 inline int window_side(int32_t p1) { return p1 <= 0 ? -1 : p1 - 1 < (1 << 30) ? p1 - 1 : (1 << 30); }
 
-// Split schedule of a persistent grid on `ctas` CTAs, or none (parts = 0) where one would not pay: see abi.cu. Items: `runs` kinds of
-// n[i] tiles, `reps` items of each; by_kind: the items of a kind follow each other (and are dealt out in zigzag rounds when they are not
-// split), otherwise the kinds alternate. overhead, lead: what an item costs beside its tiles, and a piece that does not start it besides;
-// merge, merge_part: the merge, and what each partial result adds to it; all in tiles.
-int plan_split(const int* n, int runs, long long reps, bool by_kind, int ctas, float overhead, float lead, float merge, float merge_part,
-               fl_split* out);
-
 static constexpr long long kDefaultWaitCycles = 1ll << 31;
 
 }  // namespace fl

@@ -45,9 +45,6 @@
 // after the reader. All waits are bounded (sm100.cuh); a kernel that gives up writes a code to the status word and drains.
 #include "flamia_internal.h"
 
-#include <algorithm>
-#include <vector>
-
 namespace fl {
 
 static constexpr int KV_STAGES = 3;
@@ -77,8 +74,7 @@ struct FwdParams {
   const float* o_mult;        // (b, h_kv) factor on the output rows (V's mantissa with float descales), or null
   const int32_t* slot_src;    // packed output: packed row of each 128-row slot of the aligned buffer (-1: empty), or null
   const int32_t* slot_rows;   // packed output: real rows of each slot
-  void* out;                  // packed output: the (out_rows, h, d) tensor (row stores of a document's last rows); split: O, for the merge
-  float* part;                // split schedule: the partial results
+  void* out;                  // packed output: the (out_rows, h, d) tensor (row stores of a document's last rows)
   int n_docs;
   int b, s_q, s_k, h, h_kv;
   int q_len, k_len;      // batched form: a batch row's queries and keys (s_q, s_k, or fewer where those are rounded up to whole tiles)
@@ -92,6 +88,7 @@ struct FwdParams {
   FastDiv div_item, div_h, div_grp;   // items per (causal: row block; otherwise: head), query heads, group size
   int n_items;           // work items: 256-row blocks x heads x batch rows (documents: block slots x heads)
   int n_blk;             // blocks per batch row (documents: block slots of the packed buffer)
+  int blk_rows;          // batched form: query rows of a block, 256 or 128
   int zigzag;            // deal the items out in zigzag rounds (causal: they are ordered longest first)
   DevCtl ctl;
 };
@@ -108,23 +105,7 @@ struct Tile {
   int qrel;   // document-relative index of row q0
   int kofs;   // document-relative key of the first key row this item loads (a multiple of 128; > 0 under a left window)
   int n[2];   // key tiles stage 0 / 1 walks: keys [kofs, kmax_i), n_i = ceil((kmax_i - kofs) / 128)
-  // split schedule (SPLIT kernels only)
-  int part;   // where this piece's partial result goes, -1 = the whole item
-  int seed;   // 1: the piece's first key tile is the item's own first one, for its maximum alone (fwd_cut)
-  int back;   // how many tiles before the place of tile 0 that one lies
 };
-
-// A split schedule (fl_split): CTA c works from position at[c] up to at[c + 1] of the list of items, a position being a key tile of
-// an item. What lies between two positions is whole items and, at its two ends, pieces of one.
-template <bool SPLIT>
-struct Cuts {};
-template <>
-struct Cuts<true> { fl_split s; };
-__host__ __device__ inline int cut_item(uint32_t at) { return (int)(at >> FL_SPLIT_TILE_BITS); }
-__host__ __device__ inline int cut_tile(uint32_t at) { return (int)(at & ((1u << FL_SPLIT_TILE_BITS) - 1)); }
-// a piece's partial result: the rows' maxima and sums, then O as [column / 4][row][4]: a warp stores and loads 512 bytes in a row
-template <int D>
-constexpr size_t fwd_part_floats() { return 512 + 256 * D; }
 
 // barrier indices
 enum { B_Q = 0, B_QE = 2, B_KFULL = 4, B_KEMPTY = B_KFULL + KV_STAGES, B_VFULL = B_KEMPTY + KV_STAGES,
@@ -153,7 +134,7 @@ __device__ __forceinline__ void fwd_decode(const FwdParams& p, int L, Tile& t) {
     const int q = p.div_item.div(L), rq = L - q * p.div_item.d;
     const int blk = p.causal ? p.n_blk - 1 - q : rq, rem = p.causal ? rq : q;
     t.bat = p.div_h.div(rem); t.head = rem - t.bat * p.h;
-    t.q0 = blk * 256; t.nq = min(256, p.q_len - t.q0); t.k0 = 0; t.sk = p.k_len;
+    t.q0 = blk * p.blk_rows; t.nq = min(p.blk_rows, p.q_len - t.q0); t.k0 = 0; t.sk = p.k_len;
     if (p.seqused_k) t.sk = max(0, min(p.k_len, p.seqused_k[t.bat]));    // keys past it are masked like a document's end
     t.off = p.k_len - p.q_len; t.qrel = t.q0;
   } else {
@@ -191,26 +172,6 @@ __device__ __forceinline__ void fwd_decode(const FwdParams& p, int L, Tile& t) {
   }
 }
 
-// Item L of CTA `cta` cut down to the CTA's piece of it. P-hat's frame is the running maximum that was last refreshed, nearly always
-// the item's first key tile's; and the rounding to E4M3 goes with the frame. So that a row's probabilities are rounded alike
-// wherever its item is cut, a piece that starts further on takes the maximum of the item's first tile before its own tiles: a
-// product and a maximum without exponentials, 0.4 of a tile. (Pieces that frame their rows by their own first tile are as close to the exact
-// result, but 3e-2 away from the whole item's; like this 1e-3.)
-__device__ __forceinline__ void fwd_cut(const fl_split& s, int cta, int L, Tile& t) {
-  const uint32_t at0 = s.at[cta], at1 = s.at[cta + 1];
-  const int a = L == cut_item(at0) ? cut_tile(at0) : 0, b = L == cut_item(at1) ? cut_tile(at1) : 0;
-  t.part = a ? 2 * cta : b ? 2 * cta + 1 : -1;
-  t.seed = a ? 1 : 0;
-  t.back = a ? a - 1 : 0;
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int n = (b ? min(t.n[i], b) : t.n[i]) - a;
-    t.n[i] = n > 0 ? n + t.seed : 0;
-  }
-  t.kofs += 128 * t.back;
-  t.k0 += 128 * t.back;
-}
-
 // FULL: the variants that also serve packed outputs and the output-row factor, each behind a run-time check of its
 // pointer. A template flag, so that the kernels of the plain calls carry none of that code (-2 % kernel time).
 // TLV (token-local): 1 = the per-key factors come from three float tables, 2 = from the narrow ones. What bounds these kernels is the
@@ -219,11 +180,10 @@ __device__ __forceinline__ void fwd_cut(const fl_split& s, int cta, int L, Tile&
 // are powers of two, their logarithms small integers: bfloat16 holds them exactly, a shift or a mask takes each one out again, and the
 // results are the same bits; long scoreboard 1.5 of 6.4). b2 s8192 h32/8 d128 causal, one B200: 1725 -> 1475 us. 1 serves callers of
 // fl_fwd with tables of their own, in 32 bits.
-template <int D, bool FP4, int TLV, bool GF, bool SC, bool FULL = false, bool SPLIT = false>
+template <int D, bool FP4, int TLV, bool GF, bool SC, bool FULL = false>
 __global__ void __launch_bounds__(384, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-           const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const FwdParams p,
-           const __grid_constant__ Cuts<SPLIT> cuts) {
+           const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const FwdParams p) {
   constexpr bool TL = TLV != 0;
   constexpr int TILE_BYTES = 128 * D;
   constexpr uint64_t SWZ = (D == 128) ? SWZ_128 : SWZ_64;
@@ -277,14 +237,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   __syncthreads();
   tc_fence_after();
   const int n_items = FULL && p.work ? *reinterpret_cast<const volatile int*>(&p.work->x) * p.h : p.n_items;
-  auto item_of = [&](int k) {            // SPLIT: the CTA's share (the first and the last of its items may be pieces)
-    if constexpr (SPLIT) {
-      const int L = cut_item(cuts.s.at[cta]) + k;
-      return (uint32_t)L << FL_SPLIT_TILE_BITS < cuts.s.at[cta + 1] ? L : n_items;
-    } else {
-      return fwd_item(k, G, cta, p.zigzag);
-    }
-  };
   const uint32_t tmem = tmem_base_s;
   volatile int* abortp = &abort_s;
   // (a status word already set by an earlier launch is not looked at: a kernel that runs after one that gave up does no harm)
@@ -296,7 +248,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       int gj = 0;                          // key tiles issued so far, over all items (the K / V ring never restarts)
       bool ok = true;
       for (int k = 0; ok; ++k) {
-        const int L = item_of(k);
+        const int L = fwd_item(k, G, cta, p.zigzag);
         if (L >= n_items) break;
         const int kb = k & 1;
         // the Q buffer of item k - 2 (and its slot of tile_s) is free once both softmax warpgroups have written its
@@ -304,7 +256,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         if (k >= 2 && !(ok = mbar_wait(&bars[B_QE + kb], ((k >> 1) - 1) & 1, p.ctl, abortp, 12))) break;
         Tile t;
         fwd_decode<FULL>(p, L, t);
-        if constexpr (SPLIT) fwd_cut(cuts.s, cta, L, t);
         tile_s[kb] = t;
         const int hkv = t.hkv;
         if (t.nq > 0) {
@@ -321,19 +272,14 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         const int n_max = max(t.n[0], t.n[1]);
         for (int j = 0; j < n_max; ++j, ++gj) {
           const int st = gj % KV_STAGES, ph = (gj / KV_STAGES) & 1;
-          const int tj = SPLIT && j == 0 ? -t.back : j;
           if (gj >= KV_STAGES && !(ok = mbar_wait(&bars[B_KEMPTY + st], ph ^ 1, p.ctl, abortp, 10))) break;
           mbar_arrive_expect_tx(&bars[B_KFULL + st], OP_BYTES + (FP4 ? 1024 : 0));
-          tma_load_4d(sK + st * TILE_BYTES, &tm_k, &bars[B_KFULL + st], 0, hkv, t.k0 + tj * 128, t.bat);
+          tma_load_4d(sK + st * TILE_BYTES, &tm_k, &bars[B_KFULL + st], 0, hkv, t.k0 + j * 128, t.bat);
           if (FP4)
             bulk_load(sSF + SF_K + st * 1024,
-                      p.sfk4 + (((size_t)t.bat * p.h_kv + hkv) * (p.s_k / 128) + t.k0 / 128 + tj) * 1024, 1024,
+                      p.sfk4 + (((size_t)t.bat * p.h_kv + hkv) * (p.s_k / 128) + t.k0 / 128 + j) * 1024, 1024,
                       &bars[B_KFULL + st]);
           if (gj >= KV_STAGES && !(ok = mbar_wait(&bars[B_VEMPTY + st], ph ^ 1, p.ctl, abortp, 11))) break;
-          if (SPLIT && j < t.seed) {       // no P.V
-            mbar_arrive(&bars[B_VFULL + st]);
-            continue;
-          }
           mbar_arrive_expect_tx(&bars[B_VFULL + st], TILE_BYTES);
           tma_load_4d(sV + st * TILE_BYTES, &tm_v, &bars[B_VFULL + st], 0, hkv, t.k0 + j * 128, t.bat);
         }
@@ -356,11 +302,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     bool first_s = true;                   // FP4: the very first key tile of the CTA parks its scale columns in O1
     bool ok = true;
     for (int k = 0; ok; ++k) {
-      const int L = item_of(k);
+      const int L = fwd_item(k, G, cta, p.zigzag);
       if (L >= n_items) break;
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[B_Q + kb], (k >> 1) & 1, p.ctl, abortp, 20))) break;
-      const int n0 = tile_s[kb].n[0], n1 = tile_s[kb].n[1], seed = SPLIT ? tile_s[kb].seed : 0;
+      const int n0 = tile_s[kb].n[0], n1 = tile_s[kb].n[1];
       mbar_arrive_warp(&bars[B_QE + kb]);
       const int nmax = max(n0, n1);
       // issue_s(i, st): S of stage i against the K tile in ring slot st
@@ -444,10 +390,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           tc_fence_after();
           // P.V(j) completes before S(j + 1) does (issue order), which the softmax threads wait for anyway: a
           // separate completion signal is needed only after the stage's last tile (each commit costs the issuer ~60 clocks)
-          if (!(SPLIT && j < seed) && elect_one()) {
-            issue_pv(i, st, j > seed, (ci - 1) & 1);
-            if (j + 1 == n_i) tc_commit(&bars[B_PVDONE + i]);
-          }
+          if (elect_one()) { issue_pv(i, st, j > 0, (ci - 1) & 1); if (j + 1 == n_i) tc_commit(&bars[B_PVDONE + i]); }
           __syncwarp();
           if (j + 1 < n_i) {
             if (!k_next_ready) {
@@ -493,12 +436,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     int epi = 0, gfn = 0;                             // uses of the epilogue barrier / group-frame scale atoms so far
     bool ok = true;
     for (int k = 0; ok; ++k) {
-      const int L = item_of(k);
+      const int L = fwd_item(k, G, cta, p.zigzag);
       if (L >= n_items) break;
       const int kb = k & 1;
       if (!(ok = mbar_wait(&bars[B_Q + kb], (k >> 1) & 1, p.ctl, abortp, 36))) break;
       const Tile& T = tile_s[kb];                       // (valid until this item's Q buffer is released)
-      const int n_i = T.n[i], seed = SPLIT ? T.seed : 0;
+      const int n_i = T.n[i];
       const size_t bh_k = (size_t)T.bat * p.h_kv + T.hkv;
       float fq;
       int col_limit, col_first;                         // last and first visible key of this row, counted from the item's first key
@@ -519,27 +462,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       constexpr float P_OFF = GF ? P_LOG2_448 : P_LOG2_OFFSET;
 
       float m_used = -INFINITY, l_sum = 0.f;
-      if (SPLIT && seed && n_i > 0) {                   // the maximum of the item's first key tile (fwd_cut; rows that see a later key see all of it)
-        if (!(ok = mbar_wait(&bars[B_SFULL + i], cs & 1, p.ctl, abortp, 30 + i))) break;
-        tc_fence_after();
-#pragma unroll 1
-        for (int kbk = 0; kbk < 4; ++kbk) {
-          uint32_t v[32];
-          FL_TMEM_LD_32(t_s + 32 * kbk, v);
-          const float ck = FP4 ? fq : fq * fk_row[kbk - 4 * T.back];
-          tc_wait_ld();
-          float m = -INFINITY;
-#pragma unroll
-          for (int e = 0; e < 32; e += 2) m = fmax3(m, __uint_as_float(v[e]), __uint_as_float(v[e + 1]));
-          m_used = fmaxf(m_used, SC ? p.cap_a * tanh_fast(m * (ck * p.cap_b)) : m * ck);
-        }
-        tc_fence_before();
-        if (FP4) mbar_arrive_warp(&bars[B_SDRAIN + i]);
-        mbar_arrive_warp(&bars[B_PFULL + i]);           // (there is no P-hat: the scores have been read)
-        ++cs;
-        ++gfn;
-      }
-      for (int j = seed; j < n_i; ++j, ++cs) {
+      for (int j = 0; j < n_i; ++j, ++cs) {
         float c[4];
         uint32_t sfv = 0;
 #pragma unroll
@@ -603,7 +526,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 #pragma unroll
           for (int kbk = 0; kbk < 4; ++kbk) c[kbk] = 1.f;
         }
-        const int kb0 = j * 128;                               // key of column 0, as the limits
+        const int kb0 = j * 128;                                // key of column 0, as the limits
         const bool need_mask = (kb0 + 127 > col_limit) || (kb0 < col_first);    // only on boundary tiles
         if (need_mask) {   // scale first, then mask: the factor product may underflow to zero and 0 * inf is NaN
           // a bit per column (the code stands in the loop whether it runs or not, and bits take half the instructions)
@@ -639,7 +562,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
           alpha = ex2(m_used - mx);     // 0 on the first tile (m_used = -inf)
           m_used = mx;
         }
-        if (j > seed && __any_sync(0xFFFFFFFFu, refresh)) {
+        if (j > 0 && __any_sync(0xFFFFFFFFu, refresh)) {
           // rescale this row of O in tensor memory once the previous P.V has finished
           // P.V(j - 1) has completed: S(j), which this thread has read, was issued after it
 #pragma unroll 1
@@ -741,39 +664,16 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         tc_wait_st();
         tc_fence_before();
         mbar_arrive_warp(&bars[B_PFULL + i]);
-        if (!SPLIT) confirm();           // (in the loop it costs the split kernel 2 %, whose CTAs have few items)
+        confirm();
       }
       if (!ok) break;
-      confirm();                         // (an item without tiles; split schedules)
+      confirm();                         // (an item without tiles)
       // ---- item epilogue: O / l -> bf16 rows through this stage's Q tile buffer, LSE
       if (n_i > 0) {
         if (!(ok = mbar_wait(&bars[B_PVDONE + i], cd & 1, p.ctl, abortp, 34 + i))) break;
         ++cd;
       }
       tc_fence_after();
-      if constexpr (SPLIT) {
-        if (T.part >= 0) {               // a piece: O as it stands, in 32 bits, with the row's maximum and sum, for fwd_merge_kernel
-          float* const stat = p.part + (size_t)T.part * fwd_part_floats<D>() + 128 * i + r;
-          float4* const rows = reinterpret_cast<float4*>(stat - (128 * i + r) + 512) + 128 * i + r;
-          stat[0] = m_used;
-          stat[256] = l_sum;
-          if (n_i > 0) {                 // (a stage without keys has a sum of zero and no rows)
-#pragma unroll 1
-            for (int cc = 0; cc < D / 32; ++cc) {
-              uint32_t ov[32];
-              FL_TMEM_LD_32(t_o + 32 * cc, ov);
-              tc_wait_ld();
-#pragma unroll
-              for (int q4 = 0; q4 < 8; ++q4)
-                rows[(8 * cc + q4) * 256] = make_float4(__uint_as_float(ov[4 * q4]), __uint_as_float(ov[4 * q4 + 1]),
-                                                        __uint_as_float(ov[4 * q4 + 2]), __uint_as_float(ov[4 * q4 + 3]));
-            }
-          }
-          tc_fence_before();
-          mbar_arrive_warp(&bars[B_QE + kb]);
-          continue;
-        }
-      }
       const int head = T.head, qrow = T.q0 + 128 * i + r;
       const bool row_valid = (128 * i + r) < T.nq;
       const bool stage_present = T.nq > 128 * i;        // (warpgroup-uniform) an absent stage's rows belong to someone else
@@ -856,70 +756,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
-// O and LSE of the items that a split schedule cut: the partial results of an item's pieces, each relative to its own running
-// maximum, weighed and added. Block (c, g): the item that the boundary between CTAs c and c + 1 cuts for the first time, rows 32 g ..
-// + 31; lane = row, warp = a quarter of the columns.
-template <int D>
-__global__ void __launch_bounds__(128) fwd_merge_kernel(const FwdParams p, const __grid_constant__ fl_split cuts, float p_off) {
-  const int c = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = blockIdx.y * 32 + lane;
-  grid_dependency();
-  const uint32_t at = cuts.at[c + 1], before = cuts.at[c];
-  const int L = cut_item(at);
-  if (!cut_tile(at) || (cut_item(before) == L && cut_tile(before))) return;
-  int last = c + 1;                      // the CTA with the item's last piece
-  while (last + 1 < cuts.parts && cut_item(cuts.at[last + 1]) == L && cut_tile(cuts.at[last + 1])) ++last;
-  Tile t;
-  fwd_decode<false>(p, L, t);
-  if (row >= t.nq) return;
-  auto piece = [&](int j) { return p.part + (size_t)(j == c ? 2 * c + 1 : 2 * j) * fwd_part_floats<D>(); };
-  float m = -INFINITY;
-  for (int j = c; j <= last; ++j) m = piece(j)[256 + row] == 0.f ? m : fmaxf(m, piece(j)[row]);
-  constexpr int N = D / 16;              // groups of four columns
-  float4 acc[N];
-#pragma unroll
-  for (int e = 0; e < N; ++e) acc[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-  float l = 0.f;
-  for (int j = c; j <= last; ++j) {
-    const float* s = piece(j);
-    const float lj = s[256 + row];
-    if (lj == 0.f) continue;             // no key of the piece is visible (a stage without keys wrote no rows)
-    const float w = ex2(s[row] - m);
-    l = fmaf(lj, w, l);
-    const float4* o = reinterpret_cast<const float4*>(s + 512) + warp * N * 256 + row;
-#pragma unroll
-    for (int e = 0; e < N; ++e) {
-      const float4 v = o[e * 256];
-      acc[e].x = fmaf(v.x, w, acc[e].x); acc[e].y = fmaf(v.y, w, acc[e].y);
-      acc[e].z = fmaf(v.z, w, acc[e].z); acc[e].w = fmaf(v.w, w, acc[e].w);
-    }
-  }
-  const float inv = l > 0.f ? 1.0f / l : 0.f;
-  const size_t qrow = (size_t)t.bat * p.q_len + t.q0 + row;
-  uint16_t* const out = reinterpret_cast<uint16_t*>(p.out) + (qrow * p.h + t.head) * p.d_out;
-#pragma unroll
-  for (int e = 0; e < N; e += 2) {
-    const int col = (warp * N + e) * 4;
-    if (col >= p.d_out) break;
-    const float v[8] = {acc[e].x, acc[e].y, acc[e].z, acc[e].w, acc[e + 1].x, acc[e + 1].y, acc[e + 1].z, acc[e + 1].w};
-    uint32_t w[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (p.out_f16) {
-        const __half2 hh = __floats2half2_rn(v[2 * i] * inv, v[2 * i + 1] * inv);
-        w[i] = *reinterpret_cast<const uint32_t*>(&hh);
-      } else {
-        w[i] = pack_bf16x2(v[2 * i] * inv, v[2 * i + 1] * inv);
-      }
-    }
-    *reinterpret_cast<uint4*>(out + col) = make_uint4(w[0], w[1], w[2], w[3]);
-  }
-  if (warp == 0 && p.lse) p.lse[((size_t)t.bat * p.h + t.head) * p.s_q + t.q0 + row] = l > 0.f ? (m - p_off + lg2(l)) * 0.6931471805599453f : -INFINITY;
-}
-
 }  // namespace fl
 
 static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, const uint32_t* tok_kv = nullptr,
-                      const uint16_t* tok_r16 = nullptr, const fl_split* split = nullptr, void* partials = nullptr) {
+                      const uint16_t* tok_r16 = nullptr) {
   using namespace fl;
   if (!a || !a->q_codes || !a->k_codes || !a->v_codes || !a->out || !a->status) return FL_ERR_BAD_ARG;
   if (!a->fac_q || !a->fac_k || !a->fac_v) return FL_ERR_BAD_ARG;
@@ -968,7 +808,13 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, con
   p.out_f16 = (a->flags & FL_A_OUT_F16) ? 1 : 0;
   p.ctl = dev_ctl(a->status, a->wait_cycles > 0 ? a->wait_cycles : kDefaultWaitCycles);
   // packed documents: at most one extra 256-row block per document beyond total / 256
-  const int nblk = work ? a->s_q / 128 : a->doc_start ? (a->s_q / 256 + a->n_docs + 1) : (q_len + 255) / 256;
+  // Blocks of 256 query rows keep both stages of a CTA busy. Where twice the items still have an SM each, blocks of 128: one stage alone takes
+  // about 0.8 of the two stages' time a tile, and a row is computed alike in either, to the last bit. One B200, quantisers and forward, us:
+  // 4608 x 18432 h4 228 / 187, 768 x 3072 h4 44 / 38, 8832 h2 mixed route 125 / 104, 640 x 10240 h1 d64 120 / 95, 256 h16/4 mixed
+  // route 14.4 / 13.6. (Pieces of an item's key tiles, merged by a second launch, take 127, 25, 55, 33 and 14.6 there, but sum in an order that
+  // the number of batch rows and heads decides: a request's output is the same bytes whatever else is in its call.)
+  p.blk_rows = !a->doc_start && 2ll * ((q_len + 255) / 256) * a->h * a->b <= sm_count() ? 128 : 256;
+  const int nblk = work ? a->s_q / 128 : a->doc_start ? (a->s_q / 256 + a->n_docs + 1) : (q_len + p.blk_rows - 1) / p.blk_rows;
   const int nb = a->doc_start ? 1 : a->b;
   p.n_blk = nblk;
   const long long n_items = (long long)nblk * a->h * nb;
@@ -980,21 +826,12 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, con
   p.div_item = FastDiv(a->doc_start ? 1 : p.causal ? a->h * a->b : nblk);
   p.div_h = FastDiv(a->h);
   p.div_grp = FastDiv(a->h / a->h_kv);
-  p.part = (float*)partials;
-  if (split) {
-    p.out = a->out;
-    if (!partials || a->doc_start || a->o_mult || tl || p.win_l >= 0) return FL_ERR_UNSUPPORTED;
-    if (split->parts < 2 || split->parts > FL_SPLIT_MAX || split->at[0] != 0) return FL_ERR_BAD_ARG;
-    for (int c = 0; c < split->parts; ++c)
-      if (split->at[c + 1] < split->at[c]) return FL_ERR_BAD_ARG;
-    if (split->at[split->parts] != (uint32_t)p.n_items << FL_SPLIT_TILE_BITS) return FL_ERR_BAD_ARG;
-  }
-  const int grid = split ? split->parts : (int)(n_items < sm_count() ? n_items : sm_count());     // one persistent CTA per SM
+  const int grid = (int)(n_items < sm_count() ? n_items : sm_count());     // one persistent CTA per SM
   const int smem = (a->d == 128 ? 6 : 4) * Q_STRIDE + 2 * KV_STAGES * 128 * a->d + 1024 + (fp4 ? 4096 + KV_STAGES * 1024 : 0);
   cudaStream_t st = (cudaStream_t)stream;
-  auto launch = [&](auto kern, auto cuts) -> int {
+  auto launch = [&](auto kern) -> int {
     if (int e = set_smem(kern, smem, "fl_fwd: cudaFuncSetAttribute")) return e;
-    launch_after(kern, grid, 384, smem, st, mq, mk, mv, mo, p, cuts);
+    launch_after(kern, grid, 384, smem, st, mq, mk, mv, mo, p);
     return FL_OK;
   };
   const bool sc = a->softcap > 0.f;
@@ -1003,10 +840,8 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, con
   p.cap_b = sc ? 1.0f / p.cap_a : 0.f;
   // the lean kernels serve the plain calls; documents, packed outputs and the output-row factor take the full variant
   const bool full = a->doc_start != nullptr || a->o_mult != nullptr;
-#define FL_FWD_LAUNCH(D_, FP4_, TL_, GF_, SC_)                                                                          \
-  (split  ? launch(fwd_kernel<D_, FP4_, 0, GF_, SC_, false, true>, Cuts<true>{*split})   \
-   : full ? launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, true>, Cuts<false>{})                                         \
-          : launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, false>, Cuts<false>{}))
+#define FL_FWD_LAUNCH(D_, FP4_, TL_, GF_, SC_) \
+  (full ? launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, true>) : launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, false>))
   if (sc) {
     if (fp4) rc = gf ? FL_FWD_LAUNCH(128, true, 0, true, true) : FL_FWD_LAUNCH(128, true, 0, false, true);
     else if (a->d == 128) rc = gf ? FL_FWD_LAUNCH(128, false, 0, true, true) : FL_FWD_LAUNCH(128, false, 0, false, true);
@@ -1022,12 +857,6 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, con
   }
 #undef FL_FWD_LAUNCH
   if (rc) return rc;
-  if (split) {
-    const dim3 g(split->parts - 1, 8);
-    const float p_off = gf ? P_LOG2_448 : P_LOG2_OFFSET;
-    if (a->d == 128) launch_after(fwd_merge_kernel<128>, g, 128, 0, st, p, *split, p_off);
-    else launch_after(fwd_merge_kernel<64>, g, 128, 0, st, p, *split, p_off);
-  }
   return launch_result("fl_fwd: kernel launch");
 }
 
@@ -1042,35 +871,4 @@ extern "C" int fl_fwd_tokens(const fl_attn_args* a, const uint32_t* kv, const ui
   if (!a || !kv || !rcp || !(a->flags & FL_A_TOKEN_LOCAL)) return FL_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(kv) | reinterpret_cast<uintptr_t>(rcp)) & 15) return FL_ERR_BAD_ARG;     // read 16 bytes at a time
   return fwd_launch(a, nullptr, stream, kv, rcp);
-}
-
-extern "C" int fl_fwd_split(const fl_attn_args* a, const fl_split* split, void* partials, void* stream) {
-  using namespace fl;
-  if (!a || !split || !partials || (reinterpret_cast<uintptr_t>(partials) & 15)) return FL_ERR_BAD_ARG;
-  return fwd_launch(a, nullptr, stream, nullptr, nullptr, split, partials);
-}
-
-extern "C" int fl_fwd_split_plan(const fl_attn_args* a, int32_t ctas, fl_split* split) {
-  using namespace fl;
-  if (!a || !split || ctas < 0) return FL_ERR_BAD_ARG;
-  split->parts = 0;
-  if (a->doc_start || a->o_mult || a->b <= 0 || a->s_q <= 0 || a->s_k <= 0 || a->h <= 0) return FL_OK;
-  // (under a left window the first key tile of a row is not that of its item; with token factors and outlier channels, where the running
-  // maximum is refreshed again and again, pieces would frame some rows otherwise than whole items: 2.5e-2 on gradients)
-  if (a->window_left_p1 > 0 || (a->flags & FL_A_TOKEN_LOCAL)) return FL_OK;
-  const int s_q = a->out_rows > 0 ? a->out_rows : a->s_q, s_k = a->out_rows > 0 ? a->out_rows : a->s_k;
-  const int n_blk = (s_q + 255) / 256, off = s_k - s_q;
-  const bool causal = a->flags & FL_A_CAUSAL;
-  const int win_r = causal ? 0 : window_side(a->window_right_p1);
-  auto tiles = [&](int blk) {            // as fwd_decode
-    const int q0 = blk * 256, nq = std::min(256, s_q - q0);
-    const int to = win_r >= 0 ? std::min<int64_t>(s_k, (int64_t)q0 + nq + off + win_r) : s_k;
-    return to > 0 ? (to + 127) / 128 : 0;
-  };
-  std::vector<int> n(n_blk);
-  for (int i = 0; i < n_blk; ++i) n[i] = tiles(causal ? n_blk - 1 - i : i);
-  // What an item costs beside its tiles, and the merge, in key tiles of 256 query rows (1.45 us). One B200, whole items / pieces and merge, us:
-  // 4608 x 18432 h4 210 / 112; 3072 x 6144 h5 75 / 41; 768 x 3072 h4 41 / 21; 8832 h2 mixed route 112 / 48; 1792 h5 26 / 19; 6784 h2 d64
-  // 76 / 31; and 512 x 8192 b4 h32/8 194 / 193, 2048 h16 29 / 30, which are not worth it.
-  return plan_split(n.data(), n_blk, a->h * (long long)a->b, causal, ctas ? ctas : sm_count(), 1.2f, 0.4f, 3.2f, 0.01f, split);
 }

@@ -30,7 +30,6 @@
 #include <cstring>
 #include <deque>
 #include <map>
-#include <memory>
 #include <mutex>
 #include <sstream>
 #include <tuple>
@@ -55,13 +54,6 @@ struct Plan {
   double softcap, softmax_scale;
   int64_t b, s_q, s_k, h, h_kv, d, tot_q;
   int64_t d_call;            // the call's own head dim: d, or less where the kernels run it with zero columns up to d
-  // batched calls without gradients: the forward's split schedule, made at the plan's first call. (With gradients O, dK and dV of a (batch
-  // row, head) are the same bytes in whatever call it stands, so that training can be sharded over both; pieces are sums in another order.)
-  struct Schedule {
-    std::once_flag once;
-    fl_split s;
-  };
-  std::shared_ptr<Schedule> sched = std::make_shared<Schedule>();
 };
 struct Entry {
   int64_t plan, capacity;    // capacity < 0: the batched form
@@ -470,13 +462,8 @@ State forward(int64_t handle, const Tensor& q_, const Tensor& k_, const Tensor& 
     check(fl_token_tables(ptr<float>(kq.token_factors), ptr<float>(vq.token_factors), n, ptr<uint32_t>(tok), ptr<uint16_t>(tok) + 2 * n, st),
           "fl_token_tables");
   }
-  const bool may_split = !has_docs && !p.need_bwd;
-  if (may_split) std::call_once(p.sched->once, [&] { check(fl_fwd_split_plan(&a, 0, &p.sched->s), "fl_fwd_split_plan"); });
   if (has_docs) {
     check(fl_fwd_work(&a, ptr<int32_t>(docs.work), st), "fl_fwd_work");
-  } else if (may_split && p.sched->s.parts) {
-    const Tensor partials = empty({FL_FWD_SPLIT_BYTES(p.sched->s.parts, p.d)}, at::kByte, dev);
-    check(fl_fwd_split(&a, &p.sched->s, ptr<void>(partials), st), "fl_fwd_split");
   } else if (p.token_local) {
     check(fl_fwd_tokens(&a, ptr<uint32_t>(tok), ptr<uint16_t>(tok) + 2 * vq.token_factors.numel(), st), "fl_fwd_tokens");
   } else {

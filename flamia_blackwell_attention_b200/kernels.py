@@ -189,13 +189,12 @@ def attn_args(q, k, v, *, causal, softmax_scale, mode=L.FL_MODE_FP8, flags=0, st
 
 def attn_fwd(q, k, v, *, causal, softmax_scale, out_dtype=torch.bfloat16, mode=L.FL_MODE_FP8, status=None,
              doc_start=None, doc_len=None, wait_cycles=0, token_local=False, window=None, p_group=False, seqused_k=None,
-             softcap=0.0, o_mult=None, packed_out=None, work=None, split=None):
+             softcap=0.0, o_mult=None, packed_out=None, work=None):
     """Forward kernel on quantised operands. Returns (out (b, s_q, h, d), lse (b, h, s_q) float32, status).
     p_group: group-frame P-hat (one UE8M0 exponent per query row and 32 keys) instead of the row frame.
     o_mult: (b, h_kv) f32 factor on the output rows (the mantissa of a V factor that is no power of two).
     packed_out = (slot_src, slot_rows, total): documents; out is (1, total, h, d) with the documents stored back to back
-    (the kernel writes the caller's packed rows itself); lse keeps the aligned buffer's rows. work: the documents' work lists (doc_work).
-    split: a schedule (_lib.Split) that deals out the items' key tiles instead of whole items."""
+    (the kernel writes the caller's packed rows itself); lse keeps the aligned buffer's rows. work: the documents' work lists (doc_work)."""
     qc = q["codes"]
     b, s_q, h, d = qc.shape
     dev = qc.device
@@ -221,10 +220,6 @@ def attn_fwd(q, k, v, *, causal, softmax_scale, out_dtype=torch.bfloat16, mode=L
     if token_local:     # log2 f_V and 1 / f_V per key, which the forward applies to every score
         lg, rcp = token_aux(v["token_factors"])
         a.tok_lg_v, a.tok_rcp_v = L.ptr(lg), L.ptr(rcp)
-    if split is not None:
-        part = torch.empty(2 * split.parts * (512 + 256 * d), dtype=torch.float32, device=dev)
-        L.check(L.load().fl_fwd_split(C.byref(a), C.byref(split), L.ptr(part), _stream()), "fl_fwd_split")
-        return out, lse, status
     L.check(L.load().fl_fwd(C.byref(a), _stream()) if work is None else L.load().fl_fwd_work(C.byref(a), L.ptr(work), _stream()), "fl_fwd")
     return out, lse, status
 

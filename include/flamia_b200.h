@@ -183,24 +183,6 @@ typedef struct fl_attn_args {
  * FlashAttentionForwardSm100. */
 int fl_fwd(const fl_attn_args* args, void* stream);
 
-/* Split schedules. The forward deals out whole items (256 query rows of a head) to one CTA per SM; where that leaves much of the chip
- * waiting (few items, or a last round that is nearly empty) it can deal out equal shares of the items' key tiles instead: CTA c
- * works from position at[c] up to at[c + 1], a position being item << FL_SPLIT_TILE_BITS | key tile of it. Pieces of an item leave their
- * unnormalised rows with maxima and sums in `partials`, and a second launch merges them (the counterpart of the reference's num_splits
- * and its combine kernel, flash_attn/cute/interface_fwd_fp4.py:301).
- * fl_fwd_split_plan (host arithmetic on sizes and masks; reads no device memory): the schedule on at most `ctas` CTAs (0 = the
- * current device's SMs) that is expected to be faster than whole items, or parts = 0. fl_fwd_split: fl_fwd on that schedule; batched form without a left
- * window, o_mult and token factors. partials: FL_FWD_SPLIT_BYTES bytes, 16-byte aligned. */
-#define FL_SPLIT_MAX 160
-#define FL_SPLIT_TILE_BITS 12
-typedef struct fl_split {
-  int32_t parts;                     /* CTAs of the schedule */
-  uint32_t at[FL_SPLIT_MAX + 1];
-} fl_split;
-#define FL_FWD_SPLIT_BYTES(parts, d) ((int64_t)2 * (parts) * (512 + 256 * (d)) * 4)
-int fl_fwd_split_plan(const fl_attn_args* args, int32_t ctas, fl_split* split);
-int fl_fwd_split(const fl_attn_args* args, const fl_split* split, void* partials, void* stream);
-
 /* Backward main kernel: dK, dV and the pre-scaled f16 dQ accumulator.
  * Replaces flash_attn/cute/interface_bwd_fp4.py:1207 _flash_attn_bwd_fp4 -> flash_bwd_sm100_fp4.py:82
  * FlashAttentionBackwardSm100FP4 (and the 2-CTA variant flash_bwd_sm100_2cta8.py:74). */

@@ -10,7 +10,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("b,sq,sk,h,hk,d,kw", [
     (1, 128, 128, 1, 1, 128, dict(causal=True)),
     (2, 640, 640, 2, 1, 128, dict(causal=True)),                 # the last block without a second stage
-    (1, 384, 512, 3, 1, 128, dict()),
+    (1, 384, 1152, 3, 1, 128, dict()),
+    (1, 128, 8192, 1, 1, 128, dict(causal=True)),                # few items of many key tiles
+    (1, 2049, 2049, 2, 1, 96, dict(causal=True)),
     (1, 896, 896, 2, 2, 64, dict(causal=True)),
     (2, 512, 512, 2, 1, 64, dict()),
     (2, 1000, 1000, 2, 1, 64, dict()),                           # rows that are no whole tiles
