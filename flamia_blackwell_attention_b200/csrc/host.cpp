@@ -484,8 +484,8 @@ State forward(int64_t handle, const Tensor& q_, const Tensor& k_, const Tensor& 
     } else {
       lse_user = empty({0}, at::kFloat, dev);
     }
-  } else if (p.ragged) {                      // (the kernels' LSE has whole tiles of rows)
-    lse_user = p.return_lse ? lse.narrow(2, 0, p.s_q).contiguous() : empty({0}, at::kFloat, dev);
+  } else if (p.ragged) {                      // the kernels' LSE has whole tiles of rows: a copy (of one row and head, too, whose rows are contiguous)
+    lse_user = p.return_lse ? lse.narrow(2, 0, p.s_q).clone(at::MemoryFormat::Contiguous) : empty({0}, at::kFloat, dev);
   }
   check_status_if_asked(dev);
   return S;

@@ -40,3 +40,19 @@ def test_batch_rows_equal_documents(b, s, h, hk, d, dtype, kw):
         assert torch.equal(got, want.view(got.shape))
     assert float((dq.float() - pdq.view(dq.shape).float()).norm()) <= 8e-3 * float(pdq.float().norm())
     assert F.check_status() == 0
+
+
+@pytest.mark.parametrize("b,h,s", [(1, 1, 200), (1, 1, 1), (1, 2, 200), (2, 1, 130)])
+def test_returned_lse_is_the_callers_own(b, h, s):
+    """What a caller writes into the returned LSE reaches no gradient, and the tensor holds no more memory than its rows."""
+    import flamia_blackwell_attention_b200 as F
+    q, k, v, g = (t.cuda() for t in attention_inputs(b, s, h, h, 64, seed=22))
+    for t in (q, k, v):
+        t.requires_grad_(True)
+    out, lse = F.flash_attn_fp8(q, k, v, causal=True, return_lse=True)
+    assert lse.shape == (b, h, s) and lse.untyped_storage().nbytes() == 4 * b * h * s
+    want = torch.autograd.grad(out, (q, k, v), g, retain_graph=True)
+    lse.fill_(7.0)
+    got = torch.autograd.grad(out, (q, k, v), g)
+    assert all(torch.equal(x, y) for x, y in zip(got[1:], want[1:]))
+    assert float((got[0].float() - want[0].float()).norm()) <= 8e-3 * float(want[0].float().norm())     # (the order of dQ's f16 sums)
