@@ -937,7 +937,7 @@ static int check_quant_args(const fl_quant_args* a) {
   if ((a->flags & FL_Q_HADAMARD) && (a->flags & FL_Q_TOKEN_LOCAL)) return FL_ERR_UNSUPPORTED;
   if ((a->flags & FL_Q_D_PER_FACTOR) && !(a->flags & FL_Q_TOKEN_LOCAL)) return FL_ERR_BAD_ARG;
   if ((a->flags & FL_Q_HADAMARD_NVFP4_ONLY) && !a->x4) return FL_ERR_BAD_ARG;
-  if (a->h > 65535 || a->b > 65535) return FL_ERR_TOO_LARGE;
+  if (a->h > 65535) return FL_ERR_TOO_LARGE;
   if ((long long)a->b * (a->s / 128) * a->h > 0x7FFFFFFF) return FL_ERR_TOO_LARGE;
   if (a->row_stat && (a->row_stat_kind < 1 || a->row_stat_kind > 3)) return FL_ERR_BAD_ARG;
   if (a->slot_src && (!a->slot_rows || a->b != 1 || a->src_rows <= 0)) return FL_ERR_BAD_ARG;

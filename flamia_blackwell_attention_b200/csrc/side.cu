@@ -2,7 +2,12 @@
 #include "doc_work.cuh"
 #include "flamia_internal.h"
 
+#include <algorithm>
+
 namespace fl {
+
+// blocks in y and z of a grid: calls of more batch rows are several launches
+static constexpr int GRID_YZ = 65535;
 
 // ------------------------------------------------------------------------------------------------ dQ pre-scale
 // Restates flash_attn/cute/device_scales.py:124-132 (_dq_bound_pow2) and :158-184, 234-319 (_dq_row_bound,
@@ -369,8 +374,11 @@ extern "C" int fl_dq_prescale(const float* stats_do, const float* stats_v, const
   if (!stats_do || !stats_v || !stats_k || !kernel_scale || !post_scale || b <= 0 || nt_q <= 0 || nt_k <= 0)
     return FL_ERR_BAD_ARG;
   const int threads = causal_local ? 128 : 1024;
-  launch_after(dq_prescale_kernel, dim3(causal_local ? nt_q : 1, b), threads, 0, (cudaStream_t)stream, stats_do, stats_v, stats_k, h, h_kv, nt_q, nt_k,
-                                                                      causal_local, unit, kernel_scale, post_scale);
+  for (int b0 = 0; b0 < b; b0 += GRID_YZ) {
+    const size_t q0 = (size_t)b0 * nt_q, k0 = (size_t)b0 * h_kv * nt_k * 2;
+    launch_after(dq_prescale_kernel, dim3(causal_local ? nt_q : 1, std::min(b - b0, GRID_YZ)), threads, 0, (cudaStream_t)stream,
+                 stats_do + q0 * h * 2, stats_v + k0, stats_k + k0, h, h_kv, nt_q, nt_k, causal_local, unit, kernel_scale + q0, post_scale + q0);
+  }
   return launch_result("fl_dq_prescale: kernel launch");
 }
 
@@ -382,11 +390,19 @@ static int dq_post_launch(const void* dq_acc, const float* post_scale, float mul
   using namespace fl;
   if (!dq_acc || !post_scale || !dq || b <= 0 || s <= 0 || (s % 128) || h <= 0) return FL_ERR_BAD_ARG;
   if ((d != 64 && d != 128) || (unrotate && d != 128)) return FL_ERR_UNSUPPORTED;
-  if (h > 65535 || b > 65535) return FL_ERR_TOO_LARGE;
+  if (h > 65535) return FL_ERR_TOO_LARGE;
   if (d_out == 0) d_out = d;
   if (d_out < 0 || d_out > d || d_out % 8) return FL_ERR_BAD_ARG;
   if (rows == 0) rows = s;
   if (rows < 0 || rows > s || rows <= s - 128) return FL_ERR_BAD_ARG;
+  if (b > GRID_YZ) {
+    for (int b0 = 0; b0 < b; b0 += GRID_YZ)
+      if (int rc = dq_post_launch((const __half*)dq_acc + (size_t)b0 * h * s * d, post_scale + (size_t)b0 * (per_row ? s : s / 128), mult,
+                                  (uint16_t*)dq + (size_t)b0 * rows * h * d_out, std::min(b - b0, GRID_YZ), s, h, d, unrotate, out_f16, per_row,
+                                  head_mult ? head_mult + (size_t)b0 * h : nullptr, stream, slot_src, slot_rows, d_out, rows))
+        return rc;
+    return FL_OK;
+  }
   dim3 grid(s / 128, h, b);
   cudaStream_t st = (cudaStream_t)stream;
   if (d == 128) {

@@ -56,3 +56,21 @@ def test_returned_lse_is_the_callers_own(b, h, s):
     got = torch.autograd.grad(out, (q, k, v), g)
     assert all(torch.equal(x, y) for x, y in zip(got[1:], want[1:]))
     assert float((got[0].float() - want[0].float()).norm()) <= 8e-3 * float(want[0].float().norm())     # (the order of dQ's f16 sums)
+
+
+@pytest.mark.parametrize("s,d", [(8, 64), (3, 128)])
+def test_more_batch_rows_than_a_grid_has_in_y_and_z(s, d):
+    """65540 batch rows of two kinds: every row has the bytes of its kind in a call of two rows (dQ to the order of its f16 sums, of which a
+    row of up to 128 keys has one)."""
+    import flamia_blackwell_attention_b200 as F
+    b = 65540
+    two = [t.cuda() for t in attention_inputs(2, s, 1, 1, d, seed=23)]
+
+    def step(x):
+        q, k, v = (t.requires_grad_(True) for t in x[:3])
+        out = F.flash_attn_fp8(q, k, v, causal=True)
+        return out.detach(), *torch.autograd.grad(out, (q, k, v), x[3])
+    many = step([t.repeat(b // 2, 1, 1, 1) for t in two])
+    assert F.check_status() == 0
+    for got, want in zip(many, step(two)):
+        assert torch.equal(got.view(b // 2, 2, s, 1, d), want.view(1, 2, s, 1, d).expand(b // 2, -1, -1, -1, -1))
