@@ -19,10 +19,10 @@ FL_DEV_WAIT_TIMEOUT = 0x100
 FL_DEV_BAD_TABLE = 0x200
 ERR_NAMES = {1: "bad argument", 2: "CUDA error", 3: "unsupported configuration", 4: "size beyond the supported maximum"}
 
-FL_Q_HADAMARD, FL_Q_TOKEN_LOCAL, FL_Q_HADAMARD_NVFP4_ONLY, FL_Q_O_PACKED, FL_Q_LEGACY, FL_Q_D_PER_FACTOR = 1, 2, 4, 8, 16, 32
+FL_Q_HADAMARD, FL_Q_TOKEN_LOCAL, FL_Q_HADAMARD_NVFP4_ONLY, FL_Q_O_PACKED, FL_Q_LEGACY, FL_Q_D_PER_FACTOR, FL_Q_ROWS = 1, 2, 4, 8, 16, 32, 64
 FL_MODE_FP8, FL_MODE_FP4 = 0, 1
-FL_A_CAUSAL, FL_A_OUT_F16, FL_A_TOKEN_LOCAL, FL_A_DQ_ROWLOCAL, FL_A_HAD_DQ, FL_A_HAD_DK, FL_A_P_GROUP, FL_A_D_PER_FACTOR = \
-    1, 2, 4, 8, 16, 32, 64, 256
+FL_A_CAUSAL, FL_A_OUT_F16, FL_A_TOKEN_LOCAL, FL_A_DQ_ROWLOCAL, FL_A_HAD_DQ, FL_A_HAD_DK, FL_A_P_GROUP, FL_A_D_PER_FACTOR, FL_A_ROWS = \
+    1, 2, 4, 8, 16, 32, 64, 256, 512
 
 vp, i32, i64, f32 = C.c_void_p, C.c_int32, C.c_int64, C.c_float
 

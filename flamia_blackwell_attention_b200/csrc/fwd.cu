@@ -777,8 +777,8 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, con
   if (a->doc_start && (a->b != 1 || a->n_docs <= 0 || !a->doc_len || a->s_q != a->s_k)) return FL_ERR_BAD_ARG;
   if (a->seqused_k && a->doc_start) return FL_ERR_UNSUPPORTED;      // documents carry their own lengths
   // batch rows of fewer rows than the whole tiles of the intermediates
-  const bool trim = a->out_rows > 0 && !a->doc_start;
-  if (trim && (a->s_q != a->s_k || a->out_rows > a->s_q || a->out_rows <= a->s_q - 128)) return FL_ERR_BAD_ARG;
+  const bool trim = (a->flags & FL_A_ROWS) && !a->doc_start;
+  if (trim && (a->s_q != a->s_k || a->out_rows <= 0 || a->out_rows > a->s_q || a->out_rows <= a->s_q - 128)) return FL_ERR_BAD_ARG;
   const int q_len = trim ? a->out_rows : a->s_q;
   CUtensorMap mq, mk, mv, mo;
   int rc;

@@ -309,7 +309,7 @@ void quantise_args(Quantised& o, const Plan& p, const Tensor& x, int64_t b, int6
     a.slot_src = ptr<int32_t>(docs->slot_src); a.slot_rows = ptr<int32_t>(docs->slot_rows);
     a.src_rows = (int32_t)(x.numel() / (heads * p.d_call));
   } else if (p.ragged) {
-    a.src_rows = (int32_t)p.s_q;
+    a.flags |= FL_Q_ROWS; a.src_rows = (int32_t)p.s_q;
   }
   if (row_stat.defined()) { a.row_stat = ptr<float>(row_stat); a.row_stat_kind = row_stat_kind; }
   a.status = status;
@@ -324,7 +324,7 @@ void attn_common(fl_attn_args& a, const Plan& p, const Shapes& sh, bool f16) {
             (p.d_call != p.d ? FL_A_COLS(p.d_call) : 0);
   a.window_left_p1 = p.window_left_p1; a.window_right_p1 = p.window_right_p1;
   a.softcap = (float)p.softcap;
-  if (p.ragged) a.out_rows = (int32_t)p.s_q;
+  if (p.ragged) { a.flags |= FL_A_ROWS; a.out_rows = (int32_t)p.s_q; }
 }
 
 // One call's tensors: the results in the caller's layout and what the backward needs.
@@ -569,7 +569,7 @@ std::tuple<Tensor, Tensor, Tensor> backward(int64_t handle, int64_t capacity, bo
     g.slot_src = slot_src; g.slot_rows = slot_rows; g.src_rows = (int32_t)total;
     g.flags |= FL_Q_O_PACKED;                  // the forward output has the packed rows
   } else if (p.ragged) {
-    g.src_rows = (int32_t)p.s_q;
+    g.flags |= FL_Q_ROWS; g.src_rows = (int32_t)p.s_q;
   }
   check(fl_quant_blocks(&g, st), "fl_quant_blocks");
 

@@ -41,6 +41,7 @@ extern "C" int fl_bwd_static_acc(const fl_attn_args* args, const float* post_sca
   using namespace fl;
   if (!args || !post_scale || !dq) return FL_ERR_BAD_ARG;
   if (args->b <= 0 || args->h <= 0 || args->s_q <= 0 || args->d <= 0) return FL_ERR_BAD_ARG;
+  if (args->flags & FL_A_ROWS) return FL_ERR_UNSUPPORTED;      // (dq has s_q rows)
   // each factor is checked against the limit first, so the product below cannot overflow
   const long long lim = (long long)FL_STATIC_ACC_MAX_ELEMS;
   if (args->b > lim || args->h > lim || args->s_q > lim || args->d > lim) return FL_ERR_TOO_LARGE;

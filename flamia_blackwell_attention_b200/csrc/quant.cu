@@ -926,7 +926,7 @@ static int prologue_steps(long long n_tiles, bool want_t) {
 static int quant_cols(const fl_quant_args* a) { return (a->flags >> 16) > 0 ? (a->flags >> 16) : a->d; }
 
 // rows of a batch row of x (the outputs have a->s): the tensor maps read the missing ones as zeros
-static int quant_src_rows(const fl_quant_args* a) { return a->src_rows > 0 ? a->src_rows : a->s; }
+static int quant_src_rows(const fl_quant_args* a) { return a->slot_src || (a->flags & FL_Q_ROWS) ? a->src_rows : a->s; }
 
 static int check_quant_args(const fl_quant_args* a) {
   if (!a || !a->x || !a->codes) return FL_ERR_BAD_ARG;
@@ -941,7 +941,7 @@ static int check_quant_args(const fl_quant_args* a) {
   if ((long long)a->b * (a->s / 128) * a->h > 0x7FFFFFFF) return FL_ERR_TOO_LARGE;
   if (a->row_stat && (a->row_stat_kind < 1 || a->row_stat_kind > 3)) return FL_ERR_BAD_ARG;
   if (a->slot_src && (!a->slot_rows || a->b != 1 || a->src_rows <= 0)) return FL_ERR_BAD_ARG;
-  if (!a->slot_src && a->src_rows != 0 && (a->src_rows > a->s || a->src_rows <= a->s - 128)) return FL_ERR_BAD_ARG;
+  if (!a->slot_src && (a->flags & FL_Q_ROWS) && (a->src_rows <= 0 || a->src_rows > a->s || a->src_rows <= a->s - 128)) return FL_ERR_BAD_ARG;
   return FL_OK;
 }
 

@@ -26,6 +26,7 @@ extern "C" {
 #define FL_Q_HADAMARD_NVFP4_ONLY 4 /* rotate only the values of the NVFP4 copy; the E4M3 codes stay unrotated */
 #define FL_Q_O_PACKED 8            /* packed source with the prologue: o has x's packed rows (else the outputs' rows) */
 #define FL_Q_D_PER_FACTOR 32       /* with FL_Q_TOKEN_LOCAL and the prologue: d_out divided by the token's factor */
+#define FL_Q_ROWS 64               /* no slot tables: x and o have src_rows rows per batch row, see there */
 #define FL_Q_LEGACY 16             /* keep the four-lanes-per-row kernel where the one-thread-per-row kernel would serve
                                       (the two are bit-identical; for tests that compare them) */
 /* Columns of a row of x and o when they are fewer than d (a multiple of 8; bits 16.. of the flags): the missing columns read
@@ -66,7 +67,8 @@ typedef struct fl_quant_args {
    * of s rows; slot_src[i] = first row of x that goes to rows [128 i, 128 i + 128) of the outputs (-1: the slot is
    * empty), slot_rows[i] = how many of them are real (the others quantise as zeros). Replaces the row gather of
    * flash_attn/cute/lp_docmaps.py (the quantisers read Q / K / V / dO through the row map). NULL = x has the outputs' rows, or, with
-   * src_rows > 0, that many of each batch row's (s: those rounded up to whole tiles; the missing rows, of o too, read as zeros). */
+   * FL_Q_ROWS, src_rows of each batch row's (s: those rounded up to whole tiles; the missing rows, of o too, read as zeros); without
+   * the flag src_rows is not read. */
   const int32_t* slot_src;
   const int32_t* slot_rows;
   int32_t src_rows;
@@ -96,6 +98,7 @@ int fl_quant_qkv(const fl_quant_args* q, const fl_quant_args* k, const fl_quant_
 #define FL_A_HAD_DQ 16       /* backward: dQ accumulator holds rotated rows (post kernel rotates back) */
 #define FL_A_HAD_DK 32       /* backward: rotate dK back in the epilogue */
 #define FL_A_COLS(n) ((int32_t)(n) << 16) /* columns of a row of out / dk / dv when they are fewer than d (see FL_Q_COLS) */
+#define FL_A_ROWS 512        /* batched form: out_rows rows per batch row, see there */
 #define FL_A_P_GROUP 64      /* forward: group-frame P-hat (one UE8M0 exponent per query row and 32 keys) instead of the row frame */
 #define FL_A_D_PER_FACTOR 256 /* backward with FL_A_TOKEN_LOCAL: d_rows are divided by f_dO (FL_Q_D_PER_FACTOR): two loads and two products fewer a pair of scores */
 
@@ -166,8 +169,8 @@ typedef struct fl_attn_args {
    * documents stored back to back; slot_src[i] = the packed row of row 128 i of the aligned buffer the kernels work in
    * (-1: an empty slot), slot_rows[i] = how many rows of that slot are real. A full slot leaves as one TMA store, a
    * document's last rows as row stores. NULL = the outputs have the aligned buffer's rows. lse keeps those rows.
-   * Batched form: out_rows > 0 is the number of queries and keys of a batch row where s_q = s_k is that rounded up to whole tiles:
-   * out, dk and dv are (b, out_rows, heads, d), every intermediate and lse have s_q rows. */
+   * Batched form with FL_A_ROWS: out_rows is the number of queries and keys of a batch row where s_q = s_k is that rounded up to whole
+   * tiles: out, dk and dv are (b, out_rows, heads, d), every intermediate and lse have s_q rows. Without the flag out_rows is not read. */
   const int32_t* slot_src;
   const int32_t* slot_rows;
   int32_t out_rows;

@@ -74,3 +74,25 @@ def test_more_batch_rows_than_a_grid_has_in_y_and_z(s, d):
     assert F.check_status() == 0
     for got, want in zip(many, step(two)):
         assert torch.equal(got.view(b // 2, 2, s, 1, d), want.view(1, 2, s, 1, d).expand(b // 2, -1, -1, -1, -1))
+
+
+@pytest.mark.parametrize("rows", [3, 250, 1 << 20, -7])
+@pytest.mark.parametrize("d", [64, 128])
+def test_rows_of_the_c_entries_are_read_with_their_flag(rows, d, monkeypatch):
+    """src_rows and out_rows hold anything where neither slot tables nor FL_Q_ROWS / FL_A_ROWS ask for them."""
+    from flamia_blackwell_attention_b200 import _lib as L
+    from test_gpu_bwd import run_step
+    x = attention_inputs(1, 256, 2, 1, d, seed=24)
+    want = run_step(*x, True)
+
+    class Quant(L.QuantArgs):
+        def __init__(self):
+            super().__init__(src_rows=rows)
+
+    class Attn(L.AttnArgs):
+        def __init__(self):
+            super().__init__(out_rows=rows)
+    monkeypatch.setattr(L, "QuantArgs", Quant)
+    monkeypatch.setattr(L, "AttnArgs", Attn)
+    for got, w in zip(run_step(*x, True), want):
+        assert torch.equal(got, w)
