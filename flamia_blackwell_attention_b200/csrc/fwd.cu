@@ -173,18 +173,19 @@ __device__ __forceinline__ void fwd_decode(const FwdParams& p, int L, Tile& t) {
 }
 
 // FULL: the variants that also serve packed outputs and the output-row factor, each behind a run-time check of its
-// pointer. A template flag, so that the kernels of the plain calls carry none of that code (-2 % kernel time).
+// pointer. A template flag, so that the kernels of the plain calls carry none of that code (-2 % kernel time). 2: short documents (fwd_launch),
+// whose slots mostly leave row by row: both boxes of a full slot through the Q buffer, waited for.
 // TLV (token-local): 1 = the per-key factors come from three float tables, 2 = from the narrow ones. What bounds these kernels is the
 // wait for the table loads (long scoreboard 3.0 of the 9.0 clocks a warp takes to an instruction, no pipe above half): a broadcast load
 // of 16 bytes returns 512 to a warp, and three float tables are 96 of them per 128 keys, the narrow ones 48 (the quantiser's factors
 // are powers of two, their logarithms small integers: bfloat16 holds them exactly, a shift or a mask takes each one out again, and the
 // results are the same bits; long scoreboard 1.5 of 6.4). b2 s8192 h32/8 d128 causal, one B200: 1725 -> 1475 us. 1 serves callers of
 // fl_fwd with tables of their own, in 32 bits.
-template <int D, bool FP4, int TLV, bool GF, bool SC, bool FULL = false>
+template <int D, bool FP4, int TLV, bool GF, bool SC, int FULL = 0>
 __global__ void __launch_bounds__(384, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
            const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const FwdParams p) {
-  constexpr bool TL = TLV != 0;
+  constexpr bool TL = TLV != 0, TWO_BOXES = D == 128 && FULL != 2;
   constexpr int TILE_BYTES = 128 * D;
   constexpr uint64_t SWZ = (D == 128) ? SWZ_128 : SWZ_64;
   constexpr uint32_t SBO = 8 * D;                       // bytes between 8-row groups
@@ -193,8 +194,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
   uint8_t* sQ = smem;                                   // [item buffer 2][stage 2] x Q_STRIDE
   uint8_t* sK = sQ + 4 * Q_STRIDE;                      // KV_STAGES tiles
   uint8_t* sV = sK + KV_STAGES * TILE_BYTES;            // KV_STAGES tiles
-  uint8_t* sO = sV + KV_STAGES * TILE_BYTES;            // d = 128: [stage 2] x Q_STRIDE, the second box of the output rows
-  uint8_t* sSF = sO + (D == 128 ? 2 * Q_STRIDE : 0);    // FP4: scale atoms, Q [item buffer 2] x 2 KB then K KV_STAGES x 1 KB
+  uint8_t* sO = sV + KV_STAGES * TILE_BYTES;            // TWO_BOXES: [stage 2] x Q_STRIDE, the second box of the output rows
+  uint8_t* sSF = sO + (TWO_BOXES ? 2 * Q_STRIDE : 0);   // FP4: scale atoms, Q [item buffer 2] x 2 KB then K KV_STAGES x 1 KB
   constexpr int SF_K = 4096;                            // offset of the K atoms inside sSF
   constexpr int OP_BYTES = FP4 ? TILE_BYTES / 2 : TILE_BYTES;   // bytes of one Q / K operand tile (4-bit codes: half)
   __shared__ __align__(8) uint64_t bars[B_COUNT];
@@ -255,7 +256,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         // output rows out of it and everyone has read the slot
         if (k >= 2 && !(ok = mbar_wait(&bars[B_QE + kb], ((k >> 1) - 1) & 1, p.ctl, abortp, 12))) break;
         Tile t;
-        fwd_decode<FULL>(p, L, t);
+        fwd_decode<(FULL != 0)>(p, L, t);
         tile_s[kb] = t;
         const int hkv = t.hkv;
         if (t.nq > 0) {
@@ -664,10 +665,10 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         tc_wait_st();
         tc_fence_before();
         mbar_arrive_warp(&bars[B_PFULL + i]);
-        confirm();
+        if (FULL != 2) confirm();
       }
       if (!ok) break;
-      confirm();                         // (an item without tiles)
+      if (FULL != 2) confirm();          // (an item without tiles)
       // ---- item epilogue: O / l -> bf16 rows through this stage's Q tile buffer, LSE
       if (n_i > 0) {
         if (!(ok = mbar_wait(&bars[B_PVDONE + i], cd & 1, p.ctl, abortp, 34 + i))) break;
@@ -678,7 +679,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
       const bool row_valid = (128 * i + r) < T.nq;
       const bool stage_present = T.nq > 128 * i;        // (warpgroup-uniform) an absent stage's rows belong to someone else
       const float inv_l = ((l_sum > 0.f) ? 1.0f / l_sum : 0.f) * ((FULL && p.o_mult) ? p.o_mult[T.bat * p.h_kv + T.hkv] : 1.0f);
-      auto stage_of = [&](int cc) { return cc < 2 ? sQ + (2 * kb + i) * Q_STRIDE : sO + i * Q_STRIDE; };
+      auto stage_of = [&](int cc) { return !TWO_BOXES || cc < 2 ? sQ + (2 * kb + i) * Q_STRIDE : sO + i * Q_STRIDE; };
       // packed output: this stage's 128 rows are slot (T.q0 + 128 i) / 128 of the aligned buffer; they go to the packed
       // rows out_row .. + out_n of the caller's tensor: a full slot as TMA stores, a document's last rows row by row
       int out_row = T.q0 + 128 * i, out_n = stage_present ? 128 : 0;
@@ -732,6 +733,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         if (r == 0 && out_n == 128) {
           tma_store_4d(&tm_o, stage_of(cc), 32 * (cc - 1), head, out_row, T.bat);
           tma_store_commit();
+          if (FULL == 2) tma_store_wait_read<0>();
+        }
+        if (FULL == 2 && cc + 1 < D / 32) {
+          mbar_arrive_warp(&bars[B_EPI + i]);           // the buffer has been read: the next box may take it
+          if (!(ok = mbar_wait(&bars[B_EPI + i], epi & 1, p.ctl, abortp, 38))) break;
+          ++epi;
         }
       }
       if (!ok) break;
@@ -741,7 +748,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         p.lse[((size_t)T.bat * p.h + head) * p.s_q + qrow] = v;
       }
       tc_fence_before();                 // this stage's output has left tensor memory before the next item's P-hat is announced
-      if ((warp & 3) || by_rows) mbar_arrive_warp(&bars[B_QE + kb]);     // (by rows: no copy reads the buffer)
+      if (FULL == 2 || (warp & 3) || by_rows) mbar_arrive_warp(&bars[B_QE + kb]);     // (by rows: no copy reads the buffer)
       else pend = kb;
     }
     if (r == 0) tma_store_wait_read<0>();   // (shared memory must outlive the copies; the writes complete with the grid)
@@ -827,7 +834,12 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, con
   p.div_h = FastDiv(a->h);
   p.div_grp = FastDiv(a->h / a->h_kv);
   const int grid = (int)(n_items < sm_count() ? n_items : sm_count());     // one persistent CTA per SM
-  const int smem = (a->d == 128 ? 6 : 4) * Q_STRIDE + 2 * KV_STAGES * 128 * a->d + 1024 + (fp4 ? 4096 + KV_STAGES * 1024 : 0);
+  // Documents of up to 192 rows on average, where fewer slots are full than not: the second output box and what is owed to the producer between
+  // items cost them more than the full slots gain. One B200, quantiser and forward, us, two boxes / one: 8 documents of 30 to 60 rows h16/4
+  // 14.37 / 14.20, 33 of 30 to 120 h20/5 42.1 / 41.4, mixed route 50.0 / 49.1, 300 of 30 to 60 h16 286 / 281, 33 of 100 to 300 mixed route 69.9
+  // / 69.5; and 16 of 384 h12/4 41.3 / 41.8, 40 of 250 to 520 h8 78.0 / 78.5. (Token factors do not go with documents.)
+  const bool padded = a->slot_src && !tl && a->out_rows < 192ll * a->n_docs;
+  const int smem = (a->d == 128 && !padded ? 6 : 4) * Q_STRIDE + 2 * KV_STAGES * 128 * a->d + 1024 + (fp4 ? 4096 + KV_STAGES * 1024 : 0);
   cudaStream_t st = (cudaStream_t)stream;
   auto launch = [&](auto kern) -> int {
     if (int e = set_smem(kern, smem, "fl_fwd: cudaFuncSetAttribute")) return e;
@@ -841,7 +853,9 @@ static int fwd_launch(const fl_attn_args* a, const void* work, void* stream, con
   // the lean kernels serve the plain calls; documents, packed outputs and the output-row factor take the full variant
   const bool full = a->doc_start != nullptr || a->o_mult != nullptr;
 #define FL_FWD_LAUNCH(D_, FP4_, TL_, GF_, SC_) \
-  (full ? launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, true>) : launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, false>))
+  (padded ? launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, TL_ ? 0 : 2>) \
+   : full ? launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, 1>)           \
+          : launch(fwd_kernel<D_, FP4_, TL_, GF_, SC_, 0>))
   if (sc) {
     if (fp4) rc = gf ? FL_FWD_LAUNCH(128, true, 0, true, true) : FL_FWD_LAUNCH(128, true, 0, false, true);
     else if (a->d == 128) rc = gf ? FL_FWD_LAUNCH(128, false, 0, true, true) : FL_FWD_LAUNCH(128, false, 0, false, true);

@@ -1,5 +1,5 @@
 """Quantiser launches of more tiles than three rounds, whose warps past a document's end write zeros and do nothing else, against launches
-that treat every row alike, bit for bit."""
+that treat every row alike; and the forward's form for short documents against its other ones: bit for bit."""
 import pytest
 import torch
 
@@ -65,3 +65,34 @@ def test_prologue(d, o_packed):
             assert torch.equal(many["codes"][:, :, i].view(torch.uint8), one["codes"][:, :, 0].view(torch.uint8))
             _same({k: many[k][:, i].contiguous() for k in ("fac", "D", "lse_log2", "tile_stats")},
                   {k: one[k][:, 0].contiguous() for k in ("fac", "D", "lse_log2", "tile_stats")}, ("fac", "D", "lse_log2", "tile_stats"))
+
+
+@pytest.mark.parametrize("lens", [[1, 127, 128, 129, 2, 256, 64, 130, 3], [40] * 30 + [128, 384], [190, 193] * 4])
+@pytest.mark.parametrize("entry,d,kw", [("fp8", 128, dict(causal=True)), ("fp8", 64, dict()), ("fp8", 80, dict(causal=True, softcap=20.0)),
+                                        ("fp8", 128, dict(causal=True, window_size=(60, 0))), ("fp4", 128, dict(causal=True)), ("fp4", 128, dict())])
+def test_forward(lens, entry, d, kw):
+    """Documents of fewer than 192 rows on average, against the same documents with a long one behind them that lifts the average."""
+    import flamia_blackwell_attention_b200 as F
+    fn = F.flash_attn_fp4 if entry == "fp4" else F.flash_attn_fp8
+    long = lens + [192 * (len(lens) + 1)]
+    x = [t[0].cuda() for t in attention_inputs(1, sum(long), 4, 2, d, seed=63)[:3]]
+    (o, lse), (ol, lsel) = _forward(fn, x, lens, **kw), _forward(fn, x, long, **kw)
+    assert F.check_status() == 0
+    n = sum(lens)
+    assert torch.equal(o, ol[:n]) and torch.equal(lse, lsel[:, :n])
+
+
+def _forward(fn, x, lens, **kw):
+    import flamia_blackwell_attention_b200 as F
+    maps = F.DocMaps.from_cu_seqlens(torch.tensor([0] + lens, dtype=torch.int32).cumsum(0, dtype=torch.int32)).to("cuda")
+    with torch.no_grad():
+        return fn(*(t[:sum(lens)] for t in x), doc_maps=maps, return_lse=True, **kw)
+
+
+def test_which_documents_are_short(tmp_path):
+    import flamia_blackwell_attention_b200 as F
+    from launches import launches
+    x = [torch.zeros(400, 1, 128, dtype=torch.bfloat16, device="cuda") for _ in range(3)]
+    for lens, form in (([191, 192], ", 2>"), ([191, 193], ", 1>")):
+        names = [n for n, _, _ in launches(lambda: _forward(F.flash_attn_fp8, x, lens), tmp_path) if "fwd_kernel" in n]
+        assert len(names) == 1 and form in names[0], names
