@@ -123,8 +123,8 @@ def _run(call, q, k, v, cu_q, cu_k, su_q, su_k, return_lse, doc_maps=None):
                 _fail("B8", NotImplementedError, f"packed documents are self-attention documents here: pass the SAME tensor "
                                                  f"as {name}_q and {name}_k (distinct query / key tables are not built)")
     if plan.fwd.ragged_documents and sh.s_q != sh.s_k:
-        _fail("B8", NotImplementedError, "lengths that are no multiple of 128 run the batch rows as self-attention "
-                                         f"documents: s_q must equal s_k; got {sh.s_q} and {sh.s_k}")
+        _fail("B8", NotImplementedError, "lengths that are no multiple of 128 are built for self-attention: s_q must equal s_k; "
+                                         f"got {sh.s_q} and {sh.s_k}")
     if sh.varlen and not sh.aligned_varlen and doc_maps is None and not _REPACK_WARNED:
         _REPACK_WARNED = True
         warnings.warn(REPACK_WARNING.format(entry=plan.entry), UserWarning, stacklevel=3)

@@ -53,9 +53,10 @@
 // take f_K f_Q and f_V f_dO in the elementwise math; dV takes f_dO inside a block-scaled P-hat (one exponent per key row
 // x 32 queries); dK takes f_Q inside its dS-hat codes, dQ takes f_K inside its own; the operand scale tiles are unit.
 // What bounds these kernels are the loads of the per-query tables: each returns 512 bytes to a warp, four clocks of the 2 350 of a half
-// tile, and eight warps took 48 each. VAR = 3 (FL_A_D_PER_FACTOR: D'' comes divided by f_dO, exactly, as f_dO is a power of two) takes
-// 40: P' f_dO, which P-hat needs, is all that dS = (P' f_dO) (f_V dP + D'' / f_dO) needs, too. b2 s8192 h32/8 d128 causal step, one B200:
-// 4062 -> 3923 us, 56 of the 139 from fewer live registers (VAR = 2 has these as well), same bits. VAR = 2 serves callers with D'' as it is.
+// tile. VAR = 3 (FL_A_D_PER_FACTOR: D'' comes divided by f_dO, exactly, as f_dO is a power of two) takes 40 of them a warp: P' f_dO, which
+// P-hat needs, is all that dS = (P' f_dO) (f_V dP + D'' / f_dO) needs, too. VAR = 2, for callers with D'' as it is, takes 56 (48 if P' f_dO is
+// kept for its codes, in 32 registers more, which costs 1 to 3 %). b2 s8192 h32/8 d128 causal, kernel alone, one B200: VAR = 2 with 48 loads
+// 2445 us, with 56 2381 to 2431, VAR = 3 2325 to 2360; the same bits.
 #include "flamia_internal.h"
 
 namespace fl {
@@ -779,7 +780,7 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           const float sc[4] = {sc4.x, sc4.y, sc4.z, sc4.w};
           // (the words' sixteen instructions, once in the producer: d = 64 8 x 1024 x 12 93.2 -> 91.7 us, mixed route b4 s4096 h16 503 -> 496)
           const float2 words = *reinterpret_cast<const float2*>(&misc.scal[st][x][4]);
-          if constexpr (SC && D == 128) {        // from the factors (mixed route b5 s1536 h4/1 dense 126 -> 119 us, 8-bit 1 %, d = 64 +0.6 %)
+          if constexpr (SC && D == 128) {        // from the factors (b5 s1536 h4/1 dense, mixed route 127 -> 120 us, 8-bit 120 -> 119; d = 64 +0.6 %)
             auto e8 = [](float f) { return (__float_as_uint(f) >> 23) & 0xFF; };
             eq2 = e8(sc[0]) | (e8(sc[1]) << 8);
             edo2 = e8(sc[2]) | (e8(sc[3]) << 8);
@@ -803,9 +804,9 @@ bwd_kernel_pipelined(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
           return true;
         };
         // Where the scores are waited for anyway, what they are not needed for stands behind their load from tensor memory, which takes its
-        // time: of an iteration of 3250 clocks the masks took 250 and the row vectors 130 (b4 s4096 h16: 554 -> 544 us, masks alone
-        // 548). Not where registers are short or the order of waits matters more: mixed route masks alone (both: +0.3 %), d = 64 +1 %, token-local
-        // +5 %.
+        // time: of an iteration of 3250 clocks the masks took 250 and the row vectors 130 (b4 s4096 h16 causal, kernel alone: 467 ->
+        // 460.5 us, masks alone 462.6; dense 821 -> 809). Not where registers are short or the order of waits matters more: mixed route masks
+        // alone (475 us either way, both +0.3 %), d = 64 +1 %, token-local +5 %.
         constexpr bool LATE_MASK = D == 128 && VAR == 0 && !SC, LATE_VEC = LATE_MASK && !FP4;
         if constexpr (!LATE_MASK) masks();
         if constexpr (!LATE_VEC) {

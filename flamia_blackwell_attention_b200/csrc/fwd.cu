@@ -546,8 +546,8 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         float gm[4];                                             // the four 32-key groups' maxima (scaled)
 #pragma unroll
         for (int kbk = 0; kbk < 4; ++kbk) {
-          // a tree of three-input maxima (sixteen instructions, four deep; b4 s4096 h16, against twenty of mixed ones: dense 391 -> 386
-          // us, causal mixed route 227 -> 220)
+          // a tree of three-input maxima (sixteen instructions, four deep; b4 s4096 h16, kernel alone, against twenty of mixed ones: dense
+          // 369 -> 363 us, causal 202.7 -> 202, causal mixed route 229 -> 220)
           const float* z = s + 32 * kbk;
           float a[10];
 #pragma unroll

@@ -60,7 +60,7 @@ class FwdSpec:
     causal: bool
     varlen: bool
     aligned_varlen: bool
-    ragged_documents: bool
+    ragged_documents: bool # batch rows that are no whole tiles (run as batch rows; the field's name is from when they ran as documents)
     return_lse: bool
     window: Optional[tuple] = None
     softcap: float = 0.0
@@ -174,8 +174,8 @@ def _common(entry, shape, log, *, causal, window_size, softcap, score_mod, score
         if shape.varlen:
             _fail("B9", ValueError, f"flash_attn_{entry}: the aligned varlen form takes seqused_q AND seqused_k")
         if shape.s_q % 128 or shape.s_k % 128:
-            _fail("B4", NotImplementedError, "batched seqused_k with lengths that are no multiple of 128 is not built "
-                                             f"(those run as documents); got {shape.s_q} / {shape.s_k}")
+            _fail("B4", NotImplementedError, "batched seqused_k with lengths that are no multiple of 128 is not built; "
+                                             f"got {shape.s_q} / {shape.s_k}")
         if scaling_request(o) == "token_local":
             _fail("B4", NotImplementedError, "batched seqused_k with operand_scaling='token_local' is not built")
         if isinstance(seqused_k, torch.Tensor) and (seqused_k.dim() != 1 or seqused_k.shape[0] != shape.b or
@@ -258,8 +258,8 @@ def _common(entry, shape, log, *, causal, window_size, softcap, score_mod, score
         _fail(15, ValueError, "forward_two_cta='on' but the forward on CTA pairs is not built here")
     ragged = (not shape.varlen) and (shape.s_q % 128 != 0 or shape.s_k % 128 != 0)
     if scaling == "token_local" and ragged:
-        _fail(16, ValueError, "operand_scaling='token_local' runs the fold forward, which takes no documents: lengths that "
-                              f"are no multiple of 128 run as documents; got {shape.s_q} / {shape.s_k}")
+        _fail(16, ValueError, "operand_scaling='token_local' runs the fold forward, which takes no documents and no lengths that "
+                              f"are no multiple of 128; got {shape.s_q} / {shape.s_k}")
     if shape.d != 128 and shape.requires_grad and (rowlocal == "all" or scaling == "token_local"):
         _fail("B6", NotImplementedError, "ds_dq_rowlocal='all' (and with it operand_scaling='token_local') is built in "
                                          f"the head_dim 128 backward; this call runs at head_dim {shape.d}")

@@ -100,7 +100,7 @@ int fl_quant_qkv(const fl_quant_args* q, const fl_quant_args* k, const fl_quant_
 #define FL_A_COLS(n) ((int32_t)(n) << 16) /* columns of a row of out / dk / dv when they are fewer than d (see FL_Q_COLS) */
 #define FL_A_ROWS 512        /* batched form: out_rows rows per batch row, see there */
 #define FL_A_P_GROUP 64      /* forward: group-frame P-hat (one UE8M0 exponent per query row and 32 keys) instead of the row frame */
-#define FL_A_D_PER_FACTOR 256 /* backward with FL_A_TOKEN_LOCAL: d_rows are divided by f_dO (FL_Q_D_PER_FACTOR): two loads and two products fewer a pair of scores */
+#define FL_A_D_PER_FACTOR 256 /* backward with FL_A_TOKEN_LOCAL: d_rows are divided by f_dO (FL_Q_D_PER_FACTOR): two table loads fewer for every four scores */
 
 /* One attention problem. Operands are the quantiser's outputs; q / k / v / dO codes are (b, s, heads, d) E4M3. */
 typedef struct fl_attn_args {
@@ -261,7 +261,8 @@ int fl_bwd_static_acc(const fl_attn_args* args, const float* post_scale, float m
 
 /* Tables of packed documents laid out at 128-aligned starts of a buffer of `capacity` rows (capacity % 128 == 0), in one launch
  * (the counterpart of the reference's per-call map building, flash_attn/cute/lp_docmaps.py:107): cu (n_docs + 1) int32
- * boundaries in the packed rows, or NULL = n_docs documents of fixed_len rows; total = packed rows. Writes start / len
+ * boundaries in the packed rows, or NULL = n_docs documents of fixed_len rows (for hosts that run batch rows as documents; this library's
+ * own calls give the boundaries); total = packed rows. Writes start / len
  * (n_docs), row_map (capacity; packed row of each buffer row, -1 = padding) and slot_src / slot_rows (capacity / 128). */
 int fl_doc_tables(const int32_t* cu, int32_t n_docs, int32_t fixed_len, int32_t total, int32_t capacity, int32_t* start, int32_t* len,
                   int32_t* row_map, int32_t* slot_src, int32_t* slot_rows, void* stream);
@@ -283,7 +284,8 @@ int fl_fwd_work(const fl_attn_args* args, const int32_t* work, void* stream);
 int fl_bwd_work(const fl_attn_args* args, const int32_t* work, void* stream);
 
 /* The live rows of the aligned buffer's LSE (h, capacity) in the caller's rows: packed row g goes to out[g / seq][head][g % seq]
- * (packed documents: seq = total, out is (h, total); batch rows run as documents: seq = s, out is (b, h, s)). */
+ * (packed documents: seq = total, out is (h, total), as this library's own calls have it; a host that runs batch rows as documents:
+ * seq = s, out is (b, h, s)). */
 int fl_unpack_lse(const float* lse, const int32_t* slot_src, const int32_t* slot_rows, int32_t capacity, int32_t h, int32_t seq,
                   int32_t total, float* out, void* stream);
 

@@ -452,7 +452,7 @@ def test_lse_of_repacked_documents_and_ragged_batch_rows(route):
         assert lse.shape == (h, total) and lse.dtype == torch.float32
         err = (lse.cpu() - ref).abs()
         assert float(err.max()) < tol and float(err.median()) < typ
-    if route == "fp8":                               # batch rows of 200 tokens run as documents
+    if route == "fp8":                               # batch rows of 200 tokens, no whole tiles
         q, k, v, g = attention_inputs(3, 200, h, hk, d, seed=42)
         with torch.no_grad():
             out, lse = fn(q.cuda(), k.cuda(), v.cuda(), causal=True, return_lse=True)

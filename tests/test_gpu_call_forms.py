@@ -14,7 +14,7 @@ def _step(fn, q, k, v, do, **kw):
     return (out.detach(), *torch.autograd.grad(out, (q, k, v), do))
 
 
-@pytest.mark.parametrize("s", [256, 1000])             # whole tiles; batch rows run as documents
+@pytest.mark.parametrize("s", [256, 1000])             # whole tiles; batch rows that are none
 @pytest.mark.parametrize("window,same", [((2 ** 31 - 2, 2 ** 31 - 2), (None, None)), ((2 ** 31 - 2, 100), (None, 100)),
                                          ((100, 2 ** 31 - 2), (100, None)), ((2 ** 33 + 5, 2 ** 31 - 1), (None, None))])
 def test_window_longer_than_any_sequence(s, window, same):

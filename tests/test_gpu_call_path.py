@@ -69,6 +69,24 @@ def test_document_tables_in_one_launch(lens):
     assert torch.equal(lse[:, rows[rows >= 0]], st[0][0][:, rows >= 0])
 
 
+@pytest.mark.parametrize("b,s,h", [(1, 1, 1), (3, 127, 2), (5, 128, 1), (2, 300, 3), (40, 129, 1)])
+def test_documents_of_one_length(b, s, h):
+    """The forms for hosts that run batch rows as documents: fl_doc_tables without boundaries, fl_unpack_lse into (b, h, s)."""
+    from flamia_blackwell_attention_b200 import _lib as L
+    total, capacity = b * s, b * ((s + 127) // 128 * 128)
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def tables(cu):
+        t = [torch.full((n,), 7, dtype=torch.int32, device="cuda") for n in (b, b, capacity, capacity // 128, capacity // 128)]
+        L.check(L.load().fl_doc_tables(L.ptr(cu), b, s if cu is None else 0, total, capacity, *(L.ptr(x) for x in t), stream), "fl_doc_tables")
+        return t
+    got, want = tables(None), tables(torch.arange(0, total + 1, s, dtype=torch.int32, device="cuda"))
+    assert all(torch.equal(x, y) for x, y in zip(got, want))
+    lse, out = torch.randn(h, capacity, device="cuda"), torch.empty(b, h, s, device="cuda")
+    L.check(L.load().fl_unpack_lse(L.ptr(lse), L.ptr(got[3]), L.ptr(got[4]), capacity, h, s, total, L.ptr(out), stream), "fl_unpack_lse")
+    assert torch.equal(out, lse.view(h, b, -1)[..., :s].transpose(0, 1))
+
+
 @pytest.mark.parametrize("b,h,hk,nt,causal", [(1, 1, 1, 1, False), (3, 5, 5, 7, False), (2, 16, 4, 40, False), (2, 3, 1, 9, True)])
 def test_dq_prescale_of_many_tiles(b, h, hk, nt, causal):
     """The pre-scale table against the maxima taken directly (the bound's arithmetic itself is pinned elsewhere)."""

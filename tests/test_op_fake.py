@@ -21,7 +21,7 @@ CASES = [
     ("fp8", dict(causal=True), (2, 256, 4, 2, 128), True, None),
     ("fp4", dict(causal=True), (1, 384, 2, 2, 128), True, None),
     ("fp8", dict(causal=True, options="tl"), (1, 256, 4, 1, 128), True, None),
-    ("fp8", dict(causal=True), (2, 300, 2, 2, 128), True, None),               # ragged: runs as documents
+    ("fp8", dict(causal=True), (2, 300, 2, 2, 128), True, None),               # batch rows that are no whole tiles
     ("fp8", dict(causal=True), (1, 1020, 2, 2, 128), True, [300, 128, 77, 515]),  # packed, repacked
 ]
 
